@@ -5,125 +5,78 @@
 // (models/clt.py:629-709 of the reference project, which runs one dense or CSR product per (s, t) pair and one
 // all-reduce per target layer). Here the codes of a token are one padded list of (c = s * F + f, value) pairs, and
 //
-//   clt_decode_kernel   one CTA per (token, target layer) gathers the rows W_D[t][s, f, :] of that token's codes with
-//                       s <= t and accumulates them in registers: every target layer in one launch, no dense product;
+//   clt_decode_kernel   warps of a (token, target layer) gather the rows W_D[t][s, f, :] of that token's codes with
+//                       s <= t and accumulate them in registers: every target layer in one launch, no dense product;
 //   clt_dact_kernel     d a[b, j] = sum_{t >= s} d y[t, b, :] . W_D[t][s, f, :]   (one CTA per token, a warp per code);
 //   clt_wgrad_kernel    d W_D[t][s, f, :] = sum_{b in rows(c)} a[b, c] * d y[t, b, :] for every t >= s from the
 //                       by-feature lists of a counting sort: one CTA per active (s, f), no atomics; rows of features
 //                       that did not fire are not touched (the caller hands in zero-filled gradients).
 //
 // W_D[t] is its own allocation of shape [t + 1, F, d] (bf16); the kernels take the table of base pointers by value.
-#include "common.cuh"
+#include "gather.cuh"
 #include "kernels.h"
 
 namespace lmsae {
 
-namespace {
-
-__device__ __forceinline__ void bf16x8_unpack(const uint4& u, float (&f)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(h[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-
-constexpr int CLT_MAX_VEC = 2;  // 16-byte chunks of a row owned by one thread
-
-}  // namespace
-
 // ---------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512)
-clt_decode_kernel(const CltTable tab, const int* __restrict__ idx, const float* __restrict__ val, int B, int K, int L,
-                  int F, int d, const float* __restrict__ bias, float* __restrict__ out_f32,
-                  __nv_bfloat16* __restrict__ out_bf16) {
-  extern __shared__ uint8_t smem_raw[];
-  int* s_idx = reinterpret_cast<int*>(smem_raw);            // [K]
-  float* s_val = reinterpret_cast<float*>(smem_raw) + K;    // [K]
-  const int nvec = d / 8;
-  const long long items = (long long)B * L;
-  for (long long w = blockIdx.x; w < items; w += gridDim.x) {
-    const int row = (int)(w / L);
-    const int t = L - 1 - (int)(w % L);  // deepest target (longest list) first
-    __syncthreads();
-    for (int j = threadIdx.x; j < K; j += blockDim.x) {
-      s_idx[j] = idx[(size_t)row * K + j];
-      s_val[j] = val[(size_t)row * K + j];
-    }
-    __syncthreads();
-    const __nv_bfloat16* Wt = tab.W[t];
-    const long long limit = (long long)(t + 1) * F;  // codes c < limit come from source layers s <= t
-    float acc[CLT_MAX_VEC][8];
-#pragma unroll
-    for (int u = 0; u < CLT_MAX_VEC; ++u)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[u][i] = 0.0f;
-    for (int j = 0; j < K; ++j) {
-      const int c = s_idx[j];
-      if (c < 0 || c >= limit) continue;
-      const float a = s_val[j];
-      const uint4* wrow = reinterpret_cast<const uint4*>(Wt + (size_t)c * d);
-#pragma unroll
-      for (int u = 0; u < CLT_MAX_VEC; ++u) {
-        const int v = threadIdx.x + u * blockDim.x;
-        if (v < nvec) {
-          float wv[8];
-          bf16x8_unpack(__ldg(wrow + v), wv);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[u][i] = fmaf(a, wv[i], acc[u][i]);
-        }
-      }
-    }
-    const size_t obase = ((size_t)t * B + row) * d;
-#pragma unroll
-    for (int u = 0; u < CLT_MAX_VEC; ++u) {
-      const int v = threadIdx.x + u * blockDim.x;
-      if (v < nvec) {
-        const int c0 = v * 8;
-        if (bias != nullptr) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[u][i] += bias[(size_t)t * d + c0 + i];
-        }
-        if (out_f32 != nullptr) {
-          float4* o = reinterpret_cast<float4*>(out_f32 + obase + c0);
-          o[0] = make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
-          o[1] = make_float4(acc[u][4], acc[u][5], acc[u][6], acc[u][7]);
-        }
-        if (out_bf16 != nullptr) {
-          uint4 o;
-          o.x = pack_bf16x2(acc[u][0], acc[u][1]);
-          o.y = pack_bf16x2(acc[u][2], acc[u][3]);
-          o.z = pack_bf16x2(acc[u][4], acc[u][5]);
-          o.w = pack_bf16x2(acc[u][6], acc[u][7]);
-          *reinterpret_cast<uint4*>(out_bf16 + obase + c0) = o;
-        }
-      }
-    }
-  }
-}
+// One warp per (target layer, token, segment of 256 columns), ordered by target layer: all tokens of a layer are resident at
+// once and walk their lists, which are ordered by source layer, in step, so that the rows gathered at any time come from a
+// few [F, d] slices of W_D[t] that fit the L2 cache. One CTA per token and layer, token by token, read every slice from
+// HBM again for almost every row: 3.29 ms against 1.54 ms here (12 layers x 24576 features, d 768, 2048 tokens, k 64 per layer:
+// 15.7 GB of rows, 10.2 TB/s).
+constexpr int CLT_DEC_WARPS = 8;
 
-static int clt_threads_for(int d) {
-  int t = ((d / 8 + 31) / 32) * 32;
-  if (t > 512) t = ((d / 16 + 31) / 32) * 32;  // two chunks per thread
-  return t < 32 ? 32 : t;
+__global__ void __launch_bounds__(CLT_DEC_WARPS * 32)
+clt_decode_kernel(const CltTable tab, const int* __restrict__ idx, const float* __restrict__ val, int B, int K, int L,
+                  int F, int d, int nseg, const float* __restrict__ bias, float* __restrict__ out_f32,
+                  __nv_bfloat16* __restrict__ out_bf16) {
+  const int lane = threadIdx.x & 31;
+  const int nvec = d / 8;
+  const long long item = (long long)blockIdx.x * CLT_DEC_WARPS + (threadIdx.x >> 5);
+  const long long per_layer = (long long)B * nseg;
+  if (item >= per_layer * L) return;
+  const int layer_rank = (int)(item / per_layer);
+  const int t = L - 1 - layer_rank;  // deepest target (longest lists) first
+  const long long rest = item - (long long)layer_rank * per_layer;
+  const int row = (int)(rest / nseg), seg = (int)(rest - (long long)row * nseg);
+  const int v[1] = {seg * 32 + lane};
+  const bool in[1] = {v[0] < nvec};
+  float acc[1][8];
+  const long long limit = (long long)(t + 1) * F;  // codes c < limit come from source layers s <= t
+  gather_rows_warp<1>(idx + (size_t)row * K, val + (size_t)row * K, K, tab.W[t], d, limit, limit, v, in, acc);
+  if (!in[0]) return;
+  const int c0 = v[0] * 8;
+  const size_t obase = ((size_t)t * B + row) * d;
+  if (bias != nullptr) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[0][i] += bias[(size_t)t * d + c0 + i];
+  }
+  if (out_f32 != nullptr) {
+    float4* o = reinterpret_cast<float4*>(out_f32 + obase + c0);
+    o[0] = make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
+    o[1] = make_float4(acc[0][4], acc[0][5], acc[0][6], acc[0][7]);
+  }
+  if (out_bf16 != nullptr) {
+    uint4 o;
+    o.x = pack_bf16x2(acc[0][0], acc[0][1]);
+    o.y = pack_bf16x2(acc[0][2], acc[0][3]);
+    o.z = pack_bf16x2(acc[0][4], acc[0][5]);
+    o.w = pack_bf16x2(acc[0][6], acc[0][7]);
+    *reinterpret_cast<uint4*>(out_bf16 + obase + c0) = o;
+  }
 }
 
 int clt_decode_launch(const CltTable& tab, const int* idx, const float* val, int B, int K, int L, int F, int d,
                       const float* bias, float* out_f32, __nv_bfloat16* out_bf16, cudaStream_t stream) {
-  if (d % 8 != 0 || d > 512 * CLT_MAX_VEC * 8 || L < 1 || L > kMaxCltLayers) return (int)cudaErrorInvalidValue;
+  if (d % 8 != 0 || d > 8192 || L < 1 || L > kMaxCltLayers) return (int)cudaErrorInvalidValue;
   if ((long long)L * F > 2147483647LL) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)K * 8;
-  if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-  const int threads = clt_threads_for(d);
-  if (threads > 512) return (int)cudaErrorInvalidValue;
-  long long items = (long long)B * L;
-  if (items <= 0) return 0;
-  const int blocks = (int)(items < 148LL * 32 ? items : 148LL * 32);
-  clt_decode_kernel<<<blocks, threads, smem, stream>>>(tab, idx, val, B, K, L, F, d, bias, out_f32, out_bf16);
+  if (B <= 0) return 0;
+  const int nseg = (d / 8 + 31) / 32;
+  const long long blocks = ((long long)B * L * nseg + CLT_DEC_WARPS - 1) / CLT_DEC_WARPS;
+  if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
+  clt_decode_kernel<<<(int)blocks, CLT_DEC_WARPS * 32, 0, stream>>>(tab, idx, val, B, K, L, F, d, nseg, bias, out_f32, out_bf16);
   return (int)cudaGetLastError();
 }
 
@@ -153,7 +106,7 @@ clt_dact_kernel(const CltTable tab, const int* __restrict__ idx, int B, int K, i
       __syncthreads();
       for (int v = threadIdx.x; v < nvec; v += CLT_DACT_THREADS) {
         float f[8];
-        bf16x8_unpack(__ldg(reinterpret_cast<const uint4*>(dy + ((size_t)t * B + row) * d) + v), f);
+        bf16x8_to_float(__ldg(reinterpret_cast<const uint4*>(dy + ((size_t)t * B + row) * d) + v), f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) s_dy[v * 8 + i] = f[i];
       }
@@ -167,7 +120,7 @@ clt_dact_kernel(const CltTable tab, const int* __restrict__ idx, int B, int K, i
         float dot = 0.0f;
         for (int v = lane; v < nvec; v += 32) {
           float wv[8];
-          bf16x8_unpack(__ldg(wrow + v), wv);
+          bf16x8_to_float(__ldg(wrow + v), wv);
           const float* g = s_dy + v * 8;
 #pragma unroll
           for (int i = 0; i < 8; ++i) dot = fmaf(wv[i], g[i], dot);
