@@ -320,7 +320,8 @@ void auxk_loss_grad(const Tensor& xhat, const Tensor& aux_rec, const Tensor& lab
 }
 
 void csc_build(const Tensor& idx, int64_t F, const Tensor& counts, const Tensor& offsets, const Tensor& cursor,
-               const Tensor& entries, const Tensor& block_sums) {
+               const Tensor& entries, const Tensor& block_sums, const c10::optional<Tensor>& heavy) {
+  if (heavy.has_value()) { CHECK_T(*heavy, torch::kInt32); TORCH_CHECK(heavy->numel() >= 1); }
   CHECK_T(idx, torch::kInt32);
   CHECK_T(counts, torch::kInt32);
   CHECK_T(offsets, torch::kInt32);
@@ -332,7 +333,8 @@ void csc_build(const Tensor& idx, int64_t F, const Tensor& counts, const Tensor&
   const c10::cuda::CUDAGuard guard(idx.device());
   check_cuda(lmsae::csc_build_launch(idx.data_ptr<int>(), idx.numel(), (int)F, counts.data_ptr<int>(),
                                      offsets.data_ptr<int>(), cursor.data_ptr<int>(), entries.data_ptr<int>(),
-                                     block_sums.data_ptr<int>(), at::cuda::getCurrentCUDAStream()),
+                                     block_sums.data_ptr<int>(), opt_ptr<int>(heavy),
+                                     heavy.has_value() ? (int)heavy->numel() - 1 : 0, at::cuda::getCurrentCUDAStream()),
              "csc_build launch");
 }
 
@@ -362,7 +364,8 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
                       const c10::optional<Tensor>& pub_done, const c10::optional<Tensor>& extra_row,
                       const c10::optional<Tensor>& extra_gD, const c10::optional<Tensor>& extra_gE,
                       const c10::optional<Tensor>& extra_gb, const c10::optional<Tensor>& wd_self_scale,
-                      const c10::optional<Tensor>& norm_sq_accum) {
+                      const c10::optional<Tensor>& norm_sq_accum, int64_t dact_mode, const c10::optional<Tensor>& heavy,
+                      int64_t heavy_base, const c10::optional<Tensor>& sched) {
   // one-sided launches: the decoder group (WD, mD, vD, WD_bf16) or the encoder group (WE, mE, vE, WE_bf16) may be absent
   const bool has_d = WD_o.has_value(), has_e = WE_o.has_value();
   TORCH_CHECK(has_d || has_e, "at least one of the decoder / encoder groups must be given");
@@ -431,9 +434,14 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
   p.h = make_hyper(lr, beta1, beta2, eps, step);
   p.update = update ? 1 : 0;
   p.ctas_per_sm = (int)ctas_per_sm;
-  // warp-per-row kernel for short rows unless LMSAE_ADAM_ROWWARP=0 (read once)
-  static const int rowwarp = [] { const char* e = std::getenv("LMSAE_ADAM_ROWWARP"); return (e != nullptr && e[0] == '0') ? 0 : 1; }();
-  p.use_rowwarp = rowwarp;
+  TORCH_CHECK(dact_mode >= 0 && dact_mode <= 2 && (dact_mode == 0 || has_d), "code gradients come from the decoder side");
+  p.dact_mode = (int)dact_mode;
+  p.dact_out = dact_mode != 0 ? dact.data_ptr<float>() : nullptr;
+  if (heavy.has_value()) { CHECK_T(*heavy, torch::kInt32); }
+  p.heavy = opt_ptr<const int>(heavy);
+  p.heavy_base = (int)heavy_base;
+  if (sched.has_value()) { CHECK_T(*sched, torch::kInt32); TORCH_CHECK(sched->numel() >= 2); }
+  p.sched = opt_ptr<int>(sched);
   if (status.has_value()) { CHECK_T(*status, torch::kInt32); }
   p.status = opt_ptr<const int>(status);
   if (wd_self_scale.has_value()) { CHECK_T(*wd_self_scale, torch::kFloat32); TORCH_CHECK(wd_self_scale->numel() == p.F); }

@@ -103,8 +103,11 @@ int sparse_dact_launch(const int* idx, int B, int k, int d, int F, const __nv_bf
 int mse_loss_grad_launch(const float* xhat, const __nv_bfloat16* label, const float* bias, const float* row_weight,
                          int rows, int d, float grad_scale, __nv_bfloat16* dxhat, float* loss_sum, float* row_loss,
                          cudaStream_t stream);
+// heavy (optional): [0] = number of features with more than kHeavyRow entries, then those features, in no particular order
+// (at most heavy_cap of them are listed)
 int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offsets, int* cursor, int* entries,
-                     int* block_sums_buf, cudaStream_t stream);
+                     int* block_sums_buf, int* heavy, int heavy_cap, cudaStream_t stream);
+constexpr int kHeavyRow = 64;
 
 struct AdamHyper {
   float lr, beta1, beta2, eps;
@@ -130,7 +133,6 @@ struct GradAdamParams {
   int update;
   int f_begin, f_end;  // feature rows handled by this launch
   int ctas_per_sm;     // 0 = fill the GPU (4 per SM); 1..4 = leave registers free for a concurrently running kernel
-  int use_rowwarp;     // != 0: rows of at most 1024 columns (a multiple of 128) take the warp-per-row kernel
   const int* status;   // kernels' status word: a recorded error turns the update into a no-op (nullptr: not checked)
   // Dense gradient rows for a subset of the features, added to the rows rebuilt from the entry lists: feature f takes
   // row extra_row[f] (when >= 0) of the fp32 matrices extra_gD / extra_gE [rows, d] and element extra_row[f] of extra_gb.
@@ -144,6 +146,17 @@ struct GradAdamParams {
   float* norm_sq_accum;
   const __nv_bfloat16* dxhat_aux;  // output gradient seen by the code slots >= k_main of every row (nullptr: none)
   int k_main;
+  // Code gradients computed by this launch's decoder side from d x_hat and the bf16-rounded rows it updates anyway
+  // (row-streaming kernel only): dact_mode 1 stores them to dact_out, 2 adds them to what is there (one launch per decoder
+  // matrix), 0: off. dact_out may be the array dact points to: the encoder side of the same launch then reads what the
+  // decoder side wrote. Entries with a zero code get 0.
+  int dact_mode;
+  float* dact_out;
+  // Rows with more than kHeavyRow entries: heavy[0] = their number, then their row indices + heavy_base (nullptr: none known).
+  const int* heavy;
+  int heavy_base;
+  int* sched;        // two zero-initialised ints that the kernel leaves at zero: row counter, finished CTAs (nullptr: static deal)
+  int sched_chunk;   // set by the launch
   float* gD_out;  // optional dense [F, d] outputs of the rebuilt gradient rows (for autograd callers)
   float* gE_out;
   // Optimizer state sharded by feature row over data-parallel replicas: this launch owns rows [f_begin, f_end); its
@@ -164,6 +177,8 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
                           const float* alpha_factor, __nv_bfloat16* g_main, __nv_bfloat16* g_aux, float* loss_sum,
                           float* aux_sum, cudaStream_t stream);
 int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream);
+bool grad_adam_rows_supported(const GradAdamParams& p);
+int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream);
 int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cudaStream_t stream);
 int adam_flat_launch(float* p, const float* g, float* m, float* v, long long n, AdamHyper h, const float* grad_mul,
                      __nv_bfloat16* shadow, float* grad_sq_sum, int update, const int* status, cudaStream_t stream);

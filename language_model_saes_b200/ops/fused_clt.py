@@ -12,10 +12,10 @@ tokens) with Adam. How it computes it:
    dense [B, L, F] activations and the 78 per-pair products never exist. Feature shards sum their partial outputs with the
    one-kernel in-place all-reduce over peer memory (``parallel.symm.AllReduceComm``: one reduce of [L, B, d] instead of
    one collective per target layer)
-3. loss and d y in one kernel, d act in one kernel (``clt_dact``), counting sort of the codes by (layer, feature)
+3. loss and d y in one kernel, counting sort of the codes by (layer, feature) (with replicas also d act: ``clt_dact``)
 4. updates: per TARGET layer t one launch of the sparse gradient + Adam kernel over ``W_D[t]`` seen as a
-   ``[(t + 1) F, d]`` matrix (decoder side only: gradient rows rebuilt from the by-feature lists and d y[t], Adam, bf16
-   shadow, squared row norms accumulated into the per-feature norm over target layers); per SOURCE layer one launch over
+   ``[(t + 1) F, d]`` matrix (decoder side only: gradient rows rebuilt from the by-feature lists and d y[t], this layer's
+   share of the code gradients from the same gathered rows, Adam, bf16 shadow, squared row norms accumulated into the per-feature norm over target layers); per SOURCE layer one launch over
    ``W_E[s]`` (encoder side only). No dense gradient tensor exists; the reference materialises one per decoder.
 
 Restrictions: ``topk`` activation with k <= 64, no sparsity loss, Adam, fp32 parameters with bf16 compute. Features may
@@ -278,7 +278,8 @@ class FusedCLTStep:
         n_rows = L * B * self.dp  # (layer, token) pairs of the whole step: every replica brings B tokens
         dy = K.mse_loss_grad(y.view(L * B, d), label.reshape(L * B, d).contiguous(), None, None, 2.0 / n_rows, self.loss_sum)
         dy = dy.view(L, B, d)
-        dact = CK.clt_dact(idx, self.WD_bf16, dy)
+        # one process: every target layer's update launch adds its share of the code gradients before it changes the rows
+        dact = torch.zeros_like(act) if self.dp == 1 else CK.clt_dact(idx, self.WD_bf16, dy)
         if self.dp > 1:
             # Replicas: codes, their gradients, the output gradients and the inputs of every replica are gathered (rows in rank
             # order) and each replica rebuilds the same sparse rows of W_D and W_E from them: the same update everywhere, no
@@ -289,21 +290,19 @@ class FusedCLTStep:
         if self.groups is None or self.groups.entries.numel() < idx.numel():
             self.groups = K.FeatureGroups(L * F, idx.numel(), x.device)
         self.groups.build(idx)
-        off, ent = self.groups.offsets, self.groups.entries
         self.t += 1
         b1, b2 = self.betas
         self.norm_sq.zero_()
-        g = K.FeatureGroups.__new__(K.FeatureGroups)
-        g.entries = ent
         for t in range(L):  # decoder side, one launch per target layer
             rows = (t + 1) * F
-            g.F, g.offsets = rows, off[: rows + 1]
+            g = self.groups.part(0, rows)
             mD, vD = self.state["W_D"][t]
             K.sparse_grad_adam(g, act, dact, dy[t], dy[t], self.WD[t], mD, vD, self.WD_bf16[t].view(rows, d), None, None, None, None, None,
-                               None, None, None, None, None, lr, b1, b2, self.eps, self.t, True, norm_sq_accum=self.norm_sq[:rows])  # fmt: skip
+                               None, None, None, None, None, lr, b1, b2, self.eps, self.t, True, norm_sq_accum=self.norm_sq[:rows],
+                               dact_mode=2 if self.dp == 1 else 0)  # fmt: skip
         (mE, vE), (mb, vb) = self.state["W_E"], self.state["b_E"]
         for s in range(L):  # encoder side, one launch per source layer
-            g.F, g.offsets = F, off[s * F : (s + 1) * F + 1]
+            g = self.groups.part(s * F, (s + 1) * F)
             xs = xt[s]
             K.sparse_grad_adam(g, act, dact, xs, xs, None, None, None, None, self.WE[s], mE[s], vE[s], self.WE_bf16[s], self.bE[s], mb[s],
                                vb[s], None, None, None, lr, b1, b2, self.eps, self.t, True)  # fmt: skip

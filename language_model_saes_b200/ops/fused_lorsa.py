@@ -250,7 +250,14 @@ class FusedLorsaStep:
         self.loss_sum.zero_()
         WO16 = self.WO16
         bD = self.params.get("b_D")
-        if self.tp == 1:
+        early_WO = self.tp == 1 and self.dp == 1
+        if early_WO:
+            # one process: W_O is updated here, and that kernel leaves the code gradients that the attention's backward needs
+            dxhat, _, _ = K.sparse_decode_loss(idx, act, WO16, bD, Y, row_weight, grad_scale, self.loss_sum, want_dval=False)
+            dact = torch.zeros_like(act)
+            self.t += 1
+            self._update_WO(idx, act, dact, dxhat, lr, dact_mode=1)
+        elif self.tp == 1:
             dxhat, dact, _ = K.sparse_decode_loss(idx, act, WO16, bD, Y, row_weight, grad_scale, self.loss_sum)
         else:
             xhat = K.sparse_decode(idx, act, WO16, None, torch.float32)
@@ -300,21 +307,26 @@ class FusedLorsaStep:
                 off += grads[n].numel()
             idx, act, dact, dxhat = (self._gather_rows(t) for t in (idx, act, dact, dxhat))
             dist.all_reduce(self.loss_sum, group=self.dp_group)
-        self.t += 1
+        if not early_WO:
+            self.t += 1
+            self._update_WO(idx, act, dact, dxhat, lr)
         b1, b2 = self.betas
-        # W_O: rows rebuilt from the codes (act x d x_hat), Adam, bf16 shadow and row norms in one pass
-        if self.groups is None or self.groups.entries.numel() < idx.numel():
-            self.groups = K.FeatureGroups(self.F, idx.numel(), x.device)
-        self.groups.build(idx)
-        mO, vO = self.state["W_O"]
-        K.sparse_grad_adam(self.groups, act, dact, dxhat, dxhat, self.params["W_O"], mO, vO, WO16, None, None, None, None, None, None, None,
-                           self.dec_norm, None, None, lr, b1, b2, self.eps, self.t, True)  # fmt: skip
         for name, g in grads.items():
             m_, v_ = self.state[name]
             shadow = self.WV16.view(-1) if name == "W_V" else None
             K.adam_flat(self.params[name].view(-1), g.reshape(-1), m_.view(-1), v_.view(-1), lr, b1, b2, self.eps, self.t, shadow=shadow)
         self._refresh_qk()
         return (self.loss_sum / T).squeeze(0)
+
+    def _update_WO(self, idx, act, dact, dxhat, lr: float, dact_mode: int = 0) -> None:
+        """W_O: rows rebuilt from the codes (act x d x_hat), Adam, bf16 shadow and row norms in one pass."""
+        if self.groups is None or self.groups.entries.numel() < idx.numel():
+            self.groups = K.FeatureGroups(self.F, idx.numel(), idx.device)
+        self.groups.build(idx)
+        b1, b2 = self.betas
+        mO, vO = self.state["W_O"]
+        K.sparse_grad_adam(self.groups, act, dact, dxhat, dxhat, self.params["W_O"], mO, vO, self.WO16, None, None, None, None, None, None, None,
+                           self.dec_norm, None, None, lr, b1, b2, self.eps, self.t, True, dact_mode=dact_mode)  # fmt: skip
 
     def _gather_rows(self, t: torch.Tensor) -> torch.Tensor:
         """``[rows, n]`` of every replica stacked in rank order."""

@@ -7,10 +7,11 @@ squared error, backward, Adam. How it computes it:
 
 1. encoder GEMM (tcgen05) with the top-k epilogue        -> candidates per row and column range
 2. candidate merge (+ one exchange between feature shards) -> sparse codes (idx, act) [B, k]
-3. sparse decode fused with loss, d x_hat and d act        -> no dense [B, F] tensor exists at any point
+3. sparse decode fused with loss and d x_hat              -> no dense [B, F] tensor exists at any point
 4. counting sort of the codes by feature
-5. per feature row: rebuild the sparse gradient rows of W_D and W_E^T in registers and apply Adam, refresh
-   the bf16 shadows and the decoder row norms                -> no dense gradient tensor exists either
+5. per feature row: rebuild the sparse gradient rows of W_D and W_E^T in registers (and, unless shards or replicas need
+   them earlier, the code gradients) and apply Adam, refresh the bf16 shadows and the decoder row norms
+                                                          -> no dense gradient tensor exists either
 
 Optionally steps 5 (bound by HBM bandwidth: it streams every parameter and both Adam moments) and 1 of the NEXT step
 (bound by the tensor cores) overlap: the dictionary is cut into a few feature chunks, the update runs chunk by chunk on its own
@@ -459,6 +460,7 @@ class FusedTopKSAEStep:
         sharded = self.dp_comm is not None
         overlap = len(self.chunks) > 1 and k <= 64 and grad_mul is None and not want_grad_norm and not clip_grad_norm and not sharded
         self._mark("begin")
+        fused_dact = False
         if self.dp_comm is not None:
             self.dp_comm.wait_params()  # the other replicas' rows of the previous update must have landed in the shadows
         idx, act = self.encode(x, k, _in_step=overlap)
@@ -471,7 +473,11 @@ class FusedTopKSAEStep:
             dact = self.comm.dact(idx, self.WD_bf16)  # waits for the owners' gradient rows inside the kernel
             self._mark("dact")
         elif self.tp == 1:
-            dxhat, dact, _ = K.sparse_decode_loss(idx, act, self.WD_bf16, self.bD, label, row_weight, grad_scale, self.loss_sum)
+            fused_dact = self.dp == 1 and not overlap  # the update kernel computes the code gradients on its way
+            dxhat, dact, _ = K.sparse_decode_loss(idx, act, self.WD_bf16, self.bD, label, row_weight, grad_scale, self.loss_sum,
+                                                  want_dval=not fused_dact)  # fmt: skip
+            if fused_dact:
+                dact = torch.empty_like(act)
         else:
             partial = K.sparse_decode(idx, act, self.WD_bf16, None, torch.float32)
             dist.all_reduce(partial, group=self.tp_group)
@@ -502,6 +508,7 @@ class FusedTopKSAEStep:
                 self.bE, mb, vb, self.dec_norm, mul, sq, lr, b1, b2, self.eps, self.t, update,
                 f_range=f_range if not sharded else self.own_rows, ctas_per_sm=ctas_per_sm,
                 state_f0=self.own_rows[0], publish=self.dp_comm.pub_args() if sharded and update else None,
+                dact_mode=1 if fused_dact else 0,
             )  # fmt: skip
             if sharded and update:
                 self._masters_stale = True
@@ -658,7 +665,8 @@ class FusedTopKSAEStep:
         self._mark("aux_decode_and_reduce")
         g_main, g_aux = K.auxk_loss_grad(xhat, aux_rec, label, self.bD, row_weight, grad_scale, aux.coefficient, self.loss_sum,
                                          self.aux_sum, alpha_factor=alpha_on)  # fmt: skip
-        dact = K.sparse_dact(idx, self.WD_bf16, g_main)
+        fused_dact = self.tp == 1 and self.dp == 1  # the update kernel computes the code gradients on its way
+        dact = torch.empty_like(act) if fused_dact else K.sparse_dact(idx, self.WD_bf16, g_main)
         self._mark("loss_grad_dact")
         # gradient of the dead activations where they were selected (bf16 on the GPU: it is an operand of the next product)
         dA = (g_aux @ wd_dead.t() if x.is_cuda else _mm_f32(g_aux, wd_dead.t())) * (A != 0)
@@ -706,7 +714,7 @@ class FusedTopKSAEStep:
                 self.bE, mb, vb, self.dec_norm, mul, sq, lr, b1, b2, self.eps, self.t, update,
                 f_range=self.own_rows if sharded else None, state_f0=self.own_rows[0],
                 publish=self.dp_comm.pub_args() if sharded and update else None,
-                extra=(row_of, extra_gD, extra_gE, extra_gb),
+                extra=(row_of, extra_gD, extra_gE, extra_gb), dact_mode=1 if fused_dact else 0,
             )  # fmt: skip
             if sharded and update:
                 self._masters_stale = True

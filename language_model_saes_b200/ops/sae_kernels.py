@@ -448,6 +448,9 @@ def auxk_loss_grad(xhat, aux_rec, label, bias, row_weight, grad_scale, alpha, lo
 # --------------------------------------------------------------------------------------------------
 # backward / optimizer
 # --------------------------------------------------------------------------------------------------
+HEAVY_ROW = 64  # entries beyond which a feature row is shared by the groups of a CTA (kHeavyRow in csrc/kernels.h)
+
+
 class FeatureGroups:
     """(row, slot) pairs grouped by feature: ``entries[offsets[f]:offsets[f+1]]`` are flat positions
     ``row * k + slot`` whose code index is ``f``. Buffers are reused across steps."""
@@ -459,13 +462,27 @@ class FeatureGroups:
         self.cursor = torch.zeros(F, dtype=torch.int32, device=device)
         self.entries = torch.zeros(capacity, dtype=torch.int32, device=device)
         self.block_sums = torch.zeros((F + 4095) // 4096, dtype=torch.int32, device=device)
+        # features with long entry lists (count, then features) and the row counter of the update kernel's launches (left at
+        # zero by every launch; the launches that read these groups follow each other on one stream)
+        self.heavy = torch.zeros(1 + capacity // HEAVY_ROW + 1, dtype=torch.int32, device=device)
+        self.sched = torch.zeros(2, dtype=torch.int32, device=device)
+        self.heavy_base = 0
+
+    def part(self, lo: int, hi: int) -> "FeatureGroups":
+        """The groups of features ``[lo, hi)`` as groups of their own (views; features count from 0)."""
+        sub = FeatureGroups.__new__(FeatureGroups)
+        sub.F, sub.offsets, sub.entries = hi - lo, self.offsets[lo : hi + 1], self.entries
+        sub.heavy, sub.sched, sub.heavy_base = self.heavy, self.sched, self.heavy_base + lo
+        return sub
 
     def build(self, idx: torch.Tensor) -> "FeatureGroups":
         n = idx.numel()
         if self.entries.numel() < n:
             self.entries = torch.zeros(n, dtype=torch.int32, device=idx.device)
+        if self.heavy.numel() < 2 + n // HEAVY_ROW:
+            self.heavy = torch.zeros(2 + n // HEAVY_ROW, dtype=torch.int32, device=idx.device)
         if idx.is_cuda:
-            _ext().csc_build(idx, self.F, self.counts, self.offsets, self.cursor, self.entries, self.block_sums)
+            _ext().csc_build(idx, self.F, self.counts, self.offsets, self.cursor, self.entries, self.block_sums, self.heavy)
         else:
             flat = idx.reshape(-1)
             valid = flat >= 0
@@ -507,6 +524,18 @@ def ref_adam(p, g, m, v, lr, beta1, beta2, eps, step):
     p.addcdiv_(m, denom, value=-lr / bc1)
 
 
+def _ref_code_gradients(groups: FeatureGroups, act, dact, dxhat, WD, mode: int, f_range=None) -> None:
+    """Plain statement of ``dact_mode``: the code gradients of the entries listed in ``groups``."""
+    lo, hi = f_range if f_range is not None else (0, groups.F)
+    off = groups.offsets.long()
+    ent = groups.entries[int(off[lo]) : int(off[hi])].long()
+    f = torch.repeat_interleave(torch.arange(lo, hi), off[lo + 1 : hi + 1] - off[lo:hi])
+    dot = (dxhat.float()[ent // act.shape[1]] * WD[f].to(torch.bfloat16).float()).sum(-1)
+    dot = torch.where(act.reshape(-1)[ent] != 0, dot, torch.zeros_like(dot))
+    flat = dact.view(-1)
+    flat[ent] = flat[ent] + dot if mode == 2 else dot
+
+
 def sparse_grad_adam(
     groups: FeatureGroups,
     act,
@@ -543,6 +572,7 @@ def sparse_grad_adam(
     extra: tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor | None] | None = None,
     wd_self_scale: torch.Tensor | None = None,
     norm_sq_accum: torch.Tensor | None = None,
+    dact_mode: int = 0,
 ):
     """Rebuild the two sparse gradient rows per feature and apply Adam in the same pass (in place). ``f_range``
     restricts the launch to feature rows ``[begin, end)``. With ``dxhat_aux`` the code slots ``>= k_main`` of every row
@@ -554,10 +584,14 @@ def sparse_grad_adam(
     ``[F]``: the decoder row's gradient gets ``wd_self_scale[f] * W_D[f, :]`` added (the gradient that a penalty on the
     row's norm sends into the row). One-sided launches: pass ``WD = mD = vD = WD_bf16 = None`` to update the encoder side
     only, or the ``WE`` group as None for the decoder side only. ``norm_sq_accum`` fp32 ``[F]``: the squared norm of every
-    new decoder row is ADDED there instead of writing ``dec_norm``. A non-zero kernel status word turns the update into
+    new decoder row is ADDED there instead of writing ``dec_norm``. ``dact_mode``: 0 takes ``dact`` as given; 1 computes it
+    first (``d x_hat[token] . bf16(W_D row)`` with the row as it was before the update; 0 where the code is 0) and leaves it in
+    ``dact``, 2 adds to what ``dact`` holds (one launch per decoder matrix); the decoder group must be given then. A non-zero kernel status word turns the update into
     a no-op (CUDA path)."""
     ref_w = WD if WD is not None else WE
     if not ref_w.is_cuda:
+        if dact_mode:
+            _ref_code_gradients(groups, act, dact, dxhat, WD, dact_mode, f_range)
         if WD is None or WE is None:  # one-sided: run the two-sided statement on a scratch copy of the missing side
             zero = lambda: torch.zeros_like(ref_w)  # noqa: E731
             if WD is None:
@@ -576,9 +610,7 @@ def sparse_grad_adam(
             return
         if f_range is not None and tuple(f_range) != (0, groups.F):
             lo, hi = f_range
-            sub = FeatureGroups.__new__(FeatureGroups)
-            sub.F = hi - lo
-            sub.offsets, sub.entries = groups.offsets[lo : hi + 1], groups.entries
+            sub = groups.part(lo, hi)
             sl = slice(lo, hi)
             st = slice(lo - state_f0, hi - state_f0)
             sub_extra = (extra[0][sl], *extra[1:]) if extra is not None else None
@@ -630,7 +662,8 @@ def sparse_grad_adam(
         groups.offsets, groups.entries, act, dact, x, dxhat, WD, mD, vD, WD_bf16, WE, mE, vE, WE_bf16, bE, mbE, vbE,
         dec_norm, grad_mul, grad_sq_sum, lr, beta1, beta2, eps, step, update, *(f_range if f_range is not None else (0, -1)), ctas_per_sm, dxhat_aux, k_main, grad_out[0], grad_out[1],
         status_buffer(ref_w.device), state_f0, *(publish if publish is not None else ([], [], 0, None)),
-        *(extra if extra is not None else (None, None, None, None)), wd_self_scale, norm_sq_accum,
+        *(extra if extra is not None else (None, None, None, None)), wd_self_scale, norm_sq_accum, dact_mode, groups.heavy,
+        groups.heavy_base, groups.sched,
     )  # fmt: skip
 
 

@@ -1,0 +1,81 @@
+"""The row-streaming gradient + Adam kernel at the widths where its layout changes (one to eight warps per row, partial last
+chunks), with empty rows, rows longer than one batch of entries and rows long enough to be shared by a whole CTA, against
+the wrapper's plain-torch statement on CPU copies."""
+
+import pytest
+import torch
+
+from language_model_saes_b200.ops import sae_kernels as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _case(d, F, B, k, seed):
+    g = torch.Generator().manual_seed(seed)
+    idx = torch.stack([torch.randperm(F - 3, generator=g)[:k] for _ in range(B)]).to(torch.int32) + 2
+    idx[:, 0] = 0  # a feature with an entry of every token (a long list), and ...
+    idx[: K.HEAVY_ROW, 1] = 1  # ... one right at the limit
+    idx[5, 2:] = -1
+    act = torch.rand(B, k, generator=g) + 0.1
+    act[7, :] = 0.0  # listed, but inactive
+    dact = torch.randn(B, k, generator=g)
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    t = dict(idx=idx, act=act, dact=dact, x=r(B, d).to(torch.bfloat16), dx=(r(B, d) * 0.1).to(torch.bfloat16), WD=r(F, d), WE=r(F, d), b=r(F),
+             n=torch.zeros(F), gsq=torch.zeros(1), scale=torch.rand(F, generator=g) * 0.1, acc=torch.zeros(F),
+             row_of=torch.where(torch.arange(F) % 5 == 0, torch.arange(F) // 5, -1).to(torch.int32), xD=r(F, d), xE=r(F, d), xb=r(F))  # fmt: skip
+    for n, s in (("mD", (F, d)), ("vD", (F, d)), ("mE", (F, d)), ("vE", (F, d)), ("mb", (F,)), ("vb", (F,))):
+        t[n] = torch.rand(*s, generator=g) * 0.01
+    t["WD16"], t["WE16"] = t["WD"].to(torch.bfloat16), t["WE"].to(torch.bfloat16)
+    return t
+
+
+def _compare(cpu, gpu, names, d):
+    for n in names:
+        a, b = gpu[n].cpu().float(), cpu[n].float()
+        # fp32 sums of at most 200 terms (entries of a row) or d terms (code gradients) of order one, in another order
+        tol = 2**-24 * max(200, d) * 4 if n in ("dact", "gsq", "acc") else 2e-5
+        assert torch.allclose(a, b, atol=max(tol, 2e-5), rtol=3e-4), (n, float((a - b).abs().max()))
+
+
+@pytest.mark.parametrize("d", [64, 132, 768, 1024, 1028, 1160, 2052, 4100, 8192])
+@pytest.mark.parametrize("sides,mode", [("both", 0), ("both", 1), ("decoder", 2), ("encoder", 0)])
+def test_row_kernel_matches_the_plain_statement(d, sides, mode):
+    F, B, k = 230, 200, 6
+    cpu = _case(d, F, B, k, seed=d)
+    gpu = {n: t.clone().to(DEV) for n, t in cpu.items()}
+
+    def run(t, step):
+        groups = K.FeatureGroups(F, B * k, t["idx"].device).build(t["idx"])
+        D = [t["WD"], t["mD"], t["vD"], t["WD16"]] if sides != "encoder" else [None] * 4
+        E = [t["WE"], t["mE"], t["vE"], t["WE16"], t["b"], t["mb"], t["vb"]] if sides != "decoder" else [None] * 7
+        both = sides == "both"
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], *D, *E, t["n"] if both else None, None, t["gsq"] if both else None, 1e-3,
+                           0.9, 0.999, 1e-8, step, True, extra=(t["row_of"], t["xD"], t["xE"], t["xb"]) if both else None,
+                           wd_self_scale=t["scale"] if sides == "decoder" else None, norm_sq_accum=t["acc"] if sides == "decoder" else None,
+                           dact_mode=mode)  # fmt: skip
+        return groups
+
+    for step in (1, 2):
+        run(cpu, step)
+        groups = run(gpu, step)
+        K.check_status(torch.device(DEV))
+        assert int(groups.heavy[0]) == 1 and int(groups.heavy[1]) == 0
+        assert groups.sched.tolist() == [0, 0]  # ready for the next launch
+    _compare(cpu, gpu, ["dact", "WD", "mD", "vD", "WE", "mE", "vE", "b", "mb", "vb", "n", "acc"], d)
+    assert torch.allclose(gpu["gsq"].cpu(), cpu["gsq"], rtol=1e-3)
+    if sides != "encoder":
+        assert torch.equal(gpu["WD16"].float(), gpu["WD"].to(torch.bfloat16).float())
+    if sides != "decoder":
+        assert torch.equal(gpu["WE16"].float(), gpu["WE"].to(torch.bfloat16).float())
+
+
+def test_gradient_pass_without_an_update_leaves_code_gradients_and_norm_only():
+    cpu = _case(260, 230, 200, 6, seed=3)
+    gpu = {n: t.clone().to(DEV) for n, t in cpu.items()}
+    for t in (cpu, gpu):
+        groups = K.FeatureGroups(230, 1200, t["idx"].device).build(t["idx"])
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], t["WD"], t["mD"], t["vD"], t["WD16"], t["WE"], t["mE"], t["vE"], t["WE16"],
+                           t["b"], t["mb"], t["vb"], t["n"], None, t["gsq"], 1e-3, 0.9, 0.999, 1e-8, 1, False, dact_mode=1)  # fmt: skip
+    _compare(cpu, gpu, ["dact", "WD", "mD", "WE", "vE", "b", "n"], 260)
+    assert torch.allclose(gpu["gsq"].cpu(), cpu["gsq"], rtol=1e-3)
