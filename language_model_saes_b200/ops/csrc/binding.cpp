@@ -741,6 +741,26 @@ void jumprelu_window_grad(const Tensor& G, const Tensor& S, const Tensor& n, con
              "jumprelu_window_grad launch");
 }
 
+// Codes of every head and the tanh penalty's terms from the shared lists (crosscoder_ops.cu). pull, dtheta, u_sum and n_valid are
+// accumulated into.
+void jumprelu_lists(const Tensor& idx, const Tensor& s_val, const Tensor& norm, const Tensor& theta, double stretch, double coef,
+                    double window, const Tensor& act, const Tensor& dS, const Tensor& pull, const Tensor& dtheta,
+                    const Tensor& u_sum, const Tensor& n_valid) {
+  CHECK_T(idx, torch::kInt32);
+  CHECK_T(n_valid, torch::kInt32);
+  for (const Tensor* t : {&s_val, &norm, &theta, &act, &dS, &pull, &dtheta, &u_sum}) { CHECK_T(*t, torch::kFloat32); }
+  TORCH_CHECK(idx.dim() == 2 && s_val.sizes() == idx.sizes() && dS.sizes() == idx.sizes() && norm.dim() == 2, "lists [B, cap], norms [H, F]");
+  lmsae::JumpReluListParams p{};
+  p.B = (int)idx.size(0); p.cap = (int)idx.size(1); p.H = (int)norm.size(0); p.F = (int)norm.size(1);
+  TORCH_CHECK(act.numel() == (int64_t)p.H * p.B * p.cap && pull.numel() == norm.numel() && theta.numel() == p.F && dtheta.numel() >= p.F);
+  p.idx = idx.data_ptr<int>(); p.s_val = s_val.data_ptr<float>(); p.norm = norm.data_ptr<float>(); p.theta = theta.data_ptr<float>();
+  p.stretch = (float)stretch; p.coef = (float)coef; p.window = (float)window;
+  p.act = act.data_ptr<float>(); p.dS = dS.data_ptr<float>(); p.pull = pull.data_ptr<float>(); p.dtheta = dtheta.data_ptr<float>();
+  p.u_sum = u_sum.data_ptr<float>(); p.n_valid = n_valid.data_ptr<int>();
+  const c10::cuda::CUDAGuard guard(idx.device());
+  check_cuda(lmsae::jumprelu_lists_launch(p, at::cuda::getCurrentCUDAStream()), "jumprelu_lists launch");
+}
+
 // Rotary embedding (sin_sign = 1) or its inverse (-1) of xa and xb [batch x seq, heads, width] bf16 into oa and ob;
 // cos / sin fp32 [>= seq, rd] (see rotary.cu).
 void rotary_pair(const Tensor& xa, const Tensor& xb, const Tensor& oa, const Tensor& ob, const Tensor& cos_t, const Tensor& sin_t,
@@ -1128,6 +1148,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sparse_dact", &sparse_dact);
   m.def("mse_loss_grad", &mse_loss_grad);
   m.def("csc_build", &csc_build);
+  m.def("jumprelu_lists", &jumprelu_lists);
   m.def("auxk_loss_grad", &auxk_loss_grad);
   m.def("sparse_grad_adam", &sparse_grad_adam);
   m.def("colsum_bf16", &colsum_bf16);

@@ -214,6 +214,23 @@ int gather_rows_cast_launch(int in_dtype, int out_dtype, const void* src, const 
                             int d, void* out, long long out_rows, cudaStream_t stream);
 int exclusive_scan_launch(const int* counts, int n, int* offsets, int* block_sums_buf, cudaStream_t stream);
 
+// ---- lists of the JumpReLU step (crosscoder_ops.cu) ---------------------------------------------------
+struct JumpReluListParams {
+  const int* idx;      // [B, cap] features of a token's list (-1: empty slot)
+  const float* s_val;  // [B, cap] summed pre-activations
+  int B, cap, H, F;
+  const float* norm;   // [H, F] decoder row norms
+  const float* theta;  // [F]
+  float stretch, coef, window;  // tanh(stretch * a); coef = l1 * stretch / (tokens * heads), 0: no penalty
+  float* act;          // [H, B, cap] codes of every head (slots with idx >= 0)
+  float* dS;           // [B, cap] penalty's share of the shared sum's gradient (slots with idx >= 0)
+  float* pull;         // [H, F] += penalty's derivative with respect to the norms
+  float* dtheta;       // [F] += correction at active entries
+  float* u_sum;        // += sum of tanh over active entries and heads
+  int* n_valid;        // += number of listed entries
+};
+int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream);
+
 // ---- rotary embedding of two [tokens, heads, width] bf16 tensors in one launch (rotary.cu) ----------------------
 int rotary_pair_launch(const __nv_bfloat16* xa, const __nv_bfloat16* xb, __nv_bfloat16* oa, __nv_bfloat16* ob, const float* cos_t,
                        const float* sin_t, long long tokens, int seq, int heads, int width, int rd, int adjacent, float sin_sign,

@@ -209,6 +209,8 @@ class FusedCrosscoderStep:
         if self.head_size > 1:
             dist.all_reduce(t_min, op=dist.ReduceOp.MIN, group=self.head_group)
         idx, s_val = S.column_threshold_rows_to_sparse(S_sum, t_min, cap, overflow=self.list_overflow)
+        if x.is_cuda and self.tp == 1 and self.dp == 1 and not quad:
+            return self._step_on_lists(x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, float(tanh_stretch), lp_coefficient)
         safe = idx.clamp_min(0).long()
         valid = idx >= 0
         # scatter target of the per-feature sums below: empty slots go to a dump element of their own row (sending them all
@@ -224,19 +226,7 @@ class FusedCrosscoderStep:
         c = float(tanh_stretch)
         lp = None
         if lp_coefficient:
-            c_lp = lp_coefficient / (B * H)
-            Sf = S_sum.float()
-            below = Sf < theta  # [B, F]: where the penalty is active
-            count = below.sum(0).float()  # per feature: tokens below the threshold
-            gap = torch.relu(theta - Sf).sum(0)  # per feature: summed distance to the threshold
-            n_local = self.dec_norm.sum(0)  # [F]: norms summed over this rank's heads ...
-            n_all = n_local.clone()
-            if self.head_size > 1:  # ... and over all heads: the shared sum feels every head's term
-                dist.all_reduce(n_all, group=self.head_group)
-            dtheta += c_lp * n_local * count  # (summed over the head ranks below, with the rest of d theta)
-            lp = {"mask": below.to(torch.bfloat16), "row_scale": -c_lp * n_all, "gb": -c_lp * n_all * count, "gap": gap,
-                  "rows": torch.arange(F, dtype=torch.int32, device=x.device), "c": c_lp}  # fmt: skip
-            l_p_sum = c_lp * (gap * n_local).sum() * H / H_l  # mean over tokens and THIS rank's heads
+            lp, l_p_sum = self._lp_terms(S_sum, theta, lp_coefficient, dtheta)
         mult = None  # per-feature factor on every derivative of the sparsity penalty (1 for the plain tanh penalty)
         if quad:
             # tanh-quad: l_s = l1 * sum_f q_f (1 + q_f / scale) with q_f the mean of tanh(c * act * norm) over ALL tokens and
@@ -359,6 +349,86 @@ class FusedCrosscoderStep:
         l_s = l_s_quad if quad else l1_coefficient * l_s_sum / (B * H_l)
         l_p = l_p_sum if lp is not None else torch.zeros((), device=x.device)
         self.last = {"l_rec": l_rec, "l_s": l_s, "l_p": l_p, "l0": n_valid / B}
+        return l_rec + l_s + l_p
+
+    def _lp_terms(self, S_sum: torch.Tensor, theta: torch.Tensor, lp_coefficient: float, dtheta: torch.Tensor):
+        """The dense parts of the pre-activation penalty: adds its threshold gradient to ``dtheta`` (summed over the head ranks
+        with the rest of d theta) and returns what the updates need, and its value (mean over tokens and this rank's heads)."""
+        B, H, H_l, F = S_sum.shape[0] * self.dp, self.H, self.H_l, self.F
+        c_lp = lp_coefficient / (B * H)
+        Sf = S_sum.float()
+        below = Sf < theta  # [B, F]: where the penalty is active
+        count = below.sum(0).float()  # per feature: tokens below the threshold
+        gap = torch.relu(theta - Sf).sum(0)  # per feature: summed distance to the threshold
+        n_local = self.dec_norm.sum(0)  # [F]: norms summed over this rank's heads ...
+        n_all = n_local.clone()
+        if self.head_size > 1:  # ... and over all heads: the shared sum feels every head's term
+            dist.all_reduce(n_all, group=self.head_group)
+        dtheta += c_lp * n_local * count
+        lp = {"mask": below.to(torch.bfloat16), "row_scale": -c_lp * n_all, "gb": -c_lp * n_all * count, "gap": gap,
+              "rows": torch.arange(F, dtype=torch.int32, device=S_sum.device), "c": c_lp}  # fmt: skip
+        return lp, c_lp * (gap * n_local).sum() * H / H_l
+
+    def _step_on_lists(self, x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, c, lp_coefficient) -> torch.Tensor:
+        """The step from the shared lists on, one process per head group on a GPU: one kernel derives every head's codes and the
+        penalty's terms from the lists; per head decode + loss, then the decoder side of the update, which adds the head's
+        code gradients to the shared sum's gradient on its way; the encoder sides follow once that sum is complete."""
+        B, H_l, d = x.shape
+        H, F, cap = self.H, self.F, self.cap
+        dev = x.device
+        zeros = torch.zeros(H_l * F + F + 2, dtype=torch.float32, device=dev)
+        pull, dtheta, u_sum = zeros[: H_l * F].view(H_l, F), zeros[H_l * F : H_l * F + F], zeros[-2:-1]
+        n_valid = zeros[-1:].view(torch.int32)
+        act = torch.empty(H_l, B, cap, dtype=torch.float32, device=dev)
+        dS = torch.empty(B, cap, dtype=torch.float32, device=dev)
+        lp = None
+        if lp_coefficient:
+            lp, l_p_sum = self._lp_terms(S_sum, theta, lp_coefficient, dtheta)
+        coef = l1_coefficient * c / (B * H) if l1_coefficient else 0.0
+        K._ext().jumprelu_lists(idx, s_val, self.dec_norm, theta, c, coef, self.window, act, dS, pull, dtheta, u_sum, n_valid)
+        if self.groups is None or self.groups.entries.numel() < idx.numel():
+            self.groups = K.FeatureGroups(F, idx.numel(), dev)
+        self.groups.build(idx)
+        self.loss_sum.zero_()
+        self.t += 1
+        b1, b2 = self.betas
+        (mE, vE), (mD, vD), (mb, vb), (mbD, vbD) = (self.state[n] for n in ("W_E", "W_D", "b_E", "b_D"))
+        xt = x.transpose(0, 1).contiguous()  # [H_l, B, d]
+        target = xt if label is None else label.transpose(0, 1).contiguous()
+        self_scale = None
+        if coef:
+            self_scale = pull / self.dec_norm
+        if lp is not None:  # the penalty's pull on the decoder norms: d / d W_D[f] = c * gap_f * W_D[f] / ||W_D[f]||
+            p = lp["c"] * lp["gap"] / self.dec_norm
+            self_scale = p if self_scale is None else self_scale + p
+        for h in range(H_l):
+            dxhat, _, _ = K.sparse_decode_loss(idx, act[h], self.WD_bf16[h], self.bD[h], target[h], None, 2.0 / (B * H), self.loss_sum,
+                                               want_dval=False)  # fmt: skip
+            # threshold gradient: the reconstruction gradient at every entry inside the window (the tanh penalty's derivative at
+            # zero activation is coef at every entry: the dense pass adds it per window hit)
+            G = K.encoder_hidden(dxhat, self.WD_bf16[h], None)  # [B, F] bf16 = d x_hat . W_D^T
+            S.jumprelu_window_grad(G, S_sum, self.dec_norm[h], theta, self.window, dtheta, add_per_hit=coef)
+            K.sparse_grad_adam(self.groups, act[h], dS, dxhat, dxhat, self.WD[h], mD[h], vD[h], self.WD_bf16[h], None, None, None, None, None,
+                               None, None, self.dec_norm[h], None, None, lr, b1, b2, self.eps, self.t, True,
+                               wd_self_scale=self_scale[h] if self_scale is not None else None, dact_mode=2)  # fmt: skip
+            K.adam_flat(self.bD[h], K.colsum_bf16(dxhat), mbD[h], vbD[h], lr, b1, b2, self.eps, self.t)
+        if self.head_size > 1:  # the lists are the same on every rank: the sum over heads is element-wise
+            dS = torch.where(idx >= 0, dS, torch.zeros_like(dS))  # (empty slots were never written)
+            dist.all_reduce(dS, group=self.head_group)
+            dist.all_reduce(dtheta, group=self.head_group)
+        for h in range(H_l):
+            extra = None
+            if lp is not None:  # dense encoder gradient rows of the pre-activation penalty: -c N_f (1[S < theta]^T x_h)[f, :]
+                gE = _mm_f32(lp["mask"].t(), xt[h]) * lp["row_scale"].unsqueeze(1)
+                extra = (lp["rows"], None, gE, lp["gb"])
+            K.sparse_grad_adam(self.groups, act[h], dS, xt[h], xt[h], None, None, None, None, self.WE[h], mE[h], vE[h], self.WE_bf16[h],
+                               self.bE[h], mb[h], vb[h], None, None, None, lr, b1, b2, self.eps, self.t, True, extra=extra)  # fmt: skip
+        m, v = self.state["log_theta"]
+        K.adam_flat(self.log_theta, dtheta * theta, m, v, lr * self.jumprelu_lr_factor, b1, b2, self.eps, self.t)
+        l_rec = (self.loss_sum / (B * H_l)).squeeze(0)
+        l_s = l1_coefficient * u_sum.squeeze(0) / (B * H_l)
+        l_p = l_p_sum if lp is not None else torch.zeros((), device=dev)
+        self.last = {"l_rec": l_rec, "l_s": l_s, "l_p": l_p, "l0": n_valid.squeeze(0) / B}
         return l_rec + l_s + l_p
 
     def _gather_rows(self, t: torch.Tensor) -> torch.Tensor:
