@@ -25,8 +25,8 @@
 // PAIR variant (tcgen05 cta_group::2): two CTAs on neighbouring SMs form a cluster and work on two adjacent
 // 128-row panels with ONE 256x256x16 instruction stream issued by the leader (cluster rank 0). Each CTA loads
 // its own A tile and only HALF of the B tile (128 of the 256 dictionary rows), so a stage is 32 KB instead of
-// 48 KB per CTA: B crosses L2 -> shared memory once per pair, and the ring is 5-6 stages deep even with the
-// 64-slot top-k state resident. Both producers complete their bytes on the LEADER's "full" barrier; the
+// 48 KB per CTA: B crosses L2 -> shared memory once per pair, and the ring is 4-5 stages deep even with the
+// top-k candidate buffers resident. Both producers complete their bytes on the LEADER's "full" barrier; the
 // leader's commits arrive on the "empty" / "accumulator full" barriers of BOTH CTAs; both epilogues release an
 // accumulator buffer on the leader's "accumulator empty" barrier. Each CTA's epilogue is unchanged: it reads
 // its own 128 TMEM lanes (its panel's rows) x 256 columns.
@@ -43,15 +43,25 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KB
 constexpr int TMEM_COLS = 512;
 constexpr int NUM_THREADS = 256;
 
-template <int STAGES, int KS, bool PAIR>
+// Entries of a row's candidate buffer (CAP): the k best so far plus room for what is appended until the next selection. A step of
+// the sweep appends at most 16, so k + 16 entries suffice; more room means fewer selections, but costs ring stages.
+// NARROW buffers hold columns as 16-bit offsets from the start of the range (codes from kCarried on: entry code - kCarried of the
+// resumed state). 4096 rows x 24576 columns, K 768, k 50 / 64: 204 / 322 us with 80 entries and five stages, 191 / 207 with 128
+// and four; k 32: 173 and 177. But K 4096 x 131072 columns is bound by the tensor cores and takes 5 % longer with four stages than with five.
+constexpr int kNarrowTiles = 255;
+constexpr int kCarried = kNarrowTiles * BN;
+
+template <int STAGES, int CAP, bool PAIR, bool NARROW>
 struct SmemLayout {
   static constexpr int kBRows = PAIR ? BN / 2 : BN;       // dictionary rows of a B tile held by one CTA
   static constexpr int kBStageBytes = kBRows * BK * 2;    // 16 KB (pair) / 32 KB
   static constexpr int kStageBytes = A_STAGE_BYTES + kBStageBytes;
   static constexpr int kStageOff = 0;
   static constexpr int kSlotValOff = STAGES * kStageBytes;
-  static constexpr int kSlotIdxOff = kSlotValOff + BM * KS * 4;
-  static constexpr int kBarOff = kSlotIdxOff + BM * KS * 4;
+  static constexpr int kSlotIdxOff = kSlotValOff + BM * CAP * 4;
+  static constexpr int kColOff = kSlotIdxOff + BM * CAP * (NARROW ? 2 : 4);   // per epilogue warp: bias and gate of the 32 columns at work
+  static constexpr int kStoreOff = kColOff + 4 * 64 * 4;  // per epilogue warp: 32 x 32 bf16 on their way to whole sectors of H (no top-k)
+  static constexpr int kBarOff = kStoreOff + (CAP == 0 ? 4 * 2048 : 0);
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
   static constexpr int kAbortOff = kTmemPtrOff + 4;
@@ -59,25 +69,139 @@ struct SmemLayout {
   static constexpr int kDynamicBytes = kTotal + 1024;  // slack for manual 1024-byte alignment
 };
 
-// v[j] for a run-time j without spilling the register array: a 5-level tree of selects.
-__device__ __forceinline__ float select32(const float (&v)[32], int j) {
-  float a[16], b[8], c[4];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) a[i] = (j & 1) ? v[2 * i + 1] : v[2 * i];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) b[i] = (j & 2) ? a[2 * i + 1] : a[2 * i];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) c[i] = (j & 4) ? b[2 * i + 1] : b[2 * i];
-  const float d0 = (j & 8) ? c[1] : c[0];
-  const float d1 = (j & 8) ? c[3] : c[2];
-  return (j & 16) ? d1 : d0;
+struct RowState {
+  int n;      // entries in the row's buffer
+  float tau;  // at least k of them are >= tau: a column has to beat it
+};
+
+// Element-wise over pairs in one instruction each.
+__device__ __forceinline__ void add_pair(float& a0, float& a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 ra, rb;\n\tmov.b64 ra, {%0, %1};\n\tmov.b64 rb, {%2, %3};\n\tadd.rn.f32x2 ra, ra, rb;\n\tmov.b64 {%0, %1}, ra;\n\t}"
+      : "+f"(a0), "+f"(a1)
+      : "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void mul_pair(float& a0, float& a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 ra, rb;\n\tmov.b64 ra, {%0, %1};\n\tmov.b64 rb, {%2, %3};\n\tmul.rn.f32x2 ra, ra, rb;\n\tmov.b64 {%0, %1}, ra;\n\t}"
+      : "+f"(a0), "+f"(a1)
+      : "f"(b0), "f"(b1));
 }
 
-template <bool WRITE_H, bool TOPK, int STAGES, int KS, bool PAIR>
+// Entry {value, column} to shared memory where the condition holds: predicated, because a branch per column costs more than the
+// rest of the epilogue (one warp per scheduler). The address of the next entry is a NEW register of the caller's: advanced in
+// place, it would have to wait for every store to have read it (23 cycles a column).
+template <bool NARROW>
+__device__ __forceinline__ void store_entry_if(bool cond, uint32_t val_addr, uint32_t col_addr, uint32_t bits, uint32_t col) {
+  if constexpr (NARROW)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.b32 [%1], %3;\n\t@p st.shared.b16 [%2], %4;\n\t}" ::"r"((uint32_t)cond),
+                 "r"(val_addr), "r"(col_addr), "r"(bits), "h"((unsigned short)col)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.b32 [%1], %3;\n\t@p st.shared.b32 [%2], %4;\n\t}" ::"r"((uint32_t)cond),
+                 "r"(val_addr), "r"(col_addr), "r"(bits), "r"(col)
+                 : "memory");
+}
+
+// A row's buffer: entry s has its value at [s][row] of one array and its column at [s][row] of the other, both BM rows wide.
+template <int CAP, bool NARROW>
+struct RowBuffer {
+  uint32_t val;       // shared-memory address of entry 0's value
+  uint32_t val0, col0;  // the two arrays
+  __device__ __forceinline__ uint32_t col_of(uint32_t val_addr) const {
+    return NARROW ? ((val_addr - val0) >> 1) + col0 : val_addr - val0 + col0;
+  }
+  __device__ __forceinline__ uint32_t value(int s) const {
+    uint32_t x;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(val + s * (BM * 4)) : "memory");
+    return x;
+  }
+  __device__ __forceinline__ uint32_t column(int s) const {
+    const uint32_t a = col_of(val + s * (BM * 4));
+    if constexpr (NARROW) {
+      unsigned short x;
+      asm volatile("ld.shared.b16 %0, [%1];" : "=h"(x) : "r"(a) : "memory");
+      return x;
+    } else {
+      uint32_t x;
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a) : "memory");
+      return x;
+    }
+  }
+};
+
+// Cuts the buffers of a warp's 32 rows (one per lane) down to at most `limit` >= k entries each without losing any of the k
+// largest: a bisection (of values first, then of their bit patterns, which order positive floats) for a bound that between k and
+// `limit` entries reach. Where equal values leave no such bound, the first of them fill up to k. Rows that hold no more than
+// `limit` entries stay as they are. Order is kept.
+template <int CAP, bool NARROW>
+__device__ __noinline__ RowState select_entries(RowBuffer<CAP, NARROW> buf, RowState st, int k, int limit) {
+  uint32_t w[CAP];
+  uint32_t top[4] = {0u, 0u, 0u, 0u};  // (four chains at a time: a single one is bound by the latency of its links)
+#pragma unroll
+  for (int s = 0; s < CAP; ++s) w[s] = buf.value(s);
+#pragma unroll
+  for (int s = 0; s < CAP; ++s) {
+    w[s] = s < st.n ? w[s] : 0u;
+    top[s & 3] = max(top[s & 3], w[s]);
+  }
+  const bool mine = st.n > limit;
+  bool active = mine;
+  uint32_t lo = max(__float_as_uint(st.tau), 1u), hi = max(max(top[0], top[1]), max(top[2], top[3])) + 1u;  // count(>= lo) >= k > count(>= hi)
+  int at_lo = st.n;
+  for (int step = 0; __any_sync(0xffffffffu, active); ++step) {
+    uint32_t mid = step < 8 ? __float_as_uint(0.5f * __uint_as_float(lo) + 0.5f * __uint_as_float(hi - 1u)) : lo + ((hi - lo) >> 1);
+    mid = min(max(mid, lo + 1u), hi - 1u);
+    int c[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int s = 0; s < CAP; ++s) c[s & 3] += w[s] >= mid;
+    if (active) {
+      const int n = (c[0] + c[1]) + (c[2] + c[3]);
+      if (n >= k) { lo = mid; at_lo = n; } else { hi = mid; }
+      active = at_lo > limit && hi - lo > 1u;
+    }
+  }
+  const bool tied = mine && at_lo > limit;  // too many entries equal to the bound
+  uint32_t at = buf.val;
+  if (!__any_sync(0xffffffffu, tied)) {
+    const uint32_t bound = mine ? lo : 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < CAP; b += 16) {
+      uint32_t id[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) id[i] = buf.column(b + i);  // (read before anything at or behind them is overwritten)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const bool keep = w[b + i] >= bound;
+        store_entry_if<NARROW>(keep, at, buf.col_of(at), w[b + i], id[i]);
+        at = at + (keep ? BM * 4 : 0);
+      }
+    }
+  } else {
+    int ties = tied ? k : CAP;
+    if (tied) {
+#pragma unroll
+      for (int s = 0; s < CAP; ++s) ties -= w[s] > lo;
+    }
+#pragma unroll
+    for (int s = 0; s < CAP; ++s) {
+      const uint32_t id = buf.column(s);
+      const bool tie = w[s] == lo, keep = mine && (w[s] > lo || (tie && ties > 0));
+      ties -= tie;
+      store_entry_if<NARROW>(keep, at, buf.col_of(at), w[s], id);
+      at = at + (keep ? BM * 4 : 0);
+    }
+  }
+  if (mine) {
+    st.n = (int)((at - buf.val) / (BM * 4));
+    st.tau = __uint_as_float(lo);
+  }
+  return st;
+}
+
+template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const EncGemmParams p) {
-  using L = SmemLayout<STAGES, KS, PAIR>;
+  using L = SmemLayout<STAGES, CAP, PAIR, NARROW>;
   constexpr int STAGE_BYTES = L::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -88,8 +212,6 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kTmemPtrOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbortOff);
-  float* slot_val = reinterpret_cast<float*>(smem + L::kSlotValOff);
-  int* slot_idx = reinterpret_cast<int*>(smem + L::kSlotIdxOff);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -150,27 +272,6 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     } else {
       tmem_alloc(tmem_ptr_smem, TMEM_COLS);
       tmem_relinquish();
-    }
-  }
-  if constexpr (TOPK) {
-    // slots are stored slot-major, [KS][128 rows], so that the thread owning a row reads and writes its
-    // slots without bank conflicts. The first k slots hold (0, -1) = "empty, any positive value beats
-    // it"; the rest hold +inf so they are never the minimum and never replaced.
-    for (int i = threadIdx.x; i < BM * KS; i += NUM_THREADS) {
-      const int s = i / BM;
-      float v = (s < p.k) ? 0.0f : __int_as_float(0x7f800000);
-      int ix = -1;
-      if (p.resume_topk && s < p.k) {
-        // continue the sweep of an earlier launch: its result for (row, this column range) is the state
-        const int r = m0 + (i - s * BM);
-        if (r < p.M) {
-          const long long o = (long long)r * ((long long)p.num_splits * KS) + (long long)split * KS + s;
-          v = p.cand_val[o];
-          ix = p.cand_idx[o];
-        }
-      }
-      slot_val[i] = v;
-      slot_idx[i] = ix;
     }
   }
   tc_fence_before();
@@ -272,35 +373,48 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     const int row_in_tile = q * 32 + lane;
     const int row = m0 + row_in_tile;
     const bool row_ok = row < p.M;
-    // Running top-k of this thread's row. The KS slots form groups of 8; gmin[g] caches the smallest
-    // value of group g in a register, tau = min(gmin) is the value a candidate has to beat. An insert
-    // touches one group only: 8 shared-memory reads, 2 writes.
-    constexpr int NG = KS > 0 ? KS / 8 : 1;
-    float gmin[NG];
-    float tau = 0.0f;
-    float* my_slot_val = slot_val + row_in_tile;
-    int* my_slot_idx = slot_idx + row_in_tile;
+    // Running top-k of this thread's row: columns above tau are APPENDED to the row's buffer in shared memory (entry-major,
+    // [CAP][128 rows]: no bank conflicts); when a row of the warp has no room left, all 32 are cut back and get a new tau at
+    // once. An append is a few predicated instructions, and the number of selections grows with the logarithm of the
+    // columns; replacing the smallest of k entries column by column took some 400 cycles for each of the several hundred
+    // columns per row that enter, serialised over the lanes of a warp: 4096 x 24576 x 768, k 50: 332 -> 190 us.
+    RowState st = {0, row_ok ? 0.0f : __int_as_float(0x7f800000)};
+    RowBuffer<CAP, NARROW> rowbuf;
+    rowbuf.val0 = smem_u32(smem + L::kSlotValOff);
+    rowbuf.col0 = smem_u32(smem + L::kSlotIdxOff);
+    rowbuf.val = rowbuf.val0 + row_in_tile * 4;
+    const int col_base = NARROW ? p.n_index_offset + tile_begin * BN : 0;  // what the stored columns count from
+    // Bias and gate of the columns at work come through shared memory, fetched one step ahead by a coalesced load per warp
+    // (read per thread they were a miss in L1 for every step); columns past the end have gate 0.
+    float* col_bias = reinterpret_cast<float*>(smem + L::kColOff) + q * 64;
+    float* col_gate = col_bias + 32;
+    float next_bias = 0.0f, next_gate = 0.0f;
+    auto fetch_columns = [&](int c) {
+      const bool in = c + lane < p.N;
+      next_bias = in && p.bias != nullptr ? __ldg(p.bias + c + lane) : 0.0f;
+      next_gate = !in ? 0.0f : p.gate != nullptr ? __ldg(p.gate + c + lane) : 1.0f;
+    };
     if constexpr (TOPK) {
-      // (the slot arrays were filled before the CTA-wide barrier above)
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        float m = __int_as_float(0x7f800000);
-        if (p.resume_topk) {
-#pragma unroll
-          for (int t = 0; t < 8; ++t) m = fminf(m, my_slot_val[(g * 8 + t) * BM]);
-        } else if (g * 8 < p.k) {
-          m = 0.0f;
+      if (p.resume_topk && row_ok) {
+        // continue the sweep of an earlier launch: its result for (row, this column range) is the state
+        const long long o = (long long)row * ((long long)p.num_splits * KS) + (long long)split * KS;
+        for (int s = 0; s < KS; ++s) {
+          const int ix = p.cand_idx[o + s];
+          if (ix < 0) continue;
+          const uint32_t a = rowbuf.val + st.n * (BM * 4);
+          store_entry_if<NARROW>(true, a, rowbuf.col_of(a), __float_as_uint(p.cand_val[o + s]), NARROW ? kCarried + s : ix);
+          ++st.n;
         }
-        gmin[g] = m;
-        tau = (g == 0) ? m : fminf(tau, m);
       }
+      __syncwarp();
     }
+    fetch_columns(tile_begin * BN);
     int lt = 0;
     bool ok = true;
     for (int tile = tile_begin; tile < tile_end && ok; ++tile, ++lt) {
       const int buf = lt & 1;
       const uint32_t parity = (lt >> 1) & 1;
-      if (!mbar_wait_bounded(&tmem_full_bar[buf], parity, abort_flag)) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], parity, abort_flag))) {
         if (lane == 0) report_status(p.status, kTimeoutTmemFull, lt);
         *abort_flag = 1;
         ok = false;
@@ -313,107 +427,83 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       for (int chunk = 0; chunk < BN / 32; ++chunk) {
         const int c0 = n0 + chunk * 32;
         if (c0 >= p.N) break;  // uniform across the CTA
+        __syncwarp();  // (the previous step's values have been read)
+        col_bias[lane] = next_bias;
+        col_gate[lane] = next_gate;
+        __syncwarp();
+        fetch_columns(c0 + 32);
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr_row + (uint32_t)(chunk * 32), r);
         tmem_wait_ld();
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        const bool full_chunk = (c0 + 32 <= p.N);
-        if (p.bias != nullptr) {
-          if (full_chunk) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.bias + c0 + j));
-              v[j] += b4.x; v[j + 1] += b4.y; v[j + 2] += b4.z; v[j + 3] += b4.w;
-            }
-          } else {
+        for (int j = 0; j < 32; j += 4) {
+          const float4 b4 = *reinterpret_cast<const float4*>(col_bias + j);
+          add_pair(v[j], v[j + 1], b4.x, b4.y);
+          add_pair(v[j + 2], v[j + 3], b4.z, b4.w);
+        }
+        if constexpr (WRITE_H && TOPK) {  // (the ungated value)
+          if (row_ok) {
+            __nv_bfloat16* dst = p.H + (long long)row * p.ldh + c0;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) if (c0 + j < p.N) v[j] += __ldg(p.bias + c0 + j);
+            for (int j = 0; j < 32; j += 8)  // (N % 8 == 0)
+              if (c0 + j < p.N)
+                *reinterpret_cast<uint4*>(dst + j) = make_uint4(pack_bf16x2(v[j], v[j + 1]), pack_bf16x2(v[j + 2], v[j + 3]),
+                                                                pack_bf16x2(v[j + 4], v[j + 5]), pack_bf16x2(v[j + 6], v[j + 7]));
+          }
+        }
+        if (TOPK || p.gate != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const float4 g4 = *reinterpret_cast<const float4*>(col_gate + j);
+            mul_pair(v[j], v[j + 1], g4.x, g4.y);
+            mul_pair(v[j + 2], v[j + 3], g4.z, g4.w);
           }
         }
         if constexpr (WRITE_H && !TOPK) {
-          // plain store variants: an optional per-column gate (decoder row norm) is applied to the stored value
-          if (p.gate != nullptr) {
+          // A thread holds 64 bytes of its own row: through shared memory (16-byte pieces, swizzled: no bank conflicts), so that
+          // four lanes write whole sectors of a row. Stored from the registers, every instruction touched 32 rows by half a
+          // sector each: 4096 x 24576 x 768: 198 (with a gate: 425) -> 135 (149) us.
+          uint8_t* tile_s = smem + L::kStoreOff + q * 2048;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) if (full_chunk || c0 + j < p.N) v[j] *= __ldg(p.gate + c0 + j);
-          }
-        }
-        if constexpr (WRITE_H) {
-          if (row_ok) {
-            __nv_bfloat16* dst = p.H + (long long)row * p.ldh + c0;
-            if (full_chunk) {
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(tile_s + lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16)) =
+                make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
+                           pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+          __syncwarp();
 #pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 o;
-                o.x = pack_bf16x2(v[j], v[j + 1]);
-                o.y = pack_bf16x2(v[j + 2], v[j + 3]);
-                o.z = pack_bf16x2(v[j + 4], v[j + 5]);
-                o.w = pack_bf16x2(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = o;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) if (c0 + j < p.N) dst[j] = __float2bfloat16(v[j]);
-            }
+          for (int i = 0; i < 4; ++i) {
+            const int rr = i * 8 + (lane >> 2), j = lane & 3;
+            const uint4 o = *reinterpret_cast<const uint4*>(tile_s + rr * 64 + ((j ^ ((rr >> 1) & 3)) * 16));
+            if (m0 + q * 32 + rr < p.M && c0 + j * 8 < p.N)  // (N % 8 == 0)
+              *reinterpret_cast<uint4*>(p.H + (long long)(m0 + q * 32 + rr) * p.ldh + c0 + j * 8) = o;
           }
         }
         if constexpr (TOPK) {
-          if (p.gate != nullptr) {
-            if (full_chunk) {
 #pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                const float4 g4 = __ldg(reinterpret_cast<const float4*>(p.gate + c0 + j));
-                v[j] *= g4.x; v[j + 1] *= g4.y; v[j + 2] *= g4.z; v[j + 3] *= g4.w;
-              }
-            } else {
+          for (int h = 0; h < 32; h += 16) {
+            float m[4];
 #pragma unroll
-              for (int j = 0; j < 32; ++j) if (c0 + j < p.N) v[j] *= __ldg(p.gate + c0 + j);
+            for (int j = 0; j < 4; ++j) m[j] = fmaxf(fmaxf(v[h + j], v[h + 4 + j]), fmaxf(v[h + 8 + j], v[h + 12 + j]));
+            const bool enters = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) > st.tau;
+            if (!__any_sync(0xffffffffu, enters)) continue;
+            if (__any_sync(0xffffffffu, enters && st.n + 16 > CAP)) {
+              int enter = 0;
+#pragma unroll
+              for (int j = 0; j < 16; ++j) enter += v[h + j] > st.tau;
+              if (__any_sync(0xffffffffu, st.n + enter > CAP))
+                st = select_entries<CAP, NARROW>(rowbuf, st, p.k, min(p.k + max(8, (CAP - p.k) / 4), CAP - 16));
             }
-          }
-          if (!row_ok) {
+            uint32_t at = rowbuf.val + (uint32_t)st.n * (BM * 4);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = -1.0f;
-          }
-          // Which of this row's 32 values beat the current threshold? Usually none. The rare inserts run
-          // in a per-thread loop (one copy of the insert code; lanes work on different columns at once).
-          uint32_t pending = 0;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const bool in_range = full_chunk || (c0 + j < p.N);
-            pending |= (in_range && v[j] > tau) ? (1u << j) : 0u;
-          }
-          while (pending != 0) {
-            const int j = __ffs(pending) - 1;
-            pending &= pending - 1;
-            const float g = select32(v, j);
-            if (g > tau) {
-              int gi = 0;
-              float gm = gmin[0];
-#pragma unroll
-              for (int t = 1; t < NG; ++t) {
-                if (gmin[t] < gm) { gm = gmin[t]; gi = t; }
-              }
-              float* gv = my_slot_val + gi * 8 * BM;
-              float sv[8];
-#pragma unroll
-              for (int t = 0; t < 8; ++t) sv[t] = gv[t * BM];
-              int sel = 0;
-#pragma unroll
-              for (int t = 7; t >= 0; --t) sel = (sv[t] == gm) ? t : sel;
-              gv[sel * BM] = g;
-              my_slot_idx[(gi * 8 + sel) * BM] = p.n_index_offset + c0 + j;
-              float nm = g;
-#pragma unroll
-              for (int t = 0; t < 8; ++t) nm = fminf(nm, (t == sel) ? g : sv[t]);
-              float nt = nm;
-#pragma unroll
-              for (int t = 0; t < NG; ++t) {
-                gmin[t] = (t == gi) ? nm : gmin[t];
-                nt = fminf(nt, gmin[t]);
-              }
-              tau = nt;
+            for (int j = 0; j < 16; ++j) {
+              const bool above = v[h + j] > st.tau;
+              store_entry_if<NARROW>(above, at, rowbuf.col_of(at), __float_as_uint(v[h + j]), p.n_index_offset + c0 + h + j - col_base);
+              at = at + (above ? BM * 4 : 0);
             }
+            st.n = (int)((at - rowbuf.val) / (BM * 4));
           }
         }
       }
@@ -425,13 +515,26 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         else mbar_arrive(&tmem_empty_bar[buf]);
       }
     }
+    if constexpr (TOPK) {
+      __syncwarp();
+      st = select_entries<CAP, NARROW>(rowbuf, st, p.k, KS);
+    }
     if constexpr (TOPK) if (ok && row_ok) {
-      // emit this sweep's candidates: [row][split * KS + slot]
+      // emit this sweep's candidates (at least the k best, at most KS): [row][split * KS + slot]
       const long long o = (long long)row * ((long long)p.num_splits * KS) + (long long)split * KS;
-      for (int s = 0; s < KS; ++s) {
-        const bool valid = s < p.k;
-        p.cand_val[o + s] = valid ? my_slot_val[s * BM] : 0.0f;
-        p.cand_idx[o + s] = valid ? my_slot_idx[s * BM] : -1;
+      for (int s = 0; s < KS; s += 4) {
+        float v[4];
+        int ix[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const bool valid = s + i < st.n;
+          v[i] = valid ? __uint_as_float(rowbuf.value(s + i)) : 0.0f;
+          ix[i] = valid ? (int)rowbuf.column(s + i) : -1;
+          // (an entry carried over from slot c sits at or before slot c: its column there is not overwritten yet)
+          if (NARROW && valid) ix[i] = ix[i] >= kCarried ? p.cand_idx[o + ix[i] - kCarried] : ix[i] + col_base;
+        }
+        *reinterpret_cast<float4*>(p.cand_val + o + s) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<int4*>(p.cand_idx + o + s) = make_int4(ix[0], ix[1], ix[2], ix[3]);
       }
       // a panel with fewer ranges than the lists have room for: its last range also marks the unused lists empty
       if (split == my_splits - 1) {
@@ -461,12 +564,12 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 }
 
 // ---- host side -------------------------------------------------------------------------------
-template <bool WRITE_H, bool TOPK, int STAGES, int KS, bool PAIR>
+template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW = false>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p,
                                   cudaStream_t stream) {
-  using L = SmemLayout<STAGES, KS, PAIR>;
+  using L = SmemLayout<STAGES, CAP, PAIR, NARROW>;
   static_assert(L::kDynamicBytes <= 232448, "shared memory of one CTA exceeds 227 KB");
-  auto kern = enc_gemm_kernel<WRITE_H, TOPK, STAGES, KS, PAIR>;
+  auto kern = enc_gemm_kernel<WRITE_H, TOPK, STAGES, KS, CAP, PAIR, NARROW>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -486,7 +589,7 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
 
 // mode: bit 0 = WRITE_H, bit 1 = TOPK, bit 2 = 3-stage ring for the plain single-CTA variant (a tuning probe),
 // bit 3 = CTA-pair variant (needs an even number of panels; `tb` must then have a 128-row box),
-// bit 4 = with bit 3 and TOPK: a 4-stage ring (under 200 KB of shared memory), which leaves room on the SM for
+// bit 4 = with bit 3 and TOPK: a shorter ring (under 200 KB of shared memory), which leaves room on the SM for
 //         CTAs of a bandwidth-bound kernel running at the same time on another stream.
 // Returns a CUDA error code (0 = launched).
 int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p, int mode,
@@ -501,18 +604,28 @@ int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmP
       return (int)cudaErrorInvalidValue;
   }
   cudaError_t e;
+  // 16-bit columns unless a range is too wide for them. Above k 32 the larger buffer where the epilogue is the bottleneck (an output
+  // tile's MMAs take less time up to K of about 2048) or 80 entries would be cut back at nearly every step; else the longer ring.
+  const int n_tiles = (p.N + BN - 1) / BN, panel_units = pair ? p.num_panels / 2 : p.num_panels;
+  const int ranges = p.units != 0 ? p.units / panel_units : p.num_splits;
+  const bool narrow = (n_tiles + ranges - 1) / ranges <= kNarrowTiles, large = p.K <= 2048 || p.k > 56;
   if (!tk) {
-    if (pair) e = launch_variant<true, false, 6, 0, true>(ta, tb, p, stream);
-    else e = (mode & 4) ? launch_variant<true, false, 3, 0, false>(ta, tb, p, stream)
-                        : launch_variant<true, false, 4, 0, false>(ta, tb, p, stream);
+    if (pair) e = launch_variant<true, false, 6, 0, 0, true>(ta, tb, p, stream);
+    else e = (mode & 4) ? launch_variant<true, false, 3, 0, 0, false>(ta, tb, p, stream)
+                        : launch_variant<true, false, 4, 0, 0, false>(ta, tb, p, stream);
   } else if (p.k <= 32) {
-    if (pair && compact && !wh) e = launch_variant<false, true, 4, 32, true>(ta, tb, p, stream);
-    else if (pair) e = wh ? launch_variant<true, true, 6, 32, true>(ta, tb, p, stream) : launch_variant<false, true, 6, 32, true>(ta, tb, p, stream);
-    else e = wh ? launch_variant<true, true, 4, 32, false>(ta, tb, p, stream) : launch_variant<false, true, 4, 32, false>(ta, tb, p, stream);
+    if (pair && !wh && narrow) e = compact ? launch_variant<false, true, 4, 32, 80, true, true>(ta, tb, p, stream)
+                                           : launch_variant<false, true, 5, 32, 80, true, true>(ta, tb, p, stream);
+    else if (pair) e = wh ? launch_variant<true, true, 5, 32, 64, true>(ta, tb, p, stream) : launch_variant<false, true, 5, 32, 64, true>(ta, tb, p, stream);
+    else if (!wh && narrow) e = launch_variant<false, true, 3, 32, 96, false, true>(ta, tb, p, stream);
+    else e = wh ? launch_variant<true, true, 3, 32, 64, false>(ta, tb, p, stream) : launch_variant<false, true, 3, 32, 64, false>(ta, tb, p, stream);
   } else {
-    if (pair && compact && !wh) e = launch_variant<false, true, 4, 64, true>(ta, tb, p, stream);
-    else if (pair) e = wh ? launch_variant<true, true, 5, 64, true>(ta, tb, p, stream) : launch_variant<false, true, 5, 64, true>(ta, tb, p, stream);
-    else e = wh ? launch_variant<true, true, 3, 64, false>(ta, tb, p, stream) : launch_variant<false, true, 3, 64, false>(ta, tb, p, stream);
+    if (pair && !wh && narrow) e = compact ? launch_variant<false, true, 4, 64, 80, true, true>(ta, tb, p, stream)
+                                   : large ? launch_variant<false, true, 4, 64, 128, true, true>(ta, tb, p, stream)
+                                           : launch_variant<false, true, 5, 64, 80, true, true>(ta, tb, p, stream);
+    else if (pair) e = wh ? launch_variant<true, true, 4, 64, 96, true>(ta, tb, p, stream) : launch_variant<false, true, 4, 64, 96, true>(ta, tb, p, stream);
+    else if (!wh && narrow) e = launch_variant<false, true, 3, 64, 96, false, true>(ta, tb, p, stream);
+    else e = wh ? launch_variant<true, true, 3, 64, 80, false>(ta, tb, p, stream) : launch_variant<false, true, 3, 64, 80, false>(ta, tb, p, stream);
   }
   return (int)e;
 }
