@@ -157,7 +157,7 @@ int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, 
 // of it are enough), and for k well below 2048 hardly more than k are. Pass 2 collects the columns at or above that bound in
 // shared memory, where the exact k-th value is found by a descent over the value bits. Rows whose bound lets too many through
 // (values repeated thousands of times) and k > 1024 take a radix descent over the row itself: four histogram passes.
-// 4096 rows of 32768 gated columns, k 128: 546 us (histograms for every row) -> 217 us; 2048 x 8192: 125 -> 70 us.
+// 4096 rows of 32768 gated columns, k 128: 546 us (histograms for every row) -> 196 us; 2048 x 8192: 125 -> 58 us.
 // ------------------------------------------------------------------------------------------------
 constexpr int RT_THREADS = 256;  // (what is left of a row's time is latency: five CTAs of 256 threads per SM hide it as well as three of 512 with wider barriers)
 constexpr int RT_MAXIMA = 8;     // column groups per thread
@@ -277,23 +277,28 @@ __device__ __noinline__ void row_topk_radix(const __nv_bfloat16* __restrict__ hr
 }
 
 // The largest t whose lowest `skip` bits are zero with  count(values >= t) >= k  over the CTA (the values' bit patterns are those
-// of non-negative floats; fewer than k of them at all: 0). Two bits per step and one barrier: the three counts travel in one
-// word, and every step has a word of its own in `counts` (zeroed before). Every thread returns the same.
+// of non-negative floats; fewer than k of them at all: 0). Two bits per step and one barrier: a warp's three counts travel in one
+// word, which every warp adds up for itself (atomic sums cost 1500 cycles a step: 217 and 70 us; the words of two steps alternate). Every
+// thread returns the same.
+constexpr int RT_WARPS = RT_THREADS / 32;
 template <int N>
-__device__ __forceinline__ unsigned descend(const unsigned (&val)[N], int k, int skip, unsigned long long* counts) {
-  static_assert(N * 32 < 1024, "a warp's counts are packed in ten bits each");
+__device__ __forceinline__ unsigned descend(const unsigned (&val)[N], int k, int skip, unsigned (&counts)[2][RT_WARPS]) {
+  static_assert(N * 32 < 1024 && RT_WARPS <= 32, "a warp's counts are packed in ten bits each");
+  const int lane = threadIdx.x & 31;
   unsigned t = 0;
+  __syncthreads();  // (the words may still be read by an earlier call)
   for (int shift = 30; shift >= skip; shift -= 2) {  // (bit 31 is never set)
     const unsigned t1 = t | (1u << shift), t2 = t | (2u << shift), t3 = t | (3u << shift);
     unsigned n = 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) n += (unsigned)(val[i] >= t1) + ((unsigned)(val[i] >= t2) << 10) + ((unsigned)(val[i] >= t3) << 20);
     n = __reduce_add_sync(0xffffffffu, n);
-    if ((threadIdx.x & 31) == 0 && n != 0)
-      atomicAdd(&counts[shift >> 1], (unsigned long long)(n & 1023u) | ((unsigned long long)((n >> 10) & 1023u) << 21) | ((unsigned long long)(n >> 20) << 42));
+    unsigned* words = counts[(shift >> 1) & 1];
+    if (lane == 0) words[threadIdx.x >> 5] = n;
     __syncthreads();
-    const unsigned long long c = counts[shift >> 1];
-    const int c1 = (int)(c & 0x1fffffu), c2 = (int)((c >> 21) & 0x1fffffu), c3 = (int)(c >> 42);
+    n = lane < RT_WARPS ? words[lane] : 0u;
+    const int c1 = (int)__reduce_add_sync(0xffffffffu, n & 1023u), c2 = (int)__reduce_add_sync(0xffffffffu, (n >> 10) & 1023u),
+              c3 = (int)__reduce_add_sync(0xffffffffu, n >> 20);
     const int at = c3 >= k ? c3 : c2 >= k ? c2 : c1;
     if (c3 >= k) t = t3;
     else if (c2 >= k) t = t2;
@@ -312,11 +317,10 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
   const __nv_bfloat16* hrow = H + (long long)row * ldh;
   __shared__ unsigned s_bits[RT_CAP];
   __shared__ int s_col[RT_CAP];
-  __shared__ unsigned long long s_count[32];  // the two descents' steps
+  __shared__ unsigned s_count[2][RT_WARPS];
   __shared__ int s_n, s_cursor;
   bool use_radix = k > RT_BOUND_K;
   if (!use_radix) {
-    if (threadIdx.x < 32) s_count[threadIdx.x] = 0;
     if (threadIdx.x == 0) { s_n = 0; s_cursor = 0; }
     // ---- pass 1: maxima of this thread's eight column groups (non-positive values and NaN never enter)
     float mx[RT_MAXIMA];
@@ -361,7 +365,7 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
           const int j = threadIdx.x + i * RT_THREADS;
           mine[i] = j < n_cand ? s_bits[j] : 0u;
         }
-        thr = descend(mine, k, 0, s_count + 16);
+        thr = descend(mine, k, 0, s_count);
       }
       // ---- winners: what lies above it first, then as many equal ones as there are places
       auto place = [&](int j) {
