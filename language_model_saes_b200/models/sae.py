@@ -147,7 +147,15 @@ class SparseAutoEncoder(SparseDictionary):
     # ---- forward -----------------------------------------------------------------------------
     def encode(self, x: torch.Tensor, return_hidden_pre: bool = False, **kwargs):
         x = x.to(self.W_E.dtype)
-        hidden_pre = x @ self.W_E + self.b_E
+        if not return_hidden_pre and self._rowwise_topk_inference(x):
+            from ..ops.inference import topk_dense, topk_dense_supported
+
+            h = x @ self.W_E
+            if topk_dense_supported(h, k := min(self.current_k, h.shape[-1])):
+                return topk_dense(h, self.b_E, self.decoder_norm() if self.cfg.sparsity_include_decoder_norm else None, k)
+            hidden_pre = h + self.b_E
+        else:
+            hidden_pre = x @ self.W_E + self.b_E
         if self.cfg.use_glu_encoder:
             hidden_pre = hidden_pre * torch.sigmoid(x @ self.W_E_glu + self.b_E_glu)
         hidden_pre = self.hook_hidden_pre(hidden_pre)
@@ -158,6 +166,24 @@ class SparseAutoEncoder(SparseDictionary):
             feature_acts = self.activation_function(hidden_pre)
         feature_acts = self.hook_feature_acts(feature_acts)
         return (feature_acts, hidden_pre) if return_hidden_pre else feature_acts
+
+    def _rowwise_topk_inference(self, x: torch.Tensor) -> bool:
+        """A plain forward pass of a TopK encoder that nothing listens to between its operations."""
+        if not x.is_cuda or self.cfg.use_glu_encoder or type(self.current_k) is not int or not getattr(self.activation_function, "rowwise_topk", False):
+            return False
+        if any(hp.fwd_hooks or hp.bwd_hooks for hp in (self.hook_hidden_pre, self.hook_feature_acts)):
+            return False
+        from ..ops.inference import plain_inference
+
+        return plain_inference(x, self.W_E, self.b_E, self.W_D)
+
+    def _sparse_inference(self, feature_acts: torch.Tensor) -> bool:
+        """A plain fp32 forward pass of a decoder whose activation function leaves few features active."""
+        if not feature_acts.is_cuda or self.cfg.act_fn.lower() not in ("topk", "batchtopk", "jumprelu"):
+            return False
+        from ..ops.inference import plain_inference, sparse_decode_supported
+
+        return plain_inference(feature_acts, self.W_D) and sparse_decode_supported(feature_acts, self.W_D)
 
     def _use_sparse_kernels(self, feature_acts: torch.Tensor) -> bool:
         """``use_triton_kernel`` (the reference's name for "decode through the sparse kernels") applies on CUDA when
@@ -170,6 +196,10 @@ class SparseAutoEncoder(SparseDictionary):
     def decode(self, feature_acts: torch.Tensor, **kwargs) -> torch.Tensor:
         if self._use_sparse_kernels(feature_acts):
             from ..ops.sparse_autograd import sparse_decode
+
+            partial = sparse_decode(feature_acts, self.W_D)
+        elif self._sparse_inference(feature_acts):
+            from ..ops.inference import sparse_decode
 
             partial = sparse_decode(feature_acts, self.W_D)
         else:

@@ -505,6 +505,7 @@ class SparseDictionary(HookedRootModule, ABC):
                 x = x * x.gt(0).to(x.dtype)
                 return topk(x, k=min(self.current_k, x.shape[-1]), dim=-1)
 
+            topk_activation.rowwise_topk = self.tp_size == 1
             return topk_activation
 
         def batch_topk(x: torch.Tensor):

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <torch/extension.h>
 
+#include <climits>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -189,6 +190,33 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
                                       opt_ptr<int>(out_idx), opt_ptr<float>(out_val), comm,
                                       at::cuda::getCurrentCUDAStream()),
              "topk_merge launch");
+}
+
+// out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]
+void topk_dense(const Tensor& h, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, const Tensor& out) {
+  CHECK_T(h, torch::kFloat32);
+  CHECK_T(out, torch::kFloat32);
+  TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && h.size(0) <= INT_MAX && h.size(1) <= INT_MAX, "h and out must be [B, F]");
+  if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
+  if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
+  const c10::cuda::CUDAGuard guard(h.device());
+  check_cuda(lmsae::topk_dense_launch(h.data_ptr<float>(), opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
+                                      (int)k, out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "topk_dense launch");
+}
+
+// out [B, d] = acts [B, F] @ W [F, d], fp32; marks: int32 [1 + B], zeroed
+void dense_decode(const Tensor& acts, const Tensor& W, const Tensor& marks, const Tensor& out) {
+  CHECK_T(acts, torch::kFloat32);
+  CHECK_T(W, torch::kFloat32);
+  CHECK_T(marks, torch::kInt32);
+  CHECK_T(out, torch::kFloat32);
+  TORCH_CHECK(acts.dim() == 2 && W.dim() == 2 && out.dim() == 2 && acts.size(1) == W.size(0) && out.size(0) == acts.size(0) &&
+              out.size(1) == W.size(1) && marks.numel() == acts.size(0) + 1 && acts.size(0) < INT_MAX && acts.size(1) <= INT_MAX, "acts [B, F], W [F, d], out [B, d], marks [1 + B]");
+  const c10::cuda::CUDAGuard guard(acts.device());
+  check_cuda(lmsae::dense_decode_launch(acts.data_ptr<float>(), W.data_ptr<float>(), (int)acts.size(0), (int)acts.size(1), (int)W.size(1),
+                                        marks.data_ptr<int>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "dense_decode launch");
 }
 
 void row_topk(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate, const c10::optional<Tensor>& alive,
@@ -1144,6 +1172,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("topk_dense", &topk_dense);
+  m.def("dense_decode", &dense_decode);
   m.def("sparse_decode", &sparse_decode);
   m.def("sparse_dact", &sparse_dact);
   m.def("mse_loss_grad", &mse_loss_grad);

@@ -400,4 +400,175 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
   return (int)cudaGetLastError();
 }
 
+// ------------------------------------------------------------------------------------------------
+// TopK activation on fp32 pre-activations, dense in and dense out:  out = topk(relu(g)) / norm  with  g = (h + bias) * norm  (bias and
+// norm optional), k entries per row. One CTA per row: group maxima bound the k-th value, a second pass (from L1 / L2) writes the
+// row's zeros and collects the few entries at or above the bound, and the k best of them are written over the zeros. Bound by
+// reading h and writing out. 4096 x 24576, k 50, bias, gate, selection, mask and division: 3.2 ms as torch operations -> 319 us.
+// The arithmetic is that of the operations it replaces, element by element: NaN and -inf (which relu(x) = x * [x > 0] turns into
+// NaN) rank first and stay NaN everywhere, an unselected +inf becomes NaN, and so does everything over a norm of 0 or NaN.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned topk_key(float g) {
+  const unsigned b = __float_as_uint(g);
+  if ((b & 0x7fffffffu) > 0x7f800000u || b == 0xff800000u) return 0x7fffffffu;
+  return (int)b > 0 ? b : 0u;
+}
+
+struct TopkDenseParams {
+  const float* h;
+  const float* bias;
+  const float* norm;
+  float* out;
+  int N, k;
+  bool vec;
+};
+
+// g of columns [c, c + 4), and whether a zero there ends as NaN (columns past the end of the row: g = 0)
+__device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const float* h, int c, float (&g)[4], bool (&bad)[4]) {
+  float n[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+  if (p.vec) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(h + c));
+    g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
+    if (p.bias != nullptr) {
+      const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + c));
+      g[0] = __fadd_rn(g[0], b.x); g[1] = __fadd_rn(g[1], b.y); g[2] = __fadd_rn(g[2], b.z); g[3] = __fadd_rn(g[3], b.w);
+    }
+    if (p.norm != nullptr) {
+      const float4 b = __ldg(reinterpret_cast<const float4*>(p.norm + c));
+      n[0] = b.x; n[1] = b.y; n[2] = b.z; n[3] = b.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool in = c + i < p.N;
+      g[i] = in ? h[c + i] : 0.0f;
+      if (in && p.bias != nullptr) g[i] = __fadd_rn(g[i], p.bias[c + i]);
+      if (in && p.norm != nullptr) n[i] = p.norm[c + i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (p.norm != nullptr) g[i] = __fmul_rn(g[i], n[i]);
+    const unsigned nb = __float_as_uint(n[i]) & 0x7fffffffu;
+    bad[i] = (__float_as_uint(g[i]) & 0x7fffffffu) >= 0x7f800000u || nb == 0u || nb > 0x7f800000u;
+  }
+}
+
+__global__ void __launch_bounds__(RT_THREADS, 5)
+topk_dense_kernel(const TopkDenseParams p) {
+  __shared__ unsigned s_key[RT_CAP];
+  __shared__ int s_col[RT_CAP];
+  __shared__ unsigned s_count[2][RT_WARPS];
+  __shared__ int s_n, s_cursor;
+  const float* h = p.h + (size_t)blockIdx.x * p.N;
+  float* out = p.out + (size_t)blockIdx.x * p.N;
+  const int N = p.N, k = p.k;
+  if (threadIdx.x == 0) { s_n = 0; s_cursor = 0; }
+  unsigned mx[RT_MAXIMA];
+#pragma unroll
+  for (int i = 0; i < RT_MAXIMA; ++i) mx[i] = 0u;
+#pragma unroll 2
+  for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+#pragma unroll
+    for (int half = 0; half < 8; half += 4) {
+      if (c + half >= N) break;
+      float g[4];
+      bool bad[4];
+      topk_dense_load(p, h, c + half, g, bad);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mx[half + i] = max(mx[half + i], topk_key(g[i]));
+    }
+  }
+  unsigned thr = descend(mx, k, 16, s_count);  // a bound until the exact value is known (0: fewer than k positive maxima)
+  const float nan = __uint_as_float(0x7fffffffu);
+#pragma unroll 2
+  for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+#pragma unroll
+    for (int half = 0; half < 8; half += 4) {
+      if (c + half >= N) break;
+      float g[4];
+      bool bad[4];
+      topk_dense_load(p, h, c + half, g, bad);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned key = topk_key(g[i]);
+        if (key != 0u && key >= thr) {
+          const int pos = atomicAdd(&s_n, 1);
+          if (pos < RT_CAP) { s_key[pos] = key; s_col[pos] = c + half + i; }
+        }
+        g[i] = bad[i] ? nan : 0.0f;
+      }
+      if (p.vec) {
+        __stcs(reinterpret_cast<float4*>(out + c + half), make_float4(g[0], g[1], g[2], g[3]));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c + half + i < N) out[c + half + i] = g[i];
+      }
+    }
+  }
+  __syncthreads();  // (also: the zeros are written before what is written over them)
+  const int n = s_n;
+  auto put = [&](int c, unsigned key) {
+    if (atomicAdd(&s_cursor, 1) >= k || key == 0x7fffffffu) return;  // (what is NaN already stays so)
+    float v = __uint_as_float(key);
+    if (p.norm != nullptr) v = __fdiv_rn(v, p.norm[c]);
+    out[c] = v;
+  };
+  if (n <= RT_CAP) {
+    unsigned mine[RT_CAP / RT_THREADS];
+#pragma unroll
+    for (int i = 0; i < RT_CAP / RT_THREADS; ++i) {
+      const int j = threadIdx.x + i * RT_THREADS;
+      mine[i] = j < n ? s_key[j] : 0u;
+    }
+    thr = n > k ? descend(mine, k, 0, s_count) : 0u;
+    for (int j = threadIdx.x; j < n; j += RT_THREADS)
+      if (s_key[j] > thr) put(s_col[j], s_key[j]);
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += RT_THREADS)
+      if (s_key[j] == thr) put(s_col[j], thr);
+    return;
+  }
+  // values repeated thousands of times: the descent over the row itself, one pass per bit
+  auto keys_of = [&](auto&& visit) {
+    for (int c = threadIdx.x * 4; c < N; c += RT_THREADS * 4) {
+      float g[4];
+      bool bad[4];
+      topk_dense_load(p, h, c, g, bad);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned key = topk_key(g[i]);
+        if (key != 0u) visit(c + i, key);
+      }
+    }
+  };
+  thr = 0u;
+  for (int bit = 30; bit >= 0; --bit) {
+    const unsigned trial = thr | (1u << bit);
+    int mine = 0;
+    keys_of([&](int, unsigned key) { mine += key >= trial; });
+    const unsigned total = __reduce_add_sync(0xffffffffu, (unsigned)mine);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_count[0][threadIdx.x >> 5] = total;
+    __syncthreads();
+    const unsigned all = __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < RT_WARPS ? s_count[0][threadIdx.x & 31] : 0u);
+    if (all >= (unsigned)k) thr = trial;
+  }
+  keys_of([&](int c, unsigned key) { if (key > thr) put(c, key); });
+  __syncthreads();
+  keys_of([&](int c, unsigned key) { if (key == thr) put(c, key); });
+}
+
+int topk_dense_launch(const float* h, const float* bias, const float* norm, int B, int N, int k, float* out, cudaStream_t stream) {
+  if (B <= 0 || N <= 0) return 0;
+  if (k < 1 || k > RT_BOUND_K) return (int)cudaErrorInvalidValue;
+  TopkDenseParams p;
+  p.h = h; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
+                          reinterpret_cast<uintptr_t>(out)) % 16 == 0);
+  topk_dense_kernel<<<B, RT_THREADS, 0, stream>>>(p);
+  return (int)cudaGetLastError();
+}
+
 }  // namespace lmsae

@@ -1,0 +1,61 @@
+"""fp32 inference of a sparse dictionary on the GPU: TopK activation and decoder as kernels in place of dense tensor operations
+(the eager statements of models/sae.py:288-377 and utils/math.py:81-171 in the reference project).
+
+Both give what the dense operations give, NaN and infinities included, and neither makes the host wait. They apply to plain
+forward passes only: whatever listens to or rewrites tensor operations (autograd, forward-mode differentiation, function
+transforms, autocast, tracing, dispatch modes, tensor subclasses) gets the tensor operations."""
+
+from __future__ import annotations
+
+import torch
+from torch.autograd import forward_ad
+from torch.utils._python_dispatch import _get_current_dispatch_mode
+
+from . import sae_kernels as K
+
+MAX_K = 1024  # the selection kernel's bound comes from 2048 column groups
+
+
+def plain_inference(*tensors: torch.Tensor) -> bool:
+    """Whether nothing but the values of an operation on these CUDA tensors is wanted."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    if not all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32 for t in tensors):
+        return False
+    return not (
+        any(t.device != tensors[0].device for t in tensors)
+        or torch.is_autocast_enabled("cuda")
+        or torch.jit.is_tracing()
+        or torch.compiler.is_compiling()
+        or forward_ad._current_level >= 0
+        or torch._C._functorch.peek_interpreter_stack() is not None
+        or _get_current_dispatch_mode() is not None
+        or len(torch.overrides._get_current_function_mode_stack()) != 0
+    )
+
+
+def topk_dense_supported(h: torch.Tensor, k: int) -> bool:
+    return h.ndim >= 1 and h.is_contiguous() and 1 <= k <= MAX_K and 0 < h.numel() < 2**62 and 0 < h.shape[-1] < 2**31 - 64
+
+
+def topk_dense(h: torch.Tensor, bias: torch.Tensor | None, norm: torch.Tensor | None, k: int) -> torch.Tensor:
+    """``topk(relu((h + bias) * norm)) / norm`` over the last dimension (``bias`` and ``norm`` optional)."""
+    rows = h.reshape(-1, h.shape[-1])
+    out = torch.empty_like(rows)
+    K._ext().topk_dense(rows, bias.contiguous() if bias is not None else None, norm.contiguous() if norm is not None else None, k, out)
+    return out.view(h.shape)
+
+
+def sparse_decode_supported(acts: torch.Tensor, W: torch.Tensor) -> bool:
+    F, d = W.shape
+    return (acts.ndim >= 2 and acts.shape[-1] == F and acts.is_contiguous() and W.is_contiguous() and F % 4 == 0 and d % 4 == 0 and F > 0 and d > 0
+            and acts.data_ptr() % 16 == 0 and W.data_ptr() % 16 == 0 and F < 2**31 - 64 and 0 < acts.numel() // F < 2**31 - 64)  # fmt: skip
+
+
+def sparse_decode(acts: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
+    """``acts @ W`` for ``acts [..., F]`` with few non-zeros."""
+    rows = acts.reshape(-1, acts.shape[-1])
+    out = torch.empty(rows.shape[0], W.shape[1], dtype=torch.float32, device=acts.device)
+    marks = torch.zeros(1 + rows.shape[0], dtype=torch.int32, device=acts.device)
+    K._ext().dense_decode(rows, W.detach(), marks, out)
+    return out.view(*acts.shape[:-1], W.shape[1])

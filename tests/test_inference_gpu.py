@@ -1,0 +1,103 @@
+"""The kernels of fp32 inference against the tensor operations they stand for: row lengths around a vector and a CTA, unaligned
+rows, every number of features kept, repeated values, NaN, infinities and zero norms; decoders with sparse rows, rows too dense
+for the lists, and weights that are not finite; and the calls that have to take the tensor operations as before."""
+
+import pytest
+import torch
+
+from language_model_saes_b200 import SAEConfig, SparseAutoEncoder
+from language_model_saes_b200.ops import inference as I
+from language_model_saes_b200.utils.math import topk
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("F", [1, 7, 64, 2047, 2052, 24576, 50001])
+@pytest.mark.parametrize("k", [1, 50, 1024])
+@pytest.mark.parametrize("data", ["normal", "few", "repeated", "special"])
+@pytest.mark.parametrize("parts", ["both", "none"])
+def test_topk_activation(F, k, data, parts):
+    g = torch.Generator().manual_seed(F + k)
+    h = torch.randn(4, F, generator=g)
+    if data == "few":
+        h -= 3.0
+    elif data == "repeated":
+        h = h.sign() * 0.5
+        h[:, ::9] = 1.5
+    bias, norm = (0.1 * torch.randn(F, generator=g), torch.rand(F, generator=g) + 0.5) if parts == "both" and data != "repeated" else (None, None)
+    if data == "special":
+        h[0, :: max(1, F // 5)] = float("nan")
+        h[0, F // 5 // 2 if F >= 10 else 0] = float("inf")  # selected only if the NaNs leave a place (which of equals is kept is free)
+        h[1, F - 1] = float("inf")
+        h[2, F // 2] = -float("inf")
+        if norm is not None:
+            norm[F // 3] = 0.0
+    k = min(k, F)
+    h, bias, norm = (t.to(DEV) if t is not None else None for t in (h, bias, norm))
+    out = I.topk_dense(h, bias, norm, k)
+    g_ = h + bias if bias is not None else h
+    g_ = g_ * norm if norm is not None else g_
+    r = g_ * g_.gt(0).to(g_.dtype)
+    want = topk(r, k=k)
+    want = want / norm if norm is not None else want
+    assert torch.equal(out.isnan(), want.isnan())
+    if data == "repeated":  # which of the equal values are kept is free
+        assert torch.equal(out.sort(-1).values, want.sort(-1).values)
+        assert ((out == 0) | (out == h)).all()
+    else:
+        assert torch.equal(out.nan_to_num(nan=-1.0), want.nan_to_num(nan=-1.0))
+
+
+@pytest.mark.parametrize("B,F,d", [(1, 4, 4), (130, 1000, 64), (5, 24576, 768), (3, 4100, 1028), (129, 512, 256)])
+@pytest.mark.parametrize("rows", ["sparse", "some dense", "inf weight"])
+def test_decoder(B, F, d, rows):
+    g = torch.Generator().manual_seed(B + F)
+    a = torch.randn(B, F, generator=g) * (torch.rand(B, F, generator=g) < 20 / F)
+    W = torch.randn(F, d, generator=g)
+    if rows == "some dense":
+        a[B // 2] = torch.randn(F, generator=g)
+        a[0] = 0.0
+    elif rows == "inf weight":
+        W[F // 2, 1] = float("inf")
+    out = I.sparse_decode(a.to(DEV), W.to(DEV)).cpu()
+    want = a.double() @ W.double()
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    # fp32 sums: 2^-24 of the sum of magnitudes for each of the non-zero terms
+    n = (a != 0).sum(1, keepdim=True) + 1
+    bound = 2.0**-24 * n * (a.double().abs() @ W.double().abs().nan_to_num(posinf=1.0)) + 1e-30
+    ok = want.isfinite()
+    assert ((out.double() - want).abs()[ok] <= bound.expand_as(want)[ok]).all()
+
+
+def _sae(act):
+    torch.manual_seed(0)
+    cfg = SAEConfig(hook_point_in="h", hook_point_out="h", d_model=64, expansion_factor=8, act_fn=act, top_k=10, device=DEV, dtype=torch.float32)
+    sae = SparseAutoEncoder(cfg)
+    sae.init_parameters(encoder_uniform_bound=0.2, decoder_uniform_bound=0.2, init_log_jumprelu_threshold_value=-1.0)
+    return sae
+
+
+@pytest.mark.parametrize("act", ["topk", "jumprelu"])
+def test_model_routes(act):
+    sae = _sae(act)
+    x = torch.randn(3, 5, 64, device=DEV)
+    acts = sae.encode(x)  # with autograd: tensor operations
+    rec = sae.decode(acts)
+    assert acts.requires_grad and rec.requires_grad
+    with torch.no_grad():
+        a, r = sae.encode(x), sae.decode(acts.detach())
+        a2, h2 = sae.encode(x, return_hidden_pre=True)
+        assert a.shape == acts.shape and r.shape == rec.shape and h2.shape == acts.shape
+        assert torch.equal(a, acts) and torch.equal(a2, a)
+        assert torch.allclose(r, rec, atol=1e-5)
+        seen = []
+        sae.hook_hidden_pre.add_hook(lambda t, hook: seen.append(t) or t * 0)
+        assert not sae.encode(x).any() and len(seen) == 1
+        sae.hook_hidden_pre.remove_hooks()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert sae.decode(a).dtype == torch.bfloat16 or not sae.cfg.use_decoder_bias or sae.decode(a).dtype == torch.float32
+        if act == "topk":
+            assert torch.allclose(torch.vmap(lambda t: sae.decode(sae.encode(t)))(x), r, atol=1e-5)
+            _, tangent = torch.func.jvp(lambda t: sae.decode(sae.encode(t)), (x,), (torch.ones_like(x),))
+            assert tangent.any()
