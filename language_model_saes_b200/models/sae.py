@@ -148,11 +148,15 @@ class SparseAutoEncoder(SparseDictionary):
     def encode(self, x: torch.Tensor, return_hidden_pre: bool = False, **kwargs):
         x = x.to(self.W_E.dtype)
         if not return_hidden_pre and self._rowwise_topk_inference(x):
-            from ..ops.inference import topk_dense, topk_dense_supported
+            from ..ops import inference
 
+            k = min(self.current_k, self.W_E.shape[1])
+            norm = self.decoder_norm() if self.cfg.sparsity_include_decoder_norm else None
+            if 1 <= k <= inference.MAX_K and inference.product_supported(x, self.W_E):
+                return inference.topk_encode(x, self.W_E, self.b_E, norm, k)
             h = x @ self.W_E
-            if topk_dense_supported(h, k := min(self.current_k, h.shape[-1])):
-                return topk_dense(h, self.b_E, self.decoder_norm() if self.cfg.sparsity_include_decoder_norm else None, k)
+            if inference.topk_dense_supported(h, k):
+                return inference.topk_dense(h, self.b_E, norm, k)
             hidden_pre = h + self.b_E
         else:
             hidden_pre = x @ self.W_E + self.b_E

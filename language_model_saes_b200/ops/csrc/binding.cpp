@@ -192,15 +192,48 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
              "topk_merge launch");
 }
 
-// out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]
-void topk_dense(const Tensor& h, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, const Tensor& out) {
+// C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu)
+void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status) {
+  CHECK_T(A, torch::kFloat32);
+  CHECK_T(B, torch::kFloat32);
+  CHECK_T(C, torch::kFloat32);
+  CHECK_T(status, torch::kInt32);
+  TORCH_CHECK(A.dim() == 2 && B.dim() == 2 && C.dim() == 2 && A.size(1) == B.size(1) && C.size(0) == A.size(0) && C.size(1) == B.size(0),
+              "A [M,K], B [N,K], C [M,N]");
+  const int64_t M = A.size(0), N = B.size(0), K = A.size(1), kp = (K + 63) / 64 * 64;
+  TORCH_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && M < INT_MAX - 256 && N < INT_MAX - 256 && 3 * kp < INT_MAX, "unsupported sizes");
+  const c10::cuda::CUDAGuard guard(A.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  const auto b16 = A.options().dtype(torch::kBFloat16), i32 = A.options().dtype(torch::kInt32);
+  const Tensor As = torch::empty({M, 3 * kp}, b16), Bs = torch::empty({N, 3 * kp}, b16);
+  const Tensor flags = torch::zeros({M + N + 2}, i32);
+  int* fa = flags.data_ptr<int>();
+  int* fb = fa + 1 + M;
+  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, stream), "split");
+  check_cuda(lmsae::split_bf16x3_launch(B.data_ptr<float>(), (int)N, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, stream), "split");
+  const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, 3 * kp, 128);
+  const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), N, 3 * kp, 128);
+  check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), B.data_ptr<float>(), (int)M, (int)N, (int)K, (int)kp, fa, fb, C.data_ptr<float>(),
+                                     status.data_ptr<int>(), stream),
+             "fp32_gemm launch");
+}
+
+// out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]; with x [B, K] and W [F, K], h is an estimate of x W^T (and may be
+// overwritten)
+void topk_dense(const Tensor& h, const c10::optional<Tensor>& x, const c10::optional<Tensor>& W, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, const Tensor& out) {
   CHECK_T(h, torch::kFloat32);
   CHECK_T(out, torch::kFloat32);
   TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && h.size(0) <= INT_MAX && h.size(1) <= INT_MAX, "h and out must be [B, F]");
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
   if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
+  if (x.has_value()) {
+    CHECK_T(*x, torch::kFloat32);
+    TORCH_CHECK(W.has_value() && x->dim() == 2 && x->size(0) == h.size(0), "x [B, K] and W [F, K] come together");
+    CHECK_T(*W, torch::kFloat32);
+    TORCH_CHECK(W->dim() == 2 && W->size(0) == h.size(1) && W->size(1) == x->size(1) && x->size(1) <= INT_MAX, "x [B, K] and W [F, K] come together");
+  }
   const c10::cuda::CUDAGuard guard(h.device());
-  check_cuda(lmsae::topk_dense_launch(h.data_ptr<float>(), opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
+  check_cuda(lmsae::topk_dense_launch(h.data_ptr<float>(), opt_ptr<const float>(x), opt_ptr<const float>(W), x.has_value() ? (int)x->size(1) : 0, opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
                                       (int)k, out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
              "topk_dense launch");
 }
@@ -1173,6 +1206,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
   m.def("topk_dense", &topk_dense);
+  m.def("fp32_gemm", &fp32_gemm);
   m.def("dense_decode", &dense_decode);
   m.def("sparse_decode", &sparse_decode);
   m.def("sparse_dact", &sparse_dact);

@@ -1,0 +1,305 @@
+// fp32 products on the bf16 tensor cores:  C[m, n] = sum_k A[m, k] * B[n, k],  A, B and C fp32, rows of A and B along k (sm_100a).
+//
+// Each operand is split exactly into three bf16 parts (high, middle, low: 8 bits each, 24 in all), and the six products whose
+// weight is above 2^-24 of the result are accumulated: l.h, h.l, m.m, m.h, h.m, h.h, smallest first. The tensor cores cut
+// off what does not fit their fp32 accumulator where the fp32 pipes round; over a long sum that is a bias (6e-7 of the result
+// at K 768, against an error of 4.6e-7 of the fp32 pipes), so an accumulator holds a slice of 128 of k only and the slices
+// are added up, rounded, in registers. Relative error of the 32 largest of 2048 sums, against 64 bits, this and the fp32 pipes:
+//   K 64: 0.8e-7 and 1.3e-7; 256: 1.2e-7 and 2.5e-7; 768: 1.2e-7 and 4.3e-7; 2048: 1.3e-7 and 7.1e-7
+// Bound by the tensor cores, six times the operations of one bf16 product: 4096 x 24576 x 768: 2505 us (library, fp32 pipes) -> 632 us
+// and 37 us for the split. Values that bf16 cannot hold (infinities, NaN, beyond 2^127) mark their row of A or B, and what marked
+// rows take part in is redone on the fp32 pipes.
+//
+// Structure: CTA pairs (cta_group::2, 256 x 256 tiles) as in encoder_gemm.cu; a tile passes through the accumulator buffers once per
+// slice. 384 threads: TMA producer, MMA issuer, TMEM owner, and eight epilogue warps that hold 128 columns of a row each.
+#include "common.cuh"
+#include "kernels.h"
+
+namespace lmsae {
+
+namespace {
+
+constexpr int FG_BM = 128, FG_BN = 256, FG_BK = 64, FG_STAGES = 6, FG_THREADS = 384;
+constexpr int FG_SLICE = 2;  // K blocks of 64 per slice
+constexpr int FG_HALF_BYTES = 128 * FG_BK * 2;
+constexpr int FG_STAGE_BYTES = 2 * FG_HALF_BYTES;  // this CTA's 128 rows of A and 128 of the 256 rows of B
+constexpr int FG_BAR_OFF = FG_STAGES * FG_STAGE_BYTES;
+constexpr int FG_SMEM = FG_BAR_OFF + (2 * FG_STAGES + 4) * 8 + 8 + 1024;
+
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+// part of A / B (0 high, 1 middle, 2 low) of the t-th product
+__device__ __forceinline__ int part_a(int t) { return (0x201100 >> (4 * (5 - t))) & 15; }
+__device__ __forceinline__ int part_b(int t) { return (0x021010 >> (4 * (5 - t))) & 15; }
+
+// dst [rows][3][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
+// then flags[0] != 0.
+__global__ void __launch_bounds__(256)
+split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
+    const float* s = src + (size_t)r * K;
+    __nv_bfloat16* o = dst + (size_t)r * 3 * kp;
+    bool bad = false;
+    for (int c = lane * 4; c < kp; c += 128) {  // (K % 4 == 0, kp % 64 == 0)
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < K) v = __ldg(reinterpret_cast<const float4*>(s + c));
+      float x[4] = {v.x, v.y, v.z, v.w}, p[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if ((__float_as_uint(x[i]) & 0x7fffffffu) >= 0x7f000000u) { bad = true; x[i] = 0.0f; }
+        p[0][i] = __bfloat162float(__float2bfloat16(x[i]));
+        const float r1 = x[i] - p[0][i];
+        p[1][i] = __bfloat162float(__float2bfloat16(r1));
+        p[2][i] = r1 - p[1][i];
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint2*>(o + q * kp + c) = make_uint2(pack_bf16x2(p[q][0], p[q][1]), pack_bf16x2(p[q][2], p[q][3]));
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+      flags[1 + r] = bad ? 1 : 0;
+      if (bad) flags[0] = 1;
+    }
+  }
+}
+
+struct Fp32GemmParams {
+  int M, N, kp;
+  int m_tiles, n_tiles, pairs;
+  float* C;
+  int* status;
+};
+
+__global__ void __launch_bounds__(FG_THREADS, 1)
+fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Fp32GemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + FG_BAR_OFF);
+  uint64_t* empty_bar = full_bar + FG_STAGES;
+  uint64_t* tmem_full_bar = empty_bar + FG_STAGES;
+  uint64_t* tmem_empty_bar = tmem_full_bar + 2;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t cta_rank = cluster_ctarank();
+  const bool leader = cta_rank == 0;
+  const int pair = (int)(blockIdx.x >> 1);
+  const int tiles = p.m_tiles * p.n_tiles, k_blocks = p.kp / FG_BK, slices = (k_blocks + FG_SLICE - 1) / FG_SLICE;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < FG_STAGES; ++i) {
+      mbar_init(&full_bar[i], 1);
+      mbar_init(&empty_bar[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tmem_full_bar[i], 1);
+      mbar_init(&tmem_empty_bar[i], 16);  // the epilogue warps of both CTAs
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&tmap_a);
+    prefetch_tensormap(&tmap_b);
+  }
+  if (warp == 2) {
+    tmem_alloc_pair(tmem_ptr_smem, 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer's barriers exist before anything signals them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += p.pairs) {
+        // (pairs that run together work on neighbouring row panels of the same columns)
+        const int m0 = (t % p.m_tiles) * 2 * FG_BM + (int)cta_rank * FG_BM, n0 = (t / p.m_tiles) * FG_BN + (int)cta_rank * FG_BM;
+        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += FG_SLICE) {
+          const int n_kb = min(FG_SLICE, k_blocks - kb0);
+          for (int j = 0; j < 6 * n_kb; ++j, ++it) {
+            const int term = j / n_kb, kx = (kb0 + j % n_kb) * FG_BK;
+            const int s = it % FG_STAGES;
+            if (!mbar_wait_bounded(&empty_bar[s], ((it / FG_STAGES) & 1) ^ 1, abort_flag)) {
+              report_status(p.status, kTimeoutEmptyBarrier, (int)it);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            uint8_t* dst = smem + s * FG_STAGE_BYTES;
+            if (leader) mbar_arrive_expect_tx(&full_bar[s], 2 * FG_STAGE_BYTES);
+            const uint32_t bar = mapa_u32(smem_u32(&full_bar[s]), 0);
+            tma_load_2d_pair(dst, &tmap_a, bar, part_a(term) * p.kp + kx, m0);
+            tma_load_2d_pair(dst + FG_HALF_BYTES, &tmap_b, bar, part_b(term) * p.kp + kx, n0);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (leader && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(2 * FG_BM, FG_BN);
+      uint32_t it = 0, sub = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += p.pairs) {
+        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += FG_SLICE, ++sub) {
+          const int buf = sub & 1;
+          if (!mbar_wait_bounded(&tmem_empty_bar[buf], ((sub >> 1) & 1) ^ 1, abort_flag)) {
+            report_status(p.status, kTimeoutTmemEmpty, (int)sub);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t tmem_d = tmem_base + (uint32_t)(buf * FG_BN);
+          const int steps = 6 * min(FG_SLICE, k_blocks - kb0);
+          for (int j = 0; j < steps; ++j, ++it) {
+            const int s = it % FG_STAGES;
+            if (!mbar_wait_bounded(&full_bar[s], (it / FG_STAGES) & 1, abort_flag)) {
+              report_status(p.status, kTimeoutFullBarrier, (int)it);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + s * FG_STAGE_BYTES);
+            const uint64_t a_desc = make_sw128_kmajor_desc(a_addr), b_desc = make_sw128_kmajor_desc(a_addr + FG_HALF_BYTES);
+#pragma unroll
+            for (int kk = 0; kk < FG_BK / 16; ++kk)
+              umma_bf16_ss_pair(tmem_d, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2), idesc, (j > 0 || kk > 0) ? 1u : 0u);
+            umma_commit_pair(&empty_bar[s], 3);
+          }
+          if (ok) umma_commit_pair(&tmem_full_bar[buf], 3);
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter, column half
+    const bool vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    uint32_t sub = 0;
+    bool ok = true;
+    for (int t = pair; t < tiles && ok; t += p.pairs) {
+      const int row = (t % p.m_tiles) * 2 * FG_BM + (int)cta_rank * FG_BM + q * 32 + lane;
+      const int c0 = (t / p.m_tiles) * FG_BN + half * 128;
+      float acc[128];
+#pragma unroll
+      for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
+      for (int s = 0; s < slices; ++s, ++sub) {
+        const int buf = sub & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], (sub >> 1) & 1, abort_flag))) {
+          if (lane == 0) report_status(p.status, kTimeoutTmemFull, (int)sub);
+          *abort_flag = 1;
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * FG_BN + half * 128);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(taddr + (uint32_t)(g * 16), r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[g * 16 + j] += __uint_as_float(r[j]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
+      }
+      if (ok && row < p.M) {
+        float* dst = p.C + (size_t)row * p.N + c0;
+        if (vec) {
+#pragma unroll
+          for (int j = 0; j < 128; j += 4)
+            if (c0 + j < p.N) *reinterpret_cast<float4*>(dst + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 128; ++j)
+            if (c0 + j < p.N) dst[j] = acc[j];
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    // let copies that may still be in flight land before shared memory and TMEM go away
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  cluster_sync_all();  // neither CTA may free TMEM or leave while the other can still touch its barriers or accumulators
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+// C[m, n] of marked rows of A or of B on the fp32 pipes, a warp per element; leaves at once where nothing is marked.
+__global__ void __launch_bounds__(256)
+marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B, int M, int N, int K, const int* __restrict__ fa,
+                       const int* __restrict__ fb, float* __restrict__ C) {
+  if (fa[0] == 0 && fb[0] == 0) return;
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * 8;
+  for (long long e = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); e < (long long)M * N; e += warps) {
+    const int m = (int)(e / N), n = (int)(e - (long long)m * N);
+    if (fa[1 + m] == 0 && fb[1 + n] == 0) continue;
+    float s = 0.0f;
+    for (int k = lane; k < K; k += 32) s = fmaf(A[(size_t)m * K + k], B[(size_t)n * K + k], s);
+    s = warp_sum(s);
+    if (lane == 0) C[e] = s;
+  }
+}
+
+}  // namespace
+
+int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, cudaStream_t stream) {
+  if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return (int)cudaErrorInvalidValue;
+  const int blocks = (rows + 7) / 8;
+  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags);
+  return (int)cudaGetLastError();
+}
+
+int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
+                     const int* fb, float* C, int* status, cudaStream_t stream) {
+  Fp32GemmParams p;
+  p.M = M; p.N = N; p.kp = kp; p.C = C; p.status = status;
+  p.m_tiles = (M + 2 * FG_BM - 1) / (2 * FG_BM);
+  p.n_tiles = (N + FG_BN - 1) / FG_BN;
+  const long long tiles = (long long)p.m_tiles * p.n_tiles;
+  if (tiles > 2147483647LL - 148) return (int)cudaErrorInvalidValue;
+  p.pairs = (int)(tiles < 74 ? tiles : 74);
+  cudaError_t e = cudaFuncSetAttribute(fp32_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * p.pairs);
+  cfg.blockDim = dim3(FG_THREADS);
+  cfg.dynamicSmemBytes = FG_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, fp32_gemm_kernel, ta, tb, p);
+  if (e != cudaSuccess) return (int)e;
+  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C);
+  return (int)cudaGetLastError();
+}
+
+}  // namespace lmsae
