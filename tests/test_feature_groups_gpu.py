@@ -1,0 +1,26 @@
+"""Grouping codes by feature around the limits of the one-CTA kernel, with empty slots and features of every token."""
+
+import pytest
+import torch
+
+from language_model_saes_b200.ops import sae_kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,k,F", [(1, 1, 1), (37, 3, 5), (512, 8, 256), (512, 16, 4097), (512, 16, 8192), (512, 16, 8193), (513, 16, 100), (1024, 32, 4096)])
+def test_groups(B, k, F):
+    g = torch.Generator().manual_seed(B + F)
+    idx = torch.randint(-1, F, (B, k), generator=g).to(torch.int32)
+    idx[:, 0] = F // 2
+    groups = K.FeatureGroups(F, idx.numel(), torch.device("cuda"))
+    for _ in range(2):  # (buffers are used again)
+        groups.build(idx.cuda())
+        counts = torch.bincount(idx[idx >= 0].long(), minlength=F)
+        off = groups.offsets.cpu()
+        assert torch.equal(groups.counts.cpu().long(), counts) and torch.equal(off.long(), torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+        e = groups.entries.cpu()[: int(off[-1])].long()
+        assert torch.equal(idx.reshape(-1)[e], torch.repeat_interleave(torch.arange(F, dtype=torch.int32), counts)) and e.unique().numel() == e.numel()
+        heavy = groups.heavy.cpu()
+        want = torch.nonzero(counts > K.HEAVY_ROW).flatten()
+        assert int(heavy[0]) == want.numel() and torch.equal(heavy[1 : 1 + want.numel()].sort().values.long(), want)
