@@ -411,7 +411,7 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 // With x and W, h is only an estimate of x . W^T (fp32_gemm.cu: off by some 1e-6 of the scale of its terms, in which it is as good
 // as a sum in order): what is selected, and the selected values, are those of the fp32 sum in ascending order of k, as the fp32
 // product it replaces gives them, bit for bit. The bound is lowered by 2^-8, a thousand times the error of either sum, and
-// the few columns above it are summed up in order before the exact selection (319 -> 536 us; the product: 2505 -> 670 us). Rows for which that would not be sound (fewer than k
+// the few columns above it are summed up in order before the exact selection (319 -> 508 us; the product: 2505 -> 670 us). Rows for which that would not be sound (fewer than k
 // positive values, something not finite, too many columns at the bound) are summed up in order as a whole.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned topk_key(float g) {
@@ -555,7 +555,8 @@ restart:
       sum_row_in_order();
       goto restart;
     }
-    for (int j = threadIdx.x; j < n; j += RT_THREADS) {
+    // (neighbouring candidates to different warps: a few dozen of them in one or two warps wait for their rows of W alone, 536 us)
+    for (int j = (threadIdx.x & 31) * RT_WARPS + (threadIdx.x >> 5); j < n; j += RT_THREADS) {
       const int c = s_col[j];
       float g = dot_in_order(x, p.W + (size_t)c * p.K, p.K);
       if (p.bias != nullptr) g = __fadd_rn(g, p.bias[c]);
