@@ -33,13 +33,15 @@ jumprelu_lists_kernel(const JumpReluListParams p) {
     float ds = 0.0f, dth = 0.0f;
     for (int h = 0; h < p.H; ++h) {
       const float nh = p.norm[(size_t)h * p.F + f];
-      const bool active = s > th / nh;
+      const bool active = s > __fdiv_rn(th, nh);  // (the quotient that the lists were selected against)
       p.act[(size_t)h * n + i] = active ? s : 0.0f;
       if (!active || p.coef == 0.0f) continue;
       const float x = s * nh;
-      const float u = tanhf(p.stretch * x);
-      const float sech2 = 1.0f - u * u;
-      u_sum += u;
+      // in 64 bits: 1 - tanh^2 cancels, and the fast fp32 tanh that this file's flags select is a dozen times further off than
+      // tanh rounded to fp32 (1e-4 of sech^2 at x = 3 against 8e-6)
+      const double u = tanh((double)(p.stretch * x));
+      const float sech2 = (float)(1.0 - u * u);
+      u_sum += (float)u;
       ds += p.coef * nh * sech2;
       atomicAdd(p.pull + (size_t)h * p.F + f, p.coef * s * sech2);
       if (fabsf(x - th) < 0.5f * p.window) dth += p.coef * (sech2 - 1.0f) * (-th / p.window);
