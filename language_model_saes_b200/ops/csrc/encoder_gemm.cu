@@ -522,6 +522,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     if constexpr (TOPK) if (ok && row_ok) {
       // emit this sweep's candidates (at least the k best, at most KS): [row][split * KS + slot]
       const long long o = (long long)row * ((long long)p.num_splits * KS) + (long long)split * KS;
+      const bool whole = ((reinterpret_cast<uintptr_t>(p.cand_val) | reinterpret_cast<uintptr_t>(p.cand_idx)) & 15) == 0;  // (lists may be views)
       for (int s = 0; s < KS; s += 4) {
         float v[4];
         int ix[4];
@@ -533,8 +534,16 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           // (an entry carried over from slot c sits at or before slot c: its column there is not overwritten yet)
           if (NARROW && valid) ix[i] = ix[i] >= kCarried ? p.cand_idx[o + ix[i] - kCarried] : ix[i] + col_base;
         }
-        *reinterpret_cast<float4*>(p.cand_val + o + s) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<int4*>(p.cand_idx + o + s) = make_int4(ix[0], ix[1], ix[2], ix[3]);
+        if (whole) {
+          *reinterpret_cast<float4*>(p.cand_val + o + s) = make_float4(v[0], v[1], v[2], v[3]);
+          *reinterpret_cast<int4*>(p.cand_idx + o + s) = make_int4(ix[0], ix[1], ix[2], ix[3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            p.cand_val[o + s + i] = v[i];
+            p.cand_idx[o + s + i] = ix[i];
+          }
+        }
       }
       // a panel with fewer ranges than the lists have room for: its last range also marks the unused lists empty
       if (split == my_splits - 1) {

@@ -59,9 +59,14 @@ sparse_decode_kernel(const DecodeParams p, int nseg) {
       if (!in[u]) continue;
       const int c = v[u] * 8;
       if (p.bias != nullptr) {
-        const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.bias + c)), b1 = __ldg(reinterpret_cast<const float4*>(p.bias + c) + 1);
-        acc[u][0] += b0.x; acc[u][1] += b0.y; acc[u][2] += b0.z; acc[u][3] += b0.w;
-        acc[u][4] += b1.x; acc[u][5] += b1.y; acc[u][6] += b1.z; acc[u][7] += b1.w;
+        if ((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+          const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.bias + c)), b1 = __ldg(reinterpret_cast<const float4*>(p.bias + c) + 1);
+          acc[u][0] += b0.x; acc[u][1] += b0.y; acc[u][2] += b0.z; acc[u][3] += b0.w;
+          acc[u][4] += b1.x; acc[u][5] += b1.y; acc[u][6] += b1.z; acc[u][7] += b1.w;
+        } else {  // (a piece of a longer parameter vector starts anywhere)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[u][i] += __ldg(p.bias + c + i);
+        }
       }
       if (p.xhat_f32 != nullptr) {
         float4* o = reinterpret_cast<float4*>(p.xhat_f32 + (size_t)row * p.d + c);
