@@ -426,7 +426,8 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
                       const c10::optional<Tensor>& extra_gD, const c10::optional<Tensor>& extra_gE,
                       const c10::optional<Tensor>& extra_gb, const c10::optional<Tensor>& wd_self_scale,
                       const c10::optional<Tensor>& norm_sq_accum, int64_t dact_mode, const c10::optional<Tensor>& heavy,
-                      int64_t heavy_base, const c10::optional<Tensor>& sched) {
+                      int64_t heavy_base, const c10::optional<Tensor>& sched, int64_t wait_cycles) {
+  // (wait_cycles < 0: the kernels' usual limit)
   // one-sided launches: the decoder group (WD, mD, vD, WD_bf16) or the encoder group (WE, mE, vE, WE_bf16) may be absent
   const bool has_d = WD_o.has_value(), has_e = WE_o.has_value();
   TORCH_CHECK(has_d || has_e, "at least one of the decoder / encoder groups must be given");
@@ -503,6 +504,7 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
   p.heavy_base = (int)heavy_base;
   if (sched.has_value()) { CHECK_T(*sched, torch::kInt32); TORCH_CHECK(sched->numel() >= 2); }
   p.sched = opt_ptr<int>(sched);
+  p.wait_cycles = wait_cycles;
   if (status.has_value()) { CHECK_T(*status, torch::kInt32); }
   p.status = opt_ptr<const int>(status);
   if (wd_self_scale.has_value()) { CHECK_T(*wd_self_scale, torch::kFloat32); TORCH_CHECK(wd_self_scale->numel() == p.F); }

@@ -128,7 +128,8 @@ constexpr long long kWaitBudgetCycles = 3000000000LL;
 
 // Bounded wait. Returns true when the phase completed, false when the budget ran out or another
 // role of this CTA already aborted (abort_flag != 0).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  long long budget_cycles = kWaitBudgetCycles) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
@@ -136,7 +137,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 0x3ff) == 0) {
       if (abort_flag != nullptr && *abort_flag != 0) return false;
-      if (clock64() - t0 > kWaitBudgetCycles) return false;
+      if (clock64() - t0 > budget_cycles) return false;
     }
   }
 }

@@ -49,6 +49,28 @@ __device__ __forceinline__ void group_sync(int gid) {
   }
 }
 
+// Whether all threads of the group say so (a barrier of the group).
+template <int W>
+__device__ __forceinline__ bool group_all(int gid, bool ok) {
+  if constexpr (W == 1) {
+    return __all_sync(0xffffffffu, ok);
+  } else {
+    uint32_t r;
+    __syncwarp();
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %3, 0;\n\t"
+        "barrier.cta.red.and.pred p, %1, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(r)
+        : "r"(gid + 1), "n"(W * 32), "r"((uint32_t)ok)
+        : "memory");
+    return r != 0;
+  }
+}
+
 struct AdamConst {
   float b1, b2, c1, c2, inv_bc2, step, eps;
 };
@@ -180,7 +202,7 @@ __device__ __forceinline__ void round_row(const float* row, int d, const GroupCt
 // the new decoder row's squared norm.
 template <bool IS_D, int W, int NCH>
 __device__ __forceinline__ float apply_side(const GradAdamParams& p, const GroupCtx& c, int f, float gmul, const AdamConst& h,
-                                            float (&g)[NCH][4], float& gsq, bool ok) {
+                                            float (&g)[NCH][4], float& gsq) {
   float* Wp = IS_D ? p.WD : p.WE;
   float* Mp = IS_D ? p.mD : p.mE;
   float* Vp = IS_D ? p.vD : p.vE;
@@ -195,7 +217,7 @@ __device__ __forceinline__ float apply_side(const GradAdamParams& p, const Group
 #pragma unroll
     for (int q = 0; q < 4; ++q) g[i][q] *= gmul;
     if (p.grad_sq_sum != nullptr) gsq += g[i][0] * g[i][0] + g[i][1] * g[i][1] + g[i][2] * g[i][2] + g[i][3] * g[i][3];
-    if (!p.update || !ok) continue;
+    if (!p.update) continue;
     float4 w = *reinterpret_cast<const float4*>(c.stage + col);
     float4 m = *reinterpret_cast<const float4*>(c.stage + p.d + col);
     float4 v = *reinterpret_cast<const float4*>(c.stage + 2 * p.d + col);
@@ -265,9 +287,11 @@ grad_adam_rows_kernel(const GradAdamParams p) {
   uint32_t parity = 0;  // of this group's barrier
   int red_buf = 0;
 
+  bool outstanding = false;  // (one thread of the group) copies were issued and their arrival has not been seen
   auto issue = [&](int gid, bool is_d, int f) {  // one thread
     const int n = is_d ? loadsD : loadsE;
     if (n == 0) return;
+    outstanding = true;
     uint64_t* bar = &bars[gid];
     float* dst = stages + (size_t)gid * 3 * p.d;
     mbar_arrive_expect_tx(bar, row_bytes * n);
@@ -278,14 +302,16 @@ grad_adam_rows_kernel(const GradAdamParams p) {
       bulk_load(dst + 2 * p.d, (is_d ? p.vD : p.vE) + os, row_bytes, bar);
     }
   };
-  bool ok = true;  // false once a wait ran out: nothing is stored from then on, but the group keeps its barriers in step
-  auto wait_full = [&](int gid, uint32_t par) {
-    if (ok && !mbar_wait_bounded(&bars[gid], par, abort_flag)) {
-      if (c.lane == 0) report_status(const_cast<int*>(p.status), kTimeoutFullBarrier, gid);
-      *abort_flag = 1;
-      ok = false;
-    }
+  // Whether this thread has seen the copies arrive. Every caller takes a vote of all threads that share the row before anything that
+  // depends on it is stored, and a group that failed draws no further rows: nothing of the side it waited for has changed then, the
+  // other groups finish theirs, and the status word says that the update is incomplete.
+  auto arrived = [&](int gid, uint32_t par) -> bool {
+    if (p.wait_cycles > 0 && mbar_wait_bounded(&bars[gid], par, abort_flag, p.wait_cycles)) return true;
+    if (c.lane == 0) report_status(const_cast<int*>(p.status), kTimeoutFullBarrier, gid);
+    *abort_flag = 1;
+    return false;
   };
+  bool failed = false;
   auto init_grad = [&](bool is_d, int xr, float (&g)[NCH][4]) {
     const float* ex = is_d ? p.extra_gD : p.extra_gE;
 #pragma unroll
@@ -317,7 +343,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
   if (heavy_on && !skip) {
     const int n_heavy = p.heavy[0];
     uint32_t par0 = 0;
-    for (int hi = blockIdx.x; hi < n_heavy; hi += gridDim.x) {
+    for (int hi = blockIdx.x; hi < n_heavy && !failed; hi += gridDim.x) {
       const int f = p.heavy[1 + hi] - p.heavy_base;
       if (f < p.f_begin || f >= p.f_end) continue;
       const int e0 = p.offsets[f], e1 = p.offsets[f + 1];
@@ -329,11 +355,11 @@ grad_adam_rows_kernel(const GradAdamParams p) {
         float g[NCH][4];
         init_grad(is_d, c.gid == 0 ? xr : -1, g);
         float coef = 0.0f;
-        bool waited = false;
+        bool seen = true;
         if (is_d) {
           if (dot_mode) {
-            wait_full(0, par0);
-            waited = true;
+            failed = !__syncthreads_and(arrived(0, par0));
+            if (failed) break;
             round_row<W, NCH>(stages, p.d, c);
             gather_side<true, true, W, NCH>(p, c, e0, e1, c.gid, G, g);
           } else {
@@ -353,8 +379,15 @@ grad_adam_rows_kernel(const GradAdamParams p) {
             if (col < p.d) *reinterpret_cast<float4*>(c.stage + col) = make_float4(g[i][0], g[i][1], g[i][2], g[i][3]);
           }
           fence_proxy_async();  // a bulk copy writes here later
+        } else if ((is_d ? loadsD : loadsE) != 0 && !(is_d && dot_mode)) {
+          seen = arrived(0, par0);
         }
-        __syncthreads();
+        failed = !__syncthreads_and(seen);  // (also: the partial rows are in place)
+        if (failed) break;
+        if ((is_d ? loadsD : loadsE) != 0) {
+          par0 ^= 1;
+          if (c.gid == 0) outstanding = false;
+        }
         if (c.gid == 0) {
           for (int q = 1; q < G; ++q) {
             const float* part = stages + (size_t)q * 3 * p.d;
@@ -368,13 +401,9 @@ grad_adam_rows_kernel(const GradAdamParams p) {
             }
           }
         }
-        if (c.gid == 0 && (is_d ? loadsD : loadsE) != 0) {
-          if (!waited) wait_full(0, par0);
-        }
-        if ((is_d ? loadsD : loadsE) != 0) par0 ^= 1;
         if (c.gid == 0) {
           if (is_d) {
-            float ns = apply_side<true, W, NCH>(p, c, f, gmul, h, g, gsq, ok);
+            float ns = apply_side<true, W, NCH>(p, c, f, gmul, h, g, gsq);
             ns = warp_sum(ns);
             if (c.lane == 0) red[c.wg] = ns;
             group_sync<W>(0);
@@ -384,7 +413,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
               put_norm(f, t);
             }
           } else {
-            apply_side<false, W, NCH>(p, c, f, gmul, h, g, gsq, ok);
+            apply_side<false, W, NCH>(p, c, f, gmul, h, g, gsq);
             if (c.tid == 0) {
               float b = 0.0f;
               for (int q = 0; q < G; ++q) b += bias_part[q];
@@ -432,7 +461,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
     return f;
   };
 
-  if (!skip) {
+  if (!skip && !failed) {
     int e0 = 0, e1 = 0;
     int f = next_light(e0, e1);
     if (f < p.f_end && c.tid == 0) issue(c.gid, doD, f);
@@ -443,10 +472,9 @@ grad_adam_rows_kernel(const GradAdamParams p) {
       if (doD) {
         float g[NCH][4];
         init_grad(true, xr, g);
-        bool waited = false;
         if (dot_mode) {
-          wait_full(c.gid, parity);
-          waited = true;
+          failed = !group_all<W>(c.gid, arrived(c.gid, parity));
+          if (failed) break;
           if (e1 > e0) {
             round_row<W, NCH>(c.stage, p.d, c);
             gather_side<true, true, W, NCH>(p, c, e0, e1, 0, 1, g);
@@ -455,10 +483,14 @@ grad_adam_rows_kernel(const GradAdamParams p) {
           gather_side<true, false, W, NCH>(p, c, e0, e1, 0, 1, g);
         }
         if (loadsD != 0) {
-          if (!waited) wait_full(c.gid, parity);
+          if (!dot_mode) {
+            failed = !group_all<W>(c.gid, arrived(c.gid, parity));
+            if (failed) break;
+          }
           parity ^= 1;
+          outstanding = false;
         }
-        float ns = apply_side<true, W, NCH>(p, c, f, gmul, h, g, gsq, ok);
+        float ns = apply_side<true, W, NCH>(p, c, f, gmul, h, g, gsq);
         if (p.dec_norm != nullptr || p.norm_sq_accum != nullptr) ns = warp_sum(ns);
         float* rb = red + (red_buf * G + c.gid) * W;
         red_buf ^= 1;
@@ -482,10 +514,12 @@ grad_adam_rows_kernel(const GradAdamParams p) {
         init_grad(false, xr, g);
         float coef = gather_side<false, false, W, NCH>(p, c, e0, e1, 0, 1, g);
         if (loadsE != 0) {
-          wait_full(c.gid, parity);
+          failed = !group_all<W>(c.gid, arrived(c.gid, parity));
+          if (failed) break;
           parity ^= 1;
+          outstanding = false;
         }
-        apply_side<false, W, NCH>(p, c, f, gmul, h, g, gsq, ok);
+        apply_side<false, W, NCH>(p, c, f, gmul, h, g, gsq);
         group_sync<W>(c.gid);
         if (c.tid == 0 && fn < p.f_end) issue(c.gid, doD, fn);
         if (c.wg == 0) {
@@ -502,10 +536,9 @@ grad_adam_rows_kernel(const GradAdamParams p) {
     gsq = warp_sum(gsq);
     if (c.lane == 0 && gsq != 0.0f) atomicAdd(p.grad_sq_sum, gsq);
   }
+  // copies that nobody waited for land before the shared memory goes away
+  if (failed && c.tid == 0 && outstanding) mbar_wait_bounded(&bars[c.gid], parity, nullptr);
   __syncthreads();
-  if (*abort_flag != 0) {  // let copies that may still be in flight land before the shared memory goes away
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
-  }
   if (threadIdx.x == 0 && p.sched != nullptr) {
     // the last CTA leaves the counters at zero for the next launch (every CTA has drawn its last row by then)
     __threadfence();
@@ -531,6 +564,7 @@ cudaError_t launch_rows(GradAdamParams p, cudaStream_t stream) {
   const int blocks = rows < 148 ? rows : 148;  // (groups without a row of their own still share the long lists)
   // rows per draw: one at the end of the range for balance, a few where rows are short and plentiful (draws are atomics on one word)
   int chunk = rows / (blocks * G * 16);
+  if (p.wait_cycles < 0) p.wait_cycles = kWaitBudgetCycles;
   p.sched_chunk = chunk < 1 ? 1 : (chunk > 8 ? 8 : chunk);
   const size_t smem = (size_t)G * per_group + 64;
   auto kern = grad_adam_rows_kernel<W, NCH>;

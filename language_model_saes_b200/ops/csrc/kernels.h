@@ -163,6 +163,7 @@ struct GradAdamParams {
   int heavy_base;
   int* sched;        // two zero-initialised ints that the kernel leaves at zero: row counter, finished CTAs (nullptr: static deal)
   int sched_chunk;   // set by the launch
+  long long wait_cycles;  // how long a row's copies are waited for (row-streaming kernel); < 0: the usual limit, 0: not at all
   float* gD_out;  // optional dense [F, d] outputs of the rebuilt gradient rows (for autograd callers)
   float* gE_out;
   // Optimizer state sharded by feature row over data-parallel replicas: this launch owns rows [f_begin, f_end); its

@@ -573,6 +573,7 @@ def sparse_grad_adam(
     wd_self_scale: torch.Tensor | None = None,
     norm_sq_accum: torch.Tensor | None = None,
     dact_mode: int = 0,
+    wait_cycles: int = -1,
 ):
     """Rebuild the two sparse gradient rows per feature and apply Adam in the same pass (in place). ``f_range``
     restricts the launch to feature rows ``[begin, end)``. With ``dxhat_aux`` the code slots ``>= k_main`` of every row
@@ -587,7 +588,8 @@ def sparse_grad_adam(
     new decoder row is ADDED there instead of writing ``dec_norm``. ``dact_mode``: 0 takes ``dact`` as given; 1 computes it
     first (``d x_hat[token] . bf16(W_D row)`` with the row as it was before the update; 0 where the code is 0) and leaves it in
     ``dact``, 2 adds to what ``dact`` holds (one launch per decoder matrix); the decoder group must be given then. A non-zero kernel status word turns the update into
-    a no-op (CUDA path)."""
+    a no-op (CUDA path). Where a row's copies do not arrive within ``wait_cycles`` clocks (< 0: one to two seconds) that row and those
+    its group would have taken stay as they are, the others are updated, and the status word says so."""
     ref_w = WD if WD is not None else WE
     if not ref_w.is_cuda:
         if dact_mode:
@@ -663,7 +665,7 @@ def sparse_grad_adam(
         dec_norm, grad_mul, grad_sq_sum, lr, beta1, beta2, eps, step, update, *(f_range if f_range is not None else (0, -1)), ctas_per_sm, dxhat_aux, k_main, grad_out[0], grad_out[1],
         status_buffer(ref_w.device), state_f0, *(publish if publish is not None else ([], [], 0, None)),
         *(extra if extra is not None else (None, None, None, None)), wd_self_scale, norm_sq_accum, dact_mode, groups.heavy,
-        groups.heavy_base, groups.sched,
+        groups.heavy_base, groups.sched, wait_cycles,
     )  # fmt: skip
 
 

@@ -834,7 +834,8 @@ class Trainer:
         """Before parameters are written out or handed to other code on the fused path: fold the update stream back,
         raise if a kernel recorded an error (a timed-out collective leaves the step's data unusable; the update kernels
         skip themselves after one, so the parameters are those of the last good step, but nothing more must be saved as
-        if training had gone on), and gather the master rows that other replicas own."""
+        if training had gone on; a wait that ran out in the update itself leaves some rows updated and others not: the
+        parameters are to be discarded then), and gather the master rows that other replicas own."""
         if self.fused is None:
             return
         self.fused.join()

@@ -79,3 +79,28 @@ def test_gradient_pass_without_an_update_leaves_code_gradients_and_norm_only():
                            t["b"], t["mb"], t["vb"], t["n"], None, t["gsq"], 1e-3, 0.9, 0.999, 1e-8, 1, False, dact_mode=1)  # fmt: skip
     _compare(cpu, gpu, ["dact", "WD", "mD", "WE", "vE", "b", "n"], 260)
     assert torch.allclose(gpu["gsq"].cpu(), cpu["gsq"], rtol=1e-3)
+
+
+@pytest.mark.parametrize("d", [768, 1160, 4100])
+@pytest.mark.parametrize("sides,mode", [("both", 0), ("both", 1), ("decoder", 2), ("encoder", 0)])
+def test_rows_whose_copies_were_not_waited_for_stay_as_they_are(d, sides, mode):
+    cpu = _case(d, 230, 200, 6, seed=d)
+    t = {n: v.clone().to(DEV) for n, v in cpu.items()}
+    groups = K.FeatureGroups(230, 1200, t["idx"].device).build(t["idx"])
+    D = [t["WD"], t["mD"], t["vD"], t["WD16"]] if sides != "encoder" else [None] * 4
+    E = [t["WE"], t["mE"], t["vE"], t["WE16"], t["b"], t["mb"], t["vb"]] if sides != "decoder" else [None] * 7
+
+    def run(**kw):
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], *D, *E, t["n"] if sides == "both" else None, None, None, 1e-3, 0.9, 0.999,
+                           1e-8, 1, True, norm_sq_accum=t["acc"] if sides == "decoder" else None, dact_mode=mode, **kw)  # fmt: skip
+
+    K.check_status(torch.device(DEV))
+    run(wait_cycles=0)
+    with pytest.raises(K.KernelStatusError):
+        K.check_status(torch.device(DEV))
+    for n in cpu:
+        assert torch.equal(t[n].cpu(), cpu[n]), n
+    assert groups.sched.tolist() == [0, 0]
+    run()  # the next launch works as ever
+    K.check_status(torch.device(DEV))
+    assert not torch.equal((t["WD"] if sides != "encoder" else t["WE"]).cpu(), cpu["WD"] if sides != "encoder" else cpu["WE"])
