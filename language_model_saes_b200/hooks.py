@@ -53,6 +53,15 @@ class HookPoint(nn.Module):
     def clear_context(self) -> None:
         self.ctx = {}
 
+    def is_silent(self) -> bool:
+        """Whether a tensor that passes through comes out as it went in, unseen: no hook of this point and none of PyTorch's own, be
+        it on this module or on all, and the call defined here."""
+        own = (self.fwd_hooks, self.bwd_hooks, self._forward_hooks, self._forward_pre_hooks, self._backward_hooks, self._backward_pre_hooks)
+        if type(self) is not HookPoint or "forward" in self.__dict__ or any(own):
+            return False
+        M = torch.nn.modules.module
+        return not any((M._global_forward_hooks, M._global_forward_pre_hooks, M._global_backward_hooks, M._global_backward_pre_hooks))
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         for fn, _ in self.fwd_hooks:
             out = fn(x, hook=self)

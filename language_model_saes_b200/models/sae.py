@@ -173,9 +173,12 @@ class SparseAutoEncoder(SparseDictionary):
 
     def _rowwise_topk_inference(self, x: torch.Tensor) -> bool:
         """A plain forward pass of a TopK encoder that nothing listens to between its operations."""
-        if not x.is_cuda or self.cfg.use_glu_encoder or type(self.current_k) is not int or not getattr(self.activation_function, "rowwise_topk", False):
+        # (the type first: a tracer's stand-in for a tensor has no answers)
+        if type(x) not in (torch.Tensor, nn.Parameter) or torch.compiler.is_compiling() or not x.is_cuda:
             return False
-        if any(hp.fwd_hooks or hp.bwd_hooks for hp in (self.hook_hidden_pre, self.hook_feature_acts)):
+        if self.cfg.use_glu_encoder or type(self.current_k) is not int or not getattr(self.activation_function, "rowwise_topk", False):
+            return False
+        if not all(isinstance(hp, HookPoint) and hp.is_silent() for hp in (self.hook_hidden_pre, self.hook_feature_acts)):
             return False
         from ..ops.inference import plain_inference
 
@@ -183,7 +186,9 @@ class SparseAutoEncoder(SparseDictionary):
 
     def _sparse_inference(self, feature_acts: torch.Tensor) -> bool:
         """A plain fp32 forward pass of a decoder whose activation function leaves few features active."""
-        if not feature_acts.is_cuda or self.cfg.act_fn.lower() not in ("topk", "batchtopk", "jumprelu"):
+        if type(feature_acts) not in (torch.Tensor, nn.Parameter) or torch.compiler.is_compiling() or not feature_acts.is_cuda:
+            return False
+        if self.cfg.act_fn.lower() not in ("topk", "batchtopk", "jumprelu"):
             return False
         from ..ops.inference import plain_inference, sparse_decode_supported
 
