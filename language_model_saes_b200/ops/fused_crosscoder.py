@@ -209,7 +209,7 @@ class FusedCrosscoderStep:
         if self.head_size > 1:
             dist.all_reduce(t_min, op=dist.ReduceOp.MIN, group=self.head_group)
         idx, s_val = S.column_threshold_rows_to_sparse(S_sum, t_min, cap, overflow=self.list_overflow)
-        if x.is_cuda and self.tp == 1 and self.dp == 1 and not quad:
+        if self.tp == 1 and self.dp == 1 and not quad:
             return self._step_on_lists(x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, float(tanh_stretch), lp_coefficient)
         safe = idx.clamp_min(0).long()
         valid = idx >= 0
@@ -370,7 +370,7 @@ class FusedCrosscoderStep:
         return lp, c_lp * (gap * n_local).sum() * H / H_l
 
     def _step_on_lists(self, x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, c, lp_coefficient) -> torch.Tensor:
-        """The step from the shared lists on, one process per head group on a GPU: one kernel derives every head's codes and the
+        """The step from the shared lists on, one process per head group: one kernel derives every head's codes and the
         penalty's terms from the lists; per head decode + loss, then the decoder side of the update, which adds the head's
         code gradients to the shared sum's gradient on its way; the encoder sides follow once that sum is complete."""
         B, H_l, d = x.shape
@@ -385,7 +385,7 @@ class FusedCrosscoderStep:
         if lp_coefficient:
             lp, l_p_sum = self._lp_terms(S_sum, theta, lp_coefficient, dtheta)
         coef = l1_coefficient * c / (B * H) if l1_coefficient else 0.0
-        K._ext().jumprelu_lists(idx, s_val, self.dec_norm, theta, c, coef, self.window, act, dS, pull, dtheta, u_sum, n_valid)
+        K.jumprelu_lists(idx, s_val, self.dec_norm, theta, c, coef, self.window, act, dS, pull, dtheta, u_sum, n_valid)
         if self.groups is None or self.groups.entries.numel() < idx.numel():
             self.groups = K.FeatureGroups(F, idx.numel(), dev)
         self.groups.build(idx)

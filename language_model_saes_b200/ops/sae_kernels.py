@@ -669,6 +669,35 @@ def sparse_grad_adam(
     )  # fmt: skip
 
 
+def jumprelu_lists(idx, s_val, norm, theta, stretch: float, coef: float, window: float, act, dS, pull, dtheta, u_sum, n_valid) -> None:
+    """Codes of every head (``act [H, B, cap]``: the summed pre-activation where it passes ``theta / norm[h]``) and the terms of the tanh
+    penalty from the shared lists ``idx`` / ``s_val [B, cap]``: ``dS`` its derivative with respect to the sum, ``pull [H, F]`` with respect to the
+    decoder norms, ``dtheta [F]`` the correction of the threshold gradient at active entries, ``u_sum`` the sum of the tanh, ``n_valid`` the
+    number of entries. ``coef = l1 * stretch / (tokens * heads)``, 0 without the penalty. The last four are added to; empty slots of the
+    first two are left as they are."""
+    if idx.is_cuda:
+        _ext().jumprelu_lists(idx, s_val, norm, theta, stretch, coef, window, act, dS, pull, dtheta, u_sum, n_valid)
+        return
+    valid = idx >= 0
+    f, s = idx[valid].long(), s_val[valid]
+    n_valid += f.numel()
+    ds = torch.zeros_like(s)
+    for h in range(norm.shape[0]):
+        n = norm[h][f]
+        active = s > theta[f] / n
+        act[h][valid] = torch.where(active, s, 0.0)
+        if not coef:
+            continue
+        u = torch.tanh(stretch * (s * n)) * active
+        sech2 = (1.0 - u * u) * active
+        u_sum += u.sum()
+        ds += coef * n * sech2
+        pull[h].index_add_(0, f, coef * s * sech2)
+        hit = active & ((s * n - theta[f]).abs() < 0.5 * window)
+        dtheta.index_add_(0, f, torch.where(hit, coef * (sech2 - 1.0) * (-theta[f] / window), 0.0))
+    dS[valid] = ds
+
+
 def colsum_bf16(a: torch.Tensor) -> torch.Tensor:
     if not a.is_cuda:
         return a.float().sum(0)

@@ -379,6 +379,14 @@ def _heads_tanh_lp_body():
     _head_parallel_body("tanh", 2e-3)
 
 
+def _heads_tanh_on_unwritten_memory_body():
+    torch.use_deterministic_algorithms(True)  # (torch.empty gives NaN: nothing may be read that the list kernel leaves unwritten)
+    try:
+        _head_parallel_body("tanh", 0.0)
+    finally:
+        torch.use_deterministic_algorithms(False)
+
+
 def _heads_quad_body():
     _head_parallel_body("tanh-quad", 0.0)
 
@@ -387,7 +395,7 @@ def _heads_and_replicas_body():
     _head_parallel_body("tanh-quad", 0.0, dims=(2, 2, 1))
 
 
-@pytest.mark.parametrize("body", ["_heads_tanh_lp_body", "_heads_quad_body"])
+@pytest.mark.parametrize("body", ["_heads_tanh_lp_body", "_heads_tanh_on_unwritten_memory_body", "_heads_quad_body"])
 def test_fused_crosscoder_step_with_heads_over_two_ranks_matches_one_process(body):
     from language_model_saes_b200.testing import distributed_test
 
