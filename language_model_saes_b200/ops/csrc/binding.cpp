@@ -192,8 +192,10 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
              "topk_merge launch");
 }
 
-// C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu)
-void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status) {
+// C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu); na [M] and ends [2, N] (both optional): what
+// topk_estimate takes, made with its bias [N] and gate [N] (both optional)
+void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
+               const c10::optional<Tensor>& ends, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate) {
   CHECK_T(A, torch::kFloat32);
   CHECK_T(B, torch::kFloat32);
   CHECK_T(C, torch::kFloat32);
@@ -202,6 +204,11 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
               "A [M,K], B [N,K], C [M,N]");
   const int64_t M = A.size(0), N = B.size(0), K = A.size(1), kp = (K + 63) / 64 * 64;
   TORCH_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && M < INT_MAX - 256 && N < INT_MAX - 256 && 3 * kp < INT_MAX, "unsupported sizes");
+  if (na.has_value()) { CHECK_T(*na, torch::kFloat32); TORCH_CHECK(na->numel() == M); }
+  if (ends.has_value()) { CHECK_T(*ends, torch::kInt32); TORCH_CHECK(ends->numel() == 2 * N); }
+  for (const auto* t : {&bias, &gate}) {
+    if (t->has_value()) { CHECK_T(**t, torch::kFloat32); TORCH_CHECK((*t)->numel() == N); }
+  }
   const c10::cuda::CUDAGuard guard(A.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const auto b16 = A.options().dtype(torch::kBFloat16), i32 = A.options().dtype(torch::kInt32);
@@ -209,33 +216,46 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
   const Tensor flags = torch::zeros({M + N + 2}, i32);
   int* fa = flags.data_ptr<int>();
   int* fb = fa + 1 + M;
-  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, stream), "split");
-  check_cuda(lmsae::split_bf16x3_launch(B.data_ptr<float>(), (int)N, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, stream), "split");
+  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, opt_ptr<float>(na), nullptr, nullptr, nullptr, stream), "split");
+  check_cuda(lmsae::split_bf16x3_launch(B.data_ptr<float>(), (int)N, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nullptr,
+                                        reinterpret_cast<uint32_t*>(opt_ptr<int>(ends)), opt_ptr<const float>(bias), opt_ptr<const float>(gate), stream), "split");
   const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, 3 * kp, 128);
   const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), N, 3 * kp, 128);
-  check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), B.data_ptr<float>(), (int)M, (int)N, (int)K, (int)kp, fa, fb, C.data_ptr<float>(),
+  check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), B.data_ptr<float>(), (int)M, (int)N, (int)K, (int)kp, fa, fb, C.data_ptr<float>(), N,
                                      status.data_ptr<int>(), stream),
              "fp32_gemm launch");
 }
 
-// out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]; with x [B, K] and W [F, K], h is an estimate of x W^T (and may be
-// overwritten)
-void topk_dense(const Tensor& h, const c10::optional<Tensor>& x, const c10::optional<Tensor>& W, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, const Tensor& out) {
+// out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]
+void topk_dense(const Tensor& h, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, const Tensor& out) {
   CHECK_T(h, torch::kFloat32);
   CHECK_T(out, torch::kFloat32);
   TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && h.size(0) <= INT_MAX && h.size(1) <= INT_MAX, "h and out must be [B, F]");
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
   if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
-  if (x.has_value()) {
-    CHECK_T(*x, torch::kFloat32);
-    TORCH_CHECK(W.has_value() && x->dim() == 2 && x->size(0) == h.size(0), "x [B, K] and W [F, K] come together");
-    CHECK_T(*W, torch::kFloat32);
-    TORCH_CHECK(W->dim() == 2 && W->size(0) == h.size(1) && W->size(1) == x->size(1) && x->size(1) <= INT_MAX, "x [B, K] and W [F, K] come together");
-  }
   const c10::cuda::CUDAGuard guard(h.device());
-  check_cuda(lmsae::topk_dense_launch(h.data_ptr<float>(), opt_ptr<const float>(x), opt_ptr<const float>(W), x.has_value() ? (int)x->size(1) : 0, opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
+  check_cuda(lmsae::topk_dense_launch(h.data_ptr<float>(), opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
                                       (int)k, out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
              "topk_dense launch");
+}
+
+// The same with h [B, F] an estimate of x [B, K] W [F, K]^T (and overwritten) and xn [B], ends [2, F] as fp32_gemm gave them; todo: int32
+// [1 + B], todo[0] zeroed
+void topk_estimate(const Tensor& h, const Tensor& x, const Tensor& W, const Tensor& xn, const Tensor& ends, const c10::optional<Tensor>& bias,
+                   const c10::optional<Tensor>& norm, int64_t k, const Tensor& todo, const Tensor& out) {
+  for (const Tensor* t : {&h, &x, &W, &xn, &out}) { CHECK_T(*t, torch::kFloat32); }
+  for (const Tensor* t : {&ends, &todo}) { CHECK_T(*t, torch::kInt32); }
+  TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && h.size(0) < INT_MAX && h.size(1) <= INT_MAX, "h and out must be [B, F]");
+  TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.size(0) == h.size(0) && W.size(0) == h.size(1) && W.size(1) == x.size(1) &&
+              x.size(1) <= lmsae::kEstimateMaxK, "x [B, K] and W [F, K]");
+  TORCH_CHECK(xn.numel() == h.size(0) && ends.numel() == 2 * h.size(1) && todo.numel() == h.size(0) + 1);
+  if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
+  if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
+  const c10::cuda::CUDAGuard guard(h.device());
+  check_cuda(lmsae::topk_estimate_launch(h.data_ptr<float>(), x.data_ptr<float>(), W.data_ptr<float>(), xn.data_ptr<float>(),
+                                         reinterpret_cast<const uint32_t*>(ends.data_ptr<int>()), (int)x.size(1), opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
+                                         (int)k, todo.data_ptr<int>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "topk_estimate launch");
 }
 
 // out [B, d] = acts [B, F] @ W [F, d], fp32; marks: int32 [1 + B], zeroed
@@ -1208,6 +1228,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
   m.def("topk_dense", &topk_dense);
+  m.def("topk_estimate", &topk_estimate);
   m.def("fp32_gemm", &fp32_gemm);
   m.def("dense_decode", &dense_decode);
   m.def("sparse_decode", &sparse_decode);

@@ -40,21 +40,41 @@ __device__ __forceinline__ int part_a(int t) { return (0x201100 >> (4 * (5 - t))
 __device__ __forceinline__ int part_b(int t) { return (0x021010 >> (4 * (5 - t))) & 15; }
 
 // dst [rows][3][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
-// then flags[0] != 0.
+// then flags[0] != 0. What topk_estimate (topk_merge.cu) takes, both optional: norm[r], at least the row's 2-norm and at most 10 %
+// above it, and ends[0][r], ends[1][r]: gate[r] rounded down / up to bf16 (1 without a gate) in the upper half of a word, that norm rounded up to
+// bf16 in the lower. The norm is infinite where the row's largest magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r]
+// negative, NaN or beyond 2^50: products, (sum + bias) * gate and the parts of what is within stay clear of the ends of the fp32 range
+// (2^30 * 2^30 * K 2^14, doubled, * 2^50 < 2^127).
+struct SplitBounds {
+  float* norm;
+  uint32_t* ends;
+  const float* bias;
+  const float* gate;
+};
+__device__ __forceinline__ uint32_t bf16_up(float x) {  // (x >= 0)
+  const uint32_t b = __float_as_uint(x);
+  return (b >> 16) + ((b & 0xffffu) != 0u ? 1u : 0u);
+}
 __global__ void __launch_bounds__(256)
-split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags) {
+split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags,
+                    const SplitBounds b) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
     const float* s = src + (size_t)r * K;
     __nv_bfloat16* o = dst + (size_t)r * 3 * kp;
     bool bad = false;
+    unsigned top = 0u;
+    float sq = 0.0f;
     for (int c = lane * 4; c < kp; c += 128) {  // (K % 4 == 0, kp % 64 == 0)
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < K) v = __ldg(reinterpret_cast<const float4*>(s + c));
       float x[4] = {v.x, v.y, v.z, v.w}, p[3][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        if ((__float_as_uint(x[i]) & 0x7fffffffu) >= 0x7f000000u) { bad = true; x[i] = 0.0f; }
+        const unsigned mag = __float_as_uint(x[i]) & 0x7fffffffu;
+        top = max(top, mag);
+        sq = fmaf(x[i], x[i], sq);
+        if (mag >= 0x7f000000u) { bad = true; x[i] = 0.0f; }
         p[0][i] = __bfloat162float(__float2bfloat16(x[i]));
         const float r1 = x[i] - p[0][i];
         p[1][i] = __bfloat162float(__float2bfloat16(r1));
@@ -69,11 +89,29 @@ split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv
       flags[1 + r] = bad ? 1 : 0;
       if (bad) flags[0] = 1;
     }
+    if (b.norm != nullptr || b.ends != nullptr) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      sq = warp_sum(sq);
+      if (lane == 0) {
+        const float gate = b.gate != nullptr ? b.gate[r] : 1.0f;
+        bool fits = top == 0u || (top >= 0x2b800000u && top < 0x4e800000u);  // 2^-40, 2^30
+        if (b.bias != nullptr) fits &= (__float_as_uint(b.bias[r]) & 0x7fffffffu) < 0x65000000u;  // 2^75
+        const bool plain = __float_as_uint(gate) < 0x58800000u;  // 2^50 (and no sign)
+        const float n = !(fits && plain) ? __uint_as_float(0x7f800000u) : top == 0u ? 0.0f : 1.05f * sqrtf(sq);
+        if (b.norm != nullptr) b.norm[r] = n;
+        if (b.ends != nullptr) {
+          const float g = plain ? gate : 1.0f;
+          b.ends[r] = (__float_as_uint(g) & 0xffff0000u) | bf16_up(n);
+          b.ends[rows + r] = (bf16_up(g) << 16) | bf16_up(n);
+        }
+      }
+    }
   }
 }
 
 struct Fp32GemmParams {
   int M, N, kp;
+  long long ldc;
   int m_tiles, n_tiles, pairs;
   float* C;
   int* status;
@@ -187,7 +225,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter, column half
-    const bool vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t sub = 0;
     bool ok = true;
     for (int t = pair; t < tiles && ok; t += p.pairs) {
@@ -219,7 +257,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
       }
       if (ok && row < p.M) {
-        float* dst = p.C + (size_t)row * p.N + c0;
+        float* dst = p.C + row * p.ldc + c0;
         if (vec) {
 #pragma unroll
           for (int j = 0; j < 128; j += 4)
@@ -250,7 +288,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 // C[m, n] of marked rows of A or of B on the fp32 pipes, a warp per element; leaves at once where nothing is marked.
 __global__ void __launch_bounds__(256)
 marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B, int M, int N, int K, const int* __restrict__ fa,
-                       const int* __restrict__ fb, float* __restrict__ C) {
+                       const int* __restrict__ fb, float* __restrict__ C, long long ldc) {
   if (fa[0] == 0 && fb[0] == 0) return;
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * 8;
@@ -260,23 +298,24 @@ marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B,
     float s = 0.0f;
     for (int k = lane; k < K; k += 32) s = fmaf(A[(size_t)m * K + k], B[(size_t)n * K + k], s);
     s = warp_sum(s);
-    if (lane == 0) C[e] = s;
+    if (lane == 0) C[m * ldc + n] = s;
   }
 }
 
 }  // namespace
 
-int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, cudaStream_t stream) {
+int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends, const float* bias,
+                        const float* gate, cudaStream_t stream) {
   if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
-  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags);
+  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, ends, bias, gate});
   return (int)cudaGetLastError();
 }
 
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
-                     const int* fb, float* C, int* status, cudaStream_t stream) {
+                     const int* fb, float* C, long long ldc, int* status, cudaStream_t stream) {
   Fp32GemmParams p;
-  p.M = M; p.N = N; p.kp = kp; p.C = C; p.status = status;
+  p.M = M; p.N = N; p.kp = kp; p.C = C; p.ldc = ldc; p.status = status;
   p.m_tiles = (M + 2 * FG_BM - 1) / (2 * FG_BM);
   p.n_tiles = (N + FG_BN - 1) / FG_BN;
   const long long tiles = (long long)p.m_tiles * p.n_tiles;
@@ -298,7 +337,7 @@ int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* 
   cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, fp32_gemm_kernel, ta, tb, p);
   if (e != cudaSuccess) return (int)e;
-  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C);
+  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C, ldc);
   return (int)cudaGetLastError();
 }
 

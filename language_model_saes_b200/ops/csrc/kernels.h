@@ -38,9 +38,10 @@ struct EncGemmParams {
 };
 int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p, int mode, cudaStream_t stream);
 int enc_gemm_slots_for_k(int k);
-int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, cudaStream_t stream);
+int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends, const float* bias,
+                        const float* gate, cudaStream_t stream);
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
-                     const int* fb, float* C, int* status, cudaStream_t stream);
+                     const int* fb, float* C, long long ldc, int* status, cudaStream_t stream);
 
 // ---- peer-memory collectives (comm_ops.cu) -------------------------------------------------------
 constexpr int kMaxPeers = 8;
@@ -75,8 +76,24 @@ struct MergeComm {
 
 int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, int k, const float* gate, int own_lo,
                       int own_hi, int emit_gated, int* out_idx, float* out_val, const MergeComm& comm, cudaStream_t stream);
-int topk_dense_launch(float* h, const float* x, const float* W, int K, const float* bias, const float* norm, int B, int N, int k, float* out,
-                      cudaStream_t stream);
+int topk_dense_launch(const float* h, const float* bias, const float* norm, int B, int N, int k, float* out, cudaStream_t stream);
+constexpr int kEstimateMaxK = 16384;  // (above it the bound on the estimate's error rules out too few columns)
+int topk_estimate_launch(float* h, const float* x, const float* W, const float* xn, const uint32_t* ends, int K, const float* bias, const float* norm,
+                         int B, int N, int k, int* todo, float* out, cudaStream_t stream);
+struct RowsProductParams {
+  const float* A;   // [*, K]
+  const float* B;   // [N, K], or [K, N]
+  float* C;         // [*, N]
+  int N, K;
+  const int* rows;  // [0] how many, then which rows of A and C
+  int max_rows;     // of them at most
+  float* part;      // slices of sums (nullptr: none), and a zeroed counter per tile
+  long long part_floats;
+  int* part_done;
+  int part_tiles;
+  bool vec;         // set by the launch
+};
+int rows_product_launch(RowsProductParams p, bool b_by_k, cudaStream_t stream);
 int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int* marks, float* out, cudaStream_t stream);
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,
                     const uint8_t* alive, int* out_idx, float* out_val, cudaStream_t stream);

@@ -402,29 +402,74 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 
 // ------------------------------------------------------------------------------------------------
 // TopK activation on fp32 pre-activations, dense in and dense out:  out = topk(relu(g)) / norm  with  g = (h + bias) * norm  (bias and
-// norm optional), k entries per row. One CTA per row: group maxima bound the k-th value, a second pass (from L1 / L2) writes the
-// row's zeros and collects the few entries at or above the bound, and the k best of them are written over the zeros. Bound by
-// reading h and writing out. 4096 x 24576, k 50, bias, gate, selection, mask and division: 3.2 ms as torch operations -> 319 us.
-// The arithmetic is that of the operations it replaces, element by element: NaN and -inf (which relu(x) = x * [x > 0] turns into
-// NaN) rank first and stay NaN everywhere, an unselected +inf becomes NaN, and so does everything over a norm of 0 or NaN.
+// norm optional), k entries per row; of equal values the first columns. One CTA per row: group maxima bound the k-th value, a second
+// pass (from L1 / L2) writes the row's zeros and collects the few entries at or above the bound, and the k best of them are written
+// over the zeros. Bound by reading h and writing out. 4096 x 24576, k 50, bias, gate, selection, mask and division: 3.2 ms as torch
+// operations -> 319 us.
+// The arithmetic is that of the operations it replaces, element by element (subnormals included: no flush to zero): NaN and -inf (which
+// relu(x) = x * [x > 0] turns into NaN) rank first and stay NaN everywhere, an unselected +inf becomes NaN, and so does everything over a
+// norm of 0 or NaN.
 //
-// With x and W, h is only an estimate of x . W^T (fp32_gemm.cu: off by some 1e-6 of the scale of its terms, in which it is as good
-// as a sum in order): what is selected, and the selected values, are those of the fp32 sum in ascending order of k, as the fp32
-// product it replaces gives them, bit for bit. The bound is lowered by 2^-8, a thousand times the error of either sum, and
-// the few columns above it are summed up in order before the exact selection (319 -> 508 us; the product: 2505 -> 670 us). Rows for which that would not be sound (fewer than k
-// positive values, something not finite, too many columns at the bound) are summed up in order as a whole.
+// ESTIMATE: h is only an estimate of x . W^T (fp32_gemm.cu). What is selected, and the selected values, are those of the fp32 sum in
+// ascending order of k with one rounding per term. That sum lies within e = rel * xn * wn of the estimate, xn and wn the 2-norms of the
+// row of x and the row of W (Cauchy-Schwarz bounds the sum of the magnitudes of the terms by their product; rel: see estimate_rel).
+// Bias, norm and rounding are monotone, so the same operations on h - e and h + e, with the norm rounded down and up, enclose a positive g.
+// The k-th largest lower end of the group maxima is reached by at least k columns, and whatever is selected has its upper end at or
+// above it: those columns are summed up in order before the exact selection. Norms and wn come as two bf16 in one word: what bounds
+// this kernel is the columns' arrays out of the L2 cache, twice for every row (4096 x 24576 x 768, k 50: 554 us with both in fp32, 506 so; a margin of 2^-8 of the bound, which the error could exceed,
+// took 508). Rows with fewer than k positive values cost no more than others (1.16 ms for product and selection, 77 ms when such
+// rows were summed up in order as a whole), and with every row listed it is 6.5 ms at 4096 x 32768 x 2048 (torch operations: 12.6).
+// Columns that the bound says nothing about (wn is infinite there) are among them; rows with more such columns than there is room for are listed, multiplied in order as a whole
+// (rows_product.cu) and selected from exactly. All decisions are taken on the device.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned topk_key(float g) {
   const unsigned b = __float_as_uint(g);
   if ((b & 0x7fffffffu) > 0x7f800000u || b == 0xff800000u) return 0x7fffffffu;
   return (int)b > 0 ? b : 0u;
 }
+// (the intrinsics flush subnormals under this build's flags)
+#define LMSAE_F32_OP(name, op)                                             \
+  __device__ __forceinline__ float name(float a, float b) {                \
+    float r;                                                               \
+    asm(op " %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));                     \
+    return r;                                                              \
+  }
+LMSAE_F32_OP(add_rn, "add.rn.f32")
+LMSAE_F32_OP(mul_rn, "mul.rn.f32")
+LMSAE_F32_OP(mul_up, "mul.rp.f32")
+LMSAE_F32_OP(div_rn, "div.rn.f32")
+#undef LMSAE_F32_OP
+__device__ __forceinline__ float fma_rn(float a, float b, float c) {
+  float r;
+  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ bool below(float a, float b) {  // a < b: false for a NaN, subnormals as they are
+  int r;
+  asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, %2;\n\tselp.s32 %0, 1, 0, p;\n\t}" : "=r"(r) : "f"(a), "f"(b));
+  return r != 0;
+}
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f800000u; }
+
+// rel for sums of K terms, in units of 2^-24 (what the parts add up to):
+//   K        roundings of the sum in order, one per term
+//   K / 128  roundings of the estimate's slices added up
+//   384      accumulations within a slice of 128 terms: the last eight instructions add sixteen full-size products each to what is there,
+//            and each of these 17 operands may lose a unit to the alignment (136); the 40 before them add parts of 2^-8 and less (3);
+//            the rest is margin for what the hardware does not document (measured: 2 units in all)
+//   16       the three products that are left out (2^-25), the rounding of the ends themselves (|h| is at most about xn wn), and room
+// The norms are rounded up by 5 % where they are made, which covers their own rounding and K 2^-24 << 1.
+__host__ __device__ __forceinline__ float estimate_rel(int K) { return ((float)K * 1.01f + 400.0f) * 5.9604645e-8f; }
 
 struct TopkDenseParams {
   float* h;
-  const float* x;  // [B, K] and [N, K], or null: h is what it is
+  const float* x;  // ESTIMATE: [B, K] and [N, K], and what the split of x and of W left (fp32_gemm.cu)
   const float* W;
+  const float* xn;
+  const uint32_t* ends;
   int K;
+  int* todo;        // ESTIMATE: [1 + B] number of rows left over, and which
+  const int* rows;  // or the rows to work on, in this form
   const float* bias;
   const float* norm;
   float* out;
@@ -432,34 +477,39 @@ struct TopkDenseParams {
   bool vec;
 };
 
-// g of columns [c, c + 4), and whether a zero there ends as NaN (columns past the end of the row: g = 0)
-__device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const float* h /* may be rewritten: no read-only path */, int c, float (&g)[4], bool (&bad)[4]) {
-  float n[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+// g of columns [c, c + 4) and the norms (columns past the end: 0 and 1)
+// ESTIMATE: an end of g, the lower one for rx with a sign and the lower words of `ends`, else the upper one; the norms as those words have them
+template <bool ESTIMATE>
+__device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const float* __restrict__ h, int c, float rx, float (&g)[4], float (&n)[4]) {
+  float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  uint32_t w[4] = {0x3f800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u};  // norm 1, and in a word of `ends` also a 2-norm of 0
+  const uint32_t* words = ESTIMATE ? p.ends + ((int)__float_as_uint(rx) < 0 ? 0 : p.N) : reinterpret_cast<const uint32_t*>(p.norm);
   if (p.vec) {
-    const float4 a = *reinterpret_cast<const float4*>(h + c);
+    const float4 a = __ldg(reinterpret_cast<const float4*>(h + c));
     g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
     if (p.bias != nullptr) {
-      const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + c));
-      g[0] = __fadd_rn(g[0], b.x); g[1] = __fadd_rn(g[1], b.y); g[2] = __fadd_rn(g[2], b.z); g[3] = __fadd_rn(g[3], b.w);
+      const float4 t = __ldg(reinterpret_cast<const float4*>(p.bias + c));
+      b[0] = t.x; b[1] = t.y; b[2] = t.z; b[3] = t.w;
     }
-    if (p.norm != nullptr) {
-      const float4 b = __ldg(reinterpret_cast<const float4*>(p.norm + c));
-      n[0] = b.x; n[1] = b.y; n[2] = b.z; n[3] = b.w;
+    if (words != nullptr) {
+      const uint4 t = __ldg(reinterpret_cast<const uint4*>(words + c));
+      w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
     }
   } else {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool in = c + i < p.N;
-      g[i] = in ? h[c + i] : 0.0f;
-      if (in && p.bias != nullptr) g[i] = __fadd_rn(g[i], p.bias[c + i]);
-      if (in && p.norm != nullptr) n[i] = p.norm[c + i];
+      g[i] = in ? __ldg(h + c + i) : 0.0f;
+      if (in && p.bias != nullptr) b[i] = p.bias[c + i];
+      if (in && words != nullptr) w[i] = __ldg(words + c + i);
     }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if (p.norm != nullptr) g[i] = __fmul_rn(g[i], n[i]);
-    const unsigned nb = __float_as_uint(n[i]) & 0x7fffffffu;
-    bad[i] = (__float_as_uint(g[i]) & 0x7fffffffu) >= 0x7f800000u || nb == 0u || nb > 0x7f800000u;
+    n[i] = __uint_as_float(ESTIMATE ? w[i] & 0xffff0000u : w[i]);
+    if constexpr (ESTIMATE) g[i] = fma_rn(rx, __uint_as_float(w[i] << 16), g[i]);
+    if (p.bias != nullptr) g[i] = add_rn(g[i], b[i]);
+    if (ESTIMATE || p.norm != nullptr) g[i] = mul_rn(g[i], n[i]);
   }
 }
 
@@ -469,32 +519,34 @@ __device__ __forceinline__ float dot_in_order(const float* __restrict__ x, const
 #pragma unroll 8
   for (int i = 0; i < K; i += 4) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(x + i)), b = __ldg(reinterpret_cast<const float4*>(w + i));
-    s = __fmaf_rn(a.x, b.x, s);
-    s = __fmaf_rn(a.y, b.y, s);
-    s = __fmaf_rn(a.z, b.z, s);
-    s = __fmaf_rn(a.w, b.w, s);
+    s = fma_rn(a.x, b.x, s);
+    s = fma_rn(a.y, b.y, s);
+    s = fma_rn(a.z, b.z, s);
+    s = fma_rn(a.w, b.w, s);
   }
   return s;
 }
 
-__global__ void __launch_bounds__(RT_THREADS, 5)
-topk_dense_kernel(const TopkDenseParams p) {
+// Sum over the CTA, the same in every thread.
+__device__ __forceinline__ int cta_count(int mine, unsigned (&words)[RT_WARPS]) {
+  const unsigned total = __reduce_add_sync(0xffffffffu, (unsigned)mine);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = total;
+  __syncthreads();
+  return (int)__reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < RT_WARPS ? words[threadIdx.x & 31] : 0u);
+}
+
+template <bool ESTIMATE>
+__device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row) {
   __shared__ unsigned s_key[RT_CAP];
   __shared__ int s_col[RT_CAP];
   __shared__ unsigned s_count[2][RT_WARPS];
-  __shared__ int s_n, s_cursor;
-  float* h = p.h + (size_t)blockIdx.x * p.N;
-  float* out = p.out + (size_t)blockIdx.x * p.N;
+  __shared__ int s_n, s_above, s_equal;
+  const float* h = p.h + (size_t)row * p.N;
+  float* out = p.out + (size_t)row * p.N;
   const int N = p.N, k = p.k;
-  const float* x = p.x != nullptr ? p.x + (size_t)blockIdx.x * p.K : nullptr;
-  bool estimate = x != nullptr;
-  auto sum_row_in_order = [&]() {
-    for (int c = threadIdx.x; c < N; c += RT_THREADS) h[c] = dot_in_order(x, p.W + (size_t)c * p.K, p.K);
-    estimate = false;
-    __syncthreads();
-  };
-restart:
-  if (threadIdx.x == 0) { s_n = 0; s_cursor = 0; }
+  const float rx = ESTIMATE ? mul_up(estimate_rel(p.K), p.xn[row]) : 0.0f, rx_lo = __uint_as_float(__float_as_uint(rx) | 0x80000000u);
+  if (threadIdx.x == 0) { s_n = 0; s_above = 0; s_equal = 0; }
   unsigned mx[RT_MAXIMA];
 #pragma unroll
   for (int i = 0; i < RT_MAXIMA; ++i) mx[i] = 0u;
@@ -503,41 +555,42 @@ restart:
 #pragma unroll
     for (int half = 0; half < 8; half += 4) {
       if (c + half >= N) break;
-      float g[4];
-      bool bad[4];
-      topk_dense_load(p, h, c + half, g, bad);
+      float g[4], nm[4];
+      topk_dense_load<ESTIMATE>(p, h, c + half, rx_lo, g, nm);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) mx[half + i] = max(mx[half + i], topk_key(g[i]));
+      for (int i = 0; i < 4; ++i) {
+        // (ESTIMATE: where wn is infinite the lower end is -inf or NaN, and neither enters)
+        if constexpr (ESTIMATE) mx[half + i] = __float_as_uint(fmaxf(__uint_as_float(mx[half + i]), g[i]));
+        else mx[half + i] = max(mx[half + i], topk_key(g[i]));
+      }
     }
   }
   unsigned thr = descend(mx, k, 16, s_count);  // a bound until the exact value is known (0: fewer than k positive maxima)
-  if (estimate) {
-    bool special = thr == 0u;
-#pragma unroll
-    for (int i = 0; i < RT_MAXIMA; ++i) special |= mx[i] >= 0x7f800000u;
-    if (__syncthreads_or(special)) {
-      sum_row_in_order();
-      goto restart;
-    }
-    thr = __float_as_uint(__uint_as_float(thr) * (1.0f - 1.0f / 256.0f));
-  }
-  const float nan = __uint_as_float(0x7fffffffu);
+  const float nan = __uint_as_float(0x7fffffffu), thr_f = __uint_as_float(max(thr, 1u));
 #pragma unroll 2
   for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
 #pragma unroll
     for (int half = 0; half < 8; half += 4) {
       if (c + half >= N) break;
-      float g[4];
-      bool bad[4];
-      topk_dense_load(p, h, c + half, g, bad);
+      float g[4], nm[4];
+      topk_dense_load<ESTIMATE>(p, h, c + half, rx, g, nm);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const unsigned key = topk_key(g[i]);
-        if (key != 0u && key >= thr) {
+        const unsigned nb = __float_as_uint(nm[i]) & 0x7fffffffu;
+        unsigned key = 0u;
+        bool enters, bad = nb == 0u || nb > 0x7f800000u;
+        if constexpr (ESTIMATE) {  // (where wn is infinite the upper end is +inf or NaN, and enters; its value is looked at below)
+          enters = !below(g[i], thr_f);
+        } else {
+          key = topk_key(g[i]);
+          enters = key != 0u && key >= thr;
+          bad |= not_finite(g[i]);
+        }
+        if (enters) {
           const int pos = atomicAdd(&s_n, 1);
           if (pos < RT_CAP) { s_key[pos] = key; s_col[pos] = c + half + i; }
         }
-        g[i] = bad[i] ? nan : 0.0f;
+        g[i] = bad ? nan : 0.0f;
       }
       if (p.vec) {
         __stcs(reinterpret_cast<float4*>(out + c + half), make_float4(g[0], g[1], g[2], g[3]));
@@ -550,82 +603,147 @@ restart:
   }
   __syncthreads();  // (also: the zeros are written before what is written over them)
   const int n = s_n;
-  if (estimate) {
+  if constexpr (ESTIMATE) {
     if (n > RT_CAP) {
-      sum_row_in_order();
-      goto restart;
+      if (threadIdx.x == 0) p.todo[1 + atomicAdd(p.todo, 1)] = row;
+      return;
     }
+    const float* x = p.x + (size_t)row * p.K;
     // (neighbouring candidates to different warps: a few dozen of them in one or two warps wait for their rows of W alone, 536 us)
     for (int j = (threadIdx.x & 31) * RT_WARPS + (threadIdx.x >> 5); j < n; j += RT_THREADS) {
       const int c = s_col[j];
       float g = dot_in_order(x, p.W + (size_t)c * p.K, p.K);
-      if (p.bias != nullptr) g = __fadd_rn(g, p.bias[c]);
-      if (p.norm != nullptr) g = __fmul_rn(g, p.norm[c]);
+      if (p.bias != nullptr) g = add_rn(g, p.bias[c]);
+      unsigned nb = 1u;
+      if (p.norm != nullptr) {
+        g = mul_rn(g, p.norm[c]);
+        nb = __float_as_uint(p.norm[c]) & 0x7fffffffu;
+      }
       s_key[j] = topk_key(g);
+      if (not_finite(g) || nb == 0u || nb > 0x7f800000u) out[c] = nan;  // (the last two are NaN already)
     }
     __syncthreads();
   }
   auto put = [&](int c, unsigned key) {
-    if (atomicAdd(&s_cursor, 1) >= k || key == 0x7fffffffu) return;  // (what is NaN already stays so)
+    if (key == 0x7fffffffu) return;  // (what is NaN already stays so)
     float v = __uint_as_float(key);
-    if (p.norm != nullptr) v = __fdiv_rn(v, p.norm[c]);
+    if (p.norm != nullptr) v = div_rn(v, p.norm[c]);
     out[c] = v;
   };
   if (n <= RT_CAP) {
-    unsigned mine[RT_CAP / RT_THREADS];
+    if (n > k) {
+      unsigned mine[RT_CAP / RT_THREADS];
 #pragma unroll
-    for (int i = 0; i < RT_CAP / RT_THREADS; ++i) {
-      const int j = threadIdx.x + i * RT_THREADS;
-      mine[i] = j < n ? s_key[j] : 0u;
+      for (int i = 0; i < RT_CAP / RT_THREADS; ++i) {
+        const int j = threadIdx.x + i * RT_THREADS;
+        mine[i] = j < n ? s_key[j] : 0u;
+      }
+      thr = descend(mine, k, 0, s_count);
+    } else {
+      thr = 0u;
     }
-    thr = n > k ? descend(mine, k, 0, s_count) : 0u;
-    for (int j = threadIdx.x; j < n; j += RT_THREADS)
-      if (s_key[j] > thr) put(s_col[j], s_key[j]);
-    __syncthreads();
-    for (int j = threadIdx.x; j < n; j += RT_THREADS)
-      if (s_key[j] == thr) put(s_col[j], thr);
-    return;
-  }
-  // values repeated thousands of times: the descent over the row itself, one pass per bit
-  auto keys_of = [&](auto&& visit) {
-    for (int c = threadIdx.x * 4; c < N; c += RT_THREADS * 4) {
-      float g[4];
-      bool bad[4];
-      topk_dense_load(p, h, c, g, bad);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const unsigned key = topk_key(g[i]);
-        if (key != 0u) visit(c + i, key);
+    for (int j = threadIdx.x; j < n; j += RT_THREADS) {
+      const unsigned key = s_key[j];
+      if (key > thr) {
+        put(s_col[j], key);
+        if (thr != 0u) atomicAdd(&s_above, 1);
+      } else if (key == thr && thr != 0u) {
+        atomicAdd(&s_equal, 1);
       }
     }
-  };
-  thr = 0u;
-  for (int bit = 30; bit >= 0; --bit) {
-    const unsigned trial = thr | (1u << bit);
-    int mine = 0;
-    keys_of([&](int, unsigned key) { mine += key >= trial; });
-    const unsigned total = __reduce_add_sync(0xffffffffu, (unsigned)mine);
+    if (thr == 0u) return;  // (all of them)
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) s_count[0][threadIdx.x >> 5] = total;
-    __syncthreads();
-    const unsigned all = __reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < RT_WARPS ? s_count[0][threadIdx.x & 31] : 0u);
-    if (all >= (unsigned)k) thr = trial;
+    const int places = k - s_above;
+    const bool all = s_equal <= places;
+    for (int j = threadIdx.x; j < n; j += RT_THREADS) {
+      if (s_key[j] != thr) continue;
+      const int c = s_col[j];
+      int before = 0;
+      if (!all)
+        for (int i = 0; i < n; ++i) before += s_key[i] == thr && s_col[i] < c;
+      if (before < places) put(c, thr);
+    }
+    return;
   }
-  keys_of([&](int c, unsigned key) { if (key > thr) put(c, key); });
-  __syncthreads();
-  keys_of([&](int c, unsigned key) { if (key == thr) put(c, key); });
+  if constexpr (!ESTIMATE) {
+    // values repeated thousands of times: the descent over the row itself, one pass per bit
+    auto keys_of = [&](auto&& visit) {
+      for (int c = threadIdx.x * 4; c < N; c += RT_THREADS * 4) {
+        float g[4], nm[4];
+        topk_dense_load<false>(p, h, c, 0.0f, g, nm);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned key = topk_key(g[i]);
+          if (key != 0u) visit(c + i, key);
+        }
+      }
+    };
+    auto count_of = [&](auto&& which) {
+      int mine = 0;
+      keys_of([&](int c, unsigned key) { mine += which(c, key); });
+      return cta_count(mine, s_count[0]);
+    };
+    thr = 0u;
+    for (int bit = 30; bit >= 0; --bit) {
+      const unsigned trial = thr | (1u << bit);
+      if (count_of([&](int, unsigned key) { return key >= trial; }) >= k) thr = trial;
+    }
+    keys_of([&](int c, unsigned key) { if (key > thr) put(c, key); });
+    if (thr == 0u || thr == 0x7fffffffu) return;
+    // the equal ones up to the column at which the places are taken
+    const int places = k - count_of([&](int, unsigned key) { return key > thr; });
+    int end = 0;  // at most `places` equal values lie in columns below it
+    for (int bit = 30; bit >= 0; --bit) {
+      const long long trial = (long long)end + (1LL << bit);
+      if (trial <= N && count_of([&](int c, unsigned key) { return key == thr && c < trial; }) <= places) end = (int)trial;
+    }
+    keys_of([&](int c, unsigned key) { if (key == thr && c < end) put(c, thr); });
+  }
 }
 
-int topk_dense_launch(float* h, const float* x, const float* W, int K, const float* bias, const float* norm, int B, int N, int k, float* out,
-                      cudaStream_t stream) {
+template <bool ESTIMATE>
+__global__ void __launch_bounds__(RT_THREADS, 5)
+topk_dense_kernel(const TopkDenseParams p) {
+  topk_dense_row<ESTIMATE>(p, blockIdx.x);
+}
+
+__global__ void __launch_bounds__(RT_THREADS, 5)
+topk_dense_rows_kernel(const TopkDenseParams p) {
+  const int n = p.rows[0];
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    topk_dense_row<false>(p, p.rows[1 + i]);
+    __syncthreads();
+  }
+}
+
+int topk_dense_launch(const float* h, const float* bias, const float* norm, int B, int N, int k, float* out, cudaStream_t stream) {
   if (B <= 0 || N <= 0) return 0;
-  if (x != nullptr && (W == nullptr || K % 4 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) != 0)) return (int)cudaErrorInvalidValue;
   if (k < 1 || k > RT_BOUND_K) return (int)cudaErrorInvalidValue;
-  TopkDenseParams p;
-  p.h = h; p.x = x; p.W = W; p.K = K; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  TopkDenseParams p = {};
+  p.h = const_cast<float*>(h); p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
   p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
                           reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  topk_dense_kernel<<<B, RT_THREADS, 0, stream>>>(p);
+  topk_dense_kernel<false><<<B, RT_THREADS, 0, stream>>>(p);
+  return (int)cudaGetLastError();
+}
+
+// The same with h an estimate of x W^T (and overwritten where it is too coarse). todo: int [1 + B], todo[0] zeroed.
+int topk_estimate_launch(float* h, const float* x, const float* W, const float* xn, const uint32_t* ends, int K, const float* bias, const float* norm,
+                         int B, int N, int k, int* todo, float* out, cudaStream_t stream) {
+  if (B <= 0 || N <= 0) return 0;
+  if (k < 1 || k > RT_BOUND_K || K < 1 || K > kEstimateMaxK || K % 4 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) != 0)
+    return (int)cudaErrorInvalidValue;
+  TopkDenseParams p = {};
+  p.h = h; p.x = x; p.W = W; p.xn = xn; p.ends = ends; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
+                          reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ends)) % 16 == 0);
+  topk_dense_kernel<true><<<B, RT_THREADS, 0, stream>>>(p);
+  RowsProductParams r = {};
+  r.A = x; r.B = W; r.C = h; r.N = N; r.K = K; r.rows = todo; r.max_rows = B;
+  const int e = rows_product_launch(r, false, stream);
+  if (e != 0) return e;
+  p.rows = todo;
+  topk_dense_rows_kernel<<<B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }
 

@@ -14,6 +14,7 @@ from torch.utils._python_dispatch import _get_current_dispatch_mode
 from . import sae_kernels as K
 
 MAX_K = 1024  # the selection kernel's bound comes from 2048 column groups
+MAX_ESTIMATE_WIDTH = 16384  # kEstimateMaxK in csrc/kernels.h
 
 
 def plain_inference(*tensors: torch.Tensor) -> bool:
@@ -38,10 +39,10 @@ def product_supported(x: torch.Tensor, W: torch.Tensor) -> bool:
     """``x [..., K] @ W [K, N]`` with the columns of ``W`` contiguous, large enough for the split of the operands to pay (it costs
     about what 60 rows cost on the fp32 pipes) and with full fp32 precision asked for."""
     K_, N = W.shape
-    if x.ndim < 2 or x.shape[-1] != K_ or K_ % 4 != 0 or K_ == 0 or N == 0:
+    if x.ndim < 2 or x.shape[-1] != K_ or K_ % 4 != 0 or not 0 < K_ <= MAX_ESTIMATE_WIDTH or N == 0:
         return False
     M = x.numel() // K_
-    return (M >= 256 and 2 * M * N * K_ >= 4e9 and M < 2**31 - 512 and N < 2**31 - 512 and 3 * K_ < 2**31 - 256 and x.is_contiguous()
+    return (M >= 256 and 2 * M * N * K_ >= 4e9 and M < 2**31 - 512 and N < 2**31 - 512 and x.is_contiguous()
             and W.t().is_contiguous() and x.data_ptr() % 16 == 0 and W.data_ptr() % 16 == 0
             and torch.get_float32_matmul_precision() == "highest")  # fmt: skip
 
@@ -50,7 +51,7 @@ def product(x: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
     """``x @ W`` in fp32."""
     rows = x.detach().reshape(-1, x.shape[-1])
     out = torch.empty(rows.shape[0], W.shape[1], dtype=torch.float32, device=x.device)
-    K._ext().fp32_gemm(rows, W.detach().t(), out, K.status_buffer(x.device))
+    K._ext().fp32_gemm(rows, W.detach().t(), out, K.status_buffer(x.device), None, None, None, None)
     return out.view(*x.shape[:-1], W.shape[1])
 
 
@@ -62,19 +63,22 @@ def topk_dense(h: torch.Tensor, bias: torch.Tensor | None, norm: torch.Tensor | 
     """``topk(relu((h + bias) * norm)) / norm`` over the last dimension (``bias`` and ``norm`` optional)."""
     rows = h.reshape(-1, h.shape[-1])
     out = torch.empty_like(rows)
-    K._ext().topk_dense(rows, None, None, bias.contiguous() if bias is not None else None, norm.contiguous() if norm is not None else None, k, out)
+    K._ext().topk_dense(rows, bias.contiguous() if bias is not None else None, norm.contiguous() if norm is not None else None, k, out)
     return out.view(h.shape)
 
 
 def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, norm: torch.Tensor | None, k: int) -> torch.Tensor:
-    """``topk_dense(x @ W, ...)`` for operands of ``product``, which proposes: the selection sums what it considers again, in the
-    order of the fp32 pipes, so that no choice between nearly equal values depends on how the estimate was made."""
-    h = product(x, W)
-    rows = h.view(-1, h.shape[-1])
-    out = torch.empty_like(rows)
-    K._ext().topk_dense(rows, x.detach().reshape(-1, x.shape[-1]), W.detach().t(), bias.contiguous() if bias is not None else None,
-                        norm.contiguous() if norm is not None else None, k, out)  # fmt: skip
-    return out.view(h.shape)
+    """``topk_dense(x @ W, ...)`` for operands of ``product``, which proposes: what the estimate leaves in question is summed again in
+    ascending order of the input dimension, so that neither the choice nor the values depend on how the estimate was made."""
+    rows = x.detach().reshape(-1, x.shape[-1])
+    B, F = rows.shape[0], W.shape[1]
+    h, out = (torch.empty(B, F, dtype=torch.float32, device=x.device) for _ in range(2))
+    xn, ends = torch.empty(B, dtype=torch.float32, device=x.device), torch.empty(2, F, dtype=torch.int32, device=x.device)
+    todo = torch.zeros(1 + B, dtype=torch.int32, device=x.device)
+    bias, norm = (t.contiguous() if t is not None else None for t in (bias, norm))
+    K._ext().fp32_gemm(rows, W.detach().t(), h, K.status_buffer(x.device), xn, ends, bias, norm)
+    K._ext().topk_estimate(h, rows, W.detach().t(), xn, ends, bias, norm, k, todo, out)
+    return out.view(*x.shape[:-1], F)
 
 
 def sparse_decode_supported(acts: torch.Tensor, W: torch.Tensor) -> bool:

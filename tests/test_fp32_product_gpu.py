@@ -77,3 +77,83 @@ def test_selection_is_that_of_sums_in_order(B, F, K_, k, data):
         assert torch.equal((out * norm).sort(-1).values, (want * norm).sort(-1).values)
     else:
         assert torch.equal(out.nan_to_num(nan=-1.0), want.nan_to_num(nan=-1.0))
+
+
+def _in_order(x, w):
+    """fp32 sums in ascending order, one rounding per term: the sum in 64 bits is rounded to odd first (what it lost goes into its last
+    bit), or one step in 2^29 would be rounded twice."""
+    h = torch.zeros(x.shape[0], w.shape[0], device=DEV, dtype=torch.float64)
+    for i in range(x.shape[1]):
+        p = x[:, i : i + 1].double() * w[:, i].double()
+        s = h + p
+        b = s - h
+        lost = (h - (s - b)) + (p - b)
+        bits = s.view(torch.int64)
+        odd = (bits - ((lost > 0) != (s > 0)).to(torch.int64)) | 1
+        h = torch.where((lost != 0) & s.isfinite(), odd, bits).view(torch.float64).float().double()
+    return h.float()
+
+
+@pytest.mark.parametrize("data", ["cancelling", "near zero", "repeated", "out of range", "one bad column"])
+@pytest.mark.parametrize("F,K_,k", [(4104, 128, 50), (9001, 260, 700)])
+def test_selection_where_the_estimate_says_little(F, K_, k, data):
+    g = torch.Generator(device=DEV).manual_seed(F)
+    B = 270
+    x, w = torch.randn(B, K_, device=DEV, generator=g), torch.randn(F, K_, device=DEV, generator=g) / K_**0.5
+    bias, norm = 0.1 * torch.randn(F, device=DEV, generator=g), torch.rand(F, device=DEV, generator=g) + 0.5
+    if data == "cancelling":  # a common offset that the bias takes away: what is left is a few units in the last place of the sums
+        w *= 1e-3
+        x[:, 0], w[:, 0] = 1000.0, 1.0
+        bias = bias * 1e-3 - 1000.0
+        norm[:] = 1.0
+    elif data == "near zero":  # the k-th value is within rounding of zero
+        bias = -_in_order(x[:1], w)[0].topk(k).values[-1].expand(F).clone()
+        x[1:] = x[0] * (1 + 1e-6 * torch.randn(B - 1, 1, device=DEV, generator=g))
+        norm[:] = 1.0
+    elif data == "repeated":  # more equal features than there is room for, and fewer than that
+        w[: F * 3 // 4] = w[0]
+        bias[: F * 3 // 4], norm[: F * 3 // 4] = 1.0, 1.0
+        x[B // 2 :] = x[0]
+    elif data == "out of range":
+        x[0] *= 1e-25
+        x[1] *= 1e25
+        x[2] = 0.0
+        w[5] *= 1e-25
+        w[7] *= 1e20
+        w[9] = 0.0
+    else:
+        w[11, 3] = float("nan")
+        w[13, 4] = float("inf")
+    out = I.topk_encode(x, w.t(), bias, norm, k)
+    want = I.topk_dense(_in_order(x, w), bias, norm, k)
+    differ = (out.nan_to_num(nan=-1.0) != want.nan_to_num(nan=-1.0)).nonzero()
+    assert differ.numel() == 0, (differ[:4], len(differ))
+
+
+@pytest.mark.parametrize("F,k,equal", [(64, 5, 64), (3000, 7, 2400), (24576, 50, 24576), (30001, 1000, 9000)])
+def test_of_equal_values_the_first_columns_are_kept(F, k, equal):
+    g = torch.Generator().manual_seed(F)
+    h = -torch.rand(3, F, generator=g)
+    for r in range(3):
+        h[r, torch.randperm(F, generator=g)[:equal]] = 0.75
+    h[0, F // 2], h[1, F - 1] = 2.0, 3.0
+    order = h.clamp_min(0.0).sort(dim=1, descending=True, stable=True).indices[:, :k]
+    want = torch.zeros_like(h).scatter_(1, order, h.gather(1, order)).clamp_min(0.0)
+    assert torch.equal(I.topk_dense(h.to(DEV), None, None, k).cpu(), want)
+
+
+def test_rows_with_few_positive_values_cost_no_more_than_others():
+    g = torch.Generator(device=DEV).manual_seed(0)
+    x, w = torch.randn(1024, 512, device=DEV, generator=g), torch.randn(8192, 512, device=DEV, generator=g) / 512**0.5
+    bias, times = torch.zeros(8192, device=DEV), []
+    for shift in (0.0, -4.0):  # half of the features positive, hardly any
+        for i in range(8):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            I.topk_encode(x, w.t(), bias + shift, None, 50)
+            end.record()
+            end.synchronize()
+            if i == 0 or start.elapsed_time(end) < best:
+                best = start.elapsed_time(end)
+        times.append(best)
+    assert times[1] < 3 * times[0], times  # (summed up as whole rows they took thirty times as long)
