@@ -1176,11 +1176,14 @@ void comm_exchange_rows(const std::vector<int64_t>& table, const std::vector<Ten
 // violations]} since the last call (all zero in the regular build); reading clears them.
 std::map<std::string, std::vector<int64_t>> bounds_report() {
   std::map<std::string, std::vector<int64_t>> out;
-  int rec[4];
-  check_cuda(lmsae::bounds_fetch_sparse_ops(rec), "bounds_fetch_sparse_ops");
-  out["sparse_ops.cu"] = {rec[0], rec[1], rec[2], rec[3]};
-  check_cuda(lmsae::bounds_fetch_comm_ops(rec), "bounds_fetch_comm_ops");
-  out["comm_ops.cu"] = {rec[0], rec[1], rec[2], rec[3]};
+  const std::pair<const char*, int (*)(int*)> units[] = {  // every file whose kernels check an index
+      {"sparse_ops.cu", lmsae::bounds_fetch_sparse_ops}, {"comm_ops.cu", lmsae::bounds_fetch_comm_ops}, {"grad_adam.cu", lmsae::bounds_fetch_grad_adam},
+      {"clt_ops.cu", lmsae::bounds_fetch_clt_ops}, {"dense_decode.cu", lmsae::bounds_fetch_dense_decode}};
+  for (const auto& [name, fetch] : units) {
+    int rec[4];
+    check_cuda(fetch(rec), name);
+    out[name] = {rec[0], rec[1], rec[2], rec[3]};
+  }
   return out;
 }
 

@@ -18,6 +18,8 @@
 
 namespace lmsae {
 
+LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_clt_ops)
+
 // ---------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------

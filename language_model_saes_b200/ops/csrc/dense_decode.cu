@@ -13,6 +13,8 @@
 
 namespace lmsae {
 
+LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_dense_decode)
+
 namespace {
 
 constexpr int DD_THREADS = 256;

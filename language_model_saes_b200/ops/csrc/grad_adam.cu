@@ -32,6 +32,8 @@
 
 namespace lmsae {
 
+LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_grad_adam)
+
 namespace {
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

@@ -101,6 +101,9 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 // Records of the bounds-checked debug build, one per translation unit (all zero in the regular build).
 int bounds_fetch_sparse_ops(int* out);
 int bounds_fetch_comm_ops(int* out);
+int bounds_fetch_grad_adam(int* out);
+int bounds_fetch_clt_ops(int* out);
+int bounds_fetch_dense_decode(int* out);
 
 struct DecodeParams {
   const int* idx;

@@ -49,6 +49,17 @@ K.check_status(dev)
 rep = ext.bounds_report()
 assert all(v[3] == 0 for v in rep.values()), rep
 assert losses[-1] < losses[0]
+# an entry list that points past the codes: the update kernel records it, too
+F, d, B, k = 512, 64, 32, 4
+z = lambda *s, dt=torch.float32: torch.zeros(*s, dtype=dt, device=dev)  # noqa: E731
+groups = K.FeatureGroups(F, B * k, dev).build(idx)
+groups.entries[5] = B * k + 9
+xb = torch.randn(B, d, device=dev).to(torch.bfloat16)
+K.sparse_grad_adam(groups, val, z(B, k), xb, xb, z(F, d), z(F, d), z(F, d), z(F, d, dt=torch.bfloat16), z(F, d), z(F, d), z(F, d),
+                   z(F, d, dt=torch.bfloat16), z(F), z(F), z(F), z(F), None, None, 1e-3, 0.9, 0.999, 1e-8, 1, True)
+torch.cuda.synchronize()
+line, index, limit, count = ext.bounds_report()["grad_adam.cu"]
+assert count >= 1 and index == B * k + 9 and limit == B * k and line > 0, (line, index, limit, count)
 print("checked build ok")
 """
 
@@ -58,3 +69,4 @@ def test_checked_build_records_and_clamps_an_out_of_range_index():
     env = dict(os.environ, LMSAE_NATIVE_CHECKED="1", PYTHONPATH=str(root))
     r = subprocess.run([sys.executable, "-c", CHILD], env=env, cwd=str(root), capture_output=True, text=True, timeout=900)
     assert r.returncode == 0 and "checked build ok" in r.stdout, r.stdout[-2000:] + r.stderr[-3000:]
+
