@@ -300,6 +300,7 @@ void sparse_decode(const Tensor& idx, const Tensor& val, const Tensor& W, const 
   TORCH_CHECK(idx.dim() == 2 && val.sizes() == idx.sizes() && W.dim() == 2);
   const c10::cuda::CUDAGuard guard(idx.device());
   lmsae::DecodeParams p{};
+  Tensor row_part;
   p.idx = idx.data_ptr<int>();
   p.val = val.data_ptr<float>();
   p.B = (int)idx.size(0);
@@ -329,6 +330,10 @@ void sparse_decode(const Tensor& idx, const Tensor& val, const Tensor& W, const 
     p.dxhat = opt_ptr<__nv_bfloat16>(dxhat);
     p.loss_sum = opt_ptr<float>(loss_sum);
     p.row_loss = opt_ptr<float>(row_loss);
+    if (row_loss.has_value()) {
+      row_part = torch::empty({(int64_t)p.B * lmsae::sparse_decode_segments(p.d)}, val.options());
+      p.row_part = row_part.data_ptr<float>();
+    }
     p.dval = opt_ptr<float>(dval);
   }
   check_cuda(lmsae::sparse_decode_launch(p, at::cuda::getCurrentCUDAStream()), "sparse_decode launch");

@@ -30,7 +30,8 @@ __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, f
 // acc[u][:] = sum_j val[j] * W[idx[j], 8 v[u] .. 8 v[u] + 8) over the entries of one list (idx < 0: empty slot; idx >= limit:
 // not for this caller), lanes of the warp owning the 16-byte chunks v[u] of every row. Lanes fetch 32 entries at a time
 // (the next 32 while the rows of these are on their way) and hand them round by shuffles; the rows of up to eight
-// entries (four for VPT = 2) are requested before the first is used. Entries with a zero coefficient are skipped.
+// entries (four for VPT = 2) are requested before the first is used. An entry whose coefficient is zero counts like any other: a row that
+// is not finite shows in the sum (passing over them instead saved nothing: a crosscoder step of 8 heads takes 16.29 ms either way).
 template <int VPT>
 __device__ __forceinline__ void gather_rows_warp(const int* __restrict__ idx, const float* __restrict__ val, int k,
                                                  const __nv_bfloat16* __restrict__ W, int d, long long n_rows, long long limit,
@@ -49,7 +50,7 @@ __device__ __forceinline__ void gather_rows_warp(const int* __restrict__ idx, co
     const float a_l = a_next;
     f_next = -1;
     if (base + 32 + lane < k) { f_next = __ldg(idx + base + 32 + lane); a_next = __ldg(val + base + 32 + lane); }
-    unsigned mask = __ballot_sync(0xffffffffu, f_l >= 0 && f_l < limit && a_l != 0.0f);
+    unsigned mask = __ballot_sync(0xffffffffu, f_l >= 0 && f_l < limit);
     while (mask != 0u) {  // (the mask is the same in every lane)
       uint4 w[U][VPT];
       float a[U];

@@ -120,9 +120,11 @@ struct DecodeParams {
   __nv_bfloat16* dxhat;
   float* loss_sum;
   float* row_loss;
+  float* row_part;  // with row_loss: scratch, sparse_decode_segments(d) floats per row
   float* dval;
 };
 int sparse_decode_launch(const DecodeParams& p, cudaStream_t stream);
+int sparse_decode_segments(int d);
 // `wait`: optional (pt.world > 0) bounded wait for the gradient rows of the fused step (phase kPhaseDxhat) at kernel entry
 int sparse_dact_launch(const int* idx, int B, int k, int d, int F, const __nv_bfloat16* W, const __nv_bfloat16* dxhat,
                        float* dval, const PeerTable* wait, uint32_t epoch, int* status, cudaStream_t stream);

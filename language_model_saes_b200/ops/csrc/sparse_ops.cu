@@ -101,7 +101,7 @@ sparse_decode_kernel(const DecodeParams p, int nseg) {
     }
     if (p.label != nullptr) {
       local_sq = warp_sum(local_sq);
-      if (lane == 0 && p.row_loss != nullptr) atomicAdd(p.row_loss + row, local_sq);  // zeroed by the launch
+      if (lane == 0 && p.row_loss != nullptr) p.row_part[item] = local_sq;
       local_sq *= rw;
     }
   }
@@ -116,20 +116,32 @@ sparse_decode_kernel(const DecodeParams p, int nseg) {
   }
 }
 
+// The segments' losses of a row added up in order: the same sum every time.
+__global__ void __launch_bounds__(256)
+row_loss_kernel(const float* __restrict__ part, int B, int nseg, float* __restrict__ row_loss) {
+  const int row = blockIdx.x * 256 + threadIdx.x;
+  if (row >= B) return;
+  float s = 0.0f;
+  for (int i = 0; i < nseg; ++i) s += part[(size_t)row * nseg + i];
+  row_loss[row] = s;
+}
+
+static int decode_vpt(int d) { return d >= 1024 ? 2 : 1; }
+int sparse_decode_segments(int d) { return (d / 8 + 32 * decode_vpt(d) - 1) / (32 * decode_vpt(d)); }
+
 int sparse_decode_launch(const DecodeParams& p, cudaStream_t stream) {
   if (p.d % 8 != 0 || p.d > 8192) return (int)cudaErrorInvalidValue;
   if (p.B <= 0) return 0;
-  if (p.label != nullptr && p.row_loss != nullptr) {
-    cudaError_t e = cudaMemsetAsync(p.row_loss, 0, (size_t)p.B * sizeof(float), stream);
-    if (e != cudaSuccess) return (int)e;
-  }
-  const int vpt = p.d >= 1024 ? 2 : 1;
-  const int nseg = (p.d / 8 + 32 * vpt - 1) / (32 * vpt);
+  const int vpt = decode_vpt(p.d), nseg = sparse_decode_segments(p.d);
   const long long blocks = ((long long)p.B * nseg + DEC_WARPS - 1) / DEC_WARPS;
   if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
   if (vpt == 2) sparse_decode_kernel<2><<<(int)blocks, DEC_WARPS * 32, 0, stream>>>(p, nseg);
   else sparse_decode_kernel<1><<<(int)blocks, DEC_WARPS * 32, 0, stream>>>(p, nseg);
   cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && p.label != nullptr && p.row_loss != nullptr) {
+    row_loss_kernel<<<(p.B + 255) / 256, 256, 0, stream>>>(p.row_part, p.B, nseg, p.row_loss);
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess || p.label == nullptr || p.dval == nullptr) return (int)e;
   // the code gradients need the whole row's d x_hat: a pass of their own over the same decoder rows
   return sparse_dact_launch(p.idx, p.B, p.k, p.d, p.F, p.W, p.dxhat, p.dval, nullptr, 0, nullptr, stream);
