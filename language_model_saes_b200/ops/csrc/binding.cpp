@@ -193,9 +193,11 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
 }
 
 // C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu); na [M] and ends [2, N] (both optional): what
-// topk_estimate takes, made with its bias [N] and gate [N] (both optional)
+// topk_estimate takes, made with its bias [N] and gate [N] (both optional). status: int32 [4], zeroed, of this call alone: a wait in the
+// product that runs out is recorded there, and everything is done on the fp32 pipes then. tensor_cores = false leaves the product out (as if it had given up).
 void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
-               const c10::optional<Tensor>& ends, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate) {
+               const c10::optional<Tensor>& ends, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
+               bool tensor_cores) {
   CHECK_T(A, torch::kFloat32);
   CHECK_T(B, torch::kFloat32);
   CHECK_T(C, torch::kFloat32);
@@ -222,7 +224,7 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
   const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, 3 * kp, 128);
   const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), N, 3 * kp, 128);
   check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), B.data_ptr<float>(), (int)M, (int)N, (int)K, (int)kp, fa, fb, C.data_ptr<float>(), N,
-                                     status.data_ptr<int>(), stream),
+                                     status.data_ptr<int>(), tensor_cores, stream),
              "fp32_gemm launch");
 }
 

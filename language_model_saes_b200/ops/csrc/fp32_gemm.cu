@@ -8,7 +8,8 @@
 //   K 64: 0.8e-7 and 1.3e-7; 256: 1.2e-7 and 2.5e-7; 768: 1.2e-7 and 4.3e-7; 2048: 1.3e-7 and 7.1e-7
 // Bound by the tensor cores, six times the operations of one bf16 product: 4096 x 24576 x 768: 2505 us (library, fp32 pipes) -> 632 us
 // and 37 us for the split. Values that bf16 cannot hold (infinities, NaN, beyond 2^127) mark their row of A or B, and what marked
-// rows take part in is redone on the fp32 pipes.
+// rows take part in is redone on the fp32 pipes. So is everything where a wait of the product ran out: it reports to a status word of its
+// own call, which no other kernel looks at, and the result is as good as ever.
 //
 // Structure: CTA pairs (cta_group::2, 256 x 256 tiles) as in encoder_gemm.cu; a tile passes through the accumulator buffers once per
 // slice. 384 threads: TMA producer, MMA issuer, TMEM owner, and eight epilogue warps that hold 128 columns of a row each.
@@ -288,13 +289,14 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 // C[m, n] of marked rows of A or of B on the fp32 pipes, a warp per element; leaves at once where nothing is marked.
 __global__ void __launch_bounds__(256)
 marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B, int M, int N, int K, const int* __restrict__ fa,
-                       const int* __restrict__ fb, float* __restrict__ C, long long ldc) {
-  if (fa[0] == 0 && fb[0] == 0) return;
+                       const int* __restrict__ fb, float* __restrict__ C, long long ldc, const int* __restrict__ status) {
+  const bool all = status[0] != 0;
+  if (fa[0] == 0 && fb[0] == 0 && !all) return;
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * 8;
   for (long long e = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); e < (long long)M * N; e += warps) {
     const int m = (int)(e / N), n = (int)(e - (long long)m * N);
-    if (fa[1 + m] == 0 && fb[1 + n] == 0) continue;
+    if (!all && fa[1 + m] == 0 && fb[1 + n] == 0) continue;
     float s = 0.0f;
     for (int k = lane; k < K; k += 32) s = fmaf(A[(size_t)m * K + k], B[(size_t)n * K + k], s);
     s = warp_sum(s);
@@ -313,7 +315,7 @@ int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16
 }
 
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
-                     const int* fb, float* C, long long ldc, int* status, cudaStream_t stream) {
+                     const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream) {
   Fp32GemmParams p;
   p.M = M; p.N = N; p.kp = kp; p.C = C; p.ldc = ldc; p.status = status;
   p.m_tiles = (M + 2 * FG_BM - 1) / (2 * FG_BM);
@@ -335,9 +337,9 @@ int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, fp32_gemm_kernel, ta, tb, p);
+  if (tensor_cores) e = cudaLaunchKernelEx(&cfg, fp32_gemm_kernel, ta, tb, p);
   if (e != cudaSuccess) return (int)e;
-  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C, ldc);
+  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C, ldc, status);
   return (int)cudaGetLastError();
 }
 

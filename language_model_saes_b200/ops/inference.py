@@ -51,7 +51,8 @@ def product(x: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
     """``x @ W`` in fp32."""
     rows = x.detach().reshape(-1, x.shape[-1])
     out = torch.empty(rows.shape[0], W.shape[1], dtype=torch.float32, device=x.device)
-    K._ext().fp32_gemm(rows, W.detach().t(), out, K.status_buffer(x.device), None, None, None, None)
+    status = torch.zeros(4, dtype=torch.int32, device=x.device)
+    K._ext().fp32_gemm(rows, W.detach().t(), out, status, None, None, None, None, True)
     return out.view(*x.shape[:-1], W.shape[1])
 
 
@@ -74,9 +75,10 @@ def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, nor
     B, F = rows.shape[0], W.shape[1]
     h, out = (torch.empty(B, F, dtype=torch.float32, device=x.device) for _ in range(2))
     xn, ends = torch.empty(B, dtype=torch.float32, device=x.device), torch.empty(2, F, dtype=torch.int32, device=x.device)
-    todo = torch.zeros(1 + B, dtype=torch.int32, device=x.device)
+    status_todo = torch.zeros(4 + 1 + B, dtype=torch.int32, device=x.device)
+    status, todo = status_todo[:4], status_todo[4:]
     bias, norm = (t.contiguous() if t is not None else None for t in (bias, norm))
-    K._ext().fp32_gemm(rows, W.detach().t(), h, K.status_buffer(x.device), xn, ends, bias, norm)
+    K._ext().fp32_gemm(rows, W.detach().t(), h, status, xn, ends, bias, norm, True)
     K._ext().topk_estimate(h, rows, W.detach().t(), xn, ends, bias, norm, k, todo, out)
     return out.view(*x.shape[:-1], F)
 

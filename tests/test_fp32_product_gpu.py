@@ -157,3 +157,19 @@ def test_rows_with_few_positive_values_cost_no_more_than_others():
                 best = start.elapsed_time(end)
         times.append(best)
     assert times[1] < 3 * times[0], times  # (summed up as whole rows they took thirty times as long)
+
+
+def test_a_product_that_gave_up_is_made_good_and_stops_nothing_else(monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(0)
+    x, w = torch.randn(300, 128, device=DEV, generator=g), torch.randn(1000, 128, device=DEV, generator=g)
+    status = torch.ones(4, dtype=torch.int32, device=DEV)  # a wait ran out, and the tensor cores have written nothing
+    out = torch.full((300, 1000), float("nan"), device=DEV)
+    K._ext().fp32_gemm(x, w, out, status, None, None, None, None, False)
+    want, mass = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((out.double() - want).abs() <= 2.0**-24 * 128 * mass).all()
+
+    def shared(device):
+        raise AssertionError("the status word of the training kernels")
+
+    monkeypatch.setattr(K, "status_buffer", shared)
+    assert torch.isfinite(I.topk_encode(x, w.t(), None, None, 20)).all() and torch.isfinite(I.product(x, w.t())).all()
