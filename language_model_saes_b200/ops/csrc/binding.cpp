@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 #include <map>
@@ -197,7 +198,7 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
 // product that runs out is recorded there, and everything is done on the fp32 pipes then. tensor_cores = false leaves the product out (as if it had given up).
 void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
                const c10::optional<Tensor>& ends, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
-               bool tensor_cores) {
+               bool tensor_cores, int64_t workspace) {
   CHECK_T(A, torch::kFloat32);
   CHECK_T(B, torch::kFloat32);
   CHECK_T(C, torch::kFloat32);
@@ -214,18 +215,30 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
   const c10::cuda::CUDAGuard guard(A.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const auto b16 = A.options().dtype(torch::kBFloat16), i32 = A.options().dtype(torch::kInt32);
-  const Tensor As = torch::empty({M, 3 * kp}, b16), Bs = torch::empty({N, 3 * kp}, b16);
-  const Tensor flags = torch::zeros({M + N + 2}, i32);
+  // B in pieces of whole tiles, so that the parts of a large dictionary (6 bytes an element) need no more than `workspace` bytes
+  int64_t step = N;
+  if (N * kp * 6 > workspace) step = std::max<int64_t>(1, workspace / (kp * 6 * 256)) * 256;
+  step = std::min(step, N);
+  const int64_t steps = (N + step - 1) / step;
+  const Tensor As = torch::empty({M, 3 * kp}, b16), Bs = torch::empty({step, 3 * kp}, b16);
+  const Tensor flags = torch::zeros({1 + M + N + steps}, i32);
   int* fa = flags.data_ptr<int>();
   int* fb = fa + 1 + M;
-  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, opt_ptr<float>(na), nullptr, nullptr, nullptr, stream), "split");
-  check_cuda(lmsae::split_bf16x3_launch(B.data_ptr<float>(), (int)N, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nullptr,
-                                        reinterpret_cast<uint32_t*>(opt_ptr<int>(ends)), opt_ptr<const float>(bias), opt_ptr<const float>(gate), stream), "split");
+  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, opt_ptr<float>(na), nullptr, 0, nullptr, nullptr, stream), "split");
   const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, 3 * kp, 128);
-  const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), N, 3 * kp, 128);
-  check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), B.data_ptr<float>(), (int)M, (int)N, (int)K, (int)kp, fa, fb, C.data_ptr<float>(), N,
-                                     status.data_ptr<int>(), tensor_cores, stream),
-             "fp32_gemm launch");
+  for (int64_t n0 = 0; n0 < N; n0 += step) {
+    const int64_t n = std::min(step, N - n0);
+    const float* Bn = B.data_ptr<float>() + n0 * K;
+    check_cuda(lmsae::split_bf16x3_launch(Bn, (int)n, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nullptr,
+                                          ends.has_value() ? reinterpret_cast<uint32_t*>(ends->data_ptr<int>()) + n0 : nullptr, (int)N,
+                                          bias.has_value() ? bias->data_ptr<float>() + n0 : nullptr, gate.has_value() ? gate->data_ptr<float>() + n0 : nullptr, stream),
+               "split");
+    const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), n, 3 * kp, 128);
+    check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), Bn, (int)M, (int)n, (int)K, (int)kp, fa, fb, C.data_ptr<float>() + n0, N,
+                                       status.data_ptr<int>(), tensor_cores, stream),
+               "fp32_gemm launch");
+    fb += 1 + n;
+  }
 }
 
 // out = topk(relu((h + bias) * norm)) / norm per row, dense fp32 [B, F]

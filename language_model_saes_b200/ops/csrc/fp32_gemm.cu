@@ -49,6 +49,7 @@ __device__ __forceinline__ int part_b(int t) { return (0x021010 >> (4 * (5 - t))
 struct SplitBounds {
   float* norm;
   uint32_t* ends;
+  int ends_stride;
   const float* bias;
   const float* gate;
 };
@@ -103,7 +104,7 @@ split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv
         if (b.ends != nullptr) {
           const float g = plain ? gate : 1.0f;
           b.ends[r] = (__float_as_uint(g) & 0xffff0000u) | bf16_up(n);
-          b.ends[rows + r] = (bf16_up(g) << 16) | bf16_up(n);
+          b.ends[(size_t)b.ends_stride + r] = (bf16_up(g) << 16) | bf16_up(n);
         }
       }
     }
@@ -306,11 +307,11 @@ marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B,
 
 }  // namespace
 
-int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends, const float* bias,
-                        const float* gate, cudaStream_t stream) {
+int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends,
+                        int ends_stride, const float* bias, const float* gate, cudaStream_t stream) {
   if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
-  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, ends, bias, gate});
+  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, ends, ends_stride, bias, gate});
   return (int)cudaGetLastError();
 }
 

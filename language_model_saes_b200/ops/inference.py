@@ -14,6 +14,8 @@ from torch.utils._python_dispatch import _get_current_dispatch_mode
 from . import sae_kernels as K
 
 MAX_K = 1024  # the selection kernel's bound comes from 2048 column groups
+# bytes for the parts of W at a time (6 per element): up to 74 tiles of 256 features at d_model 4096, so that a piece still fills the GPU
+PRODUCT_WORKSPACE = 512 << 20
 MAX_ESTIMATE_WIDTH = 16384  # kEstimateMaxK in csrc/kernels.h
 
 
@@ -52,7 +54,7 @@ def product(x: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
     rows = x.detach().reshape(-1, x.shape[-1])
     out = torch.empty(rows.shape[0], W.shape[1], dtype=torch.float32, device=x.device)
     status = torch.zeros(4, dtype=torch.int32, device=x.device)
-    K._ext().fp32_gemm(rows, W.detach().t(), out, status, None, None, None, None, True)
+    K._ext().fp32_gemm(rows, W.detach().t(), out, status, None, None, None, None, True, PRODUCT_WORKSPACE)
     return out.view(*x.shape[:-1], W.shape[1])
 
 
@@ -78,7 +80,7 @@ def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, nor
     status_todo = torch.zeros(4 + 1 + B, dtype=torch.int32, device=x.device)
     status, todo = status_todo[:4], status_todo[4:]
     bias, norm = (t.contiguous() if t is not None else None for t in (bias, norm))
-    K._ext().fp32_gemm(rows, W.detach().t(), h, status, xn, ends, bias, norm, True)
+    K._ext().fp32_gemm(rows, W.detach().t(), h, status, xn, ends, bias, norm, True, PRODUCT_WORKSPACE)
     K._ext().topk_estimate(h, rows, W.detach().t(), xn, ends, bias, norm, k, todo, out)
     return out.view(*x.shape[:-1], F)
 

@@ -164,7 +164,7 @@ def test_a_product_that_gave_up_is_made_good_and_stops_nothing_else(monkeypatch)
     x, w = torch.randn(300, 128, device=DEV, generator=g), torch.randn(1000, 128, device=DEV, generator=g)
     status = torch.ones(4, dtype=torch.int32, device=DEV)  # a wait ran out, and the tensor cores have written nothing
     out = torch.full((300, 1000), float("nan"), device=DEV)
-    K._ext().fp32_gemm(x, w, out, status, None, None, None, None, False)
+    K._ext().fp32_gemm(x, w, out, status, None, None, None, None, False, 1 << 30)
     want, mass = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert ((out.double() - want).abs() <= 2.0**-24 * 128 * mass).all()
 
@@ -173,3 +173,23 @@ def test_a_product_that_gave_up_is_made_good_and_stops_nothing_else(monkeypatch)
 
     monkeypatch.setattr(K, "status_buffer", shared)
     assert torch.isfinite(I.topk_encode(x, w.t(), None, None, 20)).all() and torch.isfinite(I.product(x, w.t())).all()
+
+
+@pytest.mark.parametrize("M,N,K_", [(257, 1000, 200), (300, 513, 64)])
+def test_a_dictionary_in_pieces(M, N, K_, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn(M, K_, device=DEV, generator=g), torch.randn(N, K_, device=DEV, generator=g)
+    w[N - 3, 1], w[2, 0] = 3e38, float("nan")
+    bias, norm = torch.randn(N, device=DEV, generator=g), torch.rand(N, device=DEV, generator=g) + 0.5
+    whole = I.product(x, w.t()), I.topk_encode(x, w.t(), bias, norm, 9)
+    monkeypatch.setattr(I, "PRODUCT_WORKSPACE", 1)  # one tile at a time
+    for a, b in zip(whole, (I.product(x, w.t()), I.topk_encode(x, w.t(), bias, norm, 9))):
+        assert torch.equal(a.nan_to_num(nan=-1.0), b.nan_to_num(nan=-1.0))
+    # the parts of W: 6 bytes an element of one tile instead of all
+    monkeypatch.setattr(I, "PRODUCT_WORKSPACE", 1 << 20)
+    w = torch.randn(65536, K_, device=DEV, generator=g)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = I.product(x, w.t())
+    assert torch.cuda.max_memory_allocated() - before < out.numel() * 4 + x.numel() * 8 + (4 << 20)
