@@ -461,11 +461,12 @@ class FeatureGroups:
         self.offsets = torch.zeros(F + 1, dtype=torch.int32, device=device)
         self.cursor = torch.zeros(F, dtype=torch.int32, device=device)
         self.entries = torch.zeros(capacity, dtype=torch.int32, device=device)
-        self.block_sums = torch.zeros((F + 4095) // 4096, dtype=torch.int32, device=device)
-        # features with long entry lists (count, then features) and the row counter of the update kernel's launches (left at
-        # zero by every launch; the launches that read these groups follow each other on one stream)
-        self.heavy = torch.zeros(1 + capacity // HEAVY_ROW + 1, dtype=torch.int32, device=device)
-        self.sched = torch.zeros(2, dtype=torch.int32, device=device)
+        # in one piece, which is one fill on a first step: totals of the counting sort's blocks, the row counter of the update
+        # kernel's launches (left at zero by every launch; the launches that read these groups follow each other on one stream)
+        # and the features with long entry lists (count, then features)
+        n_blocks = (F + 4095) // 4096
+        scratch = torch.zeros(n_blocks + 2 + 2 + capacity // HEAVY_ROW, dtype=torch.int32, device=device)
+        self.block_sums, self.sched, self.heavy = scratch[:n_blocks], scratch[n_blocks : n_blocks + 2], scratch[n_blocks + 2 :]
         self.heavy_base = 0
 
     def part(self, lo: int, hi: int) -> "FeatureGroups":
