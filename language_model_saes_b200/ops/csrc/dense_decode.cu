@@ -5,9 +5,9 @@
 // on timing), and all threads then add up the gathered rows of W. Bound by reading acts once (HBM) and the rows of W (L2);
 // 4096 x 24576 x 768 with 50 non-zeros a row: 3073 -> 132 us.
 //
-// Results are those of the dense product also where skipping a zero is not allowed or does not pay: a W that holds an infinity or a
-// NaN (0 * inf is NaN), and rows with more than kWarpList non-zeros in an eighth, are marked and left to a tiled fp32 product that
-// follows and leaves at once where nothing is marked. The decision is taken on the device: the host waits for nothing.
+// Results are those of the dense product also where skipping a zero is not allowed or does not pay: with a W that holds an infinity or
+// a NaN (0 * inf is NaN) all rows, and else rows with more than `most` non-zeros, or more than kWarpList in an eighth, are listed and
+// left to rows_product.cu, which leaves at once where nothing is listed. The decision is taken on the device: the host waits for nothing.
 #include "gather.cuh"
 #include "kernels.h"
 
@@ -34,14 +34,14 @@ nonfinite_kernel(const float* __restrict__ w, long long n, int* __restrict__ fou
 }
 
 __global__ void __launch_bounds__(DD_THREADS, 6)
-sparse_rows_kernel(const float* __restrict__ acts, const float* __restrict__ W, int F, int d, int* __restrict__ marks, float* __restrict__ out) {
+sparse_rows_kernel(const float* __restrict__ acts, const float* __restrict__ W, int F, int d, int most, int* __restrict__ todo, float* __restrict__ out) {
   __shared__ int s_idx[8][kWarpList];
   __shared__ float s_val[8][kWarpList];
   __shared__ int s_n[8];
   __shared__ float4 s_part[DD_THREADS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x;
-  if (marks[0] != 0) {  // (W is not finite)
-    if (threadIdx.x == 0) marks[1 + row] = 1;
+  if (todo[1 + gridDim.x] != 0) {  // (W is not finite)
+    if (threadIdx.x == 0) todo[1 + atomicAdd(todo, 1)] = row;
     return;
   }
   const uint4* a = reinterpret_cast<const uint4*>(acts + (size_t)row * F);
@@ -84,10 +84,16 @@ sparse_rows_kernel(const float* __restrict__ acts, const float* __restrict__ W, 
   if (lane == 0) s_n[warp] = n;
   __syncthreads();
   bool over = false;
+  int all = 0;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) over |= s_n[w] > kWarpList;
-  if (threadIdx.x == 0) marks[1 + row] = over ? 1 : 0;
-  if (over) return;
+  for (int w = 0; w < 8; ++w) {
+    over |= s_n[w] > kWarpList;
+    all += s_n[w];
+  }
+  if (over || all > most) {
+    if (threadIdx.x == 0) todo[1 + atomicAdd(todo, 1)] = row;
+    return;
+  }
   // four columns a thread; with few columns several groups of threads share the entries and add up in a fixed order
   const int cols = d / 4, groups = cols >= DD_THREADS ? 1 : DD_THREADS / cols;
   const int g = groups == 1 ? 0 : (int)threadIdx.x / cols;
@@ -128,72 +134,23 @@ sparse_rows_kernel(const float* __restrict__ acts, const float* __restrict__ W, 
   }
 }
 
-// The marked rows of acts * W: 128 x 64 tiles, eight rows x four columns a thread, sums in ascending order of the features.
-constexpr int DT_M = 128, DT_N = 64, DT_K = 16;
-__global__ void __launch_bounds__(256)
-marked_rows_product_kernel(const float* __restrict__ acts, const float* __restrict__ W, int B, int F, int d, const int* __restrict__ marks,
-                           float* __restrict__ out) {
-  __shared__ float s_a[DT_K][DT_M + 4];
-  __shared__ float s_w[DT_K][DT_N];
-  const int m0 = blockIdx.x * DT_M, n0 = blockIdx.y * DT_N;
-  const int tid = threadIdx.x;
-  const bool mine = tid < DT_M && m0 + tid < B && marks[1 + m0 + tid] != 0;
-  if (!__syncthreads_or(mine)) return;
-  const int tm = (tid / 16) * 8, tn = (tid % 16) * 4;
-  float acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  for (int k0 = 0; k0 < F; k0 += DT_K) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {  // 128 rows x 4 vectors of acts (F % 4 == 0)
-      const int at = tid + i * 256, r = at >> 2, kk = (at & 3) * 4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (m0 + r < B && k0 + kk < F) v = __ldg(reinterpret_cast<const float4*>(acts + (size_t)(m0 + r) * F + k0 + kk));
-      s_a[kk][r] = v.x; s_a[kk + 1][r] = v.y; s_a[kk + 2][r] = v.z; s_a[kk + 3][r] = v.w;
-    }
-    {
-      const int kk = tid / 16, c = (tid % 16) * 4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k0 + kk < F && n0 + c < d) v = __ldg(reinterpret_cast<const float4*>(W + (size_t)(k0 + kk) * d + n0 + c));
-      *reinterpret_cast<float4*>(&s_w[kk][c]) = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < DT_K; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&s_a[kk][tm]), a1 = *reinterpret_cast<const float4*>(&s_a[kk][tm + 4]);
-      const float4 w = *reinterpret_cast<const float4*>(&s_w[kk][tn]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        fma2(acc[i][0], acc[i][1], w.x, w.y, av[i], av[i]);
-        fma2(acc[i][2], acc[i][3], w.z, w.w, av[i], av[i]);
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = m0 + tm + i;
-    if (r < B && marks[1 + r] != 0 && n0 + tn < d)
-      *reinterpret_cast<float4*>(out + (size_t)r * d + n0 + tn) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-  }
-}
-
 }  // namespace
 
-// marks: int [1 + B], marks[0] zeroed by the caller. F % 4 == 0, d % 4 == 0, all pointers 16-byte aligned.
-int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int* marks, float* out, cudaStream_t stream) {
+// todo: int [2 + B + part_tiles], zeroed by the caller: how many rows are left to the product, which, whether W holds an infinity or a
+// NaN, and the product's counters. most: non-zeros up to which a row is gathered. F % 4 == 0, d % 4 == 0, pointers 16-byte aligned.
+int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int most, int* todo, float* part, long long part_floats, int part_tiles,
+                        float* out, cudaStream_t stream) {
   const uintptr_t align = reinterpret_cast<uintptr_t>(acts) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(out);
   if (F % 4 != 0 || d % 4 != 0 || align % 16 != 0 || F <= 0 || d <= 0) return (int)cudaErrorInvalidValue;
   if (B <= 0) return 0;
   const long long n = (long long)F * d;
   const long long blocks = (n / 4 + 255) / 256;
-  nonfinite_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(W, n, marks);
-  sparse_rows_kernel<<<B, DD_THREADS, 0, stream>>>(acts, W, F, d, marks, out);
-  marked_rows_product_kernel<<<dim3((B + DT_M - 1) / DT_M, (d + DT_N - 1) / DT_N), 256, 0, stream>>>(acts, W, B, F, d, marks, out);
-  return (int)cudaGetLastError();
+  nonfinite_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(W, n, todo + 1 + B);
+  sparse_rows_kernel<<<B, DD_THREADS, 0, stream>>>(acts, W, F, d, most, todo, out);
+  RowsProductParams r = {};
+  r.A = acts; r.B = W; r.C = out; r.N = d; r.K = F; r.rows = todo; r.max_rows = B;
+  r.part = part; r.part_floats = part_floats; r.part_done = todo + 2 + B; r.part_tiles = part_tiles;
+  return rows_product_launch(r, true, stream);
 }
 
 }  // namespace lmsae

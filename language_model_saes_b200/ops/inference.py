@@ -86,15 +86,30 @@ def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, nor
 
 
 def sparse_decode_supported(acts: torch.Tensor, W: torch.Tensor) -> bool:
+    """Aligned operands, and a product that takes longer than the kernels that replace it: they need 24 us of launches, which a library
+    product of 1e9 operations exceeds where features are many (256 x 4096 x 512: 67 us), and with few features, of which a token's
+    50 codes are a larger share, one of 4e9 (4096 x 1024 x 256, 2.1e9: 45 against 55 us; 4096 x 1024 x 768, 6.4e9: 137 against 73 us)."""
     F, d = W.shape
-    return (acts.ndim >= 2 and acts.shape[-1] == F and acts.is_contiguous() and W.is_contiguous() and F % 4 == 0 and d % 4 == 0 and F > 0 and d > 0
-            and acts.data_ptr() % 16 == 0 and W.data_ptr() % 16 == 0 and F < 2**31 - 64 and 0 < acts.numel() // F < 2**31 - 64)  # fmt: skip
+    if not (acts.ndim >= 2 and acts.shape[-1] == F and acts.is_contiguous() and W.is_contiguous() and F % 4 == 0 and d % 4 == 0 and F > 0 and d > 0):
+        return False
+    B = acts.numel() // F
+    return (2 * B * F * d >= (1e9 if F >= 4096 else 4e9) and acts.data_ptr() % 16 == 0 and W.data_ptr() % 16 == 0
+            and F < 2**31 - 64 and 0 < B < 2**31 - 64)  # fmt: skip
+
+
+def most_gathered(F: int) -> int:
+    """Non-zeros of a row up to which gathering beats the product of the rows that are left over: 4096 tokens x 2048 x 768, 443 us as a
+    product, 222 us gathered at 12 % and 805 us at 50 % (4096 x 8192 x 768: 1684 us against 793 us at 12 %)."""
+    return F // 6
 
 
 def sparse_decode(acts: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
-    """``acts @ W`` for ``acts [..., F]`` with few non-zeros."""
+    """``acts @ W`` for ``acts [..., F]`` with few non-zeros; rows with more than ``most_gathered`` go to a product on the fp32 pipes."""
     rows = acts.reshape(-1, acts.shape[-1])
-    out = torch.empty(rows.shape[0], W.shape[1], dtype=torch.float32, device=acts.device)
-    marks = torch.zeros(1 + rows.shape[0], dtype=torch.int32, device=acts.device)
-    K._ext().dense_decode(rows, W.detach(), marks, out)
-    return out.view(*acts.shape[:-1], W.shape[1])
+    (B, F), d = rows.shape, W.shape[1]
+    tiles = min(512, -(-B // 128) * -(-d // 128) * 16)
+    out = torch.empty(B, d, dtype=torch.float32, device=acts.device)
+    part = torch.empty(tiles * 128 * 128, dtype=torch.float32, device=acts.device)
+    todo = torch.zeros(2 + B + tiles, dtype=torch.int32, device=acts.device)
+    K._ext().dense_decode(rows, W.detach(), most_gathered(F), todo, part, out)
+    return out.view(*acts.shape[:-1], d)

@@ -50,7 +50,7 @@ def test_topk_activation(F, k, data, parts):
 
 
 @pytest.mark.parametrize("B,F,d", [(1, 4, 4), (130, 1000, 64), (5, 24576, 768), (3, 4100, 1028), (129, 512, 256)])
-@pytest.mark.parametrize("rows", ["sparse", "some dense", "inf weight"])
+@pytest.mark.parametrize("rows", ["sparse", "some dense", "all dense", "at the limit", "inf weight"])
 def test_decoder(B, F, d, rows):
     g = torch.Generator().manual_seed(B + F)
     a = torch.randn(B, F, generator=g) * (torch.rand(B, F, generator=g) < 20 / F)
@@ -58,6 +58,13 @@ def test_decoder(B, F, d, rows):
     if rows == "some dense":
         a[B // 2] = torch.randn(F, generator=g)
         a[0] = 0.0
+    elif rows == "all dense":
+        a = torch.randn(B, F, generator=g)
+    elif rows == "at the limit":  # as many non-zeros as a row that is gathered may have, and one more
+        n = min(I.most_gathered(F), 8 * 256 // 2)
+        a.zero_()
+        a[:, torch.randperm(F, generator=g)[:n]] = 1.5
+        a[::2, (a[0] == 0).nonzero()[0]] = -1.0
     elif rows == "inf weight":
         W[F // 2, 1] = float("inf")
     out = I.sparse_decode(a.to(DEV), W.to(DEV)).cpu()
@@ -96,8 +103,44 @@ def test_model_routes(act):
         assert not sae.encode(x).any() and len(seen) == 1
         sae.hook_hidden_pre.remove_hooks()
         with torch.autocast("cuda", dtype=torch.bfloat16):
-            assert sae.decode(a).dtype == torch.bfloat16 or not sae.cfg.use_decoder_bias or sae.decode(a).dtype == torch.float32
+            assert not sae._rowwise_topk_inference(x) and not sae._sparse_inference(a)
+            assert torch.equal(sae.decode(a), a @ sae.W_D + sae.b_D)
         if act == "topk":
             assert torch.allclose(torch.vmap(lambda t: sae.decode(sae.encode(t)))(x), r, atol=1e-5)
             _, tangent = torch.func.jvp(lambda t: sae.decode(sae.encode(t)), (x,), (torch.ones_like(x),))
             assert tangent.any()
+
+
+@pytest.mark.parametrize("form", ["kernel", "contiguous W_E", "matmul precision"])
+def test_encode_takes_the_estimating_product(form, monkeypatch):
+    """Above the size from which the split product pays, ``encode`` runs it, and only on the operands it is made for."""
+    torch.manual_seed(0)
+    cfg = SAEConfig(hook_point_in="h", hook_point_out="h", d_model=512, expansion_factor=16, act_fn="topk", top_k=20, device=DEV, dtype=torch.float32)
+    sae = SparseAutoEncoder(cfg)
+    sae.init_parameters(encoder_uniform_bound=0.05, decoder_uniform_bound=0.05, init_log_jumprelu_threshold_value=0.0)
+    sae.b_E.data.normal_(0.0, 0.1)
+    if form == "contiguous W_E":
+        sae.W_E = torch.nn.Parameter(sae.W_E.detach().contiguous())
+    x = torch.randn(2, 256, 512, device=DEV)
+    calls = []
+    made = I.topk_encode
+    monkeypatch.setattr(I, "topk_encode", lambda *a: calls.append(1) or made(*a))
+    before = torch.get_float32_matmul_precision()
+    try:
+        if form == "matmul precision":
+            torch.set_float32_matmul_precision("high")
+        with torch.no_grad():
+            acts = sae.encode(x)
+    finally:
+        torch.set_float32_matmul_precision(before)
+    assert len(calls) == (form == "kernel") and acts.shape == (2, 256, 8192)
+    if form == "matmul precision":  # (tf32 codes may differ by more than ties)
+        return
+    norm = sae.decoder_norm().double()
+    h = (x.double() @ sae.W_E.double() + sae.b_E.double()) * norm
+    want = topk(h.clamp_min(0.0), k=20) / norm
+    same = (acts != 0) == (want != 0)
+    # fp32 sums of 512 terms: a choice may differ where the k-th values are that close, which hardly a row has
+    assert (~same).any(-1).float().mean() < 0.01
+    bound = 512 * 2.0**-24 * (x.double().abs() @ sae.W_E.double().abs() + sae.b_E.double().abs())
+    assert ((acts.double() - want).abs() <= bound + 1e-12)[same].all()

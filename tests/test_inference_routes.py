@@ -84,3 +84,11 @@ def test_listeners_of_every_kind_are_called(point, how):
         handle.remove()
         plain = sae.encode(x)
     assert plain.any() and torch.allclose(heard, plain * 2)
+
+
+@pytest.mark.parametrize("B,F,d,kernel", [(256, 1024, 768, False), (4096, 1024, 256, False), (4096, 1024, 768, True), (256, 4096, 512, True),
+                                          (4096, 24576, 768, True), (4096, 24578, 768, False), (1, 131072, 1024, False)])  # fmt: skip
+def test_decoders_below_the_cost_of_the_launches_are_products(B, F, d, kernel):
+    from language_model_saes_b200.ops.inference import sparse_decode_supported
+
+    assert sparse_decode_supported(torch.empty(B, F, device="meta"), torch.empty(F, d, device="meta")) is kernel
