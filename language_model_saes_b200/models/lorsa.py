@@ -403,11 +403,10 @@ class LowRankSparseAttention(SparseDictionary):
         """Fused causal attention: one attention head per QK head whose value / output width is the OV group."""
         b, s, h, _ = q.shape
         if v is None:
-            # tcgen05 kernels (forward, dQ, dK/dV) that take a value width different from the query/key width; the values
-            # are produced straight in the layout the forward kernel reads, [b, h, group, s]: one GEMM, no transpose pass
+            # tcgen05 kernels (forward, dQ, dK/dV) that take a value width different from the query/key width
             assert x is not None
-            vt = (torch.matmul(self.W_V, x.to(self.W_V.dtype).transpose(1, 2)) + self.b_V[:, None]).view(b, h, -1, s)
-            return attention_kernels.causal_attention(q, k, None, 1 / self.attn_scale, vt=vt).reshape(b, s, -1)
+            v = (x.to(self.W_V.dtype) @ self.W_V.T + self.b_V).view(b, s, h, -1)
+            return attention_kernels.causal_attention(q, k, v, 1 / self.attn_scale).reshape(b, s, -1)
         vg = v.view(b, s, h, -1)
         value = vg.permute(0, 2, 1, 3)
         import contextlib

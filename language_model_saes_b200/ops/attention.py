@@ -49,6 +49,12 @@ def supported(q: torch.Tensor, v: torch.Tensor) -> bool:
     )  # fmt: skip
 
 
+def _operand(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels read it: bf16, contiguous, on a 16-byte boundary (a view into another tensor may start off one)."""
+    t = t.detach().to(torch.bfloat16).contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 @torch.no_grad()
 def causal_attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float | None = None,
                          want_lse: bool = False) -> tuple[torch.Tensor, torch.Tensor | None]:  # fmt: skip
@@ -58,12 +64,21 @@ def causal_attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scal
         out, lse = ref_causal_attention(q, k, v, scale)
         return out.to(torch.bfloat16), (lse if want_lse else None)
     b, s, h, _ = q.shape
-    q16, k16 = q.to(torch.bfloat16).contiguous(), k.to(torch.bfloat16).contiguous()
-    vt = v.to(torch.bfloat16).permute(0, 2, 3, 1).contiguous()  # [b, h, d_v, s]: keys contiguous for the P V product
+    q16, k16, v16 = (_operand(t) for t in (q, k, v))
     out = torch.empty(b, s, h, v.shape[-1], dtype=torch.bfloat16, device=q.device)
     lse = torch.empty(b, h, s, dtype=torch.float32, device=q.device) if want_lse else None
-    K._ext().attn_fwd(q16, k16, vt, out, lse, float(scale), K.status_buffer(q.device))
+    K._ext().attn_fwd(q16, k16, v16, out, lse, float(scale), K.status_buffer(q.device))
     return out, lse
+
+
+def causal_attention_bwd(q16, k16, v16, do16, lse, delta, scale: float, dtype: torch.dtype):
+    """``(dq, dk, dv)`` in ``dtype`` (fp32, or bf16: fp32 sums rounded once) from contiguous bf16 ``[b, s, h, *]`` tensors and the row
+    statistics ``lse``, ``delta [b, h, s]`` (``delta`` the dot products of output and output gradient). Two kernels."""
+    dq, dk, dv = (torch.empty(t.shape, dtype=dtype, device=t.device) for t in (q16, k16, v16))
+    ext = K._ext()
+    ext.launches += 1  # two kernels in one entry point
+    ext.attn_bwd(q16, k16, v16, do16, lse, delta, dq, dk, dv, float(scale), K.status_buffer(q16.device))
+    return dq, dk, dv
 
 
 class CausalAttention(torch.autograd.Function):
@@ -71,19 +86,12 @@ class CausalAttention(torch.autograd.Function):
     rounded to bf16 for the tensor cores; gradients are accumulated in fp32 and returned in the inputs' dtypes."""
 
     @staticmethod
-    def forward(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float, v_is_transposed: bool = False) -> torch.Tensor:
-        q16, k16 = (t.detach().to(torch.bfloat16).contiguous() for t in (q, k))
+    def forward(ctx, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
+        q16, k16, v16 = (_operand(t) for t in (q, k, v))
         b, s, h, _ = q16.shape
-        if v_is_transposed:  # the caller produced V^T [b, h, d_v, s] directly (no transpose pass in the forward)
-            vt = v.detach().to(torch.bfloat16).contiguous()
-            v16 = vt.permute(0, 3, 1, 2).contiguous()  # the backward kernels read V rows ([b, s, h, d_v])
-        else:
-            v16 = v.detach().to(torch.bfloat16).contiguous()
-            vt = v16.permute(0, 2, 3, 1).contiguous()
-        ctx.v_is_transposed = v_is_transposed
-        out = torch.empty(b, s, h, v16.shape[-1], dtype=torch.bfloat16, device=q.device)
+        out = torch.empty(v16.shape, dtype=torch.bfloat16, device=q.device)
         lse = torch.empty(b, h, s, dtype=torch.float32, device=q.device)
-        K._ext().attn_fwd(q16, k16, vt, out, lse, float(scale), K.status_buffer(q.device))
+        K._ext().attn_fwd(q16, k16, v16, out, lse, float(scale), K.status_buffer(q.device))
         ctx.save_for_backward(q16, k16, v16, out, lse)
         ctx.scale, ctx.dtypes = float(scale), (q.dtype, k.dtype, v.dtype)
         return out.to(v.dtype)
@@ -91,32 +99,21 @@ class CausalAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout: torch.Tensor):
         q16, k16, v16, out, lse = ctx.saved_tensors
-        do16 = dout.to(torch.bfloat16).contiguous()
-        delta = (do16.float() * out.float()).sum(dim=-1).permute(0, 2, 1).contiguous()  # [b, h, s]
-        qt = q16.permute(0, 2, 3, 1).contiguous()
-        kt = k16.permute(0, 2, 3, 1).contiguous()
-        dot = do16.permute(0, 2, 3, 1).contiguous()
-        dq = torch.empty(q16.shape, dtype=torch.float32, device=q16.device)
-        dk = torch.empty_like(dq)
-        dv = torch.empty(v16.shape, dtype=torch.float32, device=q16.device)
-        ext = K._ext()
-        ext.launches += 1  # two kernels in one entry point
-        ext.attn_bwd(q16, k16, v16, do16, qt, kt, dot, lse, delta, dq, dk, dv, ctx.scale, K.status_buffer(q16.device))
-        if ctx.v_is_transposed:
-            dv = dv.permute(0, 2, 3, 1)
-        return dq.to(ctx.dtypes[0]), dk.to(ctx.dtypes[1]), dv.to(ctx.dtypes[2]), None, None
+        do16 = _operand(dout)
+        delta = torch.empty_like(lse)
+        K._ext().attn_delta(do16, out, delta)
+        low = all(t == torch.bfloat16 for t in ctx.dtypes)
+        dq, dk, dv = causal_attention_bwd(q16, k16, v16, do16, lse, delta, ctx.scale, torch.bfloat16 if low else torch.float32)
+        return dq.to(ctx.dtypes[0]), dk.to(ctx.dtypes[1]), dv.to(ctx.dtypes[2]), None
 
 
 def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor | None = None, scale: float | None = None,
                      vt: torch.Tensor | None = None) -> torch.Tensor:  # fmt: skip
     """Differentiable causal attention ``[b, s, h, d_qk] x [b, s, h, d_v] -> [b, s, h, d_v]``; the tensor-core kernels
     when the shape is supported on a GPU, the torch oracle otherwise. The values may be given transposed instead, as
-    ``vt [b, h, d_v, s]`` (what the forward kernel reads), which saves a transpose pass when the caller can produce
-    that layout directly."""
+    ``vt [b, h, d_v, s]``."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else scale
     if vt is not None:
-        if supported(q, vt.permute(0, 3, 1, 2)):
-            return CausalAttention.apply(q, k, vt, scale, True)
         v = vt.permute(0, 3, 1, 2)
     if not supported(q, v):
         return ref_causal_attention(q, k, v, scale)[0].to(v.dtype)

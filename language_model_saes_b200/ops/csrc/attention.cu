@@ -7,16 +7,16 @@
 // Forward (attn_fwd_kernel): one CTA per (128-query block, head, value chunk of DV columns, batch element); four warps
 // whose thread r owns query row r (= TMEM lane r) and a fifth warp that issues the TMA loads and the MMAs.
 //   per 128-key block (causal: only blocks up to the diagonal):
-//     TMA      K block [128 x DQK] and V^T block [DV x 128] (both K-major, 128-byte swizzle) -> shared memory
+//     TMA      K block [128 x DQK] and V block [128 x DV] (64-column atoms, 128-byte swizzle) -> shared memory
 //     tcgen05  S = Q K^T            (128 x 128 x DQK, accumulator in TMEM columns [0, 128))
 //     threads  read their S row from TMEM, online softmax in the exp2 domain, write P as bf16 into shared memory in the
 //              swizzled K-major layout the tensor core reads
 //     tcgen05  O += P V             (128 x DV x 128, TMEM columns [128, 128 + DV))
 //              (accumulating in TMEM; the rows rescale it in place only when their maximum has grown a lot)
 //   epilogue: O / l as bf16, log-sum-exp per row for the backward pass.
-// V is consumed as V^T [batch, heads, d_v, seq] so that both operands of P V are K-major (keys contiguous).
+// V is read as it is, [batch, seq, heads, d_v], as the MN-major operand of P V: no transposed copy of it exists.
 // Every mbarrier wait is bounded; on expiry the CTA records a status code, stops issuing work and frees its TMEM.
-#include "common.cuh"
+#include "gather.cuh"
 #include "kernels.h"
 
 namespace lmsae {
@@ -25,7 +25,6 @@ namespace {
 
 constexpr int ATT_BM = 128;  // queries per CTA
 constexpr int ATT_BN = 128;  // keys per block
-constexpr int ATT_THREADS = 128;
 constexpr int ATOM_BYTES_128 = 128 * 128;  // 128 rows x 64 bf16
 
 template <int DQK, int DV>
@@ -33,9 +32,8 @@ struct AttnSmem {
   static constexpr int kQOff = 0;
   static constexpr int kQBytes = (DQK / 64) * ATOM_BYTES_128;
   static constexpr int kKOff = kQOff + kQBytes;        // two K buffers
-  static constexpr int kVOff = kKOff + 2 * kQBytes;    // two V^T buffers
-  static constexpr int kVAtomBytes = DV * 128;         // DV rows x 64 keys
-  static constexpr int kVBytes = 2 * kVAtomBytes;
+  static constexpr int kVOff = kKOff + 2 * kQBytes;    // two V buffers
+  static constexpr int kVBytes = (DV / 64) * ATOM_BYTES_128;  // atoms of 128 keys x 64 columns
   static constexpr int kPOff = kVOff + 2 * kVBytes;    // two P buffers
   static constexpr int kPBytes = 2 * ATOM_BYTES_128;
   static constexpr int kXchOff = kPOff + 2 * kPBytes;  // float [2][4][128]: row statistics exchanged between column quarters
@@ -92,12 +90,12 @@ constexpr float kRescaleSlack = 8.0f;  // log2 units the running reference may l
 
 // Persistent: one CTA per SM walks a list of tiles (query block, head, value chunk, batch element), longest first, so
 // that the loads and first MMAs of the next tile run while the softmax warps finish and store the current one.
-// K, V^T, P (shared memory) and S (TMEM) are double-buffered over the sequence of key blocks of ALL tiles of the CTA:
+// K, V, P (shared memory) and S (TMEM) are double-buffered over the sequence of key blocks of ALL tiles of the CTA:
 // the g-th key block uses buffer g & 1 and completes phase g >> 1 of that buffer's barriers. The output accumulator is
 // double-buffered over tiles (tile t uses buffer t & 1). Roles and hand-offs (mbarriers and 64-thread named barriers; no
 // CTA-wide barrier inside the loops):
 //   issuer   loads two key blocks ahead inside a tile; S(g+1) is computed while the rows work on S(g); P V (g) as soon
-//            as P(g) is written; a K / V^T buffer is refilled when S / P V of its previous block has consumed it.
+//            as P(g) is written; a K / V buffer is refilled when S / P V of its previous block has consumed it.
 //   rows     four threads per query row, one per quarter of the 128 keys of a block (sixteen warps: the softmax work is
 //            latency-bound, so the warps are there to hide each other's TMEM loads and barrier polls): S(g) TMEM -> 32
 //            registers, release the S buffer; the four exchange their maxima through shared memory; the output accumulator stays in TMEM
@@ -108,7 +106,7 @@ constexpr float kRescaleSlack = 8.0f;  // log2 units the running reference may l
 template <int DQK, int DV>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_vt, const AttnParams p) {
+                const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
   using L = AttnSmem<DQK, DV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -181,8 +179,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const int u = (g0 + kb) & 1;
           mbar_arrive_expect_tx(&bar_k[u], L::kQBytes);
           for (int a = 0; a < DQK / 64; ++a)
-            tma_load_2d(smem + L::kKOff + u * L::kQBytes + a * ATOM_BYTES_128, &tmap_k, &bar_k[u], head * DQK + a * 64,
-                        batch * p.seq + kb * ATT_BN);
+            tma_load_3d(smem + L::kKOff + u * L::kQBytes + a * ATOM_BYTES_128, &tmap_k, &bar_k[u], head * DQK + a * 64, kb * ATT_BN, batch);
         };
         auto load_v = [&](int kb) -> bool {
           const uint32_t g = g0 + kb;
@@ -190,9 +187,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           // the buffer's previous block is g - 2: its P V must have read it
           if (g >= 2 && !mbar_wait_bounded(&bar_pv_done[u], ((g - 2) >> 1) & 1, abort_flag)) return false;
           mbar_arrive_expect_tx(&bar_v[u], L::kVBytes);
-          for (int a = 0; a < 2; ++a)
-            tma_load_2d(smem + L::kVOff + u * L::kVBytes + a * L::kVAtomBytes, &tmap_vt, &bar_v[u], kb * ATT_BN + a * 64,
-                        (batch * p.heads + head) * p.dv + dv0);
+          for (int a = 0; a < DV / 64; ++a)
+            tma_load_3d(smem + L::kVOff + u * L::kVBytes + a * ATOM_BYTES_128, &tmap_v, &bar_v[u], head * p.dv + dv0 + a * 64, kb * ATT_BN, batch);
           return true;
         };
         auto issue_s = [&](int kb) {
@@ -212,7 +208,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         where = 1;
         mbar_arrive_expect_tx(bar_q, L::kQBytes);
         for (int a = 0; a < DQK / 64; ++a)
-          tma_load_2d(smem + L::kQOff + a * ATOM_BYTES_128, &tmap_q, bar_q, head * DQK + a * 64, batch * p.seq + q0);
+          tma_load_3d(smem + L::kQOff + a * ATOM_BYTES_128, &tmap_q, bar_q, head * DQK + a * 64, q0, batch);
         load_k(0);
         if (n_kblocks > 1) load_k(1);
         ok = load_v(0);
@@ -252,13 +248,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           ok = mbar_wait_bounded(&bar_p_full[u], ph, abort_flag) && mbar_wait_bounded(&bar_v[u], ph, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          constexpr uint32_t idesc_o = make_idesc_bf16(ATT_BM, DV);
+          constexpr uint32_t idesc_o = make_idesc_bf16(ATT_BM, DV, false, true);
 #pragma unroll
           for (int kk = 0; kk < ATT_BN / 16; ++kk) {
             const uint32_t pa = smem_u32(smem + L::kPOff + u * L::kPBytes + (kk / 4) * ATOM_BYTES_128);
-            const uint32_t va = smem_u32(smem + L::kVOff + u * L::kVBytes + (kk / 4) * L::kVAtomBytes);
-            umma_bf16_ss(tmem_o, make_sw128_kmajor_desc(pa) + (uint64_t)((kk % 4) * 2),
-                         make_sw128_kmajor_desc(va) + (uint64_t)((kk % 4) * 2), idesc_o, (kb > 0 || kk > 0) ? 1u : 0u);
+            const uint32_t va = smem_u32(smem + L::kVOff + u * L::kVBytes) + kk * 2048;  // sixteen keys a step
+            umma_bf16_ss(tmem_o, make_sw128_kmajor_desc(pa) + (uint64_t)((kk % 4) * 2), make_sw128_mnmajor_desc(va, ATOM_BYTES_128), idesc_o,
+                         (kb > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(&bar_pv_done[u]);
           // the V buffer of the previous block is free once its P V has completed (it ran before this one): refill it
@@ -454,7 +450,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 }
 
 template <int DQK, int DV>
-static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tvt,
+static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                                     const AttnParams& p, cudaStream_t stream) {
   using L = AttnSmem<DQK, DV>;
   static_assert(L::kDynamicBytes <= 232448, "shared memory of one CTA exceeds 227 KB");
@@ -470,7 +466,7 @@ static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk
   const long long tiles = (long long)((p.seq + ATT_BM - 1) / ATT_BM) * p.heads * (p.dv / DV) * p.batch;
   if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
   const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  kern<<<grid, FWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tvt, p);
+  kern<<<grid, FWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -478,19 +474,27 @@ int attn_value_chunk(int dv) { return dv % 128 == 0 ? 128 : (dv % 64 == 0 ? 64 :
 
 // =============================================================================================================
 // Backward. With P = softmax(scale * Q K^T) (causal), O = P V, D = rowsum(dO * O):
-//   dV = P^T dO,   dP = dO V^T,   dS = P * (dP - D) * scale,   dQ = dS K,   dK = dS^T Q.
-// Two kernels, both built from the same pieces as the forward pass and with every MMA operand K-major (the host
-// passes transposed copies K^T, Q^T, dO^T [batch, heads, width, seq] where a product contracts over positions):
-//   attn_bwd_dq_kernel   one CTA per query block; per key block: S and dP on the tensor cores (dP contracts over
-//                        the FULL value width, streamed through a two-stage ring of 64-column atoms), the threads
-//                        (one query row each) form dS, and dQ += dS K accumulates in TMEM over the key blocks.
-//   attn_bwd_dkv_kernel  one CTA per key block (and value chunk); per query block: S^T = K Q^T and dP^T = V dO^T, the
-//                        threads (one key row each) form P^T and dS^T, and dV += P^T dO, dK += dS^T Q accumulate in
-//                        TMEM over the query blocks.
+//   dV = P^T dO,   dP = dO V^T,   dS = P * (dP - D),   dQ = scale * dS K,   dK = scale * dS^T Q.
+// Two persistent kernels of the same build (one CTA per SM, tiles dealt out longest first):
+//   attn_bwd_dq_kernel   a tile is a query block and walks its key blocks:   dQ += dS K
+//   attn_bwd_dkv_kernel  a tile is a key block (and value chunk) and walks its query blocks:   dV += P^T dO,  dK += dS^T Q
+// In both, every step computes S = Q K^T and dP = dO V^T of one 128 x 128 block with queries in the TMEM lanes, so that the row
+// statistics are one value per thread, and every operand is read from the row-major tensors: where a product contracts over
+// positions its tile is a MN-major operand of the same shared-memory copy (P and dS as MN-major A, Q, K and dO as MN-major B), so
+// that no transposed copies of Q, K, dO and V exist.
+//   warps 0-15  softmax rows: four threads per query row, 32 key columns each. S and dP go from TMEM to registers at once, which
+//               frees both buffers: the tensor core computes the next block's while these warps work on exponentials. P and
+//               dS (bf16, two 64-key swizzle atoms) are kept packed in registers until the MMAs of the previous block have read the buffer.
+//   warp 16     TMA producer; warp 17 the MMA issuer: S(g), dP(g), then the accumulating products of block g - 1
+// A finished tile is stored one block late (after the first block of the next tile), so that nothing waits for its last product.
+// What bounds a block: 1024 cycles of exponentials (16 a cycle and SM) against 1024 (dQ) or 1536 (dK/dV) cycles of MMAs at
+// d_qk 64, d_v 128; measured about 3400 and 5200 (hand-offs between the three roles, and tiles of four and a half blocks on average).
+// 2 x 64 heads x 1024 positions, d_qk 64, d_v 128: dQ 146 -> 61 us, dK/dV 226 -> 97 us against kernels of four warps that took turns with
+// the tensor core, and about 250 us of transposed copies and conversions around them are gone.
 // =============================================================================================================
 namespace {
 
-// D[tmem] (+)= A * B^T over K = 16 * steps, both tiles made of 64-column swizzle atoms `a_atom` / `b_atom` bytes apart.
+// D[tmem] (+)= A * B^T over 16 * steps of K, both tiles K-major, made of 64-column swizzle atoms `a_atom` / `b_atom` bytes apart.
 __device__ __forceinline__ void issue_mma_atoms(uint32_t tmem_d, uint32_t a_base, uint32_t a_atom, uint32_t b_base,
                                                 uint32_t b_atom, int steps, uint32_t idesc, bool accumulate) {
   for (int kk = 0; kk < steps; ++kk) {
@@ -500,85 +504,147 @@ __device__ __forceinline__ void issue_mma_atoms(uint32_t tmem_d, uint32_t a_base
   }
 }
 
-template <int DQK>
-struct BwdDqSmem {
-  // with 64-wide queries there is room for two K / K^T buffers: the next key block's tiles (and the first dO / V atom)
-  // are fetched while the threads work on the current one
-  static constexpr bool kDouble = DQK == 64;
-  static constexpr int kKBufs = kDouble ? 2 : 1;
-  static constexpr int kQBytes = (DQK / 64) * ATOM_BYTES_128;
-  static constexpr int kQOff = 0;
-  static constexpr int kKOff = kQOff + kQBytes;
-  static constexpr int kKtAtomBytes = DQK * 128;
-  static constexpr int kKtOff = kKOff + kKBufs * kQBytes;
-  static constexpr int kDsOff = kKtOff + kKBufs * 2 * kKtAtomBytes;
-  static constexpr int kRingOff = kDsOff + 2 * ATOM_BYTES_128;  // 2 stages x {dO atom, V atom}
-  static constexpr int kBarOff = kRingOff + 4 * ATOM_BYTES_128;
-  static constexpr int kNumBars = 9;
+constexpr int BWD_THREADS = FWD_ROW_THREADS + 64;  // sixteen row warps, the producer and the issuer
+constexpr int AB = ATOM_BYTES_128;
+
+// Shared memory of both kernels in atoms of 128 rows x 64 columns. FIX: the pair of tiles a CTA keeps for a whole tile (Q and dO, or
+// K and V), WALK: the ones that change from block to block. A walking Q / K tile is in use from its S to the accumulating product of
+// its block, one block later: three buffers keep the loads ahead. Fixed value tiles wider than two atoms are streamed through
+// their two slots, once per block.
+template <int DQK, bool DKV>
+struct BwdSmem {
+  static constexpr int kQkAtoms = DQK / 64;
+  static constexpr int kFixBufs = DQK == 64 && !DKV ? 2 : 1;
+  static constexpr int kWalkBufs = DQK == 64 ? 3 : (DKV ? 1 : 2);
+  static constexpr int kFixValSlots = 2, kWalkValSlots = 4;
+  static constexpr int kFixOff = 0;
+  static constexpr int kWalkOff = kFixOff + kFixBufs * kQkAtoms * AB;
+  static constexpr int kFixValOff = kWalkOff + kWalkBufs * kQkAtoms * AB;
+  static constexpr int kWalkValOff = kFixValOff + kFixValSlots * AB;
+  static constexpr int kDsOff = kWalkValOff + kWalkValSlots * AB;
+  static constexpr int kPOff = kDsOff + 2 * AB;
+  static constexpr int kBarOff = kPOff + (DKV ? 2 * AB : 0);
+  static constexpr int kNumBars = 2 * (kFixBufs + kWalkBufs + kFixValSlots + kWalkValSlots) + 6;
   static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
   static constexpr int kAbortOff = kTmemPtrOff + 4;
   static constexpr int kDynamicBytes = kAbortOff + 4 + 1024;
 };
 
-template <int DQK, int DVC>
-struct BwdDkvSmem {
-  // with 64-wide queries there is room for two Q buffers: the next query block's Q tile (and the first V / dO atom) are
-  // fetched while the threads work on the current one
-  static constexpr bool kDouble = DQK == 64;
-  static constexpr int kQBufs = kDouble ? 2 : 1;
-  static constexpr int kKBytes = (DQK / 64) * ATOM_BYTES_128;
-  static constexpr int kKOff = 0;
-  static constexpr int kQOff = kKOff + kKBytes;              // Q_i, later Q_i^T (same size), per buffer
-  static constexpr int kQtAtomBytes = DQK * 128;
-  static constexpr int kRingOff = kQOff + kQBufs * kKBytes;  // 2 stages x {V atom, dO atom}; later dO^T chunk
-  static constexpr int kDotAtomBytes = DVC * 128;
-  static constexpr int kPtOff = kRingOff + 4 * ATOM_BYTES_128;
-  static constexpr int kDstOff = kPtOff + 2 * ATOM_BYTES_128;
-  static constexpr int kLseOff = kDstOff + 2 * ATOM_BYTES_128;
-  static constexpr int kDeltaOff = kLseOff + 128 * 4;
-  static constexpr int kBarOff = kDeltaOff + 128 * 4;
-  static constexpr int kNumBars = 10;
-  static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
-  static constexpr int kAbortOff = kTmemPtrOff + 4;
-  static constexpr int kDynamicBytes = kAbortOff + 4 + 1024;
+struct BwdBars {
+  uint64_t *fix_full, *fix_free, *walk_full, *walk_free, *fval_full, *fval_free, *wval_full, *wval_free;
+  uint64_t *sdp_full;  // S and dP of a block are in TMEM
+  uint64_t *sdp_free;  // the rows have read them
+  uint64_t *out_full;  // the rows have written dS (and P)
+  uint64_t *out_free;  // the block's accumulating products are done
+  uint64_t *acc_free;  // [2] the rows have stored a finished tile
 };
+
+template <class L>
+__device__ __forceinline__ BwdBars bwd_bars(uint8_t* smem) {
+  uint64_t* b = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
+  BwdBars r;
+  r.fix_full = b; b += L::kFixBufs;
+  r.fix_free = b; b += L::kFixBufs;
+  r.walk_full = b; b += L::kWalkBufs;
+  r.walk_free = b; b += L::kWalkBufs;
+  r.fval_full = b; b += L::kFixValSlots;
+  r.fval_free = b; b += L::kFixValSlots;
+  r.wval_full = b; b += L::kWalkValSlots;
+  r.wval_free = b; b += L::kWalkValSlots;
+  r.sdp_full = b; r.sdp_free = b + 1; r.out_full = b + 2; r.out_free = b + 3; r.acc_free = b + 4;
+  return r;
+}
+
+// One block's share of a thread: 32 key columns of its query row -> P and dS (unscaled), packed to bf16 pairs.
+// `last`: columns 0 .. last are visible (31 or more: all of them).
+template <bool WANT_P, bool MASK>
+__device__ __forceinline__ void bwd_columns(const uint32_t (&rs)[32], const uint32_t (&rp)[32], float scale_log2, float neg_lse2, float neg_delta,
+                                            int last, uint32_t (&pk)[16], uint32_t (&dk)[16]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    float a0, a1, d0 = neg_delta, d1 = neg_delta;
+    fma_f32x2(a0, a1, __uint_as_float(rs[j]), __uint_as_float(rs[j + 1]), scale_log2, neg_lse2);
+    float p0 = exp2f(a0), p1 = exp2f(a1);
+    add_f32x2(d0, d1, __uint_as_float(rp[j]), __uint_as_float(rp[j + 1]));
+    if constexpr (MASK) {
+      if (j > last) { p0 = 0.0f; d0 = 0.0f; }
+      if (j + 1 > last) { p1 = 0.0f; d1 = 0.0f; }
+    }
+    if constexpr (WANT_P) pk[j / 2] = pack_bf16x2(p0, p1);
+    dk[j / 2] = pack_bf16x2(p0 * d0, p1 * d1);
+  }
+}
+template <bool WANT_P>
+__device__ __forceinline__ void bwd_block(const uint32_t (&rs)[32], const uint32_t (&rp)[32], float scale_log2, float neg_lse2, float neg_delta,
+                                          int last, uint32_t (&pk)[16], uint32_t (&dk)[16]) {
+  // (only the diagonal and the last block have anything to mask: the branch is the same for the whole warp)
+  if (__any_sync(0xffffffffu, last < 31)) bwd_columns<WANT_P, true>(rs, rp, scale_log2, neg_lse2, neg_delta, last, pk, dk);
+  else bwd_columns<WANT_P, false>(rs, rp, scale_log2, neg_lse2, neg_delta, last, pk, dk);
+}
+
+// 32 packed columns of a row to its two-atom tile: 16-byte chunks (cq % 2) * 4 .. + 3 of atom cq / 2.
+__device__ __forceinline__ void bwd_store(uint8_t* tile, int row, int cq, const uint32_t (&v)[16]) {
+  uint8_t* atom = tile + (cq >> 1) * AB;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<uint4*>(atom + sw128_chunk_off(row, (cq & 1) * 4 + i)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+
+// 32 accumulator columns of a thread's lane, times `mul`, to global memory (fp32, or bf16 in one rounding).
+__device__ __forceinline__ void bwd_emit(uint32_t taddr, float mul, void* base, size_t offset, bool bf16_out, bool row_ok) {
+  uint32_t r[32];
+  tmem_ld_32x32b_x32(taddr, r);
+  tmem_wait_ld();
+  if (!row_ok) return;
+  if (bf16_out) {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(base) + offset;
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+      *reinterpret_cast<uint4*>(dst + i) =
+          make_uint4(pack_bf16x2(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul),
+                     pack_bf16x2(__uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul),
+                     pack_bf16x2(__uint_as_float(r[i + 4]) * mul, __uint_as_float(r[i + 5]) * mul),
+                     pack_bf16x2(__uint_as_float(r[i + 6]) * mul, __uint_as_float(r[i + 7]) * mul));
+  } else {
+    float* dst = reinterpret_cast<float*>(base) + offset;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4)
+      *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul,
+                                                        __uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul);
+  }
+}
 
 }  // namespace
 
-template <int DQK>
-__global__ void __launch_bounds__(ATT_THREADS)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                   const __grid_constant__ CUtensorMap tmap_kt, const __grid_constant__ CUtensorMap tmap_do,
-                   const __grid_constant__ CUtensorMap tmap_v, const AttnBwdParams p) {
-  using L = BwdDqSmem<DQK>;
+// DVC: value columns of a tile's dV (dK/dV kernel; its chunks other than the first leave dK alone), 0 for the dQ kernel.
+template <int DQK, int DVC>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do, const AttnBwdParams p) {
+  constexpr bool DKV = DVC != 0;
+  using L = BwdSmem<DQK, DKV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* bar_q = bars + 0;
-  uint64_t* bar_k = bars + 1;      // [2]
-  uint64_t* bar_mma1 = bars + 3;
-  uint64_t* bar_mma2 = bars + 4;
-  uint64_t* ring_full = bars + 5;  // [2]
-  uint64_t* ring_free = bars + 7;  // [2]
+  const BwdBars B = bwd_bars<L>(smem);
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kTmemPtrOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbortOff);
+  constexpr int QK_BYTES = L::kQkAtoms * AB;
 
   const int warp = threadIdx.x >> 5;
-  const int n_qblocks = (p.seq + ATT_BM - 1) / ATT_BM;
-  const int qblk = n_qblocks - 1 - (int)blockIdx.x;
-  const int head = (int)blockIdx.y, batch = (int)blockIdx.z;
-  const int q0 = qblk * ATT_BM;
-  const int row = (int)threadIdx.x;
-  const int qpos = q0 + row;
-  const bool row_ok = qpos < p.seq;
+  const int n_blocks = (p.seq + 127) / 128;
+  const int chunks = DKV ? p.dv / (DKV ? DVC : 1) : 1;
+  const int per_block = p.heads * chunks * p.batch;
+  const int n_tiles = n_blocks * per_block;
   const int dv_atoms = p.dv / 64;
+  const bool stream_fix = dv_atoms > L::kFixValSlots;  // the fixed value tile does not fit: once per block instead
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < L::kNumBars; ++i) mbar_init(&bars[i], 1);
+    for (uint64_t* b = B.fix_full; b < B.fix_full + L::kNumBars; ++b)
+      mbar_init(b, b == B.sdp_free || b == B.out_full || b >= B.acc_free ? FWD_ROW_WARPS : 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 0) {
+  if (warp == FWD_ROW_WARPS + 1) {
     tmem_alloc(tmem_ptr_smem, 512);
     tmem_relinquish();
   }
@@ -586,486 +652,338 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  const uint32_t tmem_s = tmem_base, tmem_dp = tmem_base + 128, tmem_dq = tmem_base + 256;
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+  const uint32_t tmem_s = tmem_base, tmem_dp = tmem_base + 128, tmem_acc = tmem_base + 256;  // acc: dQ of two tiles, or dV and dK
 
-  const size_t stat = ((size_t)batch * p.heads + head) * p.seq + (row_ok ? qpos : 0);
-  const float lse2 = row_ok ? p.lse[stat] * 1.4426950408889634f : INFINITY;  // +inf: every probability of the row is 0
-  const float delta = row_ok ? p.delta[stat] : 0.0f;
+  // tile w: the block it belongs to (those with the longest walks first), then batch, head, value chunk
+  struct Tile { int blk, head, chunk, batch, first, steps; };
+  auto decode = [&](int w) {
+    Tile t;
+    const int i = w / per_block;
+    int r = w - i * per_block;
+    t.batch = r / (p.heads * chunks);
+    r -= t.batch * (p.heads * chunks);
+    t.head = r / chunks;
+    t.chunk = r - t.head * chunks;
+    t.blk = DKV ? i : n_blocks - 1 - i;
+    t.first = DKV ? t.blk : 0;                          // first block of the walk
+    t.steps = DKV ? n_blocks - t.blk : t.blk + 1;
+    return t;
+  };
+  // order in which a block's value atoms are used: the chunk's own last (they stay for dV)
+  auto atom_at = [&](const Tile& t, int i) {
+    if constexpr (!DKV) return i;
+    const int a = t.chunk * (DVC / 64) + DVC / 64 + i;
+    return a < dv_atoms ? a : a - dv_atoms;
+  };
 
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(bar_q, L::kQBytes);
-    for (int a = 0; a < DQK / 64; ++a)
-      tma_load_2d(smem + L::kQOff + a * ATOM_BYTES_128, &tmap_q, bar_q, head * DQK + a * 64, batch * p.seq + q0);
-  }
-
-  const int n_kblocks = qblk + 1;
-  uint32_t ring_n = 0;  // atom steps issued so far (thread 0 only)
-  bool ok = true;
-  for (int kb = 0; kb < n_kblocks && ok; ++kb) {
-    const int k0 = kb * ATT_BN;
-    const uint32_t parity = kb & 1;
-    const int ub = L::kDouble ? (kb & 1) : 0;  // K / K^T buffer of this key block
-    if (threadIdx.x == 0) {
-      bool got = true;
-      auto load_block = [&](int blk) {
-        const int u = L::kDouble ? (blk & 1) : 0;
-        mbar_arrive_expect_tx(&bar_k[u], L::kQBytes + 2 * L::kKtAtomBytes);
-        for (int a = 0; a < DQK / 64; ++a)
-          tma_load_2d(smem + L::kKOff + u * L::kQBytes + a * ATOM_BYTES_128, &tmap_k, &bar_k[u], head * DQK + a * 64,
-                      batch * p.seq + blk * ATT_BN);
-        for (int a = 0; a < 2; ++a)
-          tma_load_2d(smem + L::kKtOff + (u * 2 + a) * L::kKtAtomBytes, &tmap_kt, &bar_k[u], blk * ATT_BN + a * 64,
-                      (batch * p.heads + head) * DQK);
-      };
-      // dP = dO V^T over the whole value width: atoms through a two-stage ring, the next load in flight during the MMAs
-      auto load_atom = [&](uint32_t n, int a, int blk) -> bool {
-        const int st = n & 1;
-        if (!mbar_wait_bounded(&ring_free[st], ((n >> 1) & 1) ^ 1, abort_flag)) return false;
-        uint8_t* base = smem + L::kRingOff + st * 2 * ATOM_BYTES_128;
-        mbar_arrive_expect_tx(&ring_full[st], 2 * ATOM_BYTES_128);
-        tma_load_2d(base, &tmap_do, &ring_full[st], head * p.dv + a * 64, batch * p.seq + q0);
-        tma_load_2d(base + ATOM_BYTES_128, &tmap_v, &ring_full[st], head * p.dv + a * 64, batch * p.seq + blk * ATT_BN);
+  if (warp == FWD_ROW_WARPS) {
+    // ------------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      const CUtensorMap* m_fix = DKV ? &tmap_k : &tmap_q;
+      const CUtensorMap* m_walk = DKV ? &tmap_q : &tmap_k;
+      const CUtensorMap* m_fval = DKV ? &tmap_v : &tmap_do;
+      const CUtensorMap* m_wval = DKV ? &tmap_do : &tmap_v;
+      uint32_t t = 0, g = 0, nf = 0, nw = 0;
+      bool ok = true;
+      for (int w = (int)blockIdx.x; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
+        const Tile T = decode(w);
+        auto load_qk = [&](const CUtensorMap* m, uint8_t* dst, uint64_t* bar, int blk) {
+          mbar_arrive_expect_tx(bar, QK_BYTES);
+          for (int a = 0; a < L::kQkAtoms; ++a) tma_load_3d(dst + a * AB, m, bar, T.head * DQK + a * 64, blk * 128, T.batch);
+        };
+        auto load_val = [&](const CUtensorMap* m, uint8_t* dst, uint64_t* bar, int atom, int blk) {
+          mbar_arrive_expect_tx(bar, AB);
+          tma_load_3d(dst, m, bar, T.head * p.dv + atom * 64, blk * 128, T.batch);
+        };
+        const uint32_t fb = t % L::kFixBufs;
+        ok = mbar_wait_bounded(&B.fix_free[fb], ((t / L::kFixBufs) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        load_qk(m_fix, smem + L::kFixOff + fb * QK_BYTES, &B.fix_full[fb], T.blk);
+        for (int s = 0; s < T.steps && ok; ++s, ++g) {
+          const uint32_t wb = g % L::kWalkBufs;
+          ok = mbar_wait_bounded(&B.walk_free[wb], ((g / L::kWalkBufs) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          load_qk(m_walk, smem + L::kWalkOff + wb * QK_BYTES, &B.walk_full[wb], T.first + s);
+          for (int i = 0; i < dv_atoms && ok; ++i) {
+            const int a = atom_at(T, i);
+            if (stream_fix || s == 0) {
+              const uint32_t slot = stream_fix ? nf & 1 : (uint32_t)i, use = stream_fix ? nf >> 1 : t;
+              ok = mbar_wait_bounded(&B.fval_free[slot], (use & 1) ^ 1, abort_flag);
+              if (!ok) break;
+              load_val(m_fval, smem + L::kFixValOff + slot * AB, &B.fval_full[slot], a, T.blk);
+              ++nf;
+            }
+            const uint32_t slot = nw % L::kWalkValSlots;
+            ok = mbar_wait_bounded(&B.wval_free[slot], ((nw / L::kWalkValSlots) & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            load_val(m_wval, smem + L::kWalkValOff + slot * AB, &B.wval_full[slot], a, T.first + s);
+            ++nw;
+          }
+        }
+      }
+      if (!ok) {
+        report_status(p.status, kTimeoutEmptyBarrier, (int)g);
+        *abort_flag = 1;
+      }
+    }
+  } else if (warp == FWD_ROW_WARPS + 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128);
+      uint32_t t = 0, g = 0, nf = 0, nw = 0;
+      bool ok = true;
+      // the block whose accumulating products are still to be issued
+      bool pending = false;
+      uint32_t pg = 0, pt = 0, pval = 0;  // its index, its tile's, the slot of the first atom of its value chunk
+      int ps = 0;
+      bool pdk = false;
+      // Block g's accumulating products follow the S and dP of block g + 1, so that the tensor core has work while the rows are at block
+      // g; they come before them where the tiles that block g holds on to leave no room for those of block g + 1.
+      const bool early = L::kWalkBufs == 1 || (DKV && dv_atoms + DVC / 64 > L::kWalkValSlots);
+      auto accumulate = [&]() -> bool {
+        if (!pending) return true;
+        pending = false;
+        if (ps == 0) {  // the accumulator's previous tile has been stored
+          const uint32_t buf = DKV ? 0 : pt & 1, use = DKV ? pt : pt >> 1;
+          if (!mbar_wait_bounded(&B.acc_free[buf], (use & 1) ^ 1, abort_flag)) return false;
+        }
+        if (!mbar_wait_bounded(B.out_full, pg & 1, abort_flag)) return false;
+        tc_fence_after();
+        const uint32_t walk = smem_u32(smem + L::kWalkOff + (pg % L::kWalkBufs) * QK_BYTES);
+        const uint32_t ds = smem_u32(smem + L::kDsOff);
+        if constexpr (!DKV) {
+          const uint32_t d = tmem_acc + (pt & 1) * DQK;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)  // sixteen keys a step
+            umma_bf16_ss(d, make_sw128_kmajor_desc(ds + (kk / 4) * AB) + (uint64_t)((kk % 4) * 2), make_sw128_mnmajor_desc(walk + kk * 2048, AB),
+                         make_idesc_bf16(128, DQK, false, true), (ps > 0 || kk > 0) ? 1u : 0u);
+        } else {
+          const uint32_t pm = smem_u32(smem + L::kPOff), val = smem_u32(smem + L::kWalkValOff + pval * AB);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)  // sixteen queries a step
+            umma_bf16_ss(tmem_acc, make_sw128_mnmajor_desc(pm + kk * 2048, AB), make_sw128_mnmajor_desc(val + kk * 2048, AB),
+                         make_idesc_bf16(128, DVC, true, true), (ps > 0 || kk > 0) ? 1u : 0u);
+          for (int i = 0; i < DVC / 64; ++i) umma_commit(&B.wval_free[pval + i]);
+          if (pdk) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_bf16_ss(tmem_acc + 128, make_sw128_mnmajor_desc(ds + kk * 2048, AB), make_sw128_mnmajor_desc(walk + kk * 2048, AB),
+                           make_idesc_bf16(128, DQK, true, true), (ps > 0 || kk > 0) ? 1u : 0u);
+          }
+        }
+        umma_commit(&B.walk_free[pg % L::kWalkBufs]);
+        umma_commit(B.out_free);
         return true;
       };
-      if (kb == 0 || !L::kDouble) {  // (double-buffered: issued during the previous block, see below)
-        load_block(kb);
-        got = load_atom(ring_n, 0, kb);
-      }
-      if (kb == 0) got = got && mbar_wait_bounded(bar_q, 0, abort_flag);
-      got = got && mbar_wait_bounded(&bar_k[ub], L::kDouble ? ((kb >> 1) & 1) : parity, abort_flag);
-      if (got) {
-        tc_fence_after();
-        issue_mma_atoms(tmem_s, smem_u32(smem + L::kQOff), ATOM_BYTES_128, smem_u32(smem + L::kKOff + ub * L::kQBytes),
-                        ATOM_BYTES_128, DQK / 16, make_idesc_bf16(ATT_BM, ATT_BN), false);
-        for (int a = 0; a < dv_atoms && got; ++a) {
-          const uint32_t n = ring_n + a;
-          if (a + 1 < dv_atoms) got = load_atom(n + 1, a + 1, kb);
-          got = got && mbar_wait_bounded(&ring_full[n & 1], (n >> 1) & 1, abort_flag);
-          if (!got) break;
+      for (int w = (int)blockIdx.x; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
+        const Tile T = decode(w);
+        const uint32_t fb = t % L::kFixBufs;
+        for (int s = 0; s < T.steps; ++s, ++g) {
+          if (early && !(ok = accumulate())) break;
+          const uint32_t wb = g % L::kWalkBufs;
+          ok = (s > 0 || mbar_wait_bounded(&B.fix_full[fb], (t / L::kFixBufs) & 1, abort_flag)) &&
+               mbar_wait_bounded(&B.walk_full[wb], (g / L::kWalkBufs) & 1, abort_flag) &&
+               mbar_wait_bounded(B.sdp_free, (g & 1) ^ 1, abort_flag);  // the rows have read block g - 1
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t base = smem_u32(smem + L::kRingOff + (n & 1) * 2 * ATOM_BYTES_128);
-          issue_mma_atoms(tmem_dp, base, 0, base + ATOM_BYTES_128, 0, 4, make_idesc_bf16(ATT_BM, ATT_BN), a > 0);
-          umma_commit(&ring_free[n & 1]);
+          const uint32_t fix = smem_u32(smem + L::kFixOff + fb * QK_BYTES), walk = smem_u32(smem + L::kWalkOff + wb * QK_BYTES);
+          issue_mma_atoms(tmem_s, DKV ? walk : fix, AB, DKV ? fix : walk, AB, DQK / 16, idesc_s, false);
+          const bool last = s + 1 == T.steps;
+          if (last) umma_commit(&B.fix_free[fb]);
+          uint32_t first_kept = 0;
+          for (int i = 0; i < dv_atoms; ++i) {
+            const uint32_t fslot = stream_fix ? nf & 1 : (uint32_t)i, fuse = stream_fix ? nf >> 1 : t;
+            const uint32_t wslot = nw % L::kWalkValSlots;
+            if (stream_fix || s == 0) ok = mbar_wait_bounded(&B.fval_full[fslot], fuse & 1, abort_flag);
+            ok = ok && mbar_wait_bounded(&B.wval_full[wslot], (nw / L::kWalkValSlots) & 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t fv = smem_u32(smem + L::kFixValOff + fslot * AB), wv = smem_u32(smem + L::kWalkValOff + wslot * AB);
+            issue_mma_atoms(tmem_dp, DKV ? wv : fv, 0, DKV ? fv : wv, 0, 4, idesc_s, i > 0);
+            if (stream_fix || last) umma_commit(&B.fval_free[fslot]);
+            const bool kept = DKV && i >= dv_atoms - DVC / 64;  // (needed once more, for dV)
+            if (!kept) umma_commit(&B.wval_free[wslot]);
+            if (DKV && i == dv_atoms - DVC / 64) first_kept = wslot;
+            if (stream_fix) ++nf;
+            ++nw;
+          }
+          if (!ok) break;
+          umma_commit(B.sdp_full);
+          if (!early && !(ok = accumulate())) break;
+          pending = true;
+          pg = g; pt = t; ps = s; pval = first_kept; pdk = T.chunk == 0;
         }
-        ring_n += dv_atoms;
       }
-      if (!got) {
-        report_status(p.status, kTimeoutFullBarrier, kb);
+      ok = ok && accumulate();
+      if (!ok) {
+        report_status(p.status, kTimeoutFullBarrier, (int)g);
         *abort_flag = 1;
       }
-      umma_commit(bar_mma1);
-      if (L::kDouble && got && kb + 1 < n_kblocks) {
-        // next key block: its K / K^T buffer was last read by the MMAs of block kb - 1 (complete); the ring stage
-        // frees up when this block's last dP MMAs have read it
-        load_block(kb + 1);
-        if (!load_atom(ring_n, 0, kb + 1)) {
-          report_status(p.status, kTimeoutEmptyBarrier, kb);
-          *abort_flag = 1;
-        }
-      }
     }
-    if (!mbar_wait_bounded(bar_mma1, parity, abort_flag)) {
-      report_status(p.status, kTimeoutTmemFull, kb);
-      *abort_flag = 1;
-    }
-    __syncthreads();
-    ok = (*abort_flag == 0);
-    if (!ok) break;
-    tc_fence_after();
-
-#pragma unroll 1
-    for (int c = 0; c < ATT_BN / 32; ++c) {
-      uint32_t rs[32], rp[32];
-      tmem_ld_32x32b_x32(tmem_s + lane_off + (uint32_t)(c * 32), rs);
-      tmem_ld_32x32b_x32(tmem_dp + lane_off + (uint32_t)(c * 32), rp);
-      tmem_wait_ld();
-      float ds[32];
-      if (kb < qblk && k0 + ATT_BN <= p.seq) {
-        // a block below the diagonal and inside the sequence: nothing to mask (uniform over the CTA)
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float pr = exp2f(fmaf(__uint_as_float(rs[j]), p.scale_log2, -lse2));
-          ds[j] = pr * (__uint_as_float(rp[j]) - delta) * p.scale;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int kpos = k0 + c * 32 + j;
-          const bool valid = kpos <= qpos && kpos < p.seq;
-          const float pr = valid ? exp2f(fmaf(__uint_as_float(rs[j]), p.scale_log2, -lse2)) : 0.0f;
-          ds[j] = pr * (__uint_as_float(rp[j]) - delta) * p.scale;
-        }
-      }
-      uint8_t* atom = smem + L::kDsOff + (c / 2) * ATOM_BYTES_128;
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint4 u;
-        u.x = pack_bf16x2(ds[g * 8 + 0], ds[g * 8 + 1]);
-        u.y = pack_bf16x2(ds[g * 8 + 2], ds[g * 8 + 3]);
-        u.z = pack_bf16x2(ds[g * 8 + 4], ds[g * 8 + 5]);
-        u.w = pack_bf16x2(ds[g * 8 + 6], ds[g * 8 + 7]);
-        *reinterpret_cast<uint4*>(atom + sw128_chunk_off(row, (c % 2) * 4 + g)) = u;
-      }
-    }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  } else {
+    // ------------------------------------------------------------------ softmax rows
+    const int quarter = warp & 3, cq = warp >> 2, lane = (int)threadIdx.x & 31;
+    const int row = quarter * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    bool ok = true;
+    uint32_t g = 0, t = 0;
+    // a finished tile that is still to be stored
+    bool pending = false;
+    Tile pT{};
+    uint32_t pt = 0;
+    auto store_tile = [&]() {  // (its last accumulating product has completed)
       tc_fence_after();
-      // dQ += dS [128 q x 128 keys] * (K^T [DQK x 128 keys])^T
-      issue_mma_atoms(tmem_dq, smem_u32(smem + L::kDsOff), ATOM_BYTES_128,
-                      smem_u32(smem + L::kKtOff + ub * 2 * L::kKtAtomBytes), L::kKtAtomBytes, ATT_BN / 16,
-                      make_idesc_bf16(ATT_BM, DQK), kb > 0);
-      umma_commit(bar_mma2);
+      const int pos = pT.blk * 128 + row;
+      const bool row_ok = pos < p.seq;
+      const size_t at = ((size_t)pT.batch * p.seq + (row_ok ? pos : 0)) * p.heads + pT.head;
+      if constexpr (!DKV) {
+        if (cq < DQK / 32)
+          bwd_emit(tmem_acc + (pt & 1) * DQK + lane_off + cq * 32, p.scale, p.dq, at * DQK + cq * 32, p.bf16_out, row_ok);
+      } else {
+        if (cq < DVC / 32)
+          bwd_emit(tmem_acc + lane_off + cq * 32, 1.0f, p.dv_out, at * p.dv + pT.chunk * DVC + cq * 32, p.bf16_out, row_ok);
+        if (pT.chunk == 0 && cq < DQK / 32)
+          bwd_emit(tmem_acc + 128 + lane_off + cq * 32, p.scale, p.dk, at * DQK + cq * 32, p.bf16_out, row_ok);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&B.acc_free[DKV ? 0 : pt & 1]);
+      pending = false;
+    };
+    for (int w = (int)blockIdx.x; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
+      const Tile T = decode(w);
+      const size_t stat0 = ((size_t)T.batch * p.heads + T.head) * p.seq;
+      auto load_stats = [&](int qblk, float& nl, float& nd) {
+        const int qpos = qblk * 128 + row;
+        const bool in = qpos < p.seq;
+        nl = in ? -p.lse[stat0 + qpos] * 1.4426950408889634f : -INFINITY;  // (no position: every probability of the row is 0)
+        nd = in ? -p.delta[stat0 + qpos] : 0.0f;
+      };
+      float neg_lse2, neg_delta;
+      load_stats(DKV ? T.first : T.blk, neg_lse2, neg_delta);
+      for (int s = 0; s < T.steps; ++s, ++g) {
+        const int qblk = DKV ? T.first + s : T.blk, kblk = DKV ? T.blk : T.first + s;
+        float next_lse2 = neg_lse2, next_delta = neg_delta;
+        if (DKV && s + 1 < T.steps) load_stats(qblk + 1, next_lse2, next_delta);
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(B.sdp_full, g & 1, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t pk[16], dk[16];
+        {
+          uint32_t rs[32], rp[32];
+          tmem_ld_32x32b_x32(tmem_s + lane_off + (uint32_t)(cq * 32), rs);
+          tmem_ld_32x32b_x32(tmem_dp + lane_off + (uint32_t)(cq * 32), rp);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(B.sdp_free);
+          const int last = min(qblk * 128 + row, p.seq - 1) - (kblk * 128 + cq * 32);
+          bwd_block<DKV>(rs, rp, p.scale_log2, neg_lse2, neg_delta, last, pk, dk);
+        }
+        // the previous block's accumulating products have read P and dS
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(B.out_free, (g & 1) ^ 1, abort_flag));
+        if (!ok) break;
+        bwd_store(smem + L::kDsOff, row, cq, dk);
+        if constexpr (DKV) bwd_store(smem + L::kPOff, row, cq, pk);
+        fence_proxy_async();  // the generic-proxy stores must be visible to the tensor core's reads
+        __syncwarp();
+        if (lane == 0) mbar_arrive(B.out_full);
+        if (pending) store_tile();  // (s == 0: the tile before this one, whose last products have just been waited for)
+        neg_lse2 = next_lse2;
+        neg_delta = next_delta;
+      }
+      if (!ok) break;
+      pending = true;
+      pT = T;
+      pt = t;
     }
-    if (!mbar_wait_bounded(bar_mma2, parity, abort_flag)) {
-      report_status(p.status, kTimeoutTmemFull, 1000 + kb);
+    if (ok && pending) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(B.out_free, (g & 1) ^ 1, abort_flag));
+      if (ok) store_tile();
+    }
+    if (!ok) {
+      report_status(p.status, kTimeoutTmemFull, row);
       *abort_flag = 1;
     }
-    tc_fence_before();
-    __syncthreads();
-    ok = (*abort_flag == 0);
   }
 
-  if (ok) {
-    tc_fence_after();
-#pragma unroll 1
-    for (int c = 0; c < DQK / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_dq + lane_off + (uint32_t)(c * 32), r);
-      tmem_wait_ld();
-      if (row_ok) {
-        float* dst = p.dq + (((size_t)batch * p.seq + qpos) * p.heads + head) * DQK + c * 32;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                                            __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-      }
-    }
-  }
   tc_fence_before();
   __syncthreads();
   if (*abort_flag != 0) {
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);  // copies that may still be in flight land first
     __syncthreads();
   }
-  if (warp == 0) {
+  if (warp == FWD_ROW_WARPS + 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
 }
 
 template <int DQK, int DVC>
-__global__ void __launch_bounds__(ATT_THREADS)
-attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q,
-                    const __grid_constant__ CUtensorMap tmap_qt, const __grid_constant__ CUtensorMap tmap_v,
-                    const __grid_constant__ CUtensorMap tmap_do, const __grid_constant__ CUtensorMap tmap_dot,
-                    const AttnBwdParams p) {
-  using L = BwdDkvSmem<DQK, DVC>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* bar_k = bars + 0;
-  uint64_t* bar_q = bars + 1;      // [2] Q_i loads, one per buffer
-  uint64_t* bar_t = bars + 3;      // Q_i^T / dO_i^T loads
-  uint64_t* bar_mma1 = bars + 4;
-  uint64_t* bar_mma2 = bars + 5;
-  uint64_t* ring_full = bars + 6;  // [2]
-  uint64_t* ring_free = bars + 8;  // [2]
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kTmemPtrOff);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbortOff);
-  float* s_lse = reinterpret_cast<float*>(smem + L::kLseOff);
-  float* s_delta = reinterpret_cast<float*>(smem + L::kDeltaOff);
-
-  const int warp = threadIdx.x >> 5;
-  const int n_blocks = (p.seq + ATT_BM - 1) / ATT_BM;
-  const int kblk = (int)blockIdx.x;  // key block 0 meets every query block: longest first
-  const int dv_chunks = p.dv / DVC;
-  const int head = (int)blockIdx.y / dv_chunks;
-  const int chunk = (int)blockIdx.y - head * dv_chunks;
-  const int dv0 = chunk * DVC;
-  const bool do_dk = chunk == 0;
-  const int batch = (int)blockIdx.z;
-  const int k0 = kblk * ATT_BN;
-  const int row = (int)threadIdx.x;
-  const int kpos = k0 + row;
-  const bool row_ok = kpos < p.seq;
-  const int dv_atoms = p.dv / 64;
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < L::kNumBars; ++i) mbar_init(&bars[i], 1);
-    *abort_flag = 0;
-    fence_barrier_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(tmem_ptr_smem, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
-  const uint32_t tmem_st = tmem_base, tmem_dpt = tmem_base + 128, tmem_dv = tmem_base + 256, tmem_dk = tmem_base + 384;
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(bar_k, L::kKBytes);
-    for (int a = 0; a < DQK / 64; ++a)
-      tma_load_2d(smem + L::kKOff + a * ATOM_BYTES_128, &tmap_k, bar_k, head * DQK + a * 64, batch * p.seq + k0);
-  }
-
-  uint32_t ring_n = 0;
-  bool ok = true;
-  int it = 0;
-  for (int qb = kblk; qb < n_blocks && ok; ++qb, ++it) {
-    const int q0 = qb * ATT_BM;
-    const uint32_t parity = it & 1;
-    {
-      // statistics of this query block's rows (columns of S^T)
-      const int qp = q0 + row;
-      const size_t o = ((size_t)batch * p.heads + head) * p.seq + (qp < p.seq ? qp : 0);
-      s_lse[row] = qp < p.seq ? p.lse[o] * 1.4426950408889634f : INFINITY;
-      s_delta[row] = qp < p.seq ? p.delta[o] : 0.0f;
-    }
-    const int uq = L::kDouble ? (it & 1) : 0;  // Q buffer of this query block
-    auto load_q = [&](int blk, int u) {
-      mbar_arrive_expect_tx(&bar_q[u], L::kKBytes);
-      for (int a = 0; a < DQK / 64; ++a)
-        tma_load_2d(smem + L::kQOff + u * L::kKBytes + a * ATOM_BYTES_128, &tmap_q, &bar_q[u], head * DQK + a * 64,
-                    batch * p.seq + blk * ATT_BM);
-    };
-    auto load_atom = [&](uint32_t n, int a, int blk) -> bool {
-      const int st = n & 1;
-      if (!mbar_wait_bounded(&ring_free[st], ((n >> 1) & 1) ^ 1, abort_flag)) return false;
-      uint8_t* base = smem + L::kRingOff + st * 2 * ATOM_BYTES_128;
-      mbar_arrive_expect_tx(&ring_full[st], 2 * ATOM_BYTES_128);
-      tma_load_2d(base, &tmap_v, &ring_full[st], head * p.dv + a * 64, batch * p.seq + k0);
-      tma_load_2d(base + ATOM_BYTES_128, &tmap_do, &ring_full[st], head * p.dv + a * 64, batch * p.seq + blk * ATT_BM);
-      return true;
-    };
-    if (threadIdx.x == 0) {
-      bool got = true;
-      if (it == 0 || !L::kDouble) {  // (double-buffered: issued during the previous block, see below)
-        load_q(qb, uq);
-        got = load_atom(ring_n, 0, qb);
-      }
-      if (it == 0) got = got && mbar_wait_bounded(bar_k, 0, abort_flag);
-      got = got && mbar_wait_bounded(&bar_q[uq], L::kDouble ? ((it >> 1) & 1) : parity, abort_flag);
-      if (got) {
-        tc_fence_after();
-        // S^T = K_j Q_i^T
-        issue_mma_atoms(tmem_st, smem_u32(smem + L::kKOff), ATOM_BYTES_128, smem_u32(smem + L::kQOff + uq * L::kKBytes),
-                        ATOM_BYTES_128, DQK / 16, make_idesc_bf16(ATT_BM, ATT_BN), false);
-        // dP^T = V_j dO_i^T over the whole value width
-        for (int a = 0; a < dv_atoms && got; ++a) {
-          const uint32_t n = ring_n + a;
-          if (a + 1 < dv_atoms) got = load_atom(n + 1, a + 1, qb);
-          got = got && mbar_wait_bounded(&ring_full[n & 1], (n >> 1) & 1, abort_flag);
-          if (!got) break;
-          tc_fence_after();
-          const uint32_t base = smem_u32(smem + L::kRingOff + (n & 1) * 2 * ATOM_BYTES_128);
-          issue_mma_atoms(tmem_dpt, base, 0, base + ATOM_BYTES_128, 0, 4, make_idesc_bf16(ATT_BM, ATT_BN), a > 0);
-          umma_commit(&ring_free[n & 1]);
-        }
-        ring_n += dv_atoms;
-      }
-      if (!got) {
-        report_status(p.status, kTimeoutFullBarrier, it);
-        *abort_flag = 1;
-      }
-      umma_commit(bar_mma1);
-    }
-    if (!mbar_wait_bounded(bar_mma1, parity, abort_flag)) {
-      report_status(p.status, kTimeoutTmemFull, it);
-      *abort_flag = 1;
-    }
-    __syncthreads();  // also publishes s_lse / s_delta
-    ok = (*abort_flag == 0);
-    if (!ok) break;
-    tc_fence_after();
-
-    // Q_i and the ring are free now (their MMAs completed): fetch Q_i^T and the dO_i^T chunk while the threads work. The
-    // chunk goes into the ring stage that the NEXT query block's first atom does not use, so that atom (and the next Q
-    // tile, into the other Q buffer) can be fetched now as well.
-    const int dot_stage = L::kDouble ? (int)((ring_n & 1) ^ 1) : 0;
-    if (threadIdx.x == 0) {
-      // both ring stages must be idle before anything overwrites them (their last MMAs were committed above)
-      bool got = mbar_wait_bounded(&ring_free[0], (((ring_n + 1) >> 1) & 1) ^ 1, abort_flag) &&
-                 mbar_wait_bounded(&ring_free[1], ((ring_n >> 1) & 1) ^ 1, abort_flag);
-      if (got) {
-        mbar_arrive_expect_tx(bar_t, (do_dk ? 2 * L::kQtAtomBytes : 0) + 2 * L::kDotAtomBytes);
-        if (do_dk)
-          for (int a = 0; a < 2; ++a)
-            tma_load_2d(smem + L::kQOff + uq * L::kKBytes + a * L::kQtAtomBytes, &tmap_qt, bar_t, q0 + a * 64,
-                        (batch * p.heads + head) * DQK);
-        for (int a = 0; a < 2; ++a)
-          tma_load_2d(smem + L::kRingOff + dot_stage * 2 * ATOM_BYTES_128 + a * L::kDotAtomBytes, &tmap_dot, bar_t,
-                      q0 + a * 64, (batch * p.heads + head) * p.dv + dv0);
-        if (L::kDouble && qb + 1 < n_blocks) {
-          load_q(qb + 1, uq ^ 1);  // that buffer held Q^T of block qb - 1, read by MMAs that have completed
-          got = load_atom(ring_n, 0, qb + 1);
-        }
-      }
-      if (!got) {
-        report_status(p.status, kTimeoutEmptyBarrier, it);
-        *abort_flag = 1;
-      }
-    }
-    __syncwarp();  // warp 0 is whole again before its warp-wide TMEM loads
-
-#pragma unroll 1
-    for (int c = 0; c < ATT_BM / 32; ++c) {
-      uint32_t rs[32], rp[32];
-      tmem_ld_32x32b_x32(tmem_st + lane_off + (uint32_t)(c * 32), rs);
-      tmem_ld_32x32b_x32(tmem_dpt + lane_off + (uint32_t)(c * 32), rp);
-      tmem_wait_ld();
-      float pt[32], ds[32];
-      if (qb > kblk && q0 + ATT_BM <= p.seq && k0 + ATT_BN <= p.seq) {
-        // a query block above the diagonal, both blocks inside the sequence: nothing to mask (uniform over the CTA)
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int col = c * 32 + j;
-          pt[j] = exp2f(fmaf(__uint_as_float(rs[j]), p.scale_log2, -s_lse[col]));
-          ds[j] = pt[j] * (__uint_as_float(rp[j]) - s_delta[col]) * p.scale;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int col = c * 32 + j;
-          const int qp = q0 + col;
-          const bool valid = row_ok && kpos <= qp && qp < p.seq;
-          pt[j] = valid ? exp2f(fmaf(__uint_as_float(rs[j]), p.scale_log2, -s_lse[col])) : 0.0f;
-          ds[j] = pt[j] * (__uint_as_float(rp[j]) - s_delta[col]) * p.scale;
-        }
-      }
-      uint8_t* atom_p = smem + L::kPtOff + (c / 2) * ATOM_BYTES_128;
-      uint8_t* atom_d = smem + L::kDstOff + (c / 2) * ATOM_BYTES_128;
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint4 u, w;
-        u.x = pack_bf16x2(pt[g * 8 + 0], pt[g * 8 + 1]);
-        u.y = pack_bf16x2(pt[g * 8 + 2], pt[g * 8 + 3]);
-        u.z = pack_bf16x2(pt[g * 8 + 4], pt[g * 8 + 5]);
-        u.w = pack_bf16x2(pt[g * 8 + 6], pt[g * 8 + 7]);
-        w.x = pack_bf16x2(ds[g * 8 + 0], ds[g * 8 + 1]);
-        w.y = pack_bf16x2(ds[g * 8 + 2], ds[g * 8 + 3]);
-        w.z = pack_bf16x2(ds[g * 8 + 4], ds[g * 8 + 5]);
-        w.w = pack_bf16x2(ds[g * 8 + 6], ds[g * 8 + 7]);
-        const uint32_t off = sw128_chunk_off(row, (c % 2) * 4 + g);
-        *reinterpret_cast<uint4*>(atom_p + off) = u;
-        *reinterpret_cast<uint4*>(atom_d + off) = w;
-      }
-    }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      bool got = (*abort_flag == 0) && mbar_wait_bounded(bar_t, parity, abort_flag);
-      if (got) {
-        tc_fence_after();
-        // dV += P^T [128 keys x 128 q] * (dO^T chunk [DVC x 128 q])^T
-        issue_mma_atoms(tmem_dv, smem_u32(smem + L::kPtOff), ATOM_BYTES_128,
-                        smem_u32(smem + L::kRingOff + dot_stage * 2 * ATOM_BYTES_128), L::kDotAtomBytes, ATT_BM / 16,
-                        make_idesc_bf16(ATT_BM, DVC), it > 0);
-        // dK += dS^T [128 keys x 128 q] * (Q^T [DQK x 128 q])^T
-        if (do_dk)
-          issue_mma_atoms(tmem_dk, smem_u32(smem + L::kDstOff), ATOM_BYTES_128, smem_u32(smem + L::kQOff + uq * L::kKBytes),
-                          L::kQtAtomBytes, ATT_BM / 16, make_idesc_bf16(ATT_BM, DQK), it > 0);
-      } else {
-        report_status(p.status, kTimeoutFullBarrier, 2000 + it);
-        *abort_flag = 1;
-      }
-      umma_commit(bar_mma2);
-    }
-    if (!mbar_wait_bounded(bar_mma2, parity, abort_flag)) {
-      report_status(p.status, kTimeoutTmemFull, 1000 + it);
-      *abort_flag = 1;
-    }
-    tc_fence_before();
-    __syncthreads();
-    ok = (*abort_flag == 0);
-  }
-
-  if (ok) {
-    tc_fence_after();
-#pragma unroll 1
-    for (int c = 0; c < DVC / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_dv + lane_off + (uint32_t)(c * 32), r);
-      tmem_wait_ld();
-      if (row_ok) {
-        float* dst = p.dv_out + (((size_t)batch * p.seq + kpos) * p.heads + head) * p.dv + dv0 + c * 32;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                                            __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-      }
-    }
-    if (do_dk) {
-#pragma unroll 1
-      for (int c = 0; c < DQK / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(tmem_dk + lane_off + (uint32_t)(c * 32), r);
-        tmem_wait_ld();
-        if (row_ok) {
-          float* dst = p.dk + (((size_t)batch * p.seq + kpos) * p.heads + head) * DQK + c * 32;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                                              __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (*abort_flag != 0) {
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
-    __syncthreads();
-  }
-  if (warp == 0) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
-  }
-}
-
-template <int DQK>
-static cudaError_t attn_bwd_dq_variant(const CUtensorMap* maps, const AttnBwdParams& p, cudaStream_t stream) {
-  using L = BwdDqSmem<DQK>;
+static cudaError_t attn_bwd_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                    const AttnBwdParams& p, cudaStream_t stream) {
+  using L = BwdSmem<DQK, DVC != 0>;
   static_assert(L::kDynamicBytes <= 232448, "shared memory of one CTA exceeds 227 KB");
-  auto kern = attn_bwd_dq_kernel<DQK>;
+  auto kern = attn_bwd_kernel<DQK, DVC>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
   if (e != cudaSuccess) return e;
-  dim3 grid((p.seq + ATT_BM - 1) / ATT_BM, p.heads, p.batch);
-  kern<<<grid, ATT_THREADS, L::kDynamicBytes, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], p);
+  const long long tiles = (long long)((p.seq + 127) / 128) * p.heads * (DVC != 0 ? p.dv / (DVC != 0 ? DVC : 1) : 1) * p.batch;
+  if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
+  kern<<<(int)(tiles < 148 ? tiles : 148), BWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, tdo, p);
   return cudaGetLastError();
 }
 
-template <int DQK, int DVC>
-static cudaError_t attn_bwd_dkv_variant(const CUtensorMap* maps, const AttnBwdParams& p, cudaStream_t stream) {
-  using L = BwdDkvSmem<DQK, DVC>;
-  static_assert(L::kDynamicBytes <= 232448, "shared memory of one CTA exceeds 227 KB");
-  auto kern = attn_bwd_dkv_kernel<DQK, DVC>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
-  if (e != cudaSuccess) return e;
-  dim3 grid((p.seq + ATT_BM - 1) / ATT_BM, p.heads * (p.dv / DVC), p.batch);
-  kern<<<grid, ATT_THREADS, L::kDynamicBytes, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
-  return cudaGetLastError();
-}
-
-// maps_dq = {q, k, k^T, dO, v}; maps_dkv = {k, q, q^T, v, dO, dO^T}
-int attn_bwd_launch(const CUtensorMap* maps_dq, const CUtensorMap* maps_dkv, const AttnBwdParams& p, cudaStream_t stream) {
+int attn_bwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p,
+                    cudaStream_t stream) {
   const int dvc = attn_value_chunk(p.dv);
   if (dvc == 0 || (p.dqk != 64 && p.dqk != 128) || p.seq % 8 != 0 || p.batch > 65535 || p.heads * (p.dv / dvc) > 65535)
     return (int)cudaErrorInvalidValue;
-  cudaError_t e = p.dqk == 64 ? attn_bwd_dq_variant<64>(maps_dq, p, stream) : attn_bwd_dq_variant<128>(maps_dq, p, stream);
+  cudaError_t e = p.dqk == 64 ? attn_bwd_variant<64, 0>(tq, tk, tv, tdo, p, stream) : attn_bwd_variant<128, 0>(tq, tk, tv, tdo, p, stream);
   if (e != cudaSuccess) return (int)e;
-  if (p.dqk == 64) e = dvc == 128 ? attn_bwd_dkv_variant<64, 128>(maps_dkv, p, stream) : attn_bwd_dkv_variant<64, 64>(maps_dkv, p, stream);
-  else e = dvc == 128 ? attn_bwd_dkv_variant<128, 128>(maps_dkv, p, stream) : attn_bwd_dkv_variant<128, 64>(maps_dkv, p, stream);
+  if (p.dqk == 64) e = dvc == 128 ? attn_bwd_variant<64, 128>(tq, tk, tv, tdo, p, stream) : attn_bwd_variant<64, 64>(tq, tk, tv, tdo, p, stream);
+  else e = dvc == 128 ? attn_bwd_variant<128, 128>(tq, tk, tv, tdo, p, stream) : attn_bwd_variant<128, 64>(tq, tk, tv, tdo, p, stream);
   return (int)e;
 }
 
+// delta[b, h, s] = sum over the value columns of dO * O: eight lanes per (position, head), two 16-byte loads a lane and tensor at once.
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out, long long rows, int seq, int heads, int dv,
+                  float* __restrict__ delta) {
+  const int sub = threadIdx.x & 7;
+  const long long r = (long long)blockIdx.x * 32 + (threadIdx.x >> 3);
+  float s = 0.0f;
+  if (r < rows) {
+    for (int c = sub * 8; c < dv; c += 128) {  // (dv is a multiple of 8)
+      const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+      const bool two = c + 64 < dv;
+      const uint4 a0 = __ldg(reinterpret_cast<const uint4*>(dout + r * dv + c)), b0 = __ldg(reinterpret_cast<const uint4*>(out + r * dv + c));
+      const uint4 a1 = two ? __ldg(reinterpret_cast<const uint4*>(dout + r * dv + c + 64)) : zero;
+      const uint4 b1 = two ? __ldg(reinterpret_cast<const uint4*>(out + r * dv + c + 64)) : zero;
+      float x[8], y[8];
+      bf16x8_to_float(a0, x);
+      bf16x8_to_float(b0, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s = fmaf(x[i], y[i], s);
+      bf16x8_to_float(a1, x);
+      bf16x8_to_float(b1, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s = fmaf(x[i], y[i], s);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (r < rows && sub == 0) {
+    const long long pos = r / heads;
+    delta[((pos / seq) * heads + r % heads) * seq + pos % seq] = s;
+  }
+}
+
+int attn_delta_launch(const __nv_bfloat16* dout, const __nv_bfloat16* out, int batch, int seq, int heads, int dv, float* delta, cudaStream_t stream) {
+  const long long rows = (long long)batch * seq * heads;
+  if (rows == 0) return 0;
+  attn_delta_kernel<<<(int)((rows + 31) / 32), 256, 0, stream>>>(dout, out, rows, seq, heads, dv, delta);
+  return (int)cudaGetLastError();
+}
 
 // Value columns per CTA of the forward kernel: with 128-wide queries the double-buffered tiles only fit for 64.
 int attn_fwd_value_chunk(int dqk, int dv) {
@@ -1073,14 +991,14 @@ int attn_fwd_value_chunk(int dqk, int dv) {
   return (dqk == 128 && c == 128) ? 64 : c;
 }
 
-int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tvt, const AttnParams& p,
+int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                     cudaStream_t stream) {
   const int dvc = attn_fwd_value_chunk(p.dqk, p.dv);
   if (dvc == 0 || (p.dqk != 64 && p.dqk != 128) || p.seq % 8 != 0 || p.batch > 65535 || p.heads * (p.dv / dvc) > 65535)
     return (int)cudaErrorInvalidValue;
   cudaError_t e;
-  if (p.dqk == 64) e = dvc == 128 ? attn_fwd_variant<64, 128>(tq, tk, tvt, p, stream) : attn_fwd_variant<64, 64>(tq, tk, tvt, p, stream);
-  else e = attn_fwd_variant<128, 64>(tq, tk, tvt, p, stream);
+  if (p.dqk == 64) e = dvc == 128 ? attn_fwd_variant<64, 128>(tq, tk, tv, p, stream) : attn_fwd_variant<64, 64>(tq, tk, tv, p, stream);
+  else e = attn_fwd_variant<128, 64>(tq, tk, tv, p, stream);
   return (int)e;
 }
 

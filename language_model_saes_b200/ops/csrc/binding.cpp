@@ -90,6 +90,22 @@ CUtensorMap make_bf16_tile_map(const void* base, int64_t rows, int64_t cols, int
   return m;
 }
 
+// [batch, seq, cols] bf16 (rows `pitch` elements apart), boxes of 128 positions of one sequence x 64 columns, 128-byte swizzle.
+CUtensorMap make_bf16_seq_map(const void* base, int64_t batch, int64_t seq, int64_t cols, int64_t pitch) {
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(base) % 16 == 0, "TMA base address must be 16-byte aligned");
+  TORCH_CHECK((pitch * 2) % 16 == 0, "TMA row pitch must be a multiple of 16 bytes");
+  CUtensorMap m;
+  cuuint64_t gdim[3] = {(cuuint64_t)cols, (cuuint64_t)seq, (cuuint64_t)batch};
+  cuuint64_t gstride[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)(seq * pitch) * 2};
+  cuuint32_t box[3] = {64, 128, 1};
+  cuuint32_t estride[3] = {1, 1, 1};
+  CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estride,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  TORCH_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", (int)r);
+  return m;
+}
+
 // ---- encoder GEMM ----------------------------------------------------------------------------------
 // mode bit 0: write H (bf16 [M, N]); bit 1: fused per-row top-k candidates.
 // Returns the number of candidate slots per range (KS) so that callers can size / interpret the buffers.
@@ -651,25 +667,20 @@ Tensor jumprelu(const Tensor& x, const Tensor& log_theta, const c10::optional<Te
 }
 
 // ---- attention ---------------------------------------------------------------------------------------------
-// q, k: bf16 [batch, seq, heads, d_qk]; vt: bf16 [batch, heads, d_v, seq] (values transposed, keys contiguous);
-// out: bf16 [batch, seq, heads, d_v]; lse: fp32 [batch, heads, seq] or absent. Causal.
-void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& vt, const Tensor& out, const c10::optional<Tensor>& lse,
-              double scale, const Tensor& status) {
-  CHECK_T(q, torch::kBFloat16);
-  CHECK_T(k, torch::kBFloat16);
-  CHECK_T(vt, torch::kBFloat16);
-  CHECK_T(out, torch::kBFloat16);
+// q, k: bf16 [batch, seq, heads, d_qk]; v: bf16 [batch, seq, heads, d_v]; out: bf16 like v; lse: fp32 [batch, heads, seq] or absent.
+// Causal.
+void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const c10::optional<Tensor>& lse, double scale,
+              const Tensor& status) {
+  for (const Tensor* t : {&q, &k, &v, &out}) { CHECK_T(*t, torch::kBFloat16); }
   CHECK_T(status, torch::kInt32);
-  TORCH_CHECK(q.dim() == 4 && k.sizes() == q.sizes() && vt.dim() == 4, "q, k [b, s, h, dqk]; vt [b, h, dv, s]");
+  TORCH_CHECK(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4, "q, k [b, s, h, dqk]; v [b, s, h, dv]");
   lmsae::AttnParams p{};
   p.batch = (int)q.size(0);
   p.seq = (int)q.size(1);
   p.heads = (int)q.size(2);
   p.dqk = (int)q.size(3);
-  p.dv = (int)vt.size(2);
-  TORCH_CHECK(vt.size(0) == p.batch && vt.size(1) == p.heads && vt.size(3) == p.seq, "vt must be [b, h, dv, s]");
-  TORCH_CHECK(out.dim() == 4 && out.size(0) == p.batch && out.size(1) == p.seq && out.size(2) == p.heads && out.size(3) == p.dv,
-              "out must be [b, s, h, dv]");
+  p.dv = (int)v.size(3);
+  TORCH_CHECK(v.size(0) == p.batch && v.size(1) == p.seq && v.size(2) == p.heads && out.sizes() == v.sizes(), "v, out must be [b, s, h, dv]");
   const int dvc = lmsae::attn_fwd_value_chunk(p.dqk, p.dv);
   TORCH_CHECK(dvc != 0 && (p.dqk == 64 || p.dqk == 128) && p.seq % 8 == 0, "attn_fwd: d_qk in {64, 128}, d_v % 64 == 0, seq % 8 == 0");
   if (lse.has_value()) {
@@ -681,32 +692,33 @@ void attn_fwd(const Tensor& q, const Tensor& k, const Tensor& vt, const Tensor& 
   p.lse = opt_ptr<float>(lse);
   p.status = status.data_ptr<int>();
   const c10::cuda::CUDAGuard guard(q.device());
-  const CUtensorMap tq = make_bf16_tile_map(q.data_ptr(), (int64_t)p.batch * p.seq, (int64_t)p.heads * p.dqk, 128);
-  const CUtensorMap tk = make_bf16_tile_map(k.data_ptr(), (int64_t)p.batch * p.seq, (int64_t)p.heads * p.dqk, 128);
-  const CUtensorMap tvt = make_bf16_tile_map(vt.data_ptr(), (int64_t)p.batch * p.heads * p.dv, p.seq, dvc);
-  check_cuda(lmsae::attn_fwd_launch(tq, tk, tvt, p, at::cuda::getCurrentCUDAStream()), "attn_fwd launch");
+  const int64_t wqk = (int64_t)p.heads * p.dqk, wv = (int64_t)p.heads * p.dv;
+  const CUtensorMap tq = make_bf16_seq_map(q.data_ptr(), p.batch, p.seq, wqk, wqk);
+  const CUtensorMap tk = make_bf16_seq_map(k.data_ptr(), p.batch, p.seq, wqk, wqk);
+  const CUtensorMap tv = make_bf16_seq_map(v.data_ptr(), p.batch, p.seq, wv, wv);
+  check_cuda(lmsae::attn_fwd_launch(tq, tk, tv, p, at::cuda::getCurrentCUDAStream()), "attn_fwd launch");
 }
 
-// q, k, v, dout: bf16 [b, s, h, *]; kt, qt: bf16 [b, h, dqk, s]; dot: bf16 [b, h, dv, s]; lse, delta: fp32 [b, h, s];
-// dq, dk: fp32 [b, s, h, dqk]; dv: fp32 [b, s, h, dv].
-void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& dout, const Tensor& qt, const Tensor& kt,
-              const Tensor& dot, const Tensor& lse, const Tensor& delta, const Tensor& dq, const Tensor& dk, const Tensor& dv,
-              double scale, const Tensor& status) {
-  for (const Tensor* t : {&q, &k, &v, &dout, &qt, &kt, &dot}) { CHECK_T(*t, torch::kBFloat16); }
-  for (const Tensor* t : {&lse, &delta, &dq, &dk, &dv}) { CHECK_T(*t, torch::kFloat32); }
+// q, k, v, dout: bf16 [b, s, h, *]; lse, delta: fp32 [b, h, s]; dq, dk, dv: [b, s, h, *], all three fp32 or all three bf16.
+void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& dout, const Tensor& lse, const Tensor& delta,
+              const Tensor& dq, const Tensor& dk, const Tensor& dv, double scale, const Tensor& status) {
+  for (const Tensor* t : {&q, &k, &v, &dout}) { CHECK_T(*t, torch::kBFloat16); }
+  for (const Tensor* t : {&lse, &delta}) { CHECK_T(*t, torch::kFloat32); }
+  const auto out_type = dq.scalar_type();
+  TORCH_CHECK(out_type == torch::kFloat32 || out_type == torch::kBFloat16, "dq, dk, dv: fp32 or bf16");
+  for (const Tensor* t : {&dq, &dk, &dv}) { CHECK_T(*t, out_type); }
   CHECK_T(status, torch::kInt32);
+  TORCH_CHECK(q.dim() == 4 && v.dim() == 4, "q, k, v, dout: [b, s, h, *]");
   lmsae::AttnBwdParams p{};
   p.batch = (int)q.size(0);
   p.seq = (int)q.size(1);
   p.heads = (int)q.size(2);
   p.dqk = (int)q.size(3);
   p.dv = (int)v.size(3);
-  const int64_t bs = (int64_t)p.batch * p.seq, bh = (int64_t)p.batch * p.heads;
+  const int64_t bh = (int64_t)p.batch * p.heads, wqk = (int64_t)p.heads * p.dqk, wv = (int64_t)p.heads * p.dv;
   TORCH_CHECK(k.sizes() == q.sizes() && dq.sizes() == q.sizes() && dk.sizes() == q.sizes(), "q, k, dq, dk: [b, s, h, dqk]");
   TORCH_CHECK(v.size(0) == p.batch && v.size(1) == p.seq && v.size(2) == p.heads && dout.sizes() == v.sizes() && dv.sizes() == v.sizes(),
               "v, dout, dv: [b, s, h, dv]");
-  TORCH_CHECK(qt.numel() == q.numel() && kt.numel() == q.numel() && qt.size(3) == p.seq && kt.size(3) == p.seq &&
-                  dot.numel() == v.numel() && dot.size(3) == p.seq, "qt, kt: [b, h, dqk, s]; dot: [b, h, dv, s]");
   TORCH_CHECK(lse.numel() == bh * p.seq && delta.numel() == bh * p.seq, "lse, delta: [b, h, s]");
   const int dvc = lmsae::attn_value_chunk(p.dv);
   TORCH_CHECK(dvc != 0 && (p.dqk == 64 || p.dqk == 128) && p.seq % 8 == 0, "attn_bwd: d_qk in {64, 128}, d_v % 64 == 0, seq % 8 == 0");
@@ -714,21 +726,31 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& d
   p.scale_log2 = (float)(scale * 1.4426950408889634);
   p.lse = lse.data_ptr<float>();
   p.delta = delta.data_ptr<float>();
-  p.dq = dq.data_ptr<float>();
-  p.dk = dk.data_ptr<float>();
-  p.dv_out = dv.data_ptr<float>();
+  p.dq = dq.data_ptr();
+  p.dk = dk.data_ptr();
+  p.dv_out = dv.data_ptr();
+  p.bf16_out = out_type == torch::kBFloat16;
   p.status = status.data_ptr<int>();
   const c10::cuda::CUDAGuard guard(q.device());
-  const CUtensorMap mq = make_bf16_tile_map(q.data_ptr(), bs, (int64_t)p.heads * p.dqk, 128);
-  const CUtensorMap mk = make_bf16_tile_map(k.data_ptr(), bs, (int64_t)p.heads * p.dqk, 128);
-  const CUtensorMap mv = make_bf16_tile_map(v.data_ptr(), bs, (int64_t)p.heads * p.dv, 128);
-  const CUtensorMap mdo = make_bf16_tile_map(dout.data_ptr(), bs, (int64_t)p.heads * p.dv, 128);
-  const CUtensorMap mqt = make_bf16_tile_map(qt.data_ptr(), bh * p.dqk, p.seq, p.dqk);
-  const CUtensorMap mkt = make_bf16_tile_map(kt.data_ptr(), bh * p.dqk, p.seq, p.dqk);
-  const CUtensorMap mdot = make_bf16_tile_map(dot.data_ptr(), bh * p.dv, p.seq, dvc);
-  const CUtensorMap maps_dq[5] = {mq, mk, mkt, mdo, mv};
-  const CUtensorMap maps_dkv[6] = {mk, mq, mqt, mv, mdo, mdot};
-  check_cuda(lmsae::attn_bwd_launch(maps_dq, maps_dkv, p, at::cuda::getCurrentCUDAStream()), "attn_bwd launch");
+  const CUtensorMap mq = make_bf16_seq_map(q.data_ptr(), p.batch, p.seq, wqk, wqk);
+  const CUtensorMap mk = make_bf16_seq_map(k.data_ptr(), p.batch, p.seq, wqk, wqk);
+  const CUtensorMap mv = make_bf16_seq_map(v.data_ptr(), p.batch, p.seq, wv, wv);
+  const CUtensorMap mdo = make_bf16_seq_map(dout.data_ptr(), p.batch, p.seq, wv, wv);
+  check_cuda(lmsae::attn_bwd_launch(mq, mk, mv, mdo, p, at::cuda::getCurrentCUDAStream()), "attn_bwd launch");
+}
+
+// delta[b, h, s] = sum of dout * out over the value columns; dout, out: bf16 [b, s, h, dv].
+void attn_delta(const Tensor& dout, const Tensor& out, const Tensor& delta) {
+  CHECK_T(dout, torch::kBFloat16);
+  CHECK_T(out, torch::kBFloat16);
+  CHECK_T(delta, torch::kFloat32);
+  TORCH_CHECK(dout.dim() == 4 && out.sizes() == dout.sizes() && dout.size(3) % 8 == 0 && delta.numel() == dout.size(0) * dout.size(1) * dout.size(2),
+              "dout, out: [b, s, h, dv] with dv % 8 == 0; delta: [b, h, s]");
+  const c10::cuda::CUDAGuard guard(dout.device());
+  check_cuda(lmsae::attn_delta_launch(reinterpret_cast<const __nv_bfloat16*>(dout.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(out.data_ptr()),
+                                      (int)dout.size(0), (int)dout.size(1), (int)dout.size(2), (int)dout.size(3), delta.data_ptr<float>(),
+                                      at::cuda::getCurrentCUDAStream()),
+             "attn_delta launch");
 }
 
 // ---- selection / compaction ----------------------------------------------------------------------------
@@ -1238,6 +1260,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("jumprelu", &jumprelu);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_delta", &attn_delta);
   m.def("radix_hi_bins", &radix_hi_bins);
   m.def("radix_hist", &radix_hist);
   m.def("radix_pick", &radix_pick);

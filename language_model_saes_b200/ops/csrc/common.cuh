@@ -158,6 +158,15 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       : "memory");
 }
 
+// The same over a 3-D map (rows past the end of the middle dimension are filled with zeros, also where the outer one goes on).
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* tmap, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // ---- tcgen05 / TMEM --------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
@@ -312,11 +321,25 @@ __device__ __forceinline__ uint64_t make_sw128_kmajor_desc(uint32_t smem_addr) {
   return desc;
 }
 
-// Instruction descriptor: bf16 x bf16 -> fp32, both operands K-major, dense.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N) {
+// Descriptor for a bf16 tile whose rows run along K (the product contracts over the rows of a row-major tensor): atoms of 64 M/N
+// columns (128 bytes, 128-byte swizzle) x K rows as TMA writes them, `atom_bytes` apart along M/N. Eight rows are 1024 bytes, so
+// that a step of 16 rows advances the start address by 2048 bytes.
+__device__ __forceinline__ uint64_t make_sw128_mnmajor_desc(uint32_t smem_addr, uint32_t atom_bytes) {
+  uint64_t desc = 0;
+  desc |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+  desc |= (uint64_t)((atom_bytes >> 4) & 0x3FFF) << 16;  // leading byte offset: from one 64-column atom to the next
+  desc |= (uint64_t)(1024 >> 4) << 32;                   // stride byte offset: from eight rows to the next eight
+  desc |= (uint64_t)1 << 46;
+  desc |= (uint64_t)2 << 61;
+  return desc;
+}
+
+// Instruction descriptor: bf16 x bf16 -> fp32, dense; operands K-major unless stated otherwise.
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool a_mn_major = false, bool b_mn_major = false) {
   return (1u << 4)                     // accumulator format: f32
          | (1u << 7)                   // A format: bf16
          | (1u << 10)                  // B format: bf16
+         | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16)
          | ((uint32_t)(N >> 3) << 17)  // N / 8
          | ((uint32_t)(M >> 4) << 24); // M / 16
 }

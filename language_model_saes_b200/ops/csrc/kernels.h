@@ -279,15 +279,19 @@ struct AttnBwdParams {
   float scale, scale_log2;
   const float* lse;    // [batch, heads, seq] from the forward pass
   const float* delta;  // [batch, heads, seq] rowsum(dO * O)
-  float* dq;           // [batch, seq, heads, dqk]
-  float* dk;           // [batch, seq, heads, dqk]
-  float* dv_out;       // [batch, seq, heads, dv]
+  void* dq;            // [batch, seq, heads, dqk], fp32 or bf16
+  void* dk;            // [batch, seq, heads, dqk]
+  void* dv_out;        // [batch, seq, heads, dv]
+  bool bf16_out;
   int* status;
 };
-int attn_bwd_launch(const CUtensorMap* maps_dq, const CUtensorMap* maps_dkv, const AttnBwdParams& p, cudaStream_t stream);
+// maps: [batch, seq, heads * width], boxes of 128 positions x 64 columns
+int attn_bwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo, const AttnBwdParams& p,
+                    cudaStream_t stream);
+int attn_delta_launch(const __nv_bfloat16* dout, const __nv_bfloat16* out, int batch, int seq, int heads, int dv, float* delta, cudaStream_t stream);
 int attn_value_chunk(int dv);
 int attn_fwd_value_chunk(int dqk, int dv);
-int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tvt, const AttnParams& p,
+int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                     cudaStream_t stream);
 
 // ---- elementwise (jumprelu.cu) ---------------------------------------------------------------------

@@ -50,6 +50,43 @@ def test_backward_matches_autograd_of_the_oracle(b, s, h, dqk, dv):
         assert torch.allclose(g, t.grad, atol=0.05 * float(t.grad.abs().max()), rtol=0.05), name
 
 
+# sequences shorter than, equal to and just past a 128-position block; value widths of one atom up to ones that are streamed (320: five)
+@pytest.mark.parametrize("b,s,h,dqk,dv", [(1, 8, 1, 64, 64), (3, 72, 2, 64, 192), (2, 136, 3, 64, 320), (2, 264, 2, 128, 256), (37, 128, 5, 64, 128)])
+def test_backward_of_bf16_tensors_stays_inside_each_sequence(b, s, h, dqk, dv):
+    """bf16 inputs get bf16 gradients (fp32 sums, rounded once: 2^-9 of a value, on top of the bf16 products' error); a sequence of NaNs
+    behind another one does not reach it although their blocks of positions overlap."""
+    torch.manual_seed(2)
+    q, k = (torch.randn(b, s, h, dqk, device="cuda").to(torch.bfloat16) for _ in range(2))
+    v, dout = (torch.randn(b, s, h, dv, device="cuda").to(torch.bfloat16) for _ in range(2))
+    for t in (q, k, v, dout):
+        if b > 1:
+            t[-1] = float("nan")
+    n = max(1, b - 1)
+    args = [t.clone().requires_grad_() for t in (q, k, v)]
+    out = A.causal_attention(*args, 1.3 / dqk**0.5)
+    out.backward(dout)
+    K.check_status(torch.device("cuda"))
+    ref = [t[:n].float().requires_grad_() for t in (q, k, v)]
+    want, _ = A.ref_causal_attention(*ref, 1.3 / dqk**0.5)
+    want.backward(dout[:n].float())
+    assert torch.allclose(out[:n].float(), want, atol=2e-2, rtol=2e-2)
+    for name, g, t in zip("qkv", args, ref):
+        assert g.grad.dtype == torch.bfloat16
+        rel = float((g.grad[:n].float() - t.grad).norm() / t.grad.norm().clamp_min(1e-6))
+        assert rel < 2e-2, (name, rel)
+
+
+@pytest.mark.parametrize("b,s,h,dv", [(1, 8, 1, 8), (2, 24, 3, 64), (1, 40, 5, 136), (2, 16, 2, 256)])
+def test_delta_matches_the_plain_sum(b, s, h, dv):
+    torch.manual_seed(3)
+    x, y = (torch.randn(b, s, h, dv, device="cuda").to(torch.bfloat16) for _ in range(2))
+    delta = torch.empty(b, h, s, device="cuda")
+    K._ext().attn_delta(x, y, delta)
+    want = (x.double() * y.double()).sum(-1).permute(0, 2, 1)
+    bound = dv * 2.0**-24 * (x.double() * y.double()).abs().sum(-1).permute(0, 2, 1)  # dv roundings of partial sums
+    assert bool(((delta.double() - want).abs() <= bound).all())
+
+
 def test_lorsa_encode_uses_the_tensor_core_attention_and_matches_the_score_path():
     from language_model_saes_b200.models.lorsa import LorsaConfig, LowRankSparseAttention
 
