@@ -616,6 +616,63 @@ void colsum_bf16(const Tensor& a, const Tensor& out) {
              "colsum_bf16 launch");
 }
 
+// a: bf16 [rows, d] matrices; p, m, v: their biases and moments, fp32 [d] each; counters: int32, zero, one per 256 columns of every
+// matrix; partial: fp32 scratch. Returns the mean loss (and the second sum's share of it) when loss_sum is given.
+std::vector<Tensor> colsum_adam(const std::vector<Tensor>& a, const std::vector<Tensor>& p, const std::vector<Tensor>& m, const std::vector<Tensor>& v,
+                                const Tensor& counters, double lr, double beta1, double beta2, double eps, int64_t step,
+                                const c10::optional<Tensor>& loss_sum, const c10::optional<Tensor>& loss_sum2,
+                                const c10::optional<Tensor>& loss_weight, double loss_den, const Tensor& status) {
+  TORCH_CHECK(a.size() == p.size() && a.size() == m.size() && a.size() == v.size() && a.size() <= lmsae::kMaxColsumSegs, "colsum_adam: matrices");
+  CHECK_T(counters, torch::kInt32);
+  CHECK_T(status, torch::kInt32);
+  lmsae::ColsumAdamParams q{};
+  const c10::cuda::CUDAGuard guard(status.device());
+  int64_t blocks = 0;
+  for (size_t i = 0; i < a.size(); ++i) {
+    CHECK_T(a[i], torch::kBFloat16); CHECK_T(p[i], torch::kFloat32); CHECK_T(m[i], torch::kFloat32); CHECK_T(v[i], torch::kFloat32);
+    TORCH_CHECK(a[i].dim() == 2 && a[i].size(0) == a[0].size(0) && a[i].size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(a[i].data_ptr()) % 16 == 0,
+                "colsum_adam: matrices of one number of rows, a multiple of 8 columns, on 16-byte boundaries");
+    const int64_t d = a[i].size(1);
+    TORCH_CHECK(p[i].numel() == d && m[i].numel() == d && v[i].numel() == d && d < (1 << 30) && a[i].size(0) < (1LL << 31), "colsum_adam: sizes");
+    q.seg[i] = {reinterpret_cast<const __nv_bfloat16*>(a[i].data_ptr()), p[i].data_ptr<float>(), m[i].data_ptr<float>(), v[i].data_ptr<float>(),
+                (int)d, (int)blocks};
+    blocks += (d + 255) / 256;
+  }
+  TORCH_CHECK(counters.numel() >= blocks, "colsum_adam: one counter per 256 columns");
+  q.n_seg = blocks > 0 && a[0].size(0) > 0 ? (int)a.size() : 0;
+  q.rows = q.n_seg > 0 ? (int)a[0].size(0) : 0;
+  const auto f32 = torch::TensorOptions().dtype(torch::kFloat32).device(status.device());
+  Tensor partial;
+  if (q.n_seg > 0) {
+    const int rb = lmsae::colsum_adam_row_blocks((int)blocks, q.rows);
+    if (rb > 1) {
+      partial = torch::empty({blocks * rb * 256}, f32);
+      q.partial = partial.data_ptr<float>();
+    }
+  }
+  q.counters = counters.data_ptr<int>();
+  q.h = make_hyper(lr, beta1, beta2, eps, step);
+  q.status = status.data_ptr<int>();
+  std::vector<Tensor> out;
+  if (loss_sum.has_value()) {
+    for (const auto* t : {&loss_sum, &loss_sum2, &loss_weight})
+      if (t->has_value()) { CHECK_T(**t, torch::kFloat32); }
+    out.push_back(torch::empty({}, f32));
+    q.loss_sum = loss_sum->data_ptr<float>();
+    q.loss_out = out[0].data_ptr<float>();
+    if (loss_sum2.has_value()) {
+      out.push_back(torch::empty({}, f32));
+      q.loss_sum2 = loss_sum2->data_ptr<float>();
+      q.loss_out2 = out[1].data_ptr<float>();
+    }
+    q.loss_weight = opt_ptr<const float>(loss_weight);
+    q.loss_rows = loss_weight.has_value() ? (int)loss_weight->numel() : 0;
+    q.loss_den = (float)loss_den;
+  }
+  check_cuda(lmsae::colsum_adam_launch(q, (int)blocks, at::cuda::getCurrentCUDAStream()), "colsum_adam launch");
+  return out;
+}
+
 void adam_flat(const Tensor& p, const Tensor& g, const Tensor& m, const Tensor& v, const c10::optional<Tensor>& grad_mul,
                const c10::optional<Tensor>& shadow, const c10::optional<Tensor>& grad_sq_sum, double lr, double beta1,
                double beta2, double eps, int64_t step, bool update, const c10::optional<Tensor>& status) {
@@ -1287,6 +1344,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("auxk_loss_grad", &auxk_loss_grad);
   m.def("sparse_grad_adam", &sparse_grad_adam);
   m.def("colsum_bf16", &colsum_bf16);
+  m.def("colsum_adam", &colsum_adam);
   m.def("adam_flat", &adam_flat);
   m.def("row_norm_shadow", &row_norm_shadow);
 }

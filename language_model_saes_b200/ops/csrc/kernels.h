@@ -210,6 +210,29 @@ int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream);
 bool grad_adam_rows_supported(const GradAdamParams& p);
 int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream);
 int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cudaStream_t stream);
+// Column sums of bf16 matrices [rows, d] as bias gradients, Adam on the biases, and the step's mean loss (sparse_ops.cu).
+constexpr int kMaxColsumSegs = 16;
+struct ColsumAdamSeg {
+  const __nv_bfloat16* a;
+  float *p, *m, *v;
+  int d;            // a multiple of 8
+  int first_block;  // blocks of 256 columns before this matrix
+};
+struct ColsumAdamParams {
+  ColsumAdamSeg seg[kMaxColsumSegs];
+  int n_seg, rows, rows_per_block;
+  float* partial;  // [column blocks][row blocks][256]
+  int* counters;   // [column blocks], zero between launches
+  AdamHyper h;
+  const int* status;
+  float *loss_sum, *loss_sum2;   // read and set to zero (nullptr: absent)
+  const float* loss_weight;      // [loss_rows]: the loss is divided by their sum times loss_den, else by loss_den
+  int loss_rows;
+  float loss_den;
+  float *loss_out, *loss_out2;   // (sum + sum2) / den, sum2 / den
+};
+int colsum_adam_row_blocks(int col_blocks, int rows);
+int colsum_adam_launch(ColsumAdamParams p, int col_blocks, cudaStream_t stream);
 int adam_flat_launch(float* p, const float* g, float* m, float* v, long long n, AdamHyper h, const float* grad_mul,
                      __nv_bfloat16* shadow, float* grad_sq_sum, int update, const int* status, cudaStream_t stream);
 int row_norm_shadow_launch(const float* W, int F, int d, float* norm, __nv_bfloat16* shadow, cudaStream_t stream);

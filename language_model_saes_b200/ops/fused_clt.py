@@ -76,6 +76,7 @@ class FusedCLTStep:
                       "W_D": [(z((t + 1) * F, d), z((t + 1) * F, d)) for t in range(L)]}  # fmt: skip
         self.groups: K.FeatureGroups | None = None
         self.loss_sum = z(1)
+        self.bias_update = K.BiasUpdate([d] * L, dev)
         self.comm = None
         self.own_rows = (0, F)
         self.t = 0
@@ -307,8 +308,7 @@ class FusedCLTStep:
             K.sparse_grad_adam(g, act, dact, xs, xs, None, None, None, None, self.WE[s], mE[s], vE[s], self.WE_bf16[s], self.bE[s], mb[s],
                                vb[s], None, None, None, lr, b1, b2, self.eps, self.t, True)  # fmt: skip
         m, v = self.state["b_D"]
-        K.adam_flat(self.bD.view(-1), dy.float().sum(dim=1).reshape(-1), m.view(-1), v.view(-1), lr, b1, b2, self.eps, self.t)
-        return (self.loss_sum / n_rows).squeeze(0)
+        return self.bias_update(list(dy), list(self.bD), list(zip(m, v)), lr, b1, b2, self.eps, self.t, self.loss_sum, loss_den=float(n_rows))
 
     def _gather_rows(self, t: torch.Tensor) -> torch.Tensor:
         """``[rows, n]`` of every replica stacked in rank order."""

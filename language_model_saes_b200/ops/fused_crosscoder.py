@@ -96,6 +96,7 @@ class FusedCrosscoderStep:
                       "b_D": (z(H_l, d), z(H_l, d)), "log_theta": (z(F), z(F))}  # fmt: skip
         self.groups: K.FeatureGroups | None = None
         self.loss_sum = z(1)
+        self.bias_update = K.BiasUpdate([d] * H_l, dev)
         self.list_overflow = torch.zeros(1, dtype=torch.int64, device=dev)
         self.last: dict[str, torch.Tensor] = {}
         self.comm = None
@@ -401,6 +402,7 @@ class FusedCrosscoderStep:
         if lp is not None:  # the penalty's pull on the decoder norms: d / d W_D[f] = c * gap_f * W_D[f] / ||W_D[f]||
             p = lp["c"] * lp["gap"] / self.dec_norm
             self_scale = p if self_scale is None else self_scale + p
+        dxhats = []
         for h in range(H_l):
             dxhat, _, _ = K.sparse_decode_loss(idx, act[h], self.WD_bf16[h], self.bD[h], target[h], None, 2.0 / (B * H), self.loss_sum,
                                                want_dval=False)  # fmt: skip
@@ -411,7 +413,7 @@ class FusedCrosscoderStep:
             K.sparse_grad_adam(self.groups, act[h], dS, dxhat, dxhat, self.WD[h], mD[h], vD[h], self.WD_bf16[h], None, None, None, None, None,
                                None, None, self.dec_norm[h], None, None, lr, b1, b2, self.eps, self.t, True,
                                wd_self_scale=self_scale[h] if self_scale is not None else None, dact_mode=2)  # fmt: skip
-            K.adam_flat(self.bD[h], K.colsum_bf16(dxhat), mbD[h], vbD[h], lr, b1, b2, self.eps, self.t)
+            dxhats.append(dxhat)
         if self.head_size > 1:  # the lists are the same on every rank: the sum over heads is element-wise
             dS = torch.where(idx >= 0, dS, torch.zeros_like(dS))  # (empty slots were never written)
             dist.all_reduce(dS, group=self.head_group)
@@ -425,7 +427,7 @@ class FusedCrosscoderStep:
                                self.bE[h], mb[h], vb[h], None, None, None, lr, b1, b2, self.eps, self.t, True, extra=extra)  # fmt: skip
         m, v = self.state["log_theta"]
         K.adam_flat(self.log_theta, dtheta * theta, m, v, lr * self.jumprelu_lr_factor, b1, b2, self.eps, self.t)
-        l_rec = (self.loss_sum / (B * H_l)).squeeze(0)
+        l_rec = self.bias_update(dxhats, list(self.bD), list(zip(mbD, vbD)), lr, b1, b2, self.eps, self.t, self.loss_sum, loss_den=float(B * H_l))
         l_s = l1_coefficient * u_sum.squeeze(0) / (B * H_l)
         l_p = l_p_sum if lp is not None else torch.zeros((), device=dev)
         self.last = {"l_rec": l_rec, "l_s": l_s, "l_p": l_p, "l0": n_valid.squeeze(0) / B}

@@ -176,6 +176,8 @@ class FusedTopKSAEStep:
         self.groups: K.FeatureGroups | None = None
         self.loss_sum = z(1)
         self.aux_sum = z(1)
+        self._sums_clear = True  # whether both are zero (a step that ended left them so)
+        self.bias_update = K.BiasUpdate([d] if self.bD is not None else [], dev)
         self.batch_list_factor = int(os.environ.get("LMSAE_BATCH_LIST_FACTOR", "8"))
         self.list_overflow = torch.zeros(1, dtype=torch.int64, device=dev)  # tokens whose batch-level codes did not fit
         self.last_aux_loss: torch.Tensor | None = None
@@ -465,7 +467,7 @@ class FusedTopKSAEStep:
             self.dp_comm.wait_params()  # the other replicas' rows of the previous update must have landed in the shadows
         idx, act = self.encode(x, k, _in_step=overlap)
         self._mark("merge")
-        self.loss_sum.zero_()
+        self._clear_sums()
         if use_comm:
             # loss_sum collects the rows this rank owns; scale to a local-batch estimate for the return value
             dxhat, _ = self.comm.decode_reduce_loss(idx, act, self.WD_bf16, label, self.bD, row_weight, grad_scale, self.loss_sum)
@@ -513,6 +515,13 @@ class FusedTopKSAEStep:
             if sharded and update:
                 self._masters_stale = True
 
+        n_den = 1.0 / self.tp if use_comm else 1.0  # each rank evaluated the loss on the B / tp rows it owns
+        if not overlap and grad_mul is None and gsq is None and not clip_grad_norm:
+            sparse(None, None, True)
+            self._mark("sparse_grad_adam")
+            loss = self._end_of_step([dxhat], row_weight, n_den if row_weight is not None else B * n_den, lr)
+            self._mark("bias_update")
+            return loss
         g_bD = K.colsum_bf16(dxhat) if self.bD is not None else None
         if clip_grad_norm:
             assert grad_mul is None, "pass either a gradient factor or a clipping norm"
@@ -548,9 +557,22 @@ class FusedTopKSAEStep:
             bias_update()
             self._mark("bias_update")
         n_local = B if row_weight is None else row_weight.sum()
-        if use_comm:
-            n_local = n_local / self.tp  # each rank evaluated the loss on the B / tp rows it owns
-        return (self.loss_sum / n_local).squeeze(0)
+        return (self.loss_sum / (n_local * n_den)).squeeze(0)
+
+    def _clear_sums(self) -> None:
+        if not self._sums_clear:
+            self.loss_sum.zero_()
+            self.aux_sum.zero_()
+        self._sums_clear = False
+
+    def _end_of_step(self, mats, row_weight, loss_den, lr, aux: bool = False):
+        """The decoder bias's update from the rows of ``mats`` and the mean loss (with ``aux``: and the auxiliary loss's share)."""
+        b1, b2 = self.betas
+        has = self.bD is not None
+        out = self.bias_update(mats if has else [], [self.bD] if has else [], [self.state["b_D"]] if has else [], lr, b1, b2, self.eps, self.t,
+                               self.loss_sum, self.aux_sum if aux else None, row_weight, loss_den)  # fmt: skip
+        self._sums_clear = True
+        return out
 
     def _clip_factor(self, sparse, g_bD: torch.Tensor | None, max_norm: float, extra_fired: torch.Tensor | None = None) -> torch.Tensor:
         """The trainer's clipping factor as a 1-element device tensor. The norm is the reference project's
@@ -638,8 +660,7 @@ class FusedTopKSAEStep:
         b_dead = self.bE[order]
         g_dead = (gate[order] if gate is not None else torch.ones(cap, device=x.device)) * valid
         self._mark("dead_statistics_compact_dictionary")
-        self.loss_sum.zero_()
-        self.aux_sum.zero_()
+        self._clear_sums()
         xhat = K.sparse_decode(idx, act, self.WD_bf16, None, torch.float32)
         self._mark("main_decode")
         # The auxiliary codes hold up to k_aux (hundreds of) entries per token, several times the main codes, but all of
@@ -719,12 +740,16 @@ class FusedTopKSAEStep:
             if sharded and update:
                 self._masters_stale = True
 
+        if not clip_grad_norm:
+            sparse(None, None, True)
+            self._mark("sparse_grad_adam")
+            loss, self.last_aux_loss = self._end_of_step([g_main], row_weight, 1.0 if row_weight is not None else float(B), lr, aux=True)
+            self._mark("bias_update")
+            return loss
         g_bD = K.colsum_bf16(g_main) if self.bD is not None else None
-        grad_mul = None
-        if clip_grad_norm:
-            lo, hi = self.own_rows
-            got_aux = ((row_of[lo:hi] >= 0) & (self.groups.counts[lo:hi] == 0)).sum().float().reshape(1)
-            grad_mul = self._clip_factor(sparse, g_bD, clip_grad_norm, extra_fired=got_aux)
+        lo, hi = self.own_rows
+        got_aux = ((row_of[lo:hi] >= 0) & (self.groups.counts[lo:hi] == 0)).sum().float().reshape(1)
+        grad_mul = self._clip_factor(sparse, g_bD, clip_grad_norm, extra_fired=got_aux)
         sparse(grad_mul, None, True)
         self._mark("sparse_grad_adam")
         if self.bD is not None:

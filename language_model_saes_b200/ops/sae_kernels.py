@@ -720,6 +720,54 @@ def adam_flat(p, g, m, v, lr, beta1, beta2, eps, step, grad_mul=None, shadow=Non
     _ext().adam_flat(p, g, m, v, grad_mul, shadow, grad_sq_sum, lr, beta1, beta2, eps, step, update, status_buffer(p.device))
 
 
+def adam_turned(params, moments, grads, shadows, lr, beta1, beta2, eps, step) -> None:
+    """Adam on one or two fp32 parameters ``[heads, d, w]`` of one shape whose gradients come as ``[heads * w, d]``, and their bf16 shadows
+    ``[heads * w, d]``, in one pass."""
+    if not params[0].is_cuda:
+        for p, (m, v), g, sh in zip(params, moments, grads, shadows):
+            h, d, w = p.shape
+            ref_adam(p, g.view(h, w, d).permute(0, 2, 1), m, v, lr, beta1, beta2, eps, step)
+            sh.copy_(p.permute(0, 2, 1).reshape(h * w, d))
+        return
+    _ext().adam_turned(params, [m for m, _ in moments], [v for _, v in moments], grads, shadows, lr, beta1, beta2, eps, step,
+                       status_buffer(params[0].device))  # fmt: skip
+
+
+class BiasUpdate:
+    """The end of a step in one launch: the gradients of biases are column sums of bf16 matrices, Adam is applied to them, and the step's
+    loss sum becomes the mean loss. Belongs to one engine, whose steps follow each other on a stream (the launch's arrival
+    counters are its scratch); other cases (gradient factors, norms) take ``colsum_bf16`` and ``adam_flat``."""
+
+    MAX = 16  # matrices per launch (kMaxColsumSegs in csrc/kernels.h)
+
+    def __init__(self, widths: list[int], device: torch.device):
+        self.counters = torch.zeros(max(1, sum(-(-w // 256) for w in widths)), dtype=torch.int32, device=device)
+
+    def __call__(self, mats, params, moments, lr, beta1, beta2, eps, step, loss_sum=None, loss_sum2=None, loss_weight=None, loss_den: float = 1.0):
+        """``mats[i] [rows, d_i]`` bf16, ``params[i] [d_i]`` fp32 with ``moments[i] = (m, v)``. With ``loss_sum`` (1 element): returns
+        ``loss_sum / den`` (and with ``loss_sum2``: the mean of both and its share) as 0-d tensors and leaves the sums at zero; ``den`` is
+        ``loss_den`` times the sum of ``loss_weight`` when that is given."""
+        while len(mats) > self.MAX:
+            self(mats[: self.MAX], params[: self.MAX], moments[: self.MAX], lr, beta1, beta2, eps, step)
+            mats, params, moments = mats[self.MAX :], params[self.MAX :], moments[self.MAX :]
+        if native_ok := (self.counters.is_cuda and all(a.shape[1] % 8 == 0 and a.data_ptr() % 16 == 0 and a.is_contiguous() for a in mats)):
+            out = _ext().colsum_adam(mats, [p.view(-1) for p in params], [m.view(-1) for m, _ in moments], [v.view(-1) for _, v in moments],
+                                     self.counters, lr, beta1, beta2, eps, step, loss_sum, loss_sum2, loss_weight, loss_den,
+                                     status_buffer(self.counters.device))  # fmt: skip
+        else:
+            for a, p, (m, v) in zip(mats, params, moments):
+                adam_flat(p.view(-1), colsum_bf16(a), m.view(-1), v.view(-1), lr, beta1, beta2, eps, step)
+        if loss_sum is None:
+            return None
+        if not native_ok:
+            den = loss_den if loss_weight is None else loss_weight.sum() * loss_den
+            out = [(loss_sum / den).squeeze(0)] if loss_sum2 is None else [((loss_sum + loss_sum2) / den).squeeze(0), (loss_sum2 / den).squeeze(0)]
+            loss_sum.zero_()
+            if loss_sum2 is not None:
+                loss_sum2.zero_()
+        return out[0] if loss_sum2 is None else tuple(out)
+
+
 def row_norm_shadow(W: torch.Tensor, norm: torch.Tensor | None, shadow: torch.Tensor | None) -> None:
     """norm[f] = ||W[f,:]||_2 and shadow = bf16(W) in one pass."""
     if not W.is_cuda:
