@@ -810,6 +810,49 @@ void attn_delta(const Tensor& dout, const Tensor& out, const Tensor& delta) {
              "attn_delta launch");
 }
 
+// ---- low-rank sparse attention step ---------------------------------------------------------------------
+// Whether lorsa_dz takes rows of F features and lists of k codes.
+bool lorsa_dz_fits(int64_t F, int64_t k) {
+  return F > 0 && k > 0 && F % 8 == 0 && F < (1 << 20) && k < (1 << 16) && lmsae::lorsa_dz_smem((int)F, (int)k) <= 200 * 1024;
+}
+
+// idx int32, act, dact fp32 [tokens, k] -> dz bf16 [tokens, F] (written whole), delta fp32 [batch, heads, seq].
+void lorsa_dz(const Tensor& idx, const Tensor& act, const Tensor& dact, const Tensor& dz, const Tensor& delta) {
+  CHECK_T(idx, torch::kInt32); CHECK_T(act, torch::kFloat32); CHECK_T(dact, torch::kFloat32); CHECK_T(dz, torch::kBFloat16); CHECK_T(delta, torch::kFloat32);
+  TORCH_CHECK(idx.dim() == 2 && act.sizes() == idx.sizes() && dact.sizes() == idx.sizes() && dz.dim() == 2 && dz.size(0) == idx.size(0), "lorsa_dz: shapes");
+  TORCH_CHECK(delta.dim() == 3 && delta.size(0) * delta.size(2) == idx.size(0) && delta.size(1) > 0 && dz.size(1) % delta.size(1) == 0, "lorsa_dz: delta [b, h, s]");
+  TORCH_CHECK(lorsa_dz_fits(dz.size(1), idx.size(1)) && reinterpret_cast<uintptr_t>(dz.data_ptr()) % 16 == 0, "lorsa_dz: rows of F % 8 == 0 that fit shared memory");
+  const c10::cuda::CUDAGuard guard(idx.device());
+  check_cuda(lmsae::lorsa_dz_launch(idx.data_ptr<int>(), act.data_ptr<float>(), dact.data_ptr<float>(), idx.size(0), (int)idx.size(1), (int)dz.size(1),
+                                    (int)delta.size(1), (int)(dz.size(1) / delta.size(1)), (int)delta.size(2),
+                                    reinterpret_cast<__nv_bfloat16*>(dz.data_ptr()), delta.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "lorsa_dz launch");
+}
+
+// One or two parameter sets of one shape: p, m, v fp32 [heads, d, w]; g fp32 and shadow bf16 [heads * w, d].
+void adam_turned(const std::vector<Tensor>& p, const std::vector<Tensor>& m, const std::vector<Tensor>& v, const std::vector<Tensor>& g,
+                 const std::vector<Tensor>& shadow, double lr, double beta1, double beta2, double eps, int64_t step, const Tensor& status) {
+  const size_t n = p.size();
+  TORCH_CHECK(n >= 1 && n <= 2 && m.size() == n && v.size() == n && g.size() == n && shadow.size() == n, "adam_turned: one or two sets");
+  CHECK_T(status, torch::kInt32);
+  lmsae::AdamTurnedParams q{};
+  for (size_t i = 0; i < n; ++i) {
+    CHECK_T(p[i], torch::kFloat32); CHECK_T(m[i], torch::kFloat32); CHECK_T(v[i], torch::kFloat32); CHECK_T(g[i], torch::kFloat32);
+    CHECK_T(shadow[i], torch::kBFloat16);
+    TORCH_CHECK(p[i].dim() == 3 && p[i].sizes() == p[0].sizes() && m[i].sizes() == p[i].sizes() && v[i].sizes() == p[i].sizes(), "adam_turned: p, m, v [heads, d, w]");
+    TORCH_CHECK(g[i].dim() == 2 && g[i].size(0) == p[i].size(0) * p[i].size(2) && g[i].size(1) == p[i].size(1) && shadow[i].sizes() == g[i].sizes(),
+                "adam_turned: g, shadow [heads * w, d]");
+    q.set[i] = {p[i].data_ptr<float>(), m[i].data_ptr<float>(), v[i].data_ptr<float>(), g[i].data_ptr<float>(), reinterpret_cast<__nv_bfloat16*>(shadow[i].data_ptr())};
+  }
+  q.heads = (int)p[0].size(0);
+  q.d = (int)p[0].size(1);
+  q.w = (int)p[0].size(2);
+  q.h = make_hyper(lr, beta1, beta2, eps, step);
+  q.status = status.data_ptr<int>();
+  const c10::cuda::CUDAGuard guard(p[0].device());
+  check_cuda(lmsae::adam_turned_launch(q, (int)n, at::cuda::getCurrentCUDAStream()), "adam_turned launch");
+}
+
 // ---- selection / compaction ----------------------------------------------------------------------------
 int dtype_code(const Tensor& t) {
   if (t.scalar_type() == torch::kFloat32) return 0;
@@ -1279,7 +1322,8 @@ std::map<std::string, std::vector<int64_t>> bounds_report() {
   std::map<std::string, std::vector<int64_t>> out;
   const std::pair<const char*, int (*)(int*)> units[] = {  // every file whose kernels check an index
       {"sparse_ops.cu", lmsae::bounds_fetch_sparse_ops}, {"comm_ops.cu", lmsae::bounds_fetch_comm_ops}, {"grad_adam.cu", lmsae::bounds_fetch_grad_adam},
-      {"clt_ops.cu", lmsae::bounds_fetch_clt_ops}, {"dense_decode.cu", lmsae::bounds_fetch_dense_decode}};
+      {"clt_ops.cu", lmsae::bounds_fetch_clt_ops}, {"dense_decode.cu", lmsae::bounds_fetch_dense_decode},
+      {"lorsa_ops.cu", lmsae::bounds_fetch_lorsa_ops}};
   for (const auto& [name, fetch] : units) {
     int rec[4];
     check_cuda(fetch(rec), name);
@@ -1318,6 +1362,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_delta", &attn_delta);
+  m.def("lorsa_dz", &lorsa_dz);
+  m.def("lorsa_dz_fits", &lorsa_dz_fits);
+  m.def("adam_turned", &adam_turned);
   m.def("radix_hi_bins", &radix_hi_bins);
   m.def("radix_hist", &radix_hist);
   m.def("radix_pick", &radix_pick);

@@ -105,6 +105,7 @@ int bounds_fetch_comm_ops(int* out);
 int bounds_fetch_grad_adam(int* out);
 int bounds_fetch_clt_ops(int* out);
 int bounds_fetch_dense_decode(int* out);
+int bounds_fetch_lorsa_ops(int* out);
 
 struct DecodeParams {
   const int* idx;
@@ -316,6 +317,23 @@ int attn_value_chunk(int dv);
 int attn_fwd_value_chunk(int dqk, int dv);
 int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                     cudaStream_t stream);
+
+// ---- low-rank sparse attention step (lorsa_ops.cu) ----------------------------------------------------
+int lorsa_dz_smem(int F, int k);
+int lorsa_dz_launch(const int* idx, const float* act, const float* dact, long long tokens, int k, int F, int heads, int group, int seq,
+                    __nv_bfloat16* dz, float* delta, cudaStream_t stream);
+struct AdamTurnedSet {
+  float *p, *m, *v;        // [heads, d, w]
+  const float* g;          // [heads * w, d]
+  __nv_bfloat16* shadow;   // [heads * w, d]
+};
+struct AdamTurnedParams {
+  AdamTurnedSet set[2];
+  int heads, d, w;
+  AdamHyper h;
+  const int* status;
+};
+int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t stream);
 
 // ---- elementwise (jumprelu.cu) ---------------------------------------------------------------------
 int jumprelu_launch(int dtype, const void* x, const void* log_theta, const void* dy, void* out, float* dlog, long long n,

@@ -241,11 +241,18 @@ class FusedLorsaStep:
             q, k = self._rotated(qn.detach(), kn.detach())
         else:
             q, k, v = self._project(X, b, s)
-        # the attention alone keeps an autograd node (its backward is the library's); everything around it is explicit
-        ql, kl, vl = (t.detach().requires_grad_(True) for t in (q, k, v))
-        with torch.enable_grad():
-            out = self._attention(ql, kl, vl)  # [b, h, s, group]
-        z = out.detach().permute(0, 2, 1, 3).reshape(T_l, self.F)
+        kernels = (x.is_cuda and self.attention == "tensor_core" and attention_kernels.supported(q, v)
+                   and K._ext().lorsa_dz_fits(self.F, min(k_top, self.F)))  # fmt: skip
+        if kernels:
+            q, k, v = (t.contiguous() for t in (q, k, v))
+            out, lse = attention_kernels.causal_attention_fwd(q, k, v, 1.0 / self.m.attn_scale, want_lse=True)
+            z = out.view(T_l, self.F)
+        else:
+            # the attention alone keeps an autograd node (its backward is the library's); everything around it is explicit
+            ql, kl, vl = (t.detach().requires_grad_(True) for t in (q, k, v))
+            with torch.enable_grad():
+                out = self._attention(ql, kl, vl)  # [b, h, s, group]
+            z = out.detach().permute(0, 2, 1, 3).reshape(T_l, self.F)
         idx, act = self._select(z, k_top)
         self.loss_sum.zero_()
         WO16 = self.WO16
@@ -265,10 +272,15 @@ class FusedLorsaStep:
             dxhat = K.mse_loss_grad(xhat, Y, bD, row_weight, grad_scale, self.loss_sum)
             dact = K.sparse_dact(idx, WO16, dxhat)
         # d z: the activation passes the gradient where a head was selected (its value is the pre-activation itself)
-        dz = torch.zeros(T_l, self.F + 8, dtype=z.dtype if z.is_cuda else torch.float32, device=x.device)
-        dz.scatter_(1, torch.where(idx >= 0, idx, torch.full_like(idx, self.F)).long(), dact.to(dz.dtype))
-        dz = dz[:, : self.F].reshape(b, s, self.h, self.group_size).permute(0, 2, 1, 3)
-        dq, dk, dv = torch.autograd.grad(out, (ql, kl, vl), dz.to(out.dtype))
+        if kernels:
+            dz, delta = torch.empty_like(z), torch.empty_like(lse)
+            K._ext().lorsa_dz(idx, act, dact, dz, delta)
+            dq, dk, dv = attention_kernels.causal_attention_bwd(q, k, v, dz.view(v.shape), lse, delta, 1.0 / self.m.attn_scale, torch.bfloat16)
+        else:
+            dz = torch.zeros(T_l, self.F + 8, dtype=z.dtype if z.is_cuda else torch.float32, device=x.device)
+            dz.scatter_(1, torch.where(idx >= 0, idx, torch.full_like(idx, self.F)).long(), dact.to(dz.dtype))
+            dz = dz[:, : self.F].reshape(b, s, self.h, self.group_size).permute(0, 2, 1, 3)
+            dq, dk, dv = torch.autograd.grad(out, (ql, kl, vl), dz.to(out.dtype))
         if self.rotary:
             dq, dk = rotate_pair(dq, dk, self.m.rotary_cos, self.m.rotary_sin, self.m.cfg.rotary_adjacent_pairs, inverse=True)
         norm_grads = {}
@@ -282,11 +294,28 @@ class FusedLorsaStep:
         dK = dk.reshape(T_l, self.h * self.dqk).to(low)
         dV = dv.reshape(T_l, self.F).to(low)
         Xl = X.to(low)
+        gQ, gK, gV = _mm_f32(dQ.t(), Xl), _mm_f32(dK.t(), Xl), _mm_f32(dV.t(), Xl)  # Q, K: [head x channel, d]
+        b1, b2 = self.betas
+        if self.dp == 1:
+            if not early_WO:
+                self.t += 1
+                self._update_WO(idx, act, dact, dxhat, lr)
+            adam = (lr, b1, b2, self.eps, self.t)
+            P, M = self.params, self.state
+            K.adam_turned([P["W_Q"], P["W_K"]], [M["W_Q"], M["W_K"]], [gQ, gK], [self.WQ16, self.WK16], *adam)
+            self._adam("W_V", gV, lr)
+            for name, g in norm_grads.items():
+                self._adam(name, g, lr)
+            biases = {"b_Q": dQ, "b_K": dK, "b_V": dV} | ({} if bD is None else {"b_D": dxhat})
+            return self.bias_update(list(biases.values()), [P[n] for n in biases], [M[n] for n in biases], *adam, self.loss_sum, loss_den=float(T))
+        # Replicas: the dense gradients (some 50 MB at 8192 heads) are summed in one collective on a flat buffer; for W_O the
+        # codes and the output gradient of every replica (a few MB) are gathered and each replica rebuilds the same rows, so
+        # that no dense [F, d] gradient exists here either. Every replica then applies the same update.
         grads = {
             # [head x channel, d] -> the parameter's [head, d, channel]
-            "W_Q": _mm_f32(dQ.t(), Xl).view(self.h, self.dqk, d).permute(0, 2, 1).contiguous(),
-            "W_K": _mm_f32(dK.t(), Xl).view(self.h, self.dqk, d).permute(0, 2, 1).contiguous(),
-            "W_V": _mm_f32(dV.t(), Xl),
+            "W_Q": gQ.view(self.h, self.dqk, d).permute(0, 2, 1).contiguous(),
+            "W_K": gK.view(self.h, self.dqk, d).permute(0, 2, 1).contiguous(),
+            "W_V": gV,
             "b_Q": dQ.sum(0, dtype=torch.float32).view(self.h, self.dqk),
             "b_K": dK.sum(0, dtype=torch.float32).view(self.h, self.dqk),
             "b_V": dV.sum(0, dtype=torch.float32),
