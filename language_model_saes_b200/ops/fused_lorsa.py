@@ -13,11 +13,12 @@ them small element-wise kernels that autograd and autocast put around the few pr
 3. radix row top-k of ``z * ||W_O row||`` (positive entries)          -> codes (idx, act) [tokens, k]
 4. sparse decode fused with the loss, d x_hat and d act (the kernel of the TopK SAE step; feature shards: sparse decode,
    all-reduce, loss kernel, code-gradient kernel)
-5. d z = d act scattered to its positions; attention backward (the dQ and dK/dV kernels, or the library's, through a
-   one-node autograd call on the attention alone); inverse rotation of d q, d k
-6. three library GEMMs for the projection gradients (``d q^T x`` ...), column sums for the biases
+5. d z = d act at its positions, with the attention backward's row statistics from the same codes; attention backward (the dQ
+   and dK/dV kernels, or the library's, through a one-node autograd call on the attention alone); inverse rotation of d q, d k
+6. three library GEMMs for the projection gradients (``d q^T x`` ...)
 7. updates: ``W_O`` by the sparse gradient + Adam kernel (rows rebuilt from the codes, bf16 shadow and row norms in the
-   same pass), the dense projections and biases by the flat Adam kernel.
+   same pass), ``W_Q`` and ``W_K`` with their transposed gradients and shadows in one pass, ``W_V`` by the flat Adam kernel, the biases
+   (column sums and Adam) in one launch.
 
 Restrictions: ``topk`` activation, rotary or no positional embedding (no ``rotary_scale``; the per-head RMS norm of Q and K
 only on request, see ``QK_NORM_ON_FUSED_PATH``), Adam, fp32
@@ -113,6 +114,7 @@ class FusedLorsaStep:
         self.WV16, self.WO16 = bf(self.F, self.d), bf(self.F, self.d)
         self.dec_norm = torch.empty(self.F, dtype=torch.float32, device=dev)
         self.loss_sum = torch.zeros(1, dtype=torch.float32, device=dev)
+        self.bias_update = K.BiasUpdate([self.d, self.h * self.dqk, self.h * self.dqk, self.F], dev)
         self.groups: K.FeatureGroups | None = None
         self.t = 0
         self.refresh()
@@ -323,29 +325,26 @@ class FusedLorsaStep:
         if bD is not None:
             grads["b_D"] = K.colsum_bf16(dxhat)
         grads.update(norm_grads)
-        if self.dp > 1:
-            # Replicas: the dense gradients (some 50 MB at 8192 heads) are summed in one collective on a flat buffer; for W_O the
-            # codes and the output gradient of every replica (a few MB) are gathered and each replica rebuilds the same rows, so
-            # that no dense [F, d] gradient exists here either. Every replica then applies the same update.
-            names = list(grads)
-            flat = torch.cat([grads[n].reshape(-1) for n in names])
-            dist.all_reduce(flat, group=self.dp_group)
-            off = 0
-            for n in names:
-                grads[n] = flat[off : off + grads[n].numel()].view(grads[n].shape)
-                off += grads[n].numel()
-            idx, act, dact, dxhat = (self._gather_rows(t) for t in (idx, act, dact, dxhat))
-            dist.all_reduce(self.loss_sum, group=self.dp_group)
-        if not early_WO:
-            self.t += 1
-            self._update_WO(idx, act, dact, dxhat, lr)
-        b1, b2 = self.betas
+        names = list(grads)
+        flat = torch.cat([grads[n].reshape(-1) for n in names])
+        dist.all_reduce(flat, group=self.dp_group)
+        off = 0
+        for n in names:
+            grads[n] = flat[off : off + grads[n].numel()].view(grads[n].shape)
+            off += grads[n].numel()
+        idx, act, dact, dxhat = (self._gather_rows(t) for t in (idx, act, dact, dxhat))
+        dist.all_reduce(self.loss_sum, group=self.dp_group)
+        self.t += 1
+        self._update_WO(idx, act, dact, dxhat, lr)
         for name, g in grads.items():
-            m_, v_ = self.state[name]
-            shadow = self.WV16.view(-1) if name == "W_V" else None
-            K.adam_flat(self.params[name].view(-1), g.reshape(-1), m_.view(-1), v_.view(-1), lr, b1, b2, self.eps, self.t, shadow=shadow)
+            self._adam(name, g, lr)
         self._refresh_qk()
         return (self.loss_sum / T).squeeze(0)
+
+    def _adam(self, name: str, g: torch.Tensor, lr: float) -> None:
+        m_, v_ = self.state[name]
+        shadow = self.WV16.view(-1) if name == "W_V" else None
+        K.adam_flat(self.params[name].view(-1), g.reshape(-1), m_.view(-1), v_.view(-1), lr, *self.betas, self.eps, self.t, shadow=shadow)
 
     def _update_WO(self, idx, act, dact, dxhat, lr: float, dact_mode: int = 0) -> None:
         """W_O: rows rebuilt from the codes (act x d x_hat), Adam, bf16 shadow and row norms in one pass."""
