@@ -810,6 +810,31 @@ void attn_delta(const Tensor& dout, const Tensor& out, const Tensor& delta) {
              "attn_delta launch");
 }
 
+// dtheta[f] += -theta / window * sum over tokens inside the window of (d x_hat . W_D[f] / norm + add_per_hit).
+void window_grad_gemm(const Tensor& dxhat, const Tensor& W, const Tensor& S, const Tensor& norm, const Tensor& theta, double window,
+                      double add_per_hit, const Tensor& dtheta, const Tensor& status) {
+  CHECK_T(dxhat, torch::kBFloat16); CHECK_T(W, torch::kBFloat16); CHECK_T(S, torch::kBFloat16);
+  CHECK_T(norm, torch::kFloat32); CHECK_T(theta, torch::kFloat32); CHECK_T(dtheta, torch::kFloat32); CHECK_T(status, torch::kInt32);
+  TORCH_CHECK(dxhat.dim() == 2 && W.dim() == 2 && S.dim() == 2 && W.size(1) == dxhat.size(1) && S.size(0) == dxhat.size(0) && S.size(1) == W.size(0),
+              "window_grad_gemm: dxhat [B, d], W [F, d], S [B, F]");
+  lmsae::WindowGradParams p{};
+  p.B = (int)dxhat.size(0);
+  p.F = (int)W.size(0);
+  p.d = (int)W.size(1);
+  TORCH_CHECK(norm.numel() == p.F && theta.numel() == p.F && dtheta.numel() == p.F && p.F % 8 == 0 && p.d % 8 == 0, "window_grad_gemm: F and d multiples of 8");
+  p.norm = norm.data_ptr<float>();
+  p.theta = theta.data_ptr<float>();
+  p.window = (float)window;
+  p.add_per_hit = (float)add_per_hit;
+  p.dtheta = dtheta.data_ptr<float>();
+  p.status = status.data_ptr<int>();
+  const c10::cuda::CUDAGuard guard(W.device());
+  const CUtensorMap tw = make_bf16_tile_map(W.data_ptr(), p.F, p.d, 128);
+  const CUtensorMap tg = make_bf16_tile_map(dxhat.data_ptr(), p.B, p.d, 128);
+  const CUtensorMap ts = make_bf16_tile_map(S.data_ptr(), p.B, p.F, 128);
+  check_cuda(lmsae::window_grad_gemm_launch(tw, tg, ts, p, at::cuda::getCurrentCUDAStream()), "window_grad_gemm launch");
+}
+
 // ---- low-rank sparse attention step ---------------------------------------------------------------------
 // Whether lorsa_dz takes rows of F features and lists of k codes.
 bool lorsa_dz_fits(int64_t F, int64_t k) {
@@ -1363,6 +1388,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_delta", &attn_delta);
   m.def("lorsa_dz", &lorsa_dz);
+  m.def("window_grad_gemm", &window_grad_gemm);
   m.def("lorsa_dz_fits", &lorsa_dz_fits);
   m.def("adam_turned", &adam_turned);
   m.def("radix_hi_bins", &radix_hi_bins);

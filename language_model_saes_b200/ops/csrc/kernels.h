@@ -335,6 +335,18 @@ struct AdamTurnedParams {
 };
 int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t stream);
 
+// ---- threshold gradient of a JumpReLU head in the epilogue of its product (window_grad_gemm.cu) -------------
+struct WindowGradParams {
+  int B, F, d;
+  const float* norm;   // [F]
+  const float* theta;  // [F]
+  float window, add_per_hit;
+  float* dtheta;       // [F], added to
+  int* status;
+};
+// maps with boxes of 128 rows x 64 columns: W_D [F, d], d x_hat [B, d], S [B, F]
+int window_grad_gemm_launch(const CUtensorMap& tw, const CUtensorMap& tg, const CUtensorMap& ts, const WindowGradParams& p, cudaStream_t stream);
+
 // ---- elementwise (jumprelu.cu) ---------------------------------------------------------------------
 int jumprelu_launch(int dtype, const void* x, const void* log_theta, const void* dy, void* out, float* dlog, long long n,
                     int P, float window, int backward, cudaStream_t stream);

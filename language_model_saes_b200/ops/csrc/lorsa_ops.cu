@@ -11,7 +11,7 @@ LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_lorsa_ops)
 // dz[t, :] is bf16(dact) at the selected heads and zero elsewhere; delta[b, h, s] = sum over the head's group of dz * z, where z is the
 // code itself, so that it needs neither z nor a pass over dz. One CTA per token: the row is put together in shared memory and
 // leaves in 16-byte stores, a thread per QK head adds up its group's products in slot order. Bound by writing dz:
-// 2048 tokens of 8192: 33 MB. (As tensor operations: fill, scatter, three copies and the sum of a product: 130 us; here 9.)
+// 2048 tokens of 8192: 33 MB. (As tensor operations: fill, scatter, three copies and the sum of a product: 130 us; here 14.)
 __global__ void __launch_bounds__(256)
 lorsa_dz_kernel(const int* __restrict__ idx, const float* __restrict__ act, const float* __restrict__ dact, int k, int F, int heads, int group, int seq,
                 __nv_bfloat16* __restrict__ dz, float* __restrict__ delta) {
@@ -60,8 +60,8 @@ int lorsa_dz_launch(const int* idx, const float* act, const float* dact, long lo
 // ---------------------------------------------------------------------------------------------
 // Parameters and moments are [heads, d, w] fp32, the gradient comes out of the product as [heads * w, d] and the products read bf16
 // weights as [heads * w, d]: one pass per 64 x 64 tile turns the gradient on its way in and the new weights on their way out through
-// shared memory. As separate passes the gradient and the weights were transposed through memory (2 x 22 us for 3.1 M
-// parameters each, on top of Adam's 16). Up to two parameter sets of one shape share a launch.
+// shared memory. As separate passes the gradients and weights were transposed through memory (66 us for two times 3.1 M
+// parameters, on top of Adam's 36; here 51). Up to two parameter sets of one shape share a launch.
 __global__ void __launch_bounds__(256)
 adam_turned_kernel(const AdamTurnedParams p) {
   __shared__ float tile[64][65];  // [w][d]

@@ -283,10 +283,10 @@ class FusedCrosscoderStep:
             # threshold gradient: dense part (reconstruction gradient at every entry inside the window) ...
             # (the tanh penalty's derivative with respect to the JumpReLU output is coef at every entry with zero activation:
             # the dense pass adds it per window hit)
-            G = K.encoder_hidden(dxhat, self.WD_bf16[h], None)  # [B, F] bf16 = d x_hat . W_D^T
             if mult is None:
-                S.jumprelu_window_grad(G, S_sum, n_h, theta, self.window, dtheta, add_per_hit=coef if l1_coefficient else 0.0)
+                S.jumprelu_window_grad_of_product(dxhat, self.WD_bf16[h], S_sum, n_h, theta, self.window, dtheta, add_per_hit=coef if l1_coefficient else 0.0)
             else:
+                G = K.encoder_hidden(dxhat, self.WD_bf16[h], None)  # [B, F] bf16 = d x_hat . W_D^T
                 # the per-hit term carries a per-feature factor here: the kernel runs with 0 and with 1 per hit; the difference
                 # of the two sums is (hits of the feature) x (-theta / window), which is then scaled by coef x factor
                 d0 = torch.zeros(F, dtype=torch.float32, device=x.device)
@@ -408,8 +408,7 @@ class FusedCrosscoderStep:
                                                want_dval=False)  # fmt: skip
             # threshold gradient: the reconstruction gradient at every entry inside the window (the tanh penalty's derivative at
             # zero activation is coef at every entry: the dense pass adds it per window hit)
-            G = K.encoder_hidden(dxhat, self.WD_bf16[h], None)  # [B, F] bf16 = d x_hat . W_D^T
-            S.jumprelu_window_grad(G, S_sum, self.dec_norm[h], theta, self.window, dtheta, add_per_hit=coef)
+            S.jumprelu_window_grad_of_product(dxhat, self.WD_bf16[h], S_sum, self.dec_norm[h], theta, self.window, dtheta, add_per_hit=coef)
             K.sparse_grad_adam(self.groups, act[h], dS, dxhat, dxhat, self.WD[h], mD[h], vD[h], self.WD_bf16[h], None, None, None, None, None,
                                None, None, self.dec_norm[h], None, None, lr, b1, b2, self.eps, self.t, True,
                                wd_self_scale=self_scale[h] if self_scale is not None else None, dact_mode=2)  # fmt: skip

@@ -284,6 +284,15 @@ def jumprelu_window_grad(G: torch.Tensor, S: torch.Tensor, n: torch.Tensor, thet
                                   float(add_per_hit), dtheta)
 
 
+def jumprelu_window_grad_of_product(dxhat: torch.Tensor, W: torch.Tensor, S: torch.Tensor, n: torch.Tensor, theta: torch.Tensor, window: float,
+                                    dtheta: torch.Tensor, add_per_hit: float = 0.0) -> None:  # fmt: skip
+    """``jumprelu_window_grad`` with ``G = dxhat W^T`` (``dxhat [B, d]``, ``W [F, d]``, bf16 on the GPU), which the kernel keeps to itself."""
+    if not (dxhat.is_cuda and S.dtype == torch.bfloat16 and W.shape[0] % 8 == 0 and W.shape[1] % 8 == 0):
+        return jumprelu_window_grad(K.encoder_hidden(dxhat, W, None), S, n, theta, window, dtheta, add_per_hit)
+    K._ext().window_grad_gemm(dxhat, W, S.contiguous(), n.contiguous(), theta.contiguous(), float(window), float(add_per_hit), dtheta,
+                              K.status_buffer(W.device))  # fmt: skip
+
+
 def _ref_threshold_rows_to_sparse(g, thr, col_div, width_group, n_ties, tie_group, cap=None, overflow=None):
     """Plain-torch statement of ``threshold_rows_to_sparse`` (any device): same selection, same order."""
     gf = g.float()
