@@ -209,50 +209,64 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
              "topk_merge launch");
 }
 
-// C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu); na [M] and ends [2, N] (both optional): what
-// topk_estimate takes, made with its bias [N] and gate [N] (both optional). status: int32 [4], zeroed, of this call alone: a wait in the
-// product that runs out is recorded there, and everything is done on the fp32 pipes then. tensor_cores = false leaves the product out (as if it had given up).
+// C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu). With na [M] (written: the rows' norms) C is bf16 and
+// receives the lower ends that topk_estimate takes, made with bias [N] and gate [N] (both optional); top: int32 [2], zeroed, goes with
+// them. status: int32 [4], zeroed, of this call alone: a wait in the product that runs out is recorded there, and everything is done on the
+// fp32 pipes then (lower ends: by topk_estimate). tensor_cores = false leaves the product out (as if it had given up).
 void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
-               const c10::optional<Tensor>& ends, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
+               const c10::optional<Tensor>& top, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
                bool tensor_cores, int64_t workspace) {
+  const bool ends = na.has_value();
   CHECK_T(A, torch::kFloat32);
   CHECK_T(B, torch::kFloat32);
-  CHECK_T(C, torch::kFloat32);
+  CHECK_T(C, ends ? torch::kBFloat16 : torch::kFloat32);
   CHECK_T(status, torch::kInt32);
   TORCH_CHECK(A.dim() == 2 && B.dim() == 2 && C.dim() == 2 && A.size(1) == B.size(1) && C.size(0) == A.size(0) && C.size(1) == B.size(0),
               "A [M,K], B [N,K], C [M,N]");
-  const int64_t M = A.size(0), N = B.size(0), K = A.size(1), kp = (K + 63) / 64 * 64;
-  TORCH_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && M < INT_MAX - 256 && N < INT_MAX - 256 && 3 * kp < INT_MAX, "unsupported sizes");
-  if (na.has_value()) { CHECK_T(*na, torch::kFloat32); TORCH_CHECK(na->numel() == M); }
-  if (ends.has_value()) { CHECK_T(*ends, torch::kInt32); TORCH_CHECK(ends->numel() == 2 * N); }
+  const int64_t M = A.size(0), N = B.size(0), K = A.size(1), kp = (K + 63) / 64 * 64, parts = ends ? 2 : 3;
+  TORCH_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && M < INT_MAX - 256 && N < INT_MAX - 256 && parts * kp < INT_MAX, "unsupported sizes");
+  TORCH_CHECK(ends == top.has_value() && (ends || (!bias.has_value() && !gate.has_value())) && (!ends || tensor_cores), "na and top go together, and bias and gate with them");
+  if (ends) {
+    CHECK_T(*na, torch::kFloat32);
+    CHECK_T(*top, torch::kInt32);
+    TORCH_CHECK(na->numel() == M && top->numel() == 2);
+  }
   for (const auto* t : {&bias, &gate}) {
     if (t->has_value()) { CHECK_T(**t, torch::kFloat32); TORCH_CHECK((*t)->numel() == N); }
   }
   const c10::cuda::CUDAGuard guard(A.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const auto b16 = A.options().dtype(torch::kBFloat16), i32 = A.options().dtype(torch::kInt32);
-  // B in pieces of whole tiles, so that the parts of a large dictionary (6 bytes an element) need no more than `workspace` bytes
+  // B in pieces of whole tiles, so that the parts of a large dictionary (two bytes each) need no more than `workspace` bytes
   int64_t step = N;
-  if (N * kp * 6 > workspace) step = std::max<int64_t>(1, workspace / (kp * 6 * 256)) * 256;
+  if (N * kp * 2 * parts > workspace) step = std::max<int64_t>(1, workspace / (kp * 2 * parts * 256)) * 256;
   step = std::min(step, N);
   const int64_t steps = (N + step - 1) / step;
-  const Tensor As = torch::empty({M, 3 * kp}, b16), Bs = torch::empty({step, 3 * kp}, b16);
+  const Tensor As = torch::empty({M, parts * kp}, b16), Bs = torch::empty({step, parts * kp}, b16);
   const Tensor flags = torch::zeros({1 + M + N + steps}, i32);
+  const Tensor nb = ends ? torch::empty({N}, A.options()) : Tensor();
   int* fa = flags.data_ptr<int>();
   int* fb = fa + 1 + M;
-  check_cuda(lmsae::split_bf16x3_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa, opt_ptr<float>(na), nullptr, 0, nullptr, nullptr, stream), "split");
-  const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, 3 * kp, 128);
+  check_cuda(lmsae::split_bf16_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, (int)parts, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa,
+                                      opt_ptr<float>(na), nullptr, nullptr, nullptr, stream), "split");
+  const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, parts * kp, 128);
   for (int64_t n0 = 0; n0 < N; n0 += step) {
     const int64_t n = std::min(step, N - n0);
     const float* Bn = B.data_ptr<float>() + n0 * K;
-    check_cuda(lmsae::split_bf16x3_launch(Bn, (int)n, (int)K, (int)kp, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nullptr,
-                                          ends.has_value() ? reinterpret_cast<uint32_t*>(ends->data_ptr<int>()) + n0 : nullptr, (int)N,
-                                          bias.has_value() ? bias->data_ptr<float>() + n0 : nullptr, gate.has_value() ? gate->data_ptr<float>() + n0 : nullptr, stream),
-               "split");
-    const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), n, 3 * kp, 128);
-    check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), Bn, (int)M, (int)n, (int)K, (int)kp, fa, fb, C.data_ptr<float>() + n0, N,
-                                       status.data_ptr<int>(), tensor_cores, stream),
-               "fp32_gemm launch");
+    const float* bias_n = bias.has_value() ? bias->data_ptr<float>() + n0 : nullptr;
+    const float* gate_n = gate.has_value() ? gate->data_ptr<float>() + n0 : nullptr;
+    float* nb_n = ends ? nb.data_ptr<float>() + n0 : nullptr;
+    check_cuda(lmsae::split_bf16_launch(Bn, (int)n, (int)K, (int)kp, (int)parts, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nb_n,
+                                        ends ? reinterpret_cast<uint32_t*>(top->data_ptr<int>()) : nullptr, bias_n, gate_n, stream), "split");
+    const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), n, parts * kp, 128);
+    if (ends)
+      check_cuda(lmsae::fp32_ends_launch(ta, tb, (int)M, (int)n, (int)K, (int)kp, na->data_ptr<float>(), nb_n, bias_n, gate_n,
+                                         reinterpret_cast<__nv_bfloat16*>(C.data_ptr()) + n0, N, status.data_ptr<int>(), stream),
+                 "fp32_ends launch");
+    else
+      check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), Bn, (int)M, (int)n, (int)K, (int)kp, fa, fb, C.data_ptr<float>() + n0, N,
+                                         status.data_ptr<int>(), tensor_cores, stream),
+                 "fp32_gemm launch");
     fb += 1 + n;
   }
 }
@@ -270,22 +284,24 @@ void topk_dense(const Tensor& h, const c10::optional<Tensor>& bias, const c10::o
              "topk_dense launch");
 }
 
-// The same with h [B, F] an estimate of x [B, K] W [F, K]^T (and overwritten) and xn [B], ends [2, F] as fp32_gemm gave them; todo: int32
-// [1 + B], todo[0] zeroed
-void topk_estimate(const Tensor& h, const Tensor& x, const Tensor& W, const Tensor& xn, const Tensor& ends, const c10::optional<Tensor>& bias,
-                   const c10::optional<Tensor>& norm, int64_t k, const Tensor& todo, const Tensor& out) {
+// The same with lower ends lo (bf16 [B, F]), xn [B], top [2] and status [4] as fp32_gemm gave them for x [B, K], W [F, K]; h: fp32 [B, F], which
+// may share memory with lo, receives the products of rows that are left over; todo: int32 [1 + B], todo[0] zeroed
+void topk_estimate(const Tensor& lo, const Tensor& h, const Tensor& x, const Tensor& W, const Tensor& xn, const Tensor& top, const c10::optional<Tensor>& bias,
+                   const c10::optional<Tensor>& norm, int64_t k, const Tensor& status, const Tensor& todo, const Tensor& out) {
+  CHECK_T(lo, torch::kBFloat16);
   for (const Tensor* t : {&h, &x, &W, &xn, &out}) { CHECK_T(*t, torch::kFloat32); }
-  for (const Tensor* t : {&ends, &todo}) { CHECK_T(*t, torch::kInt32); }
-  TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && h.size(0) < INT_MAX && h.size(1) <= INT_MAX, "h and out must be [B, F]");
+  for (const Tensor* t : {&top, &status, &todo}) { CHECK_T(*t, torch::kInt32); }
+  TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && lo.sizes() == h.sizes() && h.size(0) < INT_MAX && h.size(1) <= INT_MAX, "lo, h and out must be [B, F]");
   TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.size(0) == h.size(0) && W.size(0) == h.size(1) && W.size(1) == x.size(1) &&
               x.size(1) <= lmsae::kEstimateMaxK, "x [B, K] and W [F, K]");
-  TORCH_CHECK(xn.numel() == h.size(0) && ends.numel() == 2 * h.size(1) && todo.numel() == h.size(0) + 1);
+  TORCH_CHECK(xn.numel() == h.size(0) && top.numel() == 2 && status.numel() == 4 && todo.numel() == h.size(0) + 1);
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
   if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
   const c10::cuda::CUDAGuard guard(h.device());
-  check_cuda(lmsae::topk_estimate_launch(h.data_ptr<float>(), x.data_ptr<float>(), W.data_ptr<float>(), xn.data_ptr<float>(),
-                                         reinterpret_cast<const uint32_t*>(ends.data_ptr<int>()), (int)x.size(1), opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1),
-                                         (int)k, todo.data_ptr<int>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+  check_cuda(lmsae::topk_estimate_launch(reinterpret_cast<const __nv_bfloat16*>(lo.data_ptr()), h.data_ptr<float>(), x.data_ptr<float>(), W.data_ptr<float>(),
+                                         xn.data_ptr<float>(), reinterpret_cast<const uint32_t*>(top.data_ptr<int>()), (int)x.size(1),
+                                         opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1), (int)k,
+                                         status.data_ptr<int>(), todo.data_ptr<int>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
              "topk_estimate launch");
 }
 

@@ -13,7 +13,14 @@
 //
 // Structure: CTA pairs (cta_group::2, 256 x 256 tiles) as in encoder_gemm.cu; a tile passes through the accumulator buffers once per
 // slice. 384 threads: TMA producer, MMA issuer, TMEM owner, and eight epilogue warps that hold 128 columns of a row each.
-#include "common.cuh"
+//
+// LOWER ENDS (ENDS = true), for the TopK encoder, which only needs to know what may be selected (topk_merge.cu): two parts an operand and
+// three products (m.h, h.m, h.h), and instead of the estimate h the epilogue stores a lower end of the activation
+//     lo = (h - e + bias) * gate,   e = rel * xn * wn >= the error of h   (xn, wn the rows' 2-norms, rel: estimate_rel)
+// rounded down to bf16, NaN where the bound says nothing. Bias, gate and rounding are monotone, so that lo encloses the activation of the
+// sum in order wherever that is positive; the upper end is at most lo + 2^-7 |lo| + 2 e gate. Half the products and half the bytes:
+// 4096 x 24576 x 768: 632 + 42 (split) -> 291 + 31 us.
+#include "fp32_exact.cuh"
 #include "kernels.h"
 
 namespace lmsae {
@@ -25,7 +32,8 @@ constexpr int FG_SLICE = 2;  // K blocks of 64 per slice
 constexpr int FG_HALF_BYTES = 128 * FG_BK * 2;
 constexpr int FG_STAGE_BYTES = 2 * FG_HALF_BYTES;  // this CTA's 128 rows of A and 128 of the 256 rows of B
 constexpr int FG_BAR_OFF = FG_STAGES * FG_STAGE_BYTES;
-constexpr int FG_SMEM = FG_BAR_OFF + (2 * FG_STAGES + 4) * 8 + 8 + 1024;
+constexpr int FG_STORE_OFF = (FG_BAR_OFF + (2 * FG_STAGES + 4) * 8 + 8 + 15) / 16 * 16;  // ENDS: 32 rows x 32 columns on their way to whole sectors, per epilogue warp
+constexpr int FG_SMEM = FG_STORE_OFF + 8 * 2048 + 1024;
 
 __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -37,33 +45,31 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
 }
 
 // part of A / B (0 high, 1 middle, 2 low) of the t-th product
-__device__ __forceinline__ int part_a(int t) { return (0x201100 >> (4 * (5 - t))) & 15; }
-__device__ __forceinline__ int part_b(int t) { return (0x021010 >> (4 * (5 - t))) & 15; }
+template <int TERMS>
+__device__ __forceinline__ int part_a(int t) { return TERMS == 6 ? (0x201100 >> (4 * (5 - t))) & 15 : t == 0; }
+template <int TERMS>
+__device__ __forceinline__ int part_b(int t) { return TERMS == 6 ? (0x021010 >> (4 * (5 - t))) & 15 : t == 1; }
 
-// dst [rows][3][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
-// then flags[0] != 0. What topk_estimate (topk_merge.cu) takes, both optional: norm[r], at least the row's 2-norm and at most 10 %
-// above it, and ends[0][r], ends[1][r]: gate[r] rounded down / up to bf16 (1 without a gate) in the upper half of a word, that norm rounded up to
-// bf16 in the lower. The norm is infinite where the row's largest magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r]
-// negative, NaN or beyond 2^50: products, (sum + bias) * gate and the parts of what is within stay clear of the ends of the fp32 range
-// (2^30 * 2^30 * K 2^14, doubled, * 2^50 < 2^127).
+// dst [rows][PARTS][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
+// then flags[0] != 0. For lower ends, all optional: norm[r], at least the row's 2-norm and at most 10 % above it; top[0], at least
+// norm[r] * gate[r] of every row whose norm is finite; top[1] != 0 where a gate is 0 or NaN. The norm is infinite where the row's largest
+// magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r] negative, NaN or beyond 2^50: products, (sum + bias) * gate and the
+// parts of what is within stay clear of the ends of the fp32 range (2^30 * 2^30 * K 2^14, doubled, * 2^50 < 2^127).
 struct SplitBounds {
   float* norm;
-  uint32_t* ends;
-  int ends_stride;
+  uint32_t* top;
   const float* bias;
   const float* gate;
 };
-__device__ __forceinline__ uint32_t bf16_up(float x) {  // (x >= 0)
-  const uint32_t b = __float_as_uint(x);
-  return (b >> 16) + ((b & 0xffffu) != 0u ? 1u : 0u);
-}
+template <int PARTS>
 __global__ void __launch_bounds__(256)
-split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags,
-                    const SplitBounds b) {
+split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags,
+                  const SplitBounds b) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float most = 0.0f;
   for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
     const float* s = src + (size_t)r * K;
-    __nv_bfloat16* o = dst + (size_t)r * 3 * kp;
+    __nv_bfloat16* o = dst + (size_t)r * PARTS * kp;
     bool bad = false;
     unsigned top = 0u;
     float sq = 0.0f;
@@ -83,7 +89,7 @@ split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv
         p[2][i] = r1 - p[1][i];
       }
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
+      for (int q = 0; q < PARTS; ++q)
         *reinterpret_cast<uint2*>(o + q * kp + c) = make_uint2(pack_bf16x2(p[q][0], p[q][1]), pack_bf16x2(p[q][2], p[q][3]));
     }
     bad = __any_sync(0xffffffffu, bad);
@@ -91,7 +97,7 @@ split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv
       flags[1 + r] = bad ? 1 : 0;
       if (bad) flags[0] = 1;
     }
-    if (b.norm != nullptr || b.ends != nullptr) {
+    if (b.norm != nullptr) {
       top = __reduce_max_sync(0xffffffffu, top);
       sq = warp_sum(sq);
       if (lane == 0) {
@@ -100,25 +106,38 @@ split_bf16x3_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv
         if (b.bias != nullptr) fits &= (__float_as_uint(b.bias[r]) & 0x7fffffffu) < 0x65000000u;  // 2^75
         const bool plain = __float_as_uint(gate) < 0x58800000u;  // 2^50 (and no sign)
         const float n = !(fits && plain) ? __uint_as_float(0x7f800000u) : top == 0u ? 0.0f : 1.05f * sqrtf(sq);
-        if (b.norm != nullptr) b.norm[r] = n;
-        if (b.ends != nullptr) {
-          const float g = plain ? gate : 1.0f;
-          b.ends[r] = (__float_as_uint(g) & 0xffff0000u) | bf16_up(n);
-          b.ends[(size_t)b.ends_stride + r] = (bf16_up(g) << 16) | bf16_up(n);
-        }
+        b.norm[r] = n;
+        if (fits && plain) most = fmaxf(most, mul_up(n, gate));
+        const unsigned gb = __float_as_uint(gate) & 0x7fffffffu;
+        if (b.top != nullptr && (gb == 0u || gb > 0x7f800000u)) b.top[1] = 1u;
       }
     }
   }
+  if (b.top != nullptr && lane == 0 && most > 0.0f) atomicMax(b.top, __float_as_uint(most));
 }
 
 struct Fp32GemmParams {
   int M, N, kp;
   long long ldc;
   int m_tiles, n_tiles, pairs;
-  float* C;
+  float* C;            // [M][ldc], or the lower ends
+  __nv_bfloat16* lo;
+  float rel;           // ENDS: estimate_rel, the rows' norms, and the columns' bias and gate (nullptr: 0 and 1)
+  const float* na;
+  const float* nb;
+  const float* bias;
+  const float* gate;
   int* status;
 };
 
+// Rounded down to bf16; NaN for what is not finite.
+__device__ __forceinline__ uint32_t bf16_down(float x) {
+  const uint32_t b = __float_as_uint(x);
+  if ((b & 0x7f800000u) == 0x7f800000u) return 0x7fffu;
+  return ((int)b < 0 ? b + 0xffffu : b) >> 16;
+}
+
+template <int TERMS, bool ENDS>
 __global__ void __launch_bounds__(FG_THREADS, 1)
 fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Fp32GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -133,7 +152,8 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
   const int pair = (int)(blockIdx.x >> 1);
-  const int tiles = p.m_tiles * p.n_tiles, k_blocks = p.kp / FG_BK, slices = (k_blocks + FG_SLICE - 1) / FG_SLICE;
+  const int tiles = p.m_tiles * p.n_tiles, k_blocks = p.kp / FG_BK;
+  const int slice = ENDS ? k_blocks : FG_SLICE, slices = (k_blocks + slice - 1) / slice;  // (a lower end needs no slices: estimate_rel)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < FG_STAGES; ++i) {
@@ -168,9 +188,9 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (int t = pair; t < tiles && ok; t += p.pairs) {
         // (pairs that run together work on neighbouring row panels of the same columns)
         const int m0 = (t % p.m_tiles) * 2 * FG_BM + (int)cta_rank * FG_BM, n0 = (t / p.m_tiles) * FG_BN + (int)cta_rank * FG_BM;
-        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += FG_SLICE) {
-          const int n_kb = min(FG_SLICE, k_blocks - kb0);
-          for (int j = 0; j < 6 * n_kb; ++j, ++it) {
+        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += slice) {
+          const int n_kb = min(slice, k_blocks - kb0);
+          for (int j = 0; j < TERMS * n_kb; ++j, ++it) {
             const int term = j / n_kb, kx = (kb0 + j % n_kb) * FG_BK;
             const int s = it % FG_STAGES;
             if (!mbar_wait_bounded(&empty_bar[s], ((it / FG_STAGES) & 1) ^ 1, abort_flag)) {
@@ -182,8 +202,8 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             uint8_t* dst = smem + s * FG_STAGE_BYTES;
             if (leader) mbar_arrive_expect_tx(&full_bar[s], 2 * FG_STAGE_BYTES);
             const uint32_t bar = mapa_u32(smem_u32(&full_bar[s]), 0);
-            tma_load_2d_pair(dst, &tmap_a, bar, part_a(term) * p.kp + kx, m0);
-            tma_load_2d_pair(dst + FG_HALF_BYTES, &tmap_b, bar, part_b(term) * p.kp + kx, n0);
+            tma_load_2d_pair(dst, &tmap_a, bar, part_a<TERMS>(term) * p.kp + kx, m0);
+            tma_load_2d_pair(dst + FG_HALF_BYTES, &tmap_b, bar, part_b<TERMS>(term) * p.kp + kx, n0);
           }
         }
       }
@@ -194,7 +214,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       uint32_t it = 0, sub = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += p.pairs) {
-        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += FG_SLICE, ++sub) {
+        for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += slice, ++sub) {
           const int buf = sub & 1;
           if (!mbar_wait_bounded(&tmem_empty_bar[buf], ((sub >> 1) & 1) ^ 1, abort_flag)) {
             report_status(p.status, kTimeoutTmemEmpty, (int)sub);
@@ -204,7 +224,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           tc_fence_after();
           const uint32_t tmem_d = tmem_base + (uint32_t)(buf * FG_BN);
-          const int steps = 6 * min(FG_SLICE, k_blocks - kb0);
+          const int steps = TERMS * min(slice, k_blocks - kb0);
           for (int j = 0; j < steps; ++j, ++it) {
             const int s = it % FG_STAGES;
             if (!mbar_wait_bounded(&full_bar[s], (it / FG_STAGES) & 1, abort_flag)) {
@@ -227,47 +247,123 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter, column half
-    const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    const bool vec = ENDS ? p.N % 8 == 0 && p.ldc % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.lo) | reinterpret_cast<uintptr_t>(p.nb) |
+                                                                reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.gate)) & 15) == 0
+                          : p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t sub = 0;
     bool ok = true;
     for (int t = pair; t < tiles && ok; t += p.pairs) {
       const int row = (t % p.m_tiles) * 2 * FG_BM + (int)cta_rank * FG_BM + q * 32 + lane;
       const int c0 = (t / p.m_tiles) * FG_BN + half * 128;
-      float acc[128];
-#pragma unroll
-      for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
-      for (int s = 0; s < slices; ++s, ++sub) {
+      if constexpr (ENDS) {
         const int buf = sub & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], (sub >> 1) & 1, abort_flag))) {
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], (sub >> 1) & 1, abort_flag));
+        if (!ok) {
           if (lane == 0) report_status(p.status, kTimeoutTmemFull, (int)sub);
           *abort_flag = 1;
-          ok = false;
           break;
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * FG_BN + half * 128);
+        const int row0 = row - lane;
+        const float rx = row < p.M ? -mul_up(p.rel, __ldg(p.na + row)) : 0.0f;
+        auto columns = [&](const float* v, int c, float absent, float (&x)[8]) {  // (the same for the whole warp)
+          if (v != nullptr && vec && c < p.N) {
+            const float4 t0 = __ldg(reinterpret_cast<const float4*>(v + c)), t1 = __ldg(reinterpret_cast<const float4*>(v + c + 4));
+            x[0] = t0.x; x[1] = t0.y; x[2] = t0.z; x[3] = t0.w;
+            x[4] = t1.x; x[5] = t1.y; x[6] = t1.z; x[7] = t1.w;
+          } else {
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(taddr + (uint32_t)(g * 16), r);
+            for (int i = 0; i < 8; ++i) x[i] = v != nullptr && c + i < p.N ? __ldg(v + c + i) : absent;
+          }
+        };
+        uint8_t* tile_s = smem + FG_STORE_OFF + (warp - 4) * 2048;
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(taddr + (uint32_t)(g * 32), r);
           tmem_wait_ld();
+          if (g == 3) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
+          }
+          const int cg = c0 + g * 32;
+          uint4 o[4];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[g * 16 + j] += __uint_as_float(r[j]);
+          for (int j = 0; j < 4; ++j) {
+            float wn[8], bias[8], gate[8];
+            uint32_t e[8];
+            columns(p.nb, cg + j * 8, 0.0f, wn);
+            columns(p.bias, cg + j * 8, 0.0f, bias);
+            columns(p.gate, cg + j * 8, 1.0f, gate);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              float v = fma_rn(rx, wn[i], __uint_as_float(r[j * 8 + i]));
+              if (p.bias != nullptr) v = add_rn(v, bias[i]);
+              if (p.gate != nullptr) v = mul_rn(v, gate[i]);
+              e[i] = (__float_as_uint(wn[i]) & 0x7fffffffu) >= 0x7f800000u ? 0x7fffu : bf16_down(v);
+            }
+            o[j] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+          }
+          // through shared memory, so that four lanes write whole sectors of a row (as in encoder_gemm.cu)
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(tile_s + lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16)) = o[j];
+          __syncwarp();
+          if (vec) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int rr = i * 8 + (lane >> 2), j = lane & 3;
+              const uint4 v = *reinterpret_cast<const uint4*>(tile_s + rr * 64 + ((j ^ ((rr >> 1) & 3)) * 16));
+              if (row0 + rr < p.M && cg + j * 8 < p.N) *reinterpret_cast<uint4*>(p.lo + (row0 + rr) * p.ldc + cg + j * 8) = v;
+            }
+          } else {  // lane: a column
+            for (int rr = 0; rr < 32; ++rr) {
+              const int j = lane >> 3;
+              const unsigned short v = *reinterpret_cast<const unsigned short*>(tile_s + rr * 64 + ((j ^ ((rr >> 1) & 3)) * 16) + (lane & 7) * 2);
+              if (row0 + rr < p.M && cg + lane < p.N) reinterpret_cast<unsigned short*>(p.lo)[(row0 + rr) * p.ldc + cg + lane] = v;
+            }
+          }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
-      }
-      if (ok && row < p.M) {
-        float* dst = p.C + row * p.ldc + c0;
-        if (vec) {
+        ++sub;
+      } else {
+        float acc[128];
 #pragma unroll
-          for (int j = 0; j < 128; j += 4)
-            if (c0 + j < p.N) *reinterpret_cast<float4*>(dst + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-        } else {
+        for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
+        for (int s = 0; s < slices; ++s, ++sub) {
+          const int buf = sub & 1;
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], (sub >> 1) & 1, abort_flag))) {
+            if (lane == 0) report_status(p.status, kTimeoutTmemFull, (int)sub);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * FG_BN + half * 128);
 #pragma unroll
-          for (int j = 0; j < 128; ++j)
-            if (c0 + j < p.N) dst[j] = acc[j];
+          for (int g = 0; g < 8; ++g) {
+            uint32_t r[16];
+            tmem_ld_32x32b_x16(taddr + (uint32_t)(g * 16), r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[g * 16 + j] += __uint_as_float(r[j]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
+        }
+        if (ok && row < p.M) {
+          float* dst = p.C + row * p.ldc + c0;
+          if (vec) {
+#pragma unroll
+            for (int j = 0; j < 128; j += 4)
+              if (c0 + j < p.N) *reinterpret_cast<float4*>(dst + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 128; ++j)
+              if (c0 + j < p.N) dst[j] = acc[j];
+          }
         }
       }
     }
@@ -307,25 +403,23 @@ marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B,
 
 }  // namespace
 
-int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends,
-                        int ends_stride, const float* bias, const float* gate, cudaStream_t stream) {
-  if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return (int)cudaErrorInvalidValue;
+int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* top,
+                      const float* bias, const float* gate, cudaStream_t stream) {
+  if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0 || (parts != 2 && parts != 3)) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
-  split_bf16x3_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, ends, ends_stride, bias, gate});
+  auto kern = parts == 2 ? split_bf16_kernel<2> : split_bf16_kernel<3>;
+  kern<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, top, bias, gate});
   return (int)cudaGetLastError();
 }
 
-int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
-                     const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream) {
-  Fp32GemmParams p;
-  p.M = M; p.N = N; p.kp = kp; p.C = C; p.ldc = ldc; p.status = status;
-  p.m_tiles = (M + 2 * FG_BM - 1) / (2 * FG_BM);
-  p.n_tiles = (N + FG_BN - 1) / FG_BN;
+static cudaError_t launch_product(const void* kernel, const CUtensorMap& ta, const CUtensorMap& tb, Fp32GemmParams& p, cudaStream_t stream) {
+  p.m_tiles = (p.M + 2 * FG_BM - 1) / (2 * FG_BM);
+  p.n_tiles = (p.N + FG_BN - 1) / FG_BN;
   const long long tiles = (long long)p.m_tiles * p.n_tiles;
-  if (tiles > 2147483647LL - 148) return (int)cudaErrorInvalidValue;
+  if (tiles > 2147483647LL - 148) return cudaErrorInvalidValue;
   p.pairs = (int)(tiles < 74 ? tiles : 74);
-  cudaError_t e = cudaFuncSetAttribute(fp32_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
-  if (e != cudaSuccess) return (int)e;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * p.pairs);
   cfg.blockDim = dim3(FG_THREADS);
@@ -338,10 +432,28 @@ int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (tensor_cores) e = cudaLaunchKernelEx(&cfg, fp32_gemm_kernel, ta, tb, p);
-  if (e != cudaSuccess) return (int)e;
+  void* args[3] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &p};
+  return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
+int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
+                     const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream) {
+  Fp32GemmParams p = {};
+  p.M = M; p.N = N; p.kp = kp; p.C = C; p.ldc = ldc; p.status = status;
+  if (tensor_cores) {
+    const cudaError_t e = launch_product(reinterpret_cast<const void*>(fp32_gemm_kernel<6, false>), ta, tb, p, stream);
+    if (e != cudaSuccess) return (int)e;
+  }
   marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C, ldc, status);
   return (int)cudaGetLastError();
+}
+
+int fp32_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* nb, const float* bias,
+                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, cudaStream_t stream) {
+  Fp32GemmParams p = {};
+  p.M = M; p.N = N; p.kp = kp; p.lo = lo; p.ldc = ldc; p.status = status;
+  p.rel = estimate_rel(K); p.na = na; p.nb = nb; p.bias = bias; p.gate = gate;
+  return (int)launch_product(reinterpret_cast<const void*>(fp32_gemm_kernel<3, true>), ta, tb, p, stream);
 }
 
 }  // namespace lmsae

@@ -38,10 +38,12 @@ struct EncGemmParams {
 };
 int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p, int mode, cudaStream_t stream);
 int enc_gemm_slots_for_k(int k);
-int split_bf16x3_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* ends,
-                        int ends_stride, const float* bias, const float* gate, cudaStream_t stream);
+int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* top,
+                      const float* bias, const float* gate, cudaStream_t stream);
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
                      const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream);
+int fp32_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* nb, const float* bias,
+                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, cudaStream_t stream);
 
 // ---- peer-memory collectives (comm_ops.cu) -------------------------------------------------------
 constexpr int kMaxPeers = 8;
@@ -78,8 +80,8 @@ int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, 
                       int own_hi, int emit_gated, int* out_idx, float* out_val, const MergeComm& comm, cudaStream_t stream);
 int topk_dense_launch(const float* h, const float* bias, const float* norm, int B, int N, int k, float* out, cudaStream_t stream);
 constexpr int kEstimateMaxK = 16384;  // (above it the bound on the estimate's error rules out too few columns)
-int topk_estimate_launch(float* h, const float* x, const float* W, const float* xn, const uint32_t* ends, int K, const float* bias, const float* norm,
-                         int B, int N, int k, int* todo, float* out, cudaStream_t stream);
+int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const uint32_t* top, int K, const float* bias,
+                         const float* norm, int B, int N, int k, const int* status, int* todo, float* out, cudaStream_t stream);
 struct RowsProductParams {
   const float* A;   // [*, K]
   const float* B;   // [N, K], or [K, N]

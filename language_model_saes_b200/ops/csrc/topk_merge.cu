@@ -9,6 +9,7 @@
 // distributed_topk in utils/distributed/ops.py:158-266 of the reference) with one exchange instead of
 // an iterative threshold search.
 #include "comm_common.cuh"
+#include "fp32_exact.cuh"
 
 namespace lmsae {
 
@@ -410,39 +411,22 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 // relu(x) = x * [x > 0] turns into NaN) rank first and stay NaN everywhere, an unselected +inf becomes NaN, and so does everything over a
 // norm of 0 or NaN.
 //
-// ESTIMATE: h is only an estimate of x . W^T (fp32_gemm.cu). What is selected, and the selected values, are those of the fp32 sum in
-// ascending order of k with one rounding per term. That sum lies within e = rel * xn * wn of the estimate, xn and wn the 2-norms of the
-// row of x and the row of W (Cauchy-Schwarz bounds the sum of the magnitudes of the terms by their product; rel: see estimate_rel).
-// Bias, norm and rounding are monotone, so the same operations on h - e and h + e, with the norm rounded down and up, enclose a positive g.
-// The k-th largest lower end of the group maxima is reached by at least k columns, and whatever is selected has its upper end at or
-// above it: those columns are summed up in order before the exact selection. Norms and wn come as two bf16 in one word: what bounds
-// this kernel is the columns' arrays out of the L2 cache, twice for every row (4096 x 24576 x 768, k 50: 554 us with both in fp32, 506 so; a margin of 2^-8 of the bound, which the error could exceed,
-// took 508). Rows with fewer than k positive values cost no more than others (1.16 ms for product and selection, 77 ms when such
-// rows were summed up in order as a whole), and with every row listed it is 6.5 ms at 4096 x 32768 x 2048 (torch operations: 12.6).
-// Columns that the bound says nothing about (wn is infinite there) are among them; rows with more such columns than there is room for are listed, multiplied in order as a whole
-// (rows_product.cu) and selected from exactly. All decisions are taken on the device.
+// ESTIMATE: there is no h, only lower ends of g in bf16 (fp32_gemm.cu, which says what they enclose). What is selected, and the selected
+// values, are those of the fp32 sum x . W^T in ascending order of k with one rounding per term.
+//   The k-th largest of the group maxima of the lower ends is reached by at least k columns, and whatever is selected has its upper end
+// at or above it. The upper end is the lower one plus what rounding it down to bf16 may have taken (2^-7 of it) plus twice the bound on the
+// estimate's error, taken at its largest over the columns, so that neither pass reads anything per column but the ends. The columns that
+// may be selected (k and a few) are summed up in order before the exact selection.
+//   Columns that the bound says nothing about (their lower end is NaN) are among them; rows with more such columns than there is room for,
+// and all rows where the product gave up, are listed, multiplied in order as a whole (rows_product.cu) and selected from exactly. All
+// decisions are taken on the device.
+// 4096 x 24576 x 768, k 50: with fp32 estimates, and the columns' norms, error bounds and biases read from the L2 cache twice for every row,
+// 506 us; 280 here.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned topk_key(float g) {
   const unsigned b = __float_as_uint(g);
   if ((b & 0x7fffffffu) > 0x7f800000u || b == 0xff800000u) return 0x7fffffffu;
   return (int)b > 0 ? b : 0u;
-}
-// (the intrinsics flush subnormals under this build's flags)
-#define LMSAE_F32_OP(name, op)                                             \
-  __device__ __forceinline__ float name(float a, float b) {                \
-    float r;                                                               \
-    asm(op " %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));                     \
-    return r;                                                              \
-  }
-LMSAE_F32_OP(add_rn, "add.rn.f32")
-LMSAE_F32_OP(mul_rn, "mul.rn.f32")
-LMSAE_F32_OP(mul_up, "mul.rp.f32")
-LMSAE_F32_OP(div_rn, "div.rn.f32")
-#undef LMSAE_F32_OP
-__device__ __forceinline__ float fma_rn(float a, float b, float c) {
-  float r;
-  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
 }
 __device__ __forceinline__ bool below(float a, float b) {  // a < b: false for a NaN, subnormals as they are
   int r;
@@ -451,22 +435,14 @@ __device__ __forceinline__ bool below(float a, float b) {  // a < b: false for a
 }
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f800000u; }
 
-// rel for sums of K terms, in units of 2^-24 (what the parts add up to):
-//   K        roundings of the sum in order, one per term
-//   K / 128  roundings of the estimate's slices added up
-//   384      accumulations within a slice of 128 terms: the last eight instructions add sixteen full-size products each to what is there,
-//            and each of these 17 operands may lose a unit to the alignment (136); the 40 before them add parts of 2^-8 and less (3);
-//            the rest is margin for what the hardware does not document (measured: 2 units in all)
-//   16       the three products that are left out (2^-25), the rounding of the ends themselves (|h| is at most about xn wn), and room
-// The norms are rounded up by 5 % where they are made, which covers their own rounding and K 2^-24 << 1.
-__host__ __device__ __forceinline__ float estimate_rel(int K) { return ((float)K * 1.01f + 400.0f) * 5.9604645e-8f; }
-
 struct TopkDenseParams {
-  float* h;
-  const float* x;  // ESTIMATE: [B, K] and [N, K], and what the split of x and of W left (fp32_gemm.cu)
+  const float* h;
+  const __nv_bfloat16* lo;  // ESTIMATE: [B, N] lower ends, and with them
+  const float* x;           // [B, K] and [N, K]
   const float* W;
-  const float* xn;
-  const uint32_t* ends;
+  const float* xn;          // [B] 2-norms (fp32_gemm.cu)
+  const uint32_t* top;      // the largest error bound of a column over rel * xn; and whether a norm is 0 or NaN
+  const int* status;        // of the product
   int K;
   int* todo;        // ESTIMATE: [1 + B] number of rows left over, and which
   const int* rows;  // or the rows to work on, in this form
@@ -478,12 +454,10 @@ struct TopkDenseParams {
 };
 
 // g of columns [c, c + 4) and the norms (columns past the end: 0 and 1)
-// ESTIMATE: an end of g, the lower one for rx with a sign and the lower words of `ends`, else the upper one; the norms as those words have them
-template <bool ESTIMATE>
-__device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const float* __restrict__ h, int c, float rx, float (&g)[4], float (&n)[4]) {
+__device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const float* __restrict__ h, int c, float (&g)[4], float (&n)[4]) {
   float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  uint32_t w[4] = {0x3f800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u};  // norm 1, and in a word of `ends` also a 2-norm of 0
-  const uint32_t* words = ESTIMATE ? p.ends + ((int)__float_as_uint(rx) < 0 ? 0 : p.N) : reinterpret_cast<const uint32_t*>(p.norm);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) n[i] = 1.0f;
   if (p.vec) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(h + c));
     g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
@@ -491,9 +465,9 @@ __device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const 
       const float4 t = __ldg(reinterpret_cast<const float4*>(p.bias + c));
       b[0] = t.x; b[1] = t.y; b[2] = t.z; b[3] = t.w;
     }
-    if (words != nullptr) {
-      const uint4 t = __ldg(reinterpret_cast<const uint4*>(words + c));
-      w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+    if (p.norm != nullptr) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(p.norm + c));
+      n[0] = t.x; n[1] = t.y; n[2] = t.z; n[3] = t.w;
     }
   } else {
 #pragma unroll
@@ -501,30 +475,92 @@ __device__ __forceinline__ void topk_dense_load(const TopkDenseParams& p, const 
       const bool in = c + i < p.N;
       g[i] = in ? __ldg(h + c + i) : 0.0f;
       if (in && p.bias != nullptr) b[i] = p.bias[c + i];
-      if (in && words != nullptr) w[i] = __ldg(words + c + i);
+      if (in && p.norm != nullptr) n[i] = p.norm[c + i];
     }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    n[i] = __uint_as_float(ESTIMATE ? w[i] & 0xffff0000u : w[i]);
-    if constexpr (ESTIMATE) g[i] = fma_rn(rx, __uint_as_float(w[i] << 16), g[i]);
     if (p.bias != nullptr) g[i] = add_rn(g[i], b[i]);
-    if (ESTIMATE || p.norm != nullptr) g[i] = mul_rn(g[i], n[i]);
+    if (p.norm != nullptr) g[i] = mul_rn(g[i], n[i]);
   }
 }
 
-// x . w, fp32, in ascending order (K % 4 == 0)
-__device__ __forceinline__ float dot_in_order(const float* __restrict__ x, const float* __restrict__ w, int K) {
-  float s = 0.0f;
-#pragma unroll 8
-  for (int i = 0; i < K; i += 4) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(x + i)), b = __ldg(reinterpret_cast<const float4*>(w + i));
-    s = fma_rn(a.x, b.x, s);
-    s = fma_rn(a.y, b.y, s);
-    s = fma_rn(a.z, b.z, s);
-    s = fma_rn(a.w, b.w, s);
+// Lower ends of columns [c, c + 8) (past the end: -1, which neither reaches a bound nor enters)
+__device__ __forceinline__ void topk_ends_load(const TopkDenseParams& p, const __nv_bfloat16* __restrict__ lo, int c, float (&g)[8]) {
+  if (p.vec) {
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(lo + c));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      g[2 * i] = __uint_as_float(w[i] << 16);
+      g[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) g[i] = c + i < p.N ? __bfloat162float(lo[c + i]) : -1.0f;
   }
-  return s;
+}
+
+// x . W[cols[j]], fp32, in ascending order (K % 4 == 0) for j < n: done(j, sum). A sum is one thread's chain of K roundings, but its row
+// of W is fetched by the whole warp: pieces of 32 columns of eight candidates' rows and of x are copied to shared memory, whole
+// sectors a row, one piece ahead. (Each thread reading its own row, 16 bytes at a time, kept the L1 cache busy with a line per thread and
+// load: 373 us for the whole selection.) Neighbouring candidates go to different warps.
+constexpr int DOT_ROWS = 8, DOT_K = 32, DOT_PITCH = DOT_K + 4;  // (the pitch: eight rows' 16-byte pieces in different banks)
+struct DotTiles { float w[RT_WARPS][2][DOT_ROWS + 1][DOT_PITCH]; };
+template <class Done>
+__device__ __forceinline__ void dots_in_order(DotTiles& tiles, const float* __restrict__ x, const float* __restrict__ W, int K, const int* cols, int n, Done&& done) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int PIECES = (DOT_ROWS + 1) * DOT_K / 4, PER_LANE = (PIECES + 31) / 32;
+  for (int base = warp; base < n; base += DOT_ROWS * RT_WARPS) {
+    const int rows = min(DOT_ROWS, (n - base + RT_WARPS - 1) / RT_WARPS);  // candidates base + r * RT_WARPS
+    const float* src[PER_LANE];
+    int at[PER_LANE];  // column within the piece, -1: nothing to fetch
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const int e = i * 32 + lane, r = e / (DOT_K / 4);
+      at[i] = r < rows || r == DOT_ROWS ? (e % (DOT_K / 4)) * 4 : -1;
+      src[i] = r < rows ? W + (size_t)cols[base + r * RT_WARPS] * K : x;
+    }
+    auto fetch = [&](int k0, int buf) {
+#pragma unroll
+      for (int i = 0; i < PER_LANE; ++i) {
+        const int r = (i * 32 + lane) / (DOT_K / 4);
+        if (at[i] >= 0 && k0 + at[i] < K)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&tiles.w[warp][buf][r][at[i]])), "l"(src[i] + k0 + at[i]) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float s = 0.0f;
+    fetch(0, 0);
+    for (int k0 = 0, buf = 0; k0 < K; k0 += DOT_K, buf ^= 1) {
+      fetch(k0 + DOT_K, buf ^ 1);  // (past the end: an empty group)
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      if (lane < rows) {
+        const float4* a = reinterpret_cast<const float4*>(tiles.w[warp][buf][DOT_ROWS]);
+        const float4* b = reinterpret_cast<const float4*>(tiles.w[warp][buf][lane]);
+        if (k0 + DOT_K <= K) {
+#pragma unroll
+          for (int i = 0; i < DOT_K / 4; ++i) {
+            s = fma_rn(a[i].x, b[i].x, s);
+            s = fma_rn(a[i].y, b[i].y, s);
+            s = fma_rn(a[i].z, b[i].z, s);
+            s = fma_rn(a[i].w, b[i].w, s);
+          }
+        } else {
+          for (int i = 0; i < (K - k0) / 4; ++i) {
+            s = fma_rn(a[i].x, b[i].x, s);
+            s = fma_rn(a[i].y, b[i].y, s);
+            s = fma_rn(a[i].z, b[i].z, s);
+            s = fma_rn(a[i].w, b[i].w, s);
+          }
+        }
+      }
+      __syncwarp();  // (the buffer is filled again in the next turn)
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (lane < rows) done(base + lane * RT_WARPS, s);
+  }
 }
 
 // Sum over the CTA, the same in every thread.
@@ -542,62 +578,103 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   __shared__ int s_col[RT_CAP];
   __shared__ unsigned s_count[2][RT_WARPS];
   __shared__ int s_n, s_above, s_equal;
-  const float* h = p.h + (size_t)row * p.N;
+  const float* h = ESTIMATE ? nullptr : p.h + (size_t)row * p.N;
+  const __nv_bfloat16* lo = ESTIMATE ? p.lo + (size_t)row * p.N : nullptr;
   float* out = p.out + (size_t)row * p.N;
   const int N = p.N, k = p.k;
-  const float rx = ESTIMATE ? mul_up(estimate_rel(p.K), p.xn[row]) : 0.0f, rx_lo = __uint_as_float(__float_as_uint(rx) | 0x80000000u);
+  if (ESTIMATE && p.status[0] != 0) {  // there are no ends
+    if (threadIdx.x == 0) p.todo[1 + atomicAdd(p.todo, 1)] = row;
+    return;
+  }
   if (threadIdx.x == 0) { s_n = 0; s_above = 0; s_equal = 0; }
   unsigned mx[RT_MAXIMA];
 #pragma unroll
   for (int i = 0; i < RT_MAXIMA; ++i) mx[i] = 0u;
+  if constexpr (ESTIMATE) {
+#pragma unroll 4
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+      float g[8];
+      topk_ends_load(p, lo, c, g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[i] = __float_as_uint(fmaxf(__uint_as_float(mx[i]), g[i]));  // (a NaN does not enter)
+    }
+  } else {
 #pragma unroll 2
-  for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
 #pragma unroll
-    for (int half = 0; half < 8; half += 4) {
-      if (c + half >= N) break;
-      float g[4], nm[4];
-      topk_dense_load<ESTIMATE>(p, h, c + half, rx_lo, g, nm);
+      for (int half = 0; half < 8; half += 4) {
+        if (c + half >= N) break;
+        float g[4], nm[4];
+        topk_dense_load(p, h, c + half, g, nm);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // (ESTIMATE: where wn is infinite the lower end is -inf or NaN, and neither enters)
-        if constexpr (ESTIMATE) mx[half + i] = __float_as_uint(fmaxf(__uint_as_float(mx[half + i]), g[i]));
-        else mx[half + i] = max(mx[half + i], topk_key(g[i]));
+        for (int i = 0; i < 4; ++i) mx[half + i] = max(mx[half + i], topk_key(g[i]));
       }
     }
   }
   unsigned thr = descend(mx, k, 16, s_count);  // a bound until the exact value is known (0: fewer than k positive maxima)
-  const float nan = __uint_as_float(0x7fffffffu), thr_f = __uint_as_float(max(thr, 1u));
+  const float nan = __uint_as_float(0x7fffffffu);
+  auto enter = [&](int c, unsigned key) {
+    const int pos = atomicAdd(&s_n, 1);
+    if (pos < RT_CAP) { s_key[pos] = key; s_col[pos] = c; }
+  };
+  if constexpr (ESTIMATE) {
+    // (16 units of 2^-24 more for the roundings of the ends; the last term for lower ends that are subnormal)
+    const float room = add_rn(mul_up(mul_up(2.0f * (estimate_rel(p.K) + 1e-6f), p.xn[row]), __uint_as_float(p.top[0])), 1e-37f);
+    const float thr_f = __uint_as_float(max(thr, 1u));
+    const bool any_bad = p.top[1] != 0u;
 #pragma unroll 2
-  for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+      float g[8];
+      topk_ends_load(p, lo, c, g);
+      unsigned in = 0u;
 #pragma unroll
-    for (int half = 0; half < 8; half += 4) {
-      if (c + half >= N) break;
-      float g[4], nm[4];
-      topk_dense_load<ESTIMATE>(p, h, c + half, rx, g, nm);
+      for (int i = 0; i < 8; ++i) in |= below(add_rn(fma_rn(fabsf(g[i]), 0.0079f, g[i]), room), thr_f) ? 0u : 1u << i;  // (a NaN enters)
+      while (in != 0u) {
+        const int i = __ffs(in) - 1;
+        in &= in - 1u;
+        if (c + i < N) enter(c + i, 0u);
+      }
+      float z[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const unsigned nb = __float_as_uint(nm[i]) & 0x7fffffffu;
-        unsigned key = 0u;
-        bool enters, bad = nb == 0u || nb > 0x7f800000u;
-        if constexpr (ESTIMATE) {  // (where wn is infinite the upper end is +inf or NaN, and enters; its value is looked at below)
-          enters = !below(g[i], thr_f);
-        } else {
-          key = topk_key(g[i]);
-          enters = key != 0u && key >= thr;
-          bad |= not_finite(g[i]);
+      for (int i = 0; i < 8; ++i) z[i] = 0.0f;
+      if (any_bad) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned nb = c + i < N ? __float_as_uint(p.norm[c + i]) & 0x7fffffffu : 1u;
+          if (nb == 0u || nb > 0x7f800000u) z[i] = nan;
         }
-        if (enters) {
-          const int pos = atomicAdd(&s_n, 1);
-          if (pos < RT_CAP) { s_key[pos] = key; s_col[pos] = c + half + i; }
-        }
-        g[i] = bad ? nan : 0.0f;
       }
       if (p.vec) {
-        __stcs(reinterpret_cast<float4*>(out + c + half), make_float4(g[0], g[1], g[2], g[3]));
+        __stcs(reinterpret_cast<float4*>(out + c), make_float4(z[0], z[1], z[2], z[3]));
+        __stcs(reinterpret_cast<float4*>(out + c + 4), make_float4(z[4], z[5], z[6], z[7]));
       } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (c + half + i < N) out[c + half + i] = g[i];
+        for (int i = 0; i < 8; ++i)
+          if (c + i < N) out[c + i] = z[i];
+      }
+    }
+  } else {
+#pragma unroll 2
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+#pragma unroll
+      for (int half = 0; half < 8; half += 4) {
+        if (c + half >= N) break;
+        float g[4], nm[4];
+        topk_dense_load(p, h, c + half, g, nm);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned nb = __float_as_uint(nm[i]) & 0x7fffffffu;
+          const unsigned key = topk_key(g[i]);
+          if (key != 0u && key >= thr) enter(c + half + i, key);
+          g[i] = nb == 0u || nb > 0x7f800000u || not_finite(g[i]) ? nan : 0.0f;
+        }
+        if (p.vec) {
+          __stcs(reinterpret_cast<float4*>(out + c + half), make_float4(g[0], g[1], g[2], g[3]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (c + half + i < N) out[c + half + i] = g[i];
+        }
       }
     }
   }
@@ -608,11 +685,9 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
       if (threadIdx.x == 0) p.todo[1 + atomicAdd(p.todo, 1)] = row;
       return;
     }
-    const float* x = p.x + (size_t)row * p.K;
-    // (neighbouring candidates to different warps: a few dozen of them in one or two warps wait for their rows of W alone, 536 us)
-    for (int j = (threadIdx.x & 31) * RT_WARPS + (threadIdx.x >> 5); j < n; j += RT_THREADS) {
+    __shared__ __align__(16) DotTiles tiles;
+    dots_in_order(tiles, p.x + (size_t)row * p.K, p.W, p.K, s_col, n, [&](int j, float g) {
       const int c = s_col[j];
-      float g = dot_in_order(x, p.W + (size_t)c * p.K, p.K);
       if (p.bias != nullptr) g = add_rn(g, p.bias[c]);
       unsigned nb = 1u;
       if (p.norm != nullptr) {
@@ -621,7 +696,7 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
       }
       s_key[j] = topk_key(g);
       if (not_finite(g) || nb == 0u || nb > 0x7f800000u) out[c] = nan;  // (the last two are NaN already)
-    }
+    });
     __syncthreads();
   }
   auto put = [&](int c, unsigned key) {
@@ -670,7 +745,7 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
     auto keys_of = [&](auto&& visit) {
       for (int c = threadIdx.x * 4; c < N; c += RT_THREADS * 4) {
         float g[4], nm[4];
-        topk_dense_load<false>(p, h, c, 0.0f, g, nm);
+        topk_dense_load(p, h, c, g, nm);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const unsigned key = topk_key(g[i]);
@@ -720,29 +795,32 @@ int topk_dense_launch(const float* h, const float* bias, const float* norm, int 
   if (B <= 0 || N <= 0) return 0;
   if (k < 1 || k > RT_BOUND_K) return (int)cudaErrorInvalidValue;
   TopkDenseParams p = {};
-  p.h = const_cast<float*>(h); p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.h = h; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
   p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
                           reinterpret_cast<uintptr_t>(out)) % 16 == 0);
   topk_dense_kernel<false><<<B, RT_THREADS, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }
 
-// The same with h an estimate of x W^T (and overwritten where it is too coarse). todo: int [1 + B], todo[0] zeroed.
-int topk_estimate_launch(float* h, const float* x, const float* W, const float* xn, const uint32_t* ends, int K, const float* bias, const float* norm,
-                         int B, int N, int k, int* todo, float* out, cudaStream_t stream) {
+// The same with lower ends `lo` from an estimate of x W^T; h: fp32 [B, N] for the products of rows that are left over (it may share
+// memory with lo, which is no longer read then). todo: int [1 + B], todo[0] zeroed.
+int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const uint32_t* top, int K, const float* bias,
+                         const float* norm, int B, int N, int k, const int* status, int* todo, float* out, cudaStream_t stream) {
   if (B <= 0 || N <= 0) return 0;
   if (k < 1 || k > RT_BOUND_K || K < 1 || K > kEstimateMaxK || K % 4 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) != 0)
     return (int)cudaErrorInvalidValue;
   TopkDenseParams p = {};
-  p.h = h; p.x = x; p.W = W; p.xn = xn; p.ends = ends; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
-  p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
-                          reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ends)) % 16 == 0);
+  p.lo = lo; p.x = x; p.W = W; p.xn = xn; p.top = top; p.status = status; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.vec = N % 8 == 0 && ((reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
   topk_dense_kernel<true><<<B, RT_THREADS, 0, stream>>>(p);
   RowsProductParams r = {};
   r.A = x; r.B = W; r.C = h; r.N = N; r.K = K; r.rows = todo; r.max_rows = B;
   const int e = rows_product_launch(r, false, stream);
   if (e != 0) return e;
   p.rows = todo;
+  p.h = h;
+  p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
+                          reinterpret_cast<uintptr_t>(out)) % 16 == 0);
   topk_dense_rows_kernel<<<B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }

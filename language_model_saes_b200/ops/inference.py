@@ -14,7 +14,7 @@ from torch.utils._python_dispatch import _get_current_dispatch_mode
 from . import sae_kernels as K
 
 MAX_K = 1024  # the selection kernel's bound comes from 2048 column groups
-# bytes for the parts of W at a time (6 per element): up to 74 tiles of 256 features at d_model 4096, so that a piece still fills the GPU
+# bytes for the parts of W at a time (6 per element, 4 where it only proposes): 74 tiles of 256 features at d_model 4096, so that a piece still fills the GPU
 PRODUCT_WORKSPACE = 512 << 20
 MAX_ESTIMATE_WIDTH = 16384  # kEstimateMaxK in csrc/kernels.h
 
@@ -71,17 +71,18 @@ def topk_dense(h: torch.Tensor, bias: torch.Tensor | None, norm: torch.Tensor | 
 
 
 def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, norm: torch.Tensor | None, k: int) -> torch.Tensor:
-    """``topk_dense(x @ W, ...)`` for operands of ``product``, which proposes: what the estimate leaves in question is summed again in
-    ascending order of the input dimension, so that neither the choice nor the values depend on how the estimate was made."""
+    """``topk_dense(x @ W, ...)`` for operands of ``product``: a coarser product proposes, and what it leaves in question is summed in
+    ascending order of the input dimension, so that neither the choice nor the values depend on how it was made."""
     rows = x.detach().reshape(-1, x.shape[-1])
     B, F = rows.shape[0], W.shape[1]
     h, out = (torch.empty(B, F, dtype=torch.float32, device=x.device) for _ in range(2))
-    xn, ends = torch.empty(B, dtype=torch.float32, device=x.device), torch.empty(2, F, dtype=torch.int32, device=x.device)
-    status_todo = torch.zeros(4 + 1 + B, dtype=torch.int32, device=x.device)
-    status, todo = status_todo[:4], status_todo[4:]
+    lo = h.view(-1).view(torch.bfloat16)[: B * F].view(B, F)  # (read before anything is written to h)
+    xn = torch.empty(B, dtype=torch.float32, device=x.device)
+    words = torch.zeros(4 + 2 + 1 + B, dtype=torch.int32, device=x.device)
+    status, top, todo = words[:4], words[4:6], words[6:]
     bias, norm = (t.contiguous() if t is not None else None for t in (bias, norm))
-    K._ext().fp32_gemm(rows, W.detach().t(), h, status, xn, ends, bias, norm, True, PRODUCT_WORKSPACE)
-    K._ext().topk_estimate(h, rows, W.detach().t(), xn, ends, bias, norm, k, todo, out)
+    K._ext().fp32_gemm(rows, W.detach().t(), lo, status, xn, top, bias, norm, True, PRODUCT_WORKSPACE)
+    K._ext().topk_estimate(lo, h, rows, W.detach().t(), xn, top, bias, norm, k, status, todo, out)
     return out.view(*x.shape[:-1], F)
 
 
