@@ -113,7 +113,7 @@ int64_t encoder_gemm(const Tensor& x, const Tensor& w, const c10::optional<Tenso
                      const c10::optional<Tensor>& gate, int64_t mode, int64_t k, int64_t num_splits,
                      const c10::optional<Tensor>& H, const c10::optional<Tensor>& cand_val,
                      const c10::optional<Tensor>& cand_idx, const Tensor& status, int64_t n_index_offset,
-                     bool resume_topk, int64_t units) {
+                     bool resume_topk, int64_t units, const c10::optional<Tensor>& maxima, const c10::optional<Tensor>& max_gate) {
   CHECK_T(x, torch::kBFloat16);
   CHECK_T(w, torch::kBFloat16);
   CHECK_T(status, torch::kInt32);
@@ -144,6 +144,16 @@ int64_t encoder_gemm(const Tensor& x, const Tensor& w, const c10::optional<Tenso
     TORCH_CHECK(H->size(0) == p.M && H->size(1) == p.N);
     p.H = reinterpret_cast<__nv_bfloat16*>(H->data_ptr());
     p.ldh = p.N;
+  }
+  if (maxima.has_value()) {
+    CHECK_T(*maxima, torch::kFloat32);
+    TORCH_CHECK((mode & 3) == 1 && maxima->dim() == 2 && maxima->size(0) == p.M && maxima->size(1) == n_tiles * 8 &&
+                    reinterpret_cast<uintptr_t>(maxima->data_ptr()) % 16 == 0, "maxima: [M, 8 per 256 columns], with H alone");
+    TORCH_CHECK(!max_gate.has_value() || !gate.has_value(), "max_gate: for values that are stored without a gate");
+    if (max_gate.has_value()) { CHECK_T(*max_gate, torch::kFloat32); TORCH_CHECK(max_gate->numel() == p.N); }
+    p.maxima = maxima->data_ptr<float>();
+    p.ld_maxima = maxima->size(1);
+    p.max_gate = opt_ptr<const float>(max_gate);
   }
   if (mode & 2) {
     TORCH_CHECK(k >= 1 && k <= 64, "fused top-k supports 1 <= k <= 64");
@@ -321,18 +331,28 @@ void dense_decode(const Tensor& acts, const Tensor& W, int64_t most, const Tenso
              "dense_decode launch");
 }
 
+// maxima: the largest gated value of every 32 columns, as encoder_gemm leaves them
+const float* checked_maxima(const c10::optional<Tensor>& maxima, int64_t rows, int64_t cols) {
+  if (!maxima.has_value()) return nullptr;
+  CHECK_T(*maxima, torch::kFloat32);
+  TORCH_CHECK(maxima->dim() == 2 && maxima->size(0) == rows && maxima->size(1) * 32 >= cols, "maxima: [rows, one per 32 columns at least]");
+  return maxima->data_ptr<float>();
+}
+
 void row_topk(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate, const c10::optional<Tensor>& alive,
-              const Tensor& out_idx, const Tensor& out_val) {
+              const c10::optional<Tensor>& maxima, const Tensor& out_idx, const Tensor& out_val) {
   CHECK_T(H, torch::kBFloat16);
   CHECK_T(out_idx, torch::kInt32);
   CHECK_T(out_val, torch::kFloat32);
   TORCH_CHECK(H.dim() == 2 && out_idx.numel() >= H.size(0) * k && out_val.numel() >= H.size(0) * k);
   if (alive.has_value()) { CHECK_T(*alive, torch::kUInt8); TORCH_CHECK(alive->numel() == H.size(1)); }
   if (gate.has_value()) { CHECK_T(*gate, torch::kFloat32); TORCH_CHECK(gate->numel() == H.size(1)); }
+  TORCH_CHECK(!maxima.has_value() || !alive.has_value(), "maxima are those of all columns");
+  const float* max_ptr = checked_maxima(maxima, H.size(0), H.size(1));
   const c10::cuda::CUDAGuard guard(H.device());
   check_cuda(lmsae::row_topk_launch(reinterpret_cast<const __nv_bfloat16*>(H.data_ptr()), H.size(1), (int)H.size(0),
                                     (int)H.size(1), (int)k, opt_ptr<const float>(gate), opt_ptr<const uint8_t>(alive),
-                                    out_idx.data_ptr<int>(), out_val.data_ptr<float>(),
+                                    max_ptr, max_ptr != nullptr ? maxima->size(1) : 0, out_idx.data_ptr<int>(), out_val.data_ptr<float>(),
                                     at::cuda::getCurrentCUDAStream()),
              "row_topk launch");
 }
@@ -961,6 +981,42 @@ Tensor threshold_mask(const Tensor& x, const Tensor& thr, int64_t A, int64_t S, 
 // x [B, N] -> idx / val [B, cap] (both optional: count only) and nnz [B] (optional). seg_counts int32 [B, 8, 2]
 // (optional): written by a counting call, read by a compacting call of the same matrix and thresholds, which then
 // skips its own counting pass.
+// Histogram of the values of x [B, N] (bf16) that are at least floor (> 0), as radix_hist has it, and per-row counts / lists against thr, as
+// row_compact has them with ties; maxima [B, *]: of every 32 columns.
+void chunk_hist(const Tensor& x, const Tensor& maxima, const Tensor& floor, const Tensor& hist) {
+  CHECK_T(x, torch::kBFloat16); CHECK_T(floor, torch::kFloat32); CHECK_T(hist, torch::kInt32);
+  TORCH_CHECK(x.dim() == 2 && x.size(1) < (1LL << 30) && x.size(0) < (1LL << 31) && floor.numel() >= 1 && hist.numel() >= lmsae::radix_hi_bins(), "chunk_hist: sizes");
+  const float* m = checked_maxima(maxima, x.size(0), x.size(1));
+  const c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(lmsae::chunk_hist_launch(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), m, maxima.size(1), (int)x.size(0), (int)x.size(1),
+                                      floor.data_ptr<float>(), reinterpret_cast<unsigned*>(hist.data_ptr<int>()), lmsae::radix_hi_bins(),
+                                      at::cuda::getCurrentCUDAStream()),
+             "chunk_hist launch");
+}
+
+void chunk_compact(const Tensor& x, const Tensor& maxima, const Tensor& thr, const c10::optional<Tensor>& col_div, const Tensor& nnz,
+                   const c10::optional<Tensor>& ties, const c10::optional<Tensor>& tie_quota, const c10::optional<Tensor>& idx, const c10::optional<Tensor>& val) {
+  CHECK_T(x, torch::kBFloat16); CHECK_T(thr, torch::kFloat32); CHECK_T(nnz, torch::kInt32);
+  TORCH_CHECK(x.dim() == 2 && x.size(1) < (1LL << 30) && x.size(0) < (1LL << 31) && nnz.numel() == x.size(0) && thr.numel() >= 1, "chunk_compact: sizes");
+  TORCH_CHECK(idx.has_value() == val.has_value() && idx.has_value() == tie_quota.has_value() && idx.has_value() != ties.has_value(), "chunk_compact: counts or lists");
+  int cap = 0;
+  if (idx.has_value()) {
+    CHECK_T(*idx, torch::kInt32); CHECK_T(*val, torch::kFloat32); CHECK_T(*tie_quota, torch::kInt32);
+    TORCH_CHECK(idx->dim() == 2 && idx->size(0) == x.size(0) && val->sizes() == idx->sizes() && tie_quota->numel() == x.size(0), "idx / val must be [B, cap]");
+    cap = (int)idx->size(1);
+  } else {
+    CHECK_T(*ties, torch::kInt32);
+    TORCH_CHECK(ties->numel() == x.size(0));
+  }
+  if (col_div.has_value()) { CHECK_T(*col_div, torch::kFloat32); TORCH_CHECK(col_div->numel() == x.size(1), "one divisor per column"); }
+  const float* m = checked_maxima(maxima, x.size(0), x.size(1));
+  const c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(lmsae::chunk_compact_launch(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), m, maxima.size(1), (int)x.size(0), (int)x.size(1),
+                                         thr.data_ptr<float>(), opt_ptr<const float>(col_div), nnz.data_ptr<int>(), opt_ptr<int>(ties),
+                                         opt_ptr<const int>(tie_quota), cap, opt_ptr<int>(idx), opt_ptr<float>(val), at::cuda::getCurrentCUDAStream()),
+             "chunk_compact launch");
+}
+
 void row_compact(const Tensor& x, const c10::optional<Tensor>& idx, const c10::optional<Tensor>& val,
                  const c10::optional<Tensor>& nnz, const c10::optional<Tensor>& thr, const c10::optional<Tensor>& col_div,
                  const c10::optional<Tensor>& ties, const c10::optional<Tensor>& tie_quota,
@@ -1412,6 +1468,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("radix_pick", &radix_pick);
   m.def("threshold_mask", &threshold_mask);
   m.def("row_compact", &row_compact);
+  m.def("chunk_hist", &chunk_hist);
+  m.def("chunk_compact", &chunk_compact);
   m.def("jumprelu_window_grad", &jumprelu_window_grad);
   m.def("rotary_pair", &rotary_pair);
   m.def("exclusive_scan", &exclusive_scan);

@@ -12,13 +12,13 @@
 //               at the end it emits k (value, column) candidates per row for its range. A small merge
 //               kernel (topk_merge.cu) combines the ranges (and, under feature sharding, the ranks).
 //
-// Structure (one CTA per SM, 256 threads):
+// Structure (one CTA per SM, 256 threads, 384 without top-k):
 //   warp 0    : TMA producer (one elected lane) -> STAGES-deep ring of {A 128x64, B 256x64} bf16 tiles,
 //               128-byte swizzle, no cluster multicast
 //   warp 1    : tcgen05.mma issuer (one elected lane), UMMA 128x256x16, accumulators in TMEM,
 //               two 256-column accumulator buffers so the epilogue of tile i overlaps the MMAs of tile i+1
 //   warp 2    : TMEM allocation / release
-//   warps 4-7 : epilogue; thread r of the warpgroup owns accumulator row r (TMEM lane r)
+//   warps 4-7 : epilogue; thread r of the warpgroup owns accumulator row r (TMEM lane r); without top-k warps 8-11 take half of its columns
 // Every mbarrier wait is bounded; on expiry the CTA records a status code, raises a CTA-wide abort flag,
 // drains and frees its TMEM.
 //
@@ -41,7 +41,9 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KB
 constexpr int TMEM_COLS = 512;
-constexpr int NUM_THREADS = 256;
+// Epilogue warps: four with the top-k (a thread keeps a row's buffer), else eight, two per accumulator row with half of the columns each:
+// a single warp per scheduler waits for every TMEM load. H of 4096 x 24576 x 768: 135 -> 126 us.
+__host__ __device__ constexpr int epilogue_warps(bool topk) { return topk ? 4 : 8; }
 
 // Entries of a row's candidate buffer (CAP): the k best so far plus room for what is appended until the next selection. A step of
 // the sweep appends at most 16, so k + 16 entries suffice; more room means fewer selections, but costs ring stages.
@@ -60,8 +62,10 @@ struct SmemLayout {
   static constexpr int kSlotValOff = STAGES * kStageBytes;
   static constexpr int kSlotIdxOff = kSlotValOff + BM * CAP * 4;
   static constexpr int kColOff = kSlotIdxOff + BM * CAP * (NARROW ? 2 : 4);   // per epilogue warp: bias and gate of the 32 columns at work
-  static constexpr int kStoreOff = kColOff + 4 * 64 * 4;  // per epilogue warp: 32 x 32 bf16 on their way to whole sectors of H (no top-k)
-  static constexpr int kBarOff = kStoreOff + (CAP == 0 ? 4 * 2048 : 0);
+  static constexpr int kEpilogueWarps = epilogue_warps(CAP != 0);
+  static constexpr int kStoreOff = kColOff + kEpilogueWarps * 64 * 4;  // per epilogue warp: 32 x 32 bf16 on their way to whole sectors of H (no top-k)
+  static constexpr int kMaxOff = kStoreOff + (CAP == 0 ? kEpilogueWarps * 2048 : 0);  // per 32 rows: maxima of a tile's eight groups of columns, [8][32 rows]
+  static constexpr int kBarOff = kMaxOff + (CAP == 0 ? 4 * 1024 : 0);
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
   static constexpr int kAbortOff = kTmemPtrOff + 4;
@@ -84,6 +88,13 @@ __device__ __forceinline__ void mul_pair(float& a0, float& a1, float b0, float b
   asm("{\n\t.reg .b64 ra, rb;\n\tmov.b64 ra, {%0, %1};\n\tmov.b64 rb, {%2, %3};\n\tmul.rn.f32x2 ra, ra, rb;\n\tmov.b64 {%0, %1}, ra;\n\t}"
       : "+f"(a0), "+f"(a1)
       : "f"(b0), "f"(b1));
+}
+
+// The larger one, NaN where one is NaN.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
 }
 
 // Entry {value, column} to shared memory where the condition holds: predicated, because a branch per column costs more than the
@@ -198,7 +209,7 @@ __device__ __noinline__ RowState select_entries(RowBuffer<CAP, NARROW> buf, RowS
 }
 
 template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(128 + 32 * epilogue_warps(TOPK), 1)
 enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const EncGemmParams p) {
   using L = SmemLayout<STAGES, CAP, PAIR, NARROW>;
@@ -256,8 +267,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
     mbar_init(&tmem_full_bar[0], 1);
     mbar_init(&tmem_full_bar[1], 1);
-    mbar_init(&tmem_empty_bar[0], PAIR ? 8 : 4);  // epilogue warps of the CTA (of both CTAs of a pair)
-    mbar_init(&tmem_empty_bar[1], PAIR ? 8 : 4);
+    for (int i = 0; i < 2; ++i) mbar_init(&tmem_empty_bar[i], epilogue_warps(TOPK) * (PAIR ? 2 : 1));  // epilogue warps of the CTA (of both CTAs of a pair)
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -369,7 +379,9 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ epilogue
-    const int q = warp - 4;             // TMEM lane quarter of this warp
+    const int q = warp & 3;             // TMEM lane quarter of this warp
+    const int part = (warp - 4) >> 2;   // and its share of the columns
+    constexpr int CHUNKS = BN / 32 * 4 / epilogue_warps(TOPK);
     const int row_in_tile = q * 32 + lane;
     const int row = m0 + row_in_tile;
     const bool row_ok = row < p.M;
@@ -386,13 +398,15 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     const int col_base = NARROW ? p.n_index_offset + tile_begin * BN : 0;  // what the stored columns count from
     // Bias and gate of the columns at work come through shared memory, fetched one step ahead by a coalesced load per warp
     // (read per thread they were a miss in L1 for every step); columns past the end have gate 0.
-    float* col_bias = reinterpret_cast<float*>(smem + L::kColOff) + q * 64;
+    float* col_bias = reinterpret_cast<float*>(smem + L::kColOff) + (warp - 4) * 64;
     float* col_gate = col_bias + 32;
+    const float* gate_src = !TOPK && p.gate == nullptr ? p.max_gate : p.gate;
+    float* tile_max = reinterpret_cast<float*>(smem + L::kMaxOff) + q * 256 + lane;
     float next_bias = 0.0f, next_gate = 0.0f;
     auto fetch_columns = [&](int c) {
       const bool in = c + lane < p.N;
       next_bias = in && p.bias != nullptr ? __ldg(p.bias + c + lane) : 0.0f;
-      next_gate = !in ? 0.0f : p.gate != nullptr ? __ldg(p.gate + c + lane) : 1.0f;
+      next_gate = !in ? 0.0f : gate_src != nullptr ? __ldg(gate_src + c + lane) : 1.0f;
     };
     if constexpr (TOPK) {
       if (p.resume_topk && row_ok) {
@@ -408,7 +422,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
       __syncwarp();
     }
-    fetch_columns(tile_begin * BN);
+    fetch_columns(tile_begin * BN + part * CHUNKS * 32);
     int lt = 0;
     bool ok = true;
     for (int tile = tile_begin; tile < tile_end && ok; ++tile, ++lt) {
@@ -423,15 +437,19 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       tc_fence_after();
       const int n0 = tile * BN;
       const uint32_t taddr_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
+      if constexpr (WRITE_H && !TOPK) {
+        if (p.maxima != nullptr)
+          for (int c = 0; c < CHUNKS; ++c) tile_max[(part * CHUNKS + c) * 32] = __int_as_float(0xff800000);  // (groups past the last column)
+      }
 #pragma unroll 1
-      for (int chunk = 0; chunk < BN / 32; ++chunk) {
+      for (int chunk = part * CHUNKS; chunk < (part + 1) * CHUNKS; ++chunk) {
         const int c0 = n0 + chunk * 32;
         if (c0 >= p.N) break;  // uniform across the CTA
         __syncwarp();  // (the previous step's values have been read)
         col_bias[lane] = next_bias;
         col_gate[lane] = next_gate;
         __syncwarp();
-        fetch_columns(c0 + 32);
+        fetch_columns(chunk + 1 < (part + 1) * CHUNKS ? c0 + 32 : n0 + BN + part * CHUNKS * 32);
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr_row + (uint32_t)(chunk * 32), r);
         tmem_wait_ld();
@@ -466,12 +484,29 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           // A thread holds 64 bytes of its own row: through shared memory (16-byte pieces, swizzled: no bank conflicts), so that
           // four lanes write whole sectors of a row. Stored from the registers, every instruction touched 32 rows by half a
           // sector each: 4096 x 24576 x 768: 198 (with a gate: 425) -> 135 (149) us.
-          uint8_t* tile_s = smem + L::kStoreOff + q * 2048;
+          uint8_t* tile_s = smem + L::kStoreOff + (warp - 4) * 2048;
+          uint32_t w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<uint4*>(tile_s + lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16)) =
-                make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
-                           pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+            *reinterpret_cast<uint4*>(tile_s + lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+          if (p.maxima != nullptr) {  // of the values as they are stored
+            float m[4] = {__int_as_float(0xff800000), __int_as_float(0xff800000), __int_as_float(0xff800000), __int_as_float(0xff800000)};
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const uint32_t w0 = w[j / 2], w1 = w[j / 2 + 1];
+              float x0 = __uint_as_float(w0 << 16), x1 = __uint_as_float(w0 & 0xffff0000u), x2 = __uint_as_float(w1 << 16), x3 = __uint_as_float(w1 & 0xffff0000u);
+              if (p.max_gate != nullptr) {
+                const float4 g4 = *reinterpret_cast<const float4*>(col_gate + j);
+                mul_pair(x0, x1, g4.x, g4.y);
+                mul_pair(x2, x3, g4.z, g4.w);
+              }
+              m[0] = max_nan(m[0], x0); m[1] = max_nan(m[1], x1);
+              m[2] = max_nan(m[2], x2); m[3] = max_nan(m[3], x3);
+            }
+            tile_max[chunk * 32] = max_nan(max_nan(m[0], m[1]), max_nan(m[2], m[3]));
+          }
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -505,6 +540,13 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             }
             st.n = (int)((at - rowbuf.val) / (BM * 4));
           }
+        }
+      }
+      if constexpr (WRITE_H && !TOPK) {
+        if (p.maxima != nullptr && row_ok) {  // (a lane's own entries)
+          const float* m = tile_max + part * CHUNKS * 32;
+          static_assert(TOPK || CHUNKS == 4, "one store");
+          *reinterpret_cast<float4*>(p.maxima + (long long)row * p.ld_maxima + tile * (BN / 32) + part * CHUNKS) = make_float4(m[0], m[32], m[64], m[96]);
         }
       }
       // release this accumulator buffer to the MMA warp
@@ -583,7 +625,7 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.units != 0 ? p.units * (PAIR ? 2 : 1) : p.num_panels * p.num_splits);
-  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.blockDim = dim3(128 + 32 * epilogue_warps(TOPK));
   cfg.dynamicSmemBytes = L::kDynamicBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];

@@ -35,6 +35,11 @@ struct EncGemmParams {
   // x_h . W_h^T over the heads. heads <= 1: a plain GEMM.
   int heads;
   int b_rows_per_head;
+  // H without top-k: the largest stored value of every 32 columns, times max_gate when that is given, goes to maxima
+  // [M][ld_maxima] (a whole number of eights per row; NaN where a value is NaN). nullptr: not wanted.
+  float* maxima;
+  long long ld_maxima;
+  const float* max_gate;
 };
 int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p, int mode, cudaStream_t stream);
 int enc_gemm_slots_for_k(int k);
@@ -99,7 +104,7 @@ int rows_product_launch(RowsProductParams p, bool b_by_k, cudaStream_t stream);
 int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int most, int* todo, float* part, long long part_floats, int part_tiles,
                         float* out, cudaStream_t stream);
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,
-                    const uint8_t* alive, int* out_idx, float* out_val, cudaStream_t stream);
+                    const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream);
 
 // Records of the bounds-checked debug build, one per translation unit (all zero in the regular build).
 int bounds_fetch_sparse_ops(int* out);
@@ -319,6 +324,12 @@ int attn_value_chunk(int dv);
 int attn_fwd_value_chunk(int dqk, int dv);
 int attn_fwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p,
                     cudaStream_t stream);
+
+// ---- selections that look at the maxima of 32 columns first (chunk_select.cu) -------------------------------
+int chunk_hist_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* floor, unsigned* hist, int nbins,
+                      cudaStream_t stream);
+int chunk_compact_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* thr, const float* col_div, int* nnz,
+                         int* ties, const int* tie_quota, int cap, int* idx, float* val, cudaStream_t stream);
 
 // ---- low-rank sparse attention step (lorsa_ops.cu) ----------------------------------------------------
 int lorsa_dz_smem(int F, int k);

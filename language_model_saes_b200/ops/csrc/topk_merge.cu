@@ -163,6 +163,7 @@ int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, 
 constexpr int RT_THREADS = 256;  // (what is left of a row's time is latency: five CTAs of 256 threads per SM hide it as well as three of 512 with wider barriers)
 constexpr int RT_MAXIMA = 8;     // column groups per thread
 constexpr int RT_CAP = 10 * RT_THREADS;  // candidates in shared memory
+constexpr int RT_MAX_GROUPS = 1024;  // of 32 columns that reach the bound, where their maxima are known (half as many codes are allowed for)
 constexpr int RT_BOUND_K = RT_THREADS * RT_MAXIMA / 2;  // (about 1.4 k candidates there, k + a few for small k)
 
 __device__ __forceinline__ float gated_value(const __nv_bfloat16* __restrict__ hrow, const float* __restrict__ gate,
@@ -309,30 +310,44 @@ __device__ __forceinline__ unsigned descend(const unsigned (&val)[N], int k, int
   return t;
 }
 
+// MAXIMA: the largest gated value of every 32 columns comes with H (the encoder GEMM's epilogue leaves them): those are the column groups,
+// and only groups whose maximum reaches the bound are read at all: 4096 rows of 32768, k 128: 206 -> 116 us.
+template <bool MAXIMA>
 __global__ void __launch_bounds__(RT_THREADS, 5)
 row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N, int k,
-                const float* __restrict__ gate, const uint8_t* __restrict__ alive, int vec, int* __restrict__ out_idx,
-                float* __restrict__ out_val) {
+                const float* __restrict__ gate, const uint8_t* __restrict__ alive, const float* __restrict__ maxima, long long ld_maxima, int vec,
+                int* __restrict__ out_idx, float* __restrict__ out_val) {
   const int row = blockIdx.x;
   if (row >= M) return;
   const __nv_bfloat16* hrow = H + (long long)row * ldh;
   __shared__ unsigned s_bits[RT_CAP];
   __shared__ int s_col[RT_CAP];
   __shared__ unsigned s_count[2][RT_WARPS];
-  __shared__ int s_n, s_cursor;
+  __shared__ int s_n, s_cursor, s_groups;
+  constexpr int CAP = MAXIMA ? RT_CAP - RT_MAX_GROUPS : RT_CAP;
   bool use_radix = k > RT_BOUND_K;
   if (!use_radix) {
-    if (threadIdx.x == 0) { s_n = 0; s_cursor = 0; }
+    if (threadIdx.x == 0) { s_n = 0; s_cursor = 0; s_groups = 0; }
     // ---- pass 1: maxima of this thread's eight column groups (non-positive values and NaN never enter)
     float mx[RT_MAXIMA];
 #pragma unroll
     for (int i = 0; i < RT_MAXIMA; ++i) mx[i] = 0.0f;
-#pragma unroll 4
-    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
-      float v[8];
-      gated_values8(hrow, gate, alive, c, N, vec != 0, v);
+    const float* groups = MAXIMA ? maxima + (long long)row * ld_maxima : nullptr;
+    const int n_groups = (N + 31) / 32;
+    if constexpr (MAXIMA) {
+      for (int c0 = threadIdx.x; c0 < n_groups; c0 += RT_THREADS * RT_MAXIMA) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], v[i]);
+        for (int i = 0; i < RT_MAXIMA; ++i)
+          if (c0 + i * RT_THREADS < n_groups) mx[i] = fmaxf(mx[i], __ldg(groups + c0 + i * RT_THREADS));
+      }
+    } else {
+#pragma unroll 4
+      for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+        float v[8];
+        gated_values8(hrow, gate, alive, c, N, vec != 0, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], v[i]);
+      }
     }
     __syncthreads();
     unsigned mb[RT_MAXIMA];
@@ -340,22 +355,58 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
     for (int i = 0; i < RT_MAXIMA; ++i) mb[i] = __float_as_uint(mx[i]);
     const unsigned bound = descend(mb, k, 16, s_count);
     // ---- pass 2: columns at or above the bound
-#pragma unroll 2
-    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
-      float v[8];
-      gated_values8(hrow, gate, alive, c, N, vec != 0, v);
+    auto look_at = [&](int c, const float (&v)[8]) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const unsigned b = __float_as_uint(v[i]);
         if (v[i] > 0.0f && b >= bound) {
           const int pos = atomicAdd(&s_n, 1);
-          if (pos < RT_CAP) { s_bits[pos] = b; s_col[pos] = c + i; }
+          if (pos < CAP) { s_bits[pos] = b; s_col[pos] = c + i; }
         }
+      }
+    };
+    if constexpr (MAXIMA) {
+      // the groups that reach the bound are listed first (in the columns' array, from its end), so that their reads go out together: four
+      // lanes each
+      int* s_group = s_col + RT_CAP - RT_MAX_GROUPS;
+      for (int g = threadIdx.x; g < n_groups; g += RT_THREADS) {
+        const float m = __ldg(groups + g);
+        if (m > 0.0f ? __float_as_uint(m) >= bound : m != m) {  // (a NaN hides the others' maximum)
+          const int pos = atomicAdd(&s_groups, 1);
+          if (pos < RT_MAX_GROUPS) s_group[pos] = g;
+        }
+      }
+      __syncthreads();
+      const int n_list = s_groups;
+      if (n_list <= RT_MAX_GROUPS) {
+        const int sub = threadIdx.x & 3;
+        for (int e0 = threadIdx.x >> 2; e0 < n_list; e0 += RT_THREADS / 4 * 2) {
+          float v[2][8];
+          int c[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int e = e0 + i * (RT_THREADS / 4);
+            c[i] = e < n_list ? s_group[e] * 32 + sub * 8 : N;
+            if (c[i] < N) gated_values8(hrow, gate, alive, c[i], N, vec != 0, v[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (c[i] < N) look_at(c[i], v[i]);
+        }
+      } else if (threadIdx.x == 0) {
+        s_n = RT_CAP + 1;  // (values repeated thousands of times: the descent below)
+      }
+    } else {
+#pragma unroll 2
+      for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+        float v[8];
+        gated_values8(hrow, gate, alive, c, N, vec != 0, v);
+        look_at(c, v);
       }
     }
     __syncthreads();
     const int n_cand = s_n;
-    use_radix = n_cand > RT_CAP;  // (uniform)
+    use_radix = n_cand > CAP;  // (uniform)
     if (!use_radix) {
       // ---- the exact k-th value of the candidates
       unsigned thr = 0;
@@ -394,10 +445,11 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
 }
 
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,
-                    const uint8_t* alive, int* out_idx, float* out_val, cudaStream_t stream) {
+                    const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream) {
   const bool vec = N % 8 == 0 && ldh % 8 == 0 && reinterpret_cast<uintptr_t>(H) % 16 == 0 && reinterpret_cast<uintptr_t>(gate) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(alive) % 8 == 0;
-  row_topk_kernel<<<M, RT_THREADS, 0, stream>>>(H, ldh, M, N, k, gate, alive, vec ? 1 : 0, out_idx, out_val);
+  if (maxima != nullptr) row_topk_kernel<true><<<M, RT_THREADS, 0, stream>>>(H, ldh, M, N, k, gate, alive, maxima, ld_maxima, vec ? 1 : 0, out_idx, out_val);
+  else row_topk_kernel<false><<<M, RT_THREADS, 0, stream>>>(H, ldh, M, N, k, gate, alive, nullptr, 0, vec ? 1 : 0, out_idx, out_val);
   return (int)cudaGetLastError();
 }
 

@@ -391,8 +391,10 @@ class FusedTopKSAEStep:
             idx_l, g_l = K.topk_merge(cv, ci, k, gate, emit_gated=True)
             self._mark("local_merge")
         else:
-            H = K.encoder_hidden(x, self.WE_bf16, self.bE)
-            idx_l, act_l = K.row_topk(H, k, gate, None)
+            if x.is_cuda:
+                _, idx_l, act_l = K.hidden_topk(x, self.WE_bf16, self.bE, gate, k)
+            else:
+                idx_l, act_l = K.row_topk(K.encoder_hidden(x, self.WE_bf16, self.bE), k, gate, None)
             if self.tp == 1:
                 return idx_l, act_l
             g_l = act_l * gate[idx_l.clamp_min(0).long()] if gate is not None else act_l
@@ -419,18 +421,21 @@ class FusedTopKSAEStep:
         from . import select_kernels as S
 
         self.join()
-        G = K.encoder_hidden(x, self.WE_bf16, self.bE, gate=gate)
+        if x.is_cuda:
+            G, maxima = K.encoder_hidden_maxima(x, self.WE_bf16, self.bE, gate=gate)
+        else:
+            G, maxima = K.encoder_hidden(x, self.WE_bf16, self.bE, gate=gate), None
         self._mark("encoder_gemm_hidden")
         B = x.shape[0]
         tp_group = self.tp_group if self.tp > 1 else None
-        # (the previous batch's threshold, lowered by a quarter, as the histogram pass's floor: see positive_thresholds)
-        floor = self._batch_thr * 0.75 if self._batch_thr is not None and G.is_cuda else None
-        thr, n_ties = S.positive_thresholds(G.view(1, 1, -1), k * B, tp_group, return_remaining=True, floor=floor)
+        # (the previous batch's threshold, lowered by a tenth, as the histogram pass's floor: see positive_thresholds)
+        floor = self._batch_thr * 0.9 if self._batch_thr is not None and G.is_cuda else None
+        thr, n_ties = S.positive_thresholds(G.view(1, 1, -1), k * B, tp_group, return_remaining=True, floor=floor, maxima=maxima)
         self._batch_thr = thr
         self._mark("batch_threshold_select")
         # exactly k * B codes: of the entries equal to the (bf16) threshold only as many as the selection still needs
         cap = -(-self.batch_list_factor * k // 8) * 8
-        out = S.threshold_rows_to_sparse(G, thr, gate, n_ties=n_ties, tie_group=tp_group, cap=cap, overflow=self.list_overflow)
+        out = S.threshold_rows_to_sparse(G, thr, gate, n_ties=n_ties, tie_group=tp_group, cap=cap, overflow=self.list_overflow, maxima=maxima)
         self._mark("rows_to_code_lists")
         return out
 

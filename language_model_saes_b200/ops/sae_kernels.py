@@ -192,8 +192,35 @@ def encoder_hidden(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
     M, N = x.shape[0], w.shape[0]
     H = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     units, S = _deal(M, N, pair, None)
-    _ext().encoder_gemm(x, w, bias, gate, 1 | _pair_bit(pair), 0, S, H, None, None, status_buffer(x.device), 0, False, units)
+    _ext().encoder_gemm(x, w, bias, gate, 1 | _pair_bit(pair), 0, S, H, None, None, status_buffer(x.device), 0, False, units, None, None)
     return H
+
+
+def encoder_hidden_maxima(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None = None, max_gate: torch.Tensor | None = None,
+                          pair: bool | None = None) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
+    """``encoder_hidden`` on a GPU with the maxima of every 32 columns of what it stores, times ``max_gate`` when that is given: fp32
+    ``[M, 8 per 256 columns]``, NaN where a value is NaN. Selections look at those first."""
+    M, N = x.shape[0], w.shape[0]
+    H = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    maxima = torch.empty(M, -(-N // 256) * 8, dtype=torch.float32, device=x.device)
+    units, S = _deal(M, N, pair, None)
+    _ext().encoder_gemm(x, w, bias, gate, 1 | _pair_bit(pair), 0, S, H, None, None, status_buffer(x.device), 0, False, units, maxima, max_gate)
+    return H, maxima
+
+
+def maxima_pay(N: int, k: int) -> bool:
+    """Whether the maxima of 32 columns bound the k-th value closely enough for a row's selection: with four times as many groups as codes
+    the bound leaves 1.15 k candidates (with as many groups as codes there is none). The kernel lists 1024 groups at most."""
+    return N >= 128 * k and k <= 512
+
+
+def hidden_topk(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None, k: int, pair: bool | None = None):
+    """Stored pre-activations and their row top-k on a GPU: ``(H, idx, act)``."""
+    if maxima_pay(w.shape[0], k):
+        H, maxima = encoder_hidden_maxima(x, w, bias, max_gate=gate, pair=pair)
+        return H, *row_topk(H, k, gate, maxima=maxima)
+    H = encoder_hidden(x, w, bias, pair)
+    return H, *row_topk(H, k, gate)
 
 
 def _deal(M: int, N: int, pair: bool | None, num_splits: int | None) -> tuple[int, int]:
@@ -238,7 +265,7 @@ def encoder_topk_candidates(
         cand_idx = torch.empty(M, C, dtype=torch.int32, device=x.device)
     mode = 2 | (1 if H is not None else 0) | _pair_bit(pair) | (16 if compact_smem else 0)
     _ext().encoder_gemm(x, w, bias, gate, mode, k, S, H, cand_val, cand_idx, status_buffer(x.device), n_index_offset, resume is not None,
-                        units)  # fmt: skip
+                        units, None, None)  # fmt: skip
     return cand_val, cand_idx, C
 
 
@@ -301,28 +328,26 @@ def encoder_topk(
         h = ref_hidden(x, w, bias)
         idx, act = ref_topk_codes(h, k, gate)
         return (idx, act, h.to(torch.bfloat16)) if return_hidden else (idx, act)
-    M, N = x.shape[0], w.shape[0]
-    H = torch.empty(M, N, dtype=torch.bfloat16, device=x.device) if (return_hidden or k > 64) else None
     if k <= 64:
+        H = torch.empty(x.shape[0], w.shape[0], dtype=torch.bfloat16, device=x.device) if return_hidden else None
         cv, ci, _ = encoder_topk_candidates(x, w, bias, gate, k, H=H, pair=pair)
         idx, act = topk_merge(cv, ci, k, gate)
     else:
-        units, S = _deal(M, N, pair, None)
-        _ext().encoder_gemm(x, w, bias, None, 1 | _pair_bit(pair), 0, S, H, None, None, status_buffer(x.device), 0, False, units)
-        idx, act = row_topk(H, k, gate, None)
+        H, idx, act = hidden_topk(x, w, bias, gate, k, pair)
     return (idx, act, H) if return_hidden else (idx, act)
 
 
 def row_topk(
-    H: torch.Tensor, k: int, gate: torch.Tensor | None = None, alive: torch.Tensor | None = None
+    H: torch.Tensor, k: int, gate: torch.Tensor | None = None, alive: torch.Tensor | None = None, maxima: torch.Tensor | None = None
 ) -> tuple[torch.Tensor, torch.Tensor]:
+    """``maxima``: those of ``encoder_hidden_maxima`` for these pre-activations and this gate (not with ``alive``)."""
     if not H.is_cuda:
         return ref_topk_codes(H.float(), k, gate, alive)
     M = H.shape[0]
     out_idx = torch.empty(M, k, dtype=torch.int32, device=H.device)
     out_val = torch.empty(M, k, dtype=torch.float32, device=H.device)
     alive_u8 = alive.to(torch.uint8).contiguous() if alive is not None else None
-    _ext().row_topk(H.contiguous(), k, gate, alive_u8, out_idx, out_val)
+    _ext().row_topk(H.contiguous(), k, gate, alive_u8, maxima, out_idx, out_val)
     return out_idx, out_val
 
 

@@ -37,7 +37,8 @@ def _kernel_ok(x: torch.Tensor) -> bool:
 
 
 @torch.no_grad()
-def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: bool = False, floor: torch.Tensor | None = None):
+def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: bool = False, floor: torch.Tensor | None = None,
+                        maxima: torch.Tensor | None = None):  # fmt: skip
     """``x3``: contiguous ``[A, S, N]``. Returns fp32 ``[S]``: for every segment ``s`` the k-th largest positive value of
     ``x3[:, s, :]``, taken over the union of all ranks of ``group`` when one is given. ``return_remaining`` (GPU kernels
     only) also returns int64 ``[S]``: how many of the entries equal to the threshold the selection of ``k`` includes.
@@ -46,7 +47,10 @@ def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: 
     lower bound of the result, e.g. a fraction of the previous batch's threshold. The histogram pass then counts only
     values of at least ``floor``, which removes nearly all of its shared-memory atomics. The result does not depend on
     the guess: when fewer than ``k`` values reach the floor, a second pass without it runs (decided on the device, the
-    host launches both and reads nothing)."""
+    host launches both and reads nothing).
+
+    ``maxima``: of every 32 columns of the rows that ``x3`` (one segment, 16-bit) consists of (``encoder_hidden_maxima``): the floored
+    pass then reads only the groups that reach the floor."""
     A, S, N = x3.shape
     world = dist.get_world_size(group) if group is not None else 1
     if not _kernel_ok(x3):
@@ -80,7 +84,10 @@ def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: 
     floored = floor is not None and half and S == 1
     for s in range(S):
         hist_hi.zero_()
-        ext.radix_hist(x3, A, S, N, s, 0, None, hist_hi, floor.reshape(1).float() if floored else None, None)
+        if floored and maxima is not None:
+            ext.chunk_hist(x3.view(maxima.shape[0], -1), maxima, floor.reshape(1).float(), hist_hi)
+        else:
+            ext.radix_hist(x3, A, S, N, s, 0, None, hist_hi, floor.reshape(1).float() if floored else None, None)
         if world > 1:
             dist.all_reduce(hist_hi, group=group)
         ext.radix_pick(hist_hi, nhi, int(k), None, 0, sel0, thr[s : s + 1] if half else None, None)
@@ -188,7 +195,7 @@ def dense_rows_to_sparse(acts: torch.Tensor, cap: int | None = None) -> tuple[to
 @torch.no_grad()
 def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.Tensor | None = None, width_group=None,
                              n_ties: torch.Tensor | None = None, tie_group=None, cap: int | None = None,
-                             overflow: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
+                             overflow: torch.Tensor | None = None, maxima: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
     """Entries of ``g [B, N]`` that reach the (positive) threshold ``thr`` (one-element fp32 tensor) as padded sparse lists,
     values divided by ``col_div[column]`` when given: the codes of a batch-level top-k straight from the gated
     pre-activations, without a masked dense tensor in between.
@@ -201,7 +208,9 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
     ``cap``: fixed list width (a multiple of 8). Without it the width is the widest row's count, which costs one host
     read per call; with it nothing is read back: a row with more than ``cap`` selected entries keeps its first ``cap``
     (ascending column) and the number of such rows is added to ``overflow`` (one-element integer device tensor) for
-    the caller to look at when it next synchronises anyway."""
+    the caller to look at when it next synchronises anyway.
+
+    ``maxima`` (with ``n_ties``, 16-bit ``g``): of every 32 columns (``encoder_hidden_maxima``); groups below the threshold are not read."""
     if not _kernel_ok(g):
         return _ref_threshold_rows_to_sparse(g, thr, col_div, width_group, n_ties, tie_group, cap, overflow)
     ext = K._ext()
@@ -215,8 +224,11 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
             widest = nnz.max()
     else:
         ties = torch.empty(B, dtype=torch.int32, device=g.device)
-        seg = torch.empty(B, 8, 2, dtype=torch.int32, device=g.device)  # per warp segment: the compaction pass starts from them
-        ext.row_compact(g, None, None, nnz, thr, None, ties, None, None, seg)
+        if maxima is not None:
+            ext.chunk_compact(g, maxima, thr, None, nnz, ties, None, None, None)
+        else:
+            seg = torch.empty(B, 8, 2, dtype=torch.int32, device=g.device)  # per warp segment: the compaction pass starts from them
+            ext.row_compact(g, None, None, nnz, thr, None, ties, None, None, seg)
         budget = n_ties.reshape(()).to(torch.int64)
         if tie_group is not None and dist.get_world_size(tie_group) > 1:
             mine = ties.sum(dtype=torch.int64).reshape(1)
@@ -234,7 +246,10 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
     assert cap % 8 == 0 and cap > 0
     idx = torch.empty(B, cap, dtype=torch.int32, device=g.device)
     val = torch.empty(B, cap, dtype=torch.float32, device=g.device)
-    ext.row_compact(g, idx, val, nnz, thr, col_div, None, quota, None, seg)  # nnz: the row's full count, also beyond the list width
+    if maxima is not None and quota is not None:
+        ext.chunk_compact(g, maxima, thr, col_div, nnz, None, quota, idx, val)
+    else:
+        ext.row_compact(g, idx, val, nnz, thr, col_div, None, quota, None, seg)  # nnz: the row's full count, also beyond the list width
     if overflow is not None:
         overflow += (nnz > cap).sum()
     return idx, val

@@ -1,0 +1,84 @@
+"""Selections that look at the maxima of 32 columns first, against the ones that read the whole matrix."""
+
+import pytest
+import torch
+
+from language_model_saes_b200.ops import sae_kernels as K
+from language_model_saes_b200.ops import select_kernels as S
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one group; a group and a bit; a whole tile and eight columns more (rows for the single and the paired kernel); many tiles
+@pytest.mark.parametrize("M,N", [(1, 8), (130, 40), (256, 264), (300, 4096 + 24), (512, 9000)])
+@pytest.mark.parametrize("gated", ["stored", "max", "none"])
+def test_maxima_of_stored_pre_activations(M, N, gated):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn(M, 64, device=DEV, generator=g).to(torch.bfloat16), torch.randn(N, 64, device=DEV, generator=g).to(torch.bfloat16)
+    b, gate = torch.randn(N, device=DEV, generator=g), torch.rand(N, device=DEV, generator=g) + 0.5
+    b[N // 2] = float("nan")
+    H, maxima = K.encoder_hidden_maxima(x, w, b, gate=gate if gated == "stored" else None, max_gate=gate if gated == "max" else None)
+    K.check_status(torch.device(DEV))
+    assert torch.equal(H.nan_to_num(nan=7.0), K.encoder_hidden(x, w, b, gate=gate if gated == "stored" else None).nan_to_num(nan=7.0))
+    v = H.float() * gate if gated == "max" else H.float()
+    groups = -(-N // 32)
+    pad = torch.zeros(M, groups * 32 - N, device=DEV)  # (columns past the end inside a group count as zero)
+    want = torch.cat([v, pad], 1).view(M, groups, 32).amax(2)
+    assert torch.equal(maxima[:, :groups].nan_to_num(nan=7.0), want.nan_to_num(nan=7.0))
+    assert bool((maxima[:, groups:] <= 0).all())
+
+
+@pytest.mark.parametrize("M,N,k", [(3, 8200, 64), (40, 16384 + 40, 100), (9, 32768, 256)])
+@pytest.mark.parametrize("data", ["normal", "few positive", "ties", "nan"])
+def test_row_topk_with_maxima(M, N, k, data):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    H = torch.randn(M, N, device=DEV, generator=g).to(torch.bfloat16)
+    gate = torch.rand(N, device=DEV, generator=g) + 0.5
+    if data == "few positive":
+        H = (H - 3.3).to(torch.bfloat16)
+    elif data == "ties":
+        H, gate = (H * 2).round().to(torch.bfloat16), torch.ones(N, device=DEV)
+    elif data == "nan":
+        H[0, 5], H[1, 100:140] = float("nan"), float("nan")
+    groups = -(-N // 256) * 8
+    gated = torch.zeros(M, groups * 32, device=DEV)
+    gated[:, :N] = H.float() * gate
+    maxima = gated.view(M, groups, 32).amax(2).contiguous()
+    idx, val = K.row_topk(H, k, gate, maxima=maxima)
+    want_idx, want_val = K.row_topk(H, k, gate)
+    order, want_order = idx.sort(1), want_idx.sort(1)
+    if data != "ties":  # (which of equal values are taken is free)
+        assert torch.equal(order.values, want_order.values)
+        assert torch.equal(val.gather(1, order.indices), want_val.gather(1, want_order.indices))
+    assert torch.equal((val * (idx >= 0)).sort(1).values, (want_val * (want_idx >= 0)).sort(1).values)
+
+
+@pytest.mark.parametrize("B,N,k", [(1, 8, 1), (5, 40, 3), (70, 4104, 16), (300, 9000, 64)])
+@pytest.mark.parametrize("data", ["normal", "ties", "few positive", "huge", "nan"])
+def test_batch_level_selection_with_maxima(B, N, k, data):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x = torch.randn(B, N, device=DEV, generator=g)
+    if data == "ties":
+        x = (x * 2).round() / 2
+    elif data == "few positive":
+        x -= 3.5
+    elif data == "huge":
+        x[0, 0], x[-1, -1] = 3e38, float("inf")
+    elif data == "nan":
+        x[0, N // 3] = float("nan")
+    x = x.to(torch.bfloat16)
+    groups = -(-N // 256) * 8
+    padded = torch.zeros(B, groups * 32, dtype=torch.bfloat16, device=DEV)
+    padded[:, :N] = x
+    maxima = padded.view(B, groups, 32).float().amax(2).contiguous()
+    thr, n_ties = S.positive_thresholds(x.view(1, 1, -1), k * B, None, return_remaining=True)
+    for floor in (0.75 * thr, 2 * thr, torch.full_like(thr, 1e-3)):  # (the second one is too high: the pass is repeated)
+        got, got_ties = S.positive_thresholds(x.view(1, 1, -1), k * B, None, return_remaining=True, floor=floor, maxima=maxima)
+        assert torch.equal(got, thr) and torch.equal(got_ties, n_ties)
+    div = torch.rand(N, device=DEV, generator=g) + 0.5
+    for cap in (8, 8 * k):
+        counts = [torch.zeros(1, dtype=torch.int64, device=DEV) for _ in range(2)]
+        want = S.threshold_rows_to_sparse(x, thr, div, n_ties=n_ties, cap=cap, overflow=counts[0])
+        got = S.threshold_rows_to_sparse(x, thr, div, n_ties=n_ties, cap=cap, overflow=counts[1], maxima=maxima)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(nan=7.0), want[1].nan_to_num(nan=7.0)) and torch.equal(*counts)
