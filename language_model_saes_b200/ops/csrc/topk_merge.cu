@@ -16,11 +16,14 @@ namespace lmsae {
 constexpr int MERGE_WARPS = 4;
 
 // One warp per row. Positive floats order like their bit patterns, so the k-th largest candidate is found by a
-// descent over the 31 value bits (count(key >= t) per trial, one warp reduction each) instead of ranking every
-// candidate against every other one; candidates equal to the threshold get the remaining places in slot order. The
-// (at most k) winners are compacted into shared memory and ranked among themselves. Only winners whose candidate
-// slot lies in [own_lo, own_hi) are written, in value-descending order FROM SLOT 0 ON (the rest of the row is
+// descent over the 31 value bits instead of ranking every candidate against every other one: two bits per step, the three counts of a
+// step in one word and one warp reduction, until exactly k are left; candidates equal to the threshold get the remaining places in slot
+// order. The (at most k) winners are compacted into shared memory in slot order and ranked among themselves. Only winners whose
+// candidate slot lies in [own_lo, own_hi) are written, in value-descending order FROM SLOT 0 ON (the rest of the row is
 // (-1, 0)): consumers of a shard's codes may stop at the first empty slot.
+// All rows are in flight at once: what bounds it is the latency of a warp's chain. PER candidates per lane are held in registers (up to 768 of
+// them; more, as small batches with many ranges have, come from shared memory and take a step per bit). 4096 rows of 256 candidates, k
+// 50: 25 us with candidates in shared memory, a step per bit and slots compared in the ranking -> 14 us; 512 of 32, k 8: 9.6 -> 4.1.
 //
 // comm.mode selects what surrounds the merge under feature sharding:
 //   kMergeLocal  nothing (single GPU, or lists that are exchanged by other means)
@@ -29,6 +32,7 @@ constexpr int MERGE_WARPS = 4;
 //                peer stores, fused into the kernel that produces them); the last block publishes the epoch
 //   kMergeWait   the kernel first waits (bounded) until every rank has published the epoch for the candidate
 //                phase, then merges the gathered lists it finds in this rank's own buffer
+template <int PER>
 __global__ void __launch_bounds__(MERGE_WARPS * 32)
 topk_merge_kernel(const float* cand_val, const int* cand_idx, int M, int C, int k,  // may be peer-written: no read-only path
                   const float* __restrict__ gate, int own_lo, int own_hi, int emit_gated,
@@ -36,79 +40,113 @@ topk_merge_kernel(const float* cand_val, const int* cand_idx, int M, int C, int 
   extern __shared__ uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  // per warp: keys[C], ids[C], winner keys[k], winner slots[k], staged output ids[k] and values[k]
-  uint32_t* skey = reinterpret_cast<uint32_t*>(smem_raw) + (size_t)warp * (2 * C + 4 * k);
-  int* sidx = reinterpret_cast<int*>(skey + C);
-  uint32_t* wkey = reinterpret_cast<uint32_t*>(sidx + C);
-  int* wslot = reinterpret_cast<int*>(wkey + k);
-  int* oidx = wslot + k;
+  // per warp: winner keys[k] and ids[k], staged output ids[k] and values[k], and where candidates are not in registers keys[C], ids[C]
+  uint32_t* wkey = reinterpret_cast<uint32_t*>(smem_raw) + (size_t)warp * (4 * k + (PER == 0 ? 2 * C : 0));
+  int* wid = reinterpret_cast<int*>(wkey + k);
+  int* oidx = wid + k;
   float* oval = reinterpret_cast<float*>(oidx + k);
+  uint32_t* skey = reinterpret_cast<uint32_t*>(oval + k);
+  int* sidx = reinterpret_cast<int*>(skey + C);
 
   bool inputs_ok = true;
   if (comm.mode == kMergeWait) inputs_ok = wait_all_sources(comm.pt, kPhaseCand, comm.epoch, comm.status);
 
   for (int row = blockIdx.x * MERGE_WARPS + warp; row < M; row += gridDim.x * MERGE_WARPS) {
-    for (int i = lane; i < k; i += 32) {
-      oidx[i] = -1;
-      oval[i] = 0.0f;
-    }
+    int n_own = 0;
     if (inputs_ok) {
       const float* cv = cand_val + (size_t)row * C;
       const int* ci = cand_idx + (size_t)row * C;
-      for (int i = lane; i < C; i += 32) {
-        const int id = ci[i];
-        const float v = cv[i];
-        sidx[i] = id;
-        skey[i] = (id >= 0 && v > 0.0f) ? __float_as_uint(v) : 0u;  // only positive candidates compete
+      uint32_t key[PER > 0 ? PER : 1];
+      int id[PER > 0 ? PER : 1];
+      if constexpr (PER > 0) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const int c = i * 32 + lane;
+          id[i] = c < C ? ci[c] : -1;
+          key[i] = c < C ? __float_as_uint(cv[c]) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) key[i] = (id[i] >= 0 && __uint_as_float(key[i]) > 0.0f) ? key[i] : 0u;  // only positive candidates compete
+      } else {
+        for (int i = lane; i < C; i += 32) {
+          const int d = ci[i];
+          const float v = cv[i];
+          sidx[i] = d;
+          skey[i] = (d >= 0 && v > 0.0f) ? __float_as_uint(v) : 0u;
+        }
+        __syncwarp();
       }
-      __syncwarp();
-      // threshold: the largest t with count(key >= t) >= k (0 when fewer than k candidates are positive)
+      // threshold: the largest t with count(key >= t) >= k (0 when fewer than k candidates are positive), or one that exactly k reach
       uint32_t t = 0;
-      for (int bit = 30; bit >= 0; --bit) {
-        const uint32_t trial = t | (1u << bit);
-        int c = 0;
-        for (int i = lane; i < C; i += 32) c += skey[i] >= trial;
-        if (__reduce_add_sync(0xffffffffu, c) >= k) t = trial;
-      }
+      bool exactly = false;
       int above = 0;
-      for (int i = lane; i < C; i += 32) above += skey[i] > t;
-      above = __reduce_add_sync(0xffffffffu, above);
-      const int ties_wanted = (t == 0u) ? 0 : k - above;  // t == 0: every positive candidate is in, nothing equals t
-      // compaction of the winners in slot order
-      int n_win = 0, ties_seen = 0;
-      for (int base = 0; base < C; base += 32) {
-        const int i = base + lane;
-        const uint32_t key = i < C ? skey[i] : 0u;
-        const bool eq = t != 0u && key == t;
+      if constexpr (PER > 0) {
+        for (int shift = 30; shift >= 0 && !exactly; shift -= 2) {  // (bit 31 is never set)
+          const uint32_t t1 = t | (1u << shift), t2 = t | (2u << shift), t3 = t | (3u << shift);
+          unsigned n = 0;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) n += (unsigned)(key[i] >= t1) + ((unsigned)(key[i] >= t2) << 10) + ((unsigned)(key[i] >= t3) << 20);
+          n = __reduce_add_sync(0xffffffffu, n);
+          const int c1 = (int)(n & 1023u), c2 = (int)((n >> 10) & 1023u), c3 = (int)(n >> 20);
+          if (c3 >= k) { t = t3; exactly = c3 == k; }
+          else if (c2 >= k) { t = t2; exactly = c2 == k; }
+          else if (c1 >= k) { t = t1; exactly = c1 == k; }
+        }
+        if (!exactly && t != 0u) {
+#pragma unroll
+          for (int i = 0; i < PER; ++i) above += key[i] > t;
+        }
+      } else {
+        for (int bit = 30; bit >= 0; --bit) {
+          const uint32_t trial = t | (1u << bit);
+          int c = 0;
+          for (int i = lane; i < C; i += 32) c += skey[i] >= trial;
+          if (__reduce_add_sync(0xffffffffu, c) >= k) t = trial;
+        }
+        for (int i = lane; i < C; i += 32) above += skey[i] > t;
+      }
+      const int ties_wanted = exactly ? k : t == 0u ? 0 : k - __reduce_add_sync(0xffffffffu, above);  // (t == 0: nothing equals t)
+      // compaction of the winners in slot order; [own0, own1) of them lie in this shard's slots
+      int n_win = 0, ties_seen = 0, own0 = 0, own1 = 0;
+      auto take = [&](int base, uint32_t u, int d) {
+        const bool eq = t != 0u && u == t;
         const unsigned eq_ballot = __ballot_sync(0xffffffffu, eq);
-        const bool win = key > t || (eq && ties_seen + __popc(eq_ballot & lt_mask) < ties_wanted);
+        const bool win = u > t || (eq && ties_seen + __popc(eq_ballot & lt_mask) < ties_wanted);
         const unsigned win_ballot = __ballot_sync(0xffffffffu, win);
         if (win) {
           const int pos = n_win + __popc(win_ballot & lt_mask);
-          wkey[pos] = key;
-          wslot[pos] = i;
+          wkey[pos] = u;
+          wid[pos] = d;
         }
+        const int slot = base + lane;
+        own0 += __popc(__ballot_sync(0xffffffffu, win && slot < own_lo));
+        own1 += __popc(__ballot_sync(0xffffffffu, win && slot < own_hi));
         n_win += __popc(win_ballot);
         ties_seen += __popc(eq_ballot);
+      };
+      if constexpr (PER > 0) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) take(i * 32, key[i], id[i]);
+      } else {
+        for (int base = 0; base < C; base += 32) take(base, base + lane < C ? skey[base + lane] : 0u, base + lane < C ? sidx[base + lane] : -1);
       }
       __syncwarp();
-      // place of each of this shard's winners among this shard's winners (value descending, earlier slot first
-      // among equals)
-      for (int w = lane; w < n_win; w += 32) {
-        const int slot = wslot[w];
-        if (slot < own_lo || slot >= own_hi) continue;
-        const uint32_t key = wkey[w];
+      // place of each of this shard's winners among this shard's winners (value descending, earlier slot first among equals)
+      n_own = own1 - own0;
+      for (int w = own0 + lane; w < own1; w += 32) {
+        const uint32_t u = wkey[w];
+        const int d = wid[w];
         int place = 0;
-        for (int j = 0; j < n_win; ++j) {
-          const uint32_t u = wkey[j];
-          const int sj = wslot[j];
-          place += (sj >= own_lo && sj < own_hi) && ((u > key) || (u == key && sj < slot));
-        }
-        const int id = sidx[slot];
-        const float v = __uint_as_float(key);
-        oidx[place] = id;
-        oval[place] = (!emit_gated && gate != nullptr) ? v / gate[id] : v;
+#pragma unroll 8
+        for (int j = own0; j < own1; ++j) place += wkey[j] + (j < w ? 1u : 0u) > u;  // (a key's successor is no overflow: keys are below 2^31)
+        const float v = __uint_as_float(u);
+        oidx[place] = d;
+        oval[place] = (!emit_gated && gate != nullptr) ? v / gate[d] : v;
       }
+    }
+    for (int i = n_own + lane; i < k; i += 32) {
+      oidx[i] = -1;
+      oval[i] = 0.0f;
     }
     __syncwarp();
     if (comm.mode == kMergePush) {
@@ -135,15 +173,17 @@ topk_merge_kernel(const float* cand_val, const int* cand_idx, int M, int C, int 
 int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, int k, const float* gate,
                       int own_lo, int own_hi, int emit_gated, int* out_idx, float* out_val, const MergeComm& comm,
                       cudaStream_t stream) {
-  const size_t smem = (size_t)MERGE_WARPS * (2 * (size_t)C + 4 * (size_t)k) * 4;
+  const int per = C <= 128 ? 4 : C <= 256 ? 8 : C <= 512 ? 16 : C <= 768 ? 24 : 0;
+  const size_t smem = (size_t)MERGE_WARPS * (4 * (size_t)k + (per == 0 ? 2 * (size_t)C : 0)) * 4;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   if (comm.mode != kMergePush && (out_idx == nullptr || out_val == nullptr)) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(topk_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kern = per == 4 ? topk_merge_kernel<4> : per == 8 ? topk_merge_kernel<8> : per == 16 ? topk_merge_kernel<16> : per == 24 ? topk_merge_kernel<24> : topk_merge_kernel<0>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   int blocks = (M + MERGE_WARPS - 1) / MERGE_WARPS;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  topk_merge_kernel<<<blocks, MERGE_WARPS * 32, smem, stream>>>(cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
-                                                               emit_gated, out_idx, out_val, comm);
+  kern<<<blocks, MERGE_WARPS * 32, smem, stream>>>(cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
+                                                  emit_gated, out_idx, out_val, comm);
   return (int)cudaGetLastError();
 }
 
