@@ -320,7 +320,8 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
 // ---------------------------------------------------------------------------------------------
 // group (row, slot) pairs by feature: counts -> offsets (exclusive scan) -> entries
 // ---------------------------------------------------------------------------------------------
-__global__ void csc_count_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ counts) {
+__global__ void csc_count_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ counts, int* __restrict__ heavy) {
+  if (heavy != nullptr && blockIdx.x == 0 && threadIdx.x == 0) heavy[0] = 0;  // (counted by the scan that follows)
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int f = idx[i];
     if (f >= 0 && f < F) atomicAdd(&counts[f], 1);
@@ -417,6 +418,45 @@ csc_scan_add_kernel(const int* __restrict__ block_sums, int F, int* __restrict__
   }
 }
 
+// The three in one launch: a block adds up all counts before its own 4096 instead of waiting for the other blocks' totals. The last block
+// reads the whole array from L2: up to 2^17 features (half a megabyte, 4 us) that costs less than two launches (24576 features: 9.1 ->
+// 6.0 us, and a memset less).
+constexpr int kOneScanFeatures = 1 << 17;
+__global__ void __launch_bounds__(SCAN_THREADS)
+csc_scan_kernel(const int* __restrict__ counts, int F, int* __restrict__ offsets, int* __restrict__ cursor, int* __restrict__ heavy, int heavy_cap) {
+  __shared__ int s_warp[33];
+  const int first = blockIdx.x * SCAN_ELEMS, base = first + threadIdx.x * 4;
+  int before = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < first / 4; i += SCAN_THREADS) {
+    const int4 c = __ldg(reinterpret_cast<const int4*>(counts) + i);
+    before += c.x + c.y + c.z + c.w;
+  }
+  int carry;
+  block_exclusive_scan_1024(before, s_warp, carry);
+  __syncthreads();  // (the scan's words are used again)
+  int c[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    c[i] = (base + i < F) ? counts[base + i] : 0;
+    if (heavy != nullptr && c[i] > kHeavyRow) {
+      const int pos = atomicAdd(heavy, 1);
+      if (pos < heavy_cap) heavy[1 + pos] = base + i;
+    }
+  }
+  int total;
+  int run = carry + block_exclusive_scan_1024(c[0] + c[1] + c[2] + c[3], s_warp, total);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (base + i < F) {
+      offsets[base + i] = run;
+      cursor[base + i] = run;
+    }
+    run += c[i];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) offsets[F] = carry + total;
+}
+
 __global__ void csc_fill_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ cursor,
                                 int* __restrict__ entries) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -503,22 +543,22 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
   }
   cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)F * sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;
-  if (heavy != nullptr) {
-    if ((long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;  // room for every row there can be
-    e = cudaMemsetAsync(heavy, 0, sizeof(int), stream);
-    if (e != cudaSuccess) return (int)e;
-  }
+  if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;  // room for every row there can be
   const int threads = 256;
   int blocks = (int)((n + threads - 1) / threads);
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  csc_count_kernel<<<blocks, threads, 0, stream>>>(idx, n, F, counts);
+  csc_count_kernel<<<blocks, threads, 0, stream>>>(idx, n, F, counts, heavy);
   // `block_sums_buf` holds one int per 4096 features
   const int nblocks = (F + SCAN_ELEMS - 1) / SCAN_ELEMS;
-  int* block_sums = block_sums_buf;
-  csc_scan_local_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, F, offsets, block_sums, heavy, heavy_cap);
-  csc_scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(block_sums, nblocks, offsets, F);
-  csc_scan_add_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(block_sums, F, offsets, cursor);
+  if (F <= kOneScanFeatures && reinterpret_cast<uintptr_t>(counts) % 16 == 0) {
+    csc_scan_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, F, offsets, cursor, heavy, heavy_cap);
+  } else {
+    int* block_sums = block_sums_buf;
+    csc_scan_local_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, F, offsets, block_sums, heavy, heavy_cap);
+    csc_scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(block_sums, nblocks, offsets, F);
+    csc_scan_add_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(block_sums, F, offsets, cursor);
+  }
   csc_fill_kernel<<<blocks, threads, 0, stream>>>(idx, n, F, cursor, entries);
   return (int)cudaGetLastError();
 }
