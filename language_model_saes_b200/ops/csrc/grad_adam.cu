@@ -91,12 +91,18 @@ struct GroupCtx {
   float* dots;             // [W][32] partial dot products (W > 1)
 };
 
+// Entries whose rows are requested at once, as the registers allow: with short rows a feature's time is the latency of its entries' rows, one
+// group of them after the other (512 x 8 codes of 256 rows of 64: 29 -> 23 us; four at a time of rows of 512 spilled and gained nothing).
+template <int NCH>
+__host__ __device__ constexpr int gather_batch() { return NCH == 1 ? 8 : NCH == 2 ? 4 : 2; }
+
 // Rebuilds this group's share of one gradient row: entries [e0 + 32 * first, e1) in batches of 32, every `stride`-th batch.
 // g += coefficient * row, with DOT also the code gradients against the bf16-rounded row in c.rounded. Returns (encoder side)
 // the sum of this lane's coefficients.
 template <bool IS_D, bool DOT, int W, int NCH>
 __device__ __forceinline__ float gather_side(const GradAdamParams& p, const GroupCtx& c, int e0, int e1, int first, int stride,
                                              float (&g)[NCH][4]) {
+  constexpr int Q = gather_batch<NCH>();
   const __nv_bfloat16* src = IS_D ? p.dxhat : p.x;
   float coef_sum = 0.0f;
   for (int eb = e0 + first * 32; eb < e1; eb += stride * 32) {
@@ -112,12 +118,12 @@ __device__ __forceinline__ float gather_side(const GradAdamParams& p, const Grou
     float dot_l = 0.0f;
     unsigned mask = __ballot_sync(0xffffffffu, a_l != 0.0f);  // (the same in every warp of the group)
     while (mask != 0u) {
-      // two entries at a time: all their loads are requested before the first is used
-      int j[2];
-      float a[2];
-      uint2 u[2][NCH];
+      // a few entries at a time: all their loads are requested before the first is used
+      int j[Q];
+      float a[Q];
+      uint2 u[Q][NCH];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < Q; ++q) {
         j[q] = -1;
         a[q] = 0.0f;
         if (mask != 0u) {
@@ -135,7 +141,9 @@ __device__ __forceinline__ float gather_side(const GradAdamParams& p, const Grou
           for (int i = 0; i < NCH; ++i) u[q][i] = make_uint2(0u, 0u);
         }
       }
-      float d0[2] = {0.0f, 0.0f}, d1[2] = {0.0f, 0.0f};
+      float d0[Q], d1[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) d0[q] = d1[q] = 0.0f;
 #pragma unroll
       for (int i = 0; i < NCH; ++i) {
         float w0 = 0.f, w1 = 0.f, w2 = 0.f, w3 = 0.f;
@@ -145,7 +153,7 @@ __device__ __forceinline__ float gather_side(const GradAdamParams& p, const Grou
           w2 = __uint_as_float(w.y << 16); w3 = __uint_as_float(w.y & 0xffff0000u);
         }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {  // (an absent second entry adds zeros)
+        for (int q = 0; q < Q; ++q) {  // (an absent entry adds zeros)
           const float x0 = __uint_as_float(u[q][i].x << 16), x1 = __uint_as_float(u[q][i].x & 0xffff0000u);
           const float x2 = __uint_as_float(u[q][i].y << 16), x3 = __uint_as_float(u[q][i].y & 0xffff0000u);
           fma2(g[i][0], g[i][1], x0, x1, a[q], a[q]);
@@ -158,7 +166,7 @@ __device__ __forceinline__ float gather_side(const GradAdamParams& p, const Grou
       }
       if constexpr (DOT) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < Q; ++q) {
           const float dot = warp_sum(d0[q] + d1[q]);
           if (c.lane == j[q]) dot_l = dot;
         }
