@@ -709,6 +709,19 @@ std::vector<Tensor> colsum_adam(const std::vector<Tensor>& a, const std::vector<
   return out;
 }
 
+// g bf16 [rows, d] becomes zero where mask (bf16 [rows, d], rows any multiple of 8 apart) is; part fp32 [n, d]: column sums of n blocks of rows.
+void mask_colsum(const Tensor& g, const Tensor& mask, const Tensor& part) {
+  CHECK_T(g, torch::kBFloat16); CHECK_T(part, torch::kFloat32);
+  TORCH_CHECK(mask.is_cuda() && mask.scalar_type() == torch::kBFloat16 && mask.dim() == 2 && g.dim() == 2 && mask.sizes() == g.sizes() && mask.stride(1) == 1 &&
+                  mask.stride(0) % 8 == 0 && g.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0 &&
+                  reinterpret_cast<uintptr_t>(mask.data_ptr()) % 16 == 0, "mask_colsum: aligned rows of a multiple of 8 columns");
+  TORCH_CHECK(part.dim() == 2 && part.size(1) == g.size(1) && part.size(0) >= 1 && part.size(0) < 65536 && g.size(0) < (1LL << 31), "mask_colsum: part [n, d]");
+  const c10::cuda::CUDAGuard guard(g.device());
+  check_cuda(lmsae::mask_colsum_launch(reinterpret_cast<__nv_bfloat16*>(g.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(mask.data_ptr()), mask.stride(0),
+                                       (int)g.size(0), (int)g.size(1), (int)part.size(0), part.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "mask_colsum launch");
+}
+
 void adam_flat(const Tensor& p, const Tensor& g, const Tensor& m, const Tensor& v, const c10::optional<Tensor>& grad_mul,
                const c10::optional<Tensor>& shadow, const c10::optional<Tensor>& grad_sq_sum, double lr, double beta1,
                double beta2, double eps, int64_t step, bool update, const c10::optional<Tensor>& status) {
@@ -1492,6 +1505,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sparse_grad_adam", &sparse_grad_adam);
   m.def("colsum_bf16", &colsum_bf16);
   m.def("colsum_adam", &colsum_adam);
+  m.def("mask_colsum", &mask_colsum);
   m.def("adam_flat", &adam_flat);
   m.def("row_norm_shadow", &row_norm_shadow);
 }

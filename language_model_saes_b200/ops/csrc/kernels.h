@@ -239,6 +239,7 @@ struct ColsumAdamParams {
   float loss_den;
   float *loss_out, *loss_out2;   // (sum + sum2) / den, sum2 / den
 };
+int mask_colsum_launch(__nv_bfloat16* g, const __nv_bfloat16* mask, long long ld, int rows, int d, int row_blocks, float* part, cudaStream_t stream);
 int colsum_adam_row_blocks(int col_blocks, int rows);
 int colsum_adam_launch(ColsumAdamParams p, int col_blocks, cudaStream_t stream);
 int adam_flat_launch(float* p, const float* g, float* m, float* v, long long n, AdamHyper h, const float* grad_mul,

@@ -945,6 +945,62 @@ colsum_adam_kernel(const ColsumAdamParams p) {
   g.p[c] = pi; g.m[c] = mi; g.v[c] = vi;
 }
 
+// g [rows, d] keeps its values where mask [rows, d] (rows ld elements apart) is not zero and becomes zero elsewhere, in place, and the column
+// sums of what is kept go to part [gridDim.y][d] (one row per block of rows; added up by the caller). Bound by memory: 4096 x 9216: 226 MB.
+// As tensor operations (comparison, product, sum): 86 + 127 + 28 us; here 33.
+__global__ void __launch_bounds__(256)
+mask_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ mask, long long ld, int rows, int d, int rows_per_block, float* __restrict__ part) {
+  __shared__ float s_sum[8][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col0 = blockIdx.x * 256, col = col0 + lane * 8;
+  const int r0 = blockIdx.y * rows_per_block, r1 = min(rows, r0 + rows_per_block);
+  float acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+  if (col < d) {  // (d is a multiple of 8)
+    for (int r = r0 + warp; r < r1; r += 32) {
+      uint4 u[4], m[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (r + q * 8 < r1) {
+          u[q] = *reinterpret_cast<const uint4*>(g + (size_t)(r + q * 8) * d + col);
+          m[q] = __ldg(reinterpret_cast<const uint4*>(mask + (r + q * 8) * ld + col));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (r + q * 8 >= r1) continue;
+        uint32_t w[4] = {u[q].x, u[q].y, u[q].z, u[q].w};
+        const uint32_t k[4] = {m[q].x, m[q].y, m[q].z, m[q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if ((k[i] & 0x7fffu) == 0u) w[i] &= 0xffff0000u;
+          if ((k[i] & 0x7fff0000u) == 0u) w[i] &= 0xffffu;
+          acc[2 * i] += __uint_as_float(w[i] << 16);
+          acc[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+        }
+        *reinterpret_cast<uint4*>(g + (size_t)(r + q * 8) * d + col) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s_sum[warp][i * 32 + lane] = acc[i];
+  __syncthreads();
+  float s = 0.0f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s += s_sum[w][threadIdx.x];
+  const int c = col0 + (threadIdx.x & 31) * 8 + (threadIdx.x >> 5);
+  if (c < d) part[(size_t)blockIdx.y * d + c] = s;
+}
+
+int mask_colsum_launch(__nv_bfloat16* g, const __nv_bfloat16* mask, long long ld, int rows, int d, int row_blocks, float* part, cudaStream_t stream) {
+  if (d % 8 != 0 || ld % 8 != 0 || rows < 0 || row_blocks < 1) return (int)cudaErrorInvalidValue;
+  if (d == 0) return 0;
+  const int rpb = (rows + row_blocks - 1) / row_blocks;
+  mask_colsum_kernel<<<dim3((d + 255) / 256, row_blocks), 256, 0, stream>>>(g, mask, ld, rows, d, rpb, part);
+  return (int)cudaGetLastError();
+}
+
 // Row blocks for a launch of `col_blocks` blocks of 256 columns: four CTAs per SM, at least 64 rows each.
 int colsum_adam_row_blocks(int col_blocks, int rows) {
   int n = 592 / (col_blocks > 0 ? col_blocks : 1);

@@ -695,10 +695,9 @@ class FusedTopKSAEStep:
         dact = torch.empty_like(act) if fused_dact else K.sparse_dact(idx, self.WD_bf16, g_main)
         self._mark("loss_grad_dact")
         # gradient of the dead activations where they were selected (bf16 on the GPU: it is an operand of the next product)
-        dA = (g_aux @ wd_dead.t() if x.is_cuda else _mm_f32(g_aux, wd_dead.t())) * (A != 0)
+        dA, extra_gb = K.mask_colsum_(g_aux @ wd_dead.t() if x.is_cuda else _mm_f32(g_aux, wd_dead.t()), A)
         extra_gD = _mm_f32(A.t(), g_aux)  # d W_D rows of the compact dictionary
         extra_gE = _mm_f32(dA.to(torch.bfloat16).t(), x)  # d W_E^T rows
-        extra_gb = dA.sum(0, dtype=torch.float32)
         slots = torch.arange(cap, dtype=torch.int32, device=x.device)
         if sharded:
             # dense rows: summed over replicas, each replica receiving the block of the rows it updates (the sparse main

@@ -732,6 +732,18 @@ def colsum_bf16(a: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def mask_colsum_(g: torch.Tensor, mask: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """``g [rows, d]`` where ``mask [rows, d]`` is not zero and zero elsewhere (on a GPU in place), and its column sums in fp32."""
+    ok = (g.is_cuda and g.dtype == torch.bfloat16 and mask.dtype == torch.bfloat16 and g.is_contiguous() and g.shape[1] % 8 == 0 and mask.stride(1) == 1
+          and mask.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0 and mask.data_ptr() % 16 == 0)  # fmt: skip
+    if not ok:
+        g = g * (mask != 0)
+        return g, g.sum(0, dtype=torch.float32)
+    part = torch.empty(max(1, min(32, g.shape[0] // 32)), g.shape[1], dtype=torch.float32, device=g.device)
+    _ext().mask_colsum(g, mask, part)
+    return g, part.sum(0)
+
+
 def adam_flat(p, g, m, v, lr, beta1, beta2, eps, step, grad_mul=None, shadow=None, grad_sq_sum=None, update=True):
     if not p.is_cuda:
         gg = g * (float(grad_mul) if grad_mul is not None else 1.0)
