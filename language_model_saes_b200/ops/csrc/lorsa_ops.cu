@@ -61,7 +61,9 @@ int lorsa_dz_launch(const int* idx, const float* act, const float* dact, long lo
 // Parameters and moments are [heads, d, w] fp32, the gradient comes out of the product as [heads * w, d] and the products read bf16
 // weights as [heads * w, d]: one pass per 64 x 64 tile turns the gradient on its way in and the new weights on their way out through
 // shared memory. As separate passes the gradients and weights were transposed through memory (66 us for two times 3.1 M
-// parameters, on top of Adam's 36; here 51). Up to two parameter sets of one shape share a launch.
+// parameters, on top of Adam's 36). Up to two parameter sets of one shape share a launch.
+// VEC: four columns a thread and access, where widths and addresses allow (3.1 M parameters twice: 51 -> 37 us).
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 adam_turned_kernel(const AdamTurnedParams p) {
   __shared__ float tile[64][65];  // [w][d]
@@ -69,6 +71,49 @@ adam_turned_kernel(const AdamTurnedParams p) {
   const AdamTurnedSet q = p.set[blockIdx.z];
   const int tiles_w = (p.w + 63) / 64;
   const int h = blockIdx.y / tiles_w, w0 = (blockIdx.y - h * tiles_w) * 64, d0 = blockIdx.x * 64;
+  if constexpr (VEC) {  // (d and w are multiples of 4: whole fours are inside or outside)
+    const int x = (threadIdx.x & 15) * 4, y0 = threadIdx.x >> 4;
+#pragma unroll
+    for (int y = y0; y < 64; y += 16) {
+      if (w0 + y < p.w && d0 + x < p.d) {
+        const float4 g = __ldcs(reinterpret_cast<const float4*>(q.g + ((size_t)h * p.w + w0 + y) * p.d + d0 + x));
+        tile[y][x] = g.x; tile[y][x + 1] = g.y; tile[y][x + 2] = g.z; tile[y][x + 3] = g.w;
+      }
+    }
+    float4 pp[4], pm[4], pv[4];  // (all of a thread's loads before the first is used)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int y = y0 + i * 16;
+      if (d0 + y < p.d && w0 + x < p.w) {
+        const size_t o = ((size_t)h * p.d + d0 + y) * p.w + w0 + x;
+        pp[i] = *reinterpret_cast<const float4*>(q.p + o);
+        pm[i] = *reinterpret_cast<const float4*>(q.m + o);
+        pv[i] = *reinterpret_cast<const float4*>(q.v + o);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int y = y0 + i * 16;
+      if (d0 + y < p.d && w0 + x < p.w) {
+        const size_t o = ((size_t)h * p.d + d0 + y) * p.w + w0 + x;
+        adam_elem(pp[i].x, pm[i].x, pv[i].x, tile[x][y], p.h); adam_elem(pp[i].y, pm[i].y, pv[i].y, tile[x + 1][y], p.h);
+        adam_elem(pp[i].z, pm[i].z, pv[i].z, tile[x + 2][y], p.h); adam_elem(pp[i].w, pm[i].w, pv[i].w, tile[x + 3][y], p.h);
+        *reinterpret_cast<float4*>(q.p + o) = pp[i];
+        *reinterpret_cast<float4*>(q.m + o) = pm[i];
+        *reinterpret_cast<float4*>(q.v + o) = pv[i];
+        tile[x][y] = pp[i].x; tile[x + 1][y] = pp[i].y; tile[x + 2][y] = pp[i].z; tile[x + 3][y] = pp[i].w;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int y = y0; y < 64; y += 16) {
+      if (w0 + y < p.w && d0 + x < p.d)
+        *reinterpret_cast<uint2*>(q.shadow + ((size_t)h * p.w + w0 + y) * p.d + d0 + x) =
+            make_uint2(pack_bf16x2(tile[y][x], tile[y][x + 1]), pack_bf16x2(tile[y][x + 2], tile[y][x + 3]));
+    }
+    return;
+  }
   const int x = threadIdx.x & 63, y0 = threadIdx.x >> 6;
 #pragma unroll 4
   for (int y = y0; y < 64; y += 4)
@@ -95,7 +140,12 @@ int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t strea
   if (n_sets < 1 || n_sets > 2 || p.heads <= 0 || p.d <= 0 || p.w <= 0) return (int)cudaErrorInvalidValue;
   const long long rows = (long long)p.heads * ((p.w + 63) / 64);
   if (rows > 65535) return (int)cudaErrorInvalidValue;
-  adam_turned_kernel<<<dim3((p.d + 63) / 64, (unsigned)rows, n_sets), 256, 0, stream>>>(p);
+  bool vec = p.d % 4 == 0 && p.w % 4 == 0;
+  for (int i = 0; i < n_sets; ++i)
+    vec = vec && ((reinterpret_cast<uintptr_t>(p.set[i].p) | reinterpret_cast<uintptr_t>(p.set[i].m) | reinterpret_cast<uintptr_t>(p.set[i].v) |
+                   reinterpret_cast<uintptr_t>(p.set[i].g) | reinterpret_cast<uintptr_t>(p.set[i].shadow)) % 16 == 0);
+  auto kern = vec ? adam_turned_kernel<true> : adam_turned_kernel<false>;
+  kern<<<dim3((p.d + 63) / 64, (unsigned)rows, n_sets), 256, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }
 

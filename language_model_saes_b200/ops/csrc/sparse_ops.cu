@@ -862,7 +862,7 @@ int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cuda
 //   eighth row; the row blocks' sums go through memory, and the last row block of a column block to arrive adds them up in order
 //   (the sum does not depend on the order of arrival) and applies Adam.
 // As five launches (fill, column sums by atomics, Adam; a fill and a division for the loss): 4096 rows of 768: 7.7 + 2.8 + 5 us, 4096
-// rows of 4096: 14.6 + 2.8 + 5; here 9.6 and 16.2. In steps of small dictionaries the four launches less count more than that (512 rows
+// rows of 4096: 14.6 + 2.8 + 5; here 9.6 and 14.8. In steps of small dictionaries the four launches less count more than that (512 rows
 // of 64: a step of 88 us takes 75).
 __global__ void __launch_bounds__(256)
 colsum_adam_kernel(const ColsumAdamParams p) {
@@ -1001,10 +1001,11 @@ int mask_colsum_launch(__nv_bfloat16* g, const __nv_bfloat16* mask, long long ld
   return (int)cudaGetLastError();
 }
 
-// Row blocks for a launch of `col_blocks` blocks of 256 columns: four CTAs per SM, at least 64 rows each.
+// Row blocks for a launch of `col_blocks` blocks of 256 columns: eight CTAs per SM (2048 rows of 17152: 28 us with four, 22 with eight), at least
+// 32 rows each, and no more than 64 partial sums to add up (4096 rows of 768: 9.6 us with 64, 11.0 with 128).
 int colsum_adam_row_blocks(int col_blocks, int rows) {
-  int n = 592 / (col_blocks > 0 ? col_blocks : 1);
-  const int most = (rows + 63) / 64;
+  int n = 1184 / (col_blocks > 0 ? col_blocks : 1);
+  const int most = (rows + 31) / 32;
   n = n < most ? n : most;
   return n < 1 ? 1 : (n > 64 ? 64 : n);
 }

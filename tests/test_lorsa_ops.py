@@ -21,7 +21,7 @@ def _ref(p, m, v, g, step):
 
 
 @pytest.mark.parametrize("dev", DEVICES)
-@pytest.mark.parametrize("heads,d,w,sets", [(1, 8, 8, 1), (2, 64, 64, 2), (3, 72, 16, 2), (2, 200, 136, 1)])
+@pytest.mark.parametrize("heads,d,w,sets", [(1, 8, 8, 1), (2, 64, 64, 2), (3, 72, 16, 2), (2, 200, 136, 1), (2, 70, 68, 2), (1, 9, 5, 1)])
 def test_adam_on_turned_gradients(dev, heads, d, w, sets):
     params = [_rand(dev, heads, d, w, seed=i) for i in range(sets)]
     moments = [(0.1 * _rand(dev, heads, d, w, seed=10 + i), _rand(dev, heads, d, w, seed=20 + i).square()) for i in range(sets)]
