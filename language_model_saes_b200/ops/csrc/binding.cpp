@@ -140,9 +140,12 @@ int64_t encoder_gemm(const Tensor& x, const Tensor& w, const c10::optional<Tenso
   int ks = 0;
   if (mode & 1) {
     TORCH_CHECK(H.has_value(), "mode bit 0 needs H");
-    CHECK_T(*H, torch::kBFloat16);
-    TORCH_CHECK(H->size(0) == p.M && H->size(1) == p.N);
-    p.H = reinterpret_cast<__nv_bfloat16*>(H->data_ptr());
+    const bool f32 = H->scalar_type() == torch::kFloat32;
+    CHECK_T(*H, f32 ? torch::kFloat32 : torch::kBFloat16);
+    TORCH_CHECK(H->size(0) == p.M && H->size(1) == p.N && (!f32 || ((mode & 2) == 0 && !gate.has_value() && reinterpret_cast<uintptr_t>(H->data_ptr()) % 16 == 0)),
+                "H [M, N]; in fp32 without a gate and without top-k");
+    if (f32) p.H32 = H->data_ptr<float>();
+    else p.H = reinterpret_cast<__nv_bfloat16*>(H->data_ptr());
     p.ldh = p.N;
   }
   if (maxima.has_value()) {
@@ -355,6 +358,24 @@ void row_topk(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate, con
                                     max_ptr, max_ptr != nullptr ? maxima->size(1) : 0, out_idx.data_ptr<int>(), out_val.data_ptr<float>(),
                                     at::cuda::getCurrentCUDAStream()),
              "row_topk launch");
+}
+
+// Row top-k (k <= 128) of H (bf16 or fp32 [M, N], N % 8 == 0) by its gated maxima of every 32 columns.
+bool row_select_fits(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate) {
+  return k >= 1 && k <= lmsae::row_select_max_k() && H.size(1) % 8 == 0 && H.size(1) <= 65535 * 32 && reinterpret_cast<uintptr_t>(H.data_ptr()) % 16 == 0 &&
+         (!gate.has_value() || reinterpret_cast<uintptr_t>(gate->data_ptr()) % 16 == 0);
+}
+void row_select(const Tensor& H, const Tensor& maxima, int64_t k, const c10::optional<Tensor>& gate, bool sorted, const Tensor& out_idx, const Tensor& out_val) {
+  const bool f32 = H.scalar_type() == torch::kFloat32;
+  CHECK_T(H, f32 ? torch::kFloat32 : torch::kBFloat16); CHECK_T(out_idx, torch::kInt32); CHECK_T(out_val, torch::kFloat32);
+  TORCH_CHECK(H.dim() == 2 && out_idx.numel() >= H.size(0) * k && out_val.numel() >= H.size(0) * k && H.size(0) < (1LL << 31) && row_select_fits(H, k, gate), "row_select: sizes");
+  if (gate.has_value()) { CHECK_T(*gate, torch::kFloat32); TORCH_CHECK(gate->numel() == H.size(1)); }
+  const float* m = checked_maxima(maxima, H.size(0), H.size(1));
+  const c10::cuda::CUDAGuard guard(H.device());
+  check_cuda(lmsae::row_select_launch(f32 ? nullptr : reinterpret_cast<const __nv_bfloat16*>(H.data_ptr()), f32 ? H.data_ptr<float>() : nullptr, H.size(1), m,
+                                      maxima.size(1), (int)H.size(0), (int)H.size(1), (int)k, opt_ptr<const float>(gate), sorted ? 1 : 0,
+                                      out_idx.data_ptr<int>(), out_val.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
+             "row_select launch");
 }
 
 // x_hat = decode(idx, val); optional outputs and fused loss as described in sparse_ops.cu.
@@ -1492,6 +1513,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("row_select", &row_select);
+  m.def("row_select_fits", &row_select_fits);
   m.def("topk_dense", &topk_dense);
   m.def("topk_estimate", &topk_estimate);
   m.def("fp32_gemm", &fp32_gemm);

@@ -53,7 +53,7 @@ __host__ __device__ constexpr int epilogue_warps(bool topk) { return topk ? 4 : 
 constexpr int kNarrowTiles = 255;
 constexpr int kCarried = kNarrowTiles * BN;
 
-template <int STAGES, int CAP, bool PAIR, bool NARROW>
+template <int STAGES, int CAP, bool PAIR, bool NARROW, bool F32>
 struct SmemLayout {
   static constexpr int kBRows = PAIR ? BN / 2 : BN;       // dictionary rows of a B tile held by one CTA
   static constexpr int kBStageBytes = kBRows * BK * 2;    // 16 KB (pair) / 32 KB
@@ -63,8 +63,8 @@ struct SmemLayout {
   static constexpr int kSlotIdxOff = kSlotValOff + BM * CAP * 4;
   static constexpr int kColOff = kSlotIdxOff + BM * CAP * (NARROW ? 2 : 4);   // per epilogue warp: bias and gate of the 32 columns at work
   static constexpr int kEpilogueWarps = epilogue_warps(CAP != 0);
-  static constexpr int kStoreOff = kColOff + kEpilogueWarps * 64 * 4;  // per epilogue warp: 32 x 32 bf16 on their way to whole sectors of H (no top-k)
-  static constexpr int kMaxOff = kStoreOff + (CAP == 0 ? kEpilogueWarps * 2048 : 0);  // per 32 rows: maxima of a tile's eight groups of columns, [8][32 rows]
+  static constexpr int kStoreOff = kColOff + kEpilogueWarps * 64 * 4;  // per epilogue warp: 32 x 32 values on their way to whole sectors of H (no top-k)
+  static constexpr int kMaxOff = kStoreOff + (CAP == 0 ? kEpilogueWarps * (F32 ? 4096 : 2048) : 0);  // per 32 rows: maxima of a tile's eight groups of columns, [8][32 rows]
   static constexpr int kBarOff = kMaxOff + (CAP == 0 ? 4 * 1024 : 0);
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
@@ -208,11 +208,12 @@ __device__ __noinline__ RowState select_entries(RowBuffer<CAP, NARROW> buf, RowS
   return st;
 }
 
-template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW>
+// F32: H is stored in fp32 (without top-k).
+template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW, bool F32>
 __global__ void __launch_bounds__(128 + 32 * epilogue_warps(TOPK), 1)
 enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const EncGemmParams p) {
-  using L = SmemLayout<STAGES, CAP, PAIR, NARROW>;
+  using L = SmemLayout<STAGES, CAP, PAIR, NARROW, F32>;
   constexpr int STAGE_BYTES = L::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -472,7 +473,7 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                                                                 pack_bf16x2(v[j + 4], v[j + 5]), pack_bf16x2(v[j + 6], v[j + 7]));
           }
         }
-        if (TOPK || p.gate != nullptr) {
+        if (!F32 && (TOPK || p.gate != nullptr)) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             const float4 g4 = *reinterpret_cast<const float4*>(col_gate + j);
@@ -480,7 +481,36 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             mul_pair(v[j + 2], v[j + 3], g4.z, g4.w);
           }
         }
-        if constexpr (WRITE_H && !TOPK) {
+        if constexpr (WRITE_H && !TOPK && F32) {
+          // (as below, with 128 bytes of a row: eight lanes write a line)
+          uint8_t* tile_s = smem + L::kStoreOff + (warp - 4) * 4096;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<float4*>(tile_s + lane * 128 + ((j ^ (lane & 7)) * 16)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          if (p.maxima != nullptr) {
+            float m[4] = {__int_as_float(0xff800000), __int_as_float(0xff800000), __int_as_float(0xff800000), __int_as_float(0xff800000)};
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              if (p.max_gate != nullptr) {
+                const float4 g4 = *reinterpret_cast<const float4*>(col_gate + j);
+                mul_pair(v[j], v[j + 1], g4.x, g4.y);
+                mul_pair(v[j + 2], v[j + 3], g4.z, g4.w);
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) m[i] = max_nan(m[i], v[j + i]);
+            }
+            tile_max[chunk * 32] = max_nan(max_nan(m[0], m[1]), max_nan(m[2], m[3]));
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rr = i * 4 + (lane >> 3), j = lane & 7;
+            const float4 o = *reinterpret_cast<const float4*>(tile_s + rr * 128 + ((j ^ (rr & 7)) * 16));
+            if (m0 + q * 32 + rr < p.M && c0 + j * 4 < p.N)  // (N % 8 == 0)
+              *reinterpret_cast<float4*>(p.H32 + (long long)(m0 + q * 32 + rr) * p.ldh + c0 + j * 4) = o;
+          }
+        }
+        if constexpr (WRITE_H && !TOPK && !F32) {
           // A thread holds 64 bytes of its own row: through shared memory (16-byte pieces, swizzled: no bank conflicts), so that
           // four lanes write whole sectors of a row. Stored from the registers, every instruction touched 32 rows by half a
           // sector each: 4096 x 24576 x 768: 198 (with a gate: 425) -> 135 (149) us.
@@ -615,12 +645,12 @@ enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 }
 
 // ---- host side -------------------------------------------------------------------------------
-template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW = false>
+template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool NARROW = false, bool F32 = false>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p,
                                   cudaStream_t stream) {
-  using L = SmemLayout<STAGES, CAP, PAIR, NARROW>;
+  using L = SmemLayout<STAGES, CAP, PAIR, NARROW, F32>;
   static_assert(L::kDynamicBytes <= 232448, "shared memory of one CTA exceeds 227 KB");
-  auto kern = enc_gemm_kernel<WRITE_H, TOPK, STAGES, KS, CAP, PAIR, NARROW>;
+  auto kern = enc_gemm_kernel<WRITE_H, TOPK, STAGES, KS, CAP, PAIR, NARROW, F32>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -660,7 +690,10 @@ int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmP
   const int n_tiles = (p.N + BN - 1) / BN, panel_units = pair ? p.num_panels / 2 : p.num_panels;
   const int ranges = p.units != 0 ? p.units / panel_units : p.num_splits;
   const bool narrow = (n_tiles + ranges - 1) / ranges <= kNarrowTiles, large = p.K <= 2048 || p.k > 56;
-  if (!tk) {
+  if (!tk && p.H32 != nullptr) {
+    if (p.gate != nullptr || !wh) return (int)cudaErrorInvalidValue;
+    e = pair ? launch_variant<true, false, 5, 0, 0, true, false, true>(ta, tb, p, stream) : launch_variant<true, false, 3, 0, 0, false, false, true>(ta, tb, p, stream);
+  } else if (!tk) {
     if (pair) e = launch_variant<true, false, 6, 0, 0, true>(ta, tb, p, stream);
     else e = (mode & 4) ? launch_variant<true, false, 3, 0, 0, false>(ta, tb, p, stream)
                         : launch_variant<true, false, 4, 0, 0, false>(ta, tb, p, stream);

@@ -19,6 +19,7 @@ struct EncGemmParams {
   const float* bias;
   const float* gate;
   __nv_bfloat16* H;
+  float* H32;  // or H in fp32 (without a gate and without top-k)
   long long ldh;
   int k;
   float* cand_val;
@@ -331,6 +332,11 @@ int chunk_hist_launch(const __nv_bfloat16* x, const float* maxima, long long ld_
                       cudaStream_t stream);
 int chunk_compact_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* thr, const float* col_div, int* nnz,
                          int* ties, const int* tie_quota, int cap, int* idx, float* val, cudaStream_t stream);
+
+// Row top-k of stored pre-activations (one of H16, H32) by the maxima of 32 columns; sorted: values in descending order.
+int row_select_launch(const __nv_bfloat16* H16, const float* H32, long long ldh, const float* maxima, long long ld_maxima, int M, int N, int k,
+                      const float* gate, int sorted, int* out_idx, float* out_val, cudaStream_t stream);
+int row_select_max_k();
 
 // ---- low-rank sparse attention step (lorsa_ops.cu) ----------------------------------------------------
 int lorsa_dz_smem(int F, int k);

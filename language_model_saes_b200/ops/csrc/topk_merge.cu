@@ -206,9 +206,12 @@ constexpr int RT_CAP = 10 * RT_THREADS;  // candidates in shared memory
 constexpr int RT_MAX_GROUPS = 1024;  // of 32 columns that reach the bound, where their maxima are known (half as many codes are allowed for)
 constexpr int RT_BOUND_K = RT_THREADS * RT_MAXIMA / 2;  // (about 1.4 k candidates there, k + a few for small k)
 
-__device__ __forceinline__ float gated_value(const __nv_bfloat16* __restrict__ hrow, const float* __restrict__ gate,
+__device__ __forceinline__ float stored_value(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ float stored_value(const float* p) { return *p; }
+template <typename T>
+__device__ __forceinline__ float gated_value(const T* __restrict__ hrow, const float* __restrict__ gate,
                                              const uint8_t* __restrict__ alive, int c) {
-  float v = __bfloat162float(hrow[c]);
+  float v = stored_value(hrow + c);
   if (gate != nullptr) v *= gate[c];
   if (alive != nullptr && alive[c] == 0) v = 0.0f;
   return v;
@@ -243,7 +246,8 @@ __device__ __forceinline__ void gated_values8(const __nv_bfloat16* __restrict__ 
 }
 
 // The radix descent over the row: 4 passes of 8 bits, 256-bin histogram in shared memory, then one pass over the survivors.
-__device__ __noinline__ void row_topk_radix(const __nv_bfloat16* __restrict__ hrow, int row, int N, int k, const float* __restrict__ gate,
+template <typename T>
+__device__ __noinline__ void row_topk_radix(const T* __restrict__ hrow, int row, int N, int k, const float* __restrict__ gate,
                                             const uint8_t* __restrict__ alive, int* __restrict__ out_idx, float* __restrict__ out_val) {
   __shared__ unsigned hist[256];
   __shared__ unsigned s_prefix, s_remaining, s_count_gt, s_cursor_gt, s_cursor_eq;
@@ -482,6 +486,270 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
     }
   }
   row_topk_radix(hrow, row, N, k, gate, alive, out_idx, out_val);
+}
+
+// Row top-k of stored pre-activations whose gated maxima per 32 columns are known, a warp per row (the encoder GEMM's epilogue leaves
+// the maxima; T is how it stored the values). The rows of a batch are all in flight at once, and what a row takes is a short chain:
+//   bound     512 groups of one or more neighbouring maxima at most, in registers: their k-th largest, 16 leading bits of it, which at
+//             least k columns reach and with four times as many groups as codes few more do
+//   groups    of 32 columns whose maximum reaches it, about k of them, listed in order; their columns, eight a lane
+//   candidates above the bound listed in order; the exact k-th value of them; of equal ones the first columns
+// Rows with more groups or candidates than there is room for (values repeated hundreds of times) are taken by the whole CTA afterwards, in
+// the descent over the row that other kernels end in, too.
+// As a CTA per row with barriers between the steps, 4096 rows of 32768 bf16, k 128: 153 us; here 61 (1024 rows: 46 and 37; 512 rows, where
+// the chain is all there is: 29 and 36). 1024 rows of 16384 fp32, k 32: 20 us.
+constexpr int RS_WARPS = 8, RS_PER = 16, RS_GROUPS = 256, RS_CAND = 384, RS_MAX_K = 128;
+static_assert(RS_WARPS * 32 == RT_THREADS, "the fallback's CTA");
+template <typename T>
+__device__ __forceinline__ void stored_values8(const T* p, float (&v)[8]);
+template <>
+__device__ __forceinline__ void stored_values8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+  const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+template <>
+__device__ __forceinline__ void stored_values8<float>(const float* p, float (&v)[8]) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// The largest t whose lowest `skip` bits are zero with count(key >= t) >= k over the warp, or (exactly = true) one that exactly k reach.
+template <int N>
+__device__ __forceinline__ unsigned warp_descend(const unsigned (&key)[N], int k, int skip, bool& exactly) {
+  static_assert(N * 32 < 1024, "counts are packed in ten bits each");
+  unsigned t = 0;
+  exactly = false;
+  for (int shift = 30; shift >= skip && !exactly; shift -= 2) {  // (bit 31 is never set)
+    const unsigned t1 = t | (1u << shift), t2 = t | (2u << shift), t3 = t | (3u << shift);
+    unsigned n = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) n += (unsigned)(key[i] >= t1) + ((unsigned)(key[i] >= t2) << 10) + ((unsigned)(key[i] >= t3) << 20);
+    n = __reduce_add_sync(0xffffffffu, n);
+    const int c1 = (int)(n & 1023u), c2 = (int)((n >> 10) & 1023u), c3 = (int)(n >> 20);
+    if (c3 >= k) { t = t3; exactly = c3 == k; }
+    else if (c2 >= k) { t = t2; exactly = c2 == k; }
+    else if (c1 >= k) { t = t1; exactly = c1 == k; }
+  }
+  return t;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(RT_THREADS)
+row_select_kernel(const T* __restrict__ H, long long ldh, const float* __restrict__ maxima, long long ld_maxima, int M, int N, int k,
+                  const float* __restrict__ gate, int sorted, int* __restrict__ out_idx, float* __restrict__ out_val) {
+  __shared__ unsigned short s_group[RS_WARPS][RS_GROUPS];
+  __shared__ unsigned s_key[RS_WARPS][RS_CAND];
+  __shared__ int s_col[RS_WARPS][RS_CAND];
+  __shared__ int s_full[RS_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int row = blockIdx.x * RS_WARPS + warp;
+  if (lane == 0) s_full[warp] = 0;
+  if (row < M) {
+    const T* hrow = H + (long long)row * ldh;
+    const float* mrow = maxima + (long long)row * ld_maxima;
+    const int n_groups = (N + 31) / 32, fold = (n_groups + RS_PER * 32 - 1) / (RS_PER * 32);
+    unsigned mx[RS_PER];
+#pragma unroll
+    for (int i = 0; i < RS_PER; ++i) mx[i] = 0u;  // (non-positive values and NaN never enter)
+    for (int f = 0; f < fold; ++f) {
+      float m[RS_PER];
+#pragma unroll
+      for (int i = 0; i < RS_PER; ++i) {
+        const int g = (f * RS_PER + i) * 32 + lane;
+        m[i] = g < n_groups ? __ldg(mrow + g) : 0.0f;
+      }
+#pragma unroll
+      for (int i = 0; i < RS_PER; ++i) mx[i] = max(mx[i], __float_as_uint(fmaxf(m[i], 0.0f)) & 0x7fffffffu);
+    }
+    bool exactly;
+    const unsigned bound = warp_descend(mx, k, 16, exactly);
+    int n_list = 0;
+    for (int g0 = 0; g0 < n_groups; g0 += 256) {
+      float m[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m[i] = g0 + i * 32 + lane < n_groups ? __ldg(mrow + g0 + i * 32 + lane) : 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool hit = m[i] > 0.0f ? __float_as_uint(m[i]) >= bound : m[i] != m[i];  // (a NaN hides the others' maximum)
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        const int pos = n_list + __popc(hits & below);
+        if (hit && pos < RS_GROUPS) s_group[warp][pos] = (unsigned short)(g0 + i * 32 + lane);
+        n_list += __popc(hits);
+      }
+    }
+    __syncwarp();
+    int n_cand = n_list > RS_GROUPS ? RS_CAND + 1 : 0;
+    if (n_list <= RS_GROUPS) {
+      for (int e0 = 0; e0 < n_list; e0 += 16) {  // sixteen groups, four lanes each, two per lane in flight
+        float v[2][8];
+        int c[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = e0 + h * 8 + (lane >> 2);
+          c[h] = e < n_list ? s_group[warp][e] * 32 + (lane & 3) * 8 : N;
+          if (c[h] < N) {  // (N is a multiple of 8)
+            stored_values8<T>(hrow + c[h], v[h]);
+            if (gate != nullptr) {
+              const float4 a = __ldg(reinterpret_cast<const float4*>(gate + c[h])), b = __ldg(reinterpret_cast<const float4*>(gate + c[h]) + 1);
+              v[h][0] *= a.x; v[h][1] *= a.y; v[h][2] *= a.z; v[h][3] *= a.w;
+              v[h][4] *= b.x; v[h][5] *= b.y; v[h][6] *= b.z; v[h][7] *= b.w;
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[h][i] = 0.0f;
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          unsigned in = 0u;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) in |= (v[h][i] > 0.0f && __float_as_uint(v[h][i]) >= bound) ? 1u << i : 0u;
+          int inc = __popc(in);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += a;
+          }
+          int pos = n_cand + inc - __popc(in);
+          n_cand += __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if ((in >> i) & 1u) {
+              if (pos < RS_CAND) {
+                s_key[warp][pos] = __float_as_uint(v[h][i]);
+                s_col[warp][pos] = c[h] + i;
+              }
+              ++pos;
+            }
+          }
+        }
+      }
+    }
+    if (n_cand > RS_CAND) {
+      if (lane == 0) s_full[warp] = 1;
+    } else {
+      __syncwarp();
+      unsigned key[RS_CAND / 32];
+#pragma unroll
+      for (int i = 0; i < RS_CAND / 32; ++i) key[i] = i * 32 + lane < n_cand ? s_key[warp][i * 32 + lane] : 0u;
+      unsigned t = 0;
+      exactly = false;
+      if (n_cand > k) t = warp_descend(key, k, 0, exactly);
+      int above = 0;
+#pragma unroll
+      for (int i = 0; i < RS_CAND / 32; ++i) above += key[i] > t;
+      const int ties_wanted = exactly ? k : t == 0u ? 0 : k - __reduce_add_sync(0xffffffffu, above);
+      int n_win = 0, ties_seen = 0;
+#pragma unroll
+      for (int i = 0; i < RS_CAND / 32; ++i) {
+        const bool eq = t != 0u && key[i] == t;
+        const unsigned eqs = __ballot_sync(0xffffffffu, eq);
+        const bool win = key[i] > t || (eq && ties_seen + __popc(eqs & below) < ties_wanted);
+        const unsigned wins = __ballot_sync(0xffffffffu, win);
+        const int col = win ? s_col[warp][i * 32 + lane] : 0;
+        __syncwarp();
+        if (win) {  // (to the front, at or before its own place)
+          const int pos = n_win + __popc(wins & below);
+          s_key[warp][pos] = key[i];
+          s_col[warp][pos] = col;
+        }
+        n_win += __popc(wins);
+        ties_seen += __popc(eqs);
+        __syncwarp();
+      }
+      for (int w = lane; w < k; w += 32) {
+        int place = w, col = -1;
+        float val = 0.0f;
+        if (w < n_win) {
+          const unsigned u = s_key[warp][w];
+          col = s_col[warp][w];
+          val = __uint_as_float(u);
+          if (gate != nullptr) val /= __ldg(gate + col);
+          if (sorted) {
+            place = 0;
+#pragma unroll 8
+            for (int j = 0; j < n_win; ++j) place += s_key[warp][j] + (j < w ? 1u : 0u) > u;
+          }
+        }
+        out_idx[(size_t)row * k + place] = col;
+        out_val[(size_t)row * k + place] = val;
+      }
+    }
+  }
+  __syncthreads();
+  for (int w = 0; w < RS_WARPS; ++w) {
+    const int r = blockIdx.x * RS_WARPS + w;
+    if (s_full[w] != 0) {
+      const T* hrow = H + (long long)r * ldh;
+      int* idx = out_idx + (size_t)r * k;
+      float* val = out_val + (size_t)r * k;
+      row_topk_radix(hrow, r, N, k, gate, nullptr, out_idx, out_val);
+      __syncthreads();
+      // (which takes any of equal values, in any order) the first columns of the k-th value; values in descending order
+      const int i = threadIdx.x;
+      if (i < k) {
+        s_col[0][i] = idx[i];
+        s_key[0][i] = idx[i] >= 0 ? __float_as_uint(gated_value(hrow, gate, nullptr, idx[i])) : 0u;
+      }
+      __syncthreads();
+      unsigned least = 0xffffffffu;
+      for (int j = 0; j < k; ++j) least = min(least, s_key[0][j]);
+      int n_above = 0;
+      for (int j = 0; j < k; ++j) n_above += s_key[0][j] > least;
+      if (least != 0u && warp == 0) {
+        int n = 0;
+        for (int c0 = 0; c0 < N && n < k - n_above; c0 += 256) {
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = c0 + j * 32 + lane < N ? gated_value(hrow, gate, nullptr, c0 + j * 32 + lane) : 0.0f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const bool eq = v[j] > 0.0f && __float_as_uint(v[j]) == least;
+            const unsigned eqs = __ballot_sync(0xffffffffu, eq);
+            const int pos = n + __popc(eqs & below);
+            if (eq && pos < k - n_above) s_col[1][pos] = c0 + j * 32 + lane;
+            n += __popc(eqs);
+          }
+        }
+      }
+      __syncthreads();
+      if (i < k) {
+        const unsigned u = s_key[0][i];
+        const int col = s_col[0][i];
+        if (u > least) {
+          int place = 0;
+          for (int j = 0; j < k; ++j) place += s_key[0][j] > u || (s_key[0][j] == u && s_col[0][j] < col);
+          idx[place] = col;
+          val[place] = gate != nullptr ? __uint_as_float(u) / gate[col] : __uint_as_float(u);
+        }
+        if (i < k - n_above) {
+          const int c = least != 0u ? s_col[1][i] : -1;
+          idx[n_above + i] = c;
+          val[n_above + i] = c < 0 ? 0.0f : gate != nullptr ? __uint_as_float(least) / gate[c] : __uint_as_float(least);
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+int row_select_max_k() { return RS_MAX_K; }
+
+int row_select_launch(const __nv_bfloat16* H16, const float* H32, long long ldh, const float* maxima, long long ld_maxima, int M, int N, int k,
+                      const float* gate, int sorted, int* out_idx, float* out_val, cudaStream_t stream) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(H16) | reinterpret_cast<uintptr_t>(H32) | reinterpret_cast<uintptr_t>(gate);
+  if ((H16 != nullptr) == (H32 != nullptr) || k < 1 || k > RS_MAX_K || N % 8 != 0 || N > 65535 * 32 || ldh % 8 != 0 || at % 16 != 0) return (int)cudaErrorInvalidValue;
+  if (M <= 0) return 0;
+  const int blocks = (M + RS_WARPS - 1) / RS_WARPS;
+  if (H16 != nullptr) row_select_kernel<__nv_bfloat16><<<blocks, RT_THREADS, 0, stream>>>(H16, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
+  else row_select_kernel<float><<<blocks, RT_THREADS, 0, stream>>>(H32, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
+  return (int)cudaGetLastError();
 }
 
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,

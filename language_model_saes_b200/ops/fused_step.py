@@ -373,6 +373,9 @@ class FusedTopKSAEStep:
         fused_topk = k <= 64 and x.is_cuda
         use_comm = self.tp > 1 and self.comm is not None and x.shape[0] == self.comm.B and k <= self.comm.k_max
         if fused_topk:
+            if self.tp == 1 and not chunked and (out := K.stored_topk(x, self.WE_bf16, self.bE, gate, k)) is not None:
+                self._mark("encoder_gemm_topk")
+                return out
             if chunked:
                 cv, ci = self._candidates_chunked(x, k, gate)
             else:

@@ -197,11 +197,11 @@ def encoder_hidden(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
 
 
 def encoder_hidden_maxima(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None = None, max_gate: torch.Tensor | None = None,
-                          pair: bool | None = None) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
-    """``encoder_hidden`` on a GPU with the maxima of every 32 columns of what it stores, times ``max_gate`` when that is given: fp32
-    ``[M, 8 per 256 columns]``, NaN where a value is NaN. Selections look at those first."""
+                          pair: bool | None = None, dtype: torch.dtype = torch.bfloat16) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
+    """``encoder_hidden`` on a GPU (in ``dtype``: bf16, or fp32 without a gate) with the maxima of every 32 columns of what it stores, times
+    ``max_gate`` when that is given: fp32 ``[M, 8 per 256 columns]``, NaN where a value is NaN. Selections look at those first."""
     M, N = x.shape[0], w.shape[0]
-    H = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    H = torch.empty(M, N, dtype=dtype, device=x.device)
     maxima = torch.empty(M, -(-N // 256) * 8, dtype=torch.float32, device=x.device)
     units, S = _deal(M, N, pair, None)
     _ext().encoder_gemm(x, w, bias, gate, 1 | _pair_bit(pair), 0, S, H, None, None, status_buffer(x.device), 0, False, units, maxima, max_gate)
@@ -214,11 +214,44 @@ def maxima_pay(N: int, k: int) -> bool:
     return N >= 128 * k and k <= 512
 
 
+def row_select(H: torch.Tensor, maxima: torch.Tensor, k: int, gate: torch.Tensor | None = None, sort: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
+    """Row top-k (k <= 128) of pre-activations and the gated maxima that ``encoder_hidden_maxima`` left, of equal values the first
+    columns; ``sort``: by value."""
+    out_idx = torch.empty(H.shape[0], k, dtype=torch.int32, device=H.device)
+    out_val = torch.empty(H.shape[0], k, dtype=torch.float32, device=H.device)
+    _ext().row_select(H, maxima, k, gate, sort, out_idx, out_val)
+    return out_idx, out_val
+
+
+STORED_BYTES = 512 << 20  # of pre-activations in fp32
+
+
+def storing_pays(M: int, N: int, K: int, k: int) -> bool:
+    """Whether a top-k of up to 64 takes less time from pre-activations stored in fp32 and their maxima than in the GEMM's epilogue. It does
+    where rows are few: a CTA's sweep of columns is short then, most of its values still enter the running selection, and the MMAs do not
+    cover that (us, epilogue and stored; M x N x K, k: 1024 x 16384 x 512, 32: 67, 50; 1024 x 16384 x 1024, 64: 103, 64; 512 x 8192 x 768,
+    32: 56, 34; 1000 x 24584 x 2304, 50: 151, 120; 2048 x 24576 x 768, 50: 134, 116). With more or longer rows or many more columns it does
+    not (2048 x 16384 x 2048, 32: 124, 130; 8192 x 8192 x 512, 16: 130, 146; 640 x 131072 x 4096, 50: 640, 734). The maxima have to bound the
+    k-th value, the matrix is not large, and with few columns the merge of their few candidates is shorter than the selection (a step of
+    512 x 256 x 64, k 8: 73 us, stored 79)."""
+    small = M * K <= 5 << 19 and M * N * K <= 1 << 36 and 4 * M * N <= STORED_BYTES
+    return 1 <= M <= 3072 and 4096 <= N <= 1 << 20 and small and maxima_pay(N, k)
+
+
+def stored_topk(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None, k: int, pair: bool | None = None):
+    """``(idx, act) [M, k]`` of an encoder on a GPU from pre-activations stored in fp32, by value; None where ``storing_pays`` says no."""
+    M, N = x.shape[0], w.shape[0]
+    if not storing_pays(M, N, x.shape[1], k) or N % 8 != 0 or (gate is not None and gate.data_ptr() % 16 != 0):
+        return None
+    H, maxima = encoder_hidden_maxima(x, w, bias, max_gate=gate, pair=pair, dtype=torch.float32)
+    return row_select(H, maxima, k, gate, sort=True)
+
+
 def hidden_topk(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None, k: int, pair: bool | None = None):
     """Stored pre-activations and their row top-k on a GPU: ``(H, idx, act)``."""
     if maxima_pay(w.shape[0], k):
         H, maxima = encoder_hidden_maxima(x, w, bias, max_gate=gate, pair=pair)
-        return H, *row_topk(H, k, gate, maxima=maxima)
+        return H, *(row_select(H, maxima, k, gate) if x.shape[0] >= 1024 and _ext().row_select_fits(H, k, gate) else row_topk(H, k, gate, maxima=maxima))
     H = encoder_hidden(x, w, bias, pair)
     return H, *row_topk(H, k, gate)
 
@@ -322,13 +355,15 @@ def encoder_topk(
     """Sparse codes of a TopK encoder: (idx [M,k], act [M,k]) (+ hidden_pre bf16 when asked).
 
     ``k <= 64`` uses the GEMM's fused top-k epilogue (the dense pre-activations are never written unless
-    ``return_hidden``); larger k materialises H and selects with the radix row-top-k kernel.
+    ``return_hidden``), or ``stored_topk`` where that is faster; larger k materialises H and selects with the radix row-top-k kernel.
     """
     if not x.is_cuda:
         h = ref_hidden(x, w, bias)
         idx, act = ref_topk_codes(h, k, gate)
         return (idx, act, h.to(torch.bfloat16)) if return_hidden else (idx, act)
     if k <= 64:
+        if not return_hidden and (out := stored_topk(x, w, bias, gate, k, pair)) is not None:
+            return out
         H = torch.empty(x.shape[0], w.shape[0], dtype=torch.bfloat16, device=x.device) if return_hidden else None
         cv, ci, _ = encoder_topk_candidates(x, w, bias, gate, k, H=H, pair=pair)
         idx, act = topk_merge(cv, ci, k, gate)
