@@ -223,19 +223,20 @@ def row_select(H: torch.Tensor, maxima: torch.Tensor, k: int, gate: torch.Tensor
     return out_idx, out_val
 
 
-STORED_BYTES = 512 << 20  # of pre-activations in fp32
+STORED_BYTES = 320 << 20  # of pre-activations in fp32
 
 
 def storing_pays(M: int, N: int, K: int, k: int) -> bool:
     """Whether a top-k of up to 64 takes less time from pre-activations stored in fp32 and their maxima than in the GEMM's epilogue. It does
-    where rows are few: a CTA's sweep of columns is short then, most of its values still enter the running selection, and the MMAs do not
-    cover that (us, epilogue and stored; M x N x K, k: 1024 x 16384 x 512, 32: 67, 50; 1024 x 16384 x 1024, 64: 103, 64; 512 x 8192 x 768,
-    32: 56, 34; 1000 x 24584 x 2304, 50: 151, 120; 2048 x 24576 x 768, 50: 134, 116). With more or longer rows or many more columns it does
-    not (2048 x 16384 x 2048, 32: 124, 130; 8192 x 8192 x 512, 16: 130, 146; 640 x 131072 x 4096, 50: 640, 734). The maxima have to bound the
-    k-th value, the matrix is not large, and with few columns the merge of their few candidates is shorter than the selection (a step of
-    512 x 256 x 64, k 8: 73 us, stored 79)."""
-    small = M * K <= 5 << 19 and M * N * K <= 1 << 36 and 4 * M * N <= STORED_BYTES
-    return 1 <= M <= 3072 and 4096 <= N <= 1 << 20 and small and maxima_pay(N, k)
+    where rows are few: a CTA's sweep of columns is short then, most of its values still enter the running selection (the more the larger k
+    is), and the MMAs do not cover that (us, epilogue and stored; M x N x K, k: 512 x 8192 x 768, 8: 48, 30; 1024 x 16384 x 512, 32: 67, 50;
+    1024 x 16384 x 1024, 64: 103, 64; 2048 x 24576 x 768, 50: 134, 116; 4096 x 8192 x 1024, 64: 149, 110; at the lines 1024 x 24576 x 2048, 32:
+    106, 105; 640 x 131072 x 768, 50: 202, 187). With more or longer rows or more columns it does not (2048 x 16384 x 2048, 32: 124, 130;
+    3328 x 16384 x 1024, 16: 124, 134; 3001 x 13000 x 1160, 37: 126, 132; 4096 x 32768 x 512, 32: 226, 239; 640 x 131072 x 4096, 50: 640, 734).
+    The maxima have to bound the k-th value, and with few columns the merge of their few candidates is shorter than the selection (a step
+    of 512 x 256 x 64, k 8: 73 us, stored 79)."""
+    small = M * K <= k << 16 and M * N * K <= 1 << 36 and 4 * M * N <= STORED_BYTES
+    return 1 <= M <= 4096 and 4096 <= N <= 1 << 20 and small and maxima_pay(N, k)
 
 
 def stored_topk(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gate: torch.Tensor | None, k: int, pair: bool | None = None):

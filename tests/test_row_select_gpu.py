@@ -50,8 +50,8 @@ def test_row_select(M, N, k, data, dtype, gated):
         assert bool(((got - want).abs() <= 6 * 2.0**-24 * want)[finite].all())
 
 
-# the line at 4096 columns; that of M * K; rows and columns with remainders; a gate off its alignment
-@pytest.mark.parametrize("M,N,d,k", [(1, 4088, 64, 1), (1, 4096, 64, 32), (3, 4104, 64, 7), (2560, 4096, 1024, 32), (2561, 4104, 1024, 32), (1000, 8200, 72, 64)])
+# the line at 4096 columns; that of M * K; that of 4096 rows; rows and columns with remainders; a gate off its alignment
+@pytest.mark.parametrize("M,N,d,k", [(1, 4088, 64, 1), (1, 4096, 64, 32), (3, 4104, 64, 7), (2048, 4096, 1024, 32), (2049, 4104, 1024, 32), (4096, 8200, 64, 64), (4097, 8192, 64, 8)])
 @pytest.mark.parametrize("form", ["plain", "gate", "gate off by one", "no bias", "ties"])
 def test_stored_route_is_the_epilogues(M, N, d, k, form):
     g = torch.Generator(device=DEV).manual_seed(M)
