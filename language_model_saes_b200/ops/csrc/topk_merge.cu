@@ -13,7 +13,7 @@
 
 namespace lmsae {
 
-constexpr int MERGE_WARPS = 4;
+constexpr int MERGE_WARPS = 4;  // (fewer where their candidates do not fit)
 
 // One warp per row. Positive floats order like their bit patterns, so the k-th largest candidate is found by a
 // descent over the 31 value bits instead of ranking every candidate against every other one: two bits per step, the three counts of a
@@ -51,7 +51,8 @@ topk_merge_kernel(const float* cand_val, const int* cand_idx, int M, int C, int 
   bool inputs_ok = true;
   if (comm.mode == kMergeWait) inputs_ok = wait_all_sources(comm.pt, kPhaseCand, comm.epoch, comm.status);
 
-  for (int row = blockIdx.x * MERGE_WARPS + warp; row < M; row += gridDim.x * MERGE_WARPS) {
+  const int warps = blockDim.x >> 5;
+  for (int row = blockIdx.x * warps + warp; row < M; row += gridDim.x * warps) {
     int n_own = 0;
     if (inputs_ok) {
       const float* cv = cand_val + (size_t)row * C;
@@ -174,15 +175,19 @@ int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, 
                       int own_lo, int own_hi, int emit_gated, int* out_idx, float* out_val, const MergeComm& comm,
                       cudaStream_t stream) {
   const int per = C <= 128 ? 4 : C <= 256 ? 8 : C <= 512 ? 16 : C <= 768 ? 24 : 0;
-  const size_t smem = (size_t)MERGE_WARPS * (4 * (size_t)k + (per == 0 ? 2 * (size_t)C : 0)) * 4;
+  // Up to 128 rows have 148 ranges, and 64 candidates of each are 74 KB a row: two rows a CTA.
+  const size_t warp_bytes = (4 * (size_t)k + (per == 0 ? 2 * (size_t)C : 0)) * 4;
+  int warps = MERGE_WARPS;
+  while (warps > 1 && warps * warp_bytes > 200 * 1024) warps /= 2;
+  const size_t smem = warps * warp_bytes;
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   if (comm.mode != kMergePush && (out_idx == nullptr || out_val == nullptr)) return (int)cudaErrorInvalidValue;
   auto kern = per == 4 ? topk_merge_kernel<4> : per == 8 ? topk_merge_kernel<8> : per == 16 ? topk_merge_kernel<16> : per == 24 ? topk_merge_kernel<24> : topk_merge_kernel<0>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  int blocks = (M + MERGE_WARPS - 1) / MERGE_WARPS;
+  int blocks = (M + warps - 1) / warps;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  kern<<<blocks, MERGE_WARPS * 32, smem, stream>>>(cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
+  kern<<<blocks, warps * 32, smem, stream>>>(cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
                                                   emit_gated, out_idx, out_val, comm);
   return (int)cudaGetLastError();
 }

@@ -58,6 +58,18 @@ def test_selected_values_are_exact(M, N, splits, k, kind):
     _check(idx, val, x, w, b, gate, k)
 
 
+# few rows are dealt to as many ranges as there are SMs: 98 x 64 candidates of four rows fit a CTA of the merge, 99 x 64 do not
+@pytest.mark.parametrize("M,N", [(1, 98 * 256), (5, 99 * 256), (128, 148 * 256), (127, 150 * 256 + 40)])
+@pytest.mark.parametrize("k", [32, 33, 64])
+@pytest.mark.parametrize("kind", ["normal", "few", "equal"])
+def test_few_rows_of_a_long_dictionary(M, N, k, kind):
+    x, w, b, gate = _data(M, N, 72, kind, seed=N + k)
+    idx, val, H = K.encoder_topk(x.to(DEV), w.to(DEV), b.to(DEV), gate.to(DEV), k, return_hidden=True)
+    K.check_status(torch.device(DEV))
+    _check(idx, val, x, w, b, gate, k)
+    assert torch.equal(H.cpu(), (x.float() @ w.float().t() + b).to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("k", [20, 50, 64])
 @pytest.mark.parametrize("compact", [False, True])
 @pytest.mark.parametrize("kind", ["normal", "equal"])
