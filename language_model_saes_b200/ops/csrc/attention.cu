@@ -285,11 +285,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     bool ok = true;
     uint32_t g0 = 0;
     int t = 0;
-    for (int w = (int)blockIdx.x; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
+    int w = (int)blockIdx.x;
+    int owed = 0;  // barriers of the row quarter that are left in this tile
+    for (; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
       int qblk, head, dv0, batch;
       decode_tile(w, qblk, head, dv0, batch);
       const int q0 = qblk * ATT_BM;
       const int n_kblocks = qblk + 1;
+      owed = n_kblocks + 2;
       const int qpos = q0 + row;
       const bool row_ok = qpos < p.seq;
       const uint32_t tmem_o = tmem_base + 2 * ATT_BN + (uint32_t)((t & 1) * DV);
@@ -327,6 +330,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         float* xr = xch + (u * 4) * ATT_BM + row;
         xr[cq * ATT_BM] = m_raw;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
+        --owed;
         const float m_blk = fmaxf(fmaxf(xr[0], xr[ATT_BM]), fmaxf(xr[2 * ATT_BM], xr[3 * ATT_BM])) * sc;  // sc > 0
         float alpha = 1.0f;
         bool rescale = false;
@@ -399,6 +403,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       float* xl = xch + (int)((g_last + 1) & 1) * 4 * ATT_BM + row;
       xl[cq * ATT_BM] = l_run;
       asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
+      --owed;
       const float l_tot = (xl[0] + xl[ATT_BM]) + (xl[2 * ATT_BM] + xl[3 * ATT_BM]);
       const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
       if (o_active) {
@@ -429,11 +434,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // keep the four warps of a row quarter together across tiles: the sum exchange above and the next maximum exchange
       // use the same slots
       asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
+      --owed;
       g0 += (uint32_t)n_kblocks;
     }
     if (!ok) {
       report_status(p.status, kTimeoutTmemFull, row);
       *abort_flag = 1;
+      // the other warps of the quarter may have passed the wait that this one gave up at: it keeps them company at their barriers, which
+      // have no limit, until they give up or are through (every warp comes to as many in a tile)
+      __syncwarp();
+      for (; w < n_tiles; w += (int)gridDim.x) {
+        if (owed < 0) owed = n_qblocks - w / per_qblock + 2;  // (n_kblocks of this tile)
+        for (; owed > 0; --owed) asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
+        owed = -1;
+      }
     }
   }
 
