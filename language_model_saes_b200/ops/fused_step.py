@@ -632,7 +632,7 @@ class FusedTopKSAEStep:
         self.groups.build(idx)
         self.main_counts = self.groups.counts[: self.F].clone()  # fire counts of the real codes (for metrics)
         fired = self.main_counts
-        n_valid = torch.tensor(B, device=x.device) if row_weight is None else (row_weight > 0).sum()
+        n_valid = torch.full((), B, device=x.device) if row_weight is None else (row_weight > 0).sum()  # (a copy from the host would wait)
         if self.dp > 1:  # a feature is alive when it fired on any replica; the counters advance by the global token count
             fired, n_valid = fired.clone(), n_valid.clone()
             dist.all_reduce(fired, group=self.dp_group)

@@ -164,6 +164,28 @@ def test_fused_auxk_matches_autograd(k_aux):
     assert torch.nn.functional.cosine_similarity(moved_ref, moved_fus, dim=0) > 0.9
 
 
+@pytest.mark.parametrize("act", ["topk", "batchtopk"])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_auxk_step_does_not_wait_for_the_gpu(act, weighted):
+    from language_model_saes_b200.ops.fused_step import AuxK
+
+    d, B, k = 256, 512, 16
+    sae = _model(d=d, k=k)
+    sae.cfg.act_fn = act
+    sae.activation_function = sae.activation_function_factory(None)
+    engine, aux = FusedTopKSAEStep(sae), AuxK(sae.cfg.d_sae, 96, 1 / 32, 1000, "cuda")
+    w = torch.ones(B, device="cuda") if weighted else None
+    data = _data(5, B, d)
+    for x in data[:4]:
+        engine.step(x, x, k, 1e-3, row_weight=w, aux=aux)
+    torch.cuda.synchronize()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        engine.step(data[4], data[4], k, 1e-3, row_weight=w, aux=aux)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+
+
 @pytest.mark.parametrize("gate,k", [(True, 16), (False, 8)])
 def test_fused_batchtopk_matches_autograd(gate, k):
     """Batch-level top-k on the fused path (radix-select threshold + threshold compaction) against the generic model."""
