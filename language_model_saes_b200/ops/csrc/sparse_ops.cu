@@ -864,6 +864,7 @@ int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cuda
 // As five launches (fill, column sums by atomics, Adam; a fill and a division for the loss): 4096 rows of 768: 7.7 + 2.8 + 5 us, 4096
 // rows of 4096: 14.6 + 2.8 + 5; here 9.6 and 14.8. In steps of small dictionaries the four launches less count more than that (512 rows
 // of 64: a step of 88 us takes 75).
+constexpr int kSerialPartials = 64;  // up to so many partial sums are added up one after the other
 __global__ void __launch_bounds__(256)
 colsum_adam_kernel(const ColsumAdamParams p) {
   __shared__ float s_sum[8][256];
@@ -934,9 +935,27 @@ colsum_adam_kernel(const ColsumAdamParams p) {
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    s = 0.0f;
+    if (gridDim.y <= kSerialPartials) {
+      s = 0.0f;
 #pragma unroll 8
-    for (int b = 0; b < (int)gridDim.y; ++b) s += __ldcg(part + b * 256 + threadIdx.x);
+      for (int b = 0; b < (int)gridDim.y; ++b) s += __ldcg(part + b * 256 + threadIdx.x);
+    } else {  // every warp an eighth of them, eight columns a lane
+      float sum[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum[i] = 0.0f;
+#pragma unroll 4
+      for (int b = warp; b < (int)gridDim.y; b += 8) {
+        const float4 u0 = __ldcg(reinterpret_cast<const float4*>(part + b * 256) + lane), u1 = __ldcg(reinterpret_cast<const float4*>(part + b * 256) + 32 + lane);
+        sum[0] += u0.x; sum[1] += u0.y; sum[2] += u0.z; sum[3] += u0.w;
+        sum[4] += u1.x; sum[5] += u1.y; sum[6] += u1.z; sum[7] += u1.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s_sum[warp][(i >> 2) * 128 + lane * 4 + (i & 3)] = sum[i];
+      __syncthreads();
+      s = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += s_sum[w][threadIdx.x];
+    }
     if (threadIdx.x == 0) p.counters[blockIdx.x] = 0;  // for the next launch
   }
   if (c >= g.d || (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0)) return;  // see sparse_grad_adam_kernel
@@ -1002,12 +1021,14 @@ int mask_colsum_launch(__nv_bfloat16* g, const __nv_bfloat16* mask, long long ld
 }
 
 // Row blocks for a launch of `col_blocks` blocks of 256 columns: eight CTAs per SM (2048 rows of 17152: 28 us with four, 22 with eight), at least
-// 32 rows each, and no more than 64 partial sums to add up (4096 rows of 768: 9.6 us with 64, 11.0 with 128).
+// 32 rows each, and no more than 64 partial sums to add up (4096 rows of 768: 9.6 us with 64, 11.0 with 128) while that leaves a block 64
+// rows or less; with more rows a block of 64 to itself, up to 512 blocks, whose sums all warps add up (65536 rows of 64: 74 us with 64 blocks, 27 so;
+// 262144 of 128: 258 and 45; 65536 of 768: 87 and 45).
 int colsum_adam_row_blocks(int col_blocks, int rows) {
   int n = 1184 / (col_blocks > 0 ? col_blocks : 1);
-  const int most = (rows + 31) / 32;
+  const int most = rows <= 64 * kSerialPartials ? (rows + 31) / 32 : (rows + 63) / 64, cap = rows <= 64 * kSerialPartials ? kSerialPartials : 512;
   n = n < most ? n : most;
-  return n < 1 ? 1 : (n > 64 ? 64 : n);
+  return n < 1 ? 1 : (n > cap ? cap : n);
 }
 
 int colsum_adam_launch(ColsumAdamParams p, int col_blocks, cudaStream_t stream) {

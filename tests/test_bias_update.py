@@ -19,9 +19,10 @@ def _ref(p, m, v, g, step):
     return p, m, v
 
 
-# one row, a row block and one more row, no multiple of anything; 8 columns, a column block and a bit, several matrices, 18 of them
+# one row, a row block and one more row, no multiple of anything; 8 columns, a column block and a bit, several matrices, 18 of them;
+# the most rows whose partial sums are added up one by one, one more, and as many row blocks as there can be
 @pytest.mark.parametrize("dev", DEVICES)
-@pytest.mark.parametrize("rows,widths", [(1, [8]), (64, [256]), (65, [264, 8]), (3001, [768, 40, 2312]), (700, [64] * 18), (40, [12])])
+@pytest.mark.parametrize("rows,widths", [(1, [8]), (64, [256]), (65, [264, 8]), (3001, [768, 40, 2312]), (700, [64] * 18), (40, [12]), (4096, [8]), (4097, [264]), (33000, [72, 8])])
 def test_bias_update(dev, rows, widths):
     mats = [_rand(dev, rows, w, seed=i).to(torch.bfloat16) for i, w in enumerate(widths)]
     params = [_rand(dev, w, seed=50 + i) for i, w in enumerate(widths)]
@@ -45,3 +46,24 @@ def test_bias_update(dev, rows, widths):
         sure = a.double().sum(0).abs() > 8 * err
         assert bool(((m.double() - wm).abs() <= 1e-5 * wm.abs() + err).all())
         assert torch.allclose(p.double()[sure], wp[sure], rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.gpu
+def test_many_rows_of_few_columns_take_no_longer_than_separate_launches():
+    rows, d = 262144, 128
+    a, p, m, v, loss = _rand("cuda", rows, d).to(torch.bfloat16), *(torch.zeros(d, device="cuda") for _ in range(3)), torch.zeros(1, device="cuda")
+    update, best = K.BiasUpdate([d], torch.device("cuda")), [1e9, 1e9]
+
+    def separate():
+        loss.zero_()
+        K.adam_flat(p, K.colsum_bf16(a), m, v, *HYPER, 1)
+
+    for _ in range(8):
+        for i, fn in enumerate((separate, lambda: update([a], [p], [(m, v)], *HYPER, 1, loss))):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            fn()
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+    assert best[1] < 1.5 * best[0], best  # (with 64 row blocks: four times as long)
