@@ -223,8 +223,8 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
 }
 
 // C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu). With na [M] (written: the rows' norms) C is bf16 and
-// receives the lower ends that topk_estimate takes, made with bias [N] and gate [N] (both optional); top: int32 [2], zeroed, goes with
-// them. status: int32 [4], zeroed, of this call alone: a wait in the product that runs out is recorded there, and everything is done on the
+// receives the lower ends that topk_estimate takes, made with bias [N] and gate [N] (both optional); top: int32 [4 + (N + 1) / 2], the first four
+// zeroed, on a 16-byte boundary, goes with them (the largest width of a column, whether a gate is 0 or NaN, 0, 0, every column's width in bf16). status: int32 [4], zeroed, of this call alone: a wait in the product that runs out is recorded there, and everything is done on the
 // fp32 pipes then (lower ends: by topk_estimate). tensor_cores = false leaves the product out (as if it had given up).
 void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
                const c10::optional<Tensor>& top, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
@@ -242,7 +242,7 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
   if (ends) {
     CHECK_T(*na, torch::kFloat32);
     CHECK_T(*top, torch::kInt32);
-    TORCH_CHECK(na->numel() == M && top->numel() == 2);
+    TORCH_CHECK(na->numel() == M && top->numel() == 4 + (N + 1) / 2 && reinterpret_cast<uintptr_t>(top->data_ptr()) % 16 == 0);
   }
   for (const auto* t : {&bias, &gate}) {
     if (t->has_value()) { CHECK_T(**t, torch::kFloat32); TORCH_CHECK((*t)->numel() == N); }
@@ -261,7 +261,7 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
   int* fa = flags.data_ptr<int>();
   int* fb = fa + 1 + M;
   check_cuda(lmsae::split_bf16_launch(A.data_ptr<float>(), (int)M, (int)K, (int)kp, (int)parts, reinterpret_cast<__nv_bfloat16*>(As.data_ptr()), fa,
-                                      opt_ptr<float>(na), nullptr, nullptr, nullptr, stream), "split");
+                                      opt_ptr<float>(na), nullptr, nullptr, nullptr, nullptr, stream), "split");
   const CUtensorMap ta = make_bf16_tile_map(As.data_ptr(), M, parts * kp, 128);
   for (int64_t n0 = 0; n0 < N; n0 += step) {
     const int64_t n = std::min(step, N - n0);
@@ -270,6 +270,7 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
     const float* gate_n = gate.has_value() ? gate->data_ptr<float>() + n0 : nullptr;
     float* nb_n = ends ? nb.data_ptr<float>() + n0 : nullptr;
     check_cuda(lmsae::split_bf16_launch(Bn, (int)n, (int)K, (int)kp, (int)parts, reinterpret_cast<__nv_bfloat16*>(Bs.data_ptr()), fb, nb_n,
+                                        ends ? reinterpret_cast<uint16_t*>(top->data_ptr<int>() + 4) + n0 : nullptr,
                                         ends ? reinterpret_cast<uint32_t*>(top->data_ptr<int>()) : nullptr, bias_n, gate_n, stream), "split");
     const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), n, parts * kp, 128);
     if (ends)
@@ -297,7 +298,7 @@ void topk_dense(const Tensor& h, const c10::optional<Tensor>& bias, const c10::o
              "topk_dense launch");
 }
 
-// The same with lower ends lo (bf16 [B, F]), xn [B], top [2] and status [4] as fp32_gemm gave them for x [B, K], W [F, K]; h: fp32 [B, F], which
+// The same with lower ends lo (bf16 [B, F]), xn [B], top and status [4] as fp32_gemm gave them for x [B, K], W [F, K]; h: fp32 [B, F], which
 // may share memory with lo, receives the products of rows that are left over; todo: int32 [1 + B], todo[0] zeroed
 void topk_estimate(const Tensor& lo, const Tensor& h, const Tensor& x, const Tensor& W, const Tensor& xn, const Tensor& top, const c10::optional<Tensor>& bias,
                    const c10::optional<Tensor>& norm, int64_t k, const Tensor& status, const Tensor& todo, const Tensor& out) {
@@ -307,7 +308,8 @@ void topk_estimate(const Tensor& lo, const Tensor& h, const Tensor& x, const Ten
   TORCH_CHECK(h.dim() == 2 && out.sizes() == h.sizes() && lo.sizes() == h.sizes() && h.size(0) < INT_MAX && h.size(1) <= INT_MAX, "lo, h and out must be [B, F]");
   TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.size(0) == h.size(0) && W.size(0) == h.size(1) && W.size(1) == x.size(1) &&
               x.size(1) <= lmsae::kEstimateMaxK, "x [B, K] and W [F, K]");
-  TORCH_CHECK(xn.numel() == h.size(0) && top.numel() == 2 && status.numel() == 4 && todo.numel() == h.size(0) + 1);
+  TORCH_CHECK(xn.numel() == h.size(0) && top.numel() == 4 + (h.size(1) + 1) / 2 && reinterpret_cast<uintptr_t>(top.data_ptr()) % 16 == 0 && status.numel() == 4 &&
+              todo.numel() == h.size(0) + 1);
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == h.size(1)); }
   if (norm.has_value()) { CHECK_T(*norm, torch::kFloat32); TORCH_CHECK(norm->numel() == h.size(1)); }
   const c10::cuda::CUDAGuard guard(h.device());

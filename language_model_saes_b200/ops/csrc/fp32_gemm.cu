@@ -51,12 +51,13 @@ template <int TERMS>
 __device__ __forceinline__ int part_b(int t) { return TERMS == 6 ? (0x021010 >> (4 * (5 - t))) & 15 : t == 1; }
 
 // dst [rows][PARTS][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
-// then flags[0] != 0. For lower ends, all optional: norm[r], at least the row's 2-norm and at most 10 % above it; top[0], at least
-// norm[r] * gate[r] of every row whose norm is finite; top[1] != 0 where a gate is 0 or NaN. The norm is infinite where the row's largest
+// then flags[0] != 0. For lower ends, all optional: norm[r], at least the row's 2-norm and at most 10 % above it; wide[r], at least
+// norm[r] * gate[r]; top[0], at least that of every row whose norm is finite; top[1] != 0 where a gate is 0 or NaN. The norm is infinite where the row's largest
 // magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r] negative, NaN or beyond 2^50: products, (sum + bias) * gate and the
 // parts of what is within stay clear of the ends of the fp32 range (2^30 * 2^30 * K 2^14, doubled, * 2^50 < 2^127).
 struct SplitBounds {
   float* norm;
+  uint16_t* wide;  // bf16
   uint32_t* top;
   const float* bias;
   const float* gate;
@@ -107,7 +108,9 @@ split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_b
         const bool plain = __float_as_uint(gate) < 0x58800000u;  // 2^50 (and no sign)
         const float n = !(fits && plain) ? __uint_as_float(0x7f800000u) : top == 0u ? 0.0f : 1.05f * sqrtf(sq);
         b.norm[r] = n;
-        if (fits && plain) most = fmaxf(most, mul_up(n, gate));
+        const float w = mul_up(n, gate);
+        if (fits && plain) most = fmaxf(most, w);
+        if (b.wide != nullptr) b.wide[r] = fits && plain ? (uint16_t)((__float_as_uint(w) + 0xffffu) >> 16) : (uint16_t)0x7f80u;
         const unsigned gb = __float_as_uint(gate) & 0x7fffffffu;
         if (b.top != nullptr && (gb == 0u || gb > 0x7f800000u)) b.top[1] = 1u;
       }
@@ -403,12 +406,12 @@ marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B,
 
 }  // namespace
 
-int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* top,
+int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint16_t* wide, uint32_t* top,
                       const float* bias, const float* gate, cudaStream_t stream) {
   if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0 || (parts != 2 && parts != 3)) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
   auto kern = parts == 2 ? split_bf16_kernel<2> : split_bf16_kernel<3>;
-  kern<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, top, bias, gate});
+  kern<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, wide, top, bias, gate});
   return (int)cudaGetLastError();
 }
 

@@ -44,7 +44,7 @@ struct EncGemmParams {
 };
 int enc_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const EncGemmParams& p, int mode, cudaStream_t stream);
 int enc_gemm_slots_for_k(int k);
-int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint32_t* top,
+int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv_bfloat16* dst, int* flags, float* norm, uint16_t* wide, uint32_t* top,
                       const float* bias, const float* gate, cudaStream_t stream);
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
                      const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream);

@@ -780,8 +780,11 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 // values, are those of the fp32 sum x . W^T in ascending order of k with one rounding per term.
 //   The k-th largest of the group maxima of the lower ends is reached by at least k columns, and whatever is selected has its upper end
 // at or above it. The upper end is the lower one plus what rounding it down to bf16 may have taken (2^-7 of it) plus twice the bound on the
-// estimate's error, taken at its largest over the columns, so that neither pass reads anything per column but the ends. The columns that
-// may be selected (k and a few) are summed up in order before the exact selection.
+// estimate's error. Where that is small against the k-th end (a 64th) for the column where it is largest, all columns take that one's, and
+// neither pass reads anything per column but the ends; elsewhere (a few features of large norm, long rows, few positive values) the second pass
+// reads every column's own: 4096 x 24576 x 768, k 50, at an 108th 660 us with the largest for all and 664 with each its own, at a 54th 698 and
+// 664, at a 39th 722 and 664. (2048 x 24576 x 4096 with one row of W thirty times the others: 11.3 ms with the largest for all, 1.66 so.)
+// The columns that may be selected (k and a few) are summed up in order before the exact selection.
 //   Columns that the bound says nothing about (their lower end is NaN) are among them; rows with more such columns than there is room for,
 // and all rows where the product gave up, are listed, multiplied in order as a whole (rows_product.cu) and selected from exactly. All
 // decisions are taken on the device.
@@ -806,7 +809,7 @@ struct TopkDenseParams {
   const float* x;           // [B, K] and [N, K]
   const float* W;
   const float* xn;          // [B] 2-norms (fp32_gemm.cu)
-  const uint32_t* top;      // the largest error bound of a column over rel * xn; and whether a norm is 0 or NaN
+  const uint32_t* top;      // the largest error bound of a column over rel * xn; whether a norm is 0 or NaN; from the fifth word on every column's bound, bf16
   const int* status;        // of the product
   int K;
   int* todo;        // ESTIMATE: [1 + B] number of rows left over, and which
@@ -984,16 +987,25 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   };
   if constexpr (ESTIMATE) {
     // (16 units of 2^-24 more for the roundings of the ends; the last term for lower ends that are subnormal)
-    const float room = add_rn(mul_up(mul_up(2.0f * (estimate_rel(p.K) + 1e-6f), p.xn[row]), __uint_as_float(p.top[0])), 1e-37f);
+    const float width = mul_up(2.0f * (estimate_rel(p.K) + 1e-6f), p.xn[row]);
+    const float room = add_rn(mul_up(width, __uint_as_float(p.top[0])), 1e-37f);
     const float thr_f = __uint_as_float(max(thr, 1u));
+    const __nv_bfloat16* widths = below(mul_rn(room, 64.0f), thr_f) ? nullptr : reinterpret_cast<const __nv_bfloat16*>(p.top + 4);
     const bool any_bad = p.top[1] != 0u;
 #pragma unroll 2
     for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
-      float g[8];
+      float g[8], r[8];
       topk_ends_load(p, lo, c, g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r[i] = room;
+      if (widths != nullptr) {
+        topk_ends_load(p, widths, c, r);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = add_rn(mul_up(width, r[i]), 1e-37f);
+      }
       unsigned in = 0u;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) in |= below(add_rn(fma_rn(fabsf(g[i]), 0.0079f, g[i]), room), thr_f) ? 0u : 1u << i;  // (a NaN enters)
+      for (int i = 0; i < 8; ++i) in |= below(add_rn(fma_rn(fabsf(g[i]), 0.0079f, g[i]), r[i]), thr_f) ? 0u : 1u << i;  // (a NaN enters)
       while (in != 0u) {
         const int i = __ffs(in) - 1;
         in &= in - 1u;

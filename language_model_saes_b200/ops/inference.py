@@ -78,8 +78,9 @@ def topk_encode(x: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None, nor
     h, out = (torch.empty(B, F, dtype=torch.float32, device=x.device) for _ in range(2))
     lo = h.view(-1).view(torch.bfloat16)[: B * F].view(B, F)  # (read before anything is written to h)
     xn = torch.empty(B, dtype=torch.float32, device=x.device)
-    words = torch.zeros(4 + 2 + 1 + B, dtype=torch.int32, device=x.device)
-    status, top, todo = words[:4], words[4:6], words[6:]
+    widths = 4 + (F + 1) // 2  # (the columns' widths as bf16 behind four words)
+    words = torch.zeros(4 + widths + 1 + B, dtype=torch.int32, device=x.device)
+    status, top, todo = words[:4], words[4 : 4 + widths], words[4 + widths :]
     bias, norm = (t.contiguous() if t is not None else None for t in (bias, norm))
     K._ext().fp32_gemm(rows, W.detach().t(), lo, status, xn, top, bias, norm, True, PRODUCT_WORKSPACE)
     K._ext().topk_estimate(lo, h, rows, W.detach().t(), xn, top, bias, norm, k, status, todo, out)

@@ -159,6 +159,44 @@ def test_rows_with_few_positive_values_cost_no_more_than_others():
     assert times[1] < 3 * times[0], times  # (summed up as whole rows they took thirty times as long)
 
 
+@pytest.mark.parametrize("share,factor", [(0.0, 1.0), (1 / 16384, 30.0), (1 / 16384, 1000.0), (0.01, 30.0), (0.01, 1000.0), (0.5, 10.0)])
+def test_features_of_large_norm_do_not_widen_the_others_bounds(share, factor):
+    """Codes bit for bit, and at most twice the time that a dictionary of equal norms takes (with one bound for all columns every row was
+    multiplied in order as a whole: thirty times as long)."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    B, F, K_, k = 512, 16384, 4096, 50
+    x = torch.randn(B, K_, device=DEV, generator=g)
+    bias, norm = 0.02 * torch.randn(F, device=DEV, generator=g), torch.rand(F, device=DEV, generator=g) * 0.1 + 1.0
+    even = torch.randn(F, K_, device=DEV, generator=g) / K_**0.5
+    uneven = even.clone()
+    uneven[torch.randperm(F, device=DEV, generator=g)[: int(share * F)]] *= factor
+    best = [1e9, 1e9]
+    for _ in range(6):
+        for i, w in enumerate((even, uneven)):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            out = I.topk_encode(x, w.t(), bias, norm, k)
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+    assert torch.equal(out[:64], I.topk_dense(_in_order(x[:64], uneven), bias, norm, k))
+    assert best[1] < 2 * best[0], best
+
+
+@pytest.mark.parametrize("B,F,K_,k", [(300, 1001, 128, 20), (257, 4104, 72, 64)])
+def test_selection_where_the_product_gave_up(B, F, K_, k):
+    g = torch.Generator(device=DEV).manual_seed(F)
+    x, w = torch.randn(B, K_, device=DEV, generator=g), torch.randn(F, K_, device=DEV, generator=g) / K_**0.5
+    bias, norm = 0.1 * torch.randn(F, device=DEV, generator=g), torch.rand(F, device=DEV, generator=g) + 0.5
+    h, out = torch.randn(B, F, device=DEV, generator=g) * 100, torch.full((B, F), float("nan"), device=DEV)
+    lo = h.view(-1).view(torch.bfloat16)[: B * F].view(B, F)  # what was there before
+    xn, top = torch.full((B,), float("nan"), device=DEV), torch.zeros(4 + (F + 1) // 2, dtype=torch.int32, device=DEV)
+    status, todo = torch.ones(4, dtype=torch.int32, device=DEV), torch.zeros(1 + B, dtype=torch.int32, device=DEV)
+    K._ext().topk_estimate(lo, h, x, w, xn, top, bias, norm, k, status, todo, out)
+    assert todo[0] == B and torch.equal(todo[1:].sort().values, torch.arange(B, dtype=torch.int32, device=DEV))
+    assert torch.equal(out, I.topk_dense(_in_order(x, w), bias, norm, k))
+
+
 def test_a_product_that_gave_up_is_made_good_and_stops_nothing_else(monkeypatch):
     g = torch.Generator(device=DEV).manual_seed(0)
     x, w = torch.randn(300, 128, device=DEV, generator=g), torch.randn(1000, 128, device=DEV, generator=g)
