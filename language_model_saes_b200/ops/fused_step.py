@@ -424,21 +424,23 @@ class FusedTopKSAEStep:
         from . import select_kernels as S
 
         self.join()
-        if x.is_cuda:
+        B = x.shape[0]
+        by_maxima, lists_by_maxima = (x.is_cuda and rule(B, self.WE_bf16.shape[0], k) for rule in (S.maxima_pay_for_threshold, S.maxima_pay_for_lists))
+        if by_maxima or lists_by_maxima:
             G, maxima = K.encoder_hidden_maxima(x, self.WE_bf16, self.bE, gate=gate)
         else:
             G, maxima = K.encoder_hidden(x, self.WE_bf16, self.bE, gate=gate), None
         self._mark("encoder_gemm_hidden")
-        B = x.shape[0]
         tp_group = self.tp_group if self.tp > 1 else None
-        # (the previous batch's threshold, lowered by a tenth, as the histogram pass's floor: see positive_thresholds)
-        floor = self._batch_thr * 0.9 if self._batch_thr is not None and G.is_cuda else None
-        thr, n_ties = S.positive_thresholds(G.view(1, 1, -1), k * B, tp_group, return_remaining=True, floor=floor, maxima=maxima)
+        # (the previous batch's threshold, lowered, as the histogram pass's floor: see positive_thresholds, maxima_pay_for_threshold)
+        floor = self._batch_thr * (0.9 if by_maxima else 0.75) if self._batch_thr is not None and G.is_cuda else None
+        thr, n_ties = S.positive_thresholds(G.view(1, 1, -1), k * B, tp_group, return_remaining=True, floor=floor, maxima=maxima if by_maxima else None)
         self._batch_thr = thr
         self._mark("batch_threshold_select")
         # exactly k * B codes: of the entries equal to the (bf16) threshold only as many as the selection still needs
         cap = -(-self.batch_list_factor * k // 8) * 8
-        out = S.threshold_rows_to_sparse(G, thr, gate, n_ties=n_ties, tie_group=tp_group, cap=cap, overflow=self.list_overflow, maxima=maxima)
+        out = S.threshold_rows_to_sparse(G, thr, gate, n_ties=n_ties, tie_group=tp_group, cap=cap, overflow=self.list_overflow,
+                                         maxima=maxima if lists_by_maxima else None)  # fmt: skip
         self._mark("rows_to_code_lists")
         return out
 

@@ -36,6 +36,24 @@ def _kernel_ok(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.numel() > 0
 
 
+def maxima_pay_for_threshold(B: int, N: int, k: int) -> bool:
+    """Whether the floored histogram of a batch-level selection of ``k`` codes per row is faster by the maxima of 32 columns (and a floor of nine
+    tenths of the previous threshold, below which few groups lie) than over the whole matrix (and a floor of three quarters). It is where the
+    matrix is large and few of its groups hold a code (us, by maxima and whole; B x N, k: 2048 x 16384, 64: 83, 87; 1024 x 32768, 128: 85, 87;
+    4096 x 32768, 64: 122, 179; 8192 x 65536, 64: 198, 506; below the lines 2048 x 16384, 128: 95, 89; 2048 x 8192, 32: 81, 71; 512 x 16384, 32:
+    75, 62; 4096 x 4096, 64: 97, 71). When the threshold falls by more than the floor allows for, a second pass reads the whole matrix: 4096 x 32768, 64:
+    222 us."""
+    return N >= 256 * k and B * N >= 1 << 25
+
+
+def maxima_pay_for_lists(B: int, N: int, k: int) -> bool:
+    """Whether the lists of a batch-level selection are made faster by the maxima of 32 columns, a warp per row and a group per code, than by CTAs
+    that read whole rows. It is where many rows share the time of a warp's row (us, by maxima and whole; 4096 x 16384, 32: 157, 200; 4096 x 32768,
+    64: 247, 308; 2048 x 65536, 32: 210, 226; 8192 x 65536, 64: 380, 818; 4096 x 131072, 128: 648, 749; beyond the lines 2048 x 16384, 16: 120, 126; 4096 x
+    16384, 64: 208, 216; 1024 x 65536, 16: 159, 146; 1024 x 65536, 64: 302, 169; 4096 x 32768, 128: 384, 339; 8192 x 8192, 128: 280, 241)."""
+    return N >= 128 * k and ((B >= 64 * k and B * B * N >= k << 33) or (B >= 32 * k and B * N >= 1 << 29))
+
+
 @torch.no_grad()
 def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: bool = False, floor: torch.Tensor | None = None,
                         maxima: torch.Tensor | None = None):  # fmt: skip

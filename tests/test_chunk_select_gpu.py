@@ -82,3 +82,35 @@ def test_batch_level_selection_with_maxima(B, N, k, data):
         want = S.threshold_rows_to_sparse(x, thr, div, n_ties=n_ties, cap=cap, overflow=counts[0])
         got = S.threshold_rows_to_sparse(x, thr, div, n_ties=n_ties, cap=cap, overflow=counts[1], maxima=maxima)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(nan=7.0), want[1].nan_to_num(nan=7.0)) and torch.equal(*counts)
+
+
+# on both sides of the lines of both rules
+@pytest.mark.parametrize("B,N,k", [(512, 65536, 64), (1024, 16384, 64), (1024, 65536, 16), (4096, 8192, 128), (4096, 32768, 64), (8192, 16384, 32)])
+def test_maxima_are_used_where_they_pay(B, N, k):
+    g = torch.Generator(device=DEV).manual_seed(0)
+    x, w = torch.randn(B, 64, device=DEV, generator=g).to(torch.bfloat16), torch.randn(N, 64, device=DEV, generator=g).to(torch.bfloat16)
+    H, maxima = K.encoder_hidden_maxima(x, w, None)
+    thr, n_ties = S.positive_thresholds(H.view(1, 1, -1), k * B, None, return_remaining=True)
+    overflow = torch.zeros(1, dtype=torch.int64, device=DEV)
+
+    def threshold(by_maxima):
+        return S.positive_thresholds(H.view(1, 1, -1), k * B, None, return_remaining=True, floor=thr * (0.9 if by_maxima else 0.75), maxima=maxima if by_maxima else None)
+
+    def lists(by_maxima):
+        return S.threshold_rows_to_sparse(H, thr, None, n_ties=n_ties, cap=8 * k, overflow=overflow, maxima=maxima if by_maxima else None)
+
+    def best(fn, by_maxima):
+        times = []
+        for _ in range(8):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(200000)  # (so that the launches wait for the GPU and not the other way round)
+            start.record()
+            fn(by_maxima)
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+
+    for fn, rule in ((threshold, S.maxima_pay_for_threshold), (lists, S.maxima_pay_for_lists)):
+        taken = rule(B, N, k)
+        assert best(fn, taken) < 1.3 * best(fn, not taken), (fn.__name__, taken)
