@@ -47,21 +47,29 @@ __device__ __forceinline__ void load8f(const float* p, float (&v)[8]) {
 }
 
 // A CTA per token and tensor (the position is found once; with one flat index per thread three 64-bit divisions each took as long as the
-// memory: 2 x 2048 x 64 x 64: 19 -> 15 us).
-template <bool ADJACENT>
+// memory: 2 x 2048 x 64 x 64: 19 -> 15 us), or, MANY, per as many tokens as its threads can take where the heads of one leave half of
+// them idle or more (65536 tokens of one head of 64: 82 -> 18 us, of two: 80 -> 28, of four of 128: 102 -> 86; 16384 of eight of 64: 33 -> 27).
+template <bool ADJACENT, bool MANY>
 __global__ void __launch_bounds__(256)
 rotary_pair_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat16* __restrict__ xb, __nv_bfloat16* __restrict__ oa,
                    __nv_bfloat16* __restrict__ ob, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                   int seq, int heads, int width, int rd, float sin_sign) {
-  const unsigned per_head = (unsigned)width / 8;
+                   unsigned tokens, unsigned tokens_per_cta, int seq, int heads, int width, int rd, float sin_sign) {
+  const unsigned per_head = (unsigned)width / 8, per_token = (unsigned)heads * per_head;
   const __nv_bfloat16* x = blockIdx.y == 0 ? xa : xb;
   __nv_bfloat16* o = blockIdx.y == 0 ? oa : ob;
-  const int pos = (int)(blockIdx.x % (unsigned)seq);
-  const long long token = (long long)blockIdx.x * heads * width;
-  for (unsigned j = threadIdx.x; j < (unsigned)heads * per_head; j += blockDim.x) {
+  unsigned token = blockIdx.x * (MANY ? tokens_per_cta : 1u), j0 = threadIdx.x;
+  if constexpr (MANY) {
+    const unsigned t = j0 / per_token;
+    token += t;
+    if (t >= tokens_per_cta || token >= tokens) return;
+    j0 -= t * per_token;
+  }
+  const int pos = (int)(token % (unsigned)seq);
+  const long long first = (long long)token * heads * width;
+  for (unsigned j = j0; j < per_token; j += MANY ? per_token : blockDim.x) {
     const unsigned head = j / per_head;
     const int c0 = (int)(j - head * per_head) * 8;    // first channel of this thread's block
-    const long long base = token + (long long)head * width;
+    const long long base = first + (long long)head * width;
     float v[8], r[8];
     load8(x + base + c0, v);
     if (c0 >= rd) {  // channels past the rotated ones pass through
@@ -97,11 +105,12 @@ int rotary_pair_launch(const __nv_bfloat16* xa, const __nv_bfloat16* xb, __nv_bf
                        cudaStream_t stream) {
   if (tokens * heads * (width / 8) == 0) return (int)cudaSuccess;
   if (tokens > 2147483647LL || (long long)heads * (width / 8) > 2147483647LL) return (int)cudaErrorInvalidValue;
-  const dim3 grid((unsigned)tokens, 2);
-  if (adjacent)
-    rotary_pair_kernel<true><<<grid, 256, 0, stream>>>(xa, xb, oa, ob, cos_t, sin_t, seq, heads, width, rd, sin_sign);
-  else
-    rotary_pair_kernel<false><<<grid, 256, 0, stream>>>(xa, xb, oa, ob, cos_t, sin_t, seq, heads, width, rd, sin_sign);
+  const int per_token = heads * (width / 8);
+  const unsigned per_cta = per_token <= 128 ? 256u / (unsigned)per_token : 1u;
+  const dim3 grid(((unsigned)tokens + per_cta - 1) / per_cta, 2);
+  auto kern = per_cta > 1 ? (adjacent ? rotary_pair_kernel<true, true> : rotary_pair_kernel<false, true>)
+                          : (adjacent ? rotary_pair_kernel<true, false> : rotary_pair_kernel<false, false>);
+  kern<<<grid, 256, 0, stream>>>(xa, xb, oa, ob, cos_t, sin_t, (unsigned)tokens, per_cta, seq, heads, width, rd, sin_sign);
   return (int)cudaGetLastError();
 }
 

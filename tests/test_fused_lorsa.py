@@ -89,6 +89,40 @@ def test_rotation_of_two_tensors_matches_the_plain_statement(dev, adjacent, widt
             assert float((got != want.to(torch.bfloat16)).float().mean()) < 1e-3
 
 
+# tokens that share a CTA: 32 of one head of 64, 15 of one of 136 (and a part), two of sixteen of 64; one of seventeen; a last CTA that is not full
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,s,h,width", [(1, 1, 1, 64), (3, 11, 1, 64), (5, 7, 1, 136), (3, 9, 16, 64), (2, 5, 17, 64)])
+@pytest.mark.parametrize("adjacent", [False, True])
+def test_rotation_of_tokens_that_share_a_cta(b, s, h, width, adjacent):
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k = (torch.randn(b, s, h, width, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    ang = torch.rand(s, 32, device="cuda", generator=g) * 6
+    ang = ang.repeat_interleave(2, dim=1) if adjacent else ang.repeat(1, 2)
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    for got, x in zip(rotate_pair(q, k, cos, sin, adjacent), (q, k)):
+        want = _rotate(x.float(), cos[None, :, None], sin[None, :, None], adjacent, 64)
+        # fp32 products and their sum: three roundings of 2^-24 each, of values up to 1.42 times the largest input; then one to bf16, whose
+        # eight bits of significand round to 2^-8 of the value at most
+        assert bool(((got.float() - want).abs() <= want.abs() * 2.0**-8 + 2.0**-21 * x.float().abs().max()).all())
+
+
+@pytest.mark.gpu
+def test_rotation_of_few_heads_takes_about_as_long_as_a_copy():
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k = (torch.randn(32, 2048, 1, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    cos, sin, out, best = *(torch.randn(2048, 64, device="cuda", generator=g) for _ in range(2)), torch.empty_like(q), [1e9, 1e9]
+    for _ in range(8):
+        for i, fn in enumerate((lambda: (out.copy_(q), out.copy_(k)), lambda: rotate_pair(q, k, cos, sin, False))):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(200000)
+            start.record()
+            fn()
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+    assert best[1] < 3 * best[0], best  # (a CTA per token: five times as long)
+
+
 @pytest.mark.parametrize("dev", DEVICES)
 @pytest.mark.parametrize("variant", ["rotary", "half_split_partial_rotary", "no_positions_no_gate", "rotary_wide_heads",
                                      "rotary_wide_heads_library", "qk_norm"])  # fmt: skip
