@@ -286,13 +286,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     uint32_t g0 = 0;
     int t = 0;
     int w = (int)blockIdx.x;
-    int owed = 0;  // barriers of the row quarter that are left in this tile
+    int met = 0;  // where a wait ran out: barriers of the row quarter that this warp came to in the tile
     for (; w < n_tiles && ok; w += (int)gridDim.x, ++t) {
       int qblk, head, dv0, batch;
       decode_tile(w, qblk, head, dv0, batch);
       const int q0 = qblk * ATT_BM;
       const int n_kblocks = qblk + 1;
-      owed = n_kblocks + 2;
       const int qpos = q0 + row;
       const bool row_ok = qpos < p.seq;
       const uint32_t tmem_o = tmem_base + 2 * ATT_BN + (uint32_t)((t & 1) * DV);
@@ -303,7 +302,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const uint32_t ph = (g >> 1) & 1;
         const int k0 = kb * ATT_BN + (int)s_col;
         // (a failed wait ends the loops for the whole warp: the TMEM accesses and votes below are warp-wide)
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_s_full[u], ph, abort_flag))) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_s_full[u], ph, abort_flag))) { ok = false; met = kb; break; }
         tc_fence_after();
         uint32_t s[32];
         tmem_ld_32x32b_x32(tmem_base + (uint32_t)(u * ATT_BN) + lane_off + s_col, s);
@@ -330,7 +329,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         float* xr = xch + (u * 4) * ATT_BM + row;
         xr[cq * ATT_BM] = m_raw;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
-        --owed;
         const float m_blk = fmaxf(fmaxf(xr[0], xr[ATT_BM]), fmaxf(xr[2 * ATT_BM], xr[3 * ATT_BM])) * sc;  // sc > 0
         float alpha = 1.0f;
         bool rescale = false;
@@ -345,7 +343,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
         if (__any_sync(0xffffffffu, rescale)) {  // this warp's share of the output columns
           // the accumulator belongs to the tensor core until P V (g - 1) has completed
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_pv_done[u ^ 1], ((g - 1) >> 1) & 1, abort_flag))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_pv_done[u ^ 1], ((g - 1) >> 1) & 1, abort_flag))) { ok = false; met = kb + 1; break; }
           tc_fence_after();
           if (o_active) {
 #pragma unroll 1
@@ -362,7 +360,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         if (g >= 2) {
           // P buffer u was read by P V (g - 2)
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_pv_done[u], ((g - 2) >> 1) & 1, abort_flag))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar_pv_done[u], ((g - 2) >> 1) & 1, abort_flag))) { ok = false; met = kb + 1; break; }
         }
         l_run *= alpha;
         float l_blk = 0.0f, l_blk1 = 0.0f;
@@ -396,14 +394,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       // ---- the tile's epilogue
       const uint32_t g_last = g0 + (uint32_t)n_kblocks - 1;
-      ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(&bar_pv_done[g_last & 1], (g_last >> 1) & 1, abort_flag));
       if (!ok) break;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar_pv_done[g_last & 1], (g_last >> 1) & 1, abort_flag));
+      if (!ok) { met = n_kblocks; break; }
       tc_fence_after();
       // total of the four partial sums; slot parity continues the per-block sequence (block g_last used g_last & 1)
       float* xl = xch + (int)((g_last + 1) & 1) * 4 * ATT_BM + row;
       xl[cq * ATT_BM] = l_run;
       asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
-      --owed;
       const float l_tot = (xl[0] + xl[ATT_BM]) + (xl[2 * ATT_BM] + xl[3 * ATT_BM]);
       const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
       if (o_active) {
@@ -434,7 +432,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // keep the four warps of a row quarter together across tiles: the sum exchange above and the next maximum exchange
       // use the same slots
       asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
-      --owed;
       g0 += (uint32_t)n_kblocks;
     }
     if (!ok) {
@@ -443,11 +440,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // the other warps of the quarter may have passed the wait that this one gave up at: it keeps them company at their barriers, which
       // have no limit, until they give up or are through (every warp comes to as many in a tile)
       __syncwarp();
-      for (; w < n_tiles; w += (int)gridDim.x) {
-        if (owed < 0) owed = n_qblocks - w / per_qblock + 2;  // (n_kblocks of this tile)
-        for (; owed > 0; --owed) asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
-        owed = -1;
-      }
+      for (; w < n_tiles; w += (int)gridDim.x, met = 0)
+        for (int left = n_qblocks - w / per_qblock + 2 - met; left > 0; --left)  // (n_kblocks and two a tile)
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
     }
   }
 
