@@ -68,9 +68,10 @@ __global__ void __launch_bounds__(256)
 adam_turned_kernel(const AdamTurnedParams p) {
   __shared__ float tile[64][65];  // [w][d]
   if (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0) return;  // see sparse_grad_adam_kernel
-  const AdamTurnedSet q = p.set[blockIdx.z];
+  const AdamTurnedSet q = p.set[blockIdx.y];
   const int tiles_w = (p.w + 63) / 64;
-  const int h = blockIdx.y / tiles_w, w0 = (blockIdx.y - h * tiles_w) * 64, d0 = blockIdx.x * 64;
+  const unsigned tiles_d = (unsigned)(p.d + 63) / 64, row = blockIdx.x / tiles_d;
+  const int h = (int)row / tiles_w, w0 = ((int)row - h * tiles_w) * 64, d0 = (int)(blockIdx.x - row * tiles_d) * 64;
   if constexpr (VEC) {  // (d and w are multiples of 4: whole fours are inside or outside)
     const int x = (threadIdx.x & 15) * 4, y0 = threadIdx.x >> 4;
 #pragma unroll
@@ -138,14 +139,14 @@ adam_turned_kernel(const AdamTurnedParams p) {
 
 int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t stream) {
   if (n_sets < 1 || n_sets > 2 || p.heads <= 0 || p.d <= 0 || p.w <= 0) return (int)cudaErrorInvalidValue;
-  const long long rows = (long long)p.heads * ((p.w + 63) / 64);
-  if (rows > 65535) return (int)cudaErrorInvalidValue;
+  const long long tiles = (long long)p.heads * ((p.w + 63) / 64) * ((p.d + 63) / 64);
+  if (tiles > 2147483647LL) return (int)cudaErrorInvalidValue;
   bool vec = p.d % 4 == 0 && p.w % 4 == 0;
   for (int i = 0; i < n_sets; ++i)
     vec = vec && ((reinterpret_cast<uintptr_t>(p.set[i].p) | reinterpret_cast<uintptr_t>(p.set[i].m) | reinterpret_cast<uintptr_t>(p.set[i].v) |
                    reinterpret_cast<uintptr_t>(p.set[i].g) | reinterpret_cast<uintptr_t>(p.set[i].shadow)) % 16 == 0);
   auto kern = vec ? adam_turned_kernel<true> : adam_turned_kernel<false>;
-  kern<<<dim3((p.d + 63) / 64, (unsigned)rows, n_sets), 256, 0, stream>>>(p);
+  kern<<<dim3((unsigned)tiles, n_sets), 256, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }
 

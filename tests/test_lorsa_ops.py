@@ -36,6 +36,19 @@ def test_adam_on_turned_gradients(dev, heads, d, w, sets):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("d,w", [(4, 4), (3, 70)])
+def test_adam_on_more_heads_than_a_grid_dimension_holds(d, w):
+    heads = 65537
+    p, m, g = (_rand("cuda", *s, seed=i) for i, s in enumerate(((heads, d, w), (heads, d, w), (heads * w, d))))
+    v, shadow = 0.5 + torch.rand(heads, d, w, device="cuda"), torch.empty(heads * w, d, dtype=torch.bfloat16, device="cuda")
+    want = _ref(p, m, v, g.view(heads, w, d).permute(0, 2, 1), 3)
+    K.adam_turned([p], [(m, v)], [g], [shadow], *HYPER, 3)
+    for got, r in zip((p, m, v), want):  # (second moments of 0.5 and more: an update is of the learning rate's size, as are its roundings)
+        assert torch.allclose(got.double(), r, rtol=1e-5, atol=1e-6)
+    assert torch.equal(shadow, p.permute(0, 2, 1).reshape(heads * w, d).to(torch.bfloat16))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("b,s,heads,group,k", [(1, 8, 1, 8, 1), (2, 24, 3, 64, 7), (1, 40, 300, 8, 513), (2, 16, 64, 128, 128)])
 def test_pre_activation_gradient_and_statistics_from_codes(b, s, heads, group, k):
     F, T = heads * group, b * s
