@@ -111,8 +111,10 @@ def causal_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor | None = 
                      vt: torch.Tensor | None = None) -> torch.Tensor:  # fmt: skip
     """Differentiable causal attention ``[b, s, h, d_qk] x [b, s, h, d_v] -> [b, s, h, d_v]``; the tensor-core kernels
     when the shape is supported on a GPU, the torch oracle otherwise. The values may be given transposed instead, as
-    ``vt [b, h, d_v, s]``."""
+    ``vt [b, h, d_v, s]``, which costs a copy into the kernels' layout."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else scale
+    if v is None and vt is None:
+        raise ValueError("causal_attention takes the values as v or as vt")
     if vt is not None:
         v = vt.permute(0, 3, 1, 2)
     if not supported(q, v):

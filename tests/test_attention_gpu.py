@@ -109,3 +109,17 @@ def test_lorsa_encode_uses_the_tensor_core_attention_and_matches_the_score_path(
     hidden_slow.float().pow(2).sum().backward()
     rel = float((g_fast.float() - x.grad.float()).norm() / x.grad.float().norm())
     assert rel < 5e-2, rel
+
+
+def test_transposed_values():
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k = (torch.randn(2, 136, 3, 64, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    v = torch.randn(2, 136, 3, 128, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    vt = v.detach().permute(0, 2, 3, 1).contiguous().requires_grad_()
+    a, b = A.causal_attention(q, k, v), A.causal_attention(q, k, vt=vt)
+    a.float().square().sum().backward()
+    b.float().square().sum().backward()
+    K.check_status(torch.device("cuda"))
+    assert torch.equal(a, b) and torch.equal(vt.grad, v.grad.permute(0, 2, 3, 1))
+    with pytest.raises(ValueError):
+        A.causal_attention(q, k)
