@@ -24,3 +24,22 @@ def test_groups(B, k, F):
         heavy = groups.heavy.cpu()
         want = torch.nonzero(counts > K.HEAVY_ROW).flatten()
         assert int(heavy[0]) == want.numel() and torch.equal(heavy[1 : 1 + want.numel()].sort().values.long(), want)
+
+
+# the most features that one scan launch takes, one more (three launches), and as many as twelve layers of 24576 have; a feature of every token in
+# the last part of the scan
+@pytest.mark.parametrize("F", [(1 << 17) - 1, 1 << 17, (1 << 17) + 1, 294912])
+def test_long_dictionaries(F):
+    g = torch.Generator().manual_seed(F)
+    groups = K.FeatureGroups(F, 700 * 16, torch.device("cuda"))
+    for B in (700, 150, 700):  # (buffers are used again)
+        idx = torch.randint(-1, F, (B, 16), generator=g).to(torch.int32)
+        idx[:, 0], idx[:, 1] = F - 1, F // 2
+        groups.build(idx.cuda())
+        counts = torch.bincount(idx[idx >= 0].long(), minlength=F)
+        off = groups.offsets.cpu()
+        assert torch.equal(groups.counts.cpu().long()[:F], counts) and torch.equal(off.long()[: F + 1], torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+        e = groups.entries.cpu()[: int(off[F])].long()
+        assert torch.equal(idx.reshape(-1)[e], torch.repeat_interleave(torch.arange(F, dtype=torch.int32), counts)) and e.unique().numel() == e.numel()
+        heavy, want = groups.heavy.cpu(), torch.nonzero(counts > K.HEAVY_ROW).flatten()
+        assert want.numel() == 2 and int(heavy[0]) == 2 and torch.equal(heavy[1:3].sort().values.long(), want)

@@ -69,3 +69,22 @@ def test_stored_route_is_the_epilogues(M, N, d, k, form):
     assert idx.dtype == want_idx.dtype and val.dtype == want_val.dtype
     assert torch.equal(val * (idx >= 0), want_val * (want_idx >= 0))
     assert torch.equal(idx, want_idx)
+
+
+# the lines at 1024 rows and 128 codes, that of 128 columns a code (one group of eight more and less), the most codes the maxima serve
+@pytest.mark.parametrize("M,N,k", [(1023, 8320, 65), (1024, 8320, 65), (1024, 8312, 65), (1025, 16384, 128), (1024, 16512, 129), (130, 65536, 512), (40, 65536 + 8, 513)])
+@pytest.mark.parametrize("form", ["gate", "gate off by one", "none"])
+def test_stored_hidden_and_its_codes(M, N, k, form):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, w = torch.randn(M, 64, device=DEV, generator=g).to(torch.bfloat16), torch.randn(N, 64, device=DEV, generator=g).to(torch.bfloat16)
+    bias, gate = torch.randn(N, device=DEV, generator=g), torch.rand(N + 1, device=DEV, generator=g) + 0.5
+    gate = gate[:N] if form == "gate" else gate[1:] if form == "gate off by one" else None
+    H, idx, val = K.hidden_topk(x, w, bias, gate, k)
+    K.check_status(torch.device(DEV))
+    assert torch.equal(H, K.encoder_hidden(x, w, bias))
+    assert bool((idx >= 0).all()) and bool((idx.long().sort(1).values.diff(dim=1) > 0).all())
+    gated = H.float() * gate if gate is not None else H.float()
+    assert torch.equal(gated.gather(1, idx.long()).sort(1, descending=True).values, gated.topk(k, dim=1).values)
+    got = H.float().gather(1, idx.long())
+    # with a gate: a product with it and a division by it, three units in the last place together
+    assert bool(((val - got).abs() <= (4 * 2.0**-24 if gate is not None else 0.0) * got.abs()).all())
