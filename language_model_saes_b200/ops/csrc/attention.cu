@@ -4,8 +4,8 @@
 // attention per QK head whose value / output width is the head's OV group: q, k are [batch, seq, heads, d_qk] and
 // v is [batch, seq, heads, d_v] with d_v != d_qk in general, which the flash kernels of the usual libraries do not take.
 //
-// Forward (attn_fwd_kernel): one CTA per (128-query block, head, value chunk of DV columns, batch element); four warps
-// whose thread r owns query row r (= TMEM lane r) and a fifth warp that issues the TMA loads and the MMAs.
+// Forward (attn_fwd_kernel): tiles of a 128-query block, head, value chunk of DV columns and batch element; sixteen warps, four threads
+// to a query row (= TMEM lane), and one that issues the TMA loads and the MMAs.
 //   per 128-key block (causal: only blocks up to the diagonal):
 //     TMA      K block [128 x DQK] and V block [128 x DV] (64-column atoms, 128-byte swizzle) -> shared memory
 //     tcgen05  S = Q K^T            (128 x 128 x DQK, accumulator in TMEM columns [0, 128))
@@ -92,7 +92,7 @@ constexpr float kRescaleSlack = 8.0f;  // log2 units the running reference may l
 // that the loads and first MMAs of the next tile run while the softmax warps finish and store the current one.
 // K, V, P (shared memory) and S (TMEM) are double-buffered over the sequence of key blocks of ALL tiles of the CTA:
 // the g-th key block uses buffer g & 1 and completes phase g >> 1 of that buffer's barriers. The output accumulator is
-// double-buffered over tiles (tile t uses buffer t & 1). Roles and hand-offs (mbarriers and 64-thread named barriers; no
+// double-buffered over tiles (tile t uses buffer t & 1). Roles and hand-offs (mbarriers and 128-thread named barriers; no
 // CTA-wide barrier inside the loops):
 //   issuer   loads two key blocks ahead inside a tile; S(g+1) is computed while the rows work on S(g); P V (g) as soon
 //            as P(g) is written; a K / V buffer is refilled when S / P V of its previous block has consumed it.
@@ -458,6 +458,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
 }
 
+// Persistent grids: one CTA per SM.
+static int persistent_grid(long long tiles) {
+  static const int num_sms = [] {
+    int dev = 0, n = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+    return n;
+  }();
+  return (int)(tiles < num_sms ? tiles : num_sms);
+}
+
 template <int DQK, int DV>
 static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                                     const AttnParams& p, cudaStream_t stream) {
@@ -466,16 +476,9 @@ static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk
   auto kern = attn_fwd_kernel<DQK, DV>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
   if (e != cudaSuccess) return e;
-  static int num_sms = 0;  // persistent grid: one CTA per SM
-  if (num_sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      num_sms = 148;
-  }
   const long long tiles = (long long)((p.seq + ATT_BM - 1) / ATT_BM) * p.heads * (p.dv / DV) * p.batch;
   if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
-  const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  kern<<<grid, FWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, p);
+  kern<<<persistent_grid(tiles), FWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -484,9 +487,9 @@ int attn_value_chunk(int dv) { return dv % 128 == 0 ? 128 : (dv % 64 == 0 ? 64 :
 // =============================================================================================================
 // Backward. With P = softmax(scale * Q K^T) (causal), O = P V, D = rowsum(dO * O):
 //   dV = P^T dO,   dP = dO V^T,   dS = P * (dP - D),   dQ = scale * dS K,   dK = scale * dS^T Q.
-// Two persistent kernels of the same build (one CTA per SM, tiles dealt out longest first):
-//   attn_bwd_dq_kernel   a tile is a query block and walks its key blocks:   dQ += dS K
-//   attn_bwd_dkv_kernel  a tile is a key block (and value chunk) and walks its query blocks:   dV += P^T dO,  dK += dS^T Q
+// Two launches of one persistent template, attn_bwd_kernel (one CTA per SM, tiles dealt out longest first):
+//   DVC 0   a tile is a query block and walks its key blocks:   dQ += dS K
+//   else    a tile is a key block (and value chunk) and walks its query blocks:   dV += P^T dO,  dK += dS^T Q
 // In both, every step computes S = Q K^T and dP = dO V^T of one 128 x 128 block with queries in the TMEM lanes, so that the row
 // statistics are one value per thread, and every operand is read from the row-major tensors: where a product contracts over
 // positions its tile is a MN-major operand of the same shared-memory copy (P and dS as MN-major A, Q, K and dO as MN-major B), so
@@ -497,7 +500,8 @@ int attn_value_chunk(int dv) { return dv % 128 == 0 ? 128 : (dv % 64 == 0 ? 64 :
 //   warp 16     TMA producer; warp 17 the MMA issuer: S(g), dP(g), then the accumulating products of block g - 1
 // A finished tile is stored one block late (after the first block of the next tile), so that nothing waits for its last product.
 // What bounds a block: 1024 cycles of exponentials (16 a cycle and SM) against 1024 (dQ) or 1536 (dK/dV) cycles of MMAs at
-// d_qk 64, d_v 128; measured about 3400 and 5200 (hand-offs between the three roles, and tiles of four and a half blocks on average).
+// d_qk 64, d_v 128; measured about 3400 and 5300 (4608 blocks on 148 CTAs at the size below): hand-offs between the three roles. The tensor
+// pipe is active 34 and 30 % of the time, the exponential pipe 36 and 22 %.
 // 2 x 64 heads x 1024 positions, d_qk 64, d_v 128: dQ 146 -> 61 us, dK/dV 226 -> 97 us against kernels of four warps that took turns with
 // the tensor core, and about 250 us of transposed copies and conversions around them are gone.
 // =============================================================================================================
@@ -938,7 +942,7 @@ static cudaError_t attn_bwd_variant(const CUtensorMap& tq, const CUtensorMap& tk
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)((p.seq + 127) / 128) * p.heads * (DVC != 0 ? p.dv / (DVC != 0 ? DVC : 1) : 1) * p.batch;
   if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
-  kern<<<(int)(tiles < 148 ? tiles : 148), BWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, tdo, p);
+  kern<<<persistent_grid(tiles), BWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, tdo, p);
   return cudaGetLastError();
 }
 

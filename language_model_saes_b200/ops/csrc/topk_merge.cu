@@ -360,7 +360,7 @@ __device__ __forceinline__ unsigned descend(const unsigned (&val)[N], int k, int
 }
 
 // MAXIMA: the largest gated value of every 32 columns comes with H (the encoder GEMM's epilogue leaves them): those are the column groups,
-// and only groups whose maximum reaches the bound are read at all: 4096 rows of 32768, k 128: 206 -> 116 us.
+// and only groups whose maximum reaches the bound are read at all: 4096 rows of 32768, k 128, with a gate: 195 -> 111 us (211 -> 135 without).
 template <bool MAXIMA>
 __global__ void __launch_bounds__(RT_THREADS, 5)
 row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N, int k,
@@ -501,8 +501,8 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
 //   candidates above the bound listed in order; the exact k-th value of them; of equal ones the first columns
 // Rows with more groups or candidates than there is room for (values repeated hundreds of times) are taken by the whole CTA afterwards, in
 // the descent over the row that other kernels end in, too.
-// As a CTA per row with barriers between the steps, 4096 rows of 32768 bf16, k 128: 153 us; here 61 (1024 rows: 46 and 37; 512 rows, where
-// the chain is all there is: 29 and 36). 1024 rows of 16384 fp32, k 32: 20 us.
+// As a CTA per row with barriers between the steps (row_topk_kernel<true>), 4096 rows of 32768 bf16, k 128, with a gate: 111 us; here 49
+// (without: 135 and 53; 1024 rows: 46 and 37; 512 rows, where the chain is all there is: 29 and 36). 1024 rows of 16384 fp32, k 32: 20 us.
 constexpr int RS_WARPS = 8, RS_PER = 16, RS_GROUPS = 256, RS_CAND = 384, RS_MAX_K = 128;
 static_assert(RS_WARPS * 32 == RT_THREADS, "the fallback's CTA");
 template <typename T>

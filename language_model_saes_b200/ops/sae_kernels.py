@@ -233,8 +233,9 @@ def storing_pays(M: int, N: int, K: int, k: int) -> bool:
     1024 x 16384 x 1024, 64: 103, 64; 2048 x 24576 x 768, 50: 134, 116; 4096 x 8192 x 1024, 64: 149, 110; at the lines 1024 x 24576 x 2048, 32:
     106, 105; 640 x 131072 x 768, 50: 202, 187). With more or longer rows or more columns it does not (2048 x 16384 x 2048, 32: 124, 130;
     3328 x 16384 x 1024, 16: 124, 134; 3001 x 13000 x 1160, 37: 126, 132; 4096 x 32768 x 512, 32: 226, 239; 640 x 131072 x 4096, 50: 640, 734).
-    The maxima have to bound the k-th value, and with few columns the merge of their few candidates is shorter than the selection (a step
-    of 512 x 256 x 64, k 8: 73 us, stored 79)."""
+    The maxima have to bound the k-th value. With fewer columns than 4096 many rows lose (4096 x 1024 x 256, 8: 32, 38; 4096 x 2048 x 512, 16: 42, 48;
+    4096 x 3072 x 768, 16: 51, 56) what few rows would gain (1024 x 2048 x 512, 16: 34, 30; 512 x 1024 x 64, 8: 28, 24; but a step of 512 x 256 x 64,
+    k 8, is 73 us, stored 79)."""
     small = M * K <= k << 16 and M * N * K <= 1 << 36 and 4 * M * N <= STORED_BYTES
     return 1 <= M <= 4096 and 4096 <= N <= 1 << 20 and small and maxima_pay(N, k)
 
@@ -356,7 +357,7 @@ def encoder_topk(
     """Sparse codes of a TopK encoder: (idx [M,k], act [M,k]) (+ hidden_pre bf16 when asked).
 
     ``k <= 64`` uses the GEMM's fused top-k epilogue (the dense pre-activations are never written unless
-    ``return_hidden``), or ``stored_topk`` where that is faster; larger k materialises H and selects with the radix row-top-k kernel.
+    ``return_hidden``), or ``stored_topk`` where that is faster; larger k materialises H and selects from it (``hidden_topk``).
     """
     if not x.is_cuda:
         h = ref_hidden(x, w, bias)
