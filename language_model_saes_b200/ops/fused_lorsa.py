@@ -275,9 +275,13 @@ class FusedLorsaStep:
             dact = K.sparse_dact(idx, WO16, dxhat)
         # d z: the activation passes the gradient where a head was selected (its value is the pre-activation itself)
         if kernels:
-            dz, delta = torch.empty_like(z), torch.empty_like(lse)
+            # (the codes hold what is still wanted of z: the gradient takes its memory, and what follows takes that of the attention's
+            # operands. A step's buffers are 16 to 33 MB each, and every one that the allocator has no free block for costs a new engine's first
+            # step a device allocation, a millisecond or two on a busy machine.)
+            dz, delta = z, torch.empty_like(lse)
             K._ext().lorsa_dz(idx, act, dact, dz, delta)
             dq, dk, dv = attention_kernels.causal_attention_bwd(q, k, v, dz.view(v.shape), lse, delta, 1.0 / self.m.attn_scale, torch.bfloat16)
+            del q, k, v, z, dz, out, lse, delta
         else:
             dz = torch.zeros(T_l, self.F + 8, dtype=z.dtype if z.is_cuda else torch.float32, device=x.device)
             dz.scatter_(1, torch.where(idx >= 0, idx, torch.full_like(idx, self.F)).long(), dact.to(dz.dtype))

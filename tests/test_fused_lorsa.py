@@ -398,3 +398,24 @@ def test_fused_lorsa_step_head_shards_and_replicas_on_four_ranks_match_single():
     from language_model_saes_b200.testing import distributed_test
 
     distributed_test(nproc_per_node=4, backend="gloo")(_tp_dp_body)()
+
+
+@pytest.mark.gpu
+def test_a_step_holds_each_buffer_as_long_as_it_is_read():
+    """At most the queries and keys before and after the rotation (or their gradients) and three matrices of the values' size at a time."""
+    b, s, heads, group, d, k = 2, 512, 16, 128, 256, 32
+    F, T, qk = heads * group, b * s, heads * 64
+    cfg = LorsaConfig(hook_point_in="a", hook_point_out="b", d_model=d, expansion_factor=F / d, n_qk_heads=heads, d_qk_head=64, rotary_dim=64, n_ctx=s,
+                      act_fn="topk", top_k=k, device="cuda", dtype=torch.float32)  # fmt: skip
+    m = LowRankSparseAttention(cfg)
+    m.init_parameters()
+    engine = FusedLorsaStep(m)
+    x = torch.randn(b, s, d, device="cuda").to(torch.bfloat16)
+    for _ in range(2):
+        engine.step(x, x, k, 1e-4)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    engine.step(x, x, k, 1e-4)
+    small = T * k * 12 + T * d * 2 + 3 * b * heads * s * 4 + (1 << 20)  # codes and their gradients, d x_hat, row statistics, odds and ends
+    assert torch.cuda.max_memory_allocated() - before <= 2 * T * (4 * qk + 3 * F) + small
