@@ -223,9 +223,11 @@ void topk_merge(const Tensor& cand_val, const Tensor& cand_idx, int64_t M, int64
 }
 
 // C [M, N] = A [M, K] @ B [N, K]^T in fp32 on the bf16 tensor cores (fp32_gemm.cu). With na [M] (written: the rows' norms) C is bf16 and
-// receives the lower ends that topk_estimate takes, made with bias [N] and gate [N] (both optional); top: int32 [4 + (N + 1) / 2], the first four
-// zeroed, on a 16-byte boundary, goes with them (the largest width of a column, whether a gate is 0 or NaN, 0, 0, every column's width in bf16). status: int32 [4], zeroed, of this call alone: a wait in the product that runs out is recorded there, and everything is done on the
-// fp32 pipes then (lower ends: by topk_estimate). tensor_cores = false leaves the product out (as if it had given up).
+// receives the lower ends that topk_estimate takes, made with bias [N] and gate [N] (both optional); top: int32 [4 + (N + 1) / 2], the
+// first four zeroed, on a 16-byte boundary, goes with them (the largest width of a column; whether a gate is 0 or NaN; two words of
+// room; every column's width in bf16). status: int32 [4], zeroed, of this call alone: a wait in the product that runs out is recorded there,
+// and everything is done on the fp32 pipes then (lower ends: by topk_estimate). tensor_cores = false leaves the product out (as if it had
+// given up).
 void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& status, const c10::optional<Tensor>& na,
                const c10::optional<Tensor>& top, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate,
                bool tensor_cores, int64_t workspace) {

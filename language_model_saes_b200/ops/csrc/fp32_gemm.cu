@@ -52,8 +52,8 @@ __device__ __forceinline__ int part_b(int t) { return TERMS == 6 ? (0x021010 >> 
 
 // dst [rows][PARTS][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
 // then flags[0] != 0. For lower ends, all optional: norm[r], at least the row's 2-norm and at most 10 % above it; wide[r], at least
-// norm[r] * gate[r]; top[0], at least that of every row whose norm is finite; top[1] != 0 where a gate is 0 or NaN. The norm is infinite where the row's largest
-// magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r] negative, NaN or beyond 2^50: products, (sum + bias) * gate and the
+// norm[r] * gate[r]; top[0], at least that of every row whose norm is finite; top[1] != 0 where a gate is 0 or NaN. The norm (and the
+// width) is infinite where the row's largest magnitude is outside [2^-40, 2^30), bias[r] beyond 2^75 or gate[r] negative, NaN or beyond 2^50: products, (sum + bias) * gate and the
 // parts of what is within stay clear of the ends of the fp32 range (2^30 * 2^30 * K 2^14, doubled, * 2^50 < 2^127).
 struct SplitBounds {
   float* norm;

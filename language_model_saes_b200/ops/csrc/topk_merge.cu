@@ -782,8 +782,8 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 // at or above it. The upper end is the lower one plus what rounding it down to bf16 may have taken (2^-7 of it) plus twice the bound on the
 // estimate's error. Where that is small against the k-th end (a 64th) for the column where it is largest, all columns take that one's, and
 // neither pass reads anything per column but the ends; elsewhere (a few features of large norm, long rows, few positive values) the second pass
-// reads every column's own: 4096 x 24576 x 768, k 50, at an 108th 660 us with the largest for all and 664 with each its own, at a 54th 698 and
-// 664, at a 39th 722 and 664. (2048 x 24576 x 4096 with one row of W thirty times the others: 11.3 ms with the largest for all, 1.66 so.)
+// reads every column's own: 4096 x 24576 x 768, k 50, at a hundredth 660 us with the largest for all and 664 with each its own, at a fiftieth 698
+// and 660, at a 36th 722 and 661. (2048 x 24576 x 4096 with one row of W thirty times the others: 11.3 ms with the largest for all, 1.66 so.)
 // The columns that may be selected (k and a few) are summed up in order before the exact selection.
 //   Columns that the bound says nothing about (their lower end is NaN) are among them; rows with more such columns than there is room for,
 // and all rows where the product gave up, are listed, multiplied in order as a whole (rows_product.cu) and selected from exactly. All
