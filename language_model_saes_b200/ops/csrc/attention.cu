@@ -107,6 +107,7 @@ template <int DQK, int DV>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
+  pdl_wait();
   using L = AttnSmem<DQK, DV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -478,7 +479,7 @@ static cudaError_t attn_fwd_variant(const CUtensorMap& tq, const CUtensorMap& tk
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)((p.seq + ATT_BM - 1) / ATT_BM) * p.heads * (p.dv / DV) * p.batch;
   if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
-  kern<<<persistent_grid(tiles), FWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, p);
+  launch(kern, persistent_grid(tiles), FWD_THREADS, L::kDynamicBytes, stream, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -634,6 +635,7 @@ template <int DQK, int DVC>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do, const AttnBwdParams p) {
+  pdl_wait();
   constexpr bool DKV = DVC != 0;
   using L = BwdSmem<DQK, DKV>;
   extern __shared__ uint8_t smem_raw[];
@@ -942,7 +944,7 @@ static cudaError_t attn_bwd_variant(const CUtensorMap& tq, const CUtensorMap& tk
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)((p.seq + 127) / 128) * p.heads * (DVC != 0 ? p.dv / (DVC != 0 ? DVC : 1) : 1) * p.batch;
   if (tiles <= 0 || tiles > 2147483647LL) return cudaErrorInvalidValue;
-  kern<<<persistent_grid(tiles), BWD_THREADS, L::kDynamicBytes, stream>>>(tq, tk, tv, tdo, p);
+  launch(kern, persistent_grid(tiles), BWD_THREADS, L::kDynamicBytes, stream, tq, tk, tv, tdo, p);
   return cudaGetLastError();
 }
 
@@ -962,6 +964,7 @@ int attn_bwd_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out, long long rows, int seq, int heads, int dv,
                   float* __restrict__ delta) {
+  pdl_wait();
   const int sub = threadIdx.x & 7;
   const long long r = (long long)blockIdx.x * 32 + (threadIdx.x >> 3);
   float s = 0.0f;
@@ -994,7 +997,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
 int attn_delta_launch(const __nv_bfloat16* dout, const __nv_bfloat16* out, int batch, int seq, int heads, int dv, float* delta, cudaStream_t stream) {
   const long long rows = (long long)batch * seq * heads;
   if (rows == 0) return 0;
-  attn_delta_kernel<<<(int)((rows + 31) / 32), 256, 0, stream>>>(dout, out, rows, seq, heads, dv, delta);
+  launch(attn_delta_kernel, (int)((rows + 31) / 32), 256, 0, stream, dout, out, rows, seq, heads, dv, delta);
   return (int)cudaGetLastError();
 }
 

@@ -54,6 +54,7 @@ constexpr int CH_BINS = 2048;
 __global__ void __launch_bounds__(CS_THREADS)
 chunk_hist_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ maxima, long long ld_maxima, int B, int N, const float* __restrict__ floor,
                   unsigned* __restrict__ hist, int nbins) {
+  pdl_wait();
   __shared__ unsigned s_hist[CH_BINS];
   for (int i = threadIdx.x; i < CH_BINS; i += CS_THREADS) s_hist[i] = 0u;
   __syncthreads();
@@ -80,7 +81,7 @@ chunk_hist_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
 int chunk_hist_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* floor, unsigned* hist, int nbins,
                       cudaStream_t stream) {
   if (B <= 0 || N <= 0) return 0;
-  chunk_hist_kernel<<<148 * 8, CS_THREADS, 0, stream>>>(x, maxima, ld_maxima, B, N, floor, hist, nbins);
+  launch(chunk_hist_kernel, 148 * 8, CS_THREADS, 0, stream, x, maxima, ld_maxima, B, N, floor, hist, nbins);
   return (int)cudaGetLastError();
 }
 
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(CS_THREADS)
 chunk_compact_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ maxima, long long ld_maxima, int B, int N, const float* __restrict__ thr,
                      const float* __restrict__ col_div, int* __restrict__ nnz, int* __restrict__ ties, const int* __restrict__ tie_quota, int cap,
                      int* __restrict__ idx, float* __restrict__ val) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int row = blockIdx.x * (CS_THREADS / 32) + (threadIdx.x >> 5);
@@ -133,10 +135,10 @@ int chunk_compact_launch(const __nv_bfloat16* x, const float* maxima, long long 
   const int blocks = (B + CS_THREADS / 32 - 1) / (CS_THREADS / 32);
   if (idx != nullptr) {
     if (tie_quota == nullptr || cap <= 0) return (int)cudaErrorInvalidValue;
-    chunk_compact_kernel<true><<<blocks, CS_THREADS, 0, stream>>>(x, maxima, ld_maxima, B, N, thr, col_div, nnz, nullptr, tie_quota, cap, idx, val);
+    launch(chunk_compact_kernel<true>, blocks, CS_THREADS, 0, stream, x, maxima, ld_maxima, B, N, thr, col_div, nnz, nullptr, tie_quota, cap, idx, val);
   } else {
     if (ties == nullptr) return (int)cudaErrorInvalidValue;
-    chunk_compact_kernel<false><<<blocks, CS_THREADS, 0, stream>>>(x, maxima, ld_maxima, B, N, thr, nullptr, nnz, ties, nullptr, 0, nullptr, nullptr);
+    launch(chunk_compact_kernel<false>, blocks, CS_THREADS, 0, stream, x, maxima, ld_maxima, B, N, thr, nullptr, nnz, ties, nullptr, 0, nullptr, nullptr);
   }
   return (int)cudaGetLastError();
 }

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(CLT_DEC_WARPS * 32)
 clt_decode_kernel(const CltTable tab, const int* __restrict__ idx, const float* __restrict__ val, int B, int K, int L,
                   int F, int d, int nseg, const float* __restrict__ bias, float* __restrict__ out_f32,
                   __nv_bfloat16* __restrict__ out_bf16) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = d / 8;
   const long long item = (long long)blockIdx.x * CLT_DEC_WARPS + (threadIdx.x >> 5);
@@ -78,7 +79,7 @@ int clt_decode_launch(const CltTable& tab, const int* idx, const float* val, int
   const int nseg = (d / 8 + 31) / 32;
   const long long blocks = ((long long)B * L * nseg + CLT_DEC_WARPS - 1) / CLT_DEC_WARPS;
   if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
-  clt_decode_kernel<<<(int)blocks, CLT_DEC_WARPS * 32, 0, stream>>>(tab, idx, val, B, K, L, F, d, nseg, bias, out_f32, out_bf16);
+  launch(clt_decode_kernel, (int)blocks, CLT_DEC_WARPS * 32, 0, stream, tab, idx, val, B, K, L, F, d, nseg, bias, out_f32, out_bf16);
   return (int)cudaGetLastError();
 }
 

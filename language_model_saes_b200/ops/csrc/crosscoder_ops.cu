@@ -19,6 +19,7 @@ constexpr int JL_THREADS = 256;
 
 __global__ void __launch_bounds__(JL_THREADS)
 jumprelu_lists_kernel(const JumpReluListParams p) {
+  pdl_wait();
   __shared__ float s_u[JL_THREADS / 32];
   __shared__ int s_n[JL_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -66,7 +67,7 @@ jumprelu_lists_kernel(const JumpReluListParams p) {
 int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream) {
   if (p.B <= 0 || p.cap <= 0 || p.H <= 0 || p.F <= 0) return (int)cudaErrorInvalidValue;
   const long long blocks = ((long long)p.B * p.cap + JL_THREADS - 1) / JL_THREADS;
-  jumprelu_lists_kernel<<<(int)(blocks < 148LL * 16 ? blocks : 148LL * 16), JL_THREADS, 0, stream>>>(p);
+  launch(jumprelu_lists_kernel, (int)(blocks < 148LL * 16 ? blocks : 148LL * 16), JL_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 

@@ -22,6 +22,7 @@ constexpr int kWarpList = 256;
 
 __global__ void __launch_bounds__(256)
 nonfinite_kernel(const float* __restrict__ w, long long n, int* __restrict__ found) {
+  pdl_wait();
   bool bad = false;
   const long long n4 = n / 4, stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
@@ -35,6 +36,7 @@ nonfinite_kernel(const float* __restrict__ w, long long n, int* __restrict__ fou
 
 __global__ void __launch_bounds__(DD_THREADS, 6)
 sparse_rows_kernel(const float* __restrict__ acts, const float* __restrict__ W, int F, int d, int most, int* __restrict__ todo, float* __restrict__ out) {
+  pdl_wait();
   __shared__ int s_idx[8][kWarpList];
   __shared__ float s_val[8][kWarpList];
   __shared__ int s_n[8];
@@ -145,8 +147,8 @@ int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, 
   if (B <= 0) return 0;
   const long long n = (long long)F * d;
   const long long blocks = (n / 4 + 255) / 256;
-  nonfinite_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(W, n, todo + 1 + B);
-  sparse_rows_kernel<<<B, DD_THREADS, 0, stream>>>(acts, W, F, d, most, todo, out);
+  launch(nonfinite_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, W, n, todo + 1 + B);
+  launch(sparse_rows_kernel, B, DD_THREADS, 0, stream, acts, W, F, d, most, todo, out);
   RowsProductParams r = {};
   r.A = acts; r.B = W; r.C = out; r.N = d; r.K = F; r.rows = todo; r.max_rows = B;
   r.part = part; r.part_floats = part_floats; r.part_done = todo + 2 + B; r.part_tiles = part_tiles;

@@ -213,6 +213,7 @@ template <bool WRITE_H, bool TOPK, int STAGES, int KS, int CAP, bool PAIR, bool 
 __global__ void __launch_bounds__(128 + 32 * epilogue_warps(TOPK), 1)
 enc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                 const EncGemmParams p) {
+  pdl_wait();
   using L = SmemLayout<STAGES, CAP, PAIR, NARROW, F32>;
   constexpr int STAGE_BYTES = L::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -658,13 +659,15 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
   cfg.blockDim = dim3(128 + 32 * epilogue_warps(TOPK));
   cfg.dynamicSmemBytes = L::kDynamicBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = PAIR ? 2 : 1;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
 }
 

@@ -66,6 +66,7 @@ template <int PARTS>
 __global__ void __launch_bounds__(256)
 split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags,
                   const SplitBounds b) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float most = 0.0f;
   for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
@@ -143,6 +144,7 @@ __device__ __forceinline__ uint32_t bf16_down(float x) {
 template <int TERMS, bool ENDS>
 __global__ void __launch_bounds__(FG_THREADS, 1)
 fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Fp32GemmParams p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + FG_BAR_OFF);
@@ -390,6 +392,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 __global__ void __launch_bounds__(256)
 marked_products_kernel(const float* __restrict__ A, const float* __restrict__ B, int M, int N, int K, const int* __restrict__ fa,
                        const int* __restrict__ fb, float* __restrict__ C, long long ldc, const int* __restrict__ status) {
+  pdl_wait();
   const bool all = status[0] != 0;
   if (fa[0] == 0 && fb[0] == 0 && !all) return;
   const int lane = threadIdx.x & 31;
@@ -411,7 +414,7 @@ int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv
   if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0 || (parts != 2 && parts != 3)) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
   auto kern = parts == 2 ? split_bf16_kernel<2> : split_bf16_kernel<3>;
-  kern<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream>>>(src, rows, K, kp, dst, flags, SplitBounds{norm, wide, top, bias, gate});
+  launch(kern, blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream, src, rows, K, kp, dst, flags, SplitBounds{norm, wide, top, bias, gate});
   return (int)cudaGetLastError();
 }
 
@@ -428,13 +431,15 @@ static cudaError_t launch_product(const void* kernel, const CUtensorMap& ta, con
   cfg.blockDim = dim3(FG_THREADS);
   cfg.dynamicSmemBytes = FG_SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   void* args[3] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &p};
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
@@ -447,7 +452,7 @@ int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* 
     const cudaError_t e = launch_product(reinterpret_cast<const void*>(fp32_gemm_kernel<6, false>), ta, tb, p, stream);
     if (e != cudaSuccess) return (int)e;
   }
-  marked_products_kernel<<<148 * 8, 256, 0, stream>>>(A, B, M, N, K, fa, fb, C, ldc, status);
+  launch(marked_products_kernel, 148 * 8, 256, 0, stream, A, B, M, N, K, fa, fb, C, ldc, status);
   return (int)cudaGetLastError();
 }
 

@@ -257,6 +257,7 @@ constexpr int rows_threads() { return NCH <= 4 ? 768 : NCH <= 6 ? 640 : 512; }
 template <int W, int NCH>
 __global__ void __launch_bounds__(rows_threads<NCH>(), 1)
 grad_adam_rows_kernel(const GradAdamParams p) {
+  pdl_wait();
   constexpr int T = 32 * W;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int G = (int)blockDim.x / T;
@@ -580,7 +581,7 @@ cudaError_t launch_rows(GradAdamParams p, cudaStream_t stream) {
   auto kern = grad_adam_rows_kernel<W, NCH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemBudget + 1024));
   if (e != cudaSuccess) return e;
-  kern<<<blocks, G * T, smem, stream>>>(p);
+  launch(kern, blocks, G * T, smem, stream, p);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@ LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_lorsa_ops)
 __global__ void __launch_bounds__(256)
 lorsa_dz_kernel(const int* __restrict__ idx, const float* __restrict__ act, const float* __restrict__ dact, int k, int F, int heads, int group, int seq,
                 __nv_bfloat16* __restrict__ dz, float* __restrict__ delta) {
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(smem_raw);  // [F] (a multiple of 8)
   int* s_head = reinterpret_cast<int*>(row + F);                    // [k]
@@ -51,7 +52,7 @@ int lorsa_dz_launch(const int* idx, const float* act, const float* dact, long lo
   if (tokens == 0) return 0;
   cudaError_t e = cudaFuncSetAttribute(lorsa_dz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e != cudaSuccess) return (int)e;
-  lorsa_dz_kernel<<<(int)tokens, 256, smem, stream>>>(idx, act, dact, k, F, heads, group, seq, dz, delta);
+  launch(lorsa_dz_kernel, (int)tokens, 256, smem, stream, idx, act, dact, k, F, heads, group, seq, dz, delta);
   return (int)cudaGetLastError();
 }
 
@@ -66,6 +67,7 @@ int lorsa_dz_launch(const int* idx, const float* act, const float* dact, long lo
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 adam_turned_kernel(const AdamTurnedParams p) {
+  pdl_wait();
   __shared__ float tile[64][65];  // [w][d]
   if (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0) return;  // see sparse_grad_adam_kernel
   const AdamTurnedSet q = p.set[blockIdx.y];
@@ -146,7 +148,7 @@ int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t strea
     vec = vec && ((reinterpret_cast<uintptr_t>(p.set[i].p) | reinterpret_cast<uintptr_t>(p.set[i].m) | reinterpret_cast<uintptr_t>(p.set[i].v) |
                    reinterpret_cast<uintptr_t>(p.set[i].g) | reinterpret_cast<uintptr_t>(p.set[i].shadow)) % 16 == 0);
   auto kern = vec ? adam_turned_kernel<true> : adam_turned_kernel<false>;
-  kern<<<dim3((unsigned)tiles, n_sets), 256, 0, stream>>>(p);
+  launch(kern, dim3((unsigned)tiles, n_sets), 256, 0, stream, p);
   return (int)cudaGetLastError();
 }
 

@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(256)
 rotary_pair_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat16* __restrict__ xb, __nv_bfloat16* __restrict__ oa,
                    __nv_bfloat16* __restrict__ ob, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                    unsigned tokens, unsigned tokens_per_cta, int seq, int heads, int width, int rd, float sin_sign) {
+  pdl_wait();
   const unsigned per_head = (unsigned)width / 8, per_token = (unsigned)heads * per_head;
   const __nv_bfloat16* x = blockIdx.y == 0 ? xa : xb;
   __nv_bfloat16* o = blockIdx.y == 0 ? oa : ob;
@@ -110,7 +111,7 @@ int rotary_pair_launch(const __nv_bfloat16* xa, const __nv_bfloat16* xb, __nv_bf
   const dim3 grid(((unsigned)tokens + per_cta - 1) / per_cta, 2);
   auto kern = per_cta > 1 ? (adjacent ? rotary_pair_kernel<true, true> : rotary_pair_kernel<false, true>)
                           : (adjacent ? rotary_pair_kernel<true, false> : rotary_pair_kernel<false, false>);
-  kern<<<grid, 256, 0, stream>>>(xa, xb, oa, ob, cos_t, sin_t, (unsigned)tokens, per_cta, seq, heads, width, rd, sin_sign);
+  launch(kern, grid, 256, 0, stream, xa, xb, oa, ob, cos_t, sin_t, (unsigned)tokens, per_cta, seq, heads, width, rd, sin_sign);
   return (int)cudaGetLastError();
 }
 

@@ -18,6 +18,7 @@ constexpr int RP_SLOTS = 148 * 2;
 template <bool B_BY_K>  // B is [K, N] (else [N, K])
 __global__ void __launch_bounds__(RP_THREADS, 2)
 rows_product_kernel(const RowsProductParams p) {
+  pdl_wait();
   __shared__ __align__(16) float s_a[2][RP_K][RP_LD];
   __shared__ __align__(16) float s_b[2][RP_K][RP_LD];
   __shared__ int s_last;
@@ -160,8 +161,8 @@ int rows_product_launch(RowsProductParams p, bool b_by_k, cudaStream_t stream) {
   if (p.max_rows <= 0) return 0;
   if (tiles > 2147483647LL / 16) return (int)cudaErrorInvalidValue;
   p.vec = p.N % 4 == 0 && reinterpret_cast<uintptr_t>(p.C) % 16 == 0;
-  if (b_by_k) rows_product_kernel<true><<<RP_SLOTS, RP_THREADS, 0, stream>>>(p);
-  else rows_product_kernel<false><<<RP_SLOTS, RP_THREADS, 0, stream>>>(p);
+  if (b_by_k) launch(rows_product_kernel<true>, RP_SLOTS, RP_THREADS, 0, stream, p);
+  else launch(rows_product_kernel<false>, RP_SLOTS, RP_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 

@@ -137,6 +137,7 @@ template <typename T>
 __global__ void __launch_bounds__(HIST_THREADS)
 radix_hist_hi_kernel(const T* __restrict__ x, long long A, long long S, long long N, long long s,
                      unsigned* __restrict__ hist, const float* __restrict__ floor, const long long* __restrict__ need) {
+  pdl_wait();
   // `floor`: only values of at least *floor are counted (a caller that knows a lower bound of the value it is looking
   // for saves nearly all of the shared-memory atomics). `need`: the pass runs only if need[3] != 0 (the repeat without
   // a floor, for the case that the floor turned out to lie above the value sought).
@@ -163,6 +164,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 radix_hist_lo_kernel(const T* __restrict__ x, long long A, long long S, long long N, long long s,
                      const long long* __restrict__ sel, unsigned* __restrict__ hist) {
+  pdl_wait();
   const uint32_t want = (uint32_t)sel[0];
   for_each_positive<T, 256>(x, A, S, N, s, 0u, [&](uint32_t b) {
     uint32_t bin = b >> 16;
@@ -177,6 +179,7 @@ radix_hist_lo_kernel(const T* __restrict__ x, long long A, long long S, long lon
 __global__ void __launch_bounds__(1024)
 radix_pick_kernel(const unsigned* __restrict__ hist, int nbins, long long k, const long long* __restrict__ sel_in,
                   int level, long long* __restrict__ sel_out, float* __restrict__ thr, const long long* __restrict__ need) {
+  pdl_wait();
   // sel_out[3] = 1 when the histogram held fewer than k members (with a floored histogram: the floor was too high).
   // `need`: the pick runs only if need[3] != 0 (read by every thread before anything is written: need may be sel_out).
   const bool run_it = need == nullptr || need[3] != 0;
@@ -421,6 +424,7 @@ row_compact_kernel(const T* __restrict__ x, int B, long long N, int cap, int* __
                    int* __restrict__ nnz, const float* __restrict__ thr, const float* __restrict__ col_div,
                    int* __restrict__ ties, const int* __restrict__ tie_quota, const float* __restrict__ col_thr,
                    int* __restrict__ seg_counts) {
+  pdl_wait();
   constexpr int V = RowVec<T>::V;
   constexpr int NW = RC_THREADS / 32;
   RowPredicate q;
@@ -554,6 +558,7 @@ template <int R>
 __global__ void __launch_bounds__(RC_THREADS)
 row_compact_cols_kernel(const __nv_bfloat16* __restrict__ x, int B, int N, int cap, int* __restrict__ idx, float* __restrict__ val,
                         int* __restrict__ nnz, const float* __restrict__ col_div, const float* __restrict__ col_thr) {
+  pdl_wait();
   constexpr int NW = RC_THREADS / 32;
   extern __shared__ int s_lists[];  // [NW][R][cap]
   __shared__ int s_n[NW][R];
@@ -693,19 +698,17 @@ int radix_hist_launch(int dtype, const void* x, long long A, long long S, long l
     if (dtype == 0) {
       e = cudaFuncSetAttribute(radix_hist_hi_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
-      radix_hist_hi_kernel<float><<<148, HIST_THREADS, smem, stream>>>(static_cast<const float*>(x), A, S, N, s, hist, floor, need);
+      launch(radix_hist_hi_kernel<float>, 148, HIST_THREADS, smem, stream, static_cast<const float*>(x), A, S, N, s, hist, floor, need);
     } else {
       e = cudaFuncSetAttribute(radix_hist_hi_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
-      radix_hist_hi_kernel<__nv_bfloat16>
-          <<<148, HIST_THREADS, smem, stream>>>(static_cast<const __nv_bfloat16*>(x), A, S, N, s, hist, floor, need);
+      launch(radix_hist_hi_kernel<__nv_bfloat16>, 148, HIST_THREADS, smem, stream, static_cast<const __nv_bfloat16*>(x), A, S, N, s, hist, floor, need);
     }
   } else {
     if (dtype == 0)
-      radix_hist_lo_kernel<float><<<148 * 8, 256, 0, stream>>>(static_cast<const float*>(x), A, S, N, s, sel, hist);
+      launch(radix_hist_lo_kernel<float>, 148 * 8, 256, 0, stream, static_cast<const float*>(x), A, S, N, s, sel, hist);
     else
-      radix_hist_lo_kernel<__nv_bfloat16>
-          <<<148 * 8, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), A, S, N, s, sel, hist);
+      launch(radix_hist_lo_kernel<__nv_bfloat16>, 148 * 8, 256, 0, stream, static_cast<const __nv_bfloat16*>(x), A, S, N, s, sel, hist);
   }
   return (int)cudaGetLastError();
 }
@@ -715,7 +718,7 @@ int radix_hi_bins() { return kHiBins; }
 int radix_pick_launch(const unsigned* hist, int nbins, long long k, const long long* sel_in, int level, long long* sel_out,
                       float* thr, const long long* need, cudaStream_t stream) {
   if (nbins <= 0 || nbins > 65536 || (level == 1 && sel_in == nullptr)) return (int)cudaErrorInvalidValue;
-  radix_pick_kernel<<<1, 1024, 0, stream>>>(hist, nbins, k, sel_in, level, sel_out, thr, need);
+  launch(radix_pick_kernel, 1, 1024, 0, stream, hist, nbins, k, sel_in, level, sel_out, thr, need);
   return (int)cudaGetLastError();
 }
 
@@ -745,17 +748,16 @@ int row_compact_launch(int dtype, const void* x, int B, long long N, int cap, in
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     const size_t per_row = (size_t)(RC_THREADS / 32) * cap * 4;
     if (cap <= 256 && B >= 148 * 8)
-      row_compact_cols_kernel<4><<<(B + 3) / 4, RC_THREADS, 4 * per_row, stream>>>(xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
+      launch(row_compact_cols_kernel<4>, (B + 3) / 4, RC_THREADS, 4 * per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
     else
-      row_compact_cols_kernel<1><<<B, RC_THREADS, per_row, stream>>>(xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
+      launch(row_compact_cols_kernel<1>, B, RC_THREADS, per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
     return (int)cudaGetLastError();
   }
   if (dtype == 0)
-    row_compact_kernel<float><<<blocks, RC_THREADS, 0, stream>>>(static_cast<const float*>(x), B, N, cap, idx, val, nnz, thr, col_div, ties,
+    launch(row_compact_kernel<float>, blocks, RC_THREADS, 0, stream, static_cast<const float*>(x), B, N, cap, idx, val, nnz, thr, col_div, ties,
                                                                  tie_quota, col_thr, seg_counts);
   else
-    row_compact_kernel<__nv_bfloat16>
-        <<<blocks, RC_THREADS, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), B, N, cap, idx, val, nnz, thr, col_div, ties,
+    launch(row_compact_kernel<__nv_bfloat16>, blocks, RC_THREADS, 0, stream, static_cast<const __nv_bfloat16*>(x), B, N, cap, idx, val, nnz, thr, col_div, ties,
                                             tie_quota, col_thr, seg_counts);
   return (int)cudaGetLastError();
 }
@@ -773,6 +775,7 @@ __global__ void __launch_bounds__(256)
 jumprelu_window_grad_kernel(const __nv_bfloat16* __restrict__ G, const __nv_bfloat16* __restrict__ S, int B, int F,
                             const float* __restrict__ n, const float* __restrict__ theta, float window, float add_per_hit,
                             int rows_per_block, float* __restrict__ dtheta) {
+  pdl_wait();
   const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
   if (c >= F) return;
   const int r0 = blockIdx.y * rows_per_block, r1 = min(B, r0 + rows_per_block);
@@ -807,7 +810,7 @@ int jumprelu_window_grad_launch(const __nv_bfloat16* G, const __nv_bfloat16* S, 
   if (F % 8 != 0 || B <= 0) return (int)cudaErrorInvalidValue;
   const int rows_per_block = 128;
   dim3 grid((F / 8 + 255) / 256, (B + rows_per_block - 1) / rows_per_block);
-  jumprelu_window_grad_kernel<<<grid, 256, 0, stream>>>(G, S, B, F, n, theta, window, add_per_hit, rows_per_block, dtheta);
+  launch(jumprelu_window_grad_kernel, grid, 256, 0, stream, G, S, B, F, n, theta, window, add_per_hit, rows_per_block, dtheta);
   return (int)cudaGetLastError();
 }
 

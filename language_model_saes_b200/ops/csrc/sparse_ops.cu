@@ -37,6 +37,7 @@ constexpr int DEC_WARPS = 8;
 template <int VPT>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 sparse_decode_kernel(const DecodeParams p, int nseg) {
+  pdl_wait();
   __shared__ float s_red[DEC_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = p.d / 8;  // d % 8 == 0
@@ -120,6 +121,7 @@ sparse_decode_kernel(const DecodeParams p, int nseg) {
 // The segments' losses of a row added up in order: the same sum every time.
 __global__ void __launch_bounds__(256)
 row_loss_kernel(const float* __restrict__ part, int B, int nseg, float* __restrict__ row_loss) {
+  pdl_wait();
   const int row = blockIdx.x * 256 + threadIdx.x;
   if (row >= B) return;
   float s = 0.0f;
@@ -136,11 +138,11 @@ int sparse_decode_launch(const DecodeParams& p, cudaStream_t stream) {
   const int vpt = decode_vpt(p.d), nseg = sparse_decode_segments(p.d);
   const long long blocks = ((long long)p.B * nseg + DEC_WARPS - 1) / DEC_WARPS;
   if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
-  if (vpt == 2) sparse_decode_kernel<2><<<(int)blocks, DEC_WARPS * 32, 0, stream>>>(p, nseg);
-  else sparse_decode_kernel<1><<<(int)blocks, DEC_WARPS * 32, 0, stream>>>(p, nseg);
+  if (vpt == 2) launch(sparse_decode_kernel<2>, (int)blocks, DEC_WARPS * 32, 0, stream, p, nseg);
+  else launch(sparse_decode_kernel<1>, (int)blocks, DEC_WARPS * 32, 0, stream, p, nseg);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && p.label != nullptr && p.row_loss != nullptr) {
-    row_loss_kernel<<<(p.B + 255) / 256, 256, 0, stream>>>(p.row_part, p.B, nseg, p.row_loss);
+    launch(row_loss_kernel, (p.B + 255) / 256, 256, 0, stream, p.row_part, p.B, nseg, p.row_loss);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess || p.label == nullptr || p.dval == nullptr) return (int)e;
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(DACT_THREADS)
 sparse_dact_kernel(const int* __restrict__ idx, int B, int k, int d, int F, const __nv_bfloat16* __restrict__ W,
                    const __nv_bfloat16* dxhat /* may be peer-written: no read-only path */, float* __restrict__ dval, const PeerTable wait_pt,
                    uint32_t epoch, int* status) {
+  pdl_wait();
   extern __shared__ float s_dx[];  // [d]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = d / 8;
@@ -208,7 +211,7 @@ int sparse_dact_launch(const int* idx, int B, int k, int d, int F, const __nv_bf
   int blocks = B < 148 * 8 ? B : 148 * 8;
   PeerTable pt{};
   if (wait != nullptr) pt = *wait;
-  sparse_dact_kernel<<<blocks, DACT_THREADS, (size_t)d * 4, stream>>>(idx, B, k, d, F, W, dxhat, dval, pt, epoch, status);
+  launch(sparse_dact_kernel, blocks, DACT_THREADS, (size_t)d * 4, stream, idx, B, k, d, F, W, dxhat, dval, pt, epoch, status);
   return (int)cudaGetLastError();
 }
 
@@ -220,6 +223,7 @@ mse_loss_grad_kernel(const float* __restrict__ xhat, const __nv_bfloat16* __rest
                      const float* __restrict__ bias, const float* __restrict__ row_weight, int rows, int d,
                      float grad_scale, __nv_bfloat16* __restrict__ dxhat, float* __restrict__ loss_sum,
                      float* __restrict__ row_loss) {
+  pdl_wait();
   __shared__ float s_red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -251,7 +255,7 @@ int mse_loss_grad_launch(const float* xhat, const __nv_bfloat16* label, const fl
                          int rows, int d, float grad_scale, __nv_bfloat16* dxhat, float* loss_sum, float* row_loss,
                          cudaStream_t stream) {
   int blocks = rows < 148 * 8 ? rows : 148 * 8;
-  mse_loss_grad_kernel<<<blocks, 256, 0, stream>>>(xhat, label, bias, row_weight, rows, d, grad_scale, dxhat,
+  launch(mse_loss_grad_kernel, blocks, 256, 0, stream, xhat, label, bias, row_weight, rows, d, grad_scale, dxhat,
                                                    loss_sum, row_loss);
   return (int)cudaGetLastError();
 }
@@ -269,6 +273,7 @@ auxk_loss_grad_kernel(const float* __restrict__ xhat, const float* __restrict__ 
                       const float* __restrict__ row_weight, int rows, int d, float grad_scale, float alpha_host,
                       const float* __restrict__ alpha_factor, __nv_bfloat16* __restrict__ g_main,
                       __nv_bfloat16* __restrict__ g_aux, float* __restrict__ loss_sum, float* __restrict__ aux_sum) {
+  pdl_wait();
   __shared__ float s_red[2][8];
   // alpha_factor (one device float, optional): 0 switches the auxiliary term off without the host knowing, e.g. in a step
   // that has no dead feature
@@ -312,7 +317,7 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
                           float* aux_sum, cudaStream_t stream) {
   int blocks = rows < 148 * 8 ? rows : 148 * 8;
   if (blocks <= 0) return 0;
-  auxk_loss_grad_kernel<<<blocks, 256, 0, stream>>>(xhat, aux_rec, label, bias, row_weight, rows, d, grad_scale, alpha,
+  launch(auxk_loss_grad_kernel, blocks, 256, 0, stream, xhat, aux_rec, label, bias, row_weight, rows, d, grad_scale, alpha,
                                                     alpha_factor, g_main, g_aux, loss_sum, aux_sum);
   return (int)cudaGetLastError();
 }
@@ -321,6 +326,7 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
 // group (row, slot) pairs by feature: counts -> offsets (exclusive scan) -> entries
 // ---------------------------------------------------------------------------------------------
 __global__ void csc_count_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ counts, int* __restrict__ heavy) {
+  pdl_wait();
   if (heavy != nullptr && blockIdx.x == 0 && threadIdx.x == 0) heavy[0] = 0;  // (counted by the scan that follows)
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int f = idx[i];
@@ -362,6 +368,7 @@ __device__ __forceinline__ int block_exclusive_scan_1024(int v, int* s_warp, int
 __global__ void __launch_bounds__(SCAN_THREADS)
 csc_scan_local_kernel(const int* __restrict__ counts, int F, int* __restrict__ offsets, int* __restrict__ block_sums,
                       int* __restrict__ heavy, int heavy_cap) {
+  pdl_wait();
   __shared__ int s_warp[33];
   const int base = blockIdx.x * SCAN_ELEMS + threadIdx.x * 4;
   int c[4];
@@ -386,6 +393,7 @@ csc_scan_local_kernel(const int* __restrict__ counts, int F, int* __restrict__ o
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 csc_scan_sums_kernel(int* __restrict__ block_sums, int nblocks, int* __restrict__ offsets, int F) {
+  pdl_wait();
   __shared__ int s_warp[33];
   __shared__ int s_carry;
   if (threadIdx.x == 0) s_carry = 0;
@@ -406,6 +414,7 @@ csc_scan_sums_kernel(int* __restrict__ block_sums, int nblocks, int* __restrict_
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 csc_scan_add_kernel(const int* __restrict__ block_sums, int F, int* __restrict__ offsets, int* __restrict__ cursor) {
+  pdl_wait();
   const int add = block_sums[blockIdx.x];
   const int base = blockIdx.x * SCAN_ELEMS + threadIdx.x * 4;
 #pragma unroll
@@ -424,6 +433,7 @@ csc_scan_add_kernel(const int* __restrict__ block_sums, int F, int* __restrict__
 constexpr int kOneScanFeatures = 1 << 17;
 __global__ void __launch_bounds__(SCAN_THREADS)
 csc_scan_kernel(const int* __restrict__ counts, int F, int* __restrict__ offsets, int* __restrict__ cursor, int* __restrict__ heavy, int heavy_cap) {
+  pdl_wait();
   __shared__ int s_warp[33];
   const int first = blockIdx.x * SCAN_ELEMS, base = first + threadIdx.x * 4;
   int before = 0;
@@ -459,6 +469,7 @@ csc_scan_kernel(const int* __restrict__ counts, int F, int* __restrict__ offsets
 
 __global__ void csc_fill_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ cursor,
                                 int* __restrict__ entries) {
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int f = idx[i];
     if (f >= 0 && f < F) {
@@ -476,6 +487,7 @@ constexpr int kSmallEntries = 8192, kSmallFeatures = 8192;
 __global__ void __launch_bounds__(SCAN_THREADS)
 csc_small_kernel(const int* __restrict__ idx, int n, int F, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ cursor,
                  int* __restrict__ entries, int* __restrict__ heavy, int heavy_cap) {
+  pdl_wait();
   extern __shared__ int s_cnt[];  // [F]: counts, then cursors
   __shared__ int s_warp[33];
   __shared__ int s_heavy;
@@ -538,7 +550,7 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
   if (n < 0 || n > 2147483647LL || F <= 0) return (int)cudaErrorInvalidValue;  // positions are stored as 32-bit ints
   if (n <= kSmallEntries && F <= kSmallFeatures) {
     if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;
-    csc_small_kernel<<<1, SCAN_THREADS, (size_t)F * sizeof(int), stream>>>(idx, (int)n, F, counts, offsets, cursor, entries, heavy, heavy_cap);
+    launch(csc_small_kernel, 1, SCAN_THREADS, (size_t)F * sizeof(int), stream, idx, (int)n, F, counts, offsets, cursor, entries, heavy, heavy_cap);
     return (int)cudaGetLastError();
   }
   cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)F * sizeof(int), stream);
@@ -548,18 +560,18 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
   int blocks = (int)((n + threads - 1) / threads);
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  csc_count_kernel<<<blocks, threads, 0, stream>>>(idx, n, F, counts, heavy);
+  launch(csc_count_kernel, blocks, threads, 0, stream, idx, n, F, counts, heavy);
   // `block_sums_buf` holds one int per 4096 features
   const int nblocks = (F + SCAN_ELEMS - 1) / SCAN_ELEMS;
   if (F <= kOneScanFeatures && reinterpret_cast<uintptr_t>(counts) % 16 == 0) {
-    csc_scan_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, F, offsets, cursor, heavy, heavy_cap);
+    launch(csc_scan_kernel, nblocks, SCAN_THREADS, 0, stream, counts, F, offsets, cursor, heavy, heavy_cap);
   } else {
     int* block_sums = block_sums_buf;
-    csc_scan_local_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, F, offsets, block_sums, heavy, heavy_cap);
-    csc_scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(block_sums, nblocks, offsets, F);
-    csc_scan_add_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(block_sums, F, offsets, cursor);
+    launch(csc_scan_local_kernel, nblocks, SCAN_THREADS, 0, stream, counts, F, offsets, block_sums, heavy, heavy_cap);
+    launch(csc_scan_sums_kernel, 1, SCAN_THREADS, 0, stream, block_sums, nblocks, offsets, F);
+    launch(csc_scan_add_kernel, nblocks, SCAN_THREADS, 0, stream, block_sums, F, offsets, cursor);
   }
-  csc_fill_kernel<<<blocks, threads, 0, stream>>>(idx, n, F, cursor, entries);
+  launch(csc_fill_kernel, blocks, threads, 0, stream, idx, n, F, cursor, entries);
   return (int)cudaGetLastError();
 }
 
@@ -567,9 +579,9 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
 int exclusive_scan_launch(const int* counts, int n, int* offsets, int* block_sums_buf, cudaStream_t stream) {
   if (n <= 0) return (int)cudaErrorInvalidValue;
   const int nblocks = (n + SCAN_ELEMS - 1) / SCAN_ELEMS;
-  csc_scan_local_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(counts, n, offsets, block_sums_buf, nullptr, 0);
-  csc_scan_sums_kernel<<<1, SCAN_THREADS, 0, stream>>>(block_sums_buf, nblocks, offsets, n);
-  csc_scan_add_kernel<<<nblocks, SCAN_THREADS, 0, stream>>>(block_sums_buf, n, offsets, nullptr);
+  launch(csc_scan_local_kernel, nblocks, SCAN_THREADS, 0, stream, counts, n, offsets, block_sums_buf, nullptr, 0);
+  launch(csc_scan_sums_kernel, 1, SCAN_THREADS, 0, stream, block_sums_buf, nblocks, offsets, n);
+  launch(csc_scan_add_kernel, nblocks, SCAN_THREADS, 0, stream, block_sums_buf, n, offsets, nullptr);
   return (int)cudaGetLastError();
 }
 
@@ -837,6 +849,7 @@ int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream) {
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 colsum_bf16_kernel(const __nv_bfloat16* __restrict__ a, int rows, int d, int rows_per_block, float* __restrict__ out) {
+  pdl_wait();
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = min(rows, r0 + rows_per_block);
   for (int c = blockIdx.x * 256 + threadIdx.x; c < d; c += gridDim.x * 256) {
@@ -851,7 +864,7 @@ int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cuda
   if (e != cudaSuccess) return (int)e;
   const int rows_per_block = 64;
   dim3 grid((d + 255) / 256, (rows + rows_per_block - 1) / rows_per_block);
-  colsum_bf16_kernel<<<grid, 256, 0, stream>>>(a, rows, d, rows_per_block, out);
+  launch(colsum_bf16_kernel, grid, 256, 0, stream, a, rows, d, rows_per_block, out);
   return (int)cudaGetLastError();
 }
 
@@ -867,6 +880,7 @@ int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cuda
 constexpr int kSerialPartials = 64;  // up to so many partial sums are added up one after the other
 __global__ void __launch_bounds__(256)
 colsum_adam_kernel(const ColsumAdamParams p) {
+  pdl_wait();
   __shared__ float s_sum[8][256];
   __shared__ int s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -969,6 +983,7 @@ colsum_adam_kernel(const ColsumAdamParams p) {
 // As tensor operations (comparison, product, sum): 86 + 127 + 28 us; here 33.
 __global__ void __launch_bounds__(256)
 mask_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ mask, long long ld, int rows, int d, int rows_per_block, float* __restrict__ part) {
+  pdl_wait();
   __shared__ float s_sum[8][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col0 = blockIdx.x * 256, col = col0 + lane * 8;
@@ -1016,7 +1031,7 @@ int mask_colsum_launch(__nv_bfloat16* g, const __nv_bfloat16* mask, long long ld
   if (d % 8 != 0 || ld % 8 != 0 || rows < 0 || row_blocks < 1) return (int)cudaErrorInvalidValue;
   if (d == 0) return 0;
   const int rpb = (rows + row_blocks - 1) / row_blocks;
-  mask_colsum_kernel<<<dim3((d + 255) / 256, row_blocks), 256, 0, stream>>>(g, mask, ld, rows, d, rpb, part);
+  launch(mask_colsum_kernel, dim3((d + 255) / 256, row_blocks), 256, 0, stream, g, mask, ld, rows, d, rpb, part);
   return (int)cudaGetLastError();
 }
 
@@ -1036,7 +1051,7 @@ int colsum_adam_launch(ColsumAdamParams p, int col_blocks, cudaStream_t stream) 
   if (p.n_seg == 0 && p.loss_out == nullptr) return 0;
   const int rb = p.n_seg > 0 ? colsum_adam_row_blocks(col_blocks, p.rows) : 1;
   p.rows_per_block = (p.rows + rb - 1) / rb;
-  colsum_adam_kernel<<<dim3(p.n_seg > 0 ? col_blocks : 1, rb), 256, 0, stream>>>(p);
+  launch(colsum_adam_kernel, dim3(p.n_seg > 0 ? col_blocks : 1, rb), 256, 0, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -1050,6 +1065,7 @@ __global__ void __launch_bounds__(256)
 adam_flat_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                  long long n, AdamHyper h, const float* __restrict__ grad_mul, __nv_bfloat16* __restrict__ shadow,
                  float* __restrict__ grad_sq_sum, int update, const int* __restrict__ status) {
+  pdl_wait();
   __shared__ float s_gsq[8];
   if (status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;  // see sparse_grad_adam_kernel
   const float gmul = grad_mul != nullptr ? *grad_mul : 1.0f;
@@ -1102,7 +1118,7 @@ int adam_flat_launch(float* p, const float* g, float* m, float* v, long long n, 
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) blocks = 1;
   auto kern = wide ? adam_flat_kernel<4> : adam_flat_kernel<1>;
-  kern<<<(int)blocks, 256, 0, stream>>>(p, g, m, v, n, h, grad_mul, shadow, grad_sq_sum, update, status);
+  launch(kern, (int)blocks, 256, 0, stream, p, g, m, v, n, h, grad_mul, shadow, grad_sq_sum, update, status);
   return (int)cudaGetLastError();
 }
 

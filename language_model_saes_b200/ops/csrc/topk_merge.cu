@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32)
 topk_merge_kernel(const float* cand_val, const int* cand_idx, int M, int C, int k,  // may be peer-written: no read-only path
                   const float* __restrict__ gate, int own_lo, int own_hi, int emit_gated,
                   int* __restrict__ out_idx, float* __restrict__ out_val, const MergeComm comm) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -187,7 +188,7 @@ int topk_merge_launch(const float* cand_val, const int* cand_idx, int M, int C, 
   if (e != cudaSuccess) return (int)e;
   int blocks = (M + warps - 1) / warps;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  kern<<<blocks, warps * 32, smem, stream>>>(cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
+  launch(kern, blocks, warps * 32, smem, stream, cand_val, cand_idx, M, C, k, gate, own_lo, own_hi,
                                                   emit_gated, out_idx, out_val, comm);
   return (int)cudaGetLastError();
 }
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(RT_THREADS, 5)
 row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N, int k,
                 const float* __restrict__ gate, const uint8_t* __restrict__ alive, const float* __restrict__ maxima, long long ld_maxima, int vec,
                 int* __restrict__ out_idx, float* __restrict__ out_val) {
+  pdl_wait();
   const int row = blockIdx.x;
   if (row >= M) return;
   const __nv_bfloat16* hrow = H + (long long)row * ldh;
@@ -547,6 +549,7 @@ template <typename T>
 __global__ void __launch_bounds__(RT_THREADS)
 row_select_kernel(const T* __restrict__ H, long long ldh, const float* __restrict__ maxima, long long ld_maxima, int M, int N, int k,
                   const float* __restrict__ gate, int sorted, int* __restrict__ out_idx, float* __restrict__ out_val) {
+  pdl_wait();
   __shared__ unsigned short s_group[RS_WARPS][RS_GROUPS];
   __shared__ unsigned s_key[RS_WARPS][RS_CAND];
   __shared__ int s_col[RS_WARPS][RS_CAND];
@@ -752,8 +755,8 @@ int row_select_launch(const __nv_bfloat16* H16, const float* H32, long long ldh,
   if ((H16 != nullptr) == (H32 != nullptr) || k < 1 || k > RS_MAX_K || N % 8 != 0 || N > 65535 * 32 || ldh % 8 != 0 || at % 16 != 0) return (int)cudaErrorInvalidValue;
   if (M <= 0) return 0;
   const int blocks = (M + RS_WARPS - 1) / RS_WARPS;
-  if (H16 != nullptr) row_select_kernel<__nv_bfloat16><<<blocks, RT_THREADS, 0, stream>>>(H16, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
-  else row_select_kernel<float><<<blocks, RT_THREADS, 0, stream>>>(H32, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
+  if (H16 != nullptr) launch(row_select_kernel<__nv_bfloat16>, blocks, RT_THREADS, 0, stream, H16, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
+  else launch(row_select_kernel<float>, blocks, RT_THREADS, 0, stream, H32, ldh, maxima, ld_maxima, M, N, k, gate, sorted, out_idx, out_val);
   return (int)cudaGetLastError();
 }
 
@@ -761,8 +764,8 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
                     const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream) {
   const bool vec = N % 8 == 0 && ldh % 8 == 0 && reinterpret_cast<uintptr_t>(H) % 16 == 0 && reinterpret_cast<uintptr_t>(gate) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(alive) % 8 == 0;
-  if (maxima != nullptr) row_topk_kernel<true><<<M, RT_THREADS, 0, stream>>>(H, ldh, M, N, k, gate, alive, maxima, ld_maxima, vec ? 1 : 0, out_idx, out_val);
-  else row_topk_kernel<false><<<M, RT_THREADS, 0, stream>>>(H, ldh, M, N, k, gate, alive, nullptr, 0, vec ? 1 : 0, out_idx, out_val);
+  if (maxima != nullptr) launch(row_topk_kernel<true>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, maxima, ld_maxima, vec ? 1 : 0, out_idx, out_val);
+  else launch(row_topk_kernel<false>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, nullptr, 0, vec ? 1 : 0, out_idx, out_val);
   return (int)cudaGetLastError();
 }
 
@@ -1156,11 +1159,13 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
 template <bool ESTIMATE>
 __global__ void __launch_bounds__(RT_THREADS, 5)
 topk_dense_kernel(const TopkDenseParams p) {
+  pdl_wait();
   topk_dense_row<ESTIMATE>(p, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(RT_THREADS, 5)
 topk_dense_rows_kernel(const TopkDenseParams p) {
+  pdl_wait();
   const int n = p.rows[0];
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     topk_dense_row<false>(p, p.rows[1 + i]);
@@ -1175,7 +1180,7 @@ int topk_dense_launch(const float* h, const float* bias, const float* norm, int 
   p.h = h; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
   p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
                           reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  topk_dense_kernel<false><<<B, RT_THREADS, 0, stream>>>(p);
+  launch(topk_dense_kernel<false>, B, RT_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -1189,7 +1194,7 @@ int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, cons
   TopkDenseParams p = {};
   p.lo = lo; p.x = x; p.W = W; p.xn = xn; p.top = top; p.status = status; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
   p.vec = N % 8 == 0 && ((reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  topk_dense_kernel<true><<<B, RT_THREADS, 0, stream>>>(p);
+  launch(topk_dense_kernel<true>, B, RT_THREADS, 0, stream, p);
   RowsProductParams r = {};
   r.A = x; r.B = W; r.C = h; r.N = N; r.K = K; r.rows = todo; r.max_rows = B;
   const int e = rows_product_launch(r, false, stream);
@@ -1198,7 +1203,7 @@ int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, cons
   p.h = h;
   p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
                           reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  topk_dense_rows_kernel<<<B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream>>>(p);
+  launch(topk_dense_rows_kernel, B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 

@@ -47,6 +47,7 @@ static_assert(WG_SMEM <= 232448, "shared memory of one CTA exceeds 227 KB");
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WG_THREADS, 1)
 window_grad_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_g,
                         const __grid_constant__ CUtensorMap tmap_s, const WindowGradParams p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + WG_BAR_OFF);
@@ -239,7 +240,7 @@ int window_grad_gemm_launch(const CUtensorMap& tw, const CUtensorMap& tg, const 
   if (e != cudaSuccess) return (int)e;
   const long long tiles = (long long)((p.F + 255) / 256) * ((p.B + WG_TOKENS - 1) / WG_TOKENS);
   const int pairs = (int)(tiles < 74 ? tiles : 74);
-  window_grad_gemm_kernel<<<2 * pairs, WG_THREADS, WG_SMEM, stream>>>(tw, tg, ts, p);
+  launch(window_grad_gemm_kernel, 2 * pairs, WG_THREADS, WG_SMEM, stream, tw, tg, ts, p);
   return (int)cudaGetLastError();
 }
 
