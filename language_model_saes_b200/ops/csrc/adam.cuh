@@ -12,4 +12,22 @@ __device__ __forceinline__ void adam_elem(float& p, float& m, float& v, float g,
   p -= (h.lr / h.bias_correction1) * (m / denom);
 }
 
+// The same with the factors worked out once, for the kernels that stream rows of parameters.
+struct AdamConst {
+  float b1, b2, c1, c2, inv_bc2, step, eps;
+};
+
+__device__ __forceinline__ void adam_update(float& p, float& m, float& v, float g, const AdamConst& h) {
+  m = fmaf(h.b1, m, h.c1 * g);
+  v = fmaf(h.b2, v, h.c2 * g * g);
+  p = fmaf(-h.step, m / fmaf(sqrtf(v), h.inv_bc2, h.eps), p);
+}
+
+// One row of a parameter or moment matrix to shared memory, on a bulk copy.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
 }  // namespace lmsae

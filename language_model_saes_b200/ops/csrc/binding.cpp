@@ -1457,6 +1457,7 @@ std::map<std::string, std::vector<int64_t>> bounds_report() {
   std::map<std::string, std::vector<int64_t>> out;
   const std::pair<const char*, int (*)(int*)> units[] = {  // every file whose kernels check an index
       {"sparse_ops.cu", lmsae::bounds_fetch_sparse_ops}, {"comm_ops.cu", lmsae::bounds_fetch_comm_ops}, {"grad_adam.cu", lmsae::bounds_fetch_grad_adam},
+      {"grad_adam_both.cu", lmsae::bounds_fetch_grad_adam_both},
       {"clt_ops.cu", lmsae::bounds_fetch_clt_ops}, {"dense_decode.cu", lmsae::bounds_fetch_dense_decode},
       {"lorsa_ops.cu", lmsae::bounds_fetch_lorsa_ops}};
   for (const auto& [name, fetch] : units) {

@@ -27,6 +27,7 @@
 //   12 + 78 matrices of 24576 x 768 (CLT)    8.62 + 3.05 -> 7.59 ms  (44 GB: 5.8 TB/s)
 //   24576 rows of 768, both sides, k 50      222 + 155   -> 182 us
 //   32768 rows of 2048, both sides, k 128    1103 + 590  -> 819 us (16 entries a row: bound by the gathers, 4.3 GB)
+#include "adam.cuh"
 #include "gather.cuh"
 #include "kernels.h"
 
@@ -35,12 +36,6 @@ namespace lmsae {
 LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_grad_adam)
 
 namespace {
-
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 
 template <int W>
 __device__ __forceinline__ void group_sync(int gid) {
@@ -71,16 +66,6 @@ __device__ __forceinline__ bool group_all(int gid, bool ok) {
         : "memory");
     return r != 0;
   }
-}
-
-struct AdamConst {
-  float b1, b2, c1, c2, inv_bc2, step, eps;
-};
-
-__device__ __forceinline__ void adam_update(float& p, float& m, float& v, float g, const AdamConst& h) {
-  m = fmaf(h.b1, m, h.c1 * g);
-  v = fmaf(h.b2, v, h.c2 * g * g);
-  p = fmaf(-h.step, m / fmaf(sqrtf(v), h.inv_bc2, h.eps), p);
 }
 
 // Position of a thread in its group and the group's slice of shared memory.
@@ -599,6 +584,7 @@ bool grad_adam_rows_supported(const GradAdamParams& p) {
 int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream) {
   if (!grad_adam_rows_supported(p) || (p.dact_mode != 0 && (p.WD == nullptr || p.dact_out == nullptr))) return (int)cudaErrorInvalidValue;
   if (p.f_end <= p.f_begin) return 0;
+  if (grad_adam_both_supported(p)) return grad_adam_both_launch(p, stream);
   const int d = p.d;
   cudaError_t e;
   if (d <= 1024) {

@@ -111,6 +111,7 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 int bounds_fetch_sparse_ops(int* out);
 int bounds_fetch_comm_ops(int* out);
 int bounds_fetch_grad_adam(int* out);
+int bounds_fetch_grad_adam_both(int* out);
 int bounds_fetch_clt_ops(int* out);
 int bounds_fetch_dense_decode(int* out);
 int bounds_fetch_lorsa_ops(int* out);
@@ -218,6 +219,8 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
 int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream);
 bool grad_adam_rows_supported(const GradAdamParams& p);
 int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream);
+bool grad_adam_both_supported(const GradAdamParams& p);
+int grad_adam_both_launch(const GradAdamParams& p, cudaStream_t stream);
 int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cudaStream_t stream);
 // Column sums of bf16 matrices [rows, d] as bias gradients, Adam on the biases, and the step's mean loss (sparse_ops.cu).
 constexpr int kMaxColsumSegs = 16;

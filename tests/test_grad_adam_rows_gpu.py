@@ -104,3 +104,39 @@ def test_rows_whose_copies_were_not_waited_for_stay_as_they_are(d, sides, mode):
     run()  # the next launch works as ever
     K.check_status(torch.device(DEV))
     assert not torch.equal((t["WD"] if sides != "encoder" else t["WE"]).cpu(), cpu["WD"] if sides != "encoder" else cpu["WE"])
+
+
+@pytest.mark.parametrize("d", [4, 64, 124, 128, 132, 256, 260, 508, 512, 516])
+@pytest.mark.parametrize("F,B,f_range", [(230, 200, None), (40, 200, None), (9000, 300, None), (230, 200, (1, 117))])
+def test_both_sides_in_one_pass_match_the_plain_statement(d, F, B, f_range):
+    """Widths at which the groups of warps change, one group per row and several rows per draw, a range of the features."""
+    k = 6
+    cpu = _case(d, F, B, k, seed=d + F)
+    if F == 40:  # all rows shared by a CTA, lists of 32 and a few more entries with gaps
+        cpu["idx"][:, 1:] = torch.arange(B).unsqueeze(1) % 34 + torch.arange(1, k)
+    if F == 9000:
+        cpu["idx"][0::3] = -1
+    gpu = {n: t.clone().to(DEV) for n, t in cpu.items()}
+    lo = f_range[0] if f_range else 0
+
+    def run(t, step):
+        groups = K.FeatureGroups(F, B * k, t["idx"].device).build(t["idx"])
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], t["WD"], t["mD"][lo:], t["vD"][lo:], t["WD16"], t["WE"], t["mE"][lo:], t["vE"][lo:],
+                           t["WE16"], t["b"], t["mb"][lo:], t["vb"][lo:], t["n"], t["gsq"].add_(0.5) if F == 230 else None, None, 1e-3, 0.9, 0.999, 1e-8,
+                           step, True, f_range, state_f0=lo, extra=(t["row_of"], t["xD"], t["xE"], t["xb"]) if F != 40 else None,
+                           wd_self_scale=t["scale"] if F != 40 else None, dact_mode=1)  # fmt: skip
+        return groups
+
+    for step in (1, 2):
+        run(cpu, step)
+        groups = run(gpu, step)
+        K.check_status(torch.device(DEV))
+        assert groups.sched.tolist() == [0, 0]  # ready for the next launch
+    _compare(cpu, gpu, ["dact", "WD", "mD", "vD", "WE", "mE", "vE", "b", "mb", "vb", "n"], d)
+    for n, m in (("WD16", "WD"), ("WE16", "WE")):
+        assert torch.equal(gpu[n].float(), gpu[m].to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("d", [64, 512])
+def test_one_pass_rows_whose_copies_were_not_waited_for_stay_as_they_are(d):
+    test_rows_whose_copies_were_not_waited_for_stay_as_they_are(d, "both", 1)
