@@ -277,7 +277,7 @@ void fp32_gemm(const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& 
     const CUtensorMap tb = make_bf16_tile_map(Bs.data_ptr(), n, parts * kp, 128);
     if (ends)
       check_cuda(lmsae::fp32_ends_launch(ta, tb, (int)M, (int)n, (int)K, (int)kp, na->data_ptr<float>(), nb_n, bias_n, gate_n,
-                                         reinterpret_cast<__nv_bfloat16*>(C.data_ptr()) + n0, N, status.data_ptr<int>(), stream),
+                                         reinterpret_cast<__nv_bfloat16*>(C.data_ptr()) + n0, N, status.data_ptr<int>(), nullptr, 0, stream),
                  "fp32_ends launch");
     else
       check_cuda(lmsae::fp32_gemm_launch(ta, tb, A.data_ptr<float>(), Bn, (int)M, (int)n, (int)K, (int)kp, fa, fb, C.data_ptr<float>() + n0, N,
@@ -320,6 +320,68 @@ void topk_estimate(const Tensor& lo, const Tensor& h, const Tensor& x, const Ten
                                          opt_ptr<const float>(bias), opt_ptr<const float>(norm), (int)h.size(0), (int)h.size(1), (int)k,
                                          status.data_ptr<int>(), todo.data_ptr<int>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
              "topk_estimate launch");
+}
+
+// out = topk(relu((x W^T + bias) * norm)) / norm per row, dense fp32 [B, F], for x [B, K] and W [F, K]: one fp16 product proposes; rows that it leaves
+// too much of in question are proposed for again by three bf16 products where they are more than an eighth of all rows (that is decided on the device:
+// the kernels leave at once elsewhere), and what is still too much is multiplied in order. The parts of W take `workspace` bytes at most.
+void topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, int64_t workspace,
+                 const Tensor& out) {
+  for (const Tensor* t : {&x, &W, &out}) { CHECK_T(*t, torch::kFloat32); }
+  TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.size(1) == W.size(1) && out.dim() == 2 && out.size(0) == x.size(0) && out.size(1) == W.size(0), "x [B,K], W [F,K], out [B,F]");
+  const int64_t B = x.size(0), F = W.size(0), K = x.size(1), kp = (K + 63) / 64 * 64;
+  TORCH_CHECK(B > 0 && F > 0 && K > 0 && K % 4 == 0 && K <= lmsae::kEstimateMaxK && B < INT_MAX - 256 && F < INT_MAX - 256 && k >= 1, "unsupported sizes");
+  for (const auto* t : {&bias, &norm}) {
+    if (t->has_value()) { CHECK_T(**t, torch::kFloat32); TORCH_CHECK((*t)->numel() == F); }
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  const auto f32 = x.options(), b16 = x.options().dtype(torch::kBFloat16), i32 = x.options().dtype(torch::kInt32);
+  int64_t step = F;  // four bytes an element of W in pieces of whole tiles
+  if (F * kp * 4 > workspace) step = std::max<int64_t>(1, workspace / (kp * 4 * 256)) * 256;
+  step = std::min(step, F);
+  const Tensor xs = torch::empty({B, 2 * kp}, b16), ws = torch::empty({step, 2 * kp}, b16);  // an fp16 part each, or two bf16 parts
+  const Tensor norms = torch::empty({3 * B + 2 * F + 8}, f32);  // norms and scales of both operands, and what rounding took of a row of x
+  float* xn = norms.data_ptr<float>();
+  float* xs_scale = xn + B;
+  float* lost = xs_scale + B;
+  float* wn = lost + B + (4 - 3 * B % 4) % 4;
+  float* w_scale = wn + F + (4 - F % 4) % 4;
+  // zeroed: status [4], top [4] and the columns' widths, the rows that are wide, those that are left over
+  const int64_t widths = 4 + (F + 1) / 2;
+  const Tensor words = torch::zeros({4 + widths + 2 * (1 + B)}, i32);
+  int* status = words.data_ptr<int>();
+  uint32_t* top = reinterpret_cast<uint32_t*>(status + 4);
+  int *wide = status + 4 + widths, *todo = wide + 1 + B;
+  const int wide_limit = (int)(B / 8);
+  const Tensor h = torch::empty({B, F}, f32);  // lower ends, then products of the rows that are left over
+  auto* lo = reinterpret_cast<__nv_bfloat16*>(h.data_ptr());
+  const int64_t ld_maxima = (F + 255) / 256 * 8;  // of 32 columns each
+  const Tensor maxima = torch::empty({B, ld_maxima}, f32);
+  float* maxima_p = maxima.data_ptr<float>();
+  const float *xp = x.data_ptr<float>(), *Wp = W.data_ptr<float>(), *bias_p = opt_ptr<const float>(bias), *norm_p = opt_ptr<const float>(norm);
+  auto* xs_p = reinterpret_cast<__nv_bfloat16*>(xs.data_ptr());
+  auto* ws_p = reinterpret_cast<__nv_bfloat16*>(ws.data_ptr());
+  const CUtensorMap tx1 = make_bf16_tile_map(xs_p, B, kp, 128), tx2 = make_bf16_tile_map(xs_p, B, 2 * kp, 128);
+  for (int64_t n0 = 0; n0 < F; n0 += step) {
+    const int64_t n = std::min(step, F - n0);
+    const float *bn = bias_p ? bias_p + n0 : nullptr, *gn = norm_p ? norm_p + n0 : nullptr;
+    check_cuda(lmsae::half_rows_launch(xp, n0 == 0 ? (int)B : 0, reinterpret_cast<__half*>(xs_p), xn, xs_scale, lost, Wp + n0 * K, (int)n, reinterpret_cast<__half*>(ws_p),
+                                       wn + n0, w_scale + n0, (int)K, (int)kp, reinterpret_cast<uint16_t*>(top + 4) + n0, top, bn, gn, stream), "half_rows launch");
+    check_cuda(lmsae::half_ends_launch(tx1, make_bf16_tile_map(ws_p, n, kp, 128), (int)B, (int)n, (int)K, (int)kp, xn, xs_scale, lost, top, wn + n0, w_scale + n0, bn, gn,
+                                       lo + n0, F, maxima_p + n0 / 32, ld_maxima, status, stream), "half_ends launch");
+  }
+  check_cuda(lmsae::topk_narrow_launch(lo, maxima_p, ld_maxima, xp, Wp, xn, lost, top, (int)K, bias_p, norm_p, (int)B, (int)F, (int)k, status, wide, out.data_ptr<float>(), stream),
+             "topk_narrow launch");
+  check_cuda(lmsae::split_bf16_if_launch(xp, (int)B, (int)K, (int)kp, xs_p, wide, wide_limit, stream), "split launch");
+  for (int64_t n0 = 0; n0 < F; n0 += step) {
+    const int64_t n = std::min(step, F - n0);
+    check_cuda(lmsae::split_bf16_if_launch(Wp + n0 * K, (int)n, (int)K, (int)kp, ws_p, wide, wide_limit, stream), "split launch");
+    check_cuda(lmsae::fp32_ends_launch(tx2, make_bf16_tile_map(ws_p, n, 2 * kp, 128), (int)B, (int)n, (int)K, (int)kp, xn, wn + n0, bias_p ? bias_p + n0 : nullptr,
+                                       norm_p ? norm_p + n0 : nullptr, lo + n0, F, status, wide, wide_limit, stream), "fp32_ends launch");
+  }
+  check_cuda(lmsae::topk_wide_launch(lo, h.data_ptr<float>(), xp, Wp, xn, lost, top, (int)K, bias_p, norm_p, (int)B, (int)F, (int)k, status, wide, wide_limit, todo,
+                                     out.data_ptr<float>(), stream), "topk_wide launch");
 }
 
 // out [B, d] = acts [B, F] @ W [F, d], fp32. Rows of at most `most` non-zeros are gathered. todo: int32 [2 + B + tiles], zeroed; part: fp32
@@ -1521,6 +1583,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_select", &row_select);
   m.def("row_select_fits", &row_select_fits);
   m.def("topk_dense", &topk_dense);
+  m.def("topk_encode", &topk_encode);
   m.def("topk_estimate", &topk_estimate);
   m.def("fp32_gemm", &fp32_gemm);
   m.def("dense_decode", &dense_decode);

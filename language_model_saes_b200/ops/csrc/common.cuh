@@ -373,6 +373,9 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool a_mn_m
          | ((uint32_t)(M >> 4) << 24); // M / 16
 }
 
+// The same for fp16 x fp16.
+__host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N) { return make_idesc_bf16(M, N) & ~((1u << 7) | (1u << 10)); }
+
 // ---- misc ------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

@@ -33,4 +33,12 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) {
 // The norms are rounded up by 5 % where they are made, which covers their own rounding and K 2^-24 << 1.
 __host__ __device__ __forceinline__ float estimate_rel(int K) { return ((float)K * 2.1f + 320.0f) * 5.9604645e-8f; }
 
+// The same for one fp16 part an operand, its row scaled so that the largest magnitude is in [2^14, 2^15) (half_rows_kernel): 2.1 K and 128 as
+// above (the accumulations are those of one product), 8 for the product of what the two operands lost (2^-11 of each at most), and
+// to that what they lost itself, as it was measured: `lost` of the row and the largest of all columns.
+__host__ __device__ __forceinline__ float estimate_rel_half(int K) { return ((float)K * 2.1f + 136.0f) * 5.9604645e-8f; }
+__device__ __forceinline__ float half_rel(float rel, float lost, const uint32_t* most_lost) {
+  return 1.000001f * (rel + lost + __uint_as_float(*most_lost));
+}
+
 }  // namespace lmsae

@@ -18,8 +18,14 @@
 // three products (m.h, h.m, h.h), and instead of the estimate h the epilogue stores a lower end of the activation
 //     lo = (h - e + bias) * gate,   e = rel * xn * wn >= the error of h   (xn, wn the rows' 2-norms, rel: estimate_rel)
 // rounded down to bf16, NaN where the bound says nothing. Bias, gate and rounding are monotone, so that lo encloses the activation of the
-// sum in order wherever that is positive; the upper end is at most lo + 2^-7 |lo| + 2 e gate. Half the products and half the bytes:
-// 4096 x 24576 x 768: 632 + 42 (split) -> 291 + 31 us.
+// sum in order wherever that is positive; the upper end is at most lo + 2^-7 |lo| + 2 e gate. What a column has of its own comes through shared
+// memory, a tile ahead; read from global memory where it was used it kept the epilogue at 13000 cycles a tile, twice what one product takes.
+//
+// ONE TERM: the first proposal of the TopK encoder. One fp16 part an operand (half_rows_kernel), every row scaled to the top of fp16's range, and what
+// rounding took of a row measured and not bounded: 1.9e-4 of its norm as a rule, 4.9e-4 at most. The bound is five times as wide as with two
+// bf16 parts at a third of the operations. The largest end of every 32 columns goes along, so that the selection need not read the ends.
+// 4096 x 24576 x 768: two parts and three products 24 + 7 + 315 us -> 37 + 163 us. Bound by the epilogue (201 MB of ends), the MMAs take 92.
+#include <cuda_fp16.h>
 #include "fp32_exact.cuh"
 #include "kernels.h"
 
@@ -33,7 +39,8 @@ constexpr int FG_HALF_BYTES = 128 * FG_BK * 2;
 constexpr int FG_STAGE_BYTES = 2 * FG_HALF_BYTES;  // this CTA's 128 rows of A and 128 of the 256 rows of B
 constexpr int FG_BAR_OFF = FG_STAGES * FG_STAGE_BYTES;
 constexpr int FG_STORE_OFF = (FG_BAR_OFF + (2 * FG_STAGES + 4) * 8 + 8 + 15) / 16 * 16;  // ENDS: 32 rows x 32 columns on their way to whole sectors, per epilogue warp
-constexpr int FG_SMEM = FG_STORE_OFF + 8 * 2048 + 1024;
+constexpr int FG_COL_OFF = FG_STORE_OFF + 8 * 2048;  // ENDS: what the tile's 256 columns have of their own, for two tiles in turn
+constexpr int FG_SMEM = FG_COL_OFF + 2 * 256 * 16 + 1024;
 
 __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -46,9 +53,9 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
 
 // part of A / B (0 high, 1 middle, 2 low) of the t-th product
 template <int TERMS>
-__device__ __forceinline__ int part_a(int t) { return TERMS == 6 ? (0x201100 >> (4 * (5 - t))) & 15 : t == 0; }
+__device__ __forceinline__ int part_a(int t) { return TERMS == 1 ? 0 : TERMS == 6 ? (0x201100 >> (4 * (5 - t))) & 15 : t == 0; }
 template <int TERMS>
-__device__ __forceinline__ int part_b(int t) { return TERMS == 6 ? (0x021010 >> (4 * (5 - t))) & 15 : t == 1; }
+__device__ __forceinline__ int part_b(int t) { return TERMS == 1 ? 0 : TERMS == 6 ? (0x021010 >> (4 * (5 - t))) & 15 : t == 1; }
 
 // dst [rows][PARTS][kp] bf16 = the parts of src [rows][K], zeros behind K; flags[1 + r] = 1 and zeros where a value does not fit, and
 // then flags[0] != 0. For lower ends, all optional: norm[r], at least the row's 2-norm and at most 10 % above it; wide[r], at least
@@ -65,8 +72,9 @@ struct SplitBounds {
 template <int PARTS>
 __global__ void __launch_bounds__(256)
 split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_bfloat16* __restrict__ dst, int* __restrict__ flags,
-                  const SplitBounds b) {
+                  const SplitBounds b, const int* wide, int wide_limit) {
   pdl_wait();
+  if (wide != nullptr && wide[0] <= wide_limit) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float most = 0.0f;
   for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
@@ -95,7 +103,7 @@ split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_b
         *reinterpret_cast<uint2*>(o + q * kp + c) = make_uint2(pack_bf16x2(p[q][0], p[q][1]), pack_bf16x2(p[q][2], p[q][3]));
     }
     bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) {
+    if (lane == 0 && flags != nullptr) {
       flags[1 + r] = bad ? 1 : 0;
       if (bad) flags[0] = 1;
     }
@@ -120,31 +128,119 @@ split_bf16_kernel(const float* __restrict__ src, int rows, int K, int kp, __nv_b
   if (b.top != nullptr && lane == 0 && most > 0.0f) atomicMax(b.top, __float_as_uint(most));
 }
 
+// One fp16 part of the rows of A and of B, scaled by the power of two that brings a row's largest magnitude to [2^14, 2^15):
+// dst [rows][kp], zeros behind K, scale[r] the factor that undoes it. What is below 2^-14 then is dropped. norm, wide, top as above (norm at
+// most 0.2 % above the 2-norm); a row whose norm is infinite is zeros. lost: at least the 2-norm of what rounding took over that of the row, of
+// every row of A, and bits of the largest of all rows of B in top[2].
+struct HalfRows {
+  const float* src;
+  int rows;
+  __half* dst;
+  float *norm, *scale, *lost;
+};
+__global__ void __launch_bounds__(256)
+half_rows_kernel(const HalfRows a, const HalfRows b, int K, int kp, const SplitBounds bounds) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float most = 0.0f, most_lost = 0.0f;
+  for (int i = blockIdx.x * 8 + warp; i < a.rows + b.rows; i += gridDim.x * 8) {
+    const bool is_b = i >= a.rows;
+    const HalfRows& m = is_b ? b : a;
+    const int r = is_b ? i - a.rows : i;
+    const float* s = m.src + (size_t)r * K;
+    unsigned top = 0u;
+    float sq = 0.0f;
+    for (int c = lane * 4; c < K; c += 128) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(s + c));
+      const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        top = max(top, __float_as_uint(x[j]) & 0x7fffffffu);
+        sq = fmaf(x[j], x[j], sq);
+      }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    sq = warp_sum(sq);
+    bool fits = top == 0u || (top >= 0x2b800000u && top < 0x4e800000u);  // 2^-40, 2^30
+    const float gate = is_b && bounds.gate != nullptr ? bounds.gate[r] : 1.0f;
+    if (is_b && bounds.bias != nullptr) fits &= (__float_as_uint(bounds.bias[r]) & 0x7fffffffu) < 0x65000000u;  // 2^75
+    fits &= __float_as_uint(gate) < 0x58800000u;  // 2^50 (and no sign)
+    const int shift = fits && top != 0u ? 14 + 127 - (int)(top >> 23) : 0;
+    const float up = __uint_as_float((unsigned)(127 + shift) << 23);
+    if (lane == 0) {
+      const float n = !fits ? __uint_as_float(0x7f800000u) : top == 0u ? 0.0f : 1.001f * sqrtf(sq);
+      m.norm[r] = n;
+      m.scale[r] = __uint_as_float((unsigned)(127 - shift) << 23);
+      if (is_b) {
+        const float w = mul_up(n, gate);
+        if (fits) most = fmaxf(most, w);
+        bounds.wide[r] = fits ? (uint16_t)((__float_as_uint(w) + 0xffffu) >> 16) : (uint16_t)0x7f80u;
+        const unsigned gb = __float_as_uint(gate) & 0x7fffffffu;
+        if (gb == 0u || gb > 0x7f800000u) bounds.top[1] = 1u;
+      }
+    }
+    __half* o = m.dst + (size_t)r * kp;
+    float all = 0.0f, gone = 0.0f;
+    for (int c = lane * 4; c < kp; c += 128) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < K && fits) v = __ldg(reinterpret_cast<const float4*>(s + c));
+      float x[4] = {v.x * up, v.y * up, v.z * up, v.w * up};
+      __half y[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y[j] = __float2half_rn(fabsf(x[j]) < 6.103515625e-5f ? 0.0f : x[j]);  // 2^-14: no fp16 subnormals
+        const float rest = x[j] - __half2float(y[j]);
+        all = fmaf(x[j], x[j], all);
+        gone = fmaf(rest, rest, gone);
+      }
+      const __half2 lo = __halves2half2(y[0], y[1]), hi = __halves2half2(y[2], y[3]);
+      *reinterpret_cast<uint2*>(o + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    all = warp_sum(all);
+    gone = warp_sum(gone);
+    if (lane == 0) {
+      const float lost = all > 0.0f ? 1.002f * sqrtf(gone / all) : 0.0f;
+      if (is_b) most_lost = fmaxf(most_lost, lost);
+      else m.lost[r] = lost;
+    }
+  }
+  if (lane == 0 && most_lost > 0.0f) atomicMax(bounds.top + 2, __float_as_uint(most_lost));
+  if (lane == 0 && most > 0.0f) atomicMax(bounds.top, __float_as_uint(most));
+}
+
 struct Fp32GemmParams {
   int M, N, kp;
   long long ldc;
   int m_tiles, n_tiles, pairs;
   float* C;            // [M][ldc], or the lower ends
   __nv_bfloat16* lo;
-  float rel;           // ENDS: estimate_rel, the rows' norms, and the columns' bias and gate (nullptr: 0 and 1)
+  float rel;           // ENDS: the bound's factor, the rows' norms, and the columns' bias and gate (nullptr: 0 and 1)
   const float* na;
   const float* nb;
   const float* bias;
   const float* gate;
+  const float* sa;     // one term: what a row of A and of B was divided by
+  const float* sb;
+  const float* lost;   // one term: what rounding took of a row of A, and the most that it took of one of B
+  const uint32_t* lost_b;
+  const int* wide;     // optional: nothing is done unless wide[0] > wide_limit
+  int wide_limit;
+  float* maxima;       // one term: [M][ld_maxima], the largest end of every 32 columns (group_max)
+  long long ld_maxima;
   int* status;
 };
 
-// Rounded down to bf16; NaN for what is not finite.
-__device__ __forceinline__ uint32_t bf16_down(float x) {
-  const uint32_t b = __float_as_uint(x);
-  if ((b & 0x7f800000u) == 0x7f800000u) return 0x7fffu;
-  return ((int)b < 0 ? b + 0xffffu : b) >> 16;
+// The largest end of a group of columns, none below 0, rounded down to bf16; the last bit is set where an end says nothing.
+__device__ __forceinline__ float group_max(float top, bool unknown) {
+  const uint32_t b = __float_as_uint(top);
+  return __uint_as_float((b >= 0x7f800000u ? 0u : b & 0xffff0000u) | (unknown ? 1u : 0u));
 }
 
 template <int TERMS, bool ENDS>
 __global__ void __launch_bounds__(FG_THREADS, 1)
 fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Fp32GemmParams p) {
   pdl_wait();
+  if (p.wide != nullptr && p.wide[0] <= p.wide_limit) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + FG_BAR_OFF);
@@ -215,7 +311,7 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * FG_BM, FG_BN);
+      constexpr uint32_t idesc = TERMS == 1 ? make_idesc_f16(2 * FG_BM, FG_BN) : make_idesc_bf16(2 * FG_BM, FG_BN);
       uint32_t it = 0, sub = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += p.pairs) {
@@ -252,38 +348,49 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp >= 4) {
     const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter, column half
-    const bool vec = ENDS ? p.N % 8 == 0 && p.ldc % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.lo) | reinterpret_cast<uintptr_t>(p.nb) |
-                                                                reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.gate)) & 15) == 0
+    const bool vec = ENDS ? p.N % 8 == 0 && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.lo) & 15) == 0
                           : p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t sub = 0;
     bool ok = true;
-    for (int t = pair; t < tiles && ok; t += p.pairs) {
+    // what column threadIdx.x - 128 of tile t has of its own: scale, norm, bias, gate
+    auto column = [&](int t) -> float4 {
+      const int c = (t / p.m_tiles) * FG_BN + (int)threadIdx.x - 128;
+      float4 v = make_float4(1.0f, 0.0f, 0.0f, 1.0f);
+      if (t < tiles && c < p.N) {
+        if (TERMS == 1) v.x = __ldg(p.sb + c);
+        v.y = __ldg(p.nb + c);
+        if (p.bias != nullptr) v.z = __ldg(p.bias + c);
+        if (p.gate != nullptr) v.w = __ldg(p.gate + c);
+      }
+      return v;
+    };
+    float4 ahead = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if constexpr (ENDS) ahead = column(pair);
+    for (int t = pair; t < tiles && (ENDS || ok); t += p.pairs) {
       const int row = (t % p.m_tiles) * 2 * FG_BM + (int)cta_rank * FG_BM + q * 32 + lane;
       const int c0 = (t / p.m_tiles) * FG_BN + half * 128;
       if constexpr (ENDS) {
+        // (a warp that gave up goes on to the barriers, which the others wait at without a limit)
+        float4* cols = reinterpret_cast<float4*>(smem + FG_COL_OFF) + (sub & 1) * 256;
+        cols[threadIdx.x - 128] = ahead;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        ahead = column(t + p.pairs);
         const int buf = sub & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], (sub >> 1) & 1, abort_flag));
-        if (!ok) {
+        ++sub;
+        if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(&tmem_full_bar[buf], ((sub - 1) >> 1) & 1, abort_flag))) {
           if (lane == 0) report_status(p.status, kTimeoutTmemFull, (int)sub);
           *abort_flag = 1;
-          break;
+          ok = false;
         }
+        if (!ok) continue;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * FG_BN + half * 128);
         const int row0 = row - lane;
-        const float rx = row < p.M ? -mul_up(p.rel, __ldg(p.na + row)) : 0.0f;
-        auto columns = [&](const float* v, int c, float absent, float (&x)[8]) {  // (the same for the whole warp)
-          if (v != nullptr && vec && c < p.N) {
-            const float4 t0 = __ldg(reinterpret_cast<const float4*>(v + c)), t1 = __ldg(reinterpret_cast<const float4*>(v + c + 4));
-            x[0] = t0.x; x[1] = t0.y; x[2] = t0.z; x[3] = t0.w;
-            x[4] = t1.x; x[5] = t1.y; x[6] = t1.z; x[7] = t1.w;
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = v != nullptr && c + i < p.N ? __ldg(v + c + i) : absent;
-          }
-        };
+        const float rx = row < p.M ? -mul_up(TERMS == 1 ? half_rel(p.rel, __ldg(p.lost + row), p.lost_b) : p.rel, __ldg(p.na + row)) : 0.0f;
+        const float sr = TERMS == 1 && row < p.M ? __ldg(p.sa + row) : 1.0f;
         uint8_t* tile_s = smem + FG_STORE_OFF + (warp - 4) * 2048;
-#pragma unroll 1
+        float largest[4];
+#pragma unroll
         for (int g = 0; g < 4; ++g) {
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + (uint32_t)(g * 32), r);
@@ -294,23 +401,27 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[buf]), 0));
           }
           const int cg = c0 + g * 32;
+          float top = 0.0f;
+          bool unknown = false;
           uint4 o[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            float wn[8], bias[8], gate[8];
             uint32_t e[8];
-            columns(p.nb, cg + j * 8, 0.0f, wn);
-            columns(p.bias, cg + j * 8, 0.0f, bias);
-            columns(p.gate, cg + j * 8, 1.0f, gate);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              float v = fma_rn(rx, wn[i], __uint_as_float(r[j * 8 + i]));
-              if (p.bias != nullptr) v = add_rn(v, bias[i]);
-              if (p.gate != nullptr) v = mul_rn(v, gate[i]);
-              e[i] = (__float_as_uint(wn[i]) & 0x7fffffffu) >= 0x7f800000u ? 0x7fffu : bf16_down(v);
+              const float4 c = cols[half * 128 + g * 32 + j * 8 + i];  // (the same for the whole warp)
+              float v = __uint_as_float(r[j * 8 + i]);
+              if constexpr (TERMS == 1) v = mul_rn(v, sr * c.x);  // (powers of two)
+              v = mul_rn(add_rn(fma_rn(rx, c.y, v), c.z), c.w);
+              const uint32_t b = __float_as_uint(v);
+              const bool none = (b & 0x7f800000u) == 0x7f800000u;
+              e[i] = none ? 0x7fffu : ((int)b < 0 ? b + 0xffffu : b) >> 16;  // rounded down
+              unknown |= none;
+              top = fmaxf(top, v);
             }
             o[j] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
           }
+          largest[g] = group_max(top, unknown);
           // through shared memory, so that four lanes write whole sectors of a row (as in encoder_gemm.cu)
           __syncwarp();
 #pragma unroll
@@ -331,7 +442,8 @@ fp32_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
           }
         }
-        ++sub;
+        if (p.maxima != nullptr && row < p.M)
+          *reinterpret_cast<float4*>(p.maxima + row * p.ld_maxima + c0 / 32) = make_float4(largest[0], largest[1], largest[2], largest[3]);
       } else {
         float acc[128];
 #pragma unroll
@@ -414,7 +526,7 @@ int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv
   if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0 || (parts != 2 && parts != 3)) return (int)cudaErrorInvalidValue;
   const int blocks = (rows + 7) / 8;
   auto kern = parts == 2 ? split_bf16_kernel<2> : split_bf16_kernel<3>;
-  launch(kern, blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream, src, rows, K, kp, dst, flags, SplitBounds{norm, wide, top, bias, gate});
+  launch(kern, blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream, src, rows, K, kp, dst, flags, SplitBounds{norm, wide, top, bias, gate}, nullptr, 0);
   return (int)cudaGetLastError();
 }
 
@@ -457,11 +569,37 @@ int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* 
 }
 
 int fp32_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* nb, const float* bias,
-                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, cudaStream_t stream) {
+                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, const int* wide, int wide_limit, cudaStream_t stream) {
   Fp32GemmParams p = {};
-  p.M = M; p.N = N; p.kp = kp; p.lo = lo; p.ldc = ldc; p.status = status;
+  p.M = M; p.N = N; p.kp = kp; p.lo = lo; p.ldc = ldc; p.status = status; p.wide = wide; p.wide_limit = wide_limit;
   p.rel = estimate_rel(K); p.na = na; p.nb = nb; p.bias = bias; p.gate = gate;
   return (int)launch_product(reinterpret_cast<const void*>(fp32_gemm_kernel<3, true>), ta, tb, p, stream);
+}
+
+int half_rows_launch(const float* A, int M, __half* a16, float* na, float* sa, float* lost, const float* B, int N, __half* b16, float* nb, float* sb, int K, int kp,
+                     uint16_t* widths, uint32_t* top, const float* bias, const float* gate, cudaStream_t stream) {
+  if (K % 4 != 0 || kp % 64 != 0 || kp < K || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) != 0) return (int)cudaErrorInvalidValue;
+  const long long blocks = ((long long)M + N + 7) / 8;
+  return (int)launch(half_rows_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, HalfRows{A, M, a16, na, sa, lost},
+                     HalfRows{B, N, b16, nb, sb, nullptr}, K, kp, SplitBounds{nullptr, widths, top, bias, gate});
+}
+
+int half_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* sa, const float* lost,
+                     const uint32_t* top, const float* nb, const float* sb, const float* bias, const float* gate, __nv_bfloat16* lo, long long ldc, float* maxima,
+                     long long ld_maxima, int* status, cudaStream_t stream) {
+  if (maxima != nullptr && (ld_maxima % 4 != 0 || ld_maxima < (long long)(N + FG_BN - 1) / FG_BN * 8 || (reinterpret_cast<uintptr_t>(maxima) & 15) != 0))
+    return (int)cudaErrorInvalidValue;
+  Fp32GemmParams p = {};
+  p.M = M; p.N = N; p.kp = kp; p.lo = lo; p.ldc = ldc; p.status = status;
+  p.maxima = maxima; p.ld_maxima = ld_maxima;
+  p.rel = estimate_rel_half(K); p.na = na; p.sa = sa; p.lost = lost; p.lost_b = top + 2; p.nb = nb; p.sb = sb; p.bias = bias; p.gate = gate;
+  return (int)launch_product(reinterpret_cast<const void*>(fp32_gemm_kernel<1, true>), ta, tb, p, stream);
+}
+
+int split_bf16_if_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, const int* wide, int wide_limit, cudaStream_t stream) {
+  if (K % 4 != 0 || kp % 64 != 0 || kp < K || (reinterpret_cast<uintptr_t>(src) & 15) != 0) return (int)cudaErrorInvalidValue;
+  const int blocks = (rows + 7) / 8;
+  return (int)launch(split_bf16_kernel<2>, blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, stream, src, rows, K, kp, dst, nullptr, SplitBounds{}, wide, wide_limit);
 }
 
 }  // namespace lmsae

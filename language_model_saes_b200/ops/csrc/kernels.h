@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -49,7 +50,13 @@ int split_bf16_launch(const float* src, int rows, int K, int kp, int parts, __nv
 int fp32_gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, const float* A, const float* B, int M, int N, int K, int kp, const int* fa,
                      const int* fb, float* C, long long ldc, int* status, bool tensor_cores, cudaStream_t stream);
 int fp32_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* nb, const float* bias,
-                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, cudaStream_t stream);
+                     const float* gate, __nv_bfloat16* lo, long long ldc, int* status, const int* wide, int wide_limit, cudaStream_t stream);
+int split_bf16_if_launch(const float* src, int rows, int K, int kp, __nv_bfloat16* dst, const int* wide, int wide_limit, cudaStream_t stream);
+int half_rows_launch(const float* A, int M, __half* a16, float* na, float* sa, float* lost, const float* B, int N, __half* b16, float* nb, float* sb, int K, int kp,
+                     uint16_t* widths, uint32_t* top, const float* bias, const float* gate, cudaStream_t stream);
+int half_ends_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int kp, const float* na, const float* sa, const float* lost,
+                     const uint32_t* top, const float* nb, const float* sb, const float* bias, const float* gate, __nv_bfloat16* lo, long long ldc, float* maxima,
+                     long long ld_maxima, int* status, cudaStream_t stream);
 
 // ---- peer-memory collectives (comm_ops.cu) -------------------------------------------------------
 constexpr int kMaxPeers = 8;
@@ -88,6 +95,10 @@ int topk_dense_launch(const float* h, const float* bias, const float* norm, int 
 constexpr int kEstimateMaxK = 16384;  // (above it the bound on the estimate's error rules out too few columns)
 int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const uint32_t* top, int K, const float* bias,
                          const float* norm, int B, int N, int k, const int* status, int* todo, float* out, cudaStream_t stream);
+int topk_narrow_launch(const __nv_bfloat16* lo, const float* maxima, long long ld_maxima, const float* x, const float* W, const float* xn, const float* lost, const uint32_t* top, int K, const float* bias, const float* norm,
+                       int B, int N, int k, const int* status, int* wide, float* out, cudaStream_t stream);
+int topk_wide_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const float* lost, const uint32_t* top, int K, const float* bias,
+                     const float* norm, int B, int N, int k, const int* status, const int* wide, int wide_limit, int* todo, float* out, cudaStream_t stream);
 struct RowsProductParams {
   const float* A;   // [*, K]
   const float* B;   // [N, K], or [K, N]

@@ -791,8 +791,13 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
 //   Columns that the bound says nothing about (their lower end is NaN) are among them; rows with more such columns than there is room for,
 // and all rows where the product gave up, are listed, multiplied in order as a whole (rows_product.cu) and selected from exactly. All
 // decisions are taken on the device.
-// 4096 x 24576 x 768, k 50: with fp32 estimates, and the columns' norms, error bounds and biases read from the L2 cache twice for every row,
-// 506 us; 280 here.
+//   With ends from one fp16 product (topk_narrow_launch) the bound and the columns come from the maxima of 32 columns, and the ends are
+// read only in groups that may hold something. Rows with more than 256 + 4 k columns in question are listed instead of summed up; where they are more
+// than an eighth of all rows, three bf16 products propose for the whole batch again, and the listed rows are selected from in the form above
+// (topk_wide_launch). Elsewhere the kernels of that second proposal leave at once, 11 us in all.
+// 4096 x 24576 x 768, k 50: lower ends of three products, each row's read twice, 286 us; by maxima of those of one product 244: 122 for the
+// zeros (403 MB), bound and choice, the rest are the rows of W, 3 kB for each of about 60 columns. Twelve rows of W at a time per warp take one
+// pass over those columns where eight take two (387 us with 72 columns a row).
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned topk_key(float g) {
   const unsigned b = __float_as_uint(g);
@@ -814,6 +819,14 @@ struct TopkDenseParams {
   const float* xn;          // [B] 2-norms (fp32_gemm.cu)
   const uint32_t* top;      // the largest error bound of a column over rel * xn; whether a norm is 0 or NaN; from the fifth word on every column's bound, bf16
   const int* status;        // of the product
+  float rel;                // the bound's factor (with lost: half_rel's), and another one where wide[0] > wide_limit
+  const float* lost;
+  float rel_wide;
+  const int* wide;          // [0] number of rows, then which
+  int wide_limit;
+  int most;                 // entries of a row to be summed up at most
+  const float* maxima;      // MAXIMA: [B][ld_maxima] the ends' group_max of 32 columns each
+  long long ld_maxima;
   int K;
   int* todo;        // ESTIMATE: [1 + B] number of rows left over, and which
   const int* rows;  // or the rows to work on, in this form
@@ -876,10 +889,11 @@ __device__ __forceinline__ void topk_ends_load(const TopkDenseParams& p, const _
 // of W is fetched by the whole warp: pieces of 32 columns of eight candidates' rows and of x are copied to shared memory, whole
 // sectors a row, one piece ahead. (Each thread reading its own row, 16 bytes at a time, kept the L1 cache busy with a line per thread and
 // load: 373 us for the whole selection.) Neighbouring candidates go to different warps.
-constexpr int DOT_ROWS = 8, DOT_K = 32, DOT_PITCH = DOT_K + 4;  // (the pitch: eight rows' 16-byte pieces in different banks)
+constexpr int DOT_K = 32, DOT_PITCH = DOT_K + 4;  // (the pitch: eight rows' 16-byte pieces in different banks)
+template <int DOT_ROWS>
 struct DotTiles { float w[RT_WARPS][2][DOT_ROWS + 1][DOT_PITCH]; };
-template <class Done>
-__device__ __forceinline__ void dots_in_order(DotTiles& tiles, const float* __restrict__ x, const float* __restrict__ W, int K, const int* cols, int n, Done&& done) {
+template <int DOT_ROWS, class Done>
+__device__ __forceinline__ void dots_in_order(DotTiles<DOT_ROWS>& tiles, const float* __restrict__ x, const float* __restrict__ W, int K, const int* cols, int n, Done&& done) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int PIECES = (DOT_ROWS + 1) * DOT_K / 4, PER_LANE = (PIECES + 31) / 32;
   for (int base = warp; base < n; base += DOT_ROWS * RT_WARPS) {
@@ -943,10 +957,10 @@ __device__ __forceinline__ int cta_count(int mine, unsigned (&words)[RT_WARPS]) 
   return (int)__reduce_add_sync(0xffffffffu, (threadIdx.x & 31) < RT_WARPS ? words[threadIdx.x & 31] : 0u);
 }
 
-template <bool ESTIMATE>
+template <bool ESTIMATE, int CAP = RT_CAP, int DOT_ROWS = 8, bool MAXIMA = false>
 __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row) {
-  __shared__ unsigned s_key[RT_CAP];
-  __shared__ int s_col[RT_CAP];
+  __shared__ unsigned s_key[CAP];
+  __shared__ int s_col[CAP];
   __shared__ unsigned s_count[2][RT_WARPS];
   __shared__ int s_n, s_above, s_equal;
   const float* h = ESTIMATE ? nullptr : p.h + (size_t)row * p.N;
@@ -961,7 +975,21 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   unsigned mx[RT_MAXIMA];
 #pragma unroll
   for (int i = 0; i < RT_MAXIMA; ++i) mx[i] = 0u;
-  if constexpr (ESTIMATE) {
+  const float* maxima = MAXIMA ? p.maxima + row * p.ld_maxima : nullptr;
+  const int groups = MAXIMA ? (int)p.ld_maxima : 0;
+  if constexpr (MAXIMA) {
+    for (int c = threadIdx.x * 4; c < groups; c += RT_THREADS * 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(maxima + c));
+      const float g[4] = {v.x, v.y, v.z, v.w};
+      const int h4 = c / (RT_THREADS * 4) & 1 ? 4 : 0;  // (up to 2048 groups: each by itself)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const unsigned b = __float_as_uint(g[i]) & 0xffff0000u;
+        if (h4 == 0) mx[i] = max(mx[i], b);
+        else mx[4 + i] = max(mx[4 + i], b);
+      }
+    }
+  } else if constexpr (ESTIMATE) {
 #pragma unroll 4
     for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
       float g[8];
@@ -986,17 +1014,17 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   const float nan = __uint_as_float(0x7fffffffu);
   auto enter = [&](int c, unsigned key) {
     const int pos = atomicAdd(&s_n, 1);
-    if (pos < RT_CAP) { s_key[pos] = key; s_col[pos] = c; }
+    if (pos < CAP) { s_key[pos] = key; s_col[pos] = c; }
   };
   if constexpr (ESTIMATE) {
     // (16 units of 2^-24 more for the roundings of the ends; the last term for lower ends that are subnormal)
-    const float width = mul_up(2.0f * (estimate_rel(p.K) + 1e-6f), p.xn[row]);
+    const float rel = p.wide != nullptr && p.wide[0] > p.wide_limit ? p.rel_wide : p.lost != nullptr ? half_rel(p.rel, p.lost[row], p.top + 2) : p.rel;
+    const float width = mul_up(2.0f * (rel + 1e-6f), p.xn[row]);
     const float room = add_rn(mul_up(width, __uint_as_float(p.top[0])), 1e-37f);
     const float thr_f = __uint_as_float(max(thr, 1u));
     const __nv_bfloat16* widths = below(mul_rn(room, 64.0f), thr_f) ? nullptr : reinterpret_cast<const __nv_bfloat16*>(p.top + 4);
     const bool any_bad = p.top[1] != 0u;
-#pragma unroll 2
-    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+    auto visit = [&](int c) {  // columns [c, c + 8)
       float g[8], r[8];
       topk_ends_load(p, lo, c, g);
 #pragma unroll
@@ -1014,6 +1042,33 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
         in &= in - 1u;
         if (c + i < N) enter(c + i, 0u);
       }
+    };
+    const bool by_groups = MAXIMA && widths == nullptr;
+    if (by_groups) {  // only the groups that may hold something (a lane of a group's four: eight of its columns)
+      for (int base = (int)(threadIdx.x >> 5) * 32; base < groups; base += RT_THREADS) {
+        const int j = base + (int)(threadIdx.x & 31);
+        unsigned b = 0u;
+        bool in = false;
+        if (j < groups) {
+          b = __float_as_uint(__ldg(maxima + j));
+          const float g = __uint_as_float(b & 0xffff0000u);
+          in = (b & 1u) != 0u || !below(add_rn(fma_rn(g, 0.0079f, g), room), thr_f);
+        }
+        unsigned mask = __ballot_sync(0xffffffffu, in);
+        while (mask != 0u) {  // eight groups at a time
+          unsigned mine = mask;
+          for (int s = (int)(threadIdx.x & 31) >> 2; s > 0 && mine != 0u; --s) mine &= mine - 1u;
+          if (mine != 0u) {
+            const int c = (base + __ffs(mine) - 1) * 32 + ((int)threadIdx.x & 3) * 8;
+            if (c < N) visit(c);
+          }
+          for (int s = 0; s < 8 && mask != 0u; ++s) mask &= mask - 1u;
+        }
+      }
+    }
+#pragma unroll 2
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+      if (!by_groups) visit(c);
       float z[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) z[i] = 0.0f;
@@ -1061,11 +1116,11 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   __syncthreads();  // (also: the zeros are written before what is written over them)
   const int n = s_n;
   if constexpr (ESTIMATE) {
-    if (n > RT_CAP) {
+    if (n > p.most) {
       if (threadIdx.x == 0) p.todo[1 + atomicAdd(p.todo, 1)] = row;
       return;
     }
-    __shared__ __align__(16) DotTiles tiles;
+    __shared__ __align__(16) DotTiles<DOT_ROWS> tiles;
     dots_in_order(tiles, p.x + (size_t)row * p.K, p.W, p.K, s_col, n, [&](int j, float g) {
       const int c = s_col[j];
       if (p.bias != nullptr) g = add_rn(g, p.bias[c]);
@@ -1085,11 +1140,11 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
     if (p.norm != nullptr) v = div_rn(v, p.norm[c]);
     out[c] = v;
   };
-  if (n <= RT_CAP) {
+  if (n <= CAP) {
     if (n > k) {
-      unsigned mine[RT_CAP / RT_THREADS];
+      unsigned mine[CAP / RT_THREADS];
 #pragma unroll
-      for (int i = 0; i < RT_CAP / RT_THREADS; ++i) {
+      for (int i = 0; i < CAP / RT_THREADS; ++i) {
         const int j = threadIdx.x + i * RT_THREADS;
         mine[i] = j < n ? s_key[j] : 0u;
       }
@@ -1156,11 +1211,21 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
   }
 }
 
-template <bool ESTIMATE>
+template <bool ESTIMATE, int CAP = RT_CAP, int DOT_ROWS = 8, bool MAXIMA = false>
 __global__ void __launch_bounds__(RT_THREADS, 5)
 topk_dense_kernel(const TopkDenseParams p) {
   pdl_wait();
-  topk_dense_row<ESTIMATE>(p, blockIdx.x);
+  topk_dense_row<ESTIMATE, CAP, DOT_ROWS, MAXIMA>(p, blockIdx.x);
+}
+
+__global__ void __launch_bounds__(RT_THREADS, 5)
+topk_wide_kernel(const TopkDenseParams p) {
+  pdl_wait();
+  const int n = p.wide[0];
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    topk_dense_row<true>(p, p.wide[1 + i]);
+    __syncthreads();
+  }
 }
 
 __global__ void __launch_bounds__(RT_THREADS, 5)
@@ -1184,27 +1249,73 @@ int topk_dense_launch(const float* h, const float* bias, const float* norm, int 
   return (int)cudaGetLastError();
 }
 
+constexpr int NARROW_CAP = 4 * RT_THREADS;  // (what it leaves of the shared memory holds more rows of W at a time)
+
+static bool estimate_args_fit(const float* x, const float* W, int K, int k) {
+  return k >= 1 && k <= RT_BOUND_K && K >= 1 && K <= kEstimateMaxK && K % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+}
+
+// The rows listed in todo: their products in order, and the selection from those.
+static int finish_rows(TopkDenseParams p, float* h, int B, int* todo, cudaStream_t stream) {
+  RowsProductParams r = {};
+  r.A = p.x; r.B = p.W; r.C = h; r.N = p.N; r.K = p.K; r.rows = todo; r.max_rows = B;
+  const int e = rows_product_launch(r, false, stream);
+  if (e != 0) return e;
+  p.rows = todo;
+  p.h = h;
+  p.vec = p.N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.norm) |
+                            reinterpret_cast<uintptr_t>(p.out)) % 16 == 0);
+  return (int)launch(topk_dense_rows_kernel, B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream, p);
+}
+
 // The same with lower ends `lo` from an estimate of x W^T; h: fp32 [B, N] for the products of rows that are left over (it may share
 // memory with lo, which is no longer read then). todo: int [1 + B], todo[0] zeroed.
 int topk_estimate_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const uint32_t* top, int K, const float* bias,
                          const float* norm, int B, int N, int k, const int* status, int* todo, float* out, cudaStream_t stream) {
   if (B <= 0 || N <= 0) return 0;
-  if (k < 1 || k > RT_BOUND_K || K < 1 || K > kEstimateMaxK || K % 4 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W)) & 15) != 0)
-    return (int)cudaErrorInvalidValue;
+  if (!estimate_args_fit(x, W, K, k)) return (int)cudaErrorInvalidValue;
   TopkDenseParams p = {};
   p.lo = lo; p.x = x; p.W = W; p.xn = xn; p.top = top; p.status = status; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.rel = estimate_rel(K);
+  p.most = RT_CAP;
   p.vec = N % 8 == 0 && ((reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  launch(topk_dense_kernel<true>, B, RT_THREADS, 0, stream, p);
-  RowsProductParams r = {};
-  r.A = x; r.B = W; r.C = h; r.N = N; r.K = K; r.rows = todo; r.max_rows = B;
-  const int e = rows_product_launch(r, false, stream);
-  if (e != 0) return e;
-  p.rows = todo;
-  p.h = h;
-  p.vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(norm) |
-                          reinterpret_cast<uintptr_t>(out)) % 16 == 0);
-  launch(topk_dense_rows_kernel, B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream, p);
-  return (int)cudaGetLastError();
+  const cudaError_t e = launch(topk_dense_kernel<true>, B, RT_THREADS, 0, stream, p);
+  return e != cudaSuccess ? (int)e : finish_rows(p, h, B, todo, stream);
+}
+
+// With lower ends from one fp16 product (half_ends_launch): what can be decided by them without summing up more than a few times k entries of a
+// row. The other rows go to the list `wide`, int [1 + B], wide[0] zeroed.
+int topk_narrow_launch(const __nv_bfloat16* lo, const float* maxima, long long ld_maxima, const float* x, const float* W, const float* xn, const float* lost, const uint32_t* top, int K, const float* bias, const float* norm,
+                       int B, int N, int k, const int* status, int* wide, float* out, cudaStream_t stream) {
+  if (B <= 0 || N <= 0) return 0;
+  if (!estimate_args_fit(x, W, K, k) || maxima == nullptr || ld_maxima % 4 != 0 || (reinterpret_cast<uintptr_t>(maxima) & 15) != 0) return (int)cudaErrorInvalidValue;
+  TopkDenseParams p = {};
+  p.lo = lo; p.x = x; p.W = W; p.xn = xn; p.top = top; p.status = status; p.K = K; p.todo = wide; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.rel = estimate_rel_half(K);
+  p.lost = lost;
+  p.maxima = maxima; p.ld_maxima = ld_maxima;
+  p.most = min(256 + 4 * k, RT_CAP);
+  p.vec = N % 8 == 0 && ((reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
+  return (int)(p.most <= NARROW_CAP ? launch(topk_dense_kernel<true, NARROW_CAP, 12, true>, B, RT_THREADS, 0, stream, p)
+                                         : launch(topk_dense_kernel<true, RT_CAP, 8, true>, B, RT_THREADS, 0, stream, p));
+}
+
+// The rows of that list, with lower ends from three products where they are more than wide_limit (lo holds those then), and from one elsewhere.
+int topk_wide_launch(const __nv_bfloat16* lo, float* h, const float* x, const float* W, const float* xn, const float* lost, const uint32_t* top, int K, const float* bias,
+                     const float* norm, int B, int N, int k, const int* status, const int* wide, int wide_limit, int* todo, float* out, cudaStream_t stream) {
+  if (B <= 0 || N <= 0) return 0;
+  if (!estimate_args_fit(x, W, K, k)) return (int)cudaErrorInvalidValue;
+  TopkDenseParams p = {};
+  p.lo = lo; p.x = x; p.W = W; p.xn = xn; p.top = top; p.status = status; p.K = K; p.todo = todo; p.bias = bias; p.norm = norm; p.out = out; p.N = N; p.k = k;
+  p.rel = estimate_rel_half(K);
+  p.lost = lost;
+  p.rel_wide = estimate_rel(K);
+  p.wide = wide;
+  p.wide_limit = wide_limit;
+  p.most = RT_CAP;
+  p.vec = N % 8 == 0 && ((reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
+  const cudaError_t e = launch(topk_wide_kernel, B < 148 * 5 ? B : 148 * 5, RT_THREADS, 0, stream, p);
+  return e != cudaSuccess ? (int)e : finish_rows(p, h, B, todo, stream);
 }
 
 }  // namespace lmsae

@@ -231,3 +231,66 @@ def test_a_dictionary_in_pieces(M, N, K_, monkeypatch):
     before = torch.cuda.memory_allocated()
     out = I.product(x, w.t())
     assert torch.cuda.max_memory_allocated() - before < out.numel() * 4 + x.numel() * 8 + (4 << 20)
+
+
+@pytest.mark.parametrize("data", ["normal", "spread", "cancelling", "few cancelling rows", "near zero", "repeated", "out of range", "one bad column", "no gate"])
+@pytest.mark.parametrize("B,F,K_,k", [(270, 8192, 128, 50), (259, 9001, 260, 64), (256, 33024, 68, 250)])
+def test_selection_by_one_fp16_product(B, F, K_, k, data):
+    """Codes bit for bit, wherever a row ends up: decided by the fp16 product, by the three products after it, or multiplied as a whole."""
+    g = torch.Generator(device=DEV).manual_seed(F)
+    assert I.half_product_pays(F, k)
+    x, w = torch.randn(B, K_, device=DEV, generator=g), torch.randn(F, K_, device=DEV, generator=g) / K_**0.5
+    bias, norm = 0.1 * torch.randn(F, device=DEV, generator=g), torch.rand(F, device=DEV, generator=g) + 0.5
+    if data == "spread":  # magnitudes from the largest down to what fp16 drops, rows of very different size
+        x *= torch.exp2(-24.0 * torch.rand(B, K_, device=DEV, generator=g)) * torch.exp2(20.0 * torch.rand(B, 1, device=DEV, generator=g))
+        w *= torch.exp2(-24.0 * torch.rand(F, K_, device=DEV, generator=g)) * torch.exp2(6.0 * torch.rand(F, 1, device=DEV, generator=g) - 12.0)
+        bias *= 0.0
+    elif "cancelling" in data:  # a common offset that the bias takes away
+        w *= 1e-3
+        w[:, 0] = 1.0
+        x[:, 0] = 1000.0
+        if data != "cancelling":
+            x[B // 10 :, 0] = 0.0
+            x[B // 10 :] *= 1e6
+        bias = bias * 1e-3 - 1000.0
+        norm[:] = 1.0
+    elif data == "near zero":
+        bias = -_in_order(x[:1], w)[0].topk(k).values[-1].expand(F).clone()
+        x[1:] = x[0] * (1 + 1e-6 * torch.randn(B - 1, 1, device=DEV, generator=g))
+        norm[:] = 1.0
+    elif data == "repeated":
+        w[: F * 3 // 4] = w[0]
+        bias[: F * 3 // 4], norm[: F * 3 // 4] = 1.0, 1.0
+        x[B // 2 :] = x[0]
+    elif data == "out of range":
+        x[0] *= 1e-25
+        x[1] *= 1e25
+        x[2] = 0.0
+        w[5] *= 1e-25
+        w[7] *= 1e20
+        w[9] = 0.0
+        bias[11], norm[13], norm[15] = 1e25, 0.0, 1e20
+    elif data == "one bad column":
+        w[11, 3] = float("nan")
+        w[13, 4] = float("inf")
+        w[15, 2] = -float("inf")
+    elif data == "no gate":
+        norm = None
+    out = I.topk_encode(x, w.t(), bias, norm, k)
+    want = I.topk_dense(_in_order(x, w), bias, norm, k)
+    differ = (out.nan_to_num(nan=-1.0) != want.nan_to_num(nan=-1.0)).nonzero()
+    assert differ.numel() == 0, (differ[:4], len(differ))
+
+
+def test_ends_of_one_fp16_product_enclose_the_sums():
+    """What the selection relies on, without the selection: every positive sum in order lies between its end and that plus the width."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    B, F, K_, k = 512, 8192, 768, 64
+    x, w = torch.randn(B, K_, device=DEV, generator=g), torch.randn(F, K_, device=DEV, generator=g) / K_**0.5
+    exact = _in_order(x, w)
+    half = lambda t: (lambda s: (t * s).half().double() / s.double())(torch.exp2(14 - t.abs().amax(1, keepdim=True).log2().floor()))  # noqa: E731
+    error = (half(x) @ half(w).t() - exact.double()).abs()
+    rest = lambda t: ((half(t) - t.double()).norm(dim=1) / t.double().norm(dim=1))  # noqa: E731
+    bound = (rest(x)[:, None] + rest(w).max() + (2.1 * K_ + 136) * 2.0**-24) * x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)
+    assert (error <= bound).all() and float((error / bound).max()) > 0.01  # (and says something)
+    assert torch.equal(I.topk_encode(x, w.t(), None, None, k), I.topk_dense(exact, None, None, k))
