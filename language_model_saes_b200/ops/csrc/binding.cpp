@@ -796,6 +796,45 @@ std::vector<Tensor> colsum_adam(const std::vector<Tensor>& a, const std::vector<
   return out;
 }
 
+// One training step of a TopK dictionary on one GPU, the calls of FusedTopKSAEStep.step in their order: host work between the launches is what the
+// smallest steps consist of. route (sae_kernels.topk_route): 0 top-k in the GEMM's epilogue and merge, 1 fp32 pre-activations and row_select, 2 bf16 ones
+// and row_select, 3 row_topk by maxima, 4 row_topk. groups: counts, offsets, cursor, entries, block sums, heavy, sched of a FeatureGroups; enc and dec:
+// parameter, both moments, bf16 shadow; b_E and b_D (empty: none): bias and both moments. Returns the mean loss; loss_sum is left at zero.
+Tensor topk_step(const Tensor& x, const Tensor& label, int64_t k, int64_t route, int64_t mode, int64_t splits, int64_t units, const std::vector<Tensor>& enc,
+                 const std::vector<Tensor>& dec, const std::vector<Tensor>& b_E, const std::vector<Tensor>& b_D, const Tensor& dec_norm, bool use_gate,
+                 const c10::optional<Tensor>& row_weight, double grad_scale, const Tensor& loss_sum, const std::vector<Tensor>& groups, const Tensor& counters,
+                 double lr, double beta1, double beta2, double eps, int64_t step, double loss_den, const Tensor& status) {
+  TORCH_CHECK(enc.size() == 4 && dec.size() == 4 && b_E.size() == 3 && (b_D.empty() || b_D.size() == 3) && groups.size() == 7 && x.dim() == 2, "topk_step: arguments");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto none = c10::optional<Tensor>();
+  const c10::optional<Tensor> gate = use_gate ? c10::optional<Tensor>(dec_norm) : none, bias_d = b_D.empty() ? none : c10::optional<Tensor>(b_D[0]);
+  const int64_t M = x.size(0), N = enc[3].size(0);
+  const auto f32 = x.options().dtype(torch::kFloat32), i32 = x.options().dtype(torch::kInt32);
+  const Tensor idx = torch::empty({M, k}, i32), act = torch::empty({M, k}, f32);
+  if (route == 0) {
+    const int64_t C = splits * lmsae::enc_gemm_slots_for_k((int)k);
+    const Tensor cv = torch::empty({M, C}, f32), ci = torch::empty({M, C}, i32);
+    encoder_gemm(x, enc[3], b_E[0], gate, 2 | mode, k, splits, none, cv, ci, status, 0, false, units, none, none);
+    topk_merge(cv, ci, M, C, k, gate, 0, C, false, idx, act, 0, {}, 0, none, none);
+  } else {
+    const Tensor H = torch::empty({M, N}, route == 1 ? f32 : x.options());
+    const c10::optional<Tensor> maxima = route == 4 ? none : c10::optional<Tensor>(torch::empty({M, (N + 255) / 256 * 8}, f32));
+    encoder_gemm(x, enc[3], b_E[0], none, 1 | mode, 0, splits, H, none, none, status, 0, false, units, maxima, route == 4 ? none : gate);
+    if (route <= 2) row_select(H, *maxima, k, gate, route == 1, idx, act);
+    else row_topk(H, k, gate, none, maxima, idx, act);
+  }
+  const Tensor dxhat = torch::empty({M, dec[3].size(1)}, x.options()), dact = torch::empty_like(act);
+  sparse_decode(idx, act, dec[3], bias_d, none, none, label, row_weight, grad_scale, dxhat, loss_sum, none, none);
+  csc_build(idx, N, groups[0], groups[1], groups[2], groups[3], groups[4], groups[5]);
+  sparse_grad_adam(groups[1], groups[3], act, dact, x, dxhat, dec[0], dec[1], dec[2], dec[3], enc[0], enc[1], enc[2], enc[3], b_E[0], b_E[1], b_E[2], dec_norm, none,
+                   none, lr, beta1, beta2, eps, step, true, 0, -1, 0, none, 0, none, none, status, 0, {}, {}, 0, none, none, none, none, none, none, none, 1, groups[5], 0,
+                   groups[6], -1);
+  const std::vector<Tensor> nothing;
+  return colsum_adam(b_D.empty() ? nothing : std::vector<Tensor>{dxhat}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[0]},
+                     b_D.empty() ? nothing : std::vector<Tensor>{b_D[1]}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[2]}, counters, lr, beta1, beta2, eps, step,
+                     loss_sum, none, row_weight, loss_den, status)[0];
+}
+
 // g bf16 [rows, d] becomes zero where mask (bf16 [rows, d], rows any multiple of 8 apart) is; part fp32 [n, d]: column sums of n blocks of rows.
 void mask_colsum(const Tensor& g, const Tensor& mask, const Tensor& part) {
   CHECK_T(g, torch::kBFloat16); CHECK_T(part, torch::kFloat32);
@@ -1583,6 +1622,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_select", &row_select);
   m.def("row_select_fits", &row_select_fits);
   m.def("topk_dense", &topk_dense);
+  m.def("topk_step", &topk_step);
   m.def("topk_encode", &topk_encode);
   m.def("topk_estimate", &topk_estimate);
   m.def("fp32_gemm", &fp32_gemm);

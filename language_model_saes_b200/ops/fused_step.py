@@ -199,6 +199,7 @@ class FusedTopKSAEStep:
         n_chunks = max(1, n_chunks) if self.WD.is_cuda else 1
         rows = -(-tiles // n_chunks) * 256
         self.chunks = [(lo, min(F, lo + rows)) for lo in range(0, F, rows)]
+        self._one_call = self.tp == 1 and self.dp == 1 and not self.batch_level and len(self.chunks) == 1
         self.adam_done: list[torch.cuda.Event | None] = [None] * len(self.chunks)
         self._inflight: tuple | None = None  # tensors the update stream may still be reading
         self.overlap_ctas_per_sm = int(os.environ.get("LMSAE_OVERLAP_CTAS", "2"))
@@ -465,6 +466,8 @@ class FusedTopKSAEStep:
         kernel runs twice, first without writing anything to accumulate the squared norm, then with the factor."""
         if aux is not None:
             return self._step_auxk(x, label, k, lr, row_weight, n_tokens_global, aux, clip_grad_norm)
+        if self._one_call and x.is_cuda and x.shape[0] > 0 and k <= 512 and grad_mul is None and not want_grad_norm and not clip_grad_norm and self.phase_marks is None:
+            return self._step_in_one_call(x, label, k, lr, row_weight, n_tokens_global)
         B = x.shape[0]
         n_global = n_tokens_global if n_tokens_global is not None else B * self.dp
         grad_scale = 2.0 / n_global
@@ -568,6 +571,29 @@ class FusedTopKSAEStep:
             self._mark("bias_update")
         n_local = B if row_weight is None else row_weight.sum()
         return (self.loss_sum / (n_local * n_den)).squeeze(0)
+
+    def _step_in_one_call(self, x, label, k: int, lr: float, row_weight, n_tokens_global) -> torch.Tensor:
+        """``step`` of a TopK dictionary on one GPU: the same kernels in the same order, launched from one native call. Called one by one from
+        Python they take the host 75 us, which is all of a step of 512 x 64 x 256 and most of one of 1024 x 512 x 4096."""
+        B, n = x.shape[0], x.shape[0] * k
+        groups = self.groups
+        if groups is None or groups.entries.numel() < n or groups.heavy.numel() < 2 + n // K.HEAVY_ROW:
+            groups = self.groups = K.FeatureGroups(self.F, n, x.device)
+        units, splits = K._deal(B, self.F, None, None)
+        gate = self.dec_norm if self.use_gate else None
+        self._clear_sums()
+        b1, b2 = self.betas
+        loss = K._ext().topk_step(
+            x, label, k, K.topk_route(B, self.F, self.d, k, gate), K._pair_bit(None), splits, units,
+            (self.WE, *self.state["W_E"], self.WE_bf16), (self.WD, *self.state["W_D"], self.WD_bf16), (self.bE, *self.state["b_E"]),
+            () if self.bD is None else (self.bD, *self.state["b_D"]), self.dec_norm, self.use_gate, row_weight,
+            2.0 / (n_tokens_global if n_tokens_global is not None else B), self.loss_sum,
+            (groups.counts, groups.offsets, groups.cursor, groups.entries, groups.block_sums, groups.heavy, groups.sched), self.bias_update.counters,
+            lr, b1, b2, self.eps, self.t + 1, 1.0 if row_weight is not None else float(B), K.status_buffer(x.device),
+        )  # fmt: skip
+        self.t += 1
+        self._sums_clear = True
+        return loss
 
     def _clear_sums(self) -> None:
         if not self._sums_clear:

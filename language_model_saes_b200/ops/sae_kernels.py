@@ -47,7 +47,7 @@ _STATUS_NAMES = {
 class _Counting:
     """Proxy of the extension module that counts the device kernels each entry point launches."""
 
-    KERNELS_PER_CALL = {"csc_build": 5, "exclusive_scan": 3}
+    KERNELS_PER_CALL = {"csc_build": 5, "exclusive_scan": 3, "topk_step": 8, "topk_encode": 7}
 
     def __init__(self, mod):
         self._mod = mod
@@ -256,6 +256,17 @@ def hidden_topk(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, gat
         return H, *(row_select(H, maxima, k, gate) if x.shape[0] >= 1024 and _ext().row_select_fits(H, k, gate) else row_topk(H, k, gate, maxima=maxima))
     H = encoder_hidden(x, w, bias, pair)
     return H, *row_topk(H, k, gate)
+
+
+def topk_route(M: int, N: int, K: int, k: int, gate: torch.Tensor | None) -> int:
+    """How ``encoder_topk`` finds the codes of bf16 inputs on a GPU (the ``route`` of ``topk_step``): 0 in the GEMM's epilogue, 1 from fp32
+    pre-activations (``stored_topk``), 2 to 4 from bf16 ones (``hidden_topk``: by ``row_select``, ``row_topk`` with maxima, ``row_topk``)."""
+    aligned = gate is None or gate.data_ptr() % 16 == 0
+    if k <= 64:
+        return 1 if storing_pays(M, N, K, k) and N % 8 == 0 and aligned else 0
+    if not maxima_pay(N, k):
+        return 4
+    return 2 if M >= 1024 and k <= 128 and N % 8 == 0 and N <= 65535 * 32 and aligned else 3
 
 
 def _deal(M: int, N: int, pair: bool | None, num_splits: int | None) -> tuple[int, int]:

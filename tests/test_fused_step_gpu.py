@@ -221,3 +221,47 @@ def test_fused_batchtopk_matches_autograd(gate, k):
     for name in ("W_D", "W_E"):
         a, b = getattr(ref, name).detach().float(), getattr(fused_model, name).detach().float()
         assert torch.nn.functional.cosine_similarity(a.flatten(), b.flatten(), dim=0) > 0.999, name
+
+
+@pytest.mark.parametrize("weighted,gate,bias", [(False, True, True), (True, True, False), (True, False, True)])
+@pytest.mark.parametrize("B,k,expansion,route", [(300, 9, 8, 0), (257, 32, 32, 1), (1024, 70, 40, 2), (300, 100, 64, 3), (300, 100, 8, 4), (300, 300, 8, 4)])
+def test_one_native_call_is_the_same_step(B, k, expansion, route, weighted, gate, bias):
+    """The step in one native call against the same kernels called one by one (which phase timing asks for), for every way to find the codes."""
+    a = _model(k=k, expansion=expansion, gate=gate, bias=bias)
+    b = copy.deepcopy(a)
+    one, by_one = FusedTopKSAEStep(a), FusedTopKSAEStep(b)
+    assert K.topk_route(B, one.F, one.d, k, one.dec_norm if gate else None) == route
+    w = (torch.rand(B, device="cuda") < 0.8).float() if weighted else None
+    for i, x in enumerate(_data(3, B, 256)):
+        by_one.start_phase_timing()
+        la = one.step(x, x, k, 1e-5, row_weight=w, n_tokens_global=B if weighted else None)
+        lb = by_one.step(x, x, k, 1e-5, row_weight=w, n_tokens_global=B if weighted else None)
+        assert by_one.phase_marks and one.t == by_one.t == i + 1
+        # (sums of rows' losses by atomics; later steps start from parameters of which some differ by up to twice the learning rate)
+        # row_topk takes any of the equal bf16 values that compete for a row's last place: a few rows' losses change by one of k codes
+        assert torch.allclose(la, lb, rtol=5e-3 if route >= 3 else 1e-5 if i == 0 else 1e-4)
+        # features' entries come in the order of the counting sort's atomics: fp32 sums in another order, and Adam's first steps move a
+        # parameter by the learning rate whatever its gradient's size
+        for (n, p), q in zip(a.named_parameters(), b.parameters()):
+            off = (p - q).abs()
+            assert float(off.max()) <= 2.1e-5 * (i + 1) and (route >= 3 or float(off.mean()) <= 1e-6 * (i + 1)), n
+    K.check_status(torch.device("cuda"))
+
+
+def test_step_under_capture():
+    """A captured step replays: what it needs comes from the graph's pool, and nothing in it waits for the host."""
+    sae = _model()
+    engine = FusedTopKSAEStep(sae)
+    x = _data(1, 512, 256)[0]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        first = float(engine.step(x, x, 16, 1e-3))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            loss = engine.step(x, x, 16, 1e-3)
+        losses = []
+        for _ in range(5):
+            graph.replay()
+            losses.append(float(loss))
+    torch.cuda.synchronize()
+    assert losses[0] < first and all(q < p for p, q in zip(losses, losses[1:])), (first, losses)
