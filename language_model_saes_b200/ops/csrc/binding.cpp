@@ -1156,6 +1156,25 @@ void chunk_compact(const Tensor& x, const Tensor& maxima, const Tensor& thr, con
              "chunk_compact launch");
 }
 
+// Lists [B, cap] of the values above thr and of n_ties (int64, one element) values equal to it, the first of them; nnz: the rows' full counts. overflow
+// (int64, one element, optional): the number of rows with more than cap is added.
+void chunk_lists(const Tensor& x, const Tensor& maxima, const Tensor& thr, const Tensor& n_ties, const c10::optional<Tensor>& col_div, const Tensor& nnz,
+                 const Tensor& idx, const Tensor& val, const c10::optional<Tensor>& overflow) {
+  CHECK_T(x, torch::kBFloat16); CHECK_T(thr, torch::kFloat32); CHECK_T(n_ties, torch::kInt64); CHECK_T(nnz, torch::kInt32); CHECK_T(idx, torch::kInt32); CHECK_T(val, torch::kFloat32);
+  TORCH_CHECK(x.dim() == 2 && x.size(1) < (1LL << 30) && x.size(0) < (1LL << 31) && nnz.numel() == x.size(0) && thr.numel() >= 1 && n_ties.numel() >= 1 && idx.dim() == 2 &&
+              idx.size(0) == x.size(0) && idx.size(1) < (1LL << 31) && val.sizes() == idx.sizes(), "chunk_lists: sizes");
+  if (col_div.has_value()) { CHECK_T(*col_div, torch::kFloat32); TORCH_CHECK(col_div->numel() == x.size(1), "one divisor per column"); }
+  if (overflow.has_value()) { CHECK_T(*overflow, torch::kInt64); TORCH_CHECK(overflow->numel() == 1); }
+  const float* m = checked_maxima(maxima, x.size(0), x.size(1));
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Tensor scratch = torch::empty({2 * x.size(0)}, nnz.options());
+  check_cuda(lmsae::chunk_lists_launch(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), m, maxima.size(1), (int)x.size(0), (int)x.size(1), thr.data_ptr<float>(),
+                                       reinterpret_cast<const long long*>(n_ties.data_ptr<int64_t>()), opt_ptr<const float>(col_div), nnz.data_ptr<int>(), scratch.data_ptr<int>(),
+                                       scratch.data_ptr<int>() + x.size(0), (int)idx.size(1), idx.data_ptr<int>(), val.data_ptr<float>(),
+                                       overflow.has_value() ? reinterpret_cast<unsigned long long*>(overflow->data_ptr<int64_t>()) : nullptr, at::cuda::getCurrentCUDAStream()),
+             "chunk_lists launch");
+}
+
 void row_compact(const Tensor& x, const c10::optional<Tensor>& idx, const c10::optional<Tensor>& val,
                  const c10::optional<Tensor>& nnz, const c10::optional<Tensor>& thr, const c10::optional<Tensor>& col_div,
                  const c10::optional<Tensor>& ties, const c10::optional<Tensor>& tie_quota,
@@ -1610,6 +1629,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_compact", &row_compact);
   m.def("chunk_hist", &chunk_hist);
   m.def("chunk_compact", &chunk_compact);
+  m.def("chunk_lists", &chunk_lists);
   m.def("jumprelu_window_grad", &jumprelu_window_grad);
   m.def("rotary_pair", &rotary_pair);
   m.def("exclusive_scan", &exclusive_scan);

@@ -346,6 +346,8 @@ int chunk_hist_launch(const __nv_bfloat16* x, const float* maxima, long long ld_
                       cudaStream_t stream);
 int chunk_compact_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* thr, const float* col_div, int* nnz,
                          int* ties, const int* tie_quota, int cap, int* idx, float* val, cudaStream_t stream);
+int chunk_lists_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* thr, const long long* n_ties,
+                       const float* col_div, int* nnz, int* ties, int* quota, int cap, int* idx, float* val, unsigned long long* overflow, cudaStream_t stream);
 
 // Row top-k of stored pre-activations (one of H16, H32) by the maxima of 32 columns; sorted: values in descending order.
 int row_select_launch(const __nv_bfloat16* H16, const float* H32, long long ldh, const float* maxima, long long ld_maxima, int M, int N, int k,

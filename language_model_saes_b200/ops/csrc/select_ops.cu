@@ -192,7 +192,16 @@ radix_pick_kernel(const unsigned* __restrict__ hist, int nbins, long long k, con
   // thread i owns bins [hi - per, hi) counted from the top, so that a scan over threads walks downwards
   const int hi = nbins - (int)threadIdx.x * per;
   long long mine = 0;
-  for (int b = hi - 1; b >= hi - per && b >= 0; --b) mine += hist[b];
+  if (per % 4 == 0 && hi >= per && (reinterpret_cast<uintptr_t>(hist) & 15) == 0) {  // (all loads before the first is used: one after the other they took 19 us)
+    const uint4* h4 = reinterpret_cast<const uint4*>(hist + hi - per);
+#pragma unroll 8
+    for (int i = 0; i < per / 4; ++i) {
+      const uint4 v = h4[i];
+      mine += ((long long)v.x + v.y) + ((long long)v.z + v.w);
+    }
+  } else {
+    for (int b = hi - 1; b >= hi - per && b >= 0; --b) mine += hist[b];
+  }
   // inclusive scan over the threads: within the warp, then over the warps' totals
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   long long run_incl = mine;

@@ -39,19 +39,19 @@ def _kernel_ok(x: torch.Tensor) -> bool:
 def maxima_pay_for_threshold(B: int, N: int, k: int) -> bool:
     """Whether the floored histogram of a batch-level selection of ``k`` codes per row is faster by the maxima of 32 columns (and a floor of nine
     tenths of the previous threshold, below which few groups lie) than over the whole matrix (and a floor of three quarters). It is where the
-    matrix is large and few of its groups hold a code (us, by maxima and whole; B x N, k: 2048 x 16384, 64: 83, 87; 1024 x 32768, 128: 85, 87;
-    4096 x 32768, 64: 122, 179; 8192 x 65536, 64: 198, 506; below the lines 2048 x 16384, 128: 95, 89; 2048 x 8192, 32: 81, 71; 512 x 16384, 32:
-    75, 62; 4096 x 4096, 64: 97, 71). When the threshold falls by more than the floor allows for, a second pass reads the whole matrix: 4096 x 32768, 64:
-    222 us."""
-    return N >= 256 * k and B * N >= 1 << 25
+    matrix is more than what launches cost and few of its groups hold a code (us, by maxima and whole; B x N, k: 512 x 16384, 32: 24, 30; 1024 x 8192,
+    64: 28, 30; 2048 x 8192, 32: 28, 38; 4096 x 32768, 64: 48, 143; 8192 x 65536, 64: 101, 460; at the lines 2048 x 4096, 64: 30, 30; 1024 x 8192, 128: 32, 30;
+    below them 1024 x 4096, 64: 28, 26; 4096 x 4096, 128: 40, 40; 128 x 8192, 32: 24, 22). When the threshold falls by more than the floor allows for, a
+    second pass reads the whole matrix."""
+    return N >= 64 * k and B * N >= 1 << 23
 
 
 def maxima_pay_for_lists(B: int, N: int, k: int) -> bool:
-    """Whether the lists of a batch-level selection are made faster by the maxima of 32 columns, a warp per row and a group per code, than by CTAs
-    that read whole rows. It is where many rows share the time of a warp's row (us, by maxima and whole; 4096 x 16384, 32: 157, 200; 4096 x 32768,
-    64: 247, 308; 2048 x 65536, 32: 210, 226; 8192 x 65536, 64: 380, 818; 4096 x 131072, 128: 648, 749; beyond the lines 2048 x 16384, 16: 120, 126; 4096 x
-    16384, 64: 208, 216; 1024 x 65536, 16: 159, 146; 1024 x 65536, 64: 302, 169; 4096 x 32768, 128: 384, 339; 8192 x 8192, 128: 280, 241)."""
-    return N >= 128 * k and ((B >= 64 * k and B * B * N >= k << 33) or (B >= 32 * k and B * N >= 1 << 29))
+    """Whether the lists of a batch-level selection are made faster by the maxima of 32 columns, in one pass by a warp per row, than by two passes of CTAs
+    that read whole rows and the quotas in between. They were at every size of a grid from 128 x 4096 to 8192 x 131072 with at least 32 columns per
+    code (us, by maxima and whole; 128 x 4096, 16: 15, 105; 8192 x 4096, 128: 67, 194; 1024 x 65536, 64: 67, 157; 1024 x 131072, 128: 237, 243; 4096 x 65536, 64: 85, 419;
+    8192 x 131072, 128: 237, 1357)."""
+    return N >= 32 * k
 
 
 @torch.no_grad()
@@ -92,29 +92,36 @@ def positive_thresholds(x3: torch.Tensor, k: int, group=None, return_remaining: 
     ext = K._ext()
     dev = x3.device
     nhi = int(ext.radix_hi_bins())
+    thr = torch.empty(S, dtype=torch.float32, device=dev)
+    half = x3.dtype == torch.bfloat16  # 16-bit data: the first level already resolves the value
+    floored = floor is not None and half and S == 1
+    if floored:  # everything that starts at zero in one fill: selections, the histogram and the one of the repeat
+        zeros = torch.zeros(8 + nhi, dtype=torch.int64, device=dev)
+        sel0, hist_hi, again = zeros[:4], zeros[8 : 8 + nhi // 2].view(torch.int32), zeros[8 + nhi // 2 :].view(torch.int32)[:nhi]
+        if maxima is not None:
+            ext.chunk_hist(x3.view(maxima.shape[0], -1), maxima, floor.reshape(1).float(), hist_hi)
+        else:
+            ext.radix_hist(x3, A, S, N, 0, 0, None, hist_hi, floor.reshape(1).float(), None)
+        if world > 1:
+            dist.all_reduce(hist_hi, group=group)
+        ext.radix_pick(hist_hi, nhi, int(k), None, 0, sel0, thr, None)
+        # the repeat without the floor: both kernels return at once unless sel0[3] says the floor was too high
+        ext.radix_hist(x3, A, S, N, 0, 0, None, again, None, sel0)
+        if world > 1:
+            dist.all_reduce(again, group=group)
+        ext.radix_pick(again, nhi, int(k), None, 0, sel0, thr, sel0)
+        return (thr, sel0[1:2]) if return_remaining else thr
     hist_hi = torch.empty(nhi, dtype=torch.int32, device=dev)
     hist_lo = torch.empty(65536, dtype=torch.int32, device=dev)
     sel0 = torch.zeros(4, dtype=torch.int64, device=dev)
     sel1 = torch.zeros(4, dtype=torch.int64, device=dev)
-    thr = torch.empty(S, dtype=torch.float32, device=dev)
     remaining = torch.zeros(S, dtype=torch.int64, device=dev)
-    half = x3.dtype == torch.bfloat16  # 16-bit data: the first level already resolves the value
-    floored = floor is not None and half and S == 1
     for s in range(S):
         hist_hi.zero_()
-        if floored and maxima is not None:
-            ext.chunk_hist(x3.view(maxima.shape[0], -1), maxima, floor.reshape(1).float(), hist_hi)
-        else:
-            ext.radix_hist(x3, A, S, N, s, 0, None, hist_hi, floor.reshape(1).float() if floored else None, None)
+        ext.radix_hist(x3, A, S, N, s, 0, None, hist_hi, None, None)
         if world > 1:
             dist.all_reduce(hist_hi, group=group)
         ext.radix_pick(hist_hi, nhi, int(k), None, 0, sel0, thr[s : s + 1] if half else None, None)
-        if floored:  # the repeat without the floor: both kernels return at once unless sel0[3] says the floor was too high
-            hist_hi.zero_()
-            ext.radix_hist(x3, A, S, N, s, 0, None, hist_hi, None, sel0)
-            if world > 1:
-                dist.all_reduce(hist_hi, group=group)
-            ext.radix_pick(hist_hi, nhi, int(k), None, 0, sel0, thr[s : s + 1], sel0)
         if not half:
             hist_lo.zero_()
             ext.radix_hist(x3, A, S, N, s, 1, sel0, hist_lo, None, None)
@@ -235,6 +242,12 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
     g = g.contiguous()
     B = g.shape[0]
     nnz = torch.empty(B, dtype=torch.int32, device=g.device)
+    if (maxima is not None and n_ties is not None and cap is not None and cap % 8 == 0 and cap > 0 and (tie_group is None or dist.get_world_size(tie_group) == 1)
+            and (overflow is None or overflow.dtype == torch.int64)):  # fmt: skip
+        idx = torch.empty(B, cap, dtype=torch.int32, device=g.device)
+        val = torch.empty(B, cap, dtype=torch.float32, device=g.device)
+        ext.chunk_lists(g, maxima, thr, n_ties.reshape(-1).to(torch.int64), col_div, nnz, idx, val, overflow)
+        return idx, val
     quota = seg = None
     if n_ties is None:
         if cap is None:

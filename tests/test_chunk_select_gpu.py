@@ -114,3 +114,27 @@ def test_maxima_are_used_where_they_pay(B, N, k):
     for fn, rule in ((threshold, S.maxima_pay_for_threshold), (lists, S.maxima_pay_for_lists)):
         taken = rule(B, N, k)
         assert best(fn, taken) < 1.3 * best(fn, not taken), (fn.__name__, taken)
+
+
+@pytest.mark.parametrize("B,N", [(1, 33), (9, 4100), (5000, 1000), (33, 4133)])
+@pytest.mark.parametrize("data", ["normal", "all equal", "one step", "nan"])
+def test_lists_in_one_pass_with_quotas_afterwards(B, N, data):
+    """Rows that are not whole vectors, more rows than a turn of the quotas takes, rows of equal values that overflow the list before the quota is taken
+    out, and quotas that end within a row, at a row's end, at none and at all of them."""
+    g = torch.Generator(device=DEV).manual_seed(B)
+    x = torch.randn(B, N, device=DEV, generator=g)
+    x = (torch.ones_like(x) if data == "all equal" else (x > 1).float() + 1 if data == "one step" else x).to(torch.bfloat16)
+    if data == "nan":
+        x[B // 2, N // 2] = float("nan")
+    groups = -(-N // 256) * 8
+    padded = torch.zeros(B, groups * 32, dtype=torch.bfloat16, device=DEV)
+    padded[:, :N] = x
+    maxima = padded.view(B, groups, 32).float().amax(2).contiguous()
+    thr = x.float().nan_to_num(nan=0.0).flatten().topk(max(1, B * N // 50)).values[-1].reshape(1)
+    ties = int((x.float() == thr).sum())
+    for n_ties in {0, 1, ties // 2, int((x[0].float() == thr).sum()), ties}:
+        want_n, got_n = (torch.zeros(1, dtype=torch.int64, device=DEV) for _ in range(2))
+        n = torch.tensor([n_ties], device=DEV)
+        want = S.threshold_rows_to_sparse(x, thr, None, n_ties=n, cap=24, overflow=want_n)
+        got = S.threshold_rows_to_sparse(x, thr, None, n_ties=n, cap=24, overflow=got_n, maxima=maxima)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(nan=7.0), want[1].nan_to_num(nan=7.0)) and torch.equal(got_n, want_n), n_ties
