@@ -426,6 +426,17 @@ void row_topk(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate, con
              "row_topk launch");
 }
 
+// dense [M, N] bf16: the k largest positive values of H * gate per row, as H has them, and zeros
+void row_topk_dense(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate, const Tensor& dense) {
+  CHECK_T(H, torch::kBFloat16); CHECK_T(dense, torch::kBFloat16);
+  TORCH_CHECK(H.dim() == 2 && dense.sizes() == H.sizes() && H.size(0) < (1LL << 31) && H.size(1) < (1LL << 31) && H.size(1) % 8 == 0 && k >= 1 && k < (1LL << 31), "row_topk_dense: sizes");
+  if (gate.has_value()) { CHECK_T(*gate, torch::kFloat32); TORCH_CHECK(gate->numel() == H.size(1)); }
+  const c10::cuda::CUDAGuard guard(H.device());
+  check_cuda(lmsae::row_topk_dense_launch(reinterpret_cast<const __nv_bfloat16*>(H.data_ptr()), (int)H.size(0), (int)H.size(1), (int)k, opt_ptr<const float>(gate),
+                                          reinterpret_cast<__nv_bfloat16*>(dense.data_ptr()), at::cuda::getCurrentCUDAStream()),
+             "row_topk_dense launch");
+}
+
 // Row top-k (k <= 128) of H (bf16 or fp32 [M, N], N % 8 == 0) by its gated maxima of every 32 columns.
 bool row_select_fits(const Tensor& H, int64_t k, const c10::optional<Tensor>& gate) {
   return k >= 1 && k <= lmsae::row_select_max_k() && H.size(1) % 8 == 0 && H.size(1) <= 65535 * 32 && reinterpret_cast<uintptr_t>(H.data_ptr()) % 16 == 0 &&
@@ -1639,6 +1650,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("row_topk_dense", &row_topk_dense);
   m.def("row_select", &row_select);
   m.def("row_select_fits", &row_select_fits);
   m.def("topk_dense", &topk_dense);

@@ -115,6 +115,7 @@ struct RowsProductParams {
 int rows_product_launch(RowsProductParams p, bool b_by_k, cudaStream_t stream);
 int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int most, int* todo, float* part, long long part_floats, int part_tiles,
                         float* out, cudaStream_t stream);
+int row_topk_dense_launch(const __nv_bfloat16* H, int M, int N, int k, const float* gate, __nv_bfloat16* dense, cudaStream_t stream);
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,
                     const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream);
 

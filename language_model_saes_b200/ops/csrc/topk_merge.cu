@@ -254,7 +254,8 @@ __device__ __forceinline__ void gated_values8(const __nv_bfloat16* __restrict__ 
 // The radix descent over the row: 4 passes of 8 bits, 256-bin histogram in shared memory, then one pass over the survivors.
 template <typename T>
 __device__ __noinline__ void row_topk_radix(const T* __restrict__ hrow, int row, int N, int k, const float* __restrict__ gate,
-                                            const uint8_t* __restrict__ alive, int* __restrict__ out_idx, float* __restrict__ out_val) {
+                                            const uint8_t* __restrict__ alive, int* __restrict__ out_idx, float* __restrict__ out_val,
+                                            __nv_bfloat16* __restrict__ dense_row = nullptr) {
   __shared__ unsigned hist[256];
   __shared__ unsigned s_prefix, s_remaining, s_count_gt, s_cursor_gt, s_cursor_eq;
   unsigned prefix = 0;     // bits decided so far (from the top)
@@ -304,7 +305,7 @@ __device__ __noinline__ void row_topk_radix(const T* __restrict__ hrow, int row,
     s_cursor_eq = 0;
     s_count_gt = fewer_than_k ? 0u : (unsigned)k - remaining;
   }
-  for (int i = threadIdx.x; i < k; i += RT_THREADS) {
+  for (int i = threadIdx.x; i < k && dense_row == nullptr; i += RT_THREADS) {
     out_idx[(size_t)row * k + i] = -1;
     out_val[(size_t)row * k + i] = 0.0f;
   }
@@ -321,8 +322,13 @@ __device__ __noinline__ void row_topk_radix(const T* __restrict__ hrow, int row,
         if (e < remaining) pos = (int)(s_count_gt + e);
       }
       if (pos >= 0 && pos < k) {
-        out_idx[(size_t)row * k + pos] = c;
-        out_val[(size_t)row * k + pos] = (gate != nullptr) ? v / gate[c] : v;
+        const float a = (gate != nullptr) ? v / gate[c] : v;
+        if (dense_row != nullptr) {
+          dense_row[c] = __float2bfloat16(a);
+        } else {
+          out_idx[(size_t)row * k + pos] = c;
+          out_val[(size_t)row * k + pos] = a;
+        }
       }
     }
   }
@@ -362,15 +368,21 @@ __device__ __forceinline__ unsigned descend(const unsigned (&val)[N], int k, int
 
 // MAXIMA: the largest gated value of every 32 columns comes with H (the encoder GEMM's epilogue leaves them): those are the column groups,
 // and only groups whose maximum reaches the bound are read at all: 4096 rows of 32768, k 128, with a gate: 195 -> 111 us (211 -> 135 without).
-template <bool MAXIMA>
+// DENSE: instead of lists the row itself, bf16, zero where nothing was selected (an operand of products over the columns: Aux-K's codes over a dictionary of
+// dead features, 4096 rows of 9216, k 512: 136 us and 92 for fill, conversions and scatter -> 139).
+template <bool MAXIMA, bool DENSE = false>
 __global__ void __launch_bounds__(RT_THREADS, 5)
 row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N, int k,
                 const float* __restrict__ gate, const uint8_t* __restrict__ alive, const float* __restrict__ maxima, long long ld_maxima, int vec,
-                int* __restrict__ out_idx, float* __restrict__ out_val) {
+                int* __restrict__ out_idx, float* __restrict__ out_val, __nv_bfloat16* __restrict__ dense) {
   pdl_wait();
   const int row = blockIdx.x;
   if (row >= M) return;
   const __nv_bfloat16* hrow = H + (long long)row * ldh;
+  __nv_bfloat16* dense_row = DENSE ? dense + (size_t)row * N : nullptr;
+  if constexpr (DENSE) {  // (N % 8 == 0; barriers lie between these and what is written over them)
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) *reinterpret_cast<uint4*>(dense_row + c) = make_uint4(0u, 0u, 0u, 0u);
+  }
   __shared__ unsigned s_bits[RT_CAP];
   __shared__ int s_col[RT_CAP];
   __shared__ unsigned s_count[2][RT_WARPS];
@@ -476,8 +488,13 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
         if (pos < k) {
           const int c = s_col[j];
           const float v = __uint_as_float(s_bits[j]);
-          out_idx[(size_t)row * k + pos] = c;
-          out_val[(size_t)row * k + pos] = gate != nullptr ? v / gate[c] : v;
+          const float a = gate != nullptr ? v / gate[c] : v;
+          if constexpr (DENSE) {
+            dense_row[c] = __float2bfloat16(a);
+          } else {
+            out_idx[(size_t)row * k + pos] = c;
+            out_val[(size_t)row * k + pos] = a;
+          }
         }
       };
       for (int j = threadIdx.x; j < n_cand; j += RT_THREADS)
@@ -485,14 +502,14 @@ row_topk_kernel(const __nv_bfloat16* __restrict__ H, long long ldh, int M, int N
       __syncthreads();
       for (int j = threadIdx.x; j < n_cand; j += RT_THREADS)
         if (s_bits[j] == thr) place(j);
-      for (int j = n_cand + threadIdx.x; j < k; j += RT_THREADS) {
+      for (int j = n_cand + threadIdx.x; j < k && !DENSE; j += RT_THREADS) {
         out_idx[(size_t)row * k + j] = -1;
         out_val[(size_t)row * k + j] = 0.0f;
       }
       return;
     }
   }
-  row_topk_radix(hrow, row, N, k, gate, alive, out_idx, out_val);
+  row_topk_radix(hrow, row, N, k, gate, alive, out_idx, out_val, dense_row);
 }
 
 // Row top-k of stored pre-activations whose gated maxima per 32 columns are known, a warp per row (the encoder GEMM's epilogue leaves
@@ -764,9 +781,16 @@ int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, 
                     const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream) {
   const bool vec = N % 8 == 0 && ldh % 8 == 0 && reinterpret_cast<uintptr_t>(H) % 16 == 0 && reinterpret_cast<uintptr_t>(gate) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(alive) % 8 == 0;
-  if (maxima != nullptr) launch(row_topk_kernel<true>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, maxima, ld_maxima, vec ? 1 : 0, out_idx, out_val);
-  else launch(row_topk_kernel<false>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, nullptr, 0, vec ? 1 : 0, out_idx, out_val);
+  if (maxima != nullptr) launch(row_topk_kernel<true>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, maxima, ld_maxima, vec ? 1 : 0, out_idx, out_val, nullptr);
+  else launch(row_topk_kernel<false>, M, RT_THREADS, 0, stream, H, ldh, M, N, k, gate, alive, nullptr, 0, vec ? 1 : 0, out_idx, out_val, nullptr);
   return (int)cudaGetLastError();
+}
+
+int row_topk_dense_launch(const __nv_bfloat16* H, int M, int N, int k, const float* gate, __nv_bfloat16* dense, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (N % 8 != 0 || (reinterpret_cast<uintptr_t>(dense) & 15) != 0) return (int)cudaErrorInvalidValue;
+  const bool vec = ((reinterpret_cast<uintptr_t>(H) | reinterpret_cast<uintptr_t>(gate)) & 15) == 0;
+  return (int)launch(row_topk_kernel<false, true>, M, RT_THREADS, 0, stream, H, N, M, N, k, gate, nullptr, nullptr, 0, vec ? 1 : 0, nullptr, nullptr, dense);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -704,16 +704,21 @@ class FusedTopKSAEStep:
         # gathering a decoder row per code, so the auxiliary decode and its three gradients are dense over the compact
         # dictionary and only their result rows are handed to the update kernel.
         # (the selection itself: fused into the GEMM epilogue up to 64 codes, else over stored bf16 pre-activations)
-        idx_c, act_aux = K.encoder_topk(x, w_dead, b_dead, g_dead, aux.k_aux)
+        as_matrix = x.is_cuda and self.tp == 1 and aux.k_aux > 64 and not K.maxima_pay(cap, aux.k_aux)  # (the lists are not wanted then)
+        if as_matrix:
+            A = K.row_topk_dense(K.encoder_hidden(x, w_dead, b_dead), aux.k_aux, g_dead)
+        else:
+            idx_c, act_aux = K.encoder_topk(x, w_dead, b_dead, g_dead, aux.k_aux)
         self._mark("aux_encoder_topk")
         if self.tp > 1:
             idx_c, act_aux = self._merge_shard_codes(idx_c, act_aux, g_dead, aux.k_aux)
             self._mark("aux_merge_shards")
         # dense dead activations; empty slots land in a dump column behind them (eight columns of padding: the rows of
         # the [B, cap] view below stay 16-byte aligned, which the library GEMMs need to run their fast kernels)
-        A = torch.zeros(B, cap + 8, dtype=torch.bfloat16, device=x.device)
-        A.scatter_(1, torch.where(idx_c >= 0, idx_c, torch.full_like(idx_c, cap)).long(), act_aux.to(torch.bfloat16))
-        A = A[:, :cap]
+        if not as_matrix:
+            A = torch.zeros(B, cap + 8, dtype=torch.bfloat16, device=x.device)
+            A.scatter_(1, torch.where(idx_c >= 0, idx_c, torch.full_like(idx_c, cap)).long(), act_aux.to(torch.bfloat16))
+            A = A[:, :cap]
         aux_rec = _mm_f32(A, wd_dead)
         if self.tp > 1:  # both reconstructions are sums over the shards' features
             both = torch.stack([xhat, aux_rec])

@@ -399,6 +399,17 @@ def row_topk(
     return out_idx, out_val
 
 
+def row_topk_dense(H: torch.Tensor, k: int, gate: torch.Tensor | None = None) -> torch.Tensor:
+    """``row_topk`` as a matrix like ``H`` (bf16) that is zero where nothing was selected."""
+    if not H.is_cuda or H.shape[1] % 8 != 0:
+        idx, act = row_topk(H, k, gate)
+        out = torch.zeros(H.shape[0], H.shape[1] + 1, dtype=torch.bfloat16, device=H.device)
+        return out.scatter_(1, torch.where(idx >= 0, idx, torch.full_like(idx, H.shape[1])).long(), act.to(torch.bfloat16))[:, :-1]
+    out = torch.empty(H.shape, dtype=torch.bfloat16, device=H.device)
+    _ext().row_topk_dense(H.contiguous(), k, gate, out)
+    return out
+
+
 # --------------------------------------------------------------------------------------------------
 # decoder
 # --------------------------------------------------------------------------------------------------

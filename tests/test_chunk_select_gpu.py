@@ -138,3 +138,24 @@ def test_lists_in_one_pass_with_quotas_afterwards(B, N, data):
         want = S.threshold_rows_to_sparse(x, thr, None, n_ties=n, cap=24, overflow=want_n)
         got = S.threshold_rows_to_sparse(x, thr, None, n_ties=n, cap=24, overflow=got_n, maxima=maxima)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(nan=7.0), want[1].nan_to_num(nan=7.0)) and torch.equal(got_n, want_n), n_ties
+
+
+@pytest.mark.parametrize("M,N,k", [(1, 8, 3), (5, 2048, 512), (300, 4104, 100), (40, 9216, 512), (3, 3000, 1500)])
+@pytest.mark.parametrize("data", ["normal", "few positive", "ties", "no gate"])
+def test_row_topk_as_a_matrix(M, N, k, data):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    H = torch.randn(M, N, device=DEV, generator=g).to(torch.bfloat16)
+    gate = None if data == "no gate" else torch.rand(N, device=DEV, generator=g) + 0.5
+    if gate is not None:
+        gate[:: 3] = 0.0
+    if data == "few positive":
+        H = (H - 3.0).to(torch.bfloat16)
+    elif data == "ties":
+        H = (H > 0.5).to(torch.bfloat16)
+        gate = torch.ones_like(gate)
+    out = K.row_topk_dense(H, k, gate)
+    idx, act = K.row_topk(H, k, gate)
+    want = torch.zeros(M, N + 1, device=DEV).scatter_(1, torch.where(idx >= 0, idx, torch.full_like(idx, N)).long(), act)[:, :N].to(torch.bfloat16)
+    if data == "ties" or gate is None:  # (which of equal values are taken is free)
+        out, want = out.sort(1).values, want.sort(1).values
+    assert torch.equal(out, want)
