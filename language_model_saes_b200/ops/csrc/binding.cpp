@@ -1064,6 +1064,36 @@ void adam_turned(const std::vector<Tensor>& p, const std::vector<Tensor>& m, con
   check_cuda(lmsae::adam_turned_launch(q, (int)n, at::cuda::getCurrentCUDAStream()), "adam_turned launch");
 }
 
+// ---- Aux-K ----------------------------------------------------------------------------------------------
+// fired int32 [F] (counts of the step), since int64 [F], n_valid int64 (one element) -> {since [F], is_dead bool [F], n_dead int64 [], any fp32 [1], order int32 [cap],
+// row_of int32 [F], WE rows, WD rows [cap, d] bf16, bias [cap], gate [cap]}; truncated int64 (one element) gets one more where more than capacity are dead.
+std::vector<Tensor> dead_rows(const Tensor& fired, const Tensor& since, const Tensor& n_valid, int64_t threshold, int64_t cap, int64_t capacity, const Tensor& WE,
+                              const Tensor& WD, const Tensor& bias, const c10::optional<Tensor>& gate, const Tensor& truncated) {
+  CHECK_T(fired, torch::kInt32); CHECK_T(since, torch::kInt64); CHECK_T(n_valid, torch::kInt64); CHECK_T(WE, torch::kBFloat16); CHECK_T(WD, torch::kBFloat16);
+  CHECK_T(bias, torch::kFloat32); CHECK_T(truncated, torch::kInt64);
+  const int64_t F = fired.numel(), d = WE.dim() == 2 ? WE.size(1) : 0;
+  TORCH_CHECK(F > 0 && F < INT_MAX - 1024 && since.numel() == F && n_valid.numel() == 1 && truncated.numel() == 1 && cap > 0 && cap < INT_MAX && WE.dim() == 2 && WE.size(0) == F &&
+              WD.sizes() == WE.sizes() && d % 8 == 0 && bias.numel() == F, "dead_rows: sizes");
+  if (gate.has_value()) { CHECK_T(*gate, torch::kFloat32); TORCH_CHECK(gate->numel() == F); }
+  const c10::cuda::CUDAGuard guard(fired.device());
+  const auto i32 = fired.options(), i64 = since.options(), f32 = bias.options();
+  const Tensor since_out = torch::empty_like(since), is_dead = torch::empty({F}, i32.dtype(torch::kBool)), n_dead = torch::empty({}, i64), any = torch::empty({1}, f32),
+               order = torch::empty({cap}, i32), row_of = torch::empty({F}, i32), we = torch::empty({cap, d}, WE.options()), wd = torch::empty({cap, d}, WE.options()),
+               b = torch::empty({cap}, f32), g = torch::empty({cap}, f32), blocks = torch::empty({lmsae::dead_rows_blocks((int)F)}, i32);
+  lmsae::DeadRowsParams p{};
+  p.F = (int)F; p.cap = (int)cap; p.capacity = capacity;
+  p.is_dead = reinterpret_cast<uint8_t*>(is_dead.data_ptr<bool>()); p.block_count = blocks.data_ptr<int>();
+  p.bias = bias.data_ptr<float>(); p.gate = opt_ptr<const float>(gate);
+  p.order = order.data_ptr<int>(); p.bias_out = b.data_ptr<float>(); p.gate_out = g.data_ptr<float>(); p.row_of = row_of.data_ptr<int>();
+  p.n_dead = reinterpret_cast<long long*>(n_dead.data_ptr<int64_t>()); p.truncated = reinterpret_cast<long long*>(truncated.data_ptr<int64_t>()); p.any = any.data_ptr<float>();
+  check_cuda(lmsae::dead_rows_launch(p, fired.data_ptr<int>(), reinterpret_cast<const long long*>(since.data_ptr<int64_t>()),
+                                     reinterpret_cast<const long long*>(n_valid.data_ptr<int64_t>()), threshold, reinterpret_cast<long long*>(since_out.data_ptr<int64_t>()),
+                                     reinterpret_cast<const __nv_bfloat16*>(WE.data_ptr()), reinterpret_cast<const __nv_bfloat16*>(WD.data_ptr()), (int)d,
+                                     reinterpret_cast<__nv_bfloat16*>(we.data_ptr()), reinterpret_cast<__nv_bfloat16*>(wd.data_ptr()), at::cuda::getCurrentCUDAStream()),
+             "dead_rows launch");
+  return {since_out, is_dead, n_dead, any, order, row_of, we, wd, b, g};
+}
+
 // ---- selection / compaction ----------------------------------------------------------------------------
 int dtype_code(const Tensor& t) {
   if (t.scalar_type() == torch::kFloat32) return 0;
@@ -1650,6 +1680,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("dead_rows", &dead_rows);
   m.def("row_topk_dense", &row_topk_dense);
   m.def("row_select", &row_select);
   m.def("row_select_fits", &row_select_fits);

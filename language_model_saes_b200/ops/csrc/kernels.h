@@ -372,6 +372,23 @@ struct AdamTurnedParams {
 };
 int adam_turned_launch(const AdamTurnedParams& p, int n_sets, cudaStream_t stream);
 
+// ---- dead features of an Aux-K step (dead_rows.cu) ---------------------------------------------------------
+struct DeadRowsParams {
+  int F, cap;
+  long long capacity;
+  uint8_t* is_dead;          // [F]
+  int* block_count;          // [dead_rows_blocks(F)] scratch
+  const float *bias, *gate;  // [F]; gate nullptr: 1
+  int* order;                // [cap] the compact dictionary's rows as features, and
+  float *bias_out, *gate_out;  // [cap]
+  int* row_of;               // [F] a feature's row there, -1: none
+  long long *n_dead, *truncated;  // how many are dead; one more where that is beyond capacity
+  float* any;                // 1 where any is
+};
+int dead_rows_blocks(int F);
+int dead_rows_launch(const DeadRowsParams& p, const int* fired, const long long* since, const long long* n_valid, long long threshold, long long* since_out,
+                     const __nv_bfloat16* WE, const __nv_bfloat16* WD, int d, __nv_bfloat16* we_out, __nv_bfloat16* wd_out, cudaStream_t stream);
+
 // ---- threshold gradient of a JumpReLU head in the epilogue of its product (window_grad_gemm.cu) -------------
 struct WindowGradParams {
   int B, F, d;

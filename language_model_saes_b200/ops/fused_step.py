@@ -27,6 +27,7 @@ rebuilds the identical full-batch gradient).
 
 from __future__ import annotations
 
+import math
 import os
 
 import torch
@@ -96,6 +97,15 @@ class AuxK:
         self.is_dead = self.tokens_since_last_activation >= self.dead_threshold
         return self.is_dead
 
+    def compact(self, fired: torch.Tensor, n_valid_tokens: torch.Tensor, cap: int, WE, WD, bias, gate):
+        """``update``, ``observe`` and the compact dictionary on a GPU in three launches: ``(any [1], row_of [F], WE rows, WD rows [cap, d], bias, gate [cap])``.
+        Rows behind the dead features' have gate 0 and hold zeros."""
+        threshold = min(math.ceil(min(self.dead_threshold, 2.0**62)), 2**62)
+        (self.tokens_since_last_activation, self.is_dead, n_dead, any_dead, _, row_of, *rows) = K._ext().dead_rows(
+            fired, self.tokens_since_last_activation, n_valid_tokens, threshold, cap, self.capacity, WE, WD, bias, gate, self.truncated_steps)  # fmt: skip
+        self._feed(n_dead)
+        return any_dead, row_of, *rows
+
     LAG = 2  # steps between a count leaving the device and its use: the same on every rank, so capacities agree
 
     def observe(self, n_dead: torch.Tensor) -> None:
@@ -104,6 +114,9 @@ class AuxK:
         event returns at once). The lag is a fixed number of steps rather than "whenever the copy is seen to be done",
         because replicas and shards that exchange buffers sized by the capacity must all switch in the same step."""
         self.truncated_steps += n_dead > self.capacity
+        self._feed(n_dead)
+
+    def _feed(self, n_dead: torch.Tensor) -> None:
         if not n_dead.is_cuda:
             self.capacity = self._bucket(int(n_dead))
             return
@@ -665,36 +678,41 @@ class FusedTopKSAEStep:
             fired, n_valid = fired.clone(), n_valid.clone()
             dist.all_reduce(fired, group=self.dp_group)
             dist.all_reduce(n_valid, group=self.dp_group)
-        is_dead = aux.update(fired, n_valid)
-        n_dead = is_dead.sum()
-        cap = min(aux.capacity, -(-self.F // 8) * 8)
-        aux.observe(n_dead)
-        n_dead_all = n_dead.clone()
-        if self.tp > 1:  # the auxiliary top-k runs over the dead features of ALL shards
-            dist.all_reduce(n_dead_all, group=self.tp_group)
-        alpha_on = (n_dead_all > 0).float().reshape(1)  # no dead feature anywhere: the auxiliary term is absent, not |e|^2
-        # compact dictionary of this shard's dead features: dead rows first (ascending), alive rows behind them with gate 0
         sharded = self.dp_comm is not None
-        if sharded:
-            # One block of slots per replica's share of the feature rows, so that the dense gradient rows of the compact
-            # dictionary can be reduce-scattered over the replicas (each needs only the rows it updates).
-            cap_r = max(1, min(cap // self.dp, self.F // self.dp))
-            cap = cap_r * self.dp
-            per = self.F // self.dp
-            order = torch.argsort((~is_dead).view(self.dp, per).to(torch.int8), dim=1, stable=True)[:, :cap_r]
-            order = (order + torch.arange(self.dp, device=x.device).unsqueeze(1) * per).reshape(-1)
-            valid = is_dead[order]
+        native = x.is_cuda and self.tp == 1 and self.dp == 1 and self.d % 8 == 0 and aux.tokens_since_last_activation.dtype == torch.long
+        if native:
+            cap = min(aux.capacity, -(-self.F // 8) * 8)
+            alpha_on, row_of, w_dead, wd_dead, b_dead, g_dead = aux.compact(fired, n_valid, cap, self.WE_bf16, self.WD_bf16, self.bE, gate)
         else:
-            order = torch.argsort((~is_dead).to(torch.int8), stable=True)[:cap]
-            if order.numel() < cap:  # fewer rows than the (rounded) capacity: repeat row 0 with gate 0
-                order = torch.cat([order, order.new_zeros(cap - order.numel())])
-                valid = torch.cat([is_dead[order[: self.F]], is_dead.new_zeros(cap - self.F)])
-            else:
+            is_dead = aux.update(fired, n_valid)
+            n_dead = is_dead.sum()
+            cap = min(aux.capacity, -(-self.F // 8) * 8)
+            aux.observe(n_dead)
+            n_dead_all = n_dead.clone()
+            if self.tp > 1:  # the auxiliary top-k runs over the dead features of ALL shards
+                dist.all_reduce(n_dead_all, group=self.tp_group)
+            alpha_on = (n_dead_all > 0).float().reshape(1)  # no dead feature anywhere: the auxiliary term is absent, not |e|^2
+            # compact dictionary of this shard's dead features: dead rows first (ascending), alive rows behind them with gate 0
+            if sharded:
+                # One block of slots per replica's share of the feature rows, so that the dense gradient rows of the compact
+                # dictionary can be reduce-scattered over the replicas (each needs only the rows it updates).
+                cap_r = max(1, min(cap // self.dp, self.F // self.dp))
+                cap = cap_r * self.dp
+                per = self.F // self.dp
+                order = torch.argsort((~is_dead).view(self.dp, per).to(torch.int8), dim=1, stable=True)[:, :cap_r]
+                order = (order + torch.arange(self.dp, device=x.device).unsqueeze(1) * per).reshape(-1)
                 valid = is_dead[order]
-        w_dead = self.WE_bf16[order]
-        wd_dead = self.WD_bf16[order]
-        b_dead = self.bE[order]
-        g_dead = (gate[order] if gate is not None else torch.ones(cap, device=x.device)) * valid
+            else:
+                order = torch.argsort((~is_dead).to(torch.int8), stable=True)[:cap]
+                if order.numel() < cap:  # fewer rows than the (rounded) capacity: repeat row 0 with gate 0
+                    order = torch.cat([order, order.new_zeros(cap - order.numel())])
+                    valid = torch.cat([is_dead[order[: self.F]], is_dead.new_zeros(cap - self.F)])
+                else:
+                    valid = is_dead[order]
+            w_dead = self.WE_bf16[order]
+            wd_dead = self.WD_bf16[order]
+            b_dead = self.bE[order]
+            g_dead = (gate[order] if gate is not None else torch.ones(cap, device=x.device)) * valid
         self._mark("dead_statistics_compact_dictionary")
         self._clear_sums()
         xhat = K.sparse_decode(idx, act, self.WD_bf16, None, torch.float32)
@@ -734,7 +752,7 @@ class FusedTopKSAEStep:
         dA, extra_gb = K.mask_colsum_(g_aux @ wd_dead.t() if x.is_cuda else _mm_f32(g_aux, wd_dead.t()), A)
         extra_gD = _mm_f32(A.t(), g_aux)  # d W_D rows of the compact dictionary
         extra_gE = _mm_f32(dA.to(torch.bfloat16).t(), x)  # d W_E^T rows
-        slots = torch.arange(cap, dtype=torch.int32, device=x.device)
+        slots = torch.arange(cap, dtype=torch.int32, device=x.device) if not native else None
         if sharded:
             # dense rows: summed over replicas, each replica receiving the block of the rows it updates (the sparse main
             # part is rebuilt from the exchanged rows below)
@@ -752,9 +770,10 @@ class FusedTopKSAEStep:
             if self.dp > 1:
                 for t in (extra_gD, extra_gE, extra_gb):
                     dist.all_reduce(t, group=self.dp_group)
-            valid_mine = valid
-        row_of = torch.full((self.F,), -1, dtype=torch.int32, device=x.device)
-        row_of.scatter_(0, order.long(), torch.where(valid_mine, slots, torch.full_like(slots, -1)))
+            valid_mine = valid if not native else None
+        if not native:
+            row_of = torch.full((self.F,), -1, dtype=torch.int32, device=x.device)
+            row_of.scatter_(0, order.long(), torch.where(valid_mine, slots, torch.full_like(slots, -1)))
         self._mark("aux_gradients")
         if sharded:
             g = self.dp_comm.exchange({"x": x, "dxhat": g_main, "idx": idx, "act": act, "dact": dact})
@@ -763,7 +782,8 @@ class FusedTopKSAEStep:
         elif self.dp > 1:
             x, g_main, idx, act, dact = self._gather_rows(x, g_main, idx, act, dact)
             self._mark("dp_exchange_rows")
-        self.groups.build(idx)
+        if self.dp > 1:  # (one process: they are those of the dead statistics still)
+            self.groups.build(idx)
         self._mark("sort_by_feature")
         self.t += 1
         b1, b2 = self.betas

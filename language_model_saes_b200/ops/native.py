@@ -25,7 +25,7 @@ _CSRC = Path(__file__).resolve().parent / "csrc"
 # ``bounds_report`` of the extension) and clamped instead of read out of bounds.
 _CHECKED = os.environ.get("LMSAE_NATIVE_CHECKED", "0") == "1"
 _BUILD_DIR = Path(__file__).resolve().parent / ("_native_build_checked" if _CHECKED else "_native_build")
-_SOURCES = ["binding.cpp", "encoder_gemm.cu", "topk_merge.cu", "sparse_ops.cu", "grad_adam.cu", "grad_adam_both.cu", "comm_ops.cu", "no_alloc.cu", "jumprelu.cu", "clt_ops.cu", "crosscoder_ops.cu", "select_ops.cu", "chunk_select.cu", "attention.cu", "rotary.cu", "lorsa_ops.cu", "window_grad_gemm.cu", "dense_decode.cu", "rows_product.cu", "fp32_gemm.cu"]
+_SOURCES = ["binding.cpp", "encoder_gemm.cu", "topk_merge.cu", "sparse_ops.cu", "grad_adam.cu", "grad_adam_both.cu", "comm_ops.cu", "no_alloc.cu", "jumprelu.cu", "clt_ops.cu", "crosscoder_ops.cu", "select_ops.cu", "chunk_select.cu", "attention.cu", "rotary.cu", "lorsa_ops.cu", "dead_rows.cu", "window_grad_gemm.cu", "dense_decode.cu", "rows_product.cu", "fp32_gemm.cu"]
 _CUDA_FLAGS = [
     "-gencode",
     "arch=compute_100a,code=sm_100a",

@@ -265,3 +265,34 @@ def test_step_under_capture():
             losses.append(float(loss))
     torch.cuda.synchronize()
     assert losses[0] < first and all(q < p for p, q in zip(losses, losses[1:])), (first, losses)
+
+
+@pytest.mark.parametrize("F,cap,dead", [(8, 8, 0.5), (1000, 512, 0.2), (5003, 5008, 1.0), (4096, 1024, 0.0), (70000, 2048, 0.01), (70000, 2048, 0.1)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_dead_rows_match_the_plain_statement(F, cap, dead, gated):
+    """Blocks that end within the features, a capacity beyond them, none and all dead, more dead features than there is room for."""
+    from language_model_saes_b200.ops.fused_step import AuxK
+
+    g = torch.Generator(device="cuda").manual_seed(F)
+    d = 72
+    since = torch.randint(0, 90, (F,), device="cuda", generator=g)
+    since[torch.rand(F, device="cuda", generator=g) < dead] = 95
+    fired = (torch.rand(F, device="cuda", generator=g) < 0.1).int() * 3
+    WE, WD = (torch.randn(F, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    bias, gate = torch.randn(F, device="cuda", generator=g), torch.rand(F, device="cuda", generator=g) + 0.1 if gated else None
+    n_valid = torch.full((), 7, device="cuda")
+    a, b = (AuxK(F, 16, 1 / 32, 100.5, "cuda", counter=since.clone()) for _ in range(2))
+    a.capacity = b.capacity = cap
+    any_dead, row_of, we, wd, b_dead, g_dead = a.compact(fired, n_valid, cap, WE, WD, bias, gate)
+    is_dead = b.update(fired, n_valid)
+    b.observe(is_dead.sum())
+    assert torch.equal(a.tokens_since_last_activation, b.tokens_since_last_activation) and torch.equal(a.is_dead, is_dead)
+    assert int(a.truncated_steps) == int(b.truncated_steps) and float(any_dead) == float(is_dead.any())
+    rows = is_dead.nonzero().squeeze(1)[:cap]
+    n = rows.numel()
+    want = torch.full((F,), -1, dtype=torch.int32, device="cuda")
+    want[rows] = torch.arange(n, dtype=torch.int32, device="cuda")
+    assert torch.equal(row_of, want)
+    assert torch.equal(we[:n], WE[rows]) and torch.equal(wd[:n], WD[rows]) and not we[n:].any() and not wd[n:].any()
+    assert torch.equal(b_dead[:n], bias[rows]) and torch.isfinite(b_dead).all() and not g_dead[n:].any()
+    assert torch.equal(g_dead[:n], gate[rows] if gated else torch.ones(n, device="cuda"))
