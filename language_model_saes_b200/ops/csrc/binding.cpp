@@ -1216,6 +1216,21 @@ void chunk_lists(const Tensor& x, const Tensor& maxima, const Tensor& thr, const
              "chunk_lists launch");
 }
 
+// Lists [B, cap] of the bf16 values above their columns' thresholds, in one pass; overflow (int64, one element): the number of rows with more than cap is
+// added. False, and nothing done, where rows or thresholds are not whole aligned vectors or the lists too wide for it.
+bool column_lists(const Tensor& x, const Tensor& col_thr, const Tensor& idx, const Tensor& val, const Tensor& overflow) {
+  CHECK_T(x, torch::kBFloat16); CHECK_T(col_thr, torch::kFloat32); CHECK_T(idx, torch::kInt32); CHECK_T(val, torch::kFloat32); CHECK_T(overflow, torch::kInt64);
+  TORCH_CHECK(x.dim() == 2 && x.size(0) < (1LL << 31) && col_thr.numel() == x.size(1) && idx.dim() == 2 && idx.size(0) == x.size(0) && idx.size(1) < (1LL << 31) &&
+              val.sizes() == idx.sizes() && overflow.numel() == 1, "column_lists: sizes");
+  if (!lmsae::row_compact_cols_fits(x.data_ptr(), x.size(1), col_thr.data_ptr<float>(), (int)idx.size(1))) return false;
+  const c10::cuda::CUDAGuard guard(x.device());
+  check_cuda(lmsae::row_compact_launch(1, x.data_ptr(), (int)x.size(0), x.size(1), (int)idx.size(1), idx.data_ptr<int>(), val.data_ptr<float>(), nullptr, nullptr, nullptr,
+                                       nullptr, nullptr, col_thr.data_ptr<float>(), nullptr, reinterpret_cast<unsigned long long*>(overflow.data_ptr<int64_t>()),
+                                       at::cuda::getCurrentCUDAStream()),
+             "column_lists launch");
+  return true;
+}
+
 void row_compact(const Tensor& x, const c10::optional<Tensor>& idx, const c10::optional<Tensor>& val,
                  const c10::optional<Tensor>& nnz, const c10::optional<Tensor>& thr, const c10::optional<Tensor>& col_div,
                  const c10::optional<Tensor>& ties, const c10::optional<Tensor>& tie_quota,
@@ -1243,7 +1258,7 @@ void row_compact(const Tensor& x, const c10::optional<Tensor>& idx, const c10::o
   check_cuda(lmsae::row_compact_launch(dtype_code(x), x.data_ptr(), (int)x.size(0), x.size(1), cap, opt_ptr<int>(idx),
                                        opt_ptr<float>(val), opt_ptr<int>(nnz), opt_ptr<float>(thr), opt_ptr<float>(col_div),
                                        opt_ptr<int>(ties), opt_ptr<int>(tie_quota), opt_ptr<float>(col_thr),
-                                       opt_ptr<int>(seg_counts), at::cuda::getCurrentCUDAStream()),
+                                       opt_ptr<int>(seg_counts), nullptr, at::cuda::getCurrentCUDAStream()),
              "row_compact launch");
 }
 
@@ -1282,6 +1297,46 @@ void jumprelu_lists(const Tensor& idx, const Tensor& s_val, const Tensor& norm, 
   p.u_sum = u_sum.data_ptr<float>(); p.n_valid = n_valid.data_ptr<int>();
   const c10::cuda::CUDAGuard guard(idx.device());
   check_cuda(lmsae::jumprelu_lists_launch(p, at::cuda::getCurrentCUDAStream()), "jumprelu_lists launch");
+}
+
+// log_theta [F], norm [H, F], bias [H, F] (optional) -> {theta [F], smallest theta / norm [F]} and the biases' sum [F]
+std::vector<Tensor> jumprelu_begin(const Tensor& log_theta, const Tensor& norm, const c10::optional<Tensor>& bias) {
+  CHECK_T(log_theta, torch::kFloat32); CHECK_T(norm, torch::kFloat32);
+  TORCH_CHECK(norm.dim() == 2 && norm.size(0) > 0 && norm.size(1) == log_theta.numel() && norm.size(1) > 0 && norm.size(1) < INT_MAX - 256, "log_theta [F], norm [H, F]");
+  if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->sizes() == norm.sizes(), "bias [H, F]"); }
+  const c10::cuda::CUDAGuard guard(norm.device());
+  std::vector<Tensor> out = {torch::empty({norm.size(1)}, norm.options()), torch::empty({norm.size(1)}, norm.options())};
+  if (bias.has_value()) out.push_back(torch::empty({norm.size(1)}, norm.options()));
+  check_cuda(lmsae::jumprelu_begin_launch(log_theta.data_ptr<float>(), norm.data_ptr<float>(), opt_ptr<const float>(bias), (int)norm.size(0), (int)norm.size(1),
+                                          out[0].data_ptr<float>(), out[1].data_ptr<float>(), bias.has_value() ? out[2].data_ptr<float>() : nullptr,
+                                          at::cuda::getCurrentCUDAStream()),
+             "jumprelu_begin launch");
+  return out;
+}
+
+// Adam on log_theta with the gradient dtheta * theta; returns fp32 [4]: l_rec + l_s + l_p, l_s = l1 u_sum / loss_den, l_p, n_valid / tokens
+Tensor jumprelu_end(const Tensor& log_theta, const Tensor& m, const Tensor& v, const Tensor& dtheta, const Tensor& theta, const Tensor& l_rec, const Tensor& u_sum,
+                    const c10::optional<Tensor>& l_p, const Tensor& n_valid, double l1, double loss_den, double tokens, double lr, double beta1, double beta2, double eps,
+                    int64_t step, const Tensor& status) {
+  for (const Tensor* t : {&log_theta, &m, &v, &dtheta, &theta, &l_rec, &u_sum}) { CHECK_T(*t, torch::kFloat32); }
+  CHECK_T(n_valid, torch::kInt32); CHECK_T(status, torch::kInt32);
+  const int64_t F = log_theta.numel();
+  TORCH_CHECK(F > 0 && F < INT_MAX - 256 && m.numel() == F && v.numel() == F && dtheta.numel() == F && theta.numel() == F && l_rec.numel() == 1 && u_sum.numel() == 1 &&
+              n_valid.numel() == 1, "jumprelu_end: sizes");
+  if (l_p.has_value()) { CHECK_T(*l_p, torch::kFloat32); TORCH_CHECK(l_p->numel() == 1); }
+  const c10::cuda::CUDAGuard guard(log_theta.device());
+  const Tensor out = torch::empty({4}, log_theta.options());
+  lmsae::JumpReluEndParams p{};
+  p.F = (int)F;
+  p.log_theta = log_theta.data_ptr<float>(); p.m = m.data_ptr<float>(); p.v = v.data_ptr<float>();
+  p.dtheta = dtheta.data_ptr<float>(); p.theta = theta.data_ptr<float>(); p.l_rec = l_rec.data_ptr<float>(); p.u_sum = u_sum.data_ptr<float>();
+  p.l_p = opt_ptr<const float>(l_p); p.n_valid = n_valid.data_ptr<int>();
+  p.l1 = (float)l1; p.loss_den = (float)loss_den; p.tokens = (float)tokens;
+  p.out = out.data_ptr<float>();
+  p.h = make_hyper(lr, beta1, beta2, eps, step);
+  p.status = status.data_ptr<int>();
+  check_cuda(lmsae::jumprelu_end_launch(p, at::cuda::getCurrentCUDAStream()), "jumprelu_end launch");
+  return out;
 }
 
 // Rotary embedding (sin_sign = 1) or its inverse (-1) of xa and xb [batch x seq, heads, width] bf16 into oa and ob;
@@ -1680,6 +1735,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("column_lists", &column_lists);
+  m.def("jumprelu_begin", &jumprelu_begin);
+  m.def("jumprelu_end", &jumprelu_end);
   m.def("dead_rows", &dead_rows);
   m.def("row_topk_dense", &row_topk_dense);
   m.def("row_select", &row_select);

@@ -10,8 +10,7 @@
 // arrays per head, two of them scatter-adds that also sent every empty slot somewhere (crosscoder of 8 heads, 4096 tokens,
 // lists 256 wide: 2.7 ms of a 22 ms step, and 55 launches per head that the host could not issue fast enough); here
 // empty slots cost one load.
-#include "common.cuh"
-#include "kernels.h"
+#include "adam.cuh"
 
 namespace lmsae {
 
@@ -69,6 +68,58 @@ int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream) {
   const long long blocks = ((long long)p.B * p.cap + JL_THREADS - 1) / JL_THREADS;
   launch(jumprelu_lists_kernel, (int)(blocks < 148LL * 16 ? blocks : 148LL * 16), JL_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
+}
+
+// What a step needs of its thresholds and norms: theta = exp(log theta), the smallest threshold theta / ||W_D,h row|| of the heads (a NaN stays one),
+// and where wanted the sum of the heads' encoder biases. (exp in 64 bits: the fast fp32 one that this file's flags select is further off than torch's.)
+__global__ void __launch_bounds__(256)
+jumprelu_begin_kernel(const float* __restrict__ log_theta, const float* __restrict__ norm, const float* __restrict__ bias, int H, int F, float* __restrict__ theta,
+                      float* __restrict__ t_min, float* __restrict__ bias_sum) {
+  pdl_wait();
+  const int f = blockIdx.x * 256 + threadIdx.x;
+  if (f >= F) return;
+  const float th = (float)exp((double)log_theta[f]);
+  theta[f] = th;
+  float m = __int_as_float(0x7f800000), b = 0.0f;
+  for (int h = 0; h < H; ++h) {
+    const float t = __fdiv_rn(th, norm[(size_t)h * F + f]);
+    if (m == m && (t != t || t < m)) m = t;
+    if (bias_sum != nullptr) b += bias[(size_t)h * F + f];
+  }
+  t_min[f] = m;
+  if (bias_sum != nullptr) bias_sum[f] = b;
+}
+
+int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, cudaStream_t stream) {
+  if (H <= 0 || F <= 0) return (int)cudaErrorInvalidValue;
+  return (int)launch(jumprelu_begin_kernel, (F + 255) / 256, 256, 0, stream, log_theta, norm, bias, H, F, theta, t_min, bias_sum);
+}
+
+// The end of a step: Adam on log theta, whose gradient is d theta * theta, and the step's figures out[0..4): loss l_rec + l_s + l_p, l_s, l_p, active entries per
+// token. (As tensor operations: eight launches of a few elements.)
+__global__ void __launch_bounds__(256)
+jumprelu_end_kernel(const JumpReluEndParams p) {
+  pdl_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const float l_s = __fdiv_rn(p.l1 * *p.u_sum, p.loss_den), l_p = p.l_p != nullptr ? *p.l_p : 0.0f;
+    p.out[0] = *p.l_rec + l_s + l_p;
+    p.out[1] = l_s;
+    p.out[2] = l_p;
+    p.out[3] = __fdiv_rn((float)*p.n_valid, p.tokens);
+  }
+  if (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0) return;  // see sparse_grad_adam_kernel
+  const int f = blockIdx.x * 256 + threadIdx.x;
+  if (f >= p.F) return;
+  float x = p.log_theta[f], m = p.m[f], v = p.v[f];
+  adam_elem(x, m, v, p.dtheta[f] * p.theta[f], p.h);
+  p.log_theta[f] = x;
+  p.m[f] = m;
+  p.v[f] = v;
+}
+
+int jumprelu_end_launch(const JumpReluEndParams& p, cudaStream_t stream) {
+  if (p.F <= 0) return (int)cudaErrorInvalidValue;
+  return (int)launch(jumprelu_end_kernel, (p.F + 255) / 256, 256, 0, stream, p);
 }
 
 }  // namespace lmsae

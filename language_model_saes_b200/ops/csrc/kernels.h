@@ -285,7 +285,8 @@ int threshold_mask_launch(int dtype, const void* x, const float* thr, long long 
                           cudaStream_t stream);
 int row_compact_launch(int dtype, const void* x, int B, long long N, int cap, int* idx, float* val, int* nnz,
                        const float* thr, const float* col_div, int* ties, const int* tie_quota, const float* col_thr,
-                       int* seg_counts, cudaStream_t stream);
+                       int* seg_counts, unsigned long long* overflow, cudaStream_t stream);
+bool row_compact_cols_fits(const void* x, long long N, const float* col_thr, int cap);
 int jumprelu_window_grad_launch(const __nv_bfloat16* G, const __nv_bfloat16* S, int B, int F, const float* n,
                                 const float* theta, float window, float add_per_hit, float* dtheta, cudaStream_t stream);
 int gather_rows_cast_launch(int in_dtype, int out_dtype, const void* src, const int* keep, const int* pos, long long n,
@@ -308,6 +309,19 @@ struct JumpReluListParams {
   int* n_valid;        // += number of listed entries
 };
 int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream);
+int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, cudaStream_t stream);
+struct JumpReluEndParams {
+  int F;
+  float *log_theta, *m, *v;
+  const float *dtheta, *theta;
+  const float *l_rec, *u_sum, *l_p;  // l_p nullptr: 0
+  const int* n_valid;
+  float l1, loss_den, tokens;
+  float* out;  // [4]
+  AdamHyper h;
+  const int* status;
+};
+int jumprelu_end_launch(const JumpReluEndParams& p, cudaStream_t stream);
 
 // ---- rotary embedding of two [tokens, heads, width] bf16 tensors in one launch (rotary.cu) ----------------------
 int rotary_pair_launch(const __nv_bfloat16* xa, const __nv_bfloat16* xb, __nv_bfloat16* oa, __nv_bfloat16* ob, const float* cos_t,

@@ -566,7 +566,7 @@ row_compact_kernel(const T* __restrict__ x, int B, long long N, int cap, int* __
 template <int R>
 __global__ void __launch_bounds__(RC_THREADS)
 row_compact_cols_kernel(const __nv_bfloat16* __restrict__ x, int B, int N, int cap, int* __restrict__ idx, float* __restrict__ val,
-                        int* __restrict__ nnz, const float* __restrict__ col_div, const float* __restrict__ col_thr) {
+                        int* __restrict__ nnz, const float* __restrict__ col_div, const float* __restrict__ col_thr, unsigned long long* __restrict__ overflow) {
   pdl_wait();
   constexpr int NW = RC_THREADS / 32;
   extern __shared__ int s_lists[];  // [NW][R][cap]
@@ -637,6 +637,7 @@ row_compact_cols_kernel(const __nv_bfloat16* __restrict__ x, int B, int N, int c
       val[(size_t)row * cap + before + j] = col_div != nullptr ? f / col_div[c] : f;
     }
     if (threadIdx.x == 0 && nnz != nullptr) nnz[row] = total;
+    if (threadIdx.x == 0 && overflow != nullptr && total > cap) atomicAdd(overflow, 1ULL);
     for (int j = total + threadIdx.x; j < cap; j += RC_THREADS) {
       idx[(size_t)row * cap + j] = -1;
       val[(size_t)row * cap + j] = 0.0f;
@@ -743,23 +744,28 @@ int threshold_mask_launch(int dtype, const void* x, const float* thr, long long 
   return (int)cudaGetLastError();
 }
 
+bool row_compact_cols_fits(const void* x, long long N, const float* col_thr, int cap) {
+  return N % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(col_thr) % 16 == 0 && cap <= 1024;
+}
+
 int row_compact_launch(int dtype, const void* x, int B, long long N, int cap, int* idx, float* val, int* nnz,
                        const float* thr, const float* col_div, int* ties, const int* tie_quota, const float* col_thr,
-                       int* seg_counts, cudaStream_t stream) {
+                       int* seg_counts, unsigned long long* overflow, cudaStream_t stream) {
   if (col_thr != nullptr && (thr != nullptr || ties != nullptr || tie_quota != nullptr)) return (int)cudaErrorInvalidValue;
   if (B <= 0) return 0;
   if (N > 2147483647LL) return (int)cudaErrorInvalidValue;
   const int blocks = B < 148 * 8 ? B : 148 * 8;
   // the one-pass kernel where whole vectors can be read and its lists fit the default shared memory; four rows to a CTA once
   // there are enough of them for two CTAs per SM
-  if (col_thr != nullptr && idx != nullptr && dtype == 1 && N % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(col_thr) % 16 == 0 && cap <= 1024) {
+  const bool cols = col_thr != nullptr && idx != nullptr && dtype == 1 && row_compact_cols_fits(x, N, col_thr, cap);
+  if (overflow != nullptr && !cols) return (int)cudaErrorInvalidValue;  // (counted there only)
+  if (cols) {
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
     const size_t per_row = (size_t)(RC_THREADS / 32) * cap * 4;
     if (cap <= 256 && B >= 148 * 8)
-      launch(row_compact_cols_kernel<4>, (B + 3) / 4, RC_THREADS, 4 * per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
+      launch(row_compact_cols_kernel<4>, (B + 3) / 4, RC_THREADS, 4 * per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr, overflow);
     else
-      launch(row_compact_cols_kernel<1>, B, RC_THREADS, per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr);
+      launch(row_compact_cols_kernel<1>, B, RC_THREADS, per_row, stream, xb, B, (int)N, cap, idx, val, nnz, col_div, col_thr, overflow);
     return (int)cudaGetLastError();
   }
   if (dtype == 0)

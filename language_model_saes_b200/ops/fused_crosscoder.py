@@ -96,6 +96,7 @@ class FusedCrosscoderStep:
                       "b_D": (z(H_l, d), z(H_l, d)), "log_theta": (z(F), z(F))}  # fmt: skip
         self.groups: K.FeatureGroups | None = None
         self.loss_sum = z(1)
+        self._sum_clear = True  # whether it is zero (a step on lists that ended left it so)
         self.bias_update = K.BiasUpdate([d] * H_l, dev)
         self.list_overflow = torch.zeros(1, dtype=torch.int64, device=dev)
         self.last: dict[str, torch.Tensor] = {}
@@ -160,8 +161,8 @@ class FusedCrosscoderStep:
     def sync_params(self) -> None:
         pass
 
-    def _head_sum(self, x16: torch.Tensor) -> torch.Tensor:
-        """``sum over all heads of (x_h W_E,h^T + b_E,h)`` as bf16 [B, F] on every rank."""
+    def _head_sum(self, x16: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+        """``sum over all heads of (x_h W_E,h^T + b_E,h)`` as bf16 [B, F] on every rank; ``bias``: the local heads' sum where it is known."""
         from ..parallel.symm import AllReduceComm
 
         B = x16.shape[0]
@@ -175,7 +176,7 @@ class FusedCrosscoderStep:
             self.comm = AllReduceComm(self.head_group if self.head_size > 1 else None, x16.device, B, self.F)
         # the GEMM accumulates the local heads in one K loop and stores bf16 straight into the symmetric buffer ...
         P = self.comm.matrix(B)
-        K._ext().head_sum_gemm(x16, self.WE_bf16.view(self.H_l * self.F, self.d), self.bE.sum(0).contiguous(), self.H_l, self.F, self.F,
+        K._ext().head_sum_gemm(x16, self.WE_bf16.view(self.H_l * self.F, self.d), bias if bias is not None else self.bE.sum(0).contiguous(), self.H_l, self.F, self.F,
                                True, K.status_buffer(x16.device), P)  # fmt: skip
         # ... which one kernel then sums over the head ranks in place (NVSwitch multicast loads / stores where available)
         return self.comm.all_reduce(B) if self.head_size > 1 else P
@@ -203,14 +204,19 @@ class FusedCrosscoderStep:
         H, F, cap = self.H, self.F, self.cap
         grad_scale = 2.0 / (B * H)
         x = x.contiguous()
-        S_sum = self._head_sum(x.view(B_l, H_l * d))
-        theta = self.log_theta.exp()
-        t_head = theta / self.dec_norm  # [H_l, F]: a head is active where S > theta / ||W_D,h row||
-        t_min = t_head.amin(0)
+        on_lists = self.tp == 1 and self.dp == 1 and not quad
+        if on_lists and x.is_cuda:
+            theta, t_min, *bias = K._ext().jumprelu_begin(self.log_theta, self.dec_norm, self.bE if H_l > 1 else None)
+            S_sum = self._head_sum(x.view(B_l, H_l * d), bias[0] if bias else self.bE[0])
+        else:
+            S_sum = self._head_sum(x.view(B_l, H_l * d))
+            theta = self.log_theta.exp()
+            t_head = theta / self.dec_norm  # [H_l, F]: a head is active where S > theta / ||W_D,h row||
+            t_min = t_head.amin(0)
         if self.head_size > 1:
             dist.all_reduce(t_min, op=dist.ReduceOp.MIN, group=self.head_group)
         idx, s_val = S.column_threshold_rows_to_sparse(S_sum, t_min, cap, overflow=self.list_overflow)
-        if self.tp == 1 and self.dp == 1 and not quad:
+        if on_lists:
             return self._step_on_lists(x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, float(tanh_stretch), lp_coefficient)
         safe = idx.clamp_min(0).long()
         valid = idx >= 0
@@ -219,6 +225,7 @@ class FusedCrosscoderStep:
         dump = F + (torch.arange(B_l, device=x.device) % 1024).unsqueeze(1)
         scat = torch.where(valid, safe, dump.expand_as(safe)).reshape(-1)
         self.loss_sum.zero_()
+        self._sum_clear = False
         dS = torch.zeros(B_l, cap, dtype=torch.float32, device=x.device)
         dtheta_buf = torch.zeros(F + 1024, dtype=torch.float32, device=x.device)
         dtheta = dtheta_buf[:F]
@@ -390,7 +397,9 @@ class FusedCrosscoderStep:
         if self.groups is None or self.groups.entries.numel() < idx.numel():
             self.groups = K.FeatureGroups(F, idx.numel(), dev)
         self.groups.build(idx)
-        self.loss_sum.zero_()
+        if not self._sum_clear:
+            self.loss_sum.zero_()
+        self._sum_clear = False
         self.t += 1
         b1, b2 = self.betas
         (mE, vE), (mD, vD), (mb, vb), (mbD, vbD) = (self.state[n] for n in ("W_E", "W_D", "b_E", "b_D"))
@@ -425,8 +434,16 @@ class FusedCrosscoderStep:
             K.sparse_grad_adam(self.groups, act[h], dS, xt[h], xt[h], None, None, None, None, self.WE[h], mE[h], vE[h], self.WE_bf16[h],
                                self.bE[h], mb[h], vb[h], None, None, None, lr, b1, b2, self.eps, self.t, True, extra=extra)  # fmt: skip
         m, v = self.state["log_theta"]
-        K.adam_flat(self.log_theta, dtheta * theta, m, v, lr * self.jumprelu_lr_factor, b1, b2, self.eps, self.t)
+        if not x.is_cuda:
+            K.adam_flat(self.log_theta, dtheta * theta, m, v, lr * self.jumprelu_lr_factor, b1, b2, self.eps, self.t)
         l_rec = self.bias_update(dxhats, list(self.bD), list(zip(mbD, vbD)), lr, b1, b2, self.eps, self.t, self.loss_sum, loss_den=float(B * H_l))
+        self._sum_clear = True
+        if x.is_cuda:
+            total, l_s, l_p, l0 = K._ext().jumprelu_end(
+                self.log_theta, m, v, dtheta, theta, l_rec, u_sum, l_p_sum if lp is not None else None, n_valid, float(l1_coefficient), float(B * H_l), float(B),
+                lr * self.jumprelu_lr_factor, b1, b2, self.eps, self.t, K.status_buffer(dev)).unbind()  # fmt: skip
+            self.last = {"l_rec": l_rec, "l_s": l_s, "l_p": l_p, "l0": l0}
+            return total
         l_s = l1_coefficient * u_sum.squeeze(0) / (B * H_l)
         l_p = l_p_sum if lp is not None else torch.zeros((), device=dev)
         self.last = {"l_rec": l_rec, "l_s": l_s, "l_p": l_p, "l0": n_valid.squeeze(0) / B}

@@ -308,6 +308,10 @@ def column_threshold_rows_to_sparse(x: torch.Tensor, col_thr: torch.Tensor, cap:
     x = x.contiguous()
     idx = torch.empty(B, cap, dtype=torch.int32, device=x.device)
     val = torch.empty(B, cap, dtype=torch.float32, device=x.device)
+    col_thr = col_thr.float().contiguous()
+    if (overflow is not None and overflow.dtype == torch.int64 and overflow.numel() == 1 and x.dtype == torch.bfloat16
+            and K._ext().column_lists(x, col_thr, idx, val, overflow)):  # fmt: skip
+        return idx, val
     nnz = torch.empty(B, dtype=torch.int32, device=x.device)
     K._ext().row_compact(x, idx, val, nnz, None, None, None, None, col_thr.float().contiguous(), None)
     if overflow is not None:
