@@ -618,8 +618,8 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
                       const c10::optional<Tensor>& extra_gD, const c10::optional<Tensor>& extra_gE,
                       const c10::optional<Tensor>& extra_gb, const c10::optional<Tensor>& wd_self_scale,
                       const c10::optional<Tensor>& norm_sq_accum, int64_t dact_mode, const c10::optional<Tensor>& heavy,
-                      int64_t heavy_base, const c10::optional<Tensor>& sched, int64_t wait_cycles) {
-  // (wait_cycles < 0: the kernels' usual limit)
+                      int64_t heavy_base, const c10::optional<Tensor>& sched, int64_t wait_cycles, int64_t layer_rows, bool layers_share_groups) {
+  // (wait_cycles < 0: the kernels' usual limit; layer_rows: 0, or rows of a layer where the encoder group holds several, x their inputs one after the other)
   // one-sided launches: the decoder group (WD, mD, vD, WD_bf16) or the encoder group (WE, mE, vE, WE_bf16) may be absent
   const bool has_d = WD_o.has_value(), has_e = WE_o.has_value();
   TORCH_CHECK(has_d || has_e, "at least one of the decoder / encoder groups must be given");
@@ -644,9 +644,13 @@ void sparse_grad_adam(const Tensor& offsets, const Tensor& entries, const Tensor
   p.F = (int)WD.size(0);
   p.d = (int)WD.size(1);
   p.k = (int)act.size(1);
-  p.n_rows = (int)x.size(0);
+  const int64_t layers = layer_rows > 0 ? p.F / layer_rows : 1;
+  TORCH_CHECK(layer_rows == 0 || (layer_rows > 0 && !has_d && p.F % layer_rows == 0 && x.size(0) % layers == 0), "layers: whole ones, encoder side");
+  p.layer_rows = (int)layer_rows;
+  p.layers_share_groups = layer_rows > 0 && layers_share_groups ? 1 : 0;
+  p.n_rows = (int)(x.size(0) / layers);
   p.n_codes = act.numel();
-  TORCH_CHECK(offsets.numel() >= p.F + 1 && x.size(1) == p.d && dxhat.sizes() == x.sizes());
+  TORCH_CHECK(offsets.numel() >= (p.layers_share_groups ? layer_rows : p.F) + 1 && x.size(1) == p.d && dxhat.sizes() == x.sizes());
   p.f_begin = (int)f_begin;
   p.f_end = f_end < 0 ? p.F : (int)f_end;
   TORCH_CHECK(0 <= p.f_begin && p.f_begin <= p.f_end && p.f_end <= p.F, "feature range out of bounds");
@@ -839,7 +843,7 @@ Tensor topk_step(const Tensor& x, const Tensor& label, int64_t k, int64_t route,
   csc_build(idx, N, groups[0], groups[1], groups[2], groups[3], groups[4], groups[5]);
   sparse_grad_adam(groups[1], groups[3], act, dact, x, dxhat, dec[0], dec[1], dec[2], dec[3], enc[0], enc[1], enc[2], enc[3], b_E[0], b_E[1], b_E[2], dec_norm, none,
                    none, lr, beta1, beta2, eps, step, true, 0, -1, 0, none, 0, none, none, status, 0, {}, {}, 0, none, none, none, none, none, none, none, 1, groups[5], 0,
-                   groups[6], -1);
+                   groups[6], -1, 0, false);
   const std::vector<Tensor> nothing;
   return colsum_adam(b_D.empty() ? nothing : std::vector<Tensor>{dxhat}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[0]},
                      b_D.empty() ? nothing : std::vector<Tensor>{b_D[1]}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[2]}, counters, lr, beta1, beta2, eps, step,

@@ -85,10 +85,9 @@ __host__ __device__ constexpr int gather_batch() { return NCH == 1 ? 8 : NCH == 
 // g += coefficient * row, with DOT also the code gradients against the bf16-rounded row in c.rounded. Returns (encoder side)
 // the sum of this lane's coefficients.
 template <bool IS_D, bool DOT, int W, int NCH>
-__device__ __forceinline__ float gather_side(const GradAdamParams& p, const GroupCtx& c, int e0, int e1, int first, int stride,
+__device__ __forceinline__ float gather_side(const GradAdamParams& p, const GroupCtx& c, const __nv_bfloat16* src, int e0, int e1, int first, int stride,
                                              float (&g)[NCH][4]) {
   constexpr int Q = gather_batch<NCH>();
-  const __nv_bfloat16* src = IS_D ? p.dxhat : p.x;
   float coef_sum = 0.0f;
   for (int eb = e0 + first * 32; eb < e1; eb += stride * 32) {
     const int n_e = min(32, e1 - eb);
@@ -334,15 +333,19 @@ grad_adam_rows_kernel(const GradAdamParams p) {
     }
   };
 
+  // several layers' rows one after the other: the group of entries and the inputs of row f
+  auto group_of = [&](int f) { return p.layers_share_groups ? f % p.layer_rows : f; };
+  auto inputs_of = [&](int f) { return p.layer_rows != 0 ? p.x + (size_t)(f / p.layer_rows) * p.n_rows * p.d : p.x; };
+
   const bool heavy_on = p.heavy != nullptr;
   // ---------------------------------------------------------------- rows with long entry lists: the whole CTA
   if (heavy_on && !skip) {
-    const int n_heavy = p.heavy[0];
+    const int n_heavy = p.heavy[0], n_long = p.layers_share_groups ? n_heavy * (p.F / p.layer_rows) : n_heavy;
     uint32_t par0 = 0;
-    for (int hi = blockIdx.x; hi < n_heavy && !failed; hi += gridDim.x) {
-      const int f = p.heavy[1 + hi] - p.heavy_base;
+    for (int hi = blockIdx.x; hi < n_long && !failed; hi += gridDim.x) {
+      const int layer = hi / max(n_heavy, 1), group = p.heavy[1 + hi - layer * n_heavy] - p.heavy_base, f = group + layer * p.layer_rows;
       if (f < p.f_begin || f >= p.f_end) continue;
-      const int e0 = p.offsets[f], e1 = p.offsets[f + 1];
+      const int e0 = p.offsets[group], e1 = p.offsets[group + 1];
       const int xr = p.extra_row != nullptr ? p.extra_row[f] : -1;
       for (int side = 0; side < 2; ++side) {
         const bool is_d = side == 0;
@@ -357,12 +360,12 @@ grad_adam_rows_kernel(const GradAdamParams p) {
             failed = !__syncthreads_and(arrived(0, par0));
             if (failed) break;
             round_row<W, NCH>(stages, p.d, c);
-            gather_side<true, true, W, NCH>(p, c, e0, e1, c.gid, G, g);
+            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, g);
           } else {
-            gather_side<true, false, W, NCH>(p, c, e0, e1, c.gid, G, g);
+            gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, g);
           }
         } else {
-          coef = gather_side<false, false, W, NCH>(p, c, e0, e1, c.gid, G, g);
+          coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, c.gid, G, g);
         }
         if (!is_d && c.wg == 0) {
           coef = warp_sum(coef);
@@ -449,8 +452,9 @@ grad_adam_rows_kernel(const GradAdamParams p) {
   auto next_light = [&](int& e0, int& e1) -> int {
     int f = next_row();
     while (f < p.f_end) {
-      e0 = p.offsets[f];
-      e1 = p.offsets[f + 1];
+      const int group = group_of(f);
+      e0 = p.offsets[group];
+      e1 = p.offsets[group + 1];
       if (!heavy_on || e1 - e0 <= kHeavyRow) break;
       f = next_row();
     }
@@ -473,10 +477,10 @@ grad_adam_rows_kernel(const GradAdamParams p) {
           if (failed) break;
           if (e1 > e0) {
             round_row<W, NCH>(c.stage, p.d, c);
-            gather_side<true, true, W, NCH>(p, c, e0, e1, 0, 1, g);
+            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, g);
           }
         } else {
-          gather_side<true, false, W, NCH>(p, c, e0, e1, 0, 1, g);
+          gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, g);
         }
         if (loadsD != 0) {
           if (!dot_mode) {
@@ -508,7 +512,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
       if (doE) {
         float g[NCH][4];
         init_grad(false, xr, g);
-        float coef = gather_side<false, false, W, NCH>(p, c, e0, e1, 0, 1, g);
+        float coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, 0, 1, g);
         if (loadsE != 0) {
           failed = !group_all<W>(c.gid, arrived(c.gid, parity));
           if (failed) break;

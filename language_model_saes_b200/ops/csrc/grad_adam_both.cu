@@ -480,7 +480,8 @@ static cudaError_t launch_both(GradAdamParams p, cudaStream_t stream) {
 // Whether grad_adam_rows_launch hands this launch on: short rows, both sides and their code gradients at once, parameters updated, nothing
 // else asked for.
 bool grad_adam_both_supported(const GradAdamParams& p) {
-  return p.WD != nullptr && p.WE != nullptr && p.dact_mode == 1 && p.update && p.grad_sq_sum == nullptr && p.norm_sq_accum == nullptr && p.d <= 512;
+  return p.WD != nullptr && p.WE != nullptr && p.dact_mode == 1 && p.update && p.grad_sq_sum == nullptr && p.norm_sq_accum == nullptr && p.layer_rows == 0 &&
+         p.d <= 512;
 }
 
 int grad_adam_both_launch(const GradAdamParams& p, cudaStream_t stream) {

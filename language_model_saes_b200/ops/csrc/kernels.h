@@ -183,6 +183,10 @@ struct GradAdamParams {
   AdamHyper h;
   int update;
   int f_begin, f_end;  // feature rows handled by this launch
+  // Encoder side of several layers (or heads) in one launch of the row-streaming kernel, layer_rows rows each (0: one layer): row f takes its inputs from rows
+  // [f / layer_rows * n_rows, + n_rows) of x; with layers_share_groups the entries of group f % layer_rows, else of group f.
+  int layer_rows;
+  int layers_share_groups;
   int ctas_per_sm;     // 0 = fill the GPU (4 per SM); 1..4 = leave registers free for a concurrently running kernel
   const int* status;   // kernels' status word: a recorded error turns the update into a no-op (nullptr: not checked)
   // Dense gradient rows for a subset of the features, added to the rows rebuilt from the entry lists: feature f takes

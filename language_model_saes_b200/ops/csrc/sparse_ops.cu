@@ -826,6 +826,7 @@ int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream) {
   const bool doD = p.WD != nullptr, doE = p.WE != nullptr;
   if (!doD && !doE) return (int)cudaErrorInvalidValue;
   if (!(doD && doE) && p.n_pub > 0) return (int)cudaErrorInvalidValue;  // rows are published by two-sided launches only
+  if (p.layer_rows != 0 && (doD || p.layer_rows < 0 || p.F % p.layer_rows != 0 || !grad_adam_rows_supported(p))) return (int)cudaErrorInvalidValue;
   if (grad_adam_rows_supported(p)) return grad_adam_rows_launch(p, stream);
   if (p.dact_mode != 0) return (int)cudaErrorInvalidValue;  // the kernel below takes the code gradients as an input
   if (doD && doE) {

@@ -302,11 +302,7 @@ class FusedCLTStep:
                                None, None, None, None, None, lr, b1, b2, self.eps, self.t, True, norm_sq_accum=self.norm_sq[:rows],
                                dact_mode=2 if self.dp == 1 else 0)  # fmt: skip
         (mE, vE), (mb, vb) = self.state["W_E"], self.state["b_E"]
-        for s in range(L):  # encoder side, one launch per source layer
-            g = self.groups.part(s * F, (s + 1) * F)
-            xs = xt[s]
-            K.sparse_grad_adam(g, act, dact, xs, xs, None, None, None, None, self.WE[s], mE[s], vE[s], self.WE_bf16[s], self.bE[s], mb[s],
-                               vb[s], None, None, None, lr, b1, b2, self.eps, self.t, True)  # fmt: skip
+        K.layers_encoder_adam(self.groups, act, dact, xt, self.WE, mE, vE, self.WE_bf16, self.bE, mb, vb, False, lr, b1, b2, self.eps, self.t)
         m, v = self.state["b_D"]
         return self.bias_update(list(dy), list(self.bD), list(zip(m, v)), lr, b1, b2, self.eps, self.t, self.loss_sum, loss_den=float(n_rows))
 

@@ -426,11 +426,12 @@ class FusedCrosscoderStep:
             dS = torch.where(idx >= 0, dS, torch.zeros_like(dS))  # (empty slots were never written)
             dist.all_reduce(dS, group=self.head_group)
             dist.all_reduce(dtheta, group=self.head_group)
-        for h in range(H_l):
-            extra = None
-            if lp is not None:  # dense encoder gradient rows of the pre-activation penalty: -c N_f (1[S < theta]^T x_h)[f, :]
-                gE = _mm_f32(lp["mask"].t(), xt[h]) * lp["row_scale"].unsqueeze(1)
-                extra = (lp["rows"], None, gE, lp["gb"])
+        if lp is None:
+            K.layers_encoder_adam(self.groups, act[0], dS, xt, self.WE, mE, vE, self.WE_bf16, self.bE, mb, vb, True, lr, b1, b2, self.eps, self.t)
+        for h in range(H_l if lp is not None else 0):
+            # dense encoder gradient rows of the pre-activation penalty: -c N_f (1[S < theta]^T x_h)[f, :]
+            gE = _mm_f32(lp["mask"].t(), xt[h]) * lp["row_scale"].unsqueeze(1)
+            extra = (lp["rows"], None, gE, lp["gb"])
             K.sparse_grad_adam(self.groups, act[h], dS, xt[h], xt[h], None, None, None, None, self.WE[h], mE[h], vE[h], self.WE_bf16[h],
                                self.bE[h], mb[h], vb[h], None, None, None, lr, b1, b2, self.eps, self.t, True, extra=extra)  # fmt: skip
         m, v = self.state["log_theta"]

@@ -750,7 +750,25 @@ def sparse_grad_adam(
         dec_norm, grad_mul, grad_sq_sum, lr, beta1, beta2, eps, step, update, *(f_range if f_range is not None else (0, -1)), ctas_per_sm, dxhat_aux, k_main, grad_out[0], grad_out[1],
         status_buffer(ref_w.device), state_f0, *(publish if publish is not None else ([], [], 0, None)),
         *(extra if extra is not None else (None, None, None, None)), wd_self_scale, norm_sq_accum, dact_mode, groups.heavy,
-        groups.heavy_base, groups.sched, wait_cycles,
+        groups.heavy_base, groups.sched, wait_cycles, 0, False,
+    )  # fmt: skip
+
+
+def layers_encoder_adam(groups: FeatureGroups, act, dact, x, WE, mE, vE, WE_bf16, bE, mbE, vbE, shared: bool, lr, beta1, beta2, eps, step) -> None:
+    """The encoder side of ``sparse_grad_adam`` for several layers (or heads) at once: ``x [L, rows, d]``, parameters and moments ``[L, F, d]``, biases
+    ``[L, F]``, ``groups`` of ``L * F`` features, layer by layer, or of ``F`` features that all layers share."""
+    L, F, d = WE.shape
+    if not (WE.is_cuda and d % 4 == 0 and d <= 8192 and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, WE, mE, vE, WE_bf16, bE, mbE, vbE))):
+        for i in range(L):
+            sparse_grad_adam(groups if shared else groups.part(i * F, (i + 1) * F), act, dact, x[i], x[i], None, None, None, None, WE[i], mE[i], vE[i], WE_bf16[i],
+                             bE[i], mbE[i], vbE[i], None, None, None, lr, beta1, beta2, eps, step, True)  # fmt: skip
+        return
+    flat = lambda t: t.view(L * F, -1)  # noqa: E731
+    xf = x.view(-1, d)
+    _ext().sparse_grad_adam(
+        groups.offsets, groups.entries, act, dact, xf, xf, None, None, None, None, flat(WE), flat(mE), flat(vE), flat(WE_bf16), bE.view(-1), mbE.view(-1), vbE.view(-1),
+        None, None, None, lr, beta1, beta2, eps, step, True, 0, -1, 0, None, 0, None, None, status_buffer(WE.device), 0, [], [], 0, None, None, None, None, None, None,
+        None, 0, groups.heavy, groups.heavy_base, groups.sched, -1, F, shared,
     )  # fmt: skip
 
 

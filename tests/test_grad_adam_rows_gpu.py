@@ -140,3 +140,29 @@ def test_both_sides_in_one_pass_match_the_plain_statement(d, F, B, f_range):
 @pytest.mark.parametrize("d", [64, 512])
 def test_one_pass_rows_whose_copies_were_not_waited_for_stay_as_they_are(d):
     test_rows_whose_copies_were_not_waited_for_stay_as_they_are(d, "both", 1)
+
+
+@pytest.mark.parametrize("d", [64, 768, 1160])
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("L,F", [(1, 230), (3, 230), (4, 41)])
+def test_encoder_sides_of_several_layers_in_one_launch(d, shared, L, F):
+    """Layers with entries of their own and layers that share them, with lists long enough to be shared by a CTA in more than one layer."""
+    B, k, g = 200, 6, torch.Generator().manual_seed(d + L)
+    n = F if shared else L * F
+    idx = torch.randint(0, n, (B, k), generator=g).to(torch.int32)
+    idx[:, 0] = 3
+    idx[:150, 1] = n - 2  # (the last layer's, or every layer's)
+    idx[5, 2:] = -1
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    cpu = dict(idx=idx, dact=r(B, k), x=r(L, B, d).to(torch.bfloat16), W=r(L, F, d), b=r(L, F), S=torch.zeros(L, F, d, dtype=torch.bfloat16))
+    for name, shape in (("m", (L, F, d)), ("v", (L, F, d)), ("mb", (L, F)), ("vb", (L, F))):
+        cpu[name] = torch.rand(*shape, generator=g) * 0.01
+    gpu = {n_: t.clone().to(DEV) for n_, t in cpu.items()}
+    for t in (cpu, gpu):
+        for step in (1, 2):
+            groups = K.FeatureGroups(n, B * k, t["idx"].device).build(t["idx"])
+            K.layers_encoder_adam(groups, t["dact"], t["dact"], t["x"], t["W"], t["m"], t["v"], t["S"], t["b"], t["mb"], t["vb"], shared, 1e-3, 0.9, 0.999, 1e-8, step)
+    K.check_status(torch.device(DEV))
+    assert int(groups.heavy[0]) == 2 and groups.sched.tolist() == [0, 0]
+    _compare(cpu, gpu, ["W", "m", "v", "b", "mb", "vb"], d)
+    assert torch.equal(gpu["S"].float(), gpu["W"].to(torch.bfloat16).float())
