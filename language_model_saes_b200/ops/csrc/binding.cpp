@@ -384,9 +384,9 @@ void topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& 
                                      out.data_ptr<float>(), stream), "topk_wide launch");
 }
 
-// out [B, d] = acts [B, F] @ W [F, d], fp32. Rows of at most `most` non-zeros are gathered. todo: int32 [2 + B + tiles], zeroed; part: fp32
+// out [B, d] = acts [B, F] @ W [F, d] (+ bias [d]), fp32. Rows of at most `most` non-zeros are gathered. todo: int32 [2 + B + tiles], zeroed; part: fp32
 // scratch in which the product of the other rows may cut up to `tiles` tiles of 128 x 128 into slices of the sum
-void dense_decode(const Tensor& acts, const Tensor& W, int64_t most, const Tensor& todo, const Tensor& part, const Tensor& out) {
+void dense_decode(const Tensor& acts, const Tensor& W, const c10::optional<Tensor>& bias, int64_t most, const Tensor& todo, const Tensor& part, const Tensor& out) {
   for (const Tensor* t : {&acts, &W, &part, &out}) { CHECK_T(*t, torch::kFloat32); }
   CHECK_T(todo, torch::kInt32);
   TORCH_CHECK(acts.dim() == 2 && W.dim() == 2 && out.dim() == 2 && acts.size(1) == W.size(0) && out.size(0) == acts.size(0) &&
@@ -394,7 +394,8 @@ void dense_decode(const Tensor& acts, const Tensor& W, int64_t most, const Tenso
   const int64_t tiles = todo.numel() - acts.size(0) - 2;
   TORCH_CHECK(tiles >= 0 && tiles <= INT_MAX && most >= 0 && most <= INT_MAX, "todo [2 + B + tiles]");
   const c10::cuda::CUDAGuard guard(acts.device());
-  check_cuda(lmsae::dense_decode_launch(acts.data_ptr<float>(), W.data_ptr<float>(), (int)acts.size(0), (int)acts.size(1), (int)W.size(1), (int)most,
+  if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->numel() == W.size(1), "bias [d]"); }
+  check_cuda(lmsae::dense_decode_launch(acts.data_ptr<float>(), W.data_ptr<float>(), opt_ptr<const float>(bias), (int)acts.size(0), (int)acts.size(1), (int)W.size(1), (int)most,
                                         todo.data_ptr<int>(), part.numel() > 0 ? part.data_ptr<float>() : nullptr, part.numel(), (int)tiles,
                                         out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()),
              "dense_decode launch");

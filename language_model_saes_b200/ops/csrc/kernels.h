@@ -105,6 +105,8 @@ struct RowsProductParams {
   float* C;         // [*, N]
   int N, K;
   const int* rows;  // [0] how many, then which rows of A and C
+  const int* every;   // optional: not 0: all max_rows rows
+  const float* bias;  // optional, [N]: added at the end
   int max_rows;     // of them at most
   float* part;      // slices of sums (nullptr: none), and a zeroed counter per tile
   long long part_floats;
@@ -113,8 +115,8 @@ struct RowsProductParams {
   bool vec;         // set by the launch
 };
 int rows_product_launch(RowsProductParams p, bool b_by_k, cudaStream_t stream);
-int dense_decode_launch(const float* acts, const float* W, int B, int F, int d, int most, int* todo, float* part, long long part_floats, int part_tiles,
-                        float* out, cudaStream_t stream);
+int dense_decode_launch(const float* acts, const float* W, const float* bias, int B, int F, int d, int most, int* todo, float* part, long long part_floats,
+                        int part_tiles, float* out, cudaStream_t stream);
 int row_topk_dense_launch(const __nv_bfloat16* H, int M, int N, int k, const float* gate, __nv_bfloat16* dense, cudaStream_t stream);
 int row_topk_launch(const __nv_bfloat16* H, long long ldh, int M, int N, int k, const float* gate,
                     const uint8_t* alive, const float* maxima, long long ld_maxima, int* out_idx, float* out_val, cudaStream_t stream);

@@ -22,8 +22,10 @@ rows_product_kernel(const RowsProductParams p) {
   __shared__ __align__(16) float s_a[2][RP_K][RP_LD];
   __shared__ __align__(16) float s_b[2][RP_K][RP_LD];
   __shared__ int s_last;
-  const int n_rows = p.rows[0];
+  const bool every = p.every != nullptr && *p.every != 0;
+  const int n_rows = every ? p.max_rows : p.rows[0];
   if (n_rows == 0) return;
+  auto row_at = [&](int r) { return every ? r : p.rows[1 + r]; };
   const int mt = (n_rows + RP_M - 1) / RP_M, nt = (p.N + RP_N - 1) / RP_N, tiles = mt * nt;
   const int k_blocks = (p.K + RP_K - 1) / RP_K;
   int slices = 1;
@@ -43,7 +45,7 @@ rows_product_kernel(const RowsProductParams p) {
     const int slice = item / tiles, tile = item - slice * tiles;
     const int m0 = (tile % mt) * RP_M, n0 = (tile / mt) * RP_N;
     const int kb0 = (int)((long long)k_blocks * slice / slices), kb1 = (int)((long long)k_blocks * (slice + 1) / slices);
-    const float* a_row = m0 + lr < n_rows ? p.A + (size_t)p.rows[1 + m0 + lr] * p.K : nullptr;
+    const float* a_row = m0 + lr < n_rows ? p.A + (size_t)row_at(m0 + lr) * p.K : nullptr;
     const float* b_row = !B_BY_K && n0 + lr < p.N ? p.B + (size_t)(n0 + lr) * p.K : nullptr;
     float4 ra[2], rb[2];
     auto fetch = [&](int kb) {
@@ -136,10 +138,15 @@ rows_product_kernel(const RowsProductParams p) {
     for (int i = 0; i < 8; ++i) {
       const int r = m0 + (i < 4 ? ty + i : 60 + ty + i);
       if (r >= n_rows) continue;
-      float* dst = p.C + (size_t)p.rows[1 + r] * p.N;
+      float* dst = p.C + (size_t)row_at(r) * p.N;
 #pragma unroll
       for (int j = 0; j < 8; j += 4) {
         const int n = n0 + (j == 0 ? tx : 64 + tx);
+        if (p.bias != nullptr) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (n + q < p.N) acc[i][j + q] += __ldg(p.bias + n + q);
+        }
         if (p.vec) {
           if (n < p.N) *reinterpret_cast<float4*>(dst + n) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
         } else {

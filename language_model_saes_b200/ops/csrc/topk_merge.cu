@@ -1034,8 +1034,33 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
       }
     }
   }
-  unsigned thr = descend(mx, k, 16, s_count);  // a bound until the exact value is known (0: fewer than k positive maxima)
   const float nan = __uint_as_float(0x7fffffffu);
+  // the row's zeros (NaN over a norm of 0 or NaN) for columns [c, c + 8)
+  auto clear = [&](int c, bool any_bad) {
+    float z[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) z[i] = 0.0f;
+    if (any_bad) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const unsigned nb = c + i < N ? __float_as_uint(p.norm[c + i]) & 0x7fffffffu : 1u;
+        if (nb == 0u || nb > 0x7f800000u) z[i] = nan;
+      }
+    }
+    if (p.vec) {
+      __stcs(reinterpret_cast<float4*>(out + c), make_float4(z[0], z[1], z[2], z[3]));
+      __stcs(reinterpret_cast<float4*>(out + c + 4), make_float4(z[4], z[5], z[6], z[7]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c + i < N) out[c + i] = z[i];
+    }
+  };
+  if constexpr (MAXIMA) {  // (they leave while the bound is worked out)
+    const bool any_bad = p.top[1] != 0u;
+    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) clear(c, any_bad);
+  }
+  unsigned thr = descend(mx, k, 16, s_count);  // a bound until the exact value is known (0: fewer than k positive maxima)
   auto enter = [&](int c, unsigned key) {
     const int pos = atomicAdd(&s_n, 1);
     if (pos < CAP) { s_key[pos] = key; s_col[pos] = c; }
@@ -1090,26 +1115,11 @@ __device__ __forceinline__ void topk_dense_row(const TopkDenseParams& p, int row
         }
       }
     }
+    if (!by_groups) {
 #pragma unroll 2
-    for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
-      if (!by_groups) visit(c);
-      float z[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) z[i] = 0.0f;
-      if (any_bad) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const unsigned nb = c + i < N ? __float_as_uint(p.norm[c + i]) & 0x7fffffffu : 1u;
-          if (nb == 0u || nb > 0x7f800000u) z[i] = nan;
-        }
-      }
-      if (p.vec) {
-        __stcs(reinterpret_cast<float4*>(out + c), make_float4(z[0], z[1], z[2], z[3]));
-        __stcs(reinterpret_cast<float4*>(out + c + 4), make_float4(z[4], z[5], z[6], z[7]));
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (c + i < N) out[c + i] = z[i];
+      for (int c = threadIdx.x * 8; c < N; c += RT_THREADS * 8) {
+        visit(c);
+        if constexpr (!MAXIMA) clear(c, any_bad);
       }
     }
   } else {

@@ -116,13 +116,13 @@ def most_gathered(F: int) -> int:
     return F // 6
 
 
-def sparse_decode(acts: torch.Tensor, W: torch.Tensor) -> torch.Tensor:
-    """``acts @ W`` for ``acts [..., F]`` with few non-zeros; rows with more than ``most_gathered`` go to a product on the fp32 pipes."""
+def sparse_decode(acts: torch.Tensor, W: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """``acts @ W`` (``+ bias [d]``) for ``acts [..., F]`` with few non-zeros; rows with more than ``most_gathered`` go to a product on the fp32 pipes."""
     rows = acts.reshape(-1, acts.shape[-1])
     (B, F), d = rows.shape, W.shape[1]
     tiles = min(512, -(-B // 128) * -(-d // 128) * 16)
     out = torch.empty(B, d, dtype=torch.float32, device=acts.device)
     part = torch.empty(tiles * 128 * 128, dtype=torch.float32, device=acts.device)
     todo = torch.zeros(2 + B + tiles, dtype=torch.int32, device=acts.device)
-    K._ext().dense_decode(rows, W.detach(), most_gathered(F), todo, part, out)
+    K._ext().dense_decode(rows, W.detach(), bias.detach() if bias is not None else None, most_gathered(F), todo, part, out)
     return out.view(*acts.shape[:-1], d)
