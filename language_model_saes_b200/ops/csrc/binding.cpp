@@ -1,6 +1,7 @@
 // Python bindings (torch extension) for the sm_100a kernels. Tensors are checked for device, dtype and
 // contiguity here; the kernels assume what these checks guarantee.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -1069,6 +1070,24 @@ void adam_turned(const std::vector<Tensor>& p, const std::vector<Tensor>& m, con
   check_cuda(lmsae::adam_turned_launch(q, (int)n, at::cuda::getCurrentCUDAStream()), "adam_turned launch");
 }
 
+// loss (fp32, one element) and the status word (int32 [4], optional) into pinned host memory (fp32 [5]) by a kernel. False, and nothing done, where the device
+// cannot write there.
+bool read_back(const Tensor& loss, const c10::optional<Tensor>& status, const Tensor& host) {
+  if (!loss.is_cuda() || loss.scalar_type() != torch::kFloat32 || loss.numel() != 1 || !host.device().is_cpu() || !host.is_pinned()) return false;
+  TORCH_CHECK(host.scalar_type() == torch::kFloat32 && host.is_contiguous() && host.numel() >= 5, "read_back: host fp32 [5]");
+  if (status.has_value()) { CHECK_T(*status, torch::kInt32); TORCH_CHECK(status->numel() >= 4); }
+  const c10::cuda::CUDAGuard guard(loss.device());
+  void* mapped = nullptr;
+  if (cudaHostGetDevicePointer(&mapped, host.data_ptr(), 0) != cudaSuccess || mapped == nullptr) {
+    cudaGetLastError();
+    return false;
+  }
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  check_cuda(lmsae::read_back_launch(loss.data_ptr<float>(), opt_ptr<const int>(status), static_cast<float*>(mapped), stream), "read_back launch");
+  at::getHostAllocator(at::kCUDA)->record_event(host.data_ptr(), host.storage().data_ptr().get_context(), stream.unwrap());
+  return true;
+}
+
 // ---- Aux-K ----------------------------------------------------------------------------------------------
 // fired int32 [F] (counts of the step), since int64 [F], n_valid int64 (one element) -> {since [F], is_dead bool [F], n_dead int64 [], any fp32 [1], order int32 [cap],
 // row_of int32 [F], WE rows, WD rows [cap, d] bf16, bias [cap], gate [cap]}; truncated int64 (one element) gets one more where more than capacity are dead.
@@ -1740,6 +1759,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("clt_wgrad", &clt_wgrad);
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
+  m.def("read_back", &read_back);
   m.def("column_lists", &column_lists);
   m.def("jumprelu_begin", &jumprelu_begin);
   m.def("jumprelu_end", &jumprelu_end);

@@ -149,6 +149,7 @@ struct DecodeParams {
   float* dval;
 };
 int sparse_decode_launch(const DecodeParams& p, cudaStream_t stream);
+int read_back_launch(const float* loss, const int* status, float* host, cudaStream_t stream);
 int sparse_decode_segments(int d);
 // `wait`: optional (pt.world > 0) bounded wait for the gradient rows of the fused step (phase kPhaseDxhat) at kernel entry
 int sparse_dact_launch(const int* idx, int B, int k, int d, int F, const __nv_bfloat16* W, const __nv_bfloat16* dxhat,

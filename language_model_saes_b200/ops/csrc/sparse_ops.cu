@@ -129,6 +129,19 @@ row_loss_kernel(const float* __restrict__ part, int B, int nseg, float* __restri
   row_loss[row] = s;
 }
 
+// A step's loss and the status word to mapped host memory: five floats (the codes are small integers). Two copies and a conversion on the stream, with
+// the gaps around them, held the next step up by 24 us.
+__global__ void __launch_bounds__(32)
+read_back_kernel(const float* __restrict__ loss, const int* __restrict__ status, volatile float* __restrict__ host) {
+  pdl_wait();
+  if (threadIdx.x < 5) host[threadIdx.x] = threadIdx.x == 0 ? *loss : status != nullptr ? (float)status[threadIdx.x - 1] : 0.0f;
+  __threadfence_system();
+}
+
+int read_back_launch(const float* loss, const int* status, float* host, cudaStream_t stream) {
+  return (int)launch(read_back_kernel, 1, 32, 0, stream, loss, status, host);
+}
+
 static int decode_vpt(int d) { return d >= 1024 ? 2 : 1; }
 int sparse_decode_segments(int d) { return (d / 8 + 32 * decode_vpt(d) - 1) / (32 * decode_vpt(d)); }
 

@@ -48,3 +48,24 @@ def test_rows_beyond_the_lists_width_are_counted(B, N, cap):
     cpu = torch.full((1,), 5, dtype=torch.int64)
     want_idx, want_val = S.column_threshold_rows_to_sparse(x.cpu(), thr.cpu(), cap, overflow=cpu)
     assert torch.equal(idx.cpu(), want_idx) and torch.equal(val.cpu(), want_val) and int(n) == int(cpu) > 5
+
+
+@pytest.mark.parametrize("with_status", [False, True])
+def test_loss_and_status_reach_the_host(with_status):
+    from language_model_saes_b200.trainer import _LossReader
+
+    status = torch.tensor([0, 7, 8, 9], dtype=torch.int32, device=DEV) if with_status else None
+    reader, seen = _LossReader(), []
+    for i in range(7):
+        seen.append(reader.push(torch.full((), 0.1 + i, device=DEV), status))
+    assert seen[0] is None and all(abs(s - (0.1 + i)) < 1e-6 for i, s in enumerate(seen[1:]))
+    assert abs(reader.flush() - 6.1) < 1e-6
+    host = torch.empty(5, pin_memory=True)
+    assert K._ext().read_back(torch.ones(1, device=DEV), torch.arange(4, dtype=torch.int32, device=DEV), host)
+    torch.cuda.synchronize()
+    assert host.tolist() == [1.0, 0.0, 1.0, 2.0, 3.0]
+    assert not K._ext().read_back(torch.ones(1, device=DEV, dtype=torch.float64), None, host) and not K._ext().read_back(torch.ones(1, device=DEV), None, torch.empty(5))
+    bad = torch.tensor([5, 1, 2, 3], dtype=torch.int32, device=DEV)
+    with pytest.raises(K.CollectiveTimeout):
+        reader.push(torch.ones((), device=DEV), bad)
+        reader.flush()
