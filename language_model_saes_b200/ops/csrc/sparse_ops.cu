@@ -14,6 +14,7 @@
 //                         dW_E^T[f,:] = sum d h * x[b,:] in registers from the feature's entry list and
 //                         apply Adam to both rows in the same pass -- the dense gradient is never written
 //                         (replaces kernels/kernels.py:137-225 + torch.optim.Adam in the reference).
+#include <algorithm>
 #include "adam.cuh"
 #include "comm_common.cuh"
 #include "gather.cuh"
@@ -492,79 +493,118 @@ __global__ void csc_fill_kernel(const int* __restrict__ idx, long long n, int F,
   }
 }
 
-// All of it in one CTA, counts and cursors in shared memory: for few entries the two memsets and five launches were most of the
-// time (and of the host's). Entries are read twice, eight at a time in flight per thread. A step of 512 x 8 codes over 256
-// features (d 64): 101 -> 86 us. 32768 entries take 27 us here and 16 us in the grids of the general path: the line lies where both
-// are about even, launches included.
-constexpr int kSmallEntries = 8192, kSmallFeatures = 8192;
-__global__ void __launch_bounds__(SCAN_THREADS)
-csc_small_kernel(const int* __restrict__ idx, int n, int F, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ cursor,
-                 int* __restrict__ entries, int* __restrict__ heavy, int heavy_cap) {
+// All of it in one launch, and no block waits for another: a block owns `span` features and reads all entries, keeps those of its features in lists in
+// shared memory (one per warp, feature and position in one word) and counts the entries of features before its own, which is where its offsets begin.
+// Counts, their scan and the places of the entries then come from the lists. Bound by the instructions of the reading (a subtraction with borrow, a
+// comparison and a ballot per entry in every block), so for few entries. Against a fill and three launches: 4096 entries of 256 features 10.3 -> 4.1 us,
+// 32768 of 4096 9.4 -> 6.7 (with three features in every row 11.2 -> 9.1), 512 of 131072 11.9 -> 4.4; at 111037 entries it would be 12.8 -> 13.2. The line
+// lies where a warp's list holds all that the warp reads, so that no list overflows. Lists per thread without ballots (6.7 -> 6.9), the next
+// entries fetched ahead (7.3) and places drawn by lanes of one feature together (8.1) were slower at 32768.
+// The counter of the long rows is the last word of `heavy`, zero between calls: the blocks take their places in the list from its low bits, and
+// the one that finds all others counted in its high bits leaves the number and the zero.
+constexpr int kRangeBlocks = 148, kRangeSpan = 1 << 12, kRangeTile = SCAN_THREADS * 4, kRangeTiles = 11;
+__global__ void __launch_bounds__(SCAN_THREADS, 1)
+csc_ranges_kernel(const int* __restrict__ idx, int n, int F, int span, int cap, int* __restrict__ counts, int* __restrict__ offsets,
+                  int* __restrict__ cursor, int* __restrict__ entries, int* __restrict__ heavy, int heavy_cap) {
   pdl_wait();
-  extern __shared__ int s_cnt[];  // [F]: counts, then cursors
+  extern __shared__ int s_cnt[];  // [span]: counts, then cursors; then the lists
   __shared__ int s_warp[33];
-  __shared__ int s_heavy;
-  for (int i = threadIdx.x; i < F; i += SCAN_THREADS) s_cnt[i] = 0;
+  __shared__ int s_heavy, s_heavy_at;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned* const list = reinterpret_cast<unsigned*>(s_cnt + span) + warp * cap;
+  const int lo = blockIdx.x * span, width = min(span, F - lo);
+  for (int i = threadIdx.x; i < span; i += SCAN_THREADS) s_cnt[i] = 0;
   if (threadIdx.x == 0) s_heavy = 0;
-  __syncthreads();
-  constexpr int U = 8;
-  for (int i0 = threadIdx.x; i0 < n; i0 += SCAN_THREADS * U) {
-    int f[U];
+
+  constexpr int U = 4;
+  int before = 0, mine = 0;
+  for (int i0 = warp * 128; i0 < n; i0 += kRangeTile * U) {
+    int4 f[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) f[u] = i0 + u * SCAN_THREADS < n ? __ldg(idx + i0 + u * SCAN_THREADS) : -1;
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kRangeTile + lane * 4;
+      f[u] = make_int4(-1, -1, -1, -1);
+      if (i + 3 < n) {
+        f[u] = __ldg(reinterpret_cast<const int4*>(idx + i));
+      } else if (i < n) {
+        f[u].x = idx[i];
+        if (i + 1 < n) f[u].y = idx[i + 1];
+        if (i + 2 < n) f[u].z = idx[i + 2];
+      }
+    }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (f[u] >= 0 && f[u] < F) atomicAdd(&s_cnt[f[u]], 1);
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kRangeTile;
+      if (i >= n) break;
+      const int v[4] = {f[u].x, f[u].y, f[u].z, f[u].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        unsigned rel;
+        asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, %1, 0;" : "=r"(rel), "+r"(before) : "r"(v[j]), "r"(lo));  // (before: less one for an entry below lo)
+        const bool in = rel < (unsigned)width;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (m != 0) {
+          if (in) list[LMSAE_IDX(mine + __popc(m & ((1u << lane) - 1)), cap)] = rel << 20 | (unsigned)(i + lane * 4 + j);
+          mine += __popc(m);
+        }
+      }
+    }
   }
+  int carry;
+  block_exclusive_scan_1024(-before, s_warp, carry);  // (its barriers: the counts are zero)
+  for (int e = lane; e < mine; e += 32) atomicAdd(&s_cnt[list[e] >> 20], 1);
   __syncthreads();
-  int carry = 0;
-  for (int b = 0; b < F; b += SCAN_ELEMS) {
-    const int base = b + threadIdx.x * 4;
-    int c[4];
+  int c[4], place[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      c[i] = base + i < F ? s_cnt[base + i] : 0;
-      if (heavy != nullptr && c[i] > kHeavyRow) {
-        const int pos = atomicAdd(&s_heavy, 1);
-        if (pos < heavy_cap) heavy[1 + pos] = base + i;
-      }
-    }
-    int total;
-    int run = carry + block_exclusive_scan_1024(c[0] + c[1] + c[2] + c[3], s_warp, total);
+  for (int i = 0; i < 4; ++i) {
+    const int rel = threadIdx.x * 4 + i;
+    c[i] = rel < width ? s_cnt[rel] : 0;
+    place[i] = heavy != nullptr && c[i] > kHeavyRow ? atomicAdd(&s_heavy, 1) : -1;
+  }
+  int total;
+  int run = carry + block_exclusive_scan_1024(c[0] + c[1] + c[2] + c[3], s_warp, total);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (base + i < F) {
-        counts[base + i] = c[i];
-        offsets[base + i] = run;
-        s_cnt[base + i] = run;
-        cursor[base + i] = run + c[i];
-      }
-      run += c[i];
+  for (int i = 0; i < 4; ++i) {
+    const int rel = threadIdx.x * 4 + i;
+    if (rel < width) {
+      counts[lo + rel] = c[i];
+      offsets[lo + rel] = run;
+      s_cnt[rel] = run;
+      cursor[lo + rel] = run + c[i];
     }
-    carry += total;
-    __syncthreads();  // (the scan's words are used again; the cursors are in place)
+    run += c[i];
   }
   if (threadIdx.x == 0) {
-    offsets[F] = carry;
-    if (heavy != nullptr) heavy[0] = s_heavy;
+    if (lo + width == F) offsets[F] = carry + total;
+    if (heavy != nullptr) {
+      const unsigned before_me = atomicAdd(reinterpret_cast<unsigned*>(heavy) + heavy_cap, (1u << 24) + (unsigned)s_heavy);
+      s_heavy_at = (int)(before_me & 0xffffffu);
+      if ((before_me >> 24) == gridDim.x - 1) {
+        heavy[0] = s_heavy_at + s_heavy;
+        heavy[heavy_cap] = 0;
+      }
+    }
   }
-  for (int i0 = threadIdx.x; i0 < n; i0 += SCAN_THREADS * U) {
-    int f[U];
+  __syncthreads();
+  for (int e = lane; e < mine; e += 32) entries[LMSAE_IDX(atomicAdd(&s_cnt[list[e] >> 20], 1), n)] = (int)(list[e] & 0xfffffu);
 #pragma unroll
-    for (int u = 0; u < U; ++u) f[u] = i0 + u * SCAN_THREADS < n ? __ldg(idx + i0 + u * SCAN_THREADS) : -1;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (f[u] >= 0 && f[u] < F) entries[atomicAdd(&s_cnt[f[u]], 1)] = i0 + u * SCAN_THREADS;
-  }
+  for (int i = 0; i < 4; ++i)
+    if (place[i] >= 0) heavy[1 + s_heavy_at + place[i]] = lo + threadIdx.x * 4 + i;
 }
 
 int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offsets, int* cursor, int* entries,
                      int* block_sums_buf, int* heavy, int heavy_cap, cudaStream_t stream) {
   if (n < 0 || n > 2147483647LL || F <= 0) return (int)cudaErrorInvalidValue;  // positions are stored as 32-bit ints
-  if (n <= kSmallEntries && F <= kSmallFeatures) {
-    if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;
-    launch(csc_small_kernel, 1, SCAN_THREADS, (size_t)F * sizeof(int), stream, idx, (int)n, F, counts, offsets, cursor, entries, heavy, heavy_cap);
-    return (int)cudaGetLastError();
+  if (n <= kRangeTiles * kRangeTile && F <= kRangeBlocks * kRangeSpan && reinterpret_cast<uintptr_t>(idx) % 16 == 0 &&
+      (heavy == nullptr || (long long)heavy_cap > n / (kHeavyRow + 1))) {
+    const int span = std::max(32, ((F + kRangeBlocks - 1) / kRangeBlocks + 3) & ~3);
+    const int cap = (int)((n + kRangeTile - 1) / kRangeTile) * 128;
+    const int smem = (int)sizeof(int) * (span + cap * (SCAN_THREADS / 32));
+    const cudaError_t e = cudaFuncSetAttribute(csc_ranges_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(int) * (kRangeSpan + kRangeTiles * 128 * (SCAN_THREADS / 32)));
+    if (e != cudaSuccess) return (int)e;
+    return (int)launch(csc_ranges_kernel, (F + span - 1) / span, SCAN_THREADS, smem, stream, idx, (int)n, F, span, cap, counts, offsets, cursor, entries, heavy,
+                       heavy_cap);
   }
   cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)F * sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;

@@ -44,10 +44,20 @@ _STATUS_NAMES = {
 }
 
 
+def _csc_kernels(entries: int, F: int) -> int:
+    """Launches of the counting sort (csc_build_launch): one for few entries, else three or, for long dictionaries, five."""
+    return 1 if entries <= 45056 and F <= 148 * 4096 else 3 if F <= 1 << 17 else 5
+
+
 class _Counting:
     """Proxy of the extension module that counts the device kernels each entry point launches."""
 
-    KERNELS_PER_CALL = {"csc_build": 5, "exclusive_scan": 3, "topk_step": 8, "topk_encode": 7}
+    KERNELS_PER_CALL = {
+        "csc_build": lambda idx, F, *_: _csc_kernels(idx.numel(), F),
+        "exclusive_scan": 3,
+        "topk_step": lambda x, label, k, route, mode, splits, units, enc, *_: 5 + _csc_kernels(x.shape[0] * k, enc[3].shape[0]),
+        "topk_encode": 7,
+    }
 
     def __init__(self, mod):
         self._mod = mod
@@ -58,7 +68,7 @@ class _Counting:
         n = self.KERNELS_PER_CALL.get(name, 1)
 
         def call(*args, **kwargs):
-            self.launches += n
+            self.launches += n(*args, **kwargs) if callable(n) else n
             return fn(*args, **kwargs)
 
         self.__dict__[name] = call
@@ -547,7 +557,7 @@ class FeatureGroups:
         self.entries = torch.zeros(capacity, dtype=torch.int32, device=device)
         # in one piece, which is one fill on a first step: totals of the counting sort's blocks, the row counter of the update
         # kernel's launches (left at zero by every launch; the launches that read these groups follow each other on one stream)
-        # and the features with long entry lists (count, then features)
+        # and the features with long entry lists (count, then features; the last word is the sort's counter, left at zero by every call)
         n_blocks = (F + 4095) // 4096
         scratch = torch.zeros(n_blocks + 2 + 2 + capacity // HEAVY_ROW, dtype=torch.int32, device=device)
         self.block_sums, self.sched, self.heavy = scratch[:n_blocks], scratch[n_blocks : n_blocks + 2], scratch[n_blocks + 2 :]

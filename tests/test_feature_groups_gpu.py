@@ -1,4 +1,4 @@
-"""Grouping codes by feature around the limits of the one-CTA kernel, with empty slots and features of every token."""
+"""Grouping codes by feature around the limits of its kernels, with empty slots and features of every token."""
 
 import pytest
 import torch
@@ -43,3 +43,24 @@ def test_long_dictionaries(F):
         assert torch.equal(idx.reshape(-1)[e], torch.repeat_interleave(torch.arange(F, dtype=torch.int32), counts)) and e.unique().numel() == e.numel()
         heavy, want = groups.heavy.cpu(), torch.nonzero(counts > K.HEAVY_ROW).flatten()
         assert want.numel() == 2 and int(heavy[0]) == 2 and torch.equal(heavy[1:3].sort().values.long(), want)
+
+
+# one launch up to 45056 entries and 148 * 4096 features: both sides of the lines, blocks of 32 features and of 4096, tails of a vector and of a tile,
+# all entries in one block's features, all in one feature, none, and an address that vectors cannot take
+@pytest.mark.parametrize("n,F", [(0, 40), (3, 33), (4095, 33), (4097, 4736), (45055, 4737), (45056, 100), (45057, 100), (45056, 606208), (9000, 606209)])
+def test_few_entries(n, F):
+    g = torch.Generator().manual_seed(n + F)
+    groups = K.FeatureGroups(F, 45057, torch.device("cuda"))
+    spread, narrow = torch.randint(-1, F + 3, (n,), generator=g), torch.randint(max(0, F - 20), F, (n,), generator=g)
+    for flat in (spread, narrow, torch.full((n,), F - 1), torch.full((n,), -1), spread):
+        for shift in (0, 1):
+            idx = torch.zeros(n + 1, dtype=torch.int32, device="cuda")[shift : shift + n].copy_(flat)
+            groups.build(idx)
+            valid = flat[(flat >= 0) & (flat < F)]
+            counts = torch.bincount(valid, minlength=F)
+            off = groups.offsets.cpu()
+            assert torch.equal(groups.counts.cpu().long(), counts) and torch.equal(off.long(), torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)]))
+            e = groups.entries.cpu()[: int(off[-1])].long()
+            assert torch.equal(flat[e], torch.repeat_interleave(torch.arange(F), counts)) and e.unique().numel() == e.numel()
+            heavy, want = groups.heavy.cpu(), torch.nonzero(counts > K.HEAVY_ROW).flatten()
+            assert int(heavy[0]) == want.numel() and torch.equal(heavy[1 : 1 + want.numel()].sort().values.long(), want) and int(heavy[-1]) == 0
