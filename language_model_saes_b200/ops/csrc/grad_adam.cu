@@ -20,7 +20,9 @@
 //   rows               dealt out in small chunks by a counter (entry counts are skewed: a static deal left SMs idle)
 //   long lists         a row with more than kHeavyRow entries (dense features; a few rows of a Lorsa dictionary hold an entry of
 //                      EVERY token) is processed by all groups of a CTA, which share its entries and add up their partial
-//                      rows; one warp alone took 1.1 ms for 2048 entries (the whole launch: 1167 -> 130 us, 8192 rows of 768)
+//                      rows; one warp alone took 1.1 ms for 2048 entries (the whole launch: 1167 -> 130 us, 8192 rows of 768). Pieces of the list are
+//                      cut so that every group gets the same share: 450 entries in pieces of 32 kept 6 of 20 groups idle and the others
+//                      twice as long as 23 each do (a Lorsa step whose 546 long rows hold 245000 of 262144 entries: 737 -> 713 us)
 //
 // Measured, previous kernels (+ the pass for the code gradients where this one replaces it) -> this one:
 //   131072 rows of 4096, both sides          5.09 + 0.43 -> 4.75 ms  (27.9 GB: 5.9 TB/s)
@@ -85,12 +87,12 @@ __host__ __device__ constexpr int gather_batch() { return NCH == 1 ? 8 : NCH == 
 // g += coefficient * row, with DOT also the code gradients against the bf16-rounded row in c.rounded. Returns (encoder side)
 // the sum of this lane's coefficients.
 template <bool IS_D, bool DOT, int W, int NCH>
-__device__ __forceinline__ float gather_side(const GradAdamParams& p, const GroupCtx& c, const __nv_bfloat16* src, int e0, int e1, int first, int stride,
+__device__ __forceinline__ float gather_side(const GradAdamParams& p, const GroupCtx& c, const __nv_bfloat16* src, int e0, int e1, int first, int stride, int piece,
                                              float (&g)[NCH][4]) {
   constexpr int Q = gather_batch<NCH>();
   float coef_sum = 0.0f;
-  for (int eb = e0 + first * 32; eb < e1; eb += stride * 32) {
-    const int n_e = min(32, e1 - eb);
+  for (int eb = e0 + first * piece; eb < e1; eb += stride * piece) {
+    const int n_e = min(piece, e1 - eb);
     int row_l = 0, ent_l = 0;
     float a_l = 0.0f;
     if (c.lane < n_e) {
@@ -347,6 +349,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
       if (f < p.f_begin || f >= p.f_end) continue;
       const int e0 = p.offsets[group], e1 = p.offsets[group + 1];
       const int xr = p.extra_row != nullptr ? p.extra_row[f] : -1;
+      const int rounds = (e1 - e0 + G * 32 - 1) / (G * 32), piece = (e1 - e0 + G * rounds - 1) / (G * rounds);  // (the same share to every group)
       for (int side = 0; side < 2; ++side) {
         const bool is_d = side == 0;
         if (is_d ? !doD : !doE) continue;
@@ -360,12 +363,12 @@ grad_adam_rows_kernel(const GradAdamParams p) {
             failed = !__syncthreads_and(arrived(0, par0));
             if (failed) break;
             round_row<W, NCH>(stages, p.d, c);
-            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, g);
+            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, piece, g);
           } else {
-            gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, g);
+            gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, c.gid, G, piece, g);
           }
         } else {
-          coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, c.gid, G, g);
+          coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, c.gid, G, piece, g);
         }
         if (!is_d && c.wg == 0) {
           coef = warp_sum(coef);
@@ -477,10 +480,10 @@ grad_adam_rows_kernel(const GradAdamParams p) {
           if (failed) break;
           if (e1 > e0) {
             round_row<W, NCH>(c.stage, p.d, c);
-            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, g);
+            gather_side<true, true, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, 32, g);
           }
         } else {
-          gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, g);
+          gather_side<true, false, W, NCH>(p, c, p.dxhat, e0, e1, 0, 1, 32, g);
         }
         if (loadsD != 0) {
           if (!dot_mode) {
@@ -512,7 +515,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
       if (doE) {
         float g[NCH][4];
         init_grad(false, xr, g);
-        float coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, 0, 1, g);
+        float coef = gather_side<false, false, W, NCH>(p, c, inputs_of(f), e0, e1, 0, 1, 32, g);
         if (loadsE != 0) {
           failed = !group_all<W>(c.gid, arrived(c.gid, parity));
           if (failed) break;

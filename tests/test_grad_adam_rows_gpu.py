@@ -166,3 +166,32 @@ def test_encoder_sides_of_several_layers_in_one_launch(d, shared, L, F):
     assert int(groups.heavy[0]) == 2 and groups.sched.tolist() == [0, 0]
     _compare(cpu, gpu, ["W", "m", "v", "b", "mb", "vb"], d)
     assert torch.equal(gpu["S"].float(), gpu["W"].to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("d", [132, 768, 1160, 4100, 8192])
+def test_long_lists_are_cut_evenly(d):
+    """Lists just long enough to be shared, of one entry more or less than whole pieces of 32 for every group, and of every token."""
+    B, F, g = 1300, 60, torch.Generator().manual_seed(d)
+    lengths = [65, 66, 127, 479, 480, 481, 639, 640, 641, 769, 1281, 1300]
+    idx = torch.full((B, len(lengths)), -1, dtype=torch.int32)
+    for i, n in enumerate(lengths):
+        idx[torch.randperm(B, generator=g)[:n], i] = 3 * i
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    cpu = dict(idx=idx, act=r(*idx.shape), dact=torch.zeros(idx.shape), x=r(B, d).to(torch.bfloat16), dx=r(B, d).to(torch.bfloat16), n=torch.zeros(F))
+    for s in "DE":
+        cpu |= {"W" + s: r(F, d), "S" + s: torch.zeros(F, d, dtype=torch.bfloat16), "m" + s: r(F, d) * 0.01, "v" + s: torch.rand(F, d, generator=g) + 1}
+    cpu |= {"b": r(F), "mb": torch.zeros(F), "vb": torch.ones(F)}
+    gpu = {n: t.clone().to(DEV) for n, t in cpu.items()}
+    for t in (cpu, gpu):
+        groups = K.FeatureGroups(F, idx.numel(), t["idx"].device).build(t["idx"])
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], t["WD"], t["mD"], t["vD"], t["SD"], t["WE"], t["mE"], t["vE"], t["SE"], t["b"], t["mb"],
+                           t["vb"], t["n"], None, None, 1e-3, 0.9, 0.999, 1e-8, 1, True, dact_mode=1)  # fmt: skip
+    K.check_status(torch.device(DEV))
+    assert int(groups.heavy[0]) == len(lengths)
+    # code gradients: d products of order one, added up in another order. Encoder moments: 0.1 of a sum of up to 1300 products of order sqrt(d), each
+    # addition rounding a partial sum of about sqrt(1300 d); decoder moments the same with d = 1.
+    assert torch.allclose(gpu["dact"].cpu(), cpu["dact"], atol=2**-24 * d * 4, rtol=1e-4)
+    for n, scale in (("mD", 1.0), ("mE", d**0.5)):
+        atol = 0.1 * 2**-24 * 1300 * 1300**0.5 * scale + 1e-6
+        assert torch.allclose(gpu[n].cpu(), cpu[n], atol=atol, rtol=1e-4), (n, float((gpu[n].cpu() - cpu[n]).abs().max()))
+    assert torch.allclose(gpu["mb"].cpu(), cpu["mb"], atol=0.1 * 2**-24 * 1300 * (1300 * d) ** 0.5, rtol=1e-4)
