@@ -339,9 +339,20 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
 // ---------------------------------------------------------------------------------------------
 // group (row, slot) pairs by feature: counts -> offsets (exclusive scan) -> entries
 // ---------------------------------------------------------------------------------------------
-__global__ void csc_count_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ counts, int* __restrict__ heavy) {
+// (A kernel, because a fill on the stream cannot be launched ahead: 2 us with the gaps around it.)
+__global__ void csc_zero_kernel(int* __restrict__ counts, int F, int* __restrict__ heavy) {
   pdl_wait();
-  if (heavy != nullptr && blockIdx.x == 0 && threadIdx.x == 0) heavy[0] = 0;  // (counted by the scan that follows)
+  if (heavy != nullptr && blockIdx.x == 0 && threadIdx.x == 0) heavy[0] = 0;  // (counted by the scan)
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i0 + 3 < F && reinterpret_cast<uintptr_t>(counts) % 16 == 0) {
+    *reinterpret_cast<int4*>(counts + i0) = make_int4(0, 0, 0, 0);
+  } else {
+    for (int i = i0; i < min(i0 + 4, F); ++i) counts[i] = 0;
+  }
+}
+
+__global__ void csc_count_kernel(const int* __restrict__ idx, long long n, int F, int* __restrict__ counts) {
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int f = idx[i];
     if (f >= 0 && f < F) atomicAdd(&counts[f], 1);
@@ -606,14 +617,13 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
     return (int)launch(csc_ranges_kernel, (F + span - 1) / span, SCAN_THREADS, smem, stream, idx, (int)n, F, span, cap, counts, offsets, cursor, entries, heavy,
                        heavy_cap);
   }
-  cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)F * sizeof(int), stream);
-  if (e != cudaSuccess) return (int)e;
   if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;  // room for every row there can be
+  launch(csc_zero_kernel, (int)(((long long)F + 1023) / 1024), 256, 0, stream, counts, F, heavy);
   const int threads = 256;
   int blocks = (int)((n + threads - 1) / threads);
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  launch(csc_count_kernel, blocks, threads, 0, stream, idx, n, F, counts, heavy);
+  launch(csc_count_kernel, blocks, threads, 0, stream, idx, n, F, counts);
   // `block_sums_buf` holds one int per 4096 features
   const int nblocks = (F + SCAN_ELEMS - 1) / SCAN_ELEMS;
   if (F <= kOneScanFeatures && reinterpret_cast<uintptr_t>(counts) % 16 == 0) {

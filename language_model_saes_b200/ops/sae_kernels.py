@@ -45,8 +45,8 @@ _STATUS_NAMES = {
 
 
 def _csc_kernels(entries: int, F: int) -> int:
-    """Launches of the counting sort (csc_build_launch): one for few entries, else three or, for long dictionaries, five."""
-    return 1 if entries <= 45056 and F <= 148 * 4096 else 3 if F <= 1 << 17 else 5
+    """Launches of the counting sort (csc_build_launch): one for few entries, else four or, for long dictionaries, six."""
+    return 1 if entries <= 45056 and F <= 148 * 4096 else 4 if F <= 1 << 17 else 6
 
 
 class _Counting:
