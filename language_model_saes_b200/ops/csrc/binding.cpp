@@ -1242,12 +1242,19 @@ void chunk_lists(const Tensor& x, const Tensor& maxima, const Tensor& thr, const
 
 // Lists [B, cap] of the bf16 values above their columns' thresholds, in one pass; overflow (int64, one element): the number of rows with more than cap is
 // added. False, and nothing done, where rows or thresholds are not whole aligned vectors or the lists too wide for it.
-bool column_lists(const Tensor& x, const Tensor& col_thr, const Tensor& idx, const Tensor& val, const Tensor& overflow) {
+bool column_lists(const Tensor& x, const Tensor& col_thr, const Tensor& idx, const Tensor& val, const Tensor& overflow, const c10::optional<Tensor>& maxima) {
   CHECK_T(x, torch::kBFloat16); CHECK_T(col_thr, torch::kFloat32); CHECK_T(idx, torch::kInt32); CHECK_T(val, torch::kFloat32); CHECK_T(overflow, torch::kInt64);
-  TORCH_CHECK(x.dim() == 2 && x.size(0) < (1LL << 31) && col_thr.numel() == x.size(1) && idx.dim() == 2 && idx.size(0) == x.size(0) && idx.size(1) < (1LL << 31) &&
+  TORCH_CHECK(x.dim() == 2 && x.size(0) < (1LL << 31) && x.size(1) < (1LL << 31) && col_thr.numel() == x.size(1) && idx.dim() == 2 && idx.size(0) == x.size(0) && idx.size(1) < (1LL << 31) &&
               val.sizes() == idx.sizes() && overflow.numel() == 1, "column_lists: sizes");
   if (!lmsae::row_compact_cols_fits(x.data_ptr(), x.size(1), col_thr.data_ptr<float>(), (int)idx.size(1))) return false;
   const c10::cuda::CUDAGuard guard(x.device());
+  if (maxima.has_value()) {
+    check_cuda(lmsae::chunk_columns_launch(reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), checked_maxima(maxima, x.size(0), x.size(1)), maxima->size(1),
+                                           (int)x.size(0), (int)x.size(1), col_thr.data_ptr<float>(), (int)idx.size(1), idx.data_ptr<int>(), val.data_ptr<float>(),
+                                           reinterpret_cast<unsigned long long*>(overflow.data_ptr<int64_t>()), at::cuda::getCurrentCUDAStream()),
+               "column_lists launch");
+    return true;
+  }
   check_cuda(lmsae::row_compact_launch(1, x.data_ptr(), (int)x.size(0), x.size(1), (int)idx.size(1), idx.data_ptr<int>(), val.data_ptr<float>(), nullptr, nullptr, nullptr,
                                        nullptr, nullptr, col_thr.data_ptr<float>(), nullptr, reinterpret_cast<unsigned long long*>(overflow.data_ptr<int64_t>()),
                                        at::cuda::getCurrentCUDAStream()),
@@ -1323,8 +1330,9 @@ void jumprelu_lists(const Tensor& idx, const Tensor& s_val, const Tensor& norm, 
   check_cuda(lmsae::jumprelu_lists_launch(p, at::cuda::getCurrentCUDAStream()), "jumprelu_lists launch");
 }
 
-// log_theta [F], norm [H, F], bias [H, F] (optional) -> {theta [F], smallest theta / norm [F]} and the biases' sum [F]
-std::vector<Tensor> jumprelu_begin(const Tensor& log_theta, const Tensor& norm, const c10::optional<Tensor>& bias) {
+// log_theta [F], norm [H, F], bias [H, F] (optional) -> {theta [F], smallest theta / norm [F]} and the biases' sum [F]; gate [F] (optional, written): see the kernel
+std::vector<Tensor> jumprelu_begin(const Tensor& log_theta, const Tensor& norm, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate) {
+  if (gate.has_value()) { CHECK_T(*gate, torch::kFloat32); TORCH_CHECK(gate->numel() == log_theta.numel(), "gate [F]"); }
   CHECK_T(log_theta, torch::kFloat32); CHECK_T(norm, torch::kFloat32);
   TORCH_CHECK(norm.dim() == 2 && norm.size(0) > 0 && norm.size(1) == log_theta.numel() && norm.size(1) > 0 && norm.size(1) < INT_MAX - 256, "log_theta [F], norm [H, F]");
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->sizes() == norm.sizes(), "bias [H, F]"); }
@@ -1332,7 +1340,7 @@ std::vector<Tensor> jumprelu_begin(const Tensor& log_theta, const Tensor& norm, 
   std::vector<Tensor> out = {torch::empty({norm.size(1)}, norm.options()), torch::empty({norm.size(1)}, norm.options())};
   if (bias.has_value()) out.push_back(torch::empty({norm.size(1)}, norm.options()));
   check_cuda(lmsae::jumprelu_begin_launch(log_theta.data_ptr<float>(), norm.data_ptr<float>(), opt_ptr<const float>(bias), (int)norm.size(0), (int)norm.size(1),
-                                          out[0].data_ptr<float>(), out[1].data_ptr<float>(), bias.has_value() ? out[2].data_ptr<float>() : nullptr,
+                                          out[0].data_ptr<float>(), out[1].data_ptr<float>(), bias.has_value() ? out[2].data_ptr<float>() : nullptr, opt_ptr<float>(gate),
                                           at::cuda::getCurrentCUDAStream()),
              "jumprelu_begin launch");
   return out;
@@ -1551,7 +1559,7 @@ void comm_bcast_rows(const std::vector<int64_t>& table, const Tensor& src, const
 // x_h . W_h^T over the local heads; the result (+ bias) is stored as bf16 into H_out [M, N], which may be a view of a
 // symmetric buffer that an all-reduce kernel then sums over the head ranks in place.
 void head_sum_gemm(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, int64_t heads, int64_t rows_per_head,
-                   int64_t N, bool pair, const Tensor& status, const Tensor& H_out) {
+                   int64_t N, bool pair, const Tensor& status, const Tensor& H_out, const c10::optional<Tensor>& maxima, const c10::optional<Tensor>& max_gate) {
   CHECK_T(x, torch::kBFloat16);
   CHECK_T(w, torch::kBFloat16);
   CHECK_T(status, torch::kInt32);
@@ -1579,6 +1587,15 @@ void head_sum_gemm(const Tensor& x, const Tensor& w, const c10::optional<Tensor>
   p.b_rows_per_head = (int)rows_per_head;
   p.H = reinterpret_cast<__nv_bfloat16*>(H_out.data_ptr());
   p.ldh = p.N;
+  if (maxima.has_value()) {
+    CHECK_T(*maxima, torch::kFloat32);
+    TORCH_CHECK(maxima->dim() == 2 && maxima->size(0) == p.M && maxima->size(1) == n_tiles * 8 && reinterpret_cast<uintptr_t>(maxima->data_ptr()) % 16 == 0,
+                "maxima: [M, 8 per 256 columns]");
+    if (max_gate.has_value()) { CHECK_T(*max_gate, torch::kFloat32); TORCH_CHECK(max_gate->numel() == p.N, "max_gate: one per column"); }
+    p.maxima = maxima->data_ptr<float>();
+    p.ld_maxima = maxima->size(1);
+    p.max_gate = opt_ptr<const float>(max_gate);
+  }
   int mode = 1;
   if (pair && p.num_panels % 2 == 0) mode |= 8;
   const CUtensorMap ta = make_bf16_tile_map(x.data_ptr(), p.M, p.K, 128);
@@ -1727,7 +1744,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("comm_bcast_rows", &comm_bcast_rows);
   m.def("comm_signal", &comm_signal);
   m.def("comm_allreduce_bf16", &comm_allreduce_bf16);
-  m.def("head_sum_gemm", &head_sum_gemm);
+  m.def("head_sum_gemm", &head_sum_gemm, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("heads"), py::arg("rows_per_head"), py::arg("N"), py::arg("pair"),
+        py::arg("status"), py::arg("H_out"), py::arg("maxima") = py::none(), py::arg("max_gate") = py::none());
   m.def("comm_wait_src", &comm_wait_src);
   m.def("comm_shuffle_rows", &comm_shuffle_rows);
   m.def("comm_decode_scatter", &comm_decode_scatter);
@@ -1760,8 +1778,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("topk_merge", &topk_merge);
   m.def("row_topk", &row_topk);
   m.def("read_back", &read_back);
-  m.def("column_lists", &column_lists);
-  m.def("jumprelu_begin", &jumprelu_begin);
+  m.def("column_lists", &column_lists, py::arg("x"), py::arg("col_thr"), py::arg("idx"), py::arg("val"), py::arg("overflow"), py::arg("maxima") = py::none());
+  m.def("jumprelu_begin", &jumprelu_begin, py::arg("log_theta"), py::arg("norm"), py::arg("bias"), py::arg("gate") = py::none());
   m.def("jumprelu_end", &jumprelu_end);
   m.def("dead_rows", &dead_rows);
   m.def("row_topk_dense", &row_topk_dense);

@@ -316,7 +316,8 @@ struct JumpReluListParams {
   int* n_valid;        // += number of listed entries
 };
 int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream);
-int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, cudaStream_t stream);
+int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, float* gate,
+                          cudaStream_t stream);
 struct JumpReluEndParams {
   int F;
   float *log_theta, *m, *v;
@@ -371,6 +372,9 @@ int chunk_compact_launch(const __nv_bfloat16* x, const float* maxima, long long 
 int chunk_lists_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* thr, const long long* n_ties,
                        const float* col_div, int* nnz, int* ties, int* quota, int cap, int* idx, float* val, unsigned long long* overflow, cudaStream_t stream);
 
+// Values above their column's threshold as lists (column_lists in binding.cpp), by the maxima of the values times the gate of jumprelu_begin.
+int chunk_columns_launch(const __nv_bfloat16* x, const float* maxima, long long ld_maxima, int B, int N, const float* col_thr, int cap, int* idx, float* val,
+                         unsigned long long* overflow, cudaStream_t stream);
 // Row top-k of stored pre-activations (one of H16, H32) by the maxima of 32 columns; sorted: values in descending order.
 int row_select_launch(const __nv_bfloat16* H16, const float* H32, long long ldh, const float* maxima, long long ld_maxima, int M, int N, int k,
                       const float* gate, int sorted, int* out_idx, float* out_val, cudaStream_t stream);

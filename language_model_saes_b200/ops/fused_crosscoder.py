@@ -56,6 +56,14 @@ def FEATURE_SHARDS_ON_FUSED_PATH() -> bool:
     return "1" in (os.environ.get("LMSAE_FUSED_JUMPRELU_SHARDS", "0"), os.environ.get("LMSAE_FUSED_CPU_VERIFIED", "0"))
 
 
+def _lists_by_maxima(B: int, F: int, cap: int) -> bool:
+    """Whether the lists are made by the maxima of 32 columns, which the product leaves beside ``S``, instead of from the whole matrix: product and lists
+    at lists of 256, 16 / 64 / 240 codes a row, us. 4096 x 18432 (d 2304): 269 / 296 / 312 -> 239 / 261 / 284; 4096 x 8192 (768): 73 / 77 / 83 -> 63 / 67 / 81;
+    2048 x 16384 (768): 71 / 73 / 79 -> 65 / 71 / 81; below the line 2048 x 8192: 44 / 44 / 46 -> 40 / 44 / 52, 1024 x 49152: 91 / 95 / 99 -> 95 / 100 / 124 (a
+    warp per row: too few in flight), 4096 x 4096: 48 / 48 / 50 -> 42 / 44 / 52. With fewer than 32 columns per place most groups would be read."""
+    return B >= 2048 and B * F >= 1 << 25 and F >= 32 * cap and F % 8 == 0
+
+
 class FusedCrosscoderStep:
     def __init__(self, cc, betas: tuple[float, float] = (0.9, 0.999), eps: float = 1e-8, list_width: int = 256,
                  jumprelu_lr_factor: float = 1.0):  # fmt: skip
@@ -161,7 +169,8 @@ class FusedCrosscoderStep:
     def sync_params(self) -> None:
         pass
 
-    def _head_sum(self, x16: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    def _head_sum(self, x16: torch.Tensor, bias: torch.Tensor | None = None, maxima: torch.Tensor | None = None,
+                  gate: torch.Tensor | None = None) -> torch.Tensor:  # fmt: skip
         """``sum over all heads of (x_h W_E,h^T + b_E,h)`` as bf16 [B, F] on every rank; ``bias``: the local heads' sum where it is known."""
         from ..parallel.symm import AllReduceComm
 
@@ -177,7 +186,7 @@ class FusedCrosscoderStep:
         # the GEMM accumulates the local heads in one K loop and stores bf16 straight into the symmetric buffer ...
         P = self.comm.matrix(B)
         K._ext().head_sum_gemm(x16, self.WE_bf16.view(self.H_l * self.F, self.d), bias if bias is not None else self.bE.sum(0).contiguous(), self.H_l, self.F, self.F,
-                               True, K.status_buffer(x16.device), P)  # fmt: skip
+                               True, K.status_buffer(x16.device), P, maxima, gate)  # fmt: skip
         # ... which one kernel then sums over the head ranks in place (NVSwitch multicast loads / stores where available)
         return self.comm.all_reduce(B) if self.head_size > 1 else P
 
@@ -205,9 +214,12 @@ class FusedCrosscoderStep:
         grad_scale = 2.0 / (B * H)
         x = x.contiguous()
         on_lists = self.tp == 1 and self.dp == 1 and not quad
+        maxima = gate = None
         if on_lists and x.is_cuda:
-            theta, t_min, *bias = K._ext().jumprelu_begin(self.log_theta, self.dec_norm, self.bE if H_l > 1 else None)
-            S_sum = self._head_sum(x.view(B_l, H_l * d), bias[0] if bias else self.bE[0])
+            if self.head_size == 1 and _lists_by_maxima(B_l, F, cap):
+                maxima, gate = torch.empty(B_l, -(-F // 256) * 8, device=x.device), torch.empty(F, device=x.device)
+            theta, t_min, *bias = K._ext().jumprelu_begin(self.log_theta, self.dec_norm, self.bE if H_l > 1 else None, gate)
+            S_sum = self._head_sum(x.view(B_l, H_l * d), bias[0] if bias else self.bE[0], maxima, gate)
         else:
             S_sum = self._head_sum(x.view(B_l, H_l * d))
             theta = self.log_theta.exp()
@@ -215,7 +227,7 @@ class FusedCrosscoderStep:
             t_min = t_head.amin(0)
         if self.head_size > 1:
             dist.all_reduce(t_min, op=dist.ReduceOp.MIN, group=self.head_group)
-        idx, s_val = S.column_threshold_rows_to_sparse(S_sum, t_min, cap, overflow=self.list_overflow)
+        idx, s_val = S.column_threshold_rows_to_sparse(S_sum, t_min, cap, overflow=self.list_overflow, maxima=maxima)
         if on_lists:
             return self._step_on_lists(x, label, idx, s_val, S_sum, theta, lr, l1_coefficient, float(tanh_stretch), lp_coefficient)
         safe = idx.clamp_min(0).long()

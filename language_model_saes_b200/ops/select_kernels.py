@@ -288,10 +288,12 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
 
 @torch.no_grad()
 def column_threshold_rows_to_sparse(x: torch.Tensor, col_thr: torch.Tensor, cap: int,
-                                    overflow: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+                                    overflow: torch.Tensor | None = None,
+                                    maxima: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
     """Entries of ``x [B, N]`` above their column's threshold ``col_thr [N]`` as padded sparse lists of fixed width ``cap``
     (ascending columns, values unchanged): the JumpReLU selection of pre-activations against per-feature thresholds. Rows
-    with more than ``cap`` such entries keep the first ones and are counted in ``overflow``."""
+    with more than ``cap`` such entries keep the first ones and are counted in ``overflow``. ``maxima``: those of every 32
+    columns that the product stored beside ``x`` with the gate of ``jumprelu_begin``."""
     assert x.ndim == 2 and cap % 8 == 0 and cap > 0
     B = x.shape[0]
     if not _kernel_ok(x):
@@ -310,7 +312,7 @@ def column_threshold_rows_to_sparse(x: torch.Tensor, col_thr: torch.Tensor, cap:
     val = torch.empty(B, cap, dtype=torch.float32, device=x.device)
     col_thr = col_thr.float().contiguous()
     if (overflow is not None and overflow.dtype == torch.int64 and overflow.numel() == 1 and x.dtype == torch.bfloat16
-            and K._ext().column_lists(x, col_thr, idx, val, overflow)):  # fmt: skip
+            and K._ext().column_lists(x, col_thr, idx, val, overflow, maxima)):  # fmt: skip
         return idx, val
     nnz = torch.empty(B, dtype=torch.int32, device=x.device)
     K._ext().row_compact(x, idx, val, nnz, None, None, None, None, col_thr.float().contiguous(), None)

@@ -69,3 +69,35 @@ def test_loss_and_status_reach_the_host(with_status):
     with pytest.raises(K.CollectiveTimeout):
         reader.push(torch.ones((), device=DEV), bad)
         reader.flush()
+
+
+@pytest.mark.parametrize("B,heads,d,F,cap,shift", [(256, 1, 64, 2048, 64, 2.0), (300, 2, 64, 4104, 64, 2.0), (37, 3, 128, 1000, 1024, 0.0), (512, 1, 192, 18432, 256, 2.6), (129, 1, 64, 264, 8, 1.0)])
+def test_lists_by_maxima_are_those_of_the_whole_matrix(B, heads, d, F, cap, shift):
+    """Bit for bit, with thresholds that values equal, of nothing, everything, no number, and beyond the range of their reciprocals; with NaNs and infinities
+    in the values, and rows that hold more than the list."""
+    g = torch.Generator(device=DEV).manual_seed(F)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    x, w, bias = r(B, heads * d).to(torch.bfloat16), (r(heads * F, d) / (heads * d) ** 0.5).to(torch.bfloat16), 0.1 * r(F)
+    log_theta, norm = shift + 0.2 * r(F) - 1.5 * (torch.rand(F, device=DEV, generator=g) < 0.02), torch.ones(heads, F, device=DEV)
+    log_theta[3:9] = torch.tensor([float("-inf"), float("inf"), float("nan"), -90.0, 87.5, -100.0], device=DEV)
+    norm[0, 40], norm[0, 41], norm[0, 42] = -1.0, 0.0, float("inf")
+    bias[100], bias[101], bias[3], bias[4] = 3e38, float("nan"), -1e-39, float("inf")
+    gate = torch.empty(F, device=DEV)
+    theta, t_min, *_ = K._ext().jumprelu_begin(log_theta, norm, None, gate)
+    H, maxima = torch.empty(B, F, dtype=torch.bfloat16, device=DEV), torch.full((B, -(-F // 256) * 8), float("nan"), device=DEV)
+    K._ext().head_sum_gemm(x, w, bias, heads, F, F, True, K.status_buffer(torch.device(DEV)), H, maxima, gate)
+    K.check_status(torch.device(DEV))
+    t_min[200:232] = H[0, 200:232].float().abs()  # (equal is not above; the gates of these are not their reciprocals, but the rows' are looked at below)
+    gate[200:232] = 1.0 / t_min[200:232]
+    K._ext().head_sum_gemm(x, w, bias, heads, F, F, True, K.status_buffer(torch.device(DEV)), H, maxima, gate)
+    plain = H.clone()
+    K._ext().head_sum_gemm(x, w, bias, heads, F, F, True, K.status_buffer(torch.device(DEV)), H)
+    assert torch.equal(plain.view(torch.int16), H.view(torch.int16))
+    got = []
+    for m in (None, maxima):
+        idx, val, over = torch.empty(B, cap, dtype=torch.int32, device=DEV), torch.empty(B, cap, device=DEV), torch.zeros((), dtype=torch.int64, device=DEV)
+        assert K._ext().column_lists(H, t_min, idx, val, over, m)
+        got.append((idx, val, over))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    assert torch.equal(got[1][0][0, : min(cap, int((H[0].float() > t_min).sum()))], torch.nonzero(H[0].float() > t_min).flatten()[:cap].int())
