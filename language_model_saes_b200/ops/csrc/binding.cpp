@@ -1337,10 +1337,10 @@ std::vector<Tensor> jumprelu_begin(const Tensor& log_theta, const Tensor& norm, 
   TORCH_CHECK(norm.dim() == 2 && norm.size(0) > 0 && norm.size(1) == log_theta.numel() && norm.size(1) > 0 && norm.size(1) < INT_MAX - 256, "log_theta [F], norm [H, F]");
   if (bias.has_value()) { CHECK_T(*bias, torch::kFloat32); TORCH_CHECK(bias->sizes() == norm.sizes(), "bias [H, F]"); }
   const c10::cuda::CUDAGuard guard(norm.device());
-  std::vector<Tensor> out = {torch::empty({norm.size(1)}, norm.options()), torch::empty({norm.size(1)}, norm.options())};
-  if (bias.has_value()) out.push_back(torch::empty({norm.size(1)}, norm.options()));
-  check_cuda(lmsae::jumprelu_begin_launch(log_theta.data_ptr<float>(), norm.data_ptr<float>(), opt_ptr<const float>(bias), (int)norm.size(0), (int)norm.size(1),
-                                          out[0].data_ptr<float>(), out[1].data_ptr<float>(), bias.has_value() ? out[2].data_ptr<float>() : nullptr, opt_ptr<float>(gate),
+  std::vector<Tensor> out = {at::exp(log_theta), torch::empty({norm.size(1)}, norm.options())};
+  if (bias.has_value()) out.push_back(bias->sum(0));
+  check_cuda(lmsae::jumprelu_begin_launch(out[0].data_ptr<float>(), norm.data_ptr<float>(), (int)norm.size(0), (int)norm.size(1),
+                                          out[1].data_ptr<float>(), opt_ptr<float>(gate),
                                           at::cuda::getCurrentCUDAStream()),
              "jumprelu_begin launch");
   return out;

@@ -70,33 +70,29 @@ int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream) {
   return (int)cudaGetLastError();
 }
 
-// What a step needs of its thresholds and norms: theta = exp(log theta), the smallest threshold theta / ||W_D,h row|| of the heads (a NaN stays one),
-// and where wanted the sum of the heads' encoder biases and the gate by which chunk_columns_kernel finds what passes the threshold: times its gate, such a
+// What a step needs of its thresholds theta and norms: the smallest threshold theta / ||W_D,h row|| of the heads (a NaN stays one),
+// and where wanted the gate by which chunk_columns_kernel finds what passes the threshold: times its gate, such a
 // value is at least 1 less two roundings. Where 1 / threshold would leave the range, infinity (every positive value is looked at), below zero and for a
-// NaN a NaN (everything is). (exp in 64 bits: the fast fp32 one that this file's flags select is further off than torch's.)
+// NaN a NaN (everything is). (theta and the heads' summed bias are torch's: a threshold that differs
+// in its last bit moves values across it.)
 __global__ void __launch_bounds__(256)
-jumprelu_begin_kernel(const float* __restrict__ log_theta, const float* __restrict__ norm, const float* __restrict__ bias, int H, int F, float* __restrict__ theta,
-                      float* __restrict__ t_min, float* __restrict__ bias_sum, float* __restrict__ gate) {
+jumprelu_begin_kernel(const float* __restrict__ theta, const float* __restrict__ norm, int H, int F, float* __restrict__ t_min, float* __restrict__ gate) {
   pdl_wait();
   const int f = blockIdx.x * 256 + threadIdx.x;
   if (f >= F) return;
-  const float th = (float)exp((double)log_theta[f]);
-  theta[f] = th;
-  float m = __int_as_float(0x7f800000), b = 0.0f;
+  const float th = theta[f];
+  float m = __int_as_float(0x7f800000);
   for (int h = 0; h < H; ++h) {
     const float t = __fdiv_rn(th, norm[(size_t)h * F + f]);
     if (m == m && (t != t || t < m)) m = t;
-    if (bias_sum != nullptr) b += bias[(size_t)h * F + f];
   }
   t_min[f] = m;
   if (gate != nullptr) gate[f] = m >= 0.0f ? (m > 0x1p-125f && m < 0x1p125f ? __fdiv_rn(1.0f, m) : __int_as_float(0x7f800000)) : __int_as_float(0x7fffffff);
-  if (bias_sum != nullptr) bias_sum[f] = b;
 }
 
-int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, float* gate,
-                          cudaStream_t stream) {
+int jumprelu_begin_launch(const float* theta, const float* norm, int H, int F, float* t_min, float* gate, cudaStream_t stream) {
   if (H <= 0 || F <= 0) return (int)cudaErrorInvalidValue;
-  return (int)launch(jumprelu_begin_kernel, (F + 255) / 256, 256, 0, stream, log_theta, norm, bias, H, F, theta, t_min, bias_sum, gate);
+  return (int)launch(jumprelu_begin_kernel, (F + 255) / 256, 256, 0, stream, theta, norm, H, F, t_min, gate);
 }
 
 // The end of a step: Adam on log theta, whose gradient is d theta * theta, and the step's figures out[0..4): loss l_rec + l_s + l_p, l_s, l_p, active entries per

@@ -316,8 +316,7 @@ struct JumpReluListParams {
   int* n_valid;        // += number of listed entries
 };
 int jumprelu_lists_launch(const JumpReluListParams& p, cudaStream_t stream);
-int jumprelu_begin_launch(const float* log_theta, const float* norm, const float* bias, int H, int F, float* theta, float* t_min, float* bias_sum, float* gate,
-                          cudaStream_t stream);
+int jumprelu_begin_launch(const float* theta, const float* norm, int H, int F, float* t_min, float* gate, cudaStream_t stream);
 struct JumpReluEndParams {
   int F;
   float *log_theta, *m, *v;

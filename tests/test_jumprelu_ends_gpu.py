@@ -15,10 +15,10 @@ def test_thresholds_and_bias_sum(H, F):
     log_theta, norm, bias = torch.randn(F, device=DEV, generator=g) * 3, torch.rand(H, F, device=DEV, generator=g) + 0.1, torch.randn(H, F, device=DEV, generator=g)
     norm[0, 1], norm[H - 1, 2], log_theta[3] = 0.0, float("nan"), float("nan")
     theta, t_min, total = K._ext().jumprelu_begin(log_theta, norm, bias)
-    want = log_theta.double().exp()
-    assert torch.allclose(theta.double(), want, rtol=2.0**-23, atol=0.0, equal_nan=True)
+    # the last bit of a threshold decides which values pass it: torch's, to the bit (which is up to 2 units in the last place from the exponential)
+    assert torch.equal(theta.nan_to_num(nan=-1.0), log_theta.exp().nan_to_num(nan=-1.0))
     assert torch.equal(t_min.nan_to_num(nan=-1.0), (theta / norm).amin(0).nan_to_num(nan=-1.0))
-    assert torch.allclose(total, bias.sum(0), atol=2.0**-23 * H * 4)
+    assert torch.equal(total, bias.sum(0))
     assert len(K._ext().jumprelu_begin(log_theta, norm, None)) == 2
 
 
