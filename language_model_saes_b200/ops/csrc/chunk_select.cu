@@ -208,42 +208,44 @@ chunk_compact_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
   }
 }
 
-// Places for equal values, n_ties of them for all rows, in the order of the rows: quota[row]. One CTA.
+// Places for equal values, n_ties of them for all rows, in the order of the rows: quota[row]. One CTA. (Sums in 64 bits: rows of 2^19 equal
+// values reach 2^31 within a turn of 4096.)
 __global__ void __launch_bounds__(1024)
 tie_quota_kernel(const int* __restrict__ ties, const long long* __restrict__ n_ties, int B, int* __restrict__ quota) {
   pdl_wait();
-  __shared__ int s_sum[32];
-  __shared__ int s_total;
+  __shared__ long long s_sum[32];
+  __shared__ long long s_total;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   long long left = *n_ties;
   for (int r0 = 0; r0 < B; r0 += 4096) {
-    int t[4], mine = 0;
+    int t[4];
+    long long mine = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = r0 + (int)threadIdx.x * 4 + i;
       t[i] = r < B ? ties[r] : 0;
       mine += t[i];
     }
-    int sum = mine;
+    long long sum = mine;
 #pragma unroll
     for (int o = 1; o < 32; o *= 2) {
-      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      const long long v = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += v;
     }
     if (lane == 31) s_sum[warp] = sum;
     __syncthreads();
     if (warp == 0) {
-      int w = s_sum[lane];
+      long long w = s_sum[lane];
 #pragma unroll
       for (int o = 1; o < 32; o *= 2) {
-        const int v = __shfl_up_sync(0xffffffffu, w, o);
+        const long long v = __shfl_up_sync(0xffffffffu, w, o);
         if (lane >= o) w += v;
       }
       s_sum[lane] = w;
       if (lane == 31) s_total = w;
     }
     __syncthreads();
-    long long before = (long long)(sum - mine) + (warp > 0 ? s_sum[warp - 1] : 0);
+    long long before = sum - mine + (warp > 0 ? s_sum[warp - 1] : 0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = r0 + (int)threadIdx.x * 4 + i;

@@ -140,6 +140,18 @@ def test_lists_in_one_pass_with_quotas_afterwards(B, N, data):
         assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(nan=7.0), want[1].nan_to_num(nan=7.0)) and torch.equal(got_n, want_n), n_ties
 
 
+def test_quotas_of_more_equal_values_than_31_bits_count():
+    """4096 rows of 600000 values equal to the threshold are 2.5e9: the places go to the first row, and to no other."""
+    B, N, places = 4096, 600000, 300000
+    x = torch.ones(B, N, dtype=torch.bfloat16, device=DEV)
+    maxima = torch.ones(B, N // 32, device=DEV)
+    nnz, idx = torch.empty(B, dtype=torch.int32, device=DEV), torch.empty(B, 8, dtype=torch.int32, device=DEV)
+    over = torch.zeros(1, dtype=torch.int64, device=DEV)
+    K._ext().chunk_lists(x, maxima, torch.ones(1, device=DEV), torch.tensor([places], device=DEV), None, nnz, idx, torch.empty(B, 8, device=DEV), over)
+    assert int(nnz[0]) == places and not nnz[1:].any() and int(over) == 1
+    assert torch.equal(idx[0].cpu(), torch.arange(8, dtype=torch.int32)) and bool((idx[1:] == -1).all())
+
+
 @pytest.mark.parametrize("M,N,k", [(1, 8, 3), (5, 2048, 512), (300, 4104, 100), (40, 9216, 512), (3, 3000, 1500)])
 @pytest.mark.parametrize("data", ["normal", "few positive", "ties", "no gate"])
 def test_row_topk_as_a_matrix(M, N, k, data):
