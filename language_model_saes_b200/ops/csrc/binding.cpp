@@ -575,7 +575,8 @@ void auxk_loss_grad(const Tensor& xhat, const Tensor& aux_rec, const Tensor& lab
 }
 
 void csc_build(const Tensor& idx, int64_t F, const Tensor& counts, const Tensor& offsets, const Tensor& cursor,
-               const Tensor& entries, const Tensor& block_sums, const c10::optional<Tensor>& heavy) {
+               const Tensor& entries, const Tensor& block_sums, const c10::optional<Tensor>& heavy, const c10::optional<Tensor>& places) {
+  if (places.has_value()) { CHECK_T(*places, torch::kInt32); TORCH_CHECK(places->numel() >= 1); }
   if (heavy.has_value()) { CHECK_T(*heavy, torch::kInt32); TORCH_CHECK(heavy->numel() >= 1); }
   CHECK_T(idx, torch::kInt32);
   CHECK_T(counts, torch::kInt32);
@@ -589,7 +590,7 @@ void csc_build(const Tensor& idx, int64_t F, const Tensor& counts, const Tensor&
   check_cuda(lmsae::csc_build_launch(idx.data_ptr<int>(), idx.numel(), (int)F, counts.data_ptr<int>(),
                                      offsets.data_ptr<int>(), cursor.data_ptr<int>(), entries.data_ptr<int>(),
                                      block_sums.data_ptr<int>(), opt_ptr<int>(heavy),
-                                     heavy.has_value() ? (int)heavy->numel() - 1 : 0, at::cuda::getCurrentCUDAStream()),
+                                     heavy.has_value() ? (int)heavy->numel() - 1 : 0, opt_ptr<int>(places), at::cuda::getCurrentCUDAStream()),
              "csc_build launch");
 }
 
@@ -815,13 +816,13 @@ std::vector<Tensor> colsum_adam(const std::vector<Tensor>& a, const std::vector<
 
 // One training step of a TopK dictionary on one GPU, the calls of FusedTopKSAEStep.step in their order: host work between the launches is what the
 // smallest steps consist of. route (sae_kernels.topk_route): 0 top-k in the GEMM's epilogue and merge, 1 fp32 pre-activations and row_select, 2 bf16 ones
-// and row_select, 3 row_topk by maxima, 4 row_topk. groups: counts, offsets, cursor, entries, block sums, heavy, sched of a FeatureGroups; enc and dec:
+// and row_select, 3 row_topk by maxima, 4 row_topk. groups: counts, offsets, cursor, entries, block sums, heavy, places, sched of a FeatureGroups; enc and dec:
 // parameter, both moments, bf16 shadow; b_E and b_D (empty: none): bias and both moments. Returns the mean loss; loss_sum is left at zero.
 Tensor topk_step(const Tensor& x, const Tensor& label, int64_t k, int64_t route, int64_t mode, int64_t splits, int64_t units, const std::vector<Tensor>& enc,
                  const std::vector<Tensor>& dec, const std::vector<Tensor>& b_E, const std::vector<Tensor>& b_D, const Tensor& dec_norm, bool use_gate,
                  const c10::optional<Tensor>& row_weight, double grad_scale, const Tensor& loss_sum, const std::vector<Tensor>& groups, const Tensor& counters,
                  double lr, double beta1, double beta2, double eps, int64_t step, double loss_den, const Tensor& status) {
-  TORCH_CHECK(enc.size() == 4 && dec.size() == 4 && b_E.size() == 3 && (b_D.empty() || b_D.size() == 3) && groups.size() == 7 && x.dim() == 2, "topk_step: arguments");
+  TORCH_CHECK(enc.size() == 4 && dec.size() == 4 && b_E.size() == 3 && (b_D.empty() || b_D.size() == 3) && groups.size() == 8 && x.dim() == 2, "topk_step: arguments");
   const c10::cuda::CUDAGuard guard(x.device());
   const auto none = c10::optional<Tensor>();
   const c10::optional<Tensor> gate = use_gate ? c10::optional<Tensor>(dec_norm) : none, bias_d = b_D.empty() ? none : c10::optional<Tensor>(b_D[0]);
@@ -842,10 +843,10 @@ Tensor topk_step(const Tensor& x, const Tensor& label, int64_t k, int64_t route,
   }
   const Tensor dxhat = torch::empty({M, dec[3].size(1)}, x.options()), dact = torch::empty_like(act);
   sparse_decode(idx, act, dec[3], bias_d, none, none, label, row_weight, grad_scale, dxhat, loss_sum, none, none);
-  csc_build(idx, N, groups[0], groups[1], groups[2], groups[3], groups[4], groups[5]);
+  csc_build(idx, N, groups[0], groups[1], groups[2], groups[3], groups[4], groups[5], groups[6]);
   sparse_grad_adam(groups[1], groups[3], act, dact, x, dxhat, dec[0], dec[1], dec[2], dec[3], enc[0], enc[1], enc[2], enc[3], b_E[0], b_E[1], b_E[2], dec_norm, none,
                    none, lr, beta1, beta2, eps, step, true, 0, -1, 0, none, 0, none, none, status, 0, {}, {}, 0, none, none, none, none, none, none, none, 1, groups[5], 0,
-                   groups[6], -1, 0, false);
+                   groups[7], -1, 0, false);
   const std::vector<Tensor> nothing;
   return colsum_adam(b_D.empty() ? nothing : std::vector<Tensor>{dxhat}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[0]},
                      b_D.empty() ? nothing : std::vector<Tensor>{b_D[1]}, b_D.empty() ? nothing : std::vector<Tensor>{b_D[2]}, counters, lr, beta1, beta2, eps, step,
@@ -1794,7 +1795,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sparse_decode", &sparse_decode);
   m.def("sparse_dact", &sparse_dact);
   m.def("mse_loss_grad", &mse_loss_grad);
-  m.def("csc_build", &csc_build);
+  m.def("csc_build", &csc_build, py::arg("idx"), py::arg("F"), py::arg("counts"), py::arg("offsets"), py::arg("cursor"), py::arg("entries"), py::arg("block_sums"),
+        py::arg("heavy"), py::arg("places") = py::none());
   m.def("jumprelu_lists", &jumprelu_lists);
   m.def("auxk_loss_grad", &auxk_loss_grad);
   m.def("sparse_grad_adam", &sparse_grad_adam);

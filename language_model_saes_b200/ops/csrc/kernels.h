@@ -158,9 +158,9 @@ int mse_loss_grad_launch(const float* xhat, const __nv_bfloat16* label, const fl
                          int rows, int d, float grad_scale, __nv_bfloat16* dxhat, float* loss_sum, float* row_loss,
                          cudaStream_t stream);
 // heavy (optional): [0] = number of features with more than kHeavyRow entries, then those features, in no particular order
-// (at most heavy_cap of them are listed). Its last word, heavy[heavy_cap], is zero before and after where the list cannot reach it.
+// (at most heavy_cap of them are listed). places (optional; with it few entries take one launch): a word that is zero between calls
 int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offsets, int* cursor, int* entries,
-                     int* block_sums_buf, int* heavy, int heavy_cap, cudaStream_t stream);
+                     int* block_sums_buf, int* heavy, int heavy_cap, int* places, cudaStream_t stream);
 constexpr int kHeavyRow = 64;
 
 struct AdamHyper {

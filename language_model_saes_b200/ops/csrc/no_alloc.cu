@@ -52,5 +52,5 @@ extern "C" int lmsae_csc_build_noalloc(const int* idx, long long n, int F, int* 
   int* block_sums = scratch + 2 * LMSAE_NOALLOC_MAX_FEATURES;
   // csc_build_launch zeroes the counters it uses on `stream` before counting, so the
   // leftovers of the previous call do not matter; cursor and block totals are fully overwritten.
-  return lmsae::csc_build_launch(idx, n, F, counts, offsets, cursor, entries, block_sums, nullptr, 0, stream);
+  return lmsae::csc_build_launch(idx, n, F, counts, offsets, cursor, entries, block_sums, nullptr, 0, nullptr, stream);
 }

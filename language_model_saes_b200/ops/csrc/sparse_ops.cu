@@ -511,12 +511,12 @@ __global__ void csc_fill_kernel(const int* __restrict__ idx, long long n, int F,
 // 32768 of 4096 9.4 -> 6.7 (with three features in every row 11.2 -> 9.1), 512 of 131072 11.9 -> 4.4; at 111037 entries it would be 12.8 -> 13.2. The line
 // lies where a warp's list holds all that the warp reads, so that no list overflows. Lists per thread without ballots (6.7 -> 6.9), the next
 // entries fetched ahead (7.3) and places drawn by lanes of one feature together (8.1) were slower at 32768.
-// The counter of the long rows is the last word of `heavy`, zero between calls: the blocks take their places in the list from its low bits, and
-// the one that finds all others counted in its high bits leaves the number and the zero.
+// `places` counts the long rows, a word of its own that is zero between calls: the blocks take their places in the list `heavy` from its low bits,
+// and the one that finds all others counted in its high bits leaves the number in heavy[0] and the zero.
 constexpr int kRangeBlocks = 148, kRangeSpan = 1 << 12, kRangeTile = SCAN_THREADS * 4, kRangeTiles = 11;
 __global__ void __launch_bounds__(SCAN_THREADS, 1)
 csc_ranges_kernel(const int* __restrict__ idx, int n, int F, int span, int cap, int* __restrict__ counts, int* __restrict__ offsets,
-                  int* __restrict__ cursor, int* __restrict__ entries, int* __restrict__ heavy, int heavy_cap) {
+                  int* __restrict__ cursor, int* __restrict__ entries, int* __restrict__ heavy, int* __restrict__ places) {
   pdl_wait();
   extern __shared__ int s_cnt[];  // [span]: counts, then cursors; then the lists
   __shared__ int s_warp[33];
@@ -588,11 +588,11 @@ csc_ranges_kernel(const int* __restrict__ idx, int n, int F, int span, int cap, 
   if (threadIdx.x == 0) {
     if (lo + width == F) offsets[F] = carry + total;
     if (heavy != nullptr) {
-      const unsigned before_me = atomicAdd(reinterpret_cast<unsigned*>(heavy) + heavy_cap, (1u << 24) + (unsigned)s_heavy);
+      const unsigned before_me = atomicAdd(reinterpret_cast<unsigned*>(places), (1u << 24) + (unsigned)s_heavy);
       s_heavy_at = (int)(before_me & 0xffffffu);
       if ((before_me >> 24) == gridDim.x - 1) {
         heavy[0] = s_heavy_at + s_heavy;
-        heavy[heavy_cap] = 0;
+        *places = 0;
       }
     }
   }
@@ -604,10 +604,10 @@ csc_ranges_kernel(const int* __restrict__ idx, int n, int F, int span, int cap, 
 }
 
 int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offsets, int* cursor, int* entries,
-                     int* block_sums_buf, int* heavy, int heavy_cap, cudaStream_t stream) {
+                     int* block_sums_buf, int* heavy, int heavy_cap, int* places, cudaStream_t stream) {
   if (n < 0 || n > 2147483647LL || F <= 0) return (int)cudaErrorInvalidValue;  // positions are stored as 32-bit ints
-  if (n <= kRangeTiles * kRangeTile && F <= kRangeBlocks * kRangeSpan && reinterpret_cast<uintptr_t>(idx) % 16 == 0 &&
-      (heavy == nullptr || (long long)heavy_cap > n / (kHeavyRow + 1))) {
+  if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;  // room for every row there can be
+  if (n <= kRangeTiles * kRangeTile && F <= kRangeBlocks * kRangeSpan && reinterpret_cast<uintptr_t>(idx) % 16 == 0 && (heavy == nullptr || places != nullptr)) {
     const int span = std::max(32, ((F + kRangeBlocks - 1) / kRangeBlocks + 3) & ~3);
     const int cap = (int)((n + kRangeTile - 1) / kRangeTile) * 128;
     const int smem = (int)sizeof(int) * (span + cap * (SCAN_THREADS / 32));
@@ -615,9 +615,8 @@ int csc_build_launch(const int* idx, long long n, int F, int* counts, int* offse
                                                (int)sizeof(int) * (kRangeSpan + kRangeTiles * 128 * (SCAN_THREADS / 32)));
     if (e != cudaSuccess) return (int)e;
     return (int)launch(csc_ranges_kernel, (F + span - 1) / span, SCAN_THREADS, smem, stream, idx, (int)n, F, span, cap, counts, offsets, cursor, entries, heavy,
-                       heavy_cap);
+                       places);
   }
-  if (heavy != nullptr && (long long)heavy_cap < n / (kHeavyRow + 1)) return (int)cudaErrorInvalidValue;  // room for every row there can be
   launch(csc_zero_kernel, (int)(((long long)F + 1023) / 1024), 256, 0, stream, counts, F, heavy);
   const int threads = 256;
   int blocks = (int)((n + threads - 1) / threads);

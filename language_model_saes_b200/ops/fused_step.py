@@ -601,7 +601,7 @@ class FusedTopKSAEStep:
             (self.WE, *self.state["W_E"], self.WE_bf16), (self.WD, *self.state["W_D"], self.WD_bf16), (self.bE, *self.state["b_E"]),
             () if self.bD is None else (self.bD, *self.state["b_D"]), self.dec_norm, self.use_gate, row_weight,
             2.0 / (n_tokens_global if n_tokens_global is not None else B), self.loss_sum,
-            (groups.counts, groups.offsets, groups.cursor, groups.entries, groups.block_sums, groups.heavy, groups.sched), self.bias_update.counters,
+            (groups.counts, groups.offsets, groups.cursor, groups.entries, groups.block_sums, groups.heavy, groups.places, groups.sched), self.bias_update.counters,
             lr, b1, b2, self.eps, self.t + 1, 1.0 if row_weight is not None else float(B), K.status_buffer(x.device),
         )  # fmt: skip
         self.t += 1

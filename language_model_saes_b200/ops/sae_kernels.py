@@ -557,10 +557,11 @@ class FeatureGroups:
         self.entries = torch.zeros(capacity, dtype=torch.int32, device=device)
         # in one piece, which is one fill on a first step: totals of the counting sort's blocks, the row counter of the update
         # kernel's launches (left at zero by every launch; the launches that read these groups follow each other on one stream)
-        # and the features with long entry lists (count, then features; the last word is the sort's counter, left at zero by every call)
+        # the sort's counter of long entry lists (left at zero by every call) and the features with those (count, then features)
         n_blocks = (F + 4095) // 4096
-        scratch = torch.zeros(n_blocks + 2 + 2 + capacity // HEAVY_ROW, dtype=torch.int32, device=device)
-        self.block_sums, self.sched, self.heavy = scratch[:n_blocks], scratch[n_blocks : n_blocks + 2], scratch[n_blocks + 2 :]
+        scratch = torch.zeros(n_blocks + 3 + 2 + capacity // HEAVY_ROW, dtype=torch.int32, device=device)
+        self.block_sums, self.sched = scratch[:n_blocks], scratch[n_blocks : n_blocks + 2]
+        self.places, self.heavy = scratch[n_blocks + 2 : n_blocks + 3], scratch[n_blocks + 3 :]
         self.heavy_base = 0
 
     def part(self, lo: int, hi: int) -> "FeatureGroups":
@@ -577,7 +578,7 @@ class FeatureGroups:
         if self.heavy.numel() < 2 + n // HEAVY_ROW:
             self.heavy = torch.zeros(2 + n // HEAVY_ROW, dtype=torch.int32, device=idx.device)
         if idx.is_cuda:
-            _ext().csc_build(idx, self.F, self.counts, self.offsets, self.cursor, self.entries, self.block_sums, self.heavy)
+            _ext().csc_build(idx, self.F, self.counts, self.offsets, self.cursor, self.entries, self.block_sums, self.heavy, self.places)
         else:
             flat = idx.reshape(-1)
             valid = flat >= 0

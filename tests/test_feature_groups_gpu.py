@@ -64,3 +64,22 @@ def test_few_entries(n, F):
             assert torch.equal(flat[e], torch.repeat_interleave(torch.arange(F), counts)) and e.unique().numel() == e.numel()
             heavy, want = groups.heavy.cpu(), torch.nonzero(counts > K.HEAVY_ROW).flatten()
             assert int(heavy[0]) == want.numel() and torch.equal(heavy[1 : 1 + want.numel()].sort().values.long(), want) and int(heavy[-1]) == 0
+
+
+@pytest.mark.parametrize("n", [65 * 3, 45056, 65 * 800])
+def test_what_the_list_of_long_rows_held_does_not_matter(n):
+    """The sort by itself with a list buffer that nobody zeroed and that has room for exactly the rows there can be, all of which are long; then the
+    one-launch form with a counter after a list that filled its buffer."""
+    F = n // 65 + 3
+    flat = torch.arange(n, dtype=torch.int32, device="cuda") % (n // 65)
+    new = lambda size: torch.full((size,), -(2**31) + 12345, dtype=torch.int32, device="cuda")  # noqa: E731
+    places = torch.zeros(1, dtype=torch.int32, device="cuda")
+    heavy = new(1 + n // 65)
+    for counter in (None, places, None, places):
+        counts, offsets, cursor, entries, sums = new(F), new(F + 1), new(F), new(n), new((F + 4095) // 4096)
+        K._ext().csc_build(flat, F, counts, offsets, cursor, entries, sums, heavy, counter)
+        want = torch.bincount(flat.long(), minlength=F)
+        long_rows = torch.nonzero(want > K.HEAVY_ROW).flatten()
+        assert torch.equal(counts.long(), want) and torch.equal(offsets[1:].long(), want.cumsum(0)) and int(places) == 0
+        assert long_rows.numel() == n // 65 == int(heavy[0]) and torch.equal(heavy[1:].sort().values.long(), long_rows)
+        assert torch.equal(flat[entries.long()], torch.repeat_interleave(torch.arange(F, dtype=torch.int32, device="cuda"), want))
