@@ -61,3 +61,21 @@ def test_column_threshold_lists(B, N, cap, level):
     idx, val = S.column_threshold_rows_to_sparse(x.to(DEV), thr.to(DEV), cap, overflow=over)
     ref_idx, ref_val = S.column_threshold_rows_to_sparse(x, thr, cap, overflow=ref_over)
     assert torch.equal(idx.cpu(), ref_idx) and torch.equal(val.cpu(), ref_val) and int(over) == int(ref_over)
+
+
+# bins per thread from one to 64, in whole vectors and not; numbers of bins that are no whole vectors although a thread's share is; a histogram at an odd address
+@pytest.mark.parametrize("nbins", [1, 7, 1024, 3072, 4095, 32640, 32641, 32642, 32643, 32767, 65535, 65536])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_picked_bin(nbins, shift):
+    g = torch.Generator().manual_seed(nbins)
+    hist = torch.randint(0, 5, (nbins,), generator=g, dtype=torch.int32) * (torch.rand(nbins, generator=g) < 0.3).int()
+    hist[0] += 1
+    from_top = hist.flip(0).long().cumsum(0)
+    total = int(from_top[-1])
+    dev = torch.zeros(nbins + 1, dtype=torch.int32, device=DEV)[shift : shift + nbins].copy_(hist)
+    for k in {1, total // 3 + 1, total, total + 1}:
+        out = torch.zeros(4, dtype=torch.int64, device=DEV)
+        K._ext().radix_pick(dev, nbins, k, None, 0, out, None, None)
+        i = int(torch.searchsorted(from_top, k))
+        want = [nbins - 1 - i, k - int(from_top[i - 1] if i else 0), total, 0] if k <= total else [0, 0, total, 1]
+        assert out.tolist() == want, k
