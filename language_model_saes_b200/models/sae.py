@@ -208,9 +208,9 @@ class SparseAutoEncoder(SparseDictionary):
 
             partial = sparse_decode(feature_acts, self.W_D)
         elif self._sparse_inference(feature_acts):
-            from ..ops.inference import plain_inference, sparse_decode
+            from ..ops.inference import decode_bias_supported, sparse_decode
 
-            if self.cfg.use_decoder_bias and self.tp_group is None and self.b_D.data_ptr() % 16 == 0 and plain_inference(feature_acts, self.b_D):
+            if self.cfg.use_decoder_bias and self.tp_group is None and decode_bias_supported(feature_acts, self.W_D, self.b_D):
                 return self.hook_reconstructed(sparse_decode(feature_acts, self.W_D, self.b_D))
             partial = sparse_decode(feature_acts, self.W_D)
         else:

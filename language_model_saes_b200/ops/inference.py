@@ -110,6 +110,11 @@ def sparse_decode_supported(acts: torch.Tensor, W: torch.Tensor) -> bool:
             and F < 2**31 - 64 and 0 < B < 2**31 - 64)  # fmt: skip
 
 
+def decode_bias_supported(acts: torch.Tensor, W: torch.Tensor, bias: torch.Tensor) -> bool:
+    """Whether ``sparse_decode`` can add this bias: one aligned value per column of ``W``, nothing else wanted of the sum."""
+    return plain_inference(acts, bias) and bias.shape == W.shape[1:] and bias.is_contiguous() and bias.data_ptr() % 16 == 0
+
+
 def most_gathered(F: int) -> int:
     """Non-zeros of a row up to which gathering beats the product of the rows that are left over: 4096 tokens x 2048 x 768, 443 us as a
     product, 222 us gathered at 12 % and 805 us at 50 % (4096 x 8192 x 768: 1684 us against 793 us at 12 %)."""

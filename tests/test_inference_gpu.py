@@ -77,9 +77,41 @@ def test_decoder(B, F, d, rows):
     assert ((out.double() - want).abs()[ok] <= bound.expand_as(want)[ok]).all()
 
 
-def _sae(act):
+@pytest.mark.parametrize("rows", ["sparse", "some dense", "all dense", "inf weight"])
+@pytest.mark.parametrize("B,F,d", [(130, 1000, 64), (3, 4100, 1028), (129, 512, 256)])
+def test_decoder_with_its_bias_is_the_sum_of_both(B, F, d, rows):
+    """One rounding of the finished sum, by whichever way a row is made: the same as adding the bias afterwards."""
+    g = torch.Generator().manual_seed(F)
+    a, W, b = torch.randn(B, F, generator=g), torch.randn(F, d, generator=g), torch.randn(d, generator=g)
+    if rows != "all dense":
+        a[1 if rows == "some dense" else 0 :] *= torch.rand(B - (rows == "some dense"), F, generator=g) < 20 / F
+    if rows == "inf weight":
+        W[F // 2, 1] = float("inf")
+    b[3] = float("inf")
+    a, W, b = a.to(DEV), W.to(DEV), b.to(DEV)
+    out, want = I.sparse_decode(a, W, b), I.sparse_decode(a, W) + b
+    assert torch.equal(out.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0))
+
+
+@pytest.mark.parametrize("bias", ["a column", "unaligned", "one value", "as it is"])
+def test_decode_takes_a_bias_of_any_layout(bias):
+    sae = _sae("topk", 64)
+    values = torch.randn(64, device=DEV)
+    if bias == "a column":
+        sae.b_D = torch.nn.Parameter(values[:, None].repeat(1, 3)[:, 1])
+    elif bias == "unaligned":
+        sae.b_D = torch.nn.Parameter(torch.cat([values[:1], values])[1:])
+    else:
+        sae.b_D = torch.nn.Parameter(values[:1].clone() if bias == "one value" else values)
+    with torch.no_grad():
+        acts = sae.encode(torch.randn(2048, 64, device=DEV))
+        assert sae._sparse_inference(acts)
+        assert torch.equal(sae.decode(acts), I.sparse_decode(acts, sae.W_D) + sae.b_D)
+
+
+def _sae(act, expansion=8):
     torch.manual_seed(0)
-    cfg = SAEConfig(hook_point_in="h", hook_point_out="h", d_model=64, expansion_factor=8, act_fn=act, top_k=10, device=DEV, dtype=torch.float32)
+    cfg = SAEConfig(hook_point_in="h", hook_point_out="h", d_model=64, expansion_factor=expansion, act_fn=act, top_k=10, device=DEV, dtype=torch.float32)
     sae = SparseAutoEncoder(cfg)
     sae.init_parameters(encoder_uniform_bound=0.2, decoder_uniform_bound=0.2, init_log_jumprelu_threshold_value=-1.0)
     return sae
