@@ -192,7 +192,7 @@ radix_pick_kernel(const unsigned* __restrict__ hist, int nbins, long long k, con
   // thread i owns bins [hi - per, hi) counted from the top, so that a scan over threads walks downwards
   const int hi = nbins - (int)threadIdx.x * per;
   long long mine = 0;
-  // (whole vectors at their addresses: a share of them from a number of bins that is one of them)
+  // (vectors: a share of whole ones, counted down from a number of bins that is one too)
   if (per % 4 == 0 && nbins % 4 == 0 && hi >= per && (reinterpret_cast<uintptr_t>(hist) & 15) == 0) {  // (all loads before the first is used: one after the other they took 19 us)
     const uint4* h4 = reinterpret_cast<const uint4*>(hist + hi - per);
 #pragma unroll 8

@@ -98,7 +98,7 @@ def test_decode_takes_a_bias_of_any_layout(bias):
     sae = _sae("topk", 64)
     values = torch.randn(64, device=DEV)
     if bias == "a column":
-        sae.b_D = torch.nn.Parameter(values[:, None].repeat(1, 3)[:, 1])
+        sae.b_D = torch.nn.Parameter(values[:, None].repeat(1, 3)[:, 0])
     elif bias == "unaligned":
         sae.b_D = torch.nn.Parameter(torch.cat([values[:1], values])[1:])
     else:
