@@ -176,3 +176,19 @@ def test_encode_takes_the_estimating_product(form, monkeypatch):
     assert (~same).any(-1).float().mean() < 0.01
     bound = 512 * 2.0**-24 * (x.double().abs() @ sae.W_E.double().abs() + sae.b_E.double().abs())
     assert ((acts.double() - want).abs() <= bound + 1e-12)[same].all()
+
+
+def test_decoder_of_a_dictionary_longer_than_the_batch():
+    """More CTAs look through W than rows are gathered: what they find in any part of it counts."""
+    B, F, d = 5, 4096, 4096
+    a = torch.zeros(B, F, device=DEV)
+    a[:, ::200] = 1.0
+    W = torch.randn(F, d, device=DEV)
+    want = I.sparse_decode(a, W)
+    assert torch.allclose(want, W[::200].sum(0).expand(B, d), atol=1e-4)
+    for row in (1, F // 2, F - 1):  # (features that are never active: 0 * inf)
+        V = W.clone()
+        V[row, d - 1 - row % 7] = float("inf")
+        out = I.sparse_decode(a, V)
+        assert bool(out[:, d - 1 - row % 7].isnan().all()) and int(out.isnan().sum()) == B
+        assert torch.allclose(out.nan_to_num(nan=0.0), want.masked_fill(out.isnan(), 0.0), atol=1e-4)
