@@ -75,9 +75,7 @@ def causal_attention_bwd(q16, k16, v16, do16, lse, delta, scale: float, dtype: t
     """``(dq, dk, dv)`` in ``dtype`` (fp32, or bf16: fp32 sums rounded once) from contiguous bf16 ``[b, s, h, *]`` tensors and the row
     statistics ``lse``, ``delta [b, h, s]`` (``delta`` the dot products of output and output gradient). Two kernels."""
     dq, dk, dv = (torch.empty(t.shape, dtype=dtype, device=t.device) for t in (q16, k16, v16))
-    ext = K._ext()
-    ext.launches += 1  # two kernels in one entry point
-    ext.attn_bwd(q16, k16, v16, do16, lse, delta, dq, dk, dv, float(scale), K.status_buffer(q16.device))
+    K._ext().attn_bwd(q16, k16, v16, do16, lse, delta, dq, dk, dv, float(scale), K.status_buffer(q16.device))
     return dq, dk, dv
 
 

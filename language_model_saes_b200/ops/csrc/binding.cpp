@@ -1737,6 +1737,7 @@ bool bounds_checked_build() {
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("kernel_launches", [] { return lmsae::kernel_launches.load(); });
   m.def("bounds_report", &bounds_report);
   m.def("bounds_checked_build", &bounds_checked_build);
   m.def("comm_push_candidates", &comm_push_candidates);

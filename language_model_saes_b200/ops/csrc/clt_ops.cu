@@ -146,7 +146,7 @@ int clt_dact_launch(const CltTable& tab, const int* idx, int B, int K, int L, in
   if (e != cudaSuccess) return (int)e;
   if (B <= 0) return 0;
   const int blocks = B < 148 * 8 ? B : 148 * 8;
-  clt_dact_kernel<<<blocks, CLT_DACT_THREADS, smem, stream>>>(tab, idx, B, K, L, F, d, dy, dval);
+  launch_plain(clt_dact_kernel, blocks, CLT_DACT_THREADS, smem, stream, tab, idx, B, K, L, F, d, dy, dval);
   return (int)cudaGetLastError();
 }
 
@@ -191,7 +191,7 @@ int clt_wgrad_launch(const CltGradTable& tab, const int* offsets, const int* ent
   const long long n_codes = (long long)L * F;
   if (n_codes <= 0 || n_codes > 2147483647LL) return (int)cudaErrorInvalidValue;
   const int blocks = (int)(n_codes < 148LL * 16 ? n_codes : 148LL * 16);
-  clt_wgrad_kernel<<<blocks, CLT_WG_THREADS, 0, stream>>>(tab, offsets, entries, act, B, K, L, F, d, dy);
+  launch_plain(clt_wgrad_kernel, blocks, CLT_WG_THREADS, 0, stream, tab, offsets, entries, act, B, K, L, F, d, dy);
   return (int)cudaGetLastError();
 }
 

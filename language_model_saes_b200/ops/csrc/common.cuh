@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "launch_count.h"
 
 namespace lmsae {
 
@@ -79,7 +80,7 @@ __device__ __forceinline__ long long lmsae_checked_index(long long i, long long 
 // while others still run crowd on the SMs that are free first, which costs more than the earlier start gives (116, 740 and 359 us).
 // What is launched so begins with pdl_wait(), in every thread, before it reads or writes anything in global memory and before it
 // allocates TMEM. The wait of one covers all earlier ones, since none ends before its own wait is over. A kernel without it is
-// launched with <<<>>>.
+// launched with launch_plain().
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -97,7 +98,13 @@ static inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, si
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  ++kernel_launches;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <class... P>
+static inline void launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, typename same_type<P>::type... args) {
+  ++kernel_launches;
+  kernel<<<grid, block, smem, stream>>>(args...);
 }
 
 // ---- small PTX wrappers ----------------------------------------------------------------------

@@ -668,6 +668,7 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
+  ++kernel_launches;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
 }
 

@@ -572,6 +572,7 @@ static cudaError_t launch_product(const void* kernel, const CUtensorMap& ta, con
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   void* args[3] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &p};
+  ++kernel_launches;
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 

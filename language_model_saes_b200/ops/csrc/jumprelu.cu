@@ -82,9 +82,9 @@ static int launch(const void* x, const void* log_theta, const void* dy, void* ou
   long long blocks = (n_vec + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (bwd) {
-    jumprelu_kernel<T, true><<<(int)blocks, 256, 0, stream>>>((const T*)x, (const T*)log_theta, (const T*)dy, (T*)out, dlog, n_vec, P, window);
+    launch_plain(jumprelu_kernel<T, true>, (int)blocks, 256, 0, stream, (const T*)x, (const T*)log_theta, (const T*)dy, (T*)out, dlog, n_vec, P, window);
   } else {
-    jumprelu_kernel<T, false><<<(int)blocks, 256, 0, stream>>>((const T*)x, (const T*)log_theta, nullptr, (T*)out, nullptr, n_vec, P, window);
+    launch_plain(jumprelu_kernel<T, false>, (int)blocks, 256, 0, stream, (const T*)x, (const T*)log_theta, nullptr, (T*)out, nullptr, n_vec, P, window);
   }
   return (int)cudaGetLastError();
 }

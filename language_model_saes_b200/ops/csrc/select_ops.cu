@@ -738,9 +738,9 @@ int threshold_mask_launch(int dtype, const void* x, const float* thr, long long 
   const long long rows = A * S;
   if (rows <= 0 || N <= 0) return 0;
   if (dtype == 0)
-    threshold_mask_kernel<float><<<148 * 8, 256, 0, stream>>>(static_cast<const float*>(x), thr, rows, S, N, static_cast<float*>(out));
+    launch_plain(threshold_mask_kernel<float>, 148 * 8, 256, 0, stream, static_cast<const float*>(x), thr, rows, S, N, static_cast<float*>(out));
   else
-    threshold_mask_kernel<__nv_bfloat16><<<148 * 8, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), thr, rows, S, N,
+    launch_plain(threshold_mask_kernel<__nv_bfloat16>, 148 * 8, 256, 0, stream, static_cast<const __nv_bfloat16*>(x), thr, rows, S, N,
                                                                      static_cast<__nv_bfloat16*>(out));
   return (int)cudaGetLastError();
 }
@@ -837,13 +837,13 @@ int gather_rows_cast_launch(int in_dtype, int out_dtype, const void* src, const 
   const int blocks = (int)(n < 148LL * 16 ? n : 148LL * 16);
   using bf = __nv_bfloat16;
   if (in_dtype == 0 && out_dtype == 0)
-    gather_rows_cast_kernel<float, float><<<blocks, 256, 0, stream>>>((const float*)src, keep, pos, n, d, (float*)out, out_rows);
+    launch_plain(gather_rows_cast_kernel<float, float>, blocks, 256, 0, stream, (const float*)src, keep, pos, n, d, (float*)out, out_rows);
   else if (in_dtype == 0 && out_dtype == 1)
-    gather_rows_cast_kernel<float, bf><<<blocks, 256, 0, stream>>>((const float*)src, keep, pos, n, d, (bf*)out, out_rows);
+    launch_plain(gather_rows_cast_kernel<float, bf>, blocks, 256, 0, stream, (const float*)src, keep, pos, n, d, (bf*)out, out_rows);
   else if (in_dtype == 1 && out_dtype == 0)
-    gather_rows_cast_kernel<bf, float><<<blocks, 256, 0, stream>>>((const bf*)src, keep, pos, n, d, (float*)out, out_rows);
+    launch_plain(gather_rows_cast_kernel<bf, float>, blocks, 256, 0, stream, (const bf*)src, keep, pos, n, d, (float*)out, out_rows);
   else if (in_dtype == 1 && out_dtype == 1)
-    gather_rows_cast_kernel<bf, bf><<<blocks, 256, 0, stream>>>((const bf*)src, keep, pos, n, d, (bf*)out, out_rows);
+    launch_plain(gather_rows_cast_kernel<bf, bf>, blocks, 256, 0, stream, (const bf*)src, keep, pos, n, d, (bf*)out, out_rows);
   else
     return (int)cudaErrorInvalidValue;
   return (int)cudaGetLastError();

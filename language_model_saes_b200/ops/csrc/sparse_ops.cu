@@ -893,16 +893,16 @@ int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream) {
   if (p.dact_mode != 0) return (int)cudaErrorInvalidValue;  // the kernel below takes the code gradients as an input
   if (doD && doE) {
     if (p.ctas_per_sm >= 1 && p.ctas_per_sm <= 2)
-      sparse_grad_adam_kernel<2, 2, 3><<<blocks, GA_THREADS, 0, stream>>>(p);
+      launch_plain(sparse_grad_adam_kernel<2, 2, 3>, blocks, GA_THREADS, 0, stream, p);
     else
-      sparse_grad_adam_kernel<1, 4, 3><<<blocks, GA_THREADS, 0, stream>>>(p);
+      launch_plain(sparse_grad_adam_kernel<1, 4, 3>, blocks, GA_THREADS, 0, stream, p);
   } else {
     // one-sided: fewer registers; the encoder side fits five CTAs (rows in flight) per SM, the decoder side (row norms,
     // norm penalty) four without spilling
     const int per_sm = doD ? 4 : 5;
     if (p.ctas_per_sm < 1 || p.ctas_per_sm > per_sm) blocks = rows < 148 * per_sm ? rows : 148 * per_sm;
-    if (doD) sparse_grad_adam_kernel<1, 4, 1><<<blocks, GA_THREADS, 0, stream>>>(p);
-    else sparse_grad_adam_kernel<1, 5, 2><<<blocks, GA_THREADS, 0, stream>>>(p);
+    if (doD) launch_plain(sparse_grad_adam_kernel<1, 4, 1>, blocks, GA_THREADS, 0, stream, p);
+    else launch_plain(sparse_grad_adam_kernel<1, 5, 2>, blocks, GA_THREADS, 0, stream, p);
   }
   return (int)cudaGetLastError();
 }
@@ -1213,7 +1213,7 @@ row_norm_shadow_kernel(const float* __restrict__ W, int F, int d, float* __restr
 
 int row_norm_shadow_launch(const float* W, int F, int d, float* norm, __nv_bfloat16* shadow, cudaStream_t stream) {
   int blocks = F < 148 * 16 ? F : 148 * 16;
-  row_norm_shadow_kernel<<<blocks, 256, 0, stream>>>(W, F, d, norm, shadow);
+  launch_plain(row_norm_shadow_kernel, blocks, 256, 0, stream, W, F, d, norm, shadow);
   return (int)cudaGetLastError();
 }
 

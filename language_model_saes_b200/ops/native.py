@@ -141,5 +141,10 @@ def load(required: bool | None = None) -> ModuleType | None:
             return None
 
 
+def loaded() -> ModuleType | None:
+    """The extension module if something has loaded it."""
+    return _module
+
+
 def available() -> bool:
     return load(required=False) is not None

@@ -44,50 +44,20 @@ _STATUS_NAMES = {
 }
 
 
-def _csc_kernels(entries: int, F: int) -> int:
-    """Launches of the counting sort (csc_build_launch): one for few entries, else four or, for long dictionaries, six."""
-    return 1 if entries <= 45056 and F <= 148 * 4096 else 4 if F <= 1 << 17 else 6
-
-
-class _Counting:
-    """Proxy of the extension module that counts the device kernels each entry point launches."""
-
-    KERNELS_PER_CALL = {
-        "csc_build": lambda idx, F, *_: _csc_kernels(idx.numel(), F),
-        "exclusive_scan": 3,
-        "topk_step": lambda x, label, k, route, mode, splits, units, enc, *_: 5 + _csc_kernels(x.shape[0] * k, enc[3].shape[0]),
-        "topk_encode": 7,
-    }
-
-    def __init__(self, mod):
-        self._mod = mod
-        self.launches = 0
-
-    def __getattr__(self, name):
-        fn = getattr(self._mod, name)
-        n = self.KERNELS_PER_CALL.get(name, 1)
-
-        def call(*args, **kwargs):
-            self.launches += n(*args, **kwargs) if callable(n) else n
-            return fn(*args, **kwargs)
-
-        self.__dict__[name] = call
-        return call
-
-
-_counting: _Counting | None = None
+_module = None
 
 
 def _ext():
-    global _counting
-    if _counting is None:
-        _counting = _Counting(native.load(required=True))
-    return _counting
+    global _module
+    if _module is None:
+        _module = native.load(required=True)
+    return _module
 
 
 def kernel_launch_count() -> int:
-    """Number of kernels of this package launched so far in this process."""
-    return _counting.launches if _counting is not None else 0
+    """Number of kernels of this package launched so far in this process (a captured graph's count once, when they are captured)."""
+    ext = native.loaded()
+    return ext.kernel_launches() if ext is not None else 0
 
 
 def status_buffer(device: torch.device) -> torch.Tensor:

@@ -28,8 +28,9 @@ def test_every_kernel_that_is_launched_early_waits_first():
         text = path.read_text()
         bodies = _bodies(text)
         names = set(re.findall(r"\blaunch\(\s*(\w+)", text)) - {"const"}  # (a function of that name)
-        if "ProgrammaticStreamSerialization" in text:  # clusters, with a configuration of their own
-            names |= {"enc_gemm_kernel", "fp32_gemm_kernel"} & set(bodies)
+        if "ProgrammaticStreamSerialization" in text:  # clusters, with a configuration of their own: every kernel of the file that goes nowhere else
+            plain = set(re.findall(r"\blaunch_plain\(\s*(\w+)", text))
+            names |= {n for n in bodies if n not in plain}
         for name in list(names):
             if name not in bodies:  # a variable: every kernel that it may stand for
                 names.remove(name)
@@ -40,3 +41,12 @@ def test_every_kernel_that_is_launched_early_waits_first():
             assert bodies[name] == "pdl_wait()", (path.name, name, bodies[name])
         launched += len(names)
     assert launched >= 40  # (the sources were read as they are meant to be)
+
+
+def test_every_launch_is_counted():
+    """Kernels are launched by the two helpers, which count; what launches by itself says so in the line before."""
+    for path in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp"))):
+        lines = path.read_text().split("\n")
+        for before, line in zip([""] + lines, lines):
+            if re.search(r"<<<|cudaLaunch(Cooperative)?Kernel(Ex|ExC)?\(|cuLaunchKernel", line):
+                assert "++kernel_launches;" in before, (path.name, line)
