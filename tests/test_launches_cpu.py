@@ -28,9 +28,8 @@ def test_every_kernel_that_is_launched_early_waits_first():
         text = path.read_text()
         bodies = _bodies(text)
         names = set(re.findall(r"\blaunch\(\s*(\w+)", text)) - {"const"}  # (a function of that name)
-        if "ProgrammaticStreamSerialization" in text:  # clusters, with a configuration of their own: every kernel of the file that goes nowhere else
-            plain = set(re.findall(r"\blaunch_plain\(\s*(\w+)", text))
-            names |= {n for n in bodies if n not in plain}
+        if "ProgrammaticStreamSerialization" in text:  # clusters, with a configuration of their own
+            names |= {"enc_gemm_kernel", "fp32_gemm_kernel"} & set(bodies)
         for name in list(names):
             if name not in bodies:  # a variable: every kernel that it may stand for
                 names.remove(name)
@@ -41,6 +40,15 @@ def test_every_kernel_that_is_launched_early_waits_first():
             assert bodies[name] == "pdl_wait()", (path.name, name, bodies[name])
         launched += len(names)
     assert launched >= 40  # (the sources were read as they are meant to be)
+
+
+def test_kernels_of_files_with_a_launch_of_their_own_wait_first():
+    """Where a file sets the attribute itself, every kernel of it that is not launched plainly is taken to be launched early."""
+    for path in sorted(CSRC.glob("*.cu")):
+        text = path.read_text()
+        if "ProgrammaticStreamSerialization" in text:
+            for name, first in _bodies(text).items():
+                assert first == "pdl_wait()" or re.search(rf"\blaunch_plain\(\s*{name}\b", text), (path.name, name)
 
 
 def test_every_launch_is_counted():
