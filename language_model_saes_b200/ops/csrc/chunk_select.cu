@@ -346,7 +346,7 @@ chunk_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
   if (row >= B) return;
   const RowList to = {idx + (size_t)row * cap, val + (size_t)row * cap, cap};
   int n = 0;
-  for_groups(x + (size_t)row * N, maxima + (size_t)row * ld_maxima, N, true, 0.9999f, 0, (N + 31) / 32, s_list[warp], [&](int c, const uint4& raw, int have) {
+  auto visit = [&](int c, const uint4& raw, int have) {
     float t[8];
     if (have > 0) {  // (eight columns: N % 8 == 0)
       const float4 a = __ldg(reinterpret_cast<const float4*>(col_thr + c)), b = __ldg(reinterpret_cast<const float4*>(col_thr + c) + 1);
@@ -370,7 +370,11 @@ chunk_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
         to.val[slot] = __uint_as_float(raw_value(raw, j) << 16);
       }
     }
-  });
+  };
+  // (a row with more values than places is looked at up to where that shows)
+  const int groups = (N + 31) / 32;
+  for (int g0 = 0; g0 < groups && n <= cap; g0 += CS_SPAN)
+    for_groups(x + (size_t)row * N, maxima + (size_t)row * ld_maxima, N, true, 0.9999f, g0, min(groups, g0 + CS_SPAN), s_list[warp], visit);
   pad_row(to, n);
   if (lane == 0 && n > cap) atomicAdd(overflow, 1ULL);
 }

@@ -101,3 +101,25 @@ def test_lists_by_maxima_are_those_of_the_whole_matrix(B, heads, d, F, cap, shif
     for a, b in zip(*got):
         assert torch.equal(a, b)
     assert torch.equal(got[1][0][0, : min(cap, int((H[0].float() > t_min).sum()))], torch.nonzero(H[0].float() > t_min).flatten()[:cap].int())
+
+
+@pytest.mark.parametrize("share", [0.01, 0.05, 0.4])
+def test_rows_with_far_more_values_than_places_cost_no_more_by_maxima(share):
+    """A dictionary before its thresholds have closed: one warp looked at all of a row's groups, 455 us against 335 from the whole matrix at 0.4."""
+    B, F, cap, best = 4096, 98304, 256, [1e9, 1e9]
+    x = torch.rand(B, F, device=DEV, generator=torch.Generator(device=DEV).manual_seed(0)).to(torch.bfloat16)
+    thr = torch.full((F,), 1 - share, device=DEV)
+    maxima = (x.view(B, F // 32, 32).amax(2).float() / (1 - share)).contiguous()
+    idx, val = (torch.empty(B, cap, dtype=t, device=DEV) for t in (torch.int32, torch.float32))
+    for _ in range(6):
+        for i, m in enumerate((maxima, None)):
+            over = torch.zeros((), dtype=torch.int64, device=DEV)
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(100000)
+            start.record()
+            assert K._ext().column_lists(x, thr, idx, val, over, m)
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+            assert int(over) == B
+    assert best[0] < best[1], best
