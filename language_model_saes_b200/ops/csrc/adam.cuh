@@ -30,4 +30,14 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                : "memory");
 }
 
+// Whether a feature has more than n entries, the same in every thread of the CTA (a barrier).
+__device__ __forceinline__ bool any_longer_list(const GradAdamParams& p, int n) {
+  bool any = false;
+  for (int i = threadIdx.x, n_heavy = p.heavy[0]; i < n_heavy; i += blockDim.x) {
+    const int f = p.heavy[1 + i] - p.heavy_base;
+    any |= f >= 0 && f < p.F && p.offsets[f + 1] - p.offsets[f] > n;
+  }
+  return __syncthreads_or(any) != 0;
+}
+
 }  // namespace lmsae

@@ -272,7 +272,8 @@ grad_adam_rows_kernel(const GradAdamParams p) {
   __syncthreads();
 
   // a kernel of this step that gave up on a bounded wait leaves stale inputs: parameters and moments stay as they are
-  const bool skip = p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0;
+  const bool other = p.longest < 0 && !any_longer_list(p, -p.longest);  // (the other kernel's launch)
+  const bool skip = other || (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0);
   const bool doD = p.WD != nullptr, doE = p.WE != nullptr;
   const float gmul = p.grad_mul != nullptr ? *p.grad_mul : 1.0f;
   const AdamConst h = {p.h.beta1, p.h.beta2, 1.0f - p.h.beta1, 1.0f - p.h.beta2, 1.0f / p.h.bias_correction2_sqrt,
@@ -554,6 +555,13 @@ grad_adam_rows_kernel(const GradAdamParams p) {
 
 namespace {
 
+// A list costs one CTA 40 ns an entry in one pass with two warps a row (above 256 columns) and 26 here, and the others may have ended long before: where
+// there is a longer one than this, which the kernels find out, both sides take this kernel. 512 columns, features of popularity 1 / (5 + rank), us in one pass ->
+// here: 4096 rows, 8192 tokens x 64: 475 -> 372; 8192, 4096 x 64: 348 -> 236; 4096, 4096 x 32: 168 -> 114; 4096, 2048 x 64: 132 -> 106; 512, 2048 x 16: 69 ->
+// 54; of equal popularity 4096, 4096 x 64: 181, 242. Batches of fewer tokens have no such list (4096, 1024 x 64: 87, 89 before there was the one pass) and
+// need no second launch, which costs 4 us with the look at the lists.
+constexpr int kOnePassList = 1024;
+
 template <int W, int NCH>
 cudaError_t launch_rows(GradAdamParams p, cudaStream_t stream) {
   constexpr int T = 32 * W;
@@ -588,12 +596,18 @@ bool grad_adam_rows_supported(const GradAdamParams& p) {
          p.dxhat_aux == nullptr && align % 16 == 0;
 }
 
-int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream) {
+int grad_adam_rows_launch(GradAdamParams p, cudaStream_t stream) {
   if (!grad_adam_rows_supported(p) || (p.dact_mode != 0 && (p.WD == nullptr || p.dact_out == nullptr))) return (int)cudaErrorInvalidValue;
   if (p.f_end <= p.f_begin) return 0;
-  if (grad_adam_both_supported(p)) return grad_adam_both_launch(p, stream);
   const int d = p.d;
   cudaError_t e;
+  if (grad_adam_both_supported(p)) {
+    const bool either = d > 256 && p.heavy != nullptr && p.n_rows > kOnePassList;
+    p.longest = either ? kOnePassList : 0;
+    const int err = grad_adam_both_launch(p, stream);
+    if (err != 0 || !either) return err;
+    p.longest = -kOnePassList;
+  }
   if (d <= 1024) {
     const int nch = (d + 127) / 128;
     e = nch <= 1 ? launch_rows<1, 1>(p, stream) : nch <= 2 ? launch_rows<1, 2>(p, stream) : nch <= 4 ? launch_rows<1, 4>(p, stream)

@@ -11,7 +11,8 @@
 //                      eight sums instead of forty), across the group's warps through shared memory behind one barrier
 //   ahead of the row   the entries and codes of the next row, the range of the one after it and its draw from the row counter are requested
 //                      while this one's gathers are on their way
-//   long lists         as in grad_adam.cu, in pieces of eight entries, since the lists are barely longer than kHeavyRow here
+//   long lists         as in grad_adam.cu, the same share to every group, a piece's entries and codes requested while the ones before it are gathered (in pieces
+//                      of eight, each behind the one before it: 4096 rows of 512, 4096 x 64 codes 187 us, 175 here; skewed popularity, 4096 x 32: 186, 168)
 // Bound by instructions and their latency (0.42 issued per cycle and scheduler, a thousand per row and warp with an entry or two), not by memory.
 // grad_adam.cu -> this, us; up to 128 columns NCH 1, Q 8, above NCH 2, Q 4 (in brackets the other of the two):
 //   256 x 64, 512 tokens x 8 codes        24.5 -> 15.6 (18.5)     512 x 128, 2048 x 16     41.0 -> 28.6 (36.9)
@@ -31,7 +32,6 @@ LMSAE_DEFINE_BOUNDS_FETCH(bounds_fetch_grad_adam_both)
 namespace {
 
 constexpr int GB_THREADS = 512;  // (128 registers: nothing is spilled)
-constexpr int GB_PIECE = 8;  // entries of a long list that a group takes at a time
 
 struct BothCtx {
   int gid, wg, lane, tid, W;  // group, warp within it, lane, thread within it, warps of a group
@@ -198,7 +198,8 @@ grad_adam_both_kernel(const GradAdamParams p, const int W) {
   __syncthreads();
 
   // a kernel of this step that gave up on a bounded wait leaves stale inputs: parameters and moments stay as they are
-  const bool skip = p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0;
+  const bool other = p.longest > 0 && any_longer_list(p, p.longest);  // (the other kernel's launch)
+  const bool skip = other || (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0);
   const float gmul = p.grad_mul != nullptr ? *p.grad_mul : 1.0f;
   const AdamConst h = {p.h.beta1, p.h.beta2, 1.0f - p.h.beta1, 1.0f - p.h.beta2, 1.0f / p.h.bias_correction2_sqrt,
                        p.h.lr / p.h.bias_correction1, p.h.eps};
@@ -304,6 +305,12 @@ grad_adam_both_kernel(const GradAdamParams p, const int W) {
       const int e0 = p.offsets[f], e1 = p.offsets[f + 1];
       const int xr = p.extra_row != nullptr ? p.extra_row[f] : -1;
       if (threadIdx.x == 0) issue(0, f);
+      // the same share to every group, in pieces of at most 32 entries; a piece's entries are requested two pieces ahead of it, its codes one
+      const int n = e1 - e0, rounds = (n + G * 32 - 1) / (G * 32), piece = (n + G * rounds - 1) / (G * rounds), step = G * piece;
+      auto left = [&](int i) { return max(0, min(piece, n - i)); };
+      int i0 = c.gid * piece;
+      Entry m = entry_of(p, entry_at(p, e0 + i0, left(i0), c.lane), left(i0), c.lane);
+      int at_n = entry_at(p, e0 + i0 + step, left(i0 + step), c.lane);
       float gD[NCH][4], gE[NCH][4], coef = 0.0f;
       uint2 w[NCH];
       init_grad(p.extra_gD, c.gid == 0 ? xr : -1, gD);
@@ -314,9 +321,11 @@ grad_adam_both_kernel(const GradAdamParams p, const int W) {
       parity ^= 1;
       outstanding = false;
       rounded_row(stages, w);
-      for (int e = e0 + c.gid * GB_PIECE; e < e1; e += G * GB_PIECE) {
-        const int n = min(GB_PIECE, e1 - e);
-        gather_both<NCH, Q>(p, c, entry_of(p, entry_at(p, e, n, c.lane), n, c.lane), n, w, gD, gE, coef, dot_buf);
+      for (; i0 < n; i0 += step) {
+        const Entry next = entry_of(p, at_n, left(i0 + step), c.lane);
+        at_n = entry_at(p, e0 + i0 + 2 * step, left(i0 + 2 * step), c.lane);
+        gather_both<NCH, Q>(p, c, m, left(i0), w, gD, gE, coef, dot_buf);
+        m = next;
       }
       if (c.tid == 0) bias_part[c.gid] = coef;
       if (c.gid != 0) {

@@ -191,6 +191,7 @@ struct GradAdamParams {
   // [f / layer_rows * n_rows, + n_rows) of x; with layers_share_groups the entries of group f % layer_rows, else of group f.
   int layer_rows;
   int layers_share_groups;
+  int longest;         // set by the launch: 0, or n > 0: nothing is done where a list has more than n entries, -n: unless one has
   int ctas_per_sm;     // 0 = fill the GPU (4 per SM); 1..4 = leave registers free for a concurrently running kernel
   const int* status;   // kernels' status word: a recorded error turns the update into a no-op (nullptr: not checked)
   // Dense gradient rows for a subset of the features, added to the rows rebuilt from the entry lists: feature f takes
@@ -238,7 +239,7 @@ int auxk_loss_grad_launch(const float* xhat, const float* aux_rec, const __nv_bf
                           float* aux_sum, cudaStream_t stream);
 int sparse_grad_adam_launch(const GradAdamParams& p, cudaStream_t stream);
 bool grad_adam_rows_supported(const GradAdamParams& p);
-int grad_adam_rows_launch(const GradAdamParams& p, cudaStream_t stream);
+int grad_adam_rows_launch(GradAdamParams p, cudaStream_t stream);
 bool grad_adam_both_supported(const GradAdamParams& p);
 int grad_adam_both_launch(const GradAdamParams& p, cudaStream_t stream);
 int colsum_bf16_launch(const __nv_bfloat16* a, int rows, int d, float* out, cudaStream_t stream);

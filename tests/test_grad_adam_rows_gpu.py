@@ -195,3 +195,62 @@ def test_long_lists_are_cut_evenly(d):
         atol = 0.1 * 2**-24 * 1300 * 1300**0.5 * scale + 1e-6
         assert torch.allclose(gpu[n].cpu(), cpu[n], atol=atol, rtol=1e-4), (n, float((gpu[n].cpu() - cpu[n]).abs().max()))
     assert torch.allclose(gpu["mb"].cpu(), cpu["mb"], atol=0.1 * 2**-24 * 1300 * (1300 * d) ** 0.5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("d", [4, 64, 128, 132, 256, 260, 512])
+@pytest.mark.parametrize("B", [1000, 1024, 1025])
+def test_long_lists_in_one_pass(d, B):
+    """Whole pieces of 32 for each of 8, 15 and 16 groups and one entry more or less, and a list of every token: the longest that two warps a row take in
+    one pass, and the first that they leave to the other kernel."""
+    g = torch.Generator().manual_seed(d)
+    lengths = [65, 127, 255, 256, 257, 479, 480, 481, 511, 512, 513, 769, B]
+    F, idx = 3 * len(lengths), torch.full((B, len(lengths)), -1, dtype=torch.int32)
+    for i, n in enumerate(lengths):
+        idx[torch.randperm(B, generator=g)[:n], i] = 3 * i
+    idx[5, idx[5] < 0] = 1  # (a short list)
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    cpu = dict(idx=idx, act=r(*idx.shape), dact=torch.zeros(idx.shape), x=r(B, d).to(torch.bfloat16), dx=r(B, d).to(torch.bfloat16), n=torch.zeros(F))
+    for s in "DE":
+        cpu |= {"W" + s: r(F, d), "S" + s: torch.zeros(F, d, dtype=torch.bfloat16), "m" + s: r(F, d) * 0.01, "v" + s: torch.rand(F, d, generator=g) + 1}
+    cpu |= {"b": r(F), "mb": torch.zeros(F), "vb": torch.ones(F)}
+    gpu = {n: t.clone().to(DEV) for n, t in cpu.items()}
+    for t in (cpu, gpu):
+        groups = K.FeatureGroups(F, idx.numel(), t["idx"].device).build(t["idx"])
+        K.sparse_grad_adam(groups, t["act"], t["dact"], t["x"], t["dx"], t["WD"], t["mD"], t["vD"], t["SD"], t["WE"], t["mE"], t["vE"], t["SE"], t["b"], t["mb"],
+                           t["vb"], t["n"], None, None, 1e-3, 0.9, 0.999, 1e-8, 1, True, dact_mode=1)  # fmt: skip
+    K.check_status(torch.device(DEV))
+    assert int(groups.heavy[0]) == len(lengths) and groups.sched.tolist() == [0, 0]
+    # code gradients: d products of order one, added up in another order. Encoder moments: 0.1 of a sum of up to B products of order sqrt(d), each
+    # addition rounding a partial sum of about sqrt(B d); decoder moments the same with d = 1.
+    assert torch.allclose(gpu["dact"].cpu(), cpu["dact"], atol=2**-24 * d * 4, rtol=1e-4)
+    for n, scale in (("mD", 1.0), ("mE", d**0.5), ("mb", d**0.5)):
+        atol = 0.1 * 2**-24 * B * B**0.5 * scale + 1e-6
+        assert torch.allclose(gpu[n].cpu(), cpu[n], atol=atol, rtol=1e-4), (n, float((gpu[n].cpu() - cpu[n]).abs().max()))
+    assert torch.equal(gpu["SD"].float(), gpu["WD"].to(torch.bfloat16).float()) and torch.equal(gpu["SE"].float(), gpu["WE"].to(torch.bfloat16).float())
+    assert torch.allclose(gpu["n"], gpu["WD"].norm(dim=1), rtol=1e-5)
+
+
+@pytest.mark.parametrize("d", [128, 512])
+def test_popular_features_cost_no_more_than_a_pass_per_side(d):
+    """Popular features beside rare ones take no longer than where both sides are one after the other (which a gradient norm asks for). One CTA had the
+    longest list to itself for 1.7 times as long at 512."""
+    F, B, k, g = 8 * d, 4096, 32, torch.Generator(device=DEV).manual_seed(d)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    idx = torch.multinomial((1 / (torch.arange(F, device=DEV) + 5.0)).repeat(B, 1), k, generator=g).int()
+    act, x, dx = r(B, k).abs(), r(B, d).to(torch.bfloat16), r(B, d).to(torch.bfloat16)
+    WD, WE, vD, vE = r(F, d), r(F, d), r(F, d).abs() + 1, r(F, d).abs() + 1
+    mD, mE, b, mb, vb, norm = (torch.zeros(*s, device=DEV) for s in ((F, d), (F, d), (F,), (F,), (F,), (F,)))
+    SD, SE, dact, norm_sq, best = WD.to(torch.bfloat16), WE.to(torch.bfloat16), torch.empty_like(act), torch.zeros(1, device=DEV), [1e9, 1e9]
+    groups = K.FeatureGroups(F, B * k, torch.device(DEV)).build(idx)
+    for _ in range(12):
+        for i in range(2):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(100000)  # (the launch is on its way when the first event is)
+            start.record()
+            K.sparse_grad_adam(groups, act, dact, x, dx, WD, mD, vD, SD, WE, mE, vE, SE, b, mb, vb, norm, None, norm_sq if i else None, 1e-4, 0.9, 0.999, 1e-8, 1,
+                               True, dact_mode=1)  # fmt: skip
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+    K.check_status(torch.device(DEV))
+    assert best[0] < 1.15 * best[1], best
