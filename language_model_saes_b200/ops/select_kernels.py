@@ -243,10 +243,10 @@ def threshold_rows_to_sparse(g: torch.Tensor, thr: torch.Tensor, col_div: torch.
     B = g.shape[0]
     nnz = torch.empty(B, dtype=torch.int32, device=g.device)
     if (maxima is not None and n_ties is not None and cap is not None and cap % 8 == 0 and cap > 0 and (tie_group is None or dist.get_world_size(tie_group) == 1)
-            and (overflow is None or overflow.dtype == torch.int64)):  # fmt: skip
+            and (overflow is None or (overflow.dtype == torch.int64 and overflow.numel() == 1))):  # fmt: skip
         idx = torch.empty(B, cap, dtype=torch.int32, device=g.device)
         val = torch.empty(B, cap, dtype=torch.float32, device=g.device)
-        ext.chunk_lists(g, maxima, thr, n_ties.reshape(-1).to(torch.int64), col_div, nnz, idx, val, overflow)
+        ext.chunk_lists(g, maxima, thr, n_ties.reshape(-1).to(g.device, torch.int64), col_div, nnz, idx, val, overflow)
         return idx, val
     quota = seg = None
     if n_ties is None:

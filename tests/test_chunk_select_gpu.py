@@ -171,3 +171,19 @@ def test_row_topk_as_a_matrix(M, N, k, data):
     if data == "ties" or gate is None:  # (which of equal values are taken is free)
         out, want = out.sort(1).values, want.sort(1).values
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("counter", [None, "one", "two", "32 bits"])
+@pytest.mark.parametrize("where", ["cpu", DEV])
+def test_lists_take_the_numbers_as_they_come(counter, where):
+    """The number of equal values from the host, counters of other shapes and types: as without maxima."""
+    x = torch.randint(0, 4, (40, 512), device=DEV, generator=torch.Generator(device=DEV).manual_seed(0)).to(torch.bfloat16)
+    maxima = x.float().view(40, 16, 32).amax(2).contiguous()
+    new = {"one": lambda: torch.zeros(1, dtype=torch.int64, device=DEV), "two": lambda: torch.zeros(2, dtype=torch.int64, device=DEV),
+           "32 bits": lambda: torch.zeros((), dtype=torch.int32, device=DEV), None: lambda: None}[counter]  # fmt: skip
+    thr, n_ties = torch.full((1,), 2.0, device=DEV), torch.tensor(1000, device=where)
+    outs = []
+    for m in (None, maxima):
+        over = new()
+        outs.append((*S.threshold_rows_to_sparse(x, thr, None, n_ties=n_ties, cap=136, overflow=over, maxima=m), *([over] if counter else [])))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
