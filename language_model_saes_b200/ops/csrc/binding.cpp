@@ -326,8 +326,10 @@ void topk_estimate(const Tensor& lo, const Tensor& h, const Tensor& x, const Ten
 // out = topk(relu((x W^T + bias) * norm)) / norm per row, dense fp32 [B, F], for x [B, K] and W [F, K]: one fp16 product proposes; rows that it leaves
 // too much of in question are proposed for again by three bf16 products where they are more than an eighth of all rows (that is decided on the device:
 // the kernels leave at once elsewhere), and what is still too much is multiplied in order. The parts of W take `workspace` bytes at most.
-void topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, int64_t workspace,
-                 const Tensor& out) {
+// Returns what it worked with: the lower ends (bf16, at the start of fp32 [B, F]), their maxima, norms and scales, the words; products_failed: as where a
+// product's wait ran out (every row is multiplied in order then).
+std::vector<Tensor> topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& norm, int64_t k, int64_t workspace,
+                                const Tensor& out, bool products_failed) {
   for (const Tensor* t : {&x, &W, &out}) { CHECK_T(*t, torch::kFloat32); }
   TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.size(1) == W.size(1) && out.dim() == 2 && out.size(0) == x.size(0) && out.size(1) == W.size(0), "x [B,K], W [F,K], out [B,F]");
   const int64_t B = x.size(0), F = W.size(0), K = x.size(1), kp = (K + 63) / 64 * 64;
@@ -351,6 +353,7 @@ void topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& 
   // zeroed: status [4], top [4] and the columns' widths, the rows that are wide, those that are left over
   const int64_t widths = 4 + (F + 1) / 2;
   const Tensor words = torch::zeros({4 + widths + 2 * (1 + B)}, i32);
+  if (products_failed) words.narrow(0, 0, 4).fill_(1);
   int* status = words.data_ptr<int>();
   uint32_t* top = reinterpret_cast<uint32_t*>(status + 4);
   int *wide = status + 4 + widths, *todo = wide + 1 + B;
@@ -383,6 +386,7 @@ void topk_encode(const Tensor& x, const Tensor& W, const c10::optional<Tensor>& 
   }
   check_cuda(lmsae::topk_wide_launch(lo, h.data_ptr<float>(), xp, Wp, xn, lost, top, (int)K, bias_p, norm_p, (int)B, (int)F, (int)k, status, wide, wide_limit, todo,
                                      out.data_ptr<float>(), stream), "topk_wide launch");
+  return {h, maxima, norms, words};
 }
 
 // out [B, d] = acts [B, F] @ W [F, d] (+ bias [d]), fp32. Rows of at most `most` non-zeros are gathered. todo: int32 [2 + B + tiles], zeroed; part: fp32
@@ -1789,7 +1793,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("row_select_fits", &row_select_fits);
   m.def("topk_dense", &topk_dense);
   m.def("topk_step", &topk_step);
-  m.def("topk_encode", &topk_encode);
+  m.def("topk_encode", &topk_encode, py::arg("x"), py::arg("W"), py::arg("bias"), py::arg("norm"), py::arg("k"), py::arg("workspace"), py::arg("out"),
+        py::arg("products_failed") = false);
   m.def("topk_estimate", &topk_estimate);
   m.def("fp32_gemm", &fp32_gemm);
   m.def("dense_decode", &dense_decode);

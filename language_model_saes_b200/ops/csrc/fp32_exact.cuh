@@ -30,7 +30,9 @@ __device__ __forceinline__ float fma_rn(float a, float b, float c) {
 //   192        what the two parts leave of an operand (2^-18 of it, twice) and the product of the two low parts (2^-18)
 //   128        the rounding of the ends themselves (a sum is at most about the product of the norms) and margin for what the hardware
 //              does not document (measured: 2 units in all)
-// The norms are rounded up by 5 % where they are made, which covers their own rounding and K 2^-24 << 1.
+// The norms are rounded up where they are made, by 5 % (split_bf16_kernel) or 0.1 % (half_rows_kernel), which covers their own rounding (K / 64
+// and less of these units). What is of second order is in the 2.1 K, of which the terms above take 2.08 K: parts may exceed their operands by 2^-9 each, 0.0042 K
+// of the accumulations, and K 2^-24 times the K roundings in order is less than 0.0005 K.
 __host__ __device__ __forceinline__ float estimate_rel(int K) { return ((float)K * 2.1f + 320.0f) * 5.9604645e-8f; }
 
 // The same for one fp16 part an operand, its row scaled so that the largest magnitude is in [2^14, 2^15) (half_rows_kernel): 2.1 K and 128 as
