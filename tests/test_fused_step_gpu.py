@@ -248,6 +248,25 @@ def test_one_native_call_is_the_same_step(B, k, expansion, route, weighted, gate
     K.check_status(torch.device("cuda"))
 
 
+@pytest.mark.parametrize("B,k,expansion,route", [(300, 9, 8, 0), (257, 32, 32, 1), (1024, 70, 40, 2), (300, 100, 64, 3), (300, 100, 8, 4), (300, 300, 8, 4)])
+def test_moments_of_one_native_call(B, k, expansion, route):
+    """The gradients' signs and sizes, which a parameter's first steps do not show. Where equal bf16 values compete for a row's last place (routes 3 and
+    4) at most one of its k codes differs: were it so in every row, a smallest one, sqrt(2 / k)
+    of a gradient; elsewhere only the order of fp32 sums."""
+    a = _model(k=k, expansion=expansion)
+    b = copy.deepcopy(a)
+    one, by_one = FusedTopKSAEStep(a), FusedTopKSAEStep(b)
+    assert K.topk_route(B, one.F, one.d, k, one.dec_norm) == route
+    x = _data(1, B, 256)[0]
+    by_one.start_phase_timing()
+    one.step(x, x, k, 1e-5)
+    by_one.step(x, x, k, 1e-5)
+    bound = (2.0 / k) ** 0.5 if route >= 3 else 1e-4
+    for name, moments in one.state.items():
+        for p, q in zip(moments, by_one.state[name]):
+            assert float(q.abs().max()) > 0 and float((p - q).norm() / q.norm()) <= 2 * bound, name  # (second moments: twice a gradient's share)
+
+
 def test_step_under_capture():
     """A captured step replays: what it needs comes from the graph's pool, and nothing in it waits for the host."""
     sae = _model()
