@@ -244,6 +244,7 @@ template <int W, int NCH>
 __global__ void __launch_bounds__(rows_threads<NCH>(), 1)
 grad_adam_rows_kernel(const GradAdamParams p) {
   pdl_wait();
+  if (p.longest < 0 && !any_longer_list(p, -p.longest)) return;  // (the launch of the other kernel did it)
   constexpr int T = 32 * W;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int G = (int)blockDim.x / T;
@@ -272,8 +273,7 @@ grad_adam_rows_kernel(const GradAdamParams p) {
   __syncthreads();
 
   // a kernel of this step that gave up on a bounded wait leaves stale inputs: parameters and moments stay as they are
-  const bool other = p.longest < 0 && !any_longer_list(p, -p.longest);  // (the other kernel's launch)
-  const bool skip = other || (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0);
+  const bool skip = p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0;
   const bool doD = p.WD != nullptr, doE = p.WE != nullptr;
   const float gmul = p.grad_mul != nullptr ? *p.grad_mul : 1.0f;
   const AdamConst h = {p.h.beta1, p.h.beta2, 1.0f - p.h.beta1, 1.0f - p.h.beta2, 1.0f / p.h.bias_correction2_sqrt,
@@ -556,10 +556,10 @@ grad_adam_rows_kernel(const GradAdamParams p) {
 namespace {
 
 // A list costs one CTA 40 ns an entry in one pass with two warps a row (above 256 columns) and 26 here, and the others may have ended long before: where
-// there is a longer one than this, which the kernels find out, both sides take this kernel. 512 columns, features of popularity 1 / (5 + rank), us in one pass ->
-// here: 4096 rows, 8192 tokens x 64: 475 -> 372; 8192, 4096 x 64: 348 -> 236; 4096, 4096 x 32: 168 -> 114; 4096, 2048 x 64: 132 -> 106; 512, 2048 x 16: 69 ->
-// 54; of equal popularity 4096, 4096 x 64: 181, 242. Batches of fewer tokens have no such list (4096, 1024 x 64: 87, 89 before there was the one pass) and
-// need no second launch, which costs 4 us with the look at the lists.
+// there is a longer one than this, which both kernels look at first, both sides take this kernel. 512 columns, features of popularity 1 / (5 + rank), us in
+// one pass -> here: 4096 rows, 8192 tokens x 64 codes: 475 -> 340; 8192, 4096 x 64: 348 -> 255; 4096, 4096 x 32: 168 -> 115; 4096, 2048 x 64: 132 -> 105; 512,
+// 2048 x 16: 69 -> 52; of equal popularity 4096, 4096 x 64: 179, 242. Batches of fewer tokens have no such list (4096, 1024 x 64: 80, 89 before
+// there was the one pass) and need no second launch, which costs 1 to 2 us.
 constexpr int kOnePassList = 1024;
 
 template <int W, int NCH>

@@ -172,6 +172,7 @@ template <int NCH, int Q>
 __global__ void __launch_bounds__(GB_THREADS, 1)
 grad_adam_both_kernel(const GradAdamParams p, const int W) {
   pdl_wait();
+  if (p.longest > 0 && any_longer_list(p, p.longest)) return;  // (the launch of the other kernel does it)
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int T = 32 * W, G = (int)blockDim.x / T, d = p.d;
   BothCtx c;
@@ -198,8 +199,7 @@ grad_adam_both_kernel(const GradAdamParams p, const int W) {
   __syncthreads();
 
   // a kernel of this step that gave up on a bounded wait leaves stale inputs: parameters and moments stay as they are
-  const bool other = p.longest > 0 && any_longer_list(p, p.longest);  // (the other kernel's launch)
-  const bool skip = other || (p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0);
+  const bool skip = p.status != nullptr && *reinterpret_cast<const volatile int*>(p.status) != 0;
   const float gmul = p.grad_mul != nullptr ? *p.grad_mul : 1.0f;
   const AdamConst h = {p.h.beta1, p.h.beta2, 1.0f - p.h.beta1, 1.0f - p.h.beta2, 1.0f / p.h.bias_correction2_sqrt,
                        p.h.lr / p.h.bias_correction1, p.h.eps};
