@@ -24,7 +24,7 @@
 // ONE TERM: the first proposal of the TopK encoder. One fp16 part an operand (half_rows_kernel), every row scaled to the top of fp16's range, and what
 // rounding took of a row measured and not bounded: 1.9e-4 of its norm as a rule, 4.9e-4 at most. The bound is five times as wide as with two
 // bf16 parts at a third of the operations. The largest end of every 32 columns goes along, so that the selection need not read the ends.
-// 4096 x 24576 x 768: two parts and three products 24 + 7 + 315 us -> 37 + 163 us. Bound by the epilogue (201 MB of ends), the MMAs take 92.
+// 4096 x 24576 x 768: two parts and three products 24 + 7 + 315 us -> 28 + 165 us. Bound by the epilogue (201 MB of ends), the MMAs take 92.
 #include <cuda_fp16.h>
 #include "fp32_exact.cuh"
 #include "kernels.h"

@@ -818,7 +818,7 @@ int row_topk_dense_launch(const __nv_bfloat16* H, int M, int N, int k, const flo
 //   With ends from one fp16 product (topk_narrow_launch) the bound and the columns come from the maxima of 32 columns, and the ends are
 // read only in groups that may hold something. Rows with more than 256 + 4 k columns in question are listed instead of summed up; where they are more
 // than an eighth of all rows, three bf16 products propose for the whole batch again, and the listed rows are selected from in the form above
-// (topk_wide_launch). Elsewhere the kernels of that second proposal leave at once, 11 us in all.
+// (topk_wide_launch). Elsewhere the kernels of that second proposal leave at once, 15 us in all.
 // 4096 x 24576 x 768, k 50: lower ends of three products, each row's read twice, 286 us; by maxima of those of one product 267, and 255
 // since the zeros (403 MB) leave while the bound is worked out. The rest are the rows of W, 3 kB for each of about 60 columns. Twelve rows of W at a time per warp take one
 // pass over those columns where eight take two (387 us with 72 columns a row).
